@@ -607,6 +607,7 @@ struct b200_ctx {
         float * X = nullptr, * Q = nullptr, * ATT = nullptr, * FFH = nullptr, * S = nullptr;
         uint8_t * rec = nullptr;
         int32_t * tokens = nullptr;
+        int * err = nullptr;     // pinned: raised by a kernel whose bounded wait ran out (pb_check)
     } pb;
     // persistent per-token kernel (token_kernel.cuh): phase list in device memory, grid-barrier counter, transposed scores
     Phase * d_plan = nullptr;
@@ -1321,6 +1322,7 @@ extern "C" void b200_ctx_free(b200_ctx * c) {
     cudaFree(c->x); cudaFree(c->q); cudaFree(c->att); cudaFree(c->ffh); cudaFree(c->warm_x); cudaFree(c->logits);
     cudaFree(c->d_cell_pos);
     cudaFree(c->pb.X); cudaFree(c->pb.Q); cudaFree(c->pb.ATT); cudaFree(c->pb.FFH); cudaFree(c->pb.S); cudaFree(c->pb.rec); cudaFree(c->pb.tokens);
+    cudaFreeHost(c->pb.err);
     cudaFree(c->d_trace); cudaFree(c->d_plan); cudaFree(c->d_bar); cudaFree(c->S_T); cudaFree(c->d_ttrace);
     cudaFree(c->S); cudaFree(c->tickets); cudaFree(c->amax_key); cudaFree(c->rope); cudaFree(c->d_state); cudaFree(c->d_out_tokens);
     cudaFreeHost(c->h_state); cudaFreeHost(c->h_logits); cudaFreeHost(c->h_tok);
@@ -1644,8 +1646,17 @@ static bool prefill_batch_usable(const b200_ctx * c, int n) {
     if (m.n_ff % 256 || m.n_embd % 256 || std::max(m.n_ff, m.n_embd) / 256 > 4 * 16 * 4) return false;
     return true;
 }
+static void pb_alloc_err(b200_ctx * c) {
+    CU(cudaHostAlloc(&c->pb.err, sizeof(int), cudaHostAllocMapped));
+    *c->pb.err = 0;
+}
+// after a synchronisation: a batch whose kernel gave up waiting left no result
+static void pb_check(b200_ctx * c) {
+    if (c->pb.err && *(volatile int *) c->pb.err) { *c->pb.err = 0; throw std::runtime_error("a prompt kernel's bounded wait ran out"); }
+}
 static void prefill_alloc(b200_ctx * c) {
     if (c->pb.cap) return;
+    if (!c->pb.err) pb_alloc_err(c);
     const b200_model & m = *c->m;
     const int T = PB_MAX_T, QD = m.n_head * m.head_dim;
     const size_t kmax = (size_t) std::max(std::max(m.n_ff, m.n_embd), QD);
@@ -1667,25 +1678,29 @@ static void prefill_alloc(b200_ctx * c) {
     c->pb.cap = T;
 }
 static bool has_q6k(const TMat * seg, int n_seg) { for (int i = 0; i < n_seg; i++) if (seg[i].type == T_Q6_K) return true; return false; }
-// K-quant launches run on the tensor cores (prefill_mma.cuh) when every segment has an even number of 32-row units
-static int g_prefill_mma = -1;         // 1 (default, the fastest measured): mma.sync (k_mma_batch), 2: tcgen05 (k_umma_batch), 0: the dp4a kernel
+// K-quant launches run on the tensor cores: tcgen05 (prefill_umma.cuh), or mma.sync (prefill_mma.cuh) for short rows
+static int g_prefill_mma = -1;         // 2 (default): tcgen05 (k_umma_batch) where it is the faster one, 1: mma.sync (k_mma_batch), 0: the dp4a kernel
 extern "C" void b200_set_prefill_mma(int mode) { g_prefill_mma = mode < 0 ? 0 : mode > 2 ? 2 : mode; }
-// record layout / kernel of a K-quant launch: 2 = k_umma_batch (segments of a multiple of 4 units), 1 = k_mma_batch (even), 0 = dp4a
+// A launch of k_umma_batch pays 2 to 4 us more than one of k_mma_batch before its first and after its last super-block (tensor memory, a longer pipeline),
+// and gains a quarter of a microsecond and more on each super-block between: rows of fewer than eight stay with mma.sync (k = 512..768, 8..96
+// tokens: 270 us a pass of 12 launches against 310; k = 4096, 31 tokens: 2520 against 2240 of 32).
+static constexpr int UM_MIN_K = 2048;
+// record layout / kernel of a launch: 3 = k_mma_batch_q80, 2 = k_umma_batch, 1 = k_mma_batch (segments of an even number of units), 0 = dp4a
 static int pb_mma_mode(const MatvecArgs & mv) {
-    if (g_prefill_mma < 0) { const char * e = getenv("BOOSTER_B200_PREFILL_MMA"); g_prefill_mma = e ? std::max(0, std::min(2, atoi(e))) : 1; }
+    if (g_prefill_mma < 0) { const char * e = getenv("BOOSTER_B200_PREFILL_MMA"); g_prefill_mma = e ? std::max(0, std::min(2, atoi(e))) : 2; }
     if (g_prefill_mma == 0) return 0;
+    bool even = true;
+    for (int i = 0; i < mv.n_seg; i++) even = even && !(mv.seg[i].n_units & 1);
     if (mv.act_q8_0) {   // Q8_0 x Q8_0: block-diagonal HMMA (k_mma_batch_q80)
-        for (int i = 0; i < mv.n_seg; i++) if (mv.seg[i].type != T_Q8_0 || (mv.seg[i].n_units & 1)) return 0;
-        return 3;
+        for (int i = 0; i < mv.n_seg; i++) if (mv.seg[i].type != T_Q8_0) return 0;
+        return even ? 3 : 0;
     }
-    int mode = g_prefill_mma;
     for (int i = 0; i < mv.n_seg; i++) {
         const int t = mv.seg[i].type;
         if (t != T_Q4_K && t != T_Q5_K && t != T_Q6_K) return 0;
-        if (mv.seg[i].n_units & 1) return 0;
-        if (mv.seg[i].n_units & 3) mode = 1;
     }
-    return mode;
+    if (g_prefill_mma == 2 && (mv.k >= UM_MIN_K || !even)) return 2;
+    return even ? 1 : 0;
 }
 static bool pb_use_mma(const MatvecArgs & mv) { return pb_mma_mode(mv) != 0; }
 static void pb_quant(b200_ctx * c, const float * X, int k, int T, const float * norm_w, int act_q8_0, int with_as, int mma = 0) {
@@ -1734,18 +1749,16 @@ static void pb_matmul(b200_ctx * c, const MatvecArgs & mv, int epi, int T, int p
         return;
     }
     if (mma_mode == 2) {
-        a.mb_a_bytes = (uint32_t) um_a_bytes(q6);
-        a.mb_raw_stride = (uint32_t) ((sb + 127) / 128 * 128);
-        a.mb_rec_copy = (uint32_t) um_rec_copy_bytes(q4, q5);
-        a.mb_stage_bytes = 4 * a.mb_raw_stride + (a.mb_rec_copy + 127) / 128 * 128;
-        const size_t budget = 226 * 1024;
-        a.mb_stages = (int) std::min<size_t>(UM_MAX_STAGES, (budget - a.mb_a_bytes) / a.mb_stage_bytes);
-        if (a.mb_stages < 2) throw std::runtime_error("k_umma_batch: shared memory layout does not fit");
-        const size_t smem_u = std::max((size_t) a.mb_a_bytes + (size_t) a.mb_stages * a.mb_stage_bytes, (size_t) 120 * 1024);   // one CTA per SM (TMEM)
+        a.mb_raw_stride = (uint32_t) sb;
+        a.mb_stage_bytes = (4 * a.mb_raw_stride + UM_REC_BYTES + 127) / 128 * 128;
+        a.mb_stages = (int) std::min<size_t>(UM_MAX_STAGES, ((size_t) 226 * 1024 - UM_FIXED_SMEM) / a.mb_stage_bytes);
+        a.um_tok_tiles = (T + UM_NT - 1) / UM_NT;
+        for (int i = 0; i < mv.n_seg; i++) a.um_row_tiles += (mv.seg[i].n_units + 3) / 4;
+        a.err = c->pb.err;
+        const size_t smem_u = (size_t) UM_FIXED_SMEM + (size_t) a.mb_stages * a.mb_stage_bytes;   // (more than half an SM's: one CTA per SM)
         static size_t attr_u[64] = {0};
         raise_smem(k_umma_batch, smem_u, attr_u, c->device);
-        const dim3 grid_u((unsigned) ((T + UM_NT - 1) / UM_NT), (unsigned) (a.n_units / 4));
-        k_umma_batch<<<grid_u, UM_WARPS * 32, smem_u, c->st>>>(a);
+        k_umma_batch<<<(unsigned) std::min(c->sm_count, a.um_row_tiles * a.um_tok_tiles), UM_THREADS, smem_u, c->st>>>(a);
         c->launches++;
         return;
     }
@@ -1943,6 +1956,7 @@ extern "C" int b200_decode(b200_ctx * c, const int32_t * tokens, int n, int pos0
             g_only_kind = -1;
             if (logits_out) CU(cudaMemcpyAsync(c->h_logits, c->logits, (size_t) m.n_vocab * 4, cudaMemcpyDeviceToHost, c->st));
             CU(cudaStreamSynchronize(c->st));
+            pb_check(c);
             if (logits_out) std::memcpy(logits_out, c->h_logits, (size_t) m.n_vocab * 4);
             c->t_prompt_us += now_us() - t0; c->n_prompt += n;
             return 0;
@@ -2534,6 +2548,7 @@ extern "C" int b200_stage_sync(b200_ctx * c) {
         if (c->stack) { b200::stack_sync(c->stack); return 0; }
         CU(cudaSetDevice(c->m->device));
         CU(cudaStreamSynchronize(c->st));
+        pb_check(c);
         return 0;
     } catch (const std::exception & e) { return set_err(e.what()); }
 }
@@ -2546,6 +2561,7 @@ extern "C" int b200_stage_logits(b200_ctx * c, float * logits_out) {
         CU(cudaSetDevice(c->m->device));
         CU(cudaMemcpyAsync(c->h_logits, c->logits, (size_t) c->m->n_vocab * 4, cudaMemcpyDeviceToHost, c->st));
         CU(cudaStreamSynchronize(c->st));
+        pb_check(c);
         std::memcpy(logits_out, c->h_logits, (size_t) c->m->n_vocab * 4);
         return 0;
     } catch (const std::exception & e) { return set_err(e.what()); }
@@ -2560,6 +2576,7 @@ extern "C" float * b200_stage_logits_view(b200_ctx * c) {
         CU(cudaSetDevice(c->m->device));
         CU(cudaMemcpyAsync(c->h_logits, c->logits, (size_t) c->m->n_vocab * 4, cudaMemcpyDeviceToHost, c->st));
         CU(cudaStreamSynchronize(c->st));
+        pb_check(c);
         return c->h_logits;
     } catch (const std::exception & e) { set_err(e.what()); return nullptr; }
 }
@@ -2580,6 +2597,7 @@ extern "C" int b200_stage_argmax(b200_ctx * c, int32_t * token_out) {
         enqueue_argmax(c, 0);
         CU(cudaMemcpyAsync(&c->h_state->token, c->d_out_tokens, 4, cudaMemcpyDeviceToHost, c->st));
         CU(cudaStreamSynchronize(c->st));
+        pb_check(c);
         *token_out = c->h_state->token;
         return 0;
     } catch (const std::exception & e) { return set_err(e.what()); }
@@ -2742,6 +2760,8 @@ extern "C" int b200_op_mul_mat(int type, const void * w, int64_t n_rows, int64_t
         int dev = 0; CU(cudaGetDevice(&dev));
         tmp.device = dev;
         tmp.pb.rec = drec.as<uint8_t>();
+        pb_alloc_err(&tmp);
+        std::unique_ptr<int, cudaError_t (*)(void *)> err_owner(tmp.pb.err, cudaFreeHost);
         MatvecArgs a{};
         a.seg[0] = d.m; a.n_seg = 1; a.n_units = d.m.n_units; a.k = (int) k; a.act_q8_0 = type == T_Q8_0;
         const int was = type == T_Q6_K;
@@ -2751,6 +2771,7 @@ extern "C" int b200_op_mul_mat(int type, const void * w, int64_t n_rows, int64_t
         std::vector<float> hy((size_t) T * rows_pad);
         CU(cudaMemcpyAsync(hy.data(), dy.p, hy.size() * 4, cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
+        pb_check(&tmp);
         for (int64_t t = 0; t < T; t++) memcpy(y + t * n_rows, hy.data() + t * rows_pad, (size_t) n_rows * 4);
         tmp.pb.rec = nullptr;
         return 0;

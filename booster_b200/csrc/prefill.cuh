@@ -288,6 +288,8 @@ struct MatmulBatchArgs {
     // k_mma_batch (prefill_mma.cuh): shared-memory layout chosen on the host
     uint32_t mb_a_bytes, mb_raw_stride, mb_stage_bytes, mb_rec_copy;
     int mb_stages;
+    int um_row_tiles, um_tok_tiles;       // k_umma_batch: 128-row tiles (of every segment by itself), 32-token tiles
+    int * err;                            // raised by a kernel whose bounded wait ran out
 };
 
 // resolve a unit against the segments (same rule as describe_unit)

@@ -16,11 +16,10 @@
 //     = 8 groups x (lo, hi); for Q4_K the four lanes l of the reference's _mm_madd_epi16 are four B columns per token.
 //   * the chain step acc = fma(d, C, acc) then runs on the MMA's C fragment in registers, super-block after super-block.
 //
-// mma.sync.m16n8k16 (HMMA) is the default, not tcgen05: the accumulator of every (super-block, lane) must come back to the
-// register file for its own fp32 chain step — 8 + 4 FFMA per 256 MACs and output — so the kernel is bound by that CUDA-core
-// epilogue, by the 12 live fp32 chains per output element (a 64 x 32 tile fills the register file) and by fragment traffic
-// through shared memory, not by tensor throughput (ncu: HMMA pipe 22-26 % busy). The tcgen05 / TMEM variant is
-// prefill_umma.cuh: bit-exact too, measured slower (its header says why).
+// mma.sync.m16n8k16 (HMMA): the accumulator of every (super-block, lane) is in the register file for its own fp32 chain step — 8 + 4
+// FFMA per 256 MACs and output — so the kernel is bound by that CUDA-core epilogue and by fragment traffic through shared memory (ncu:
+// HMMA pipe 22-26 % busy, shared-memory pipe 60 %). Long rows go to the tcgen05 kernel (prefill_umma.cuh), which takes the
+// fragments off the shared memory; this one has the shorter pipeline and serves short rows.
 //
 // Shape: CTA = 64 rows (two 32-row units of the tiled weight layout) x 32 tokens, 16 warps. Per super-block (K step):
 //   TMA bulk copies: the two raw weight tiles + the chunk's activation record block (fp16, MMA order, written by

@@ -191,6 +191,25 @@ def test_mul_mat_batch_extremes(name):
         assert np.array_equal(y[i], yr), f"token {i}: max abs diff {np.abs(y[i] - yr).max()}"
 
 
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K"])
+@pytest.mark.parametrize("shape", [(32, 2048, 1), (160, 2304, 32), (416, 4096, 65), (20480, 2048, 40)])
+def test_mul_mat_batch_tcgen05_edges(name, shape):
+    """k_umma_batch where its tiles end: one unit of a 128-row tile, the fewest super-blocks its rule takes, one token past a tile, more
+    tiles than SMs (a CTA's second tile starts behind its first one's epilogue) — the reference's bits"""
+    n, k, T = shape
+    rng = np.random.default_rng(n + k + T)
+    w = _extreme_blocks(name, n, k, rng)
+    x = (rng.standard_normal((T, k)) * rng.choice([0.01, 1.0, 30.0], size=(T, 1))).astype(np.float32)
+    engine.set_prefill_mma(2)
+    try:
+        y = engine.op_mul_mat(TYPES[name], w, n, k, x)
+    finally:
+        engine.set_prefill_mma(1)
+    for i in sorted({0, T // 2, T - 1}):
+        yr = port.mul_mat_vec(TYPES[name], w, n, k, x[i])
+        assert np.array_equal(y[i], yr), f"token {i}: max abs diff {np.abs(y[i] - yr).max()}"
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0"])
 def test_mul_mat_batch_kernel_variants(name, mode):
