@@ -1667,6 +1667,8 @@ static void prefill_alloc(b200_ctx * c) {
     {
         const size_t per_token = (size_t) m.n_head * c->n_ctx * 4;
         c->pb.att_z = (int) std::max<size_t>(64, std::min<size_t>((size_t) T, PB_SCORE_BYTES / per_token / 32 * 32));
+        // a long context cuts the batch into launch groups: each as many tokens as fill whole waves of P.V blocks (8 rows, two blocks per SM)
+        if (c->pb.att_z < T) { const int per_wave = std::max(1, c->sm_count * 16 / m.n_head); if (c->pb.att_z > per_wave) c->pb.att_z = c->pb.att_z / per_wave * per_wave; }
         if (g_prefill_attn_batch == 0) c->pb.att_z = 64;   // (the per-token kernels index blockIdx.z the same way)
     }
     CU(cudaMalloc(&c->pb.S, (size_t) c->pb.att_z * m.n_head * c->n_ctx * 4));
@@ -1803,14 +1805,21 @@ static void pb_attention(b200_ctx * c, int li, int T, int pos0) {
             if (!launch_attention_2k<GQA>(c, a, n_pad_max, nz)) throw std::runtime_error("batched attention does not fit");
             continue;
         }
-        const dim3 gs((unsigned) a.n_head_kv, (unsigned) ((n_pad_max + ATT_TILE - 1) / ATT_TILE), (unsigned) ((nz + SCB_TQ - 1) / SCB_TQ));
-        k_attn_scores_batch<GQA><<<gs, ATT_THREADS, 0, c->st>>>(a, nz);
-        k_attn_softmax_rows<<<(unsigned) ((nz * a.n_head + 7) / 8), 256, 0, c->st>>>(a, nz);
+        const dim3 gs((unsigned) a.n_head_kv, (unsigned) ((n_pad_max + SCB_KEYS - 1) / SCB_KEYS), (unsigned) ((nz + SCB_TQ - 1) / SCB_TQ));
+        constexpr size_t smem_sc = (size_t) SCB_TQ * GQA * 128 * 4;
+        static size_t attr_sc[64] = {0};
+        if (smem_sc > 48 * 1024) raise_smem(k_attn_scores_batch<GQA>, smem_sc, attr_sc, c->device);
+        k_attn_scores_batch<GQA><<<gs, SCB_KEYS, smem_sc, c->st>>>(a, nz);
+        const unsigned rows = (unsigned) (nz * a.n_head);
+        const int groups = (n_pad_max / 16 + SMX_THREADS - 1) / SMX_THREADS;
+        if (n_pad_max < SMX_MIN_ROW || groups > SMX_MAX_G) k_attn_softmax_rows<<<(rows + 7) / 8, 256, 0, c->st>>>(a, nz);
+        else if (groups == 1) k_attn_softmax_block<1><<<rows, SMX_THREADS, 0, c->st>>>(a, nz);
+        else if (groups == 2) k_attn_softmax_block<2><<<rows, SMX_THREADS, 0, c->st>>>(a, nz);
+        else k_attn_softmax_block<SMX_MAX_G><<<rows, SMX_THREADS, 0, c->st>>>(a, nz);
         static size_t attr_pvb[64] = {0};
-        raise_smem(k_attn_pv_batch<GQA>, pvb_smem_bytes(), attr_pvb, c->device);
+        raise_smem(k_attn_pv_batch<GQA>, PVB_SMEM, attr_pvb, c->device);
         constexpr int TQ = PVB_ROWS / GQA;
-        const dim3 gp((unsigned) a.n_head_kv, (unsigned) (128 / PVB_DIMS), (unsigned) ((nz + TQ - 1) / TQ));
-        k_attn_pv_batch<GQA><<<gp, 256, pvb_smem_bytes(), c->st>>>(a, nz);
+        k_attn_pv_batch<GQA><<<dim3((unsigned) a.n_head_kv, (unsigned) ((nz + TQ - 1) / TQ)), PVB_THREADS, PVB_SMEM, c->st>>>(a, nz);
         c->launches += 3;
     }
 }

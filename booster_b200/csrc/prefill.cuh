@@ -1,15 +1,9 @@
 // prefill.cuh — prompt batches (llama_decode with n_tokens > 1): the same arithmetic as the per-token kernels, with every
 // weight tile fetched ONCE for a chunk of 64 tokens instead of once per token.
 //
-// Why not tensor cores (ggml-cuda's mul_mat_q): the reference's CPU result keeps EIGHT separate fp32
-// accumulators per output element — AVX2 lane m owns bytes 4m..4m+3 of every 32-byte group, and acc[m] = fma(d_block,
-// (float) isum[m], acc[m]) runs block after block before the final hsum (cpp/ggml/src/ggml-quants.c:5361-5382, 6914-6977).
-// Bit-exact parity therefore needs the integer sum of every 4-byte group of every (row, token) SEPARATELY, scaled and
-// chained in fp32 in block order. An int8 MMA (mma.sync k = 16/32, tcgen05 kind::i8 k = 32) sums at least 16 products per
-// output; the 4-byte granularity is exactly dp4a's. A tensor-core prefill is possible only by giving up bit-exactness,
-// and with re-quantized activations between mat-muls that costs ~1e-2 on the logits, outside the 1e-3 bar.
-// So the batch path is a dp4a kernel whose gain is data reuse: weights are read from HBM/L2 once per 64 tokens and the
-// per-token work (integers + chains) runs out of shared memory — it is issue-bound, not HBM-bound.
+// The products run on the tensor cores (prefill_umma.cuh, prefill_mma.cuh); k_matmul_batch here is the dp4a kernel they are measured
+// against, and takes what they do not: the reference's CPU result keeps EIGHT separate fp32 accumulators per output element (AVX2 lane m owns bytes
+// 4m..4m+3 of every 32-byte group, cpp/ggml/src/ggml-quants.c:5361-5382, 6914-6977), and the 4-byte granularity is exactly dp4a's.
 //
 //   k_embed_batch   token_embd rows of T tokens -> X[T][n_embd]
 //   k_quant_batch   per token: [RMSNorm * w] + Q8_K / Q8_0 quantization (prologue_quantize, the decode path's own code) into
@@ -19,7 +13,6 @@
 //                   tile(s) + one of the chunk's activation records into a 2-stage shared-memory ring (full / empty
 //                   mbarriers); every warp computes tile_ints for its 4 tokens and advances 4 x 12 fp32 chains in
 //                   registers; epilogues as in the per-token kernel (RoPE + KV-cache rows, +residual, SiLU*up, store)
-// Attention of a batch runs the per-token attention kernels with the token index in blockIdx.z (kernels.cuh).
 #pragma once
 #include "kernels.cuh"
 
@@ -88,11 +81,11 @@ __global__ void __launch_bounds__(512) k_quant_batch(const QuantBatchArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// attention of a prompt batch: k_attn_scores (kernels.cuh, token in blockIdx.z) writes the raw score rows, then
+// attention of a prompt batch: k_attn_scores_batch writes the raw score rows, then
 //   k_attn_softmax_rows  one warp per (token, head) row, in place: k_attn_softmax's arithmetic (max, ggml_v_expf, per-16
 //                        _mm512_reduce_add_ps sums accumulated in double, * (float)(1/sum)), each row normalised ONCE
-//   k_attn_pv_batch      CTA = (KV head, 16 output dims, 32 / GQA tokens): every V chunk is staged once for the 32 (token,
-//                        head) rows of the CTA; thread (chain c, dim) advances the 32 rows' tinyBLAS chains t = c, c+16, ...
+//   k_attn_softmax_block the same for long rows, a block per row
+//   k_attn_pv_batch      tinyBLAS' 16 chains t = c, c+16, ... of every output, rows and dims tiled in registers.
 //                        A token's probabilities end at its own padded length; beyond it p = 0 and fma(v, 0, acc) == acc,
 //                        which is what the reference's masked (-inf -> 0) columns contribute (cpp/src/llama.cpp:14132-14200).
 // ------------------------------------------------------------------------------------------------------------
@@ -138,135 +131,265 @@ __global__ void __launch_bounds__(256) k_attn_softmax_rows(const AttnArgs a, int
     }
 }
 
-// scores of a prompt batch: CTA = (KV head, 64 keys, 8 tokens). The K rows of the tile are loaded ONCE into registers (4 lanes per
-// key row, as in k_attn_scores) and every (token, head) of the CTA runs ggml_vec_dot_f16 against them: q rounded to f16, 4
-// accumulators x 16 lanes over i in {0, 64}, (0+2)+(1+3), _mm512_reduce_add_ps (cpp/ggml/src/ggml.c:12345-12371) — the batch > 1
-// branch of k_attn_scores, token by token. A token's row ends at its own padded length (-inf from its n_kv to there).
-static constexpr int SCB_TQ = 8;
-template <int GQA>
-__global__ void __launch_bounds__(ATT_THREADS) k_attn_scores_batch(const AttnArgs a, int nz) {
-    constexpr int HD = 128;
-    __shared__ __align__(16) float qs[SCB_TQ][GQA][HD];
-    const int g = blockIdx.x, tile = blockIdx.y, z0 = blockIdx.z * SCB_TQ, tid = threadIdx.x;
-    const int ntok = min(SCB_TQ, nz - z0);
-    const int n_kv_last = a.n_kv_override + z0 + ntok - 1;
-    if (tile * ATT_TILE >= (n_kv_last + 31) / 32 * 32) return;
-    const int t = tile * ATT_TILE + (tid >> 2), c4 = tid & 3;
-    uint2 kv[8];
+// The same row by a whole block: every thread keeps its groups of 16 scores in registers, so that a row crosses memory once in and once out. The
+// sums of 16 meet in shared memory and one warp adds them in k_attn_softmax_rows' order, bit for bit. A warp per row reads a long row three times
+// and writes it twice, mostly past the L1: 288 tokens x 32 heads x 6288 keys 119 us against 225.
+static constexpr int SMX_THREADS = 256, SMX_MAX_G = 4;        // rows of up to 256 * 16 * 4 = 16384 scores
+static constexpr int SMX_MIN_ROW = 2048;                      // (shorter rows: most of a block would idle)
+template <int G>
+__global__ void __launch_bounds__(SMX_THREADS) k_attn_softmax_block(const AttnArgs a, int nz) {
+    __shared__ float wmax[SMX_THREADS / 32], gsum[G * SMX_THREADS];
+    __shared__ float inv_s;
+    const int tid = threadIdx.x, lane = tid & 31, row = blockIdx.x;
+    const int z = row / a.n_head, h = row - z * a.n_head;
+    const int n_pad = (a.n_kv_override + z + 31) / 32 * 32, n16 = n_pad / 16;
+    float * S = a.S + (size_t) z * a.zs + (size_t) h * a.s_stride;
+    float4 v[G][4];
+    float mx = -INFINITY;
 #pragma unroll
-    for (int s = 0; s < 8; s++) kv[s] = make_uint2(0u, 0u);
-    if (t < n_kv_last) {
-        const uint2 * kr = reinterpret_cast<const uint2 *>(a.k_cache + (size_t) t * a.kv_dim + g * HD + 4 * c4);
+    for (int i = 0; i < G; i++) {
+        const int gi = tid + i * SMX_THREADS;
+        if (gi < n16) {
+            const float4 * r4 = reinterpret_cast<const float4 *>(S + 16 * gi);
 #pragma unroll
-        for (int s = 0; s < 8; s++) kv[s] = kr[s * 4];                        // 4 halfs at element 16s + 4c4
+            for (int q = 0; q < 4; q++) v[i][q] = r4[q];
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; q++) v[i][q] = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        }
     }
-    for (int i = tid; i < ntok * GQA * HD; i += ATT_THREADS) {
-        const int tok = i / (GQA * HD), rem = i - tok * (GQA * HD);
-        const float v = a.q[(size_t) (z0 + tok) * a.zq + (size_t) (g * GQA) * HD + rem];
-        (&qs[0][0][0])[i] = __half2float(__float2half_rn(v));                 // src1 converted to the vec_dot_type F16
-    }
-    float kf[8][4];
 #pragma unroll
-    for (int s = 0; s < 8; s++) {
-        const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&kv[s].x));
-        const float2 f1 = __half22float2(*reinterpret_cast<const __half2 *>(&kv[s].y));
-        kf[s][0] = f0.x; kf[s][1] = f0.y; kf[s][2] = f1.x; kf[s][3] = f1.y;
+    for (int i = 0; i < G; i++) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) mx = fmaxf(fmaxf(mx, fmaxf(v[i][q].x, v[i][q].y)), fmaxf(v[i][q].z, v[i][q].w));
+    }
+    mx = warp_max(mx);
+    if (lane == 0) wmax[tid >> 5] = mx;
+    __syncthreads();
+    mx = wmax[0];
+#pragma unroll
+    for (int w = 1; w < SMX_THREADS / 32; w++) mx = fmaxf(mx, wmax[w]);
+#pragma unroll 1
+    for (int i = 0; i < G; i++) {
+        const int gi = tid + i * SMX_THREADS;
+        if (gi >= n16) break;
+#pragma unroll
+        for (int j = 0; j < G; j++) if (j == i) {
+            float4 t[2];
+#pragma unroll
+            for (int pq = 0; pq < 2; pq++) {                   // float4 pairs {0, 2} and {1, 3}: a[8+i] + a[i]
+                float4 lo = v[j][pq], hi = v[j][pq + 2];
+                lo.x = v_expf(__fsub_rn(lo.x, mx)); lo.y = v_expf(__fsub_rn(lo.y, mx)); lo.z = v_expf(__fsub_rn(lo.z, mx)); lo.w = v_expf(__fsub_rn(lo.w, mx));
+                hi.x = v_expf(__fsub_rn(hi.x, mx)); hi.y = v_expf(__fsub_rn(hi.y, mx)); hi.z = v_expf(__fsub_rn(hi.z, mx)); hi.w = v_expf(__fsub_rn(hi.w, mx));
+                v[j][pq] = lo; v[j][pq + 2] = hi;
+                t[pq] = make_float4(__fadd_rn(hi.x, lo.x), __fadd_rn(hi.y, lo.y), __fadd_rn(hi.z, lo.z), __fadd_rn(hi.w, lo.w));
+            }
+            const float u0 = __fadd_rn(t[1].x, t[0].x), u1 = __fadd_rn(t[1].y, t[0].y), u2 = __fadd_rn(t[1].z, t[0].z), u3 = __fadd_rn(t[1].w, t[0].w);
+            gsum[gi] = __fadd_rn(__fadd_rn(u0, u2), __fadd_rn(u1, u3));
+        }
     }
     __syncthreads();
-#pragma unroll 1
-    for (int tok = 0; tok < ntok; tok++) {
-        const int n_kv = a.n_kv_override + z0 + tok, n_pad = (n_kv + 31) / 32 * 32;
-        if (t >= n_pad) continue;                                  // n_pad % 32 == 0 and a warp holds 8 consecutive keys: warp-uniform
-        float * Srow = a.S + (size_t) (z0 + tok) * a.zs + (size_t) (g * GQA) * a.s_stride + t;
-#pragma unroll 1
-        for (int h = 0; h < GQA; h++) {
-            float aj[4][4];
+    if (tid < 32) {
+        double part = 0.0;
+        for (int gi = lane; gi < n16; gi += 32) part += (double) gsum[gi];
+        const double sum = warp_sum_d(part);
+        if (lane == 0) inv_s = (float) (1.0 / sum);
+    }
+    __syncthreads();
+    const float inv = inv_s;
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const float4 q0 = *reinterpret_cast<const float4 *>(&qs[tok][h][16 * j + 4 * c4]);
-                const float4 q1 = *reinterpret_cast<const float4 *>(&qs[tok][h][64 + 16 * j + 4 * c4]);
-                aj[j][0] = __fmaf_rn(kf[4 + j][0], q1.x, __fmul_rn(kf[j][0], q0.x));
-                aj[j][1] = __fmaf_rn(kf[4 + j][1], q1.y, __fmul_rn(kf[j][1], q0.y));
-                aj[j][2] = __fmaf_rn(kf[4 + j][2], q1.z, __fmul_rn(kf[j][2], q0.z));
-                aj[j][3] = __fmaf_rn(kf[4 + j][3], q1.w, __fmul_rn(kf[j][3], q0.w));
+    for (int i = 0; i < G; i++) {
+        const int gi = tid + i * SMX_THREADS;
+        if (gi < n16) {
+            float4 * r4 = reinterpret_cast<float4 *>(S + 16 * gi);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                float4 x = v[i][q];
+                x.x = __fmul_rn(x.x, inv); x.y = __fmul_rn(x.y, inv); x.z = __fmul_rn(x.z, inv); x.w = __fmul_rn(x.w, inv);
+                r4[q] = x;
             }
-            float ch[4], t3[4], t6[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) ch[e] = __fadd_rn(__fadd_rn(aj[0][e], aj[2][e]), __fadd_rn(aj[1][e], aj[3][e]));
-#pragma unroll
-            for (int e = 0; e < 4; e++) t3[e] = __fadd_rn(__shfl_xor_sync(0xffffffffu, ch[e], 2), ch[e]);
-#pragma unroll
-            for (int e = 0; e < 4; e++) t6[e] = __fadd_rn(__shfl_xor_sync(0xffffffffu, t3[e], 1), t3[e]);
-            const float res = __fadd_rn(__fadd_rn(t6[0], t6[2]), __fadd_rn(t6[1], t6[3]));
-            if (c4 == 0) Srow[(size_t) h * a.s_stride] = t < n_kv ? __fmul_rn(res, a.scale) : -INFINITY;
         }
     }
 }
 
-static constexpr int PVB_ROWS = 32;            // (token, head) rows per CTA: 32 / GQA tokens x GQA heads
-static constexpr int PVB_CHUNK = 256;          // positions staged at a time
-static constexpr int PVB_DIMS = 16;
-__host__ __device__ constexpr size_t pvb_smem_bytes() {
-    return (size_t) PVB_ROWS * PVB_CHUNK * 4 + (size_t) PVB_CHUNK * PVB_DIMS * 2 > (size_t) PVB_ROWS * 16 * (PVB_DIMS + 1) * 4
-               ? (size_t) PVB_ROWS * PVB_CHUNK * 4 + (size_t) PVB_CHUNK * PVB_DIMS * 2 : (size_t) PVB_ROWS * 16 * (PVB_DIMS + 1) * 4;
-}
+// packed fp32 pairs: each half is the IEEE operation of the scalar instruction (a packed multiply whose only use is a packed add is
+// contracted by the compiler: products that are added are not formed with these)
+__device__ __forceinline__ uint64_t pair_of(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ float2 unpair(uint64_t p) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p)); return r; }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+
+// scores of a prompt batch: CTA = (KV head, 128 keys, 16 tokens), a thread = one key, whose 128 values sit in registers as packed pairs for all
+// 16 x GQA dot products. Each is ggml_vec_dot_f16 on q rounded to f16: 4 accumulators x 16 lanes over i in {0, 64}, (0+2)+(1+3),
+// _mm512_reduce_add_ps (cpp/ggml/src/ggml.c:12345-12371) — the batch > 1 branch of k_attn_scores — in 96 packed instructions and 32 broadcast
+// loads of q, with no exchange between lanes. Bound by those loads and the packed arithmetic together (ncu: shared-memory pipe 84 %, fp32 pipe 58 %). Four
+// lanes per key with scalar arithmetic: 512 tokens x 32 heads x 6256 keys 2.08 ms, now 1.03 ms. Four lanes sharing four keys (a quarter of the loads, 12
+// shuffles): 1.02 ms, not worth its code. A token's row ends at its own padded length (-inf from its n_kv to there).
+static constexpr int SCB_TQ = 16, SCB_KEYS = 128;
 template <int GQA>
-__global__ void __launch_bounds__(256) k_attn_pv_batch(const AttnArgs a, int nz) {
-    constexpr int HD = 128, TQ = PVB_ROWS / GQA;
-    extern __shared__ __align__(16) uint8_t pvb_dyn[];
-    float * ps = reinterpret_cast<float *>(pvb_dyn);                                        // [32 rows][PVB_CHUNK]
-    __half (*vs)[PVB_DIMS] = reinterpret_cast<__half (*)[PVB_DIMS]>(pvb_dyn + (size_t) PVB_ROWS * PVB_CHUNK * 4);
-    const int g = blockIdx.x, slice = blockIdx.y, z0 = blockIdx.z * TQ, tid = threadIdx.x;
-    const int c = tid / PVB_DIMS, dl = tid % PVB_DIMS;
-    const int ntok = min(TQ, nz - z0);
-    const int n_kv_last = a.n_kv_override + z0 + ntok - 1;     // cells attended by the CTA's last token
-    const int n_max = (n_kv_last + 31) / 32 * 32;
-    const __half * vbase = a.v_cache + g * HD + slice * PVB_DIMS;
-    float acc[PVB_ROWS];
+__global__ void __launch_bounds__(SCB_KEYS, 3) k_attn_scores_batch(const AttnArgs a, int nz) {
+    constexpr int HD = 128;
+    extern __shared__ __align__(16) uint8_t scb_dyn[];
+    float * qs = reinterpret_cast<float *>(scb_dyn);                          // [SCB_TQ * GQA][HD]
+    const int g = blockIdx.x, tile = blockIdx.y, z0 = blockIdx.z * SCB_TQ, tid = threadIdx.x;
+    const int ntok = min(SCB_TQ, nz - z0);
+    const int n_kv_last = a.n_kv_override + z0 + ntok - 1;
+    if (tile * SCB_KEYS >= (n_kv_last + 31) / 32 * 32) return;
+    const int t = tile * SCB_KEYS + tid;
+    for (int i = tid; i < ntok * GQA * (HD / 4); i += SCB_KEYS) {
+        const int tok = i / (GQA * (HD / 4)), rem = i - tok * (GQA * (HD / 4));
+        const float4 v = *reinterpret_cast<const float4 *>(a.q + (size_t) (z0 + tok) * a.zq + (size_t) (g * GQA) * HD + 4 * rem);
+        reinterpret_cast<float4 *>(qs)[i] = make_float4(__half2float(__float2half_rn(v.x)), __half2float(__float2half_rn(v.y)),     // src1 converted to
+                                                        __half2float(__float2half_rn(v.z)), __half2float(__float2half_rn(v.w)));    // the vec_dot_type F16
+    }
+    uint64_t kp[HD / 2];
 #pragma unroll
-    for (int r = 0; r < PVB_ROWS; r++) acc[r] = 0.f;
-    for (int t0 = 0; t0 < n_max; t0 += PVB_CHUNK) {
-        const int len = min(PVB_CHUNK, n_max - t0);
-        if (t0) __syncthreads();
-        for (int i = tid; i < len * 2; i += 256) {             // V rows: 2 x 16 bytes; rows beyond the last cell are zero
-            const int t = t0 + (i >> 1);
-            if (t < n_kv_last) cp_async16(&vs[i >> 1][(i & 1) * 8], vbase + (size_t) t * a.kv_dim + (i & 1) * 8);
-            else *reinterpret_cast<uint4 *>(&vs[i >> 1][(i & 1) * 8]) = make_uint4(0u, 0u, 0u, 0u);
-        }
-        for (int i = tid; i < PVB_ROWS * (len / 4); i += 256) {
-            const int r = i / (len / 4), j = i - r * (len / 4), tok = r / GQA, h = r - tok * GQA, t = t0 + 4 * j;
-            const int n_pad_z = (a.n_kv_override + z0 + tok + 31) / 32 * 32;
-            float * dst = ps + (size_t) r * PVB_CHUNK + 4 * j;
-            if (tok < ntok && t < n_pad_z) cp_async16(dst, a.S + (size_t) (z0 + tok) * a.zs + (size_t) (g * GQA + h) * a.s_stride + t);
-            else *reinterpret_cast<float4 *>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        cp_async_commit();
-        cp_async_wait<0>();
-        __syncthreads();
-        const int steps = len / 16;
-#pragma unroll 2
-        for (int s = 0; s < steps; s++) {
-            const int tt = 16 * s + c;
-            const float v = __half2float(vs[tt][dl]);
+    for (int s = 0; s < HD / 8; s++) {
+        uint4 kv = make_uint4(0u, 0u, 0u, 0u);
+        if (t < n_kv_last) kv = *reinterpret_cast<const uint4 *>(a.k_cache + (size_t) t * a.kv_dim + g * HD + 8 * s);
+        const uint32_t w[4] = {kv.x, kv.y, kv.z, kv.w};
 #pragma unroll
-            for (int r = 0; r < PVB_ROWS; r++) acc[r] = __fmaf_rn(v, ps[(size_t) r * PVB_CHUNK + tt], acc[r]);
-        }
+        for (int i = 0; i < 4; i++) { const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[i])); kp[4 * s + i] = pair_of(f.x, f.y); }
     }
     __syncthreads();
-    float (*red)[16][PVB_DIMS + 1] = reinterpret_cast<float (*)[16][PVB_DIMS + 1]>(pvb_dyn);
+#pragma unroll 1
+    for (int r = 0; r < ntok * GQA; r++) {
+        const int tok = r / GQA, h = r - tok * GQA;
+        const int n_kv = a.n_kv_override + z0 + tok;
+        if (t >= (n_kv + 31) / 32 * 32) continue;                  // (a multiple of 32: warp-uniform)
+        const ulonglong2 * q = reinterpret_cast<const ulonglong2 *>(qs + (size_t) r * HD);       // two pairs each
+        uint64_t ch[8];
 #pragma unroll
-    for (int r = 0; r < PVB_ROWS; r++) red[r][c][dl] = acc[r];
+        for (int p = 0; p < 8; p += 2) {
+            uint64_t x[4], y[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const ulonglong2 q0 = q[(16 * j + 2 * p) / 4], q1 = q[(64 + 16 * j + 2 * p) / 4];
+                x[j] = fma2(kp[32 + 8 * j + p], q1.x, mul2(kp[8 * j + p], q0.x));
+                y[j] = fma2(kp[32 + 8 * j + p + 1], q1.y, mul2(kp[8 * j + p + 1], q0.y));
+            }
+            ch[p] = add2(add2(x[0], x[2]), add2(x[1], x[3]));
+            ch[p + 1] = add2(add2(y[0], y[2]), add2(y[1], y[3]));
+        }
+        uint64_t t3[4], t6[2];
+#pragma unroll
+        for (int i = 0; i < 4; i++) t3[i] = add2(ch[4 + i], ch[i]);
+#pragma unroll
+        for (int i = 0; i < 2; i++) t6[i] = add2(t3[2 + i], t3[i]);
+        const float2 u = unpair(add2(t6[0], t6[1]));
+        const float res = __fadd_rn(u.x, u.y);
+        a.S[(size_t) (z0 + tok) * a.zs + (size_t) (g * GQA + h) * a.s_stride + t] = t < n_kv ? __fmul_rn(res, a.scale) : -INFINITY;
+    }
+}
+
+// P.V of a prompt batch: CTA = (KV head, 8 (token, head) rows), all 128 dims, two CTAs per SM. A half-warp is one of tinyBLAS' 16 chains (positions
+// c, c + 16, ...), a lane 8 rows x 8 dims: 32 packed fmas per position on one 16-byte load of V (f16, converted in registers) and two of p.
+// Bound by the fp32 pipe, with the loads close behind. What was tried on the way (512 tokens x 32 heads x 6256 keys): a thread = chain x dim, 32 rows, a load
+// of p per fma 1.90 ms (start); lane = 4 rows x 16 dims on V staged as fp32 1.06 ms (shared-memory pipe 79 %), now 0.88 ms.
+static constexpr int PVB_CHUNK = 64;           // positions staged at a time
+static constexpr int PVB_STAGES = 3;
+static constexpr int PVB_THREADS = 256;
+static constexpr int PVB_ROWS = 8;             // (token, head) rows per CTA
+static constexpr int PVB_PS = PVB_ROWS + 4;    // floats of p per position (16-byte rows, stores two-way conflicted)
+static constexpr int PVB_V_BYTES = PVB_CHUNK * 128 * 2, PVB_BUF_BYTES = PVB_V_BYTES + PVB_CHUNK * PVB_PS * 4;
+static constexpr int PVB_RED_BYTES = 16 * PVB_ROWS * 128 * 4;  // final exchange [16 chains][8 rows][128 dims]
+static constexpr int PVB_SMEM = PVB_STAGES * PVB_BUF_BYTES > PVB_RED_BYTES ? PVB_STAGES * PVB_BUF_BYTES : PVB_RED_BYTES;
+template <int GQA>
+__global__ void __launch_bounds__(PVB_THREADS, 2) k_attn_pv_batch(const AttnArgs a, int nz) {
+    constexpr int HD = 128, TQ = PVB_ROWS / GQA;
+    extern __shared__ __align__(16) uint8_t pvb_dyn[];
+    const int g = blockIdx.x, z0 = blockIdx.y * TQ, tid = threadIdx.x, c = tid >> 4, dg = tid & 15;     // dims 8 dg .. 8 dg + 7
+    const int ntok = min(TQ, nz - z0);
+    const int n_kv_last = a.n_kv_override + z0 + ntok - 1;     // cells attended by the CTA's last token
+    const int n_max = (n_kv_last + 31) / 32 * 32, n_chunks = (n_max + PVB_CHUNK - 1) / PVB_CHUNK;
+    // p: threads 0..127 = (row, four positions); beyond a row's padded length p = 0 and fma(v, 0, acc) == acc
+    const int pr = tid & 7, pq = (tid >> 3) & 15;
+    const int ptok = pr / GQA, ph = pr - ptok * GQA;
+    const int p_end = ptok < ntok ? (a.n_kv_override + z0 + ptok + 31) / 32 * 32 : 0;
+    const float * prow = a.S + (size_t) (z0 + (ptok < ntok ? ptok : 0)) * a.zs + (size_t) (g * GQA + ph) * a.s_stride;
+    float4 sp = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto load_v = [&](int ck) {                                 // V rows: 4 x 16 bytes a thread; rows beyond the last cell are zero
+        if (ck < n_chunks) {
+            uint8_t * base = pvb_dyn + (ck % PVB_STAGES) * PVB_BUF_BYTES;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int r = (tid >> 4) + 16 * i, t = ck * PVB_CHUNK + r;
+                uint8_t * dst = base + r * (HD * 2) + dg * 16;
+                if (t < n_kv_last) cp_async16(dst, a.v_cache + (size_t) t * a.kv_dim + g * HD + 8 * dg);
+                else *reinterpret_cast<uint4 *>(dst) = make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+        cp_async_commit();
+    };
+    auto load_p = [&](int ck) {
+        const int t = ck * PVB_CHUNK + 4 * pq;
+        sp = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (tid < 128 && ck < n_chunks && t < p_end) sp = *reinterpret_cast<const float4 *>(prow + t);
+    };
+    auto stash_p = [&](int ck) {
+        if (tid < 128 && ck < n_chunks) {
+            float * pp = reinterpret_cast<float *>(pvb_dyn + (ck % PVB_STAGES) * PVB_BUF_BYTES + PVB_V_BYTES) + (4 * pq) * PVB_PS + pr;
+            pp[0] = sp.x; pp[PVB_PS] = sp.y; pp[2 * PVB_PS] = sp.z; pp[3 * PVB_PS] = sp.w;
+        }
+    };
+    uint64_t acc[PVB_ROWS][4];                                  // [row][dim pair]
+#pragma unroll
+    for (int r = 0; r < PVB_ROWS; r++) {
+#pragma unroll
+        for (int d = 0; d < 4; d++) acc[r][d] = 0ull;
+    }
+    load_p(0);
+    load_v(0); load_v(1);
+    stash_p(0);
+    load_p(1);
+#pragma unroll 1
+    for (int ck = 0; ck < n_chunks; ck++) {
+        cp_async_wait<PVB_STAGES - 2>();
+        __syncthreads();                                        // chunk ck is complete, the buffer of ck - 1 is free
+        load_v(ck + 2);
+        stash_p(ck + 1);
+        load_p(ck + 2);
+        const uint8_t * base = pvb_dyn + (ck % PVB_STAGES) * PVB_BUF_BYTES;
+#pragma unroll
+        for (int s = 0; s < PVB_CHUNK / 16; s++) {
+            const int tt = 16 * s + c;
+            const uint4 vw = *reinterpret_cast<const uint4 *>(base + tt * (HD * 2) + dg * 16);
+            const float4 * pp = reinterpret_cast<const float4 *>(base + PVB_V_BYTES + tt * (PVB_PS * 4));
+            const float4 p0 = pp[0], p1 = pp[1];
+            const uint32_t w[4] = {vw.x, vw.y, vw.z, vw.w};
+            uint64_t v[4];
+#pragma unroll
+            for (int d = 0; d < 4; d++) { const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[d])); v[d] = pair_of(f.x, f.y); }
+            const float p[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+            for (int r = 0; r < PVB_ROWS; r++) {
+                const uint64_t p2 = pair_of(p[r], p[r]);
+#pragma unroll
+                for (int d = 0; d < 4; d++) acc[r][d] = fma2(v[d], p2, acc[r][d]);
+            }
+        }
+    }
+    cp_async_wait<0>();
     __syncthreads();
-    for (int i = tid; i < PVB_ROWS * PVB_DIMS; i += 256) {
-        const int r = i / PVB_DIMS, dd = i % PVB_DIMS, tok = r / GQA, h = r - tok * GQA;
-        if (tok >= ntok) continue;
-        float t3[8], t6[4];                                   // _mm512_reduce_add_ps over the 16 chains
+    float * red = reinterpret_cast<float *>(pvb_dyn);
 #pragma unroll
-        for (int j = 0; j < 8; j++) t3[j] = __fadd_rn(red[r][8 + j][dd], red[r][j][dd]);
+    for (int r = 0; r < PVB_ROWS; r++) {
+        const float2 x0 = unpair(acc[r][0]), x1 = unpair(acc[r][1]), x2 = unpair(acc[r][2]), x3 = unpair(acc[r][3]);
+        float4 * dst = reinterpret_cast<float4 *>(red + (size_t) (c * PVB_ROWS + r) * HD + 8 * dg);
+        dst[0] = make_float4(x0.x, x0.y, x1.x, x1.y); dst[1] = make_float4(x2.x, x2.y, x3.x, x3.y);
+    }
+    __syncthreads();
+    for (int i = tid; i < PVB_ROWS * HD; i += PVB_THREADS) {
+        const int r = i / HD, d = i % HD, tok = r / GQA, h = r - tok * GQA;
+        if (tok < ntok) {
+            float t3[8], t6[4];                                   // _mm512_reduce_add_ps over the 16 chains
 #pragma unroll
-        for (int j = 0; j < 4; j++) t6[j] = __fadd_rn(t3[4 + j], t3[j]);
-        a.out[(size_t) (z0 + tok) * a.zq + (size_t) (g * GQA + h) * HD + slice * PVB_DIMS + dd] =
-            __fadd_rn(__fadd_rn(t6[0], t6[2]), __fadd_rn(t6[1], t6[3]));
+            for (int j = 0; j < 8; j++) t3[j] = __fadd_rn(red[(size_t) ((8 + j) * PVB_ROWS + r) * HD + d], red[(size_t) (j * PVB_ROWS + r) * HD + d]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) t6[j] = __fadd_rn(t3[4 + j], t3[j]);
+            a.out[(size_t) (z0 + tok) * a.zq + (size_t) (g * GQA + h) * HD + d] = __fadd_rn(__fadd_rn(t6[0], t6[2]), __fadd_rn(t6[1], t6[3]));
+        }
     }
 }
 

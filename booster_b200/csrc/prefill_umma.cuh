@@ -109,10 +109,6 @@ __device__ __forceinline__ void fma2_ld(uint64_t & acc, uint64_t d, uint32_t lo,
     asm volatile("{\n\t.reg .b64 t;\n\tmov.b64 t, {%2, %3};\n\tfma.rn.f32x2 %0, %1, t, %0;\n\t}" : "+l"(acc) : "l"(d), "r"(lo), "r"(hi));
 }
 __device__ __forceinline__ float mul_ld(float d, uint32_t v) { float r; asm volatile("mul.rn.f32 %0, %1, %2;" : "=f"(r) : "f"(d), "f"(__uint_as_float(v))); return r; }
-// packed fp32 pairs: each half is the IEEE operation of the scalar instruction
-__device__ __forceinline__ uint64_t pair_of(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
-__device__ __forceinline__ float2 unpair(uint64_t p) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p)); return r; }
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 // mbarrier wait with an iteration limit: past it *failed is raised (every other wait of the CTA then gives up too), *err tells the host, and
 // the kernel runs to its end without storing
 __device__ __forceinline__ bool um_try(uint32_t bar, uint32_t parity) {
