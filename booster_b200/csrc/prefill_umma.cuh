@@ -28,8 +28,8 @@
 //   warps 13,14 issue the MMAs of half 0 / 1 once it is expanded and the consumers have drained its accumulators (dfree). Two issuers: one
 //               thread issues an MMA in 44 clocks whatever its N, two keep the pipe at 23 each (N = 32).
 // Expansion, tensor cores and chains of neighbouring super-blocks (and tiles) overlap; every buffer is a half super-block.
-// Measured (B200, Q4_K, 28672 rows, k = 4096, 512 tokens): 1211 us with mma.sync (k_mma_batch), 605 us here; 8 layers of an 8B Q4_K_M model, 512
-// tokens: 20.8 -> 12.2 ms, 77 tokens: 5.9 -> 3.9 ms.
+// Measured (B200, Q4_K, 28672 rows, k = 4096, 512 tokens): 1211 us with mma.sync (k_mma_batch), 492 us here (Q5_K 645, Q6_K 690, where the expansion is
+// the longer side); issue slots 60 % busy, fp32 pipe 44 %, logic 35 %.
 // Tensor memory (all 512 columns, so its base is 0): D main [0, 256) = slice m at 32 m | Q4_K, Q5_K: D mins [256, 384), A [384, 512) = slice m
 //   at 16 m | Q6_K: A of slices 0-3 [384, 512), of slices 4-7 [256, 384), 16 columns per part.
 #pragma once
@@ -103,12 +103,10 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// acc += d * (lo, hi), packed, on registers that a tcgen05.ld has filled: volatile, so that it stays behind the wait, and with the pair formed
-// inside, so that nothing copies the registers before it
-__device__ __forceinline__ void fma2_ld(uint64_t & acc, uint64_t d, uint32_t lo, uint32_t hi) {
-    asm volatile("{\n\t.reg .b64 t;\n\tmov.b64 t, {%2, %3};\n\tfma.rn.f32x2 %0, %1, t, %0;\n\t}" : "+l"(acc) : "l"(d), "r"(lo), "r"(hi));
+// (behind the wait: nothing that uses the registers is moved before it)
+__device__ __forceinline__ void tmem_ld8_ready(uint32_t (&r)[8]) {
+    asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
 }
-__device__ __forceinline__ float mul_ld(float d, uint32_t v) { float r; asm volatile("mul.rn.f32 %0, %1, %2;" : "=f"(r) : "f"(d), "f"(__uint_as_float(v))); return r; }
 // mbarrier wait with an iteration limit: past it *failed is raised (every other wait of the CTA then gives up too), *err tells the host, and
 // the kernel runs to its end without storing
 __device__ __forceinline__ bool um_try(uint32_t bar, uint32_t parity) {
@@ -507,17 +505,17 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch(const __grid_const
             auto run = [&](auto tag) {
                 constexpr int TYPE = decltype(tag)::value;
                 constexpr int NM = TYPE == T_Q4_K ? 4 : TYPE == T_Q5_K ? 1 : 0;
-                uint64_t acc[8 + NM][8];                         // [chain][token pair]
+                float2 acc[8 + NM][8];                           // [chain][token pair]
 #pragma unroll
                 for (int c = 0; c < 8 + NM; c++) {
 #pragma unroll
-                    for (int i = 0; i < 8; i++) acc[c][i] = 0ull;
+                    for (int i = 0; i < 8; i++) acc[c][i] = make_float2(0.f, 0.f);
                 }
 #pragma unroll 1
                 for (int step = 0; step < n_steps; step++, it++) {
                     const uint8_t * stage = stages + st * a.mb_stage_bytes;
                     um_wait(b_full + 8 * st, fpar, failed, a.err);             // (complete long since: the MMAs below read the same stage)
-                    const ulonglong2 * yd = reinterpret_cast<const ulonglong2 *>(stage + 4 * a.mb_raw_stride + UM_OFF_YD) + 4 * th;
+                    const float4 * yd = reinterpret_cast<const float4 *>(stage + 4 * a.mb_raw_stride + UM_OFF_YD) + 4 * th;
                     float dw, dm = 0.f;
                     if (TYPE == T_Q6_K) dw = __half2float(*reinterpret_cast<const __half *>(stage + q * a.mb_raw_stride + 6656 + lane * 2));
                     else {
@@ -536,18 +534,20 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch(const __grid_const
                             return tl + 8 * o + (c < 4 ? 32 * (4 * h + c) : UM_COL_DM + (TYPE == T_Q4_K ? 64 * h + 32 * (c - 4) : 0));
                         };
                         tmem_ld8(col(0), v[0]);
-                        uint64_t d[4];
+                        float2 d[4];
 #pragma unroll
                         for (int i = 0; i < 2 * nc; i++) {
                             const int o = i / nc, c = i % nc;
                             // d = y[i].d * fp16(x[i].d) (ggml-quants.c:6922), acc[m] = fma(d, (float) isum[m], acc[m]) (:6974);
                             // dmin = -y[i].d * fp16(x[i].dmin), acc_m lane l = fma(dmin, (float) (m[2l] bsum[2l] + m[2l+1] bsum[2l+1]), .) (:6931-6934)
                             if (c == 0 || c == 4) {
-                                const uint64_t w2 = c == 0 ? pair_of(dw, dw) : pair_of(dm, dm);
-                                const ulonglong2 y0 = yd[2 * o], y1 = yd[2 * o + 1];
-                                d[0] = mul2(y0.x, w2); d[1] = mul2(y0.y, w2); d[2] = mul2(y1.x, w2); d[3] = mul2(y1.y, w2);
+                                const float2 w = c == 0 ? make_float2(dw, dw) : make_float2(dm, dm);
+                                const float4 y0 = yd[2 * o], y1 = yd[2 * o + 1];
+                                d[0] = __fmul2_rn(make_float2(y0.x, y0.y), w); d[1] = __fmul2_rn(make_float2(y0.z, y0.w), w);
+                                d[2] = __fmul2_rn(make_float2(y1.x, y1.y), w); d[3] = __fmul2_rn(make_float2(y1.z, y1.w), w);
                             }
                             tmem_ld_wait();
+                            tmem_ld8_ready(v[i & 1]);
                             if (i + 1 < 2 * nc) tmem_ld8(col(i + 1), v[(i + 1) & 1]);
                             else {                               // everything of this half is in registers
                                 tc_fence_before();
@@ -556,12 +556,11 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch(const __grid_const
                             }
 #pragma unroll
                             for (int k = 0; k < 4; k++) {
-                                uint64_t & x = acc[c < 4 ? 4 * h + c : TYPE == T_Q4_K ? 8 + 2 * h + (c - 4) : 8 + NM - 1][4 * o + k];
-                                if (TYPE == T_Q5_K && c == 4) {  // summs += dmin * (float) sum_g m[g] bsum[g] (:7516): two roundings, kept apart in scalars (a
-                                                                 // packed multiply and add are contracted)
-                                    const float2 dd = unpair(d[k]), s2 = unpair(x);
-                                    x = pair_of(__fadd_rn(s2.x, mul_ld(dd.x, v[i & 1][2 * k])), __fadd_rn(s2.y, mul_ld(dd.y, v[i & 1][2 * k + 1])));
-                                } else fma2_ld(x, d[k], v[i & 1][2 * k], v[i & 1][2 * k + 1]);
+                                float2 & x = acc[c < 4 ? 4 * h + c : TYPE == T_Q4_K ? 8 + 2 * h + (c - 4) : 8 + NM - 1][4 * o + k];
+                                const float2 f = make_float2(__uint_as_float(v[i & 1][2 * k]), __uint_as_float(v[i & 1][2 * k + 1]));
+                                if (TYPE == T_Q5_K && c == 4) {  // summs += dmin * (float) sum_g m[g] bsum[g] (:7516): two roundings
+                                    x = make_float2(__fadd_rn(x.x, __fmul_rn(d[k].x, f.x)), __fadd_rn(x.y, __fmul_rn(d[k].y, f.y)));
+                                } else x = __ffma2_rn(d[k], f, x);
                             }
                         }
                     }
@@ -573,7 +572,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch(const __grid_const
                 for (int i = 0; i < 8; i++) {
                     float c0[12], c1[12];
 #pragma unroll
-                    for (int c = 0; c < 8 + NM; c++) { const float2 f = unpair(acc[c][i]); c0[c] = f.x; c1[c] = f.y; }
+                    for (int c = 0; c < 8 + NM; c++) { c0[c] = acc[c][i].x; c1[c] = acc[c][i].y; }
                     out[(2 * i) * UM_OUT_STRIDE + lane] = finish_row<TYPE>(c0);
                     out[(2 * i + 1) * UM_OUT_STRIDE + lane] = finish_row<TYPE>(c1);
                 }
