@@ -607,7 +607,7 @@ struct b200_ctx {
         float * X = nullptr, * Q = nullptr, * ATT = nullptr, * FFH = nullptr, * S = nullptr;
         uint8_t * rec = nullptr;
         int32_t * tokens = nullptr;
-        int * err = nullptr;     // pinned: raised by a kernel whose bounded wait ran out (pb_check)
+        int * err = nullptr;     // pinned, beside h_tok: raised by a kernel whose bounded wait ran out (pb_check)
     } pb;
     // persistent per-token kernel (token_kernel.cuh): phase list in device memory, grid-barrier counter, transposed scores
     Phase * d_plan = nullptr;
@@ -1289,7 +1289,9 @@ extern "C" b200_ctx * b200_ctx_new(b200_model * m, int n_ctx) {
         CU(cudaMemsetAsync(c->d_state, 0, sizeof(DecodeState), c->st));
         CU(cudaMallocHost(&c->h_state, sizeof(DecodeState)));
         CU(cudaMallocHost(&c->h_logits, (size_t) m->n_vocab * 4));
-        CU(cudaMallocHost(&c->h_tok, sizeof(int32_t)));
+        CU(cudaMallocHost(&c->h_tok, 2 * sizeof(int32_t)));
+        c->pb.err = c->h_tok + 1;
+        *c->pb.err = 0;
         c->out_tokens_cap = c->n_ctx + 8;
         CU(cudaMalloc(&c->d_out_tokens, (size_t) c->out_tokens_cap * 4));
         CU(cudaStreamSynchronize(c->st));
@@ -1322,7 +1324,6 @@ extern "C" void b200_ctx_free(b200_ctx * c) {
     cudaFree(c->x); cudaFree(c->q); cudaFree(c->att); cudaFree(c->ffh); cudaFree(c->warm_x); cudaFree(c->logits);
     cudaFree(c->d_cell_pos);
     cudaFree(c->pb.X); cudaFree(c->pb.Q); cudaFree(c->pb.ATT); cudaFree(c->pb.FFH); cudaFree(c->pb.S); cudaFree(c->pb.rec); cudaFree(c->pb.tokens);
-    cudaFreeHost(c->pb.err);
     cudaFree(c->d_trace); cudaFree(c->d_plan); cudaFree(c->d_bar); cudaFree(c->S_T); cudaFree(c->d_ttrace);
     cudaFree(c->S); cudaFree(c->tickets); cudaFree(c->amax_key); cudaFree(c->rope); cudaFree(c->d_state); cudaFree(c->d_out_tokens);
     cudaFreeHost(c->h_state); cudaFreeHost(c->h_logits); cudaFreeHost(c->h_tok);
@@ -1646,17 +1647,12 @@ static bool prefill_batch_usable(const b200_ctx * c, int n) {
     if (m.n_ff % 256 || m.n_embd % 256 || std::max(m.n_ff, m.n_embd) / 256 > 4 * 16 * 4) return false;
     return true;
 }
-static void pb_alloc_err(b200_ctx * c) {
-    CU(cudaHostAlloc(&c->pb.err, sizeof(int), cudaHostAllocMapped));
-    *c->pb.err = 0;
-}
 // after a synchronisation: a batch whose kernel gave up waiting left no result
 static void pb_check(b200_ctx * c) {
     if (c->pb.err && *(volatile int *) c->pb.err) { *c->pb.err = 0; throw std::runtime_error("a prompt kernel's bounded wait ran out"); }
 }
 static void prefill_alloc(b200_ctx * c) {
     if (c->pb.cap) return;
-    if (!c->pb.err) pb_alloc_err(c);
     const b200_model & m = *c->m;
     const int T = PB_MAX_T, QD = m.n_head * m.head_dim;
     const size_t kmax = (size_t) std::max(std::max(m.n_ff, m.n_embd), QD);
@@ -2769,8 +2765,9 @@ extern "C" int b200_op_mul_mat(int type, const void * w, int64_t n_rows, int64_t
         int dev = 0; CU(cudaGetDevice(&dev));
         tmp.device = dev;
         tmp.pb.rec = drec.as<uint8_t>();
-        pb_alloc_err(&tmp);
+        CU(cudaMallocHost(&tmp.pb.err, sizeof(int)));
         std::unique_ptr<int, cudaError_t (*)(void *)> err_owner(tmp.pb.err, cudaFreeHost);
+        *tmp.pb.err = 0;
         MatvecArgs a{};
         a.seg[0] = d.m; a.n_seg = 1; a.n_units = d.m.n_units; a.k = (int) k; a.act_q8_0 = type == T_Q8_0;
         const int was = type == T_Q6_K;

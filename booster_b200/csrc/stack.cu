@@ -1339,9 +1339,8 @@ void norm(StackCtx * c, const float * X, int ldx, const int32_t * rows, const fl
 
 template <int DMAX>
 void launch_delta_scan(StackCtx * c, const LayerSpec & L, int T, int C, float * S) {
-    const int threads = std::min(128, (L.V + 31) / 32 * 32);
-    const dim3 grid((unsigned) L.H, (unsigned) ((L.V + threads - 1) / threads));
-    k_delta_scan<DMAX><<<grid, threads, 0, c->st>>>(c->CV, C, c->BG, T, L.H, L.KH, L.D, L.V, S, c->O);
+    const dim3 grid((unsigned) L.H, (unsigned) ((L.V + DSCAN_COLS - 1) / DSCAN_COLS));
+    k_delta_scan<DMAX><<<grid, 128, 0, c->st>>>(c->CV, C, c->BG, T, L.H, L.KH, L.D, L.V, S, c->O);
 }
 
 // mixers: c->in [T][E] -> c->out [T][E]; R names the run's state
