@@ -1259,6 +1259,26 @@ constexpr int GEMV_FEW_ROWS = 512;
 struct UmmaScratch { __nv_bfloat16 * xb = nullptr; size_t elems = 0; int * err = nullptr; float * part = nullptr; int sm_count = 148; };
 size_t umma_part_floats(int sm_count) { return (size_t) sm_count * UM_BM * UM_BN; }      // one K part of an output tile per SM
 
+// tensor map of a bf16 matrix batch [nz][rows][K] (strides in elements): boxes of 64 columns, one 128-byte swizzled row each, by box_rows
+CUtensorMap map_bf16(const void * base, int K, int rows, int nz, long long ld, long long sz, int box_rows) {
+    static const auto encode = [] {
+        void * fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) fn = nullptr;
+        return reinterpret_cast<CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
+                                             CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill)>(fn);
+    }();
+    if (!encode) throw std::runtime_error("the driver has no cuTensorMapEncodeTiled");
+    CUtensorMap m;
+    const cuuint64_t dims[3] = {(cuuint64_t) K, (cuuint64_t) rows, (cuuint64_t) nz};
+    const cuuint64_t strides[2] = {(cuuint64_t) ld * 2, (cuuint64_t) (nz > 1 ? sz : (long long) rows * ld) * 2};
+    const cuuint32_t box[3] = {(cuuint32_t) UM_BK, (cuuint32_t) box_rows, 1}, one[3] = {1, 1, 1};
+    const CUresult r = encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(base), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed: " + std::to_string((int) r));
+    return m;
+}
+
 // what a product may ask for beyond its operands: the gated unit's kind and constants (y = g sigmoid(alpha g) (u + shift), g and u clamped
 // at +-limit, or gelu(g) u), rows sorted into segments per batch entry (tile kernels), an indexed batch (mat-vec)
 struct LinOpt {
@@ -1293,19 +1313,20 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
             else if (dtype == STACK_F32) k_gemv<float, 1><<<grid, 256, 0, st>>>(a); else k_gemv<__nv_bfloat16, 1><<<grid, 256, 0, st>>>(a);
         }
     } else if (dtype == STACK_BF16 && a.vec && us && us->xb && umma_enabled() && T >= 64 && N >= 128 && K >= 64 && (size_t) xbatch * T * K <= us->elems) {
-        // tensor memory path: activations to bfloat16 once, then tcgen05.mma over cp.async-fed stages
+        // tensor memory path: activations to bfloat16 once, then tcgen05.mma over TMA-fed stages (a.vec: rows and batch strides are multiples of 16 bytes)
         static const bool attr = [] { return cudaFuncSetAttribute(k_gemm_bf16_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM) == cudaSuccess; }();
         if (!attr) throw std::runtime_error("cannot reserve shared memory for k_gemm_bf16_umma");
         k_to_bf16<<<dim3((unsigned) std::min((K + 255) / 256, 64), (unsigned) T, (unsigned) xbatch), 256, 0, st>>>(X, ldx, T, K, sX, us->xb, (long long) T * K);
         const dim3 grid((unsigned) ((N + UM_BN - 1) / UM_BN), (unsigned) ((T + UM_BM - 1) / UM_BM), (unsigned) batch);
+        const CUtensorMap mx = map_bf16(us->xb, K, T, xbatch, K, (long long) T * K, UM_BM), mw = map_bf16(W, K, N, batch, K, sW, UM_BN);
         const int tiles = (int) (grid.x * grid.y), nk = (K + UM_BK - 1) / UM_BK;
         const int ksplit = batch == 1 && !a.glu && !a.seg && us->part && split_k_enabled() ? std::min(us->sm_count / tiles, nk / 4) : 1;
         if (ksplit > 1) {
-            k_gemm_bf16_umma<<<dim3(grid.x, grid.y, (unsigned) ksplit), 256, UM_SMEM, st>>>(a, us->xb, (long long) T * K, us->err, ksplit, us->part);
+            k_gemm_bf16_umma<<<dim3(grid.x, grid.y, (unsigned) ksplit), 256, UM_SMEM, st>>>(mx, mw, a, us->err, ksplit, us->part);
             k_split_sum<<<dim3((unsigned) ((N + 255) / 256), (unsigned) T), 256, 0, st>>>(us->part, ksplit, T, N, bias, Y, ldy);
             if (launches) (*launches)++;
         }
-        else k_gemm_bf16_umma<<<grid, 256, UM_SMEM, st>>>(a, us->xb, (long long) T * K, us->err);
+        else k_gemm_bf16_umma<<<grid, 256, UM_SMEM, st>>>(mx, mw, a, us->err);
         if (launches) (*launches)++;
     } else if (dtype == STACK_BF16 && a.vec && mma_enabled()) {
         const dim3 grid((unsigned) ((N + MM_BN - 1) / MM_BN), (unsigned) ((T + MM_BM - 1) / MM_BM), (unsigned) batch);

@@ -11,6 +11,7 @@
 // model's storage type WT (bfloat16 or float32) and accumulate in float32; the tensor-core product (k_gemm_bf16_mma)
 // rounds its activation operand to bfloat16.
 #pragma once
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -582,11 +583,13 @@ __global__ void __launch_bounds__(256) k_gemm_bf16_mma(const LinArgs a) {
 
 // ---- prompt portions with bfloat16 weights on the 5th-generation tensor cores -------------------------------------------------
 // tcgen05.mma (kind::f16, bf16 x bf16 -> f32) with the accumulator in tensor memory: D[128 tokens][256 rows of W] per CTA.
-//   operands   both K-major in the canonical no-swizzle core-matrix order [8-row group][k-chunk][8 rows][16 B]: a 16-byte
-//              cp.async per (row, k-chunk) drops global rows straight into that order (zero-fill past T, N or K), four stages of
-//              K = 64 deep; the activations were rounded to bfloat16 by k_to_bf16 beforehand
-//   issue      one thread: four K = 16 MMAs per stage, tcgen05.commit -> the stage's mbarrier (frees the stage for the refill)
+//   operands   both K-major, tiles of K = 64 in the 128-byte swizzle: one TMA copy per operand and stage, four stages (zero-fill past T, N and K); the
+//              activations were rounded to bfloat16 by k_to_bf16 beforehand
+//   warp 0     one lane issues the copies (full[stage] by bytes), warp 1 one lane the MMAs, four K = 16 steps per stage; tcgen05.commit frees
+//              the stage (empty) and, after the last, the accumulator (done)
 //   epilogue   warp w owns TMEM lanes 32 (w & 3) .. + 31 (= tokens) and column half w >> 2: tcgen05.ld, bias / gated unit, stores
+// What bounds it: a tile moves 48 KB of L2 per 4.2 MFLOP. With 12 cp.async per thread and stage and a block-wide barrier per stage the copies were the
+// bound; 512 x 16384 x 2048 with the rounding of X: 144 us then (239 TFLOP/s), 54 us now (639), 4096 x 14336: 260 and 95 us.
 // Products with too few output tiles to fill the SMs are cut along K (ksplit > 1: blockIdx.z is the part): every part leaves its sums
 // in part [ksplit][T][N] and k_split_sum adds them in order, with the bias.
 // Every wait on an mbarrier is bounded: on a timeout the CTA raises *err, skips what is left and still frees its tensor memory.
@@ -601,6 +604,10 @@ constexpr int UM_SMEM = UM_STAGES * UM_STAGE_BYTES + 1024;                 // + 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void * src, uint32_t bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap * map, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
 __device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity, volatile int * failed, int * err) {
     if (*failed) return false;
     for (uint32_t spins = 0; spins < (1u << 22); spins++) {
@@ -613,24 +620,28 @@ __device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity,
     atomicExch(err, 1);
     return false;
 }
-__global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const LinArgs a, const __nv_bfloat16 * __restrict__ Xb, long long sXb, int * err, int ksplit = 1, float * __restrict__ part = nullptr) {
+// maps: X as bf16 [xbatch][T][K] (box 64 x 128), W [batch][N][K] (box 64 x 256)
+__global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const LinArgs a, int * err, int ksplit = 1, float * __restrict__ part = nullptr) {
     extern __shared__ uint8_t um_raw[];
-    __shared__ __align__(8) uint64_t done[UM_STAGES];
+    __shared__ __align__(8) uint64_t full[UM_STAGES], empty[UM_STAGES], done;
     __shared__ uint32_t tmem_base_s;
     __shared__ int failed_s;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t smem0 = (smem_addr(um_raw) + 1023u) & ~1023u;
     const int m0 = blockIdx.y * UM_BM, n0 = blockIdx.x * UM_BN;
     const int r0 = a.seg ? a.seg[blockIdx.z] : 0, T = a.seg ? a.seg[blockIdx.z + 1] - r0 : a.T;
     if (m0 >= T) return;                      // the whole block, before anything is allocated
     const int bz = ksplit > 1 ? 0 : blockIdx.z;
-    const __nv_bfloat16 * X = a.seg ? Xb + (size_t) r0 * a.K : Xb + (size_t) bz * sXb;
-    const __nv_bfloat16 * W = reinterpret_cast<const __nv_bfloat16 *>(a.W) + (size_t) bz * a.sW;
     volatile int * failed = &failed_s;
     if (tid == 0) {
         failed_s = 0;
-        for (int s = 0; s < UM_STAGES; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&done[s])) : "memory");
+        for (int s = 0; s < UM_STAGES; s++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&full[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&empty[s])) : "memory");
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&done)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_addr(&tmem_base_s)), "r"(256u) : "memory");
@@ -642,63 +653,48 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const LinArgs a, cons
     const uint32_t tmem = tmem_base_s;
     const int nk_all = (a.K + UM_BK - 1) / UM_BK, kbeg = ksplit > 1 ? (int) ((long long) nk_all * blockIdx.z / ksplit) : 0;
     const int nk = (ksplit > 1 ? (int) ((long long) nk_all * (blockIdx.z + 1) / ksplit) : nk_all) - kbeg;       // at least one: ksplit <= nk_all
-    // one stage: 128 x 8 chunks of A (4 per thread) and 256 x 8 chunks of B (8 per thread); a warp's 32 chunks are 512 contiguous bytes
-    const auto issue_copies = [&](int kt, int slot) {
-        const uint32_t sa = smem0 + (uint32_t) slot * UM_STAGE_BYTES, sb = sa + UM_A_BYTES;
-        const int k0 = (kbeg + kt) * UM_BK;
-#pragma unroll
-        for (int i = 0; i < 12; i++) {
-            const int idx = tid + 256 * (i < 4 ? i : i - 4);
-            const int r_in = idx & 7, kc = (idx >> 3) & 7, rg = idx >> 6;
-            const int k = k0 + kc * 8;
-            const uint32_t off = (uint32_t) rg * 1024u + (uint32_t) kc * 128u + (uint32_t) r_in * 16u;
-            if (i < 4) {
-                const int m = m0 + rg * 8 + r_in;
-                const bool ok = m < T && k < a.K;
-                cp_async16(sa + off, ok ? (const void *) (X + (size_t) m * a.K + k) : (const void *) X, ok ? 16u : 0u);
-            } else {
-                const int n = n0 + rg * 8 + r_in;
-                const bool ok = n < a.N && k < a.K;
-                cp_async16(sb + off, ok ? (const void *) (W + (size_t) n * a.K + k) : (const void *) W, ok ? 16u : 0u);
+    if (warp == 0) {
+        const int zx = a.seg ? 0 : bz;
+        if (lane == 0) {
+            for (int kt = 0; kt < nk; kt++) {
+                const int slot = kt % UM_STAGES;
+                if (kt >= UM_STAGES) mbar_wait_limited(smem_addr(&empty[slot]), (uint32_t) ((kt / UM_STAGES - 1) & 1), failed, err);
+                if (*failed) break;
+                const uint32_t sa = smem0 + (uint32_t) slot * UM_STAGE_BYTES, bar = smem_addr(&full[slot]);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"((uint32_t) UM_STAGE_BYTES) : "memory");
+                tma_load_3d(sa, &map_x, (kbeg + kt) * UM_BK, r0 + m0, zx, bar);
+                tma_load_3d(sa + UM_A_BYTES, &map_w, (kbeg + kt) * UM_BK, n0, bz, bar);
             }
+            if (*failed) for (int i = 0; i < 1000; i++) __nanosleep(1000);      // copies under way land before the block ends
         }
-    };
-    for (int s = 0; s < UM_STAGES - 1; s++) {
-        if (s < nk) issue_copies(s, s);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    // instruction descriptor: D f32, A and B bf16, both K-major, N = 256, M = 128
-    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (UM_BN >> 3) << 17) | ((uint32_t) (UM_BM >> 4) << 24);
-    for (int kt = 0; kt < nk; kt++) {
-        const int slot = kt % UM_STAGES;
-        asm volatile("cp.async.wait_group %0;" :: "n"(UM_STAGES - 2) : "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");          // the copies' writes -> visible to the tensor core's reads
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (tid == 0 && !*failed) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t sa = smem0 + (uint32_t) slot * UM_STAGE_BYTES, sb = sa + UM_A_BYTES;
+        __syncwarp();
+    } else if (warp == 1) {
+        // instruction descriptor: D f32, A and B bf16, both K-major, N = 256, M = 128
+        constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (UM_BN >> 3) << 17) | ((uint32_t) (UM_BM >> 4) << 24);
+        // K-major, 128-byte swizzle: start >> 4 | 8-row group stride 1024 B >> 4 << 32 | version 1 | layout 2; a K = 16 step is 32 bytes along the row
+        constexpr uint64_t DESC = ((uint64_t) 1 << 16) | ((uint64_t) (1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
+        if (lane == 0) {
+            for (int kt = 0; kt < nk; kt++) {
+                const int slot = kt % UM_STAGES;
+                mbar_wait_limited(smem_addr(&full[slot]), (uint32_t) ((kt / UM_STAGES) & 1), failed, err);
+                if (*failed) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t sa = smem0 + (uint32_t) slot * UM_STAGE_BYTES, sb = sa + UM_A_BYTES;
 #pragma unroll
-            for (int ks = 0; ks < UM_BK / 16; ks++) {
-                // K-major, no swizzle: start >> 4 | (k-chunk stride 128 B) >> 4 << 16 | (8-row group stride 1024 B) >> 4 << 32 | version 1
-                const uint64_t da = (uint64_t) (((sa + ks * 256u) >> 4) & 0x3fffu) | ((uint64_t) (128u >> 4) << 16) | ((uint64_t) (1024u >> 4) << 32) | (1ull << 46);
-                const uint64_t db = (uint64_t) (((sb + ks * 256u) >> 4) & 0x3fffu) | ((uint64_t) (128u >> 4) << 16) | ((uint64_t) (1024u >> 4) << 32) | (1ull << 46);
-                const uint32_t accumulate = (kt | ks) ? 1u : 0u;
-                asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                             :: "r"(tmem), "l"(da), "l"(db), "r"(IDESC), "r"(accumulate) : "memory");
+                for (int ks = 0; ks < UM_BK / 16; ks++) {
+                    const uint64_t da = DESC | (uint64_t) (((sa + ks * 32u) >> 4) & 0x3fffu), db = DESC | (uint64_t) (((sb + ks * 32u) >> 4) & 0x3fffu);
+                    const uint32_t accumulate = (kt | ks) ? 1u : 0u;
+                    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                                 :: "r"(tmem), "l"(da), "l"(db), "r"(IDESC), "r"(accumulate) : "memory");
+                }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_addr(&empty[slot])) : "memory");
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_addr(&done[slot])) : "memory");
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_addr(&done)) : "memory");
+            if (*failed) for (int i = 0; i < 1000; i++) __nanosleep(1000);      // MMAs under way end before tensor memory is given back
         }
-        // refill the slot of stage kt - 1 with stage kt + STAGES - 1 once its MMAs have read it
-        const int nxt = kt + UM_STAGES - 1;
-        if (nxt < nk) {
-            if (kt >= 1) mbar_wait_limited(smem_addr(&done[(kt - 1) % UM_STAGES]), (uint32_t) (((kt - 1) / UM_STAGES) & 1), failed, err);
-            if (!*failed) issue_copies(nxt, nxt % UM_STAGES);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        __syncwarp();
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    const bool ok = mbar_wait_limited(smem_addr(&done[(nk - 1) % UM_STAGES]), (uint32_t) (((nk - 1) / UM_STAGES) & 1), failed, err);
+    const bool ok = mbar_wait_limited(smem_addr(&done), 0u, failed, err) && !*failed;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok) {
         const int m = m0 + 32 * (warp & 3) + lane, cbase = (warp >> 2) * (UM_BN / 2);
