@@ -1254,6 +1254,7 @@ bool split_k_enabled() {
     return on;
 }
 constexpr int GEMV_FEW_ROWS = 512;
+constexpr int GX_MIN_K = 1024;                // shorter rows leave most of a block's lanes without an entry: k_gemv, a warp per row
 // what the tcgen05 product needs beside its operands: room for the activations rounded to bfloat16 and the error flag its
 // bounded waits raise
 struct UmmaScratch { __nv_bfloat16 * xb = nullptr; size_t elems = 0; int * err = nullptr; float * part = nullptr; int sm_count = 148; };
@@ -1301,7 +1302,18 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
     const auto al16 = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
     a.vec = K % vecw == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % vecw == 0 && al16(X) && al16(W);
     if (launches) (*launches)++;
-    if (T <= GEMV_MAX_T) {
+    const int gx_chunks = (K + GX_WARPS * 32 * vecw - 1) / (GX_WARPS * 32 * vecw);
+    if (T == 1 && a.vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && gx_chunks <= 8 && sX % 4 == 0) {
+        const dim3 grid((unsigned) ((N + GX_ROWS - 1) / GX_ROWS), 1, (unsigned) batch);
+        const auto go = [&](auto wt) {
+            using WT = decltype(wt);
+            if (gx_chunks <= 1) k_gemv_x<WT, 1><<<grid, GX_WARPS * 32, 0, st>>>(a);
+            else if (gx_chunks <= 2) k_gemv_x<WT, 2><<<grid, GX_WARPS * 32, 0, st>>>(a);
+            else if (gx_chunks <= 4) k_gemv_x<WT, 4><<<grid, GX_WARPS * 32, 0, st>>>(a);
+            else k_gemv_x<WT, 8><<<grid, GX_WARPS * 32, 0, st>>>(a);
+        };
+        if (dtype == STACK_F32) go(0.f); else go(__nv_bfloat16());
+    } else if (T <= GEMV_MAX_T) {
         if (a.glu) {
             const dim3 grid((unsigned) ((N / 2 + 7) / 8), 1, (unsigned) batch);
             if (dtype == STACK_F32) k_gemv<float, 2><<<grid, 256, 0, st>>>(a); else k_gemv<__nv_bfloat16, 2><<<grid, 256, 0, st>>>(a);
