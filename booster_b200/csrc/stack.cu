@@ -1253,6 +1253,10 @@ bool split_k_enabled() {
     static const bool on = [] { const char * e = std::getenv("BOOSTER_B200_STACK_SPLIT_K"); return !(e && e[0] == '0'); }();
     return on;
 }
+bool simt_big_enabled() {
+    static const bool on = [] { const char * e = std::getenv("BOOSTER_B200_STACK_SIMT_BIG"); return !(e && e[0] == '0'); }();
+    return on;
+}
 constexpr int GEMV_FEW_ROWS = 512;
 constexpr int GX_MIN_K = 1024;                // shorter rows leave most of a block's lanes without an entry: k_gemv, a warp per row
 // what the tcgen05 product needs beside its operands: room for the activations rounded to bfloat16 and the error flag its
@@ -1302,6 +1306,11 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
     const auto al16 = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
     a.vec = K % vecw == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % vecw == 0 && al16(X) && al16(W);
     if (launches) (*launches)++;
+    int f32_parts = 1;
+    if (dtype == STACK_F32 && T >= 64 && N >= SG_BN && a.vec && batch == 1 && !a.glu && !a.seg && us && us->part && split_k_enabled() && simt_big_enabled()) {
+        f32_parts = std::min(2 * us->sm_count / (((N + SG_BN - 1) / SG_BN) * ((T + SG_BM - 1) / SG_BM)), (K + SG_BK - 1) / SG_BK / 16);
+        while (f32_parts > 1 && (size_t) f32_parts * T * N > umma_part_floats(us->sm_count)) f32_parts--;
+    }
     const int gx_chunks = (K + GX_WARPS * 32 * vecw - 1) / (GX_WARPS * 32 * vecw);
     if (T == 1 && a.vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && gx_chunks <= 8 && sX % 4 == 0) {
         const dim3 grid((unsigned) ((N + GX_ROWS - 1) / GX_ROWS), 1, (unsigned) batch);
@@ -1339,6 +1348,10 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
             if (launches) (*launches)++;
         }
         else k_gemm_bf16_umma<<<grid, 256, UM_SMEM, st>>>(mx, mw, a, us->err);
+        if (launches) (*launches)++;
+    } else if (f32_parts > 1) {      // few tiles: two blocks per SM by cutting K, 256 k each at least (a gated unit needs its sums whole: k_gemm_simt, 193 us against 236 in 128 x 128 tiles)
+        k_gemm_simt_big<<<dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((T + SG_BM - 1) / SG_BM), (unsigned) f32_parts), 256, 0, st>>>(a, f32_parts, us->part);
+        k_split_sum<<<dim3((unsigned) ((N + 255) / 256), (unsigned) T), 256, 0, st>>>(us->part, f32_parts, T, N, bias, Y, ldy);
         if (launches) (*launches)++;
     } else if (dtype == STACK_BF16 && a.vec && mma_enabled()) {
         const dim3 grid((unsigned) ((N + MM_BN - 1) / MM_BN), (unsigned) ((T + MM_BM - 1) / MM_BM), (unsigned) batch);
@@ -1425,10 +1438,6 @@ AttnPlan plan_attention(const LayerSpec & L, int n_ctx, int T, int sm_count) {
     return p;
 }
 
-bool simt_big_enabled() {
-    static const bool on = [] { const char * e = std::getenv("BOOSTER_B200_STACK_SIMT_BIG"); return !(e && e[0] == '0'); }();
-    return on;
-}
 // float32 product on the CUDA cores with explicit operand layout (the attention's two products over cached rows)
 // A second batch level (nz2 products per first-level index, strides sX2 / sW2 / sY2) serves operands that are cut twice: tiles x heads.
 struct See { int rows = 0, pos = 0, step = 0; };      // LinArgs::see_*
@@ -2516,8 +2525,8 @@ StackCtx * stack_ctx_new(StackModel * m, int n_ctx) {
         if (m->dtype == STACK_BF16) {
             c->xb_elems = std::max(cap * (size_t) std::max({ 2 * m->E, m->maxA, m->maxOL, m->maxP, m->max_dense, m->side_dim }), moe_rows * (size_t) std::max(m->E, m->max_eff));
             SCU(cudaMalloc(&c->xb, c->xb_elems * 2));
-            SCU(cudaMalloc(&c->xpart, umma_part_floats(c->sm_count) * 4));
         }
+        SCU(cudaMalloc(&c->xpart, umma_part_floats(c->sm_count) * 4));
         SCU(cudaMalloc(&c->d_err, 4)); SCU(cudaMemsetAsync(c->d_err, 0, 4, c->st));
         SCU(cudaMallocHost(&c->h_err, 4)); *c->h_err = 0;
         c->caches.assign((size_t) m->n_caches, nullptr);

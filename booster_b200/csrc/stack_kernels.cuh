@@ -480,15 +480,17 @@ __global__ void __launch_bounds__(256) k_gemm_simt(const LinArgs a) {
 // the same float32 product for operands large enough to fill 128 x 128 tiles (the attention's products over a tile of tokens x all
 // heads): 256 threads with 8 x 8 outputs each (two 4 x 4 quarters 64 apart, so that the 16-byte shared-memory reads of a
 // half-warp stay free of bank conflicts), twice the FMAs per shared-memory read of the 64 x 64 kernel, the next K slice
-// of both operands in registers while the current one is multiplied. float32 operands with 16-byte aligned rows only (a.vec);
-// plain or accumulating stores; no bias, no gated unit, no segments.
+// of both operands in registers while the current one is multiplied. float32 operands with 16-byte aligned rows only (a.vec); no gated unit, no segments.
+// Products of float32 models whose tiles leave SMs idle run here too, cut along K like k_gemm_bf16_umma's (ksplit > 1: blockIdx.z is the part, sums to
+// part [ksplit][T][N], k_split_sum adds them): 300 tokens x 1024 x 4096 as 80 blocks of 64 x 64 took 234 us, in twelve parts 91. Packed fmas
+// (pairs of columns) were tried and gain nothing: the shared-memory reads are the bound.
 constexpr int SG_BM = 128, SG_BN = 128, SG_BK = 16;
-__global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a) {
+__global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a, int ksplit = 1, float * __restrict__ part = nullptr) {
     __shared__ __align__(16) float Xs[SG_BK][SG_BM + 4];
     __shared__ __align__(16) float Ws[SG_BK][SG_BN + 4];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int m0 = blockIdx.y * SG_BM, n0 = blockIdx.x * SG_BN;
-    const int z1 = blockIdx.z / a.nz2, z2 = blockIdx.z - z1 * a.nz2;
+    const int zb = ksplit > 1 ? 0 : blockIdx.z, z1 = zb / a.nz2, z2 = zb - z1 * a.nz2;
     const float * X = a.X + (size_t) z1 * a.sX + (size_t) z2 * a.sX2;
     const float * W = reinterpret_cast<const float *>(a.W) + (size_t) z1 * a.sW + (size_t) z2 * a.sW2;
     const int ldw = a.ldw > 0 ? a.ldw : a.K;
@@ -497,6 +499,12 @@ __global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a) {
         const int last = tile_sees(a, z1, m0, SG_BM);
         if (a.w_kn) K = min(K, (last + 4) / 4 * 4);
         else if (n0 > last) return;
+    }
+    int kbeg = 0;
+    if (ksplit > 1) {
+        const int nk = (K + SG_BK - 1) / SG_BK;
+        kbeg = (int) ((long long) nk * blockIdx.z / ksplit) * SG_BK;
+        K = min(K, (int) ((long long) nk * (blockIdx.z + 1) / ksplit) * SG_BK);
     }
     float acc[8][8];
 #pragma unroll
@@ -528,8 +536,8 @@ __global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a) {
             }
         }
     };
-    fetch(0);
-    for (int k0 = 0; k0 < K; k0 += SG_BK) {
+    fetch(kbeg);
+    for (int k0 = kbeg; k0 < K; k0 += SG_BK) {
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const float xv[4] = { xr[h].x, xr[h].y, xr[h].z, xr[h].w };
@@ -556,7 +564,9 @@ __global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a) {
         }
         __syncthreads();
     }
-    float * Y = a.Y + (size_t) z1 * a.sY + (size_t) z2 * a.sY2;
+    const int ldy = ksplit > 1 ? a.N : a.ldy;
+    const float * bias = ksplit > 1 ? nullptr : a.bias;
+    float * Y = ksplit > 1 ? part + (size_t) blockIdx.z * a.T * a.N : a.Y + (size_t) z1 * a.sY + (size_t) z2 * a.sY2;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
@@ -564,7 +574,7 @@ __global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a) {
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const int n = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
-            if (n < a.N) Y[(size_t) m * a.ldy + n] = acc[i][j] + (a.accum ? Y[(size_t) m * a.ldy + n] : 0.f);
+            if (n < a.N) Y[(size_t) m * ldy + n] = acc[i][j] + (bias ? bias[n] : 0.f) + (a.accum ? Y[(size_t) m * ldy + n] : 0.f);
         }
     }
 }
