@@ -642,12 +642,12 @@ def main():
             pm = float(np.mean(pms[1:]))
             line["prompt_batch"] = {"tokens": 512, "ms": pm, "tokens_per_s": 512e3 / pm,
                                     "kernels": ("k_quant_batch_mma + k_mma_batch_q80 (block-diagonal fp16 HMMA: exact 4-byte lane sums)" if ftype == "Q8_0" else
-                                                "k_quant_batch_mma + k_mma_batch (exact fp16 HMMA per AVX2 lane-slice)") +
+                                                "k_quant_batch_mma + k_umma_batch (exact fp16 tcgen05 products per AVX2 lane-slice, A operand in tensor memory)") +
                                                " + k_attn_scores_batch / k_attn_softmax_rows / k_attn_pv_batch",
                                     "what": "b200_decode of one 512-token batch at positions 0..511, wall clock incl. the final synchronisation"}
             try:   # tensor-pipe utilisation of the batch mat-mul kernel from the committed ncu --set full capture
                 with open(os.path.join(ROOT, "profiles", "prefill_tensor.json")) as f:
-                    line["prompt_batch"]["tensor_pipe"] = json.load(f)["k_mma_batch_q80" if ftype == "Q8_0" else "k_mma_batch"]
+                    line["prompt_batch"]["tensor_pipe"] = json.load(f)["k_mma_batch_q80" if ftype == "Q8_0" else "k_umma_batch"]
             except Exception:
                 pass
         except Exception as e:

@@ -192,6 +192,35 @@ def test_self_extend_bitwise_golden(golden_dir, model):
     c.close(); m.close()
 
 
+@pytest.mark.parametrize("kv_heads", [8, 4, 2, 1])
+def test_prompt_batch_attention_at_long_rows(tmp_path, kv_heads):
+    """the batch attention where its variants meet: score rows on both sides of 2048 (a warp per row, then a block), of 4096 and 8192 (more scores per
+    thread), one token past a tile of 16, every group size; equal to the token-by-token kernels bit for bit"""
+    conf = G.LlamaConfig(n_layer=1, n_embd=1024, n_head=8, n_head_kv=kv_heads, n_ff=512, n_vocab=256, n_ctx_train=16384)
+    path = str(tmp_path / "m.gguf")
+    G.synth_llama(path, conf, "Q4_K_M", seed=kv_heads)
+    rng = np.random.default_rng(kv_heads)
+    kv = rng.standard_normal((2, 8300, kv_heads * 128)).astype(np.float16)
+    m = engine.Model(path)
+    for past, n in ((0, 17), (2033, 17), (4080, 33), (8190, 9)):
+        toks = rng.integers(0, 256, size=n).tolist()
+        got = []
+        for batch in (True, False):
+            engine.set_prefill_batch(batch)
+            try:
+                c = engine.Context(m, 8448)
+                if past:
+                    c.kv_write(0, 0, kv[0, :past], kv[1, :past])
+                got.append((c.decode(toks, past), c.kv_read(0, past, n)))
+                c.close()
+            finally:
+                engine.set_prefill_batch(True)
+        _same(got[0][0], got[1][0], f"logits at {past}")
+        for a, b in zip(got[0][1], got[1][1]):
+            assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
+    m.close()
+
+
 @pytest.mark.parametrize("cfg,ftype,n_prompt", [("llama3-8b-2l", "Q4_K_M", 200), ("llama3-8b-2l", "Q8_0", 130), ("llama3-8b-2l", "Q5_K_M", 70),
                                                 ("llama3-70b-1l", "Q4_K_M", 65), ("tiny-gqa4", "Q4_K_M", 450)])
 def test_prompt_batch_kernels_equal_token_by_token_bitwise(model_dir, cfg, ftype, n_prompt):

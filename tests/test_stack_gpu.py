@@ -422,3 +422,30 @@ def test_products_pick_their_kernel_and_agree_with_numpy(dtype, T, N, K, glu):
         g, u = np.minimum(ref[:, 0::2], limit), np.clip(ref[:, 1::2], -limit, limit)
         ref = g * so.sigmoid(1.702 * g) * (u + 1.0)
     assert np.abs(y - ref).max() < 2e-5 * max(1.0, np.abs(ref).max()) * np.sqrt(K)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("T,N,K,glu", [
+    (1, 513, 1024, False), (1, 1001, 2056, False), (1, 2048, 4096, True), (1, 600, 8192, False), (1, 530, 16384, False), (1, 514, 1032, True), (1, 512, 1024, False),
+    (64, 128, 64, False), (65, 257, 72, False), (130, 300, 4096, False), (200, 2056, 1000, False), (129, 514, 264, True), (300, 130, 2064, False)])
+def test_products_where_their_rules_change(dtype, T, N, K, glu):
+    """one token: eight rows a block and each number of chunks per lane, rows and K that end inside a block; portions: TMA tiles that end inside T, N and K,
+    and float32 products in K parts. Bound: a sum of K float32 products in any order is off by at most (K + 8) 2^-24 sum |x w|."""
+    rng = np.random.default_rng(T * 7 + N + K)
+    x = rng.standard_normal((T, K)).astype(np.float32)
+    w = so.round_bf16((rng.standard_normal((N, K)) / np.sqrt(K)).astype(np.float32))
+    b = rng.standard_normal(N).astype(np.float32)
+    y = np.zeros((T, N // 2 if glu else N), np.float32)
+    f32p = C.POINTER(C.c_float)
+    L = _lib.lib()
+    rc = L.b200_stack_linear(0, 0 if dtype == "bfloat16" else 1, T, N, K, x.ctypes.data_as(f32p), w.ctypes.data_as(f32p), b.ctypes.data_as(f32p), int(glu), 7.0, y.ctypes.data_as(f32p))
+    assert rc == 0, _lib.last_error()
+    xe = (so.round_bf16(x) if dtype == "bfloat16" and T > 4 else x).astype(np.float64)
+    we = w.astype(np.float64)
+    ref = xe @ we.T + b
+    off = (K + 8) * 2.0 ** -24 * (np.abs(xe) @ np.abs(we).T + np.abs(b))
+    if glu:      # y = g sigmoid(1.702 g) (u + 1): slopes below 1.13 in g (times |u + 1|) and below |g| + 1 in u, both clamped at 7; 1e-5 for the exponential
+        g, u = np.minimum(ref[:, 0::2], 7.0), np.clip(ref[:, 1::2], -7.0, 7.0)
+        ref = g * so.sigmoid(1.702 * g) * (u + 1.0)
+        off = 1.13 * np.abs(u + 1.0) * off[:, 0::2] + (np.abs(g) + 1.0) * off[:, 1::2] + 1e-5 * (1.0 + np.abs(ref))
+    assert (np.abs(y - ref) <= off).all(), np.max(np.abs(y - ref) / off)
