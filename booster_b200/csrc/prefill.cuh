@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(SCB_KEYS, 3) k_attn_scores_batch(const AttnArg
 // P.V of a prompt batch: CTA = (KV head, 8 (token, head) rows), all 128 dims, two CTAs per SM. A half-warp is one of tinyBLAS' 16 chains (positions
 // c, c + 16, ...), a lane 8 rows x 8 dims: 32 packed fmas per position on one 16-byte load of V (f16, converted in registers) and two of p.
 // Bound by the fp32 pipe, with the loads close behind. What was tried on the way (512 tokens x 32 heads x 6256 keys): a thread = chain x dim, 32 rows, a load
-// of p per fma 1.90 ms (start); lane = 4 rows x 16 dims on V staged as fp32 1.06 ms (shared-memory pipe 79 %), now 0.88 ms.
+// of p per fma 1.90 ms; lane = 4 rows x 16 dims on V staged as fp32 1.06 ms (shared-memory pipe 79 %), now 0.88 ms.
 static constexpr int PVB_CHUNK = 64;           // positions staged at a time
 static constexpr int PVB_STAGES = 3;
 static constexpr int PVB_THREADS = 256;
