@@ -582,6 +582,7 @@ struct b200_ctx {
     cudaGraphExec_t g_pipe = nullptr;     // pipeline stage step (recv -> forward -> send)
     cudaGraphExec_t g_step = nullptr;     // H2D state -> forward -> arg-max -> D2H token (b200_step_greedy)
     int64_t n_step = 0;
+    std::shared_ptr<int32_t> pinned;      // h_tok and pb.err; later stages of a chain hold it too (pb.upstream)
     int32_t * h_tok = nullptr;            // pinned: the token b200_step_greedy hands back
     int64_t n_logits = 0, n_greedy = 0, n_pipe = 0;   // kernels per replay of g_logits / g_greedy / g_pipe
     int pipe_calls = 0;                   // b200_pipeline_generate_greedy calls so far (the first one runs un-graphed: NCCL connects lazily)
@@ -608,6 +609,9 @@ struct b200_ctx {
         uint8_t * rec = nullptr;
         int32_t * tokens = nullptr;
         int * err = nullptr;     // pinned, beside h_tok: raised by a kernel whose bounded wait ran out (pb_check)
+        // flags of the earlier stages whose residual rows this context has taken since its last check: their batches are complete when this
+        // context's stream is, so that checking the end of a chain checks all of it
+        std::vector<std::shared_ptr<int32_t>> upstream;
     } pb;
     // persistent per-token kernel (token_kernel.cuh): phase list in device memory, grid-barrier counter, transposed scores
     Phase * d_plan = nullptr;
@@ -1231,6 +1235,22 @@ static cudaGraphExec_t capture(b200_ctx * c, const std::function<void()> & body,
 }
 
 extern "C" void b200_ctx_free(b200_ctx * c);
+// [0] a token handed back by the device, [1] the error flag of the prompt kernels
+static std::shared_ptr<int32_t> pinned_token_and_flag() {
+    int32_t * p = nullptr;
+    CU(cudaMallocHost(&p, 2 * sizeof(int32_t)));
+    p[0] = p[1] = 0;
+    return std::shared_ptr<int32_t>(p, [](int32_t * q) { cudaFreeHost(q); });
+}
+// whether a prompt kernel of this context or of the stages it took rows from has given up; the flags are clear afterwards
+static bool pb_take_flags(b200_ctx * c) {
+    bool failed = false;
+    const auto take = [&](volatile int32_t * flag) { if (*flag) { *flag = 0; failed = true; } };
+    if (c->pb.err) take(c->pb.err);
+    for (const auto & f : c->pb.upstream) take(f.get() + 1);
+    c->pb.upstream.clear();
+    return failed;
+}
 extern "C" b200_ctx * b200_ctx_new(b200_model * m, int n_ctx) {
     std::unique_ptr<b200_ctx> c;
     try {
@@ -1289,9 +1309,8 @@ extern "C" b200_ctx * b200_ctx_new(b200_model * m, int n_ctx) {
         CU(cudaMemsetAsync(c->d_state, 0, sizeof(DecodeState), c->st));
         CU(cudaMallocHost(&c->h_state, sizeof(DecodeState)));
         CU(cudaMallocHost(&c->h_logits, (size_t) m->n_vocab * 4));
-        CU(cudaMallocHost(&c->h_tok, 2 * sizeof(int32_t)));
-        c->pb.err = c->h_tok + 1;
-        *c->pb.err = 0;
+        c->pinned = pinned_token_and_flag();
+        c->h_tok = c->pinned.get(); c->pb.err = c->h_tok + 1;
         c->out_tokens_cap = c->n_ctx + 8;
         CU(cudaMalloc(&c->d_out_tokens, (size_t) c->out_tokens_cap * 4));
         CU(cudaStreamSynchronize(c->st));
@@ -1326,7 +1345,7 @@ extern "C" void b200_ctx_free(b200_ctx * c) {
     cudaFree(c->pb.X); cudaFree(c->pb.Q); cudaFree(c->pb.ATT); cudaFree(c->pb.FFH); cudaFree(c->pb.S); cudaFree(c->pb.rec); cudaFree(c->pb.tokens);
     cudaFree(c->d_trace); cudaFree(c->d_plan); cudaFree(c->d_bar); cudaFree(c->S_T); cudaFree(c->d_ttrace);
     cudaFree(c->S); cudaFree(c->tickets); cudaFree(c->amax_key); cudaFree(c->rope); cudaFree(c->d_state); cudaFree(c->d_out_tokens);
-    cudaFreeHost(c->h_state); cudaFreeHost(c->h_logits); cudaFreeHost(c->h_tok);
+    cudaFreeHost(c->h_state); cudaFreeHost(c->h_logits);
     if (c->g_step) cudaGraphExecDestroy(c->g_step);
     if (c->ev_done) cudaEventDestroy(c->ev_done);
     if (c->ev_taken) cudaEventDestroy(c->ev_taken);
@@ -1342,6 +1361,7 @@ extern "C" void b200_kv_clear(b200_ctx * c) {
     // position, so the rows themselves need no clearing.
     cudaSetDevice(c->m->device);
     cudaStreamSynchronize(c->st);
+    pb_take_flags(c);                     // what a failed batch left behind goes with the rows
     c->cells = b200_ctx::KvCells();
 }
 
@@ -1647,9 +1667,9 @@ static bool prefill_batch_usable(const b200_ctx * c, int n) {
     if (m.n_ff % 256 || m.n_embd % 256 || std::max(m.n_ff, m.n_embd) / 256 > 4 * 16 * 4) return false;
     return true;
 }
-// after a synchronisation: a batch whose kernel gave up waiting left no result
+// after a synchronisation: a batch whose kernel gave up waiting left no result, here or on a stage before this one
 static void pb_check(b200_ctx * c) {
-    if (c->pb.err && *(volatile int *) c->pb.err) { *c->pb.err = 0; throw std::runtime_error("a prompt kernel's bounded wait ran out"); }
+    if (pb_take_flags(c)) throw std::runtime_error("a prompt kernel's bounded wait ran out");
 }
 static void prefill_alloc(b200_ctx * c) {
     if (c->pb.cap) return;
@@ -1896,6 +1916,12 @@ extern "C" int b200_stage_forward_batch(b200_ctx * c, const int32_t * tokens, in
             CU(cudaMemcpyPeerAsync(c->pb.X, m.device, prev->pb.X, prev->m->device, (size_t) n * m.n_embd * 4, c->st));
             CU(cudaEventRecord(prev->ev_taken, c->st));
             prev->taken_pending = true;
+            const auto note = [&](const std::shared_ptr<int32_t> & f) {
+                auto & u = c->pb.upstream;
+                if (std::find(u.begin(), u.end(), f) == u.end()) u.push_back(f);
+            };
+            note(prev->pinned);
+            for (const auto & f : prev->pb.upstream) note(f);
         } else {
             prefill_embed(c, tokens, n);
         }
@@ -1988,6 +2014,7 @@ extern "C" int b200_decode(b200_ctx * c, const int32_t * tokens, int n, int pos0
             CU(cudaGraphLaunch(c->g_logits, c->st));
             c->launches += c->n_logits;
             CU(cudaStreamSynchronize(c->st));   // h_state is reused for the next token
+            pb_check(c);
             if (last && logits_out) std::memcpy(logits_out, c->h_logits, (size_t) m.n_vocab * 4);
         }
         const double dt = now_us() - t0;
@@ -2041,6 +2068,7 @@ extern "C" int b200_generate_greedy(b200_ctx * c, int32_t first_token, int pos0,
         CU(cudaEventRecord(c->ev_t1, c->st));
         if (out_tokens) CU(cudaMemcpyAsync(out_tokens, c->d_out_tokens, (size_t) n_steps * 4, cudaMemcpyDeviceToHost, c->st));
         CU(cudaStreamSynchronize(c->st));
+        pb_check(c);
         CU(cudaEventElapsedTime(&c->last_device_ms, c->ev_t0, c->ev_t1));
         c->t_gen_us += now_us() - t0; c->n_gen += n_steps;
         return 0;
@@ -2088,6 +2116,7 @@ extern "C" int b200_step_greedy(b200_ctx * c, int32_t token, int pos, int32_t * 
             c->launches += c->n_step;
         }
         CU(cudaStreamSynchronize(c->st));
+        pb_check(c);
         *next_token = *c->h_tok;
         return 0;
     } catch (const std::exception & e) { return set_err(e.what()); }
@@ -2544,6 +2573,12 @@ extern "C" int b200_stage_forward(b200_ctx * c, int32_t token, int pos, int batc
         return 0;
     } catch (const std::exception & e) { return set_err(e.what()); }
 }
+// what a prompt kernel of this stage does when a bounded wait runs out, from the host
+extern "C" int b200_stage_raise(b200_ctx * c) {
+    if (!c || !c->pb.err) return set_err("not a context of the GGUF LLaMA path");
+    *(volatile int32_t *) c->pb.err = 1;
+    return 0;
+}
 // block until everything enqueued on this stage's stream has completed (the bridge brackets each prompt chunk with it,
 // as the reference brackets each blocking llama_decode with its timer: cpp/bridge.cpp:549-560)
 extern "C" int b200_stage_sync(b200_ctx * c) {
@@ -2743,6 +2778,7 @@ extern "C" int b200_op_mul_mat(int type, const void * w, int64_t n_rows, int64_t
     try {
         require_gpu();
         if (T <= 0 || T > PB_MAX_T) throw std::runtime_error("b200_op_mul_mat: 1..512 tokens");
+        const std::shared_ptr<int32_t> flag = pinned_token_and_flag();      // outlives the stream
         OpStream os;
         cudaStream_t st = os.st;
         const int64_t rows_pad = (n_rows + 63) / 64 * 64;
@@ -2765,9 +2801,7 @@ extern "C" int b200_op_mul_mat(int type, const void * w, int64_t n_rows, int64_t
         int dev = 0; CU(cudaGetDevice(&dev));
         tmp.device = dev;
         tmp.pb.rec = drec.as<uint8_t>();
-        CU(cudaMallocHost(&tmp.pb.err, sizeof(int)));
-        std::unique_ptr<int, cudaError_t (*)(void *)> err_owner(tmp.pb.err, cudaFreeHost);
-        *tmp.pb.err = 0;
+        tmp.pb.err = flag.get() + 1;
         MatvecArgs a{};
         a.seg[0] = d.m; a.n_seg = 1; a.n_units = d.m.n_units; a.k = (int) k; a.act_q8_0 = type == T_Q8_0;
         const int was = type == T_Q6_K;

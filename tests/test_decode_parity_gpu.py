@@ -380,3 +380,42 @@ def test_in_process_stage_split_prompt_batch(model_dir):
         x.close()
     for x in (m, m0, m1):
         x.close()
+
+
+def test_stage_chain_reports_an_earlier_stage_that_gave_up(tmp_path):
+    """a prompt kernel whose bounded wait runs out stores nothing and raises its stage's flag (raised here from the host): the end of the chain, which took
+    that stage's rows, must fail and not hand out what it computed from them; afterwards the chain works again"""
+    import ctypes as C
+    path = str(tmp_path / "m.gguf")
+    G.synth_llama(path, G.LlamaConfig(n_layer=3, n_embd=512, n_head=4, n_head_kv=1, n_ff=768, n_vocab=256, n_ctx_train=256), "Q4_K_M", seed=5)
+    ms = [engine.Model(path, 0, i, i + 1) for i in range(3)]
+    cs = [engine.Context(m, 64) for m in ms]
+    L = ms[0].L
+    toks = (C.c_int32 * 20)(*range(20))
+    out = np.empty(256, dtype=np.float32)
+    tok = C.c_int32()
+
+    def chain():
+        for i, c in enumerate(cs):
+            engine.check(L.b200_stage_forward_batch(c.h, toks, 20, 0, cs[i - 1].h if i else None), f"stage {i}")
+    reads = [lambda c: L.b200_stage_sync(c.h), lambda c: L.b200_stage_logits(c.h, out.ctypes.data_as(C.POINTER(C.c_float))),
+             lambda c: L.b200_stage_argmax(c.h, C.byref(tok)), lambda c: 0 if L.b200_stage_logits_view(c.h) else 1]
+    chain()
+    assert reads[1](cs[2]) == 0
+    want = out.copy()
+    for stage in range(3):
+        for read in reads:
+            chain()
+            engine.check(L.b200_stage_raise(cs[stage].h), "raise")
+            assert read(cs[2]) != 0 and b"bounded wait" in L.b200_last_error()
+            for c in cs:                                    # reported once, by the call that hit it
+                assert L.b200_stage_sync(c.h) == 0
+    chain()
+    engine.check(L.b200_stage_raise(cs[0].h), "raise")
+    for c in cs:                                            # a sequence that is given up takes its failure with it
+        c.kv_clear()
+    chain()
+    assert reads[1](cs[2]) == 0
+    _same(out, want, "logits after the failures")
+    for x in cs + ms:
+        x.close()
