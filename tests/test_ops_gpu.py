@@ -174,12 +174,20 @@ def _extreme_blocks(name, n, k, rng):
     return w.reshape(-1)
 
 
+@pytest.fixture
+def prefill_mma():
+    """engine.set_prefill_mma, which holds for the whole process: back at the default when the test ends"""
+    yield engine.set_prefill_mma
+    engine.set_prefill_mma(2)
+
+
+@pytest.mark.parametrize("k", [1024, 4096])
 @pytest.mark.parametrize("name", list(TYPES))
-def test_mul_mat_batch_extremes(name):
+def test_mul_mat_batch_extremes(name, k):
     """every quant at +-127 against the largest weights: the integer sums reach their bounds (Q6_K: 32 * 4096 * 127 < 2^24)
-    and must still come out of the fp16 tensor-core contraction exactly"""
+    and must still come out of the fp16 tensor-core contraction exactly, through mma.sync (short rows) and tcgen05 (long ones)"""
     rng = np.random.default_rng(11)
-    n, k, T = 64, 1024, 40
+    n, T = 64, 40
     w = _extreme_blocks(name, n, k, rng)
     x = rng.standard_normal((T, k)).astype(np.float32)
     x[0] = 3.0; x[1] = -3.0                          # every quant -127 / +127
@@ -193,18 +201,15 @@ def test_mul_mat_batch_extremes(name):
 
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K"])
 @pytest.mark.parametrize("shape", [(32, 2048, 1), (160, 2304, 32), (416, 4096, 65), (20480, 2048, 40)])
-def test_mul_mat_batch_tcgen05_edges(name, shape):
-    """k_umma_batch where its tiles end: one unit of a 128-row tile, the fewest super-blocks its rule takes, one token past a tile, more
-    tiles than SMs (a CTA's second tile starts behind its first one's epilogue) — the reference's bits"""
+def test_mul_mat_batch_tcgen05_edges(name, shape, prefill_mma):
+    """k_umma_batch where its tiles end: half of a 128-row tile (the operator pads to two units of 32 rows), the fewest super-blocks its rule takes, one
+    token past a tile, more tiles than SMs (a CTA's second tile starts behind its first one's epilogue) — the reference's bits"""
     n, k, T = shape
     rng = np.random.default_rng(n + k + T)
     w = _extreme_blocks(name, n, k, rng)
     x = (rng.standard_normal((T, k)) * rng.choice([0.01, 1.0, 30.0], size=(T, 1))).astype(np.float32)
-    engine.set_prefill_mma(2)
-    try:
-        y = engine.op_mul_mat(TYPES[name], w, n, k, x)
-    finally:
-        engine.set_prefill_mma(1)
+    prefill_mma(2)
+    y = engine.op_mul_mat(TYPES[name], w, n, k, x)
     for i in sorted({0, T // 2, T - 1}):
         yr = port.mul_mat_vec(TYPES[name], w, n, k, x[i])
         assert np.array_equal(y[i], yr), f"token {i}: max abs diff {np.abs(y[i] - yr).max()}"
@@ -212,19 +217,16 @@ def test_mul_mat_batch_tcgen05_edges(name, shape):
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0"])
-def test_mul_mat_batch_kernel_variants(name, mode):
-    """the batch kernels — mma.sync (1, default; Q8_0: the block-diagonal HMMA kernel), tcgen05 (2; K-quants), dp4a (0): A/B
+def test_mul_mat_batch_kernel_variants(name, mode, prefill_mma):
+    """the batch kernels — mma.sync (1; Q8_0: the block-diagonal HMMA kernel), tcgen05 (2, default; K-quants), dp4a (0): A/B
     switch b200_set_prefill_mma — give the reference's bits, on random blocks and on the worst-case magnitudes"""
     rng = np.random.default_rng(3)
     n, k, T = 256, 2048, 100
     x = rng.standard_normal((T, k)).astype(np.float32)
     x[0] = 3.0; x[1] = -3.0
     w = _extreme_blocks(name, n, k, rng)
-    engine.set_prefill_mma(mode)
-    try:
-        y = engine.op_mul_mat(TYPES[name], w, n, k, x)
-    finally:
-        engine.set_prefill_mma(1)
+    prefill_mma(mode)
+    y = engine.op_mul_mat(TYPES[name], w, n, k, x)
     for i in (0, 1, 2, 50, 99):
         yr = port.mul_mat_vec(TYPES[name], w, n, k, x[i])
         assert np.array_equal(y[i], yr), f"mode {mode} token {i}: max abs diff {np.abs(y[i] - yr).max()}"
