@@ -195,8 +195,9 @@ def test_self_extend_bitwise_golden(golden_dir, model):
 @pytest.mark.parametrize("kv_heads", [8, 4, 2, 1])
 def test_prompt_batch_attention_at_long_rows(tmp_path, kv_heads):
     """the batch attention where its variants meet: score rows on both sides of 2048 (a warp per row, then a block), of 4096 and 8192 (more scores per
-    thread), one token past a tile of 16, every group size; equal to the token-by-token kernels bit for bit"""
-    conf = G.LlamaConfig(n_layer=1, n_embd=1024, n_head=8, n_head_kv=kv_heads, n_ff=512, n_vocab=256, n_ctx_train=16384)
+    thread), one token past a tile of 16, every group size; equal to the token-by-token kernels bit for bit (the second layer's cached rows stand for
+    every token's attention in the first)"""
+    conf = G.LlamaConfig(n_layer=2, n_embd=1024, n_head=8, n_head_kv=kv_heads, n_ff=512, n_vocab=256, n_ctx_train=16384)
     path = str(tmp_path / "m.gguf")
     G.synth_llama(path, conf, "Q4_K_M", seed=kv_heads)
     rng = np.random.default_rng(kv_heads)
@@ -209,15 +210,46 @@ def test_prompt_batch_attention_at_long_rows(tmp_path, kv_heads):
             engine.set_prefill_batch(batch)
             try:
                 c = engine.Context(m, 8448)
-                if past:
-                    c.kv_write(0, 0, kv[0, :past], kv[1, :past])
-                got.append((c.decode(toks, past), c.kv_read(0, past, n)))
+                for layer in range(2 if past else 0):
+                    c.kv_write(layer, 0, kv[0, :past], kv[1, :past])
+                got.append((c.decode(toks, past), c.kv_read(1, past, n)))
                 c.close()
             finally:
                 engine.set_prefill_batch(True)
         _same(got[0][0], got[1][0], f"logits at {past}")
         for a, b in zip(got[0][1], got[1][1]):
             assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
+    m.close()
+
+
+@pytest.mark.parametrize("heads,kv_heads,n_ctx,past,n", [
+    (32, 8, 8192, 3000, 300),         # 1 MB of scores a token: launch groups of 222 tokens, whole waves of P.V blocks and no multiple of a tile of 16
+    (64, 8, 8192, 500, 150),          # 111 tokens
+    (8, 1, 16512, 16300, 200)])       # rows up to 16416 and 16512 scores, past what a block of the soft-max holds
+def test_prompt_batch_attention_in_launch_groups(tmp_path, heads, kv_heads, n_ctx, past, n):
+    """a batch whose scores do not fit the score buffer runs its attention in groups of tokens, and rows longer than 16384 scores go back to a warp each: the
+    same bits as token by token (the second layer's cached rows stand for every token's attention in the first)"""
+    conf = G.LlamaConfig(n_layer=2, n_embd=128 * heads, n_head=heads, n_head_kv=kv_heads, n_ff=256, n_vocab=256, n_ctx_train=16512)
+    path = str(tmp_path / "m.gguf")
+    G.synth_llama(path, conf, "Q4_K_M", seed=heads)
+    rng = np.random.default_rng(heads + n)
+    kv = rng.standard_normal((2, past, kv_heads * 128)).astype(np.float16)
+    toks = rng.integers(0, 256, size=n).tolist()
+    m = engine.Model(path)
+    got = []
+    for batch in (True, False):
+        engine.set_prefill_batch(batch)
+        try:
+            c = engine.Context(m, n_ctx)
+            for layer in range(2):
+                c.kv_write(layer, 0, kv[0], kv[1])
+            got.append((c.decode(toks, past), c.kv_read(1, past, n)))
+            c.close()
+        finally:
+            engine.set_prefill_batch(True)
+    _same(got[0][0], got[1][0], "logits")
+    for a, b in zip(got[0][1], got[1][1]):
+        assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
     m.close()
 
 
