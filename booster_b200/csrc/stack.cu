@@ -275,7 +275,8 @@ struct StackCtx {
     int sm_count = 148;
     __nv_bfloat16 * xb = nullptr;         // activations of a prompt pass rounded to bfloat16 (operand of the tcgen05 product)
     size_t xb_elems = 0;
-    float * xpart = nullptr;              // sums of the K parts of a product with few output tiles
+    float * xpart = nullptr;              // sums of the K parts of a product with few output tiles; a float32 context has it from the first such product on
+    bool no_xpart = false;                // ... or could not get it: its products stay whole
     int * d_err = nullptr, * h_err = nullptr;   // raised by a kernel whose bounded wait ran out
     bool taps = false;
     std::vector<float> tap_data;
@@ -1264,6 +1265,13 @@ constexpr int GX_MIN_K = 1024;                // shorter rows leave most of a bl
 struct UmmaScratch { __nv_bfloat16 * xb = nullptr; size_t elems = 0; int * err = nullptr; float * part = nullptr; int sm_count = 148; };
 size_t umma_part_floats(int sm_count) { return (size_t) sm_count * UM_BM * UM_BN; }      // one K part of an output tile per SM
 
+// K parts of a float32 product with few output tiles: two blocks per SM, 256 k each at least. (All parts together hold no more than two tiles of
+// 128 x 128 per SM, which is what umma_part_floats has room for.)
+int f32_k_parts(int T, int N, int K, int sm_count) {
+    if (T < 64 || N < SG_BN || !split_k_enabled() || !simt_big_enabled()) return 1;
+    return std::min(2 * sm_count / (((N + SG_BN - 1) / SG_BN) * ((T + SG_BM - 1) / SG_BM)), (K + SG_BK - 1) / SG_BK / 16);
+}
+
 // tensor map of a bf16 matrix batch [nz][rows][K] (strides in elements): boxes of 64 columns, one 128-byte swizzled row each, by box_rows
 CUtensorMap map_bf16(const void * base, int K, int rows, int nz, long long ld, long long sz, int box_rows) {
     static const auto encode = [] {
@@ -1306,11 +1314,7 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
     const auto al16 = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
     a.vec = K % vecw == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % vecw == 0 && al16(X) && al16(W);
     if (launches) (*launches)++;
-    int f32_parts = 1;
-    if (dtype == STACK_F32 && T >= 64 && N >= SG_BN && a.vec && batch == 1 && !a.glu && !a.seg && us && us->part && split_k_enabled() && simt_big_enabled()) {
-        f32_parts = std::min(2 * us->sm_count / (((N + SG_BN - 1) / SG_BN) * ((T + SG_BM - 1) / SG_BM)), (K + SG_BK - 1) / SG_BK / 16);
-        while (f32_parts > 1 && (size_t) f32_parts * T * N > umma_part_floats(us->sm_count)) f32_parts--;
-    }
+    const int f32_parts = dtype == STACK_F32 && a.vec && batch == 1 && !a.glu && !a.seg && us && us->part ? f32_k_parts(T, N, K, us->sm_count) : 1;
     const int gx_chunks = (K + GX_WARPS * 32 * vecw - 1) / (GX_WARPS * 32 * vecw);
     if (T == 1 && a.vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && gx_chunks <= 8 && sX % 4 == 0) {
         const dim3 grid((unsigned) ((N + GX_ROWS - 1) / GX_ROWS), 1, (unsigned) batch);
@@ -1349,7 +1353,7 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
         }
         else k_gemm_bf16_umma<<<grid, 256, UM_SMEM, st>>>(mx, mw, a, us->err);
         if (launches) (*launches)++;
-    } else if (f32_parts > 1) {      // few tiles: two blocks per SM by cutting K, 256 k each at least (a gated unit needs its sums whole: k_gemm_simt, 193 us against 236 in 128 x 128 tiles)
+    } else if (f32_parts > 1) {      // (a gated unit needs its sums whole: k_gemm_simt, 193 us against 236 in 128 x 128 tiles)
         k_gemm_simt_big<<<dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((T + SG_BM - 1) / SG_BM), (unsigned) f32_parts), 256, 0, st>>>(a, f32_parts, us->part);
         k_split_sum<<<dim3((unsigned) ((N + 255) / 256), (unsigned) T), 256, 0, st>>>(us->part, f32_parts, T, N, bias, Y, ldy);
         if (launches) (*launches)++;
@@ -1365,6 +1369,11 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
 
 void linear(StackCtx * c, const float * X, int ldx, const DMat & W, float * Y, int ldy, int T, int batch = 1, long long sX = 0, long long sY = 0, bool glu = false, float glu_limit = 0.f,
             const LinOpt * opt = nullptr) {
+    // (never inside a capture: only products of 64 tokens and more are cut along K)
+    if (c->m->dtype == STACK_F32 && batch == 1 && !glu && f32_k_parts(T, W.N, W.K, c->sm_count) > 1 && !c->xpart && !c->no_xpart && cudaMalloc(&c->xpart, umma_part_floats(c->sm_count) * 4) != cudaSuccess) {
+        cudaGetLastError();
+        c->xpart = nullptr; c->no_xpart = true;
+    }
     const UmmaScratch us{c->xb, c->xb_elems, c->d_err, c->xpart, c->sm_count};
     linear_on(c->st, c->m->dtype, &c->launches, X, ldx, W.w, W.bias, Y, ldy, T, W.N, W.K, batch, sX, (long long) W.N * W.K, sY, glu, glu_limit, &us, opt);
 }
@@ -2525,8 +2534,8 @@ StackCtx * stack_ctx_new(StackModel * m, int n_ctx) {
         if (m->dtype == STACK_BF16) {
             c->xb_elems = std::max(cap * (size_t) std::max({ 2 * m->E, m->maxA, m->maxOL, m->maxP, m->max_dense, m->side_dim }), moe_rows * (size_t) std::max(m->E, m->max_eff));
             SCU(cudaMalloc(&c->xb, c->xb_elems * 2));
+            SCU(cudaMalloc(&c->xpart, umma_part_floats(c->sm_count) * 4));
         }
-        SCU(cudaMalloc(&c->xpart, umma_part_floats(c->sm_count) * 4));
         SCU(cudaMalloc(&c->d_err, 4)); SCU(cudaMemsetAsync(c->d_err, 0, 4, c->st));
         SCU(cudaMallocHost(&c->h_err, 4)); *c->h_err = 0;
         c->caches.assign((size_t) m->n_caches, nullptr);

@@ -449,3 +449,21 @@ def test_products_where_their_rules_change(dtype, T, N, K, glu):
         ref = g * so.sigmoid(1.702 * g) * (u + 1.0)
         off = 1.13 * np.abs(u + 1.0) * off[:, 0::2] + (np.abs(g) + 1.0) * off[:, 1::2] + 1e-5 * (1.0 + np.abs(ref))
     assert (np.abs(y - ref) <= off).all(), np.max(np.abs(y - ref) / off)
+
+
+def test_float32_contexts_hold_no_room_for_products_they_never_run(tmp_path):
+    """a float32 context has the 19 MB for products cut along K from its first portion of 64 tokens on, and not before: sixteen small contexts stay well below
+    what that room alone would take, and one that does run such a portion decodes the same rows afterwards"""
+    torch = pytest.importorskip("torch")
+    p = Pair(tmp_path, config([mingru(width=200)], width=1056), n_ctx=160)      # 600 x 1056: four K parts
+    free = torch.cuda.mem_get_info()[0]
+    more = [engine.Context(p.model, 160) for _ in range(16)]
+    used = free - torch.cuda.mem_get_info()[0]
+    assert used < 16 * 16 << 20, used
+    toks = np.random.default_rng(3).integers(0, 61, size=128).tolist()
+    a, b = (c.decode_rows(toks, 0, [5, 127]) for c in more[:2])
+    assert np.array_equal(a, b)
+    assert err(a, p.expected(toks)[[5, 127]]) < TOL32
+    for c in more:
+        c.close()
+    p.close()
