@@ -1803,6 +1803,20 @@ static void pb_matmul(b200_ctx * c, const MatvecArgs & mv, int epi, int T, int p
     k_matmul_batch<<<grid, PB_WARPS * 32, smem, c->st>>>(a, sb);
     c->launches++;
 }
+// tokens per block of k_attn_scores_batch for nz tokens, the first of which sees n_kv cells. A block walks its tokens x GQA rows one after the other on
+// keys that it loads once: many rows save loads, few keep the SMs busy to the end. Halved from 16 until there are six blocks of 64 rows per SM, or as many more
+// as they are shorter (measured with 1, 2, 4, 8 and 16 tokens, 8 to 512 tokens at 0 to 8000, 8 heads on 1 key head to 64 on 8: within 5 % of the best of them, and
+// 16 heads on 2 key heads, 512 tokens at 0, two layers: 797 us with 16 tokens, 704 with four; 32 on 8, 512 at 8000: 7.1 ms with 16, 7.9 with four).
+static int scb_tokens(int n_head_kv, int gqa, int n_kv, int nz, int sm_count) {
+    for (int tq = SCB_TQ; ; tq /= 2) {
+        int64_t blocks = 0;                                // those with keys that a token of theirs sees
+        for (int z = 0; z < nz; z += tq) blocks += ((n_kv + std::min(z + tq, nz) - 1 + 31) / 32 * 32 + SCB_KEYS - 1) / SCB_KEYS;
+        if (tq == 1 || blocks * n_head_kv * 64 >= (int64_t) 6 * sm_count * tq * gqa) return tq;
+    }
+}
+extern "C" int b200_op_score_tokens(int n_head_kv, int gqa, int past, int n, int sm_count) {
+    return n_head_kv > 0 && gqa > 0 && past >= 0 && n > 0 && sm_count > 0 ? scb_tokens(n_head_kv, gqa, past + 1, n, sm_count) : 0;
+}
 template <int GQA>
 static void pb_attention(b200_ctx * c, int li, int T, int pos0) {
     const b200_model & m = *c->m;
@@ -1821,11 +1835,12 @@ static void pb_attention(b200_ctx * c, int li, int T, int pos0) {
             if (!launch_attention_2k<GQA>(c, a, n_pad_max, nz)) throw std::runtime_error("batched attention does not fit");
             continue;
         }
-        const dim3 gs((unsigned) a.n_head_kv, (unsigned) ((n_pad_max + SCB_KEYS - 1) / SCB_KEYS), (unsigned) ((nz + SCB_TQ - 1) / SCB_TQ));
-        constexpr size_t smem_sc = (size_t) SCB_TQ * GQA * 128 * 4;
+        const int tq = scb_tokens(a.n_head_kv, GQA, a.n_kv_override, nz, c->sm_count);
+        const dim3 gs((unsigned) a.n_head_kv, (unsigned) ((n_pad_max + SCB_KEYS - 1) / SCB_KEYS), (unsigned) ((nz + tq - 1) / tq));
+        const size_t smem_sc = (size_t) tq * GQA * 128 * 4;
         static size_t attr_sc[64] = {0};
         if (smem_sc > 48 * 1024) raise_smem(k_attn_scores_batch<GQA>, smem_sc, attr_sc, c->device);
-        k_attn_scores_batch<GQA><<<gs, SCB_KEYS, smem_sc, c->st>>>(a, nz);
+        k_attn_scores_batch<GQA><<<gs, SCB_KEYS, smem_sc, c->st>>>(a, nz, tq);
         const unsigned rows = (unsigned) (nz * a.n_head);
         const int groups = (n_pad_max / 16 + SMX_THREADS - 1) / SMX_THREADS;
         if (n_pad_max < SMX_MIN_ROW || groups > SMX_MAX_G) k_attn_softmax_rows<<<(rows + 7) / 8, 256, 0, c->st>>>(a, nz);

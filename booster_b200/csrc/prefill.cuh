@@ -220,20 +220,20 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; a
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
-// scores of a prompt batch: CTA = (KV head, 128 keys, 16 tokens), a thread = one key, whose 128 values sit in registers as packed pairs for all
-// 16 x GQA dot products. Each is ggml_vec_dot_f16 on q rounded to f16: 4 accumulators x 16 lanes over i in {0, 64}, (0+2)+(1+3),
+// scores of a prompt batch: CTA = (KV head, 128 keys, tq <= 16 tokens), a thread = one key, whose 128 values sit in registers as packed pairs for all
+// tq x GQA dot products. Each is ggml_vec_dot_f16 on q rounded to f16: 4 accumulators x 16 lanes over i in {0, 64}, (0+2)+(1+3),
 // _mm512_reduce_add_ps (cpp/ggml/src/ggml.c:12345-12371) — the batch > 1 branch of k_attn_scores — in 96 packed instructions and 32 broadcast
 // loads of q, with no exchange between lanes. Bound by those loads and the packed arithmetic together (ncu: shared-memory pipe 84 %, fp32 pipe 58 %). Four
-// lanes per key with scalar arithmetic: 512 tokens x 32 heads x 6256 keys 2.08 ms, now 1.03 ms. Four lanes sharing four keys (a quarter of the loads, 12
-// shuffles): 1.02 ms, not worth its code. A token's row ends at its own padded length (-inf from its n_kv to there).
+// lanes per key with scalar arithmetic: 512 tokens x 32 heads x 6256 keys 2.08 ms, now 1.03 ms. A token's row ends at its own padded length
+// (-inf from its n_kv to there).
 static constexpr int SCB_TQ = 16, SCB_KEYS = 128;
 template <int GQA>
-__global__ void __launch_bounds__(SCB_KEYS, 3) k_attn_scores_batch(const AttnArgs a, int nz) {
+__global__ void __launch_bounds__(SCB_KEYS, 3) k_attn_scores_batch(const AttnArgs a, int nz, int tq) {
     constexpr int HD = 128;
     extern __shared__ __align__(16) uint8_t scb_dyn[];
-    float * qs = reinterpret_cast<float *>(scb_dyn);                          // [SCB_TQ * GQA][HD]
-    const int g = blockIdx.x, tile = blockIdx.y, z0 = blockIdx.z * SCB_TQ, tid = threadIdx.x;
-    const int ntok = min(SCB_TQ, nz - z0);
+    float * qs = reinterpret_cast<float *>(scb_dyn);                          // [tq * GQA][HD]
+    const int g = blockIdx.x, tile = blockIdx.y, z0 = blockIdx.z * tq, tid = threadIdx.x;
+    const int ntok = min(tq, nz - z0);
     const int n_kv_last = a.n_kv_override + z0 + ntok - 1;
     if (tile * SCB_KEYS >= (n_kv_last + 31) / 32 * 32) return;
     const int t = tile * SCB_KEYS + tid;

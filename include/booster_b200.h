@@ -229,6 +229,8 @@ float * b200_decode_view(b200_ctx * c, int32_t token, int pos);
 /* launch shape (warps per CTA, warps sharing a 32-row unit, ring stages per warp) the engine picks for a mat-vec whose
  * segments have the given block types: pure host arithmetic, exposed so that tests pin the shapes */
 int b200_op_launch_shape(const int32_t * types, int n_types, int64_t n_units, int64_t k, int norm, int sm_count, int32_t wgs[3]);
+/* tokens per block of a prompt batch's score kernel: n tokens behind `past` cells (host arithmetic, as above) */
+int b200_op_score_tokens(int n_head_kv, int gqa, int past, int n, int sm_count);
 
 /* ---- tokenizer (host side) ----------------------------------------------------------------------
  * The vocabulary of a GGUF (tokenizer.ggml.model = "llama" (SPM), "gpt2" (byte-level BPE, LLaMA-3 pre-tokenizer) or
