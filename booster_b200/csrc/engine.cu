@@ -1696,15 +1696,17 @@ static void prefill_alloc(b200_ctx * c) {
     c->pb.cap = T;
 }
 static bool has_q6k(const TMat * seg, int n_seg) { for (int i = 0; i < n_seg; i++) if (seg[i].type == T_Q6_K) return true; return false; }
-// K-quant launches run on the tensor cores: tcgen05 (prefill_umma.cuh), or mma.sync (prefill_mma.cuh) for short rows
+// K-quant launches run on the tensor cores: tcgen05 (prefill_umma.cuh), or mma.sync (prefill_mma.cuh) for few and short rows
 static int g_prefill_mma = -1;         // 2 (default): tcgen05 (k_umma_batch) where it is the faster one, 1: mma.sync (k_mma_batch), 0: the dp4a kernel
 extern "C" void b200_set_prefill_mma(int mode) { g_prefill_mma = mode < 0 ? 0 : mode > 2 ? 2 : mode; }
-// A launch of k_umma_batch pays 2 to 4 us more than one of k_mma_batch before its first and after its last super-block (tensor memory, a longer pipeline),
-// and gains a quarter of a microsecond and more on each super-block between: rows of fewer than eight stay with mma.sync (k = 512..768, 8..96
-// tokens: 270 us a pass of 12 launches against 310; k = 4096, 31 tokens: 2520 against 2240 of 32).
+// Where the two K-quant products part. Both run one block per SM; k_mma_batch's tiles are 64 rows x 32 tokens, k_umma_batch's twice as many rows, and a
+// super-block takes either 1.2 to 2 us. So as soon as mma.sync needs a second wave, tcgen05 is ahead at every k and type (k = 256 to 14336, 512 to 28672 rows, 8 to
+// 512 tokens: 0.40 to 0.90 of its time; Q4_K, 1024 rows x k = 1024, 512 tokens 29 and 22 us). While one wave is enough, it is the super-blocks that count: Q4_K and Q6_K gain
+// 2 us of 21 to 40 from k = 2048 on, on weights that come from memory (4096 x 4096, 32 tokens: 32 and 30 us); shorter rows lose what the longer pipeline
+// costs, 1 to 3 us a launch (k = 512 and 768, 8 tokens, 16 launches: 350 and 389 us). Q5_K expands slowest and is behind at every k (4096 x 4096, 32 tokens: 34 and 37 us).
 static constexpr int UM_MIN_K = 2048;
 // record layout / kernel of a launch: 3 = k_mma_batch_q80, 2 = k_umma_batch, 1 = k_mma_batch (segments of an even number of units), 0 = dp4a
-static int pb_mma_mode(const MatvecArgs & mv) {
+static int pb_mma_mode(const MatvecArgs & mv, int T, int sm_count) {
     if (g_prefill_mma < 0) { const char * e = getenv("BOOSTER_B200_PREFILL_MMA"); g_prefill_mma = e ? std::max(0, std::min(2, atoi(e))) : 2; }
     if (g_prefill_mma == 0) return 0;
     bool even = true;
@@ -1717,10 +1719,23 @@ static int pb_mma_mode(const MatvecArgs & mv) {
         const int t = mv.seg[i].type;
         if (t != T_Q4_K && t != T_Q5_K && t != T_Q6_K) return 0;
     }
-    if (g_prefill_mma == 2 && (mv.k >= UM_MIN_K || !even)) return 2;
-    return even ? 1 : 0;
+    if (!even) return 0;
+    if (g_prefill_mma == 2) {
+        int64_t tiles = 0;
+        bool q5 = false;
+        for (int i = 0; i < mv.n_seg; i++) { tiles += mv.seg[i].n_units / 2; q5 = q5 || mv.seg[i].type == T_Q5_K; }
+        if (tiles * ((T + MB_NT - 1) / MB_NT) > sm_count || (mv.k >= UM_MIN_K && !q5)) return 2;
+    }
+    return 1;
 }
-static bool pb_use_mma(const MatvecArgs & mv) { return pb_mma_mode(mv) != 0; }
+// the kernel of one prompt product of a matrix with the given block types (host arithmetic; segments share the units evenly)
+extern "C" int b200_op_prompt_kernel(const int32_t * types, int n_types, int64_t n_units, int64_t k, int T, int sm_count) {
+    if (!types || n_types <= 0 || n_types > 3 || n_units <= 0 || k <= 0 || k % 256 || T <= 0 || sm_count <= 0) { set_err("bad arguments"); return -1; }
+    MatvecArgs mv{};
+    mv.n_seg = n_types; mv.n_units = (int) n_units; mv.k = (int) k; mv.act_q8_0 = types[0] == T_Q8_0;
+    for (int i = 0; i < n_types; i++) { mv.seg[i].type = types[i]; mv.seg[i].n_units = (int) (n_units / n_types + (i < n_units % n_types ? 1 : 0)); }
+    return pb_mma_mode(mv, T, sm_count);
+}
 static void pb_quant(b200_ctx * c, const float * X, int k, int T, const float * norm_w, int act_q8_0, int with_as, int mma = 0) {
     QuantBatchArgs a{};
     a.X = X; a.k = k; a.T = T; a.norm_w = norm_w; a.eps = norm_w ? c->m->rms_eps : 0.f; a.inv_k = (k & (k - 1)) == 0 ? 1.0 / (double) k : 0.0;
@@ -1748,7 +1763,7 @@ static void pb_matmul(b200_ctx * c, const MatvecArgs & mv, int epi, int T, int p
     a.n_q = mv.n_q; a.n_k = mv.n_k; a.head_dim = mv.head_dim; a.kv_dim = mv.kv_dim; a.rope = mv.rope; a.pos0 = pos0;
     int sb = 0;
     for (int i = 0; i < mv.n_seg; i++) sb = std::max(sb, tile_bytes_of(mv.seg[i].type));
-    const int mma_mode = pb_mma_mode(mv);
+    const int mma_mode = pb_mma_mode(mv, T, c->sm_count);
     bool q4 = false, q5 = false, q6 = false;
     for (int i = 0; i < mv.n_seg; i++) { q4 |= mv.seg[i].type == T_Q4_K; q5 |= mv.seg[i].type == T_Q5_K; q6 |= mv.seg[i].type == T_Q6_K; }
     if (mma_mode == 3) {
@@ -1863,7 +1878,7 @@ static void prefill_layers(b200_ctx * c, int T, int p0) {
         const int q80 = L.qkv.seg[0].type == T_Q8_0;
         const MatvecArgs aq = args_qkv(c, li), ao = args_wo(c, li), ag = args_gateup(c, li), ad = args_down(c, li);
         int was = has_q6k(aq.seg, aq.n_seg);
-        pb_quant(c, c->pb.X, E, T, L.attn_norm, q80, was, pb_mma_mode(aq));
+        pb_quant(c, c->pb.X, E, T, L.attn_norm, q80, was, pb_mma_mode(aq, T, c->sm_count));
         pb_matmul(c, aq, EPI_QKV, T, p0, nullptr, 0, nullptr, was);
         switch (m.n_head / m.n_head_kv) {
             case 1: pb_attention<1>(c, li, T, p0); break;
@@ -1872,13 +1887,13 @@ static void prefill_layers(b200_ctx * c, int T, int p0) {
             default: pb_attention<8>(c, li, T, p0); break;
         }
         was = has_q6k(ao.seg, 1);
-        pb_quant(c, c->pb.ATT, QD, T, nullptr, q80, was, pb_mma_mode(ao));
+        pb_quant(c, c->pb.ATT, QD, T, nullptr, q80, was, pb_mma_mode(ao, T, c->sm_count));
         pb_matmul(c, ao, EPI_RESID, T, p0, c->pb.X, E, c->pb.X, was);
         was = has_q6k(ag.seg, 1);
-        pb_quant(c, c->pb.X, E, T, L.ffn_norm, q80, was, pb_mma_mode(ag));
+        pb_quant(c, c->pb.X, E, T, L.ffn_norm, q80, was, pb_mma_mode(ag, T, c->sm_count));
         pb_matmul(c, ag, EPI_SILU, T, p0, c->pb.FFH, FF, nullptr, was);
         was = has_q6k(ad.seg, 1);
-        pb_quant(c, c->pb.FFH, FF, T, nullptr, q80, was, pb_mma_mode(ad));
+        pb_quant(c, c->pb.FFH, FF, T, nullptr, q80, was, pb_mma_mode(ad, T, c->sm_count));
         pb_matmul(c, ad, EPI_RESID, T, p0, c->pb.X, E, c->pb.X, was);
     }
     CU(cudaGetLastError());
@@ -2820,7 +2835,7 @@ extern "C" int b200_op_mul_mat(int type, const void * w, int64_t n_rows, int64_t
         MatvecArgs a{};
         a.seg[0] = d.m; a.n_seg = 1; a.n_units = d.m.n_units; a.k = (int) k; a.act_q8_0 = type == T_Q8_0;
         const int was = type == T_Q6_K;
-        pb_quant(&tmp, dx.as<float>(), (int) k, (int) T, nullptr, a.act_q8_0, was, pb_mma_mode(a));
+        pb_quant(&tmp, dx.as<float>(), (int) k, (int) T, nullptr, a.act_q8_0, was, pb_mma_mode(a, (int) T, tmp.sm_count));
         pb_matmul(&tmp, a, EPI_STORE, (int) T, 0, dy.as<float>(), (int) rows_pad, nullptr, was);
         CU(cudaGetLastError());
         std::vector<float> hy((size_t) T * rows_pad);

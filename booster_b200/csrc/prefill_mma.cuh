@@ -18,8 +18,8 @@
 //
 // mma.sync.m16n8k16 (HMMA): the accumulator of every (super-block, lane) is in the register file for its own fp32 chain step — 8 + 4
 // FFMA per 256 MACs and output — so the kernel is bound by that CUDA-core epilogue and by fragment traffic through shared memory (ncu:
-// HMMA pipe 22-26 % busy, shared-memory pipe 60 %). Long rows go to the tcgen05 kernel (prefill_umma.cuh), which takes the
-// fragments off the shared memory; this one has the shorter pipeline and serves short rows.
+// HMMA pipe 22-26 % busy, shared-memory pipe 60 %). Larger products go to the tcgen05 kernel (prefill_umma.cuh), which takes the fragments
+// off the shared memory; this one has smaller tiles and the shorter pipeline and serves what one wave of them covers (pb_mma_mode).
 //
 // Shape: CTA = 64 rows (two 32-row units of the tiled weight layout) x 32 tokens, 16 warps. Per super-block (K step):
 //   TMA bulk copies: the two raw weight tiles + the chunk's activation record block (fp16, MMA order, written by

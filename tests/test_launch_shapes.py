@@ -53,3 +53,13 @@ def test_launch_shape_rejects_oversized_vectors():
 def test_score_tile(kv, gqa, past, n, want):
     """tokens per block of a prompt batch's score kernel: few enough that the grid fills 148 SMs"""
     assert _lib.lib().b200_op_score_tokens(kv, gqa, past, n, 148) == want
+
+
+@pytest.mark.parametrize("types,rows,k,T,want", [
+    ([Q4_K], 28672, 4096, 8, 2), ([Q5_K], 28672, 4096, 8, 2), ([Q4_K], 2048, 1024, 512, 2), ([Q5_K], 9536, 256, 32, 2),    # a second wave of 64 x 32 tiles
+    ([Q4_K], 4096, 4096, 32, 2), ([Q6_K], 1024, 2816, 8, 2), ([Q4_K, Q6_K], 6144, 4096, 32, 2),                            # one wave, long rows
+    ([Q5_K], 4096, 4096, 32, 1), ([Q5_K, Q6_K], 2560, 2048, 33, 1), ([Q4_K], 768, 512, 100, 1), ([Q4_K], 4096, 1792, 8, 1),
+    ([Q8_0], 4096, 4096, 32, 3), ([Q4_K], 96, 4096, 512, 0), ([Q4_K, Q8_0], 128, 4096, 32, 0)])
+def test_prompt_product_kernel(types, rows, k, T, want):
+    """which kernel a prompt product takes (2 tcgen05, 1 mma.sync, 3 Q8_0's mma.sync, 0 dp4a); an odd number of 32-row units goes to dp4a"""
+    assert _lib.lib().b200_op_prompt_kernel((C.c_int32 * len(types))(*types), len(types), rows // 32, k, T, 148) == want

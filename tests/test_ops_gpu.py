@@ -1,13 +1,14 @@
 """Operator-level parity of the CUDA kernels (through the C-ABI, same kernels the engine launches) against
 the golden vectors the reference produced and against the port oracle on seeded inputs.
 EVERYTHING is bit-exact: the kernels reproduce the reference's fp32 operation order (see kernels.cuh)."""
+import ctypes as C
 import os
 
 import numpy as np
 import pytest
 
 from conftest import q8k_equal, rel_err
-from booster_b200 import engine, gguf_io as G
+from booster_b200 import _lib, engine, gguf_io as G
 from oracle import port
 
 pytestmark = pytest.mark.gpu
@@ -185,7 +186,7 @@ def prefill_mma():
 @pytest.mark.parametrize("name", list(TYPES))
 def test_mul_mat_batch_extremes(name, k):
     """every quant at +-127 against the largest weights: the integer sums reach their bounds (Q6_K: 32 * 4096 * 127 < 2^24)
-    and must still come out of the fp16 tensor-core contraction exactly, through mma.sync (short rows) and tcgen05 (long ones)"""
+    and must still come out of the fp16 tensor-core contraction exactly, through mma.sync (short rows, Q5_K) and tcgen05 (long ones)"""
     rng = np.random.default_rng(11)
     n, T = 64, 40
     w = _extreme_blocks(name, n, k, rng)
@@ -200,15 +201,20 @@ def test_mul_mat_batch_extremes(name, k):
 
 
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K"])
-@pytest.mark.parametrize("shape", [(32, 2048, 1), (160, 2304, 32), (416, 4096, 65), (20480, 2048, 40)])
+@pytest.mark.parametrize("shape", [(32, 2048, 1), (160, 2304, 32), (416, 4096, 65), (20480, 2048, 40), (9536, 256, 1), (9536, 2304, 32), (4800, 4096, 65)])
 def test_mul_mat_batch_tcgen05_edges(name, shape, prefill_mma):
-    """k_umma_batch where its tiles end: half of a 128-row tile (the operator pads to two units of 32 rows), the fewest super-blocks its rule takes, one
-    token past a tile, more tiles than SMs (a CTA's second tile starts behind its first one's epilogue) — the reference's bits"""
+    """k_umma_batch where its tiles end: half of a 128-row tile (the operator pads to two units of 32 rows), one super-block, one token past a tile, more tiles
+    than SMs (a CTA's second tile starts behind its first one's epilogue), and where its rule begins: one tile of mma.sync past a wave, for every type — the
+    reference's bits, on the largest weights and, for the first and last token, the largest quants"""
     n, k, T = shape
     rng = np.random.default_rng(n + k + T)
     w = _extreme_blocks(name, n, k, rng)
     x = (rng.standard_normal((T, k)) * rng.choice([0.01, 1.0, 30.0], size=(T, 1))).astype(np.float32)
+    x[0], x[-1] = 3.0, -3.0
     prefill_mma(2)
+    if n > 1000 or name != "Q5_K":
+        rows = (n + 63) // 64 * 64
+        assert _lib.lib().b200_op_prompt_kernel((C.c_int32 * 1)(TYPES[name]), 1, rows // 32, k, T, 148) == 2
     y = engine.op_mul_mat(TYPES[name], w, n, k, x)
     for i in sorted({0, T // 2, T - 1}):
         yr = port.mul_mat_vec(TYPES[name], w, n, k, x[i])
