@@ -2152,6 +2152,10 @@ extern "C" int b200_step_greedy(b200_ctx * c, int32_t token, int pos, int32_t * 
     } catch (const std::exception & e) { return set_err(e.what()); }
 }
 
+extern "C" int b200_stack_product_kernel(int dtype, int T, int N, int K, int glu, int sm_count) {
+    if (T <= 0 || N <= 0 || K <= 0 || sm_count <= 0 || (dtype != 0 && dtype != 1)) { set_err("bad arguments"); return -1; }
+    return b200::stack_product_kernel(dtype, T, N, K, glu != 0, sm_count);
+}
 extern "C" float b200_stack_time_linear(int device, int dtype, int T, int N, int K, int reps) {
     try {
         require_gpu();

@@ -1265,11 +1265,30 @@ constexpr int GX_MIN_K = 1024;                // shorter rows leave most of a bl
 struct UmmaScratch { __nv_bfloat16 * xb = nullptr; size_t elems = 0; int * err = nullptr; float * part = nullptr; int sm_count = 148; };
 size_t umma_part_floats(int sm_count) { return (size_t) sm_count * UM_BM * UM_BN; }      // one K part of an output tile per SM
 
-// K parts of a float32 product with few output tiles: two blocks per SM, 256 k each at least. (All parts together hold no more than two tiles of
-// 128 x 128 per SM, which is what umma_part_floats has room for.)
+// K parts of a float32 product with few output tiles: two blocks of 128 x 128 per SM, 256 k each at least, where that is faster than 64 x 64 tiles (else 1). (All
+// parts together hold no more than two tiles per SM, which is what umma_part_floats has room for.)
+// The two times in us, from T = 64 to 600, N = 128 to 16000, K = 512 to 4096 on 148 SMs: a thin wave of 64 x 64 tiles takes 0.0725 per k, a fuller one more with its blocks per
+// SM (more still on weights that do not fit the L2); a part takes 0.137 per k with an SM to itself, 0.208 beside a second one. At K = 512 it goes either way: 600 x 1024 50
+// us whole and 44 in two parts, 600 x 640 41 and 44; so it does where half of each tile's rows are empty: 64 x 16000 x 1024 118 and 121. Long sums gain most: 300 x 1024 x 4096 355 and 88.
 int f32_k_parts(int T, int N, int K, int sm_count) {
     if (T < 64 || N < SG_BN || !split_k_enabled() || !simt_big_enabled()) return 1;
-    return std::min(2 * sm_count / (((N + SG_BN - 1) / SG_BN) * ((T + SG_BM - 1) / SG_BM)), (K + SG_BK - 1) / SG_BK / 16);
+    const int tiles = ((N + SG_BN - 1) / SG_BN) * ((T + SG_BM - 1) / SG_BM), parts = std::min(2 * sm_count / tiles, (K + SG_BK - 1) / SG_BK / 16);
+    if (parts <= 1) return 1;
+    const float per_sm = (float) (((N + 63) / 64) * ((T + 63) / 64)) / (float) sm_count;
+    const float whole = 4.f + (float) K * (per_sm <= 0.7f ? 0.0725f : 0.075f + 0.024f * per_sm);
+    const float cut = tiles * parts > sm_count ? 15.f + 0.208f * (float) K / (float) parts : 6.f + 0.137f * (float) K / (float) parts;
+    return cut < 0.97f * whole ? parts : 1;
+}
+
+// the kernel a product goes to: mat-vecs of few tokens, then tile kernels
+enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG, LIN_ROWS_X, LIN_UMMA, LIN_F32_PARTS, LIN_MMA, LIN_SIMT };
+// vec: LinArgs::vec; x_elems: entries of X; xb_elems, part: what the scratch has room for
+LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu, bool seg, size_t x_elems, size_t xb_elems, bool part, int sm_count) {
+    if (T == 1 && vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && K / (dtype == STACK_F32 ? 4 : 8) <= 8 * GX_WARPS * 32) return LIN_ROWS_X;
+    if (T <= GEMV_MAX_T) return !glu && batch == 1 && N <= GEMV_FEW_ROWS && K >= 1024 ? LIN_ROWS_LONG : LIN_ROWS;      // few, long rows: a block each
+    if (dtype == STACK_BF16 && vec && umma_enabled() && T >= 64 && N >= 128 && K >= 64 && x_elems <= xb_elems) return LIN_UMMA;
+    if (dtype == STACK_F32 && vec && batch == 1 && !glu && !seg && part && f32_k_parts(T, N, K, sm_count) > 1) return LIN_F32_PARTS;
+    return dtype == STACK_BF16 && vec && mma_enabled() ? LIN_MMA : LIN_SIMT;
 }
 
 // tensor map of a bf16 matrix batch [nz][rows][K] (strides in elements): boxes of 64 columns, one 128-byte swizzled row each, by box_rows
@@ -1314,9 +1333,9 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
     const auto al16 = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
     a.vec = K % vecw == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % vecw == 0 && al16(X) && al16(W);
     if (launches) (*launches)++;
-    const int f32_parts = dtype == STACK_F32 && a.vec && batch == 1 && !a.glu && !a.seg && us && us->part ? f32_k_parts(T, N, K, us->sm_count) : 1;
-    const int gx_chunks = (K + GX_WARPS * 32 * vecw - 1) / (GX_WARPS * 32 * vecw);
-    if (T == 1 && a.vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && gx_chunks <= 8 && sX % 4 == 0) {
+    const LinRoute route = lin_route(dtype, T, N, K, batch, a.vec != 0, a.glu != 0, a.seg != nullptr, (size_t) xbatch * T * K, us && us->xb ? us->elems : 0, us && us->part, us ? us->sm_count : 148);
+    if (route == LIN_ROWS_X) {
+        const int gx_chunks = (K + GX_WARPS * 32 * vecw - 1) / (GX_WARPS * 32 * vecw);
         const dim3 grid((unsigned) ((N + GX_ROWS - 1) / GX_ROWS), 1, (unsigned) batch);
         const auto go = [&](auto wt) {
             using WT = decltype(wt);
@@ -1326,18 +1345,17 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
             else k_gemv_x<WT, 8><<<grid, GX_WARPS * 32, 0, st>>>(a);
         };
         if (dtype == STACK_F32) go(0.f); else go(__nv_bfloat16());
-    } else if (T <= GEMV_MAX_T) {
+    } else if (route == LIN_ROWS_LONG) {
+        if (dtype == STACK_F32) k_gemv<float, 1, 8><<<(unsigned) N, 256, 0, st>>>(a); else k_gemv<__nv_bfloat16, 1, 8><<<(unsigned) N, 256, 0, st>>>(a);
+    } else if (route == LIN_ROWS) {
         if (a.glu) {
             const dim3 grid((unsigned) ((N / 2 + 7) / 8), 1, (unsigned) batch);
             if (dtype == STACK_F32) k_gemv<float, 2><<<grid, 256, 0, st>>>(a); else k_gemv<__nv_bfloat16, 2><<<grid, 256, 0, st>>>(a);
         } else {
             const dim3 grid((unsigned) ((N + 7) / 8), 1, (unsigned) batch);
-            if (batch == 1 && N <= GEMV_FEW_ROWS && K >= 1024) {       // few, long rows: a block each
-                if (dtype == STACK_F32) k_gemv<float, 1, 8><<<(unsigned) N, 256, 0, st>>>(a); else k_gemv<__nv_bfloat16, 1, 8><<<(unsigned) N, 256, 0, st>>>(a);
-            }
-            else if (dtype == STACK_F32) k_gemv<float, 1><<<grid, 256, 0, st>>>(a); else k_gemv<__nv_bfloat16, 1><<<grid, 256, 0, st>>>(a);
+            if (dtype == STACK_F32) k_gemv<float, 1><<<grid, 256, 0, st>>>(a); else k_gemv<__nv_bfloat16, 1><<<grid, 256, 0, st>>>(a);
         }
-    } else if (dtype == STACK_BF16 && a.vec && us && us->xb && umma_enabled() && T >= 64 && N >= 128 && K >= 64 && (size_t) xbatch * T * K <= us->elems) {
+    } else if (route == LIN_UMMA) {
         // tensor memory path: activations to bfloat16 once, then tcgen05.mma over TMA-fed stages (a.vec: rows and batch strides are multiples of 16 bytes)
         static const bool attr = [] { return cudaFuncSetAttribute(k_gemm_bf16_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM) == cudaSuccess; }();
         if (!attr) throw std::runtime_error("cannot reserve shared memory for k_gemm_bf16_umma");
@@ -1353,11 +1371,12 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
         }
         else k_gemm_bf16_umma<<<grid, 256, UM_SMEM, st>>>(mx, mw, a, us->err);
         if (launches) (*launches)++;
-    } else if (f32_parts > 1) {      // (a gated unit needs its sums whole: k_gemm_simt, 193 us against 236 in 128 x 128 tiles)
+    } else if (route == LIN_F32_PARTS) {      // (a gated unit needs its sums whole: k_gemm_simt, 193 us against 236 in 128 x 128 tiles)
+        const int f32_parts = f32_k_parts(T, N, K, us->sm_count);
         k_gemm_simt_big<<<dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((T + SG_BM - 1) / SG_BM), (unsigned) f32_parts), 256, 0, st>>>(a, f32_parts, us->part);
         k_split_sum<<<dim3((unsigned) ((N + 255) / 256), (unsigned) T), 256, 0, st>>>(us->part, f32_parts, T, N, bias, Y, ldy);
         if (launches) (*launches)++;
-    } else if (dtype == STACK_BF16 && a.vec && mma_enabled()) {
+    } else if (route == LIN_MMA) {
         const dim3 grid((unsigned) ((N + MM_BN - 1) / MM_BN), (unsigned) ((T + MM_BM - 1) / MM_BM), (unsigned) batch);
         k_gemm_bf16_mma<<<grid, 256, 0, st>>>(a);
     } else {
@@ -2789,6 +2808,10 @@ int32_t stack_argmax(StackCtx * c) {
     SCU(cudaMemcpyAsync(c->h_arg, c->d_arg, 4, cudaMemcpyDeviceToHost, c->st));
     SCU(cudaStreamSynchronize(c->st));
     return *c->h_arg;
+}
+
+int stack_product_kernel(int dtype, int T, int N, int K, bool glu, int sm_count) {
+    return lin_route(dtype, T, N, K, 1, K % (dtype == STACK_F32 ? 4 : 8) == 0, glu, false, 0, 0, true, sm_count);
 }
 
 float stack_time_linear(int device, int dtype, int T, int N, int K, int reps) {

@@ -63,3 +63,18 @@ def test_score_tile(kv, gqa, past, n, want):
 def test_prompt_product_kernel(types, rows, k, T, want):
     """which kernel a prompt product takes (2 tcgen05, 1 mma.sync, 3 Q8_0's mma.sync, 0 dp4a); an odd number of 32-row units goes to dp4a"""
     assert _lib.lib().b200_op_prompt_kernel((C.c_int32 * len(types))(*types), len(types), rows // 32, k, T, 148) == want
+
+
+BF16, F32 = 0, 1
+
+
+@pytest.mark.parametrize("dtype,T,N,K,glu,want", [
+    (BF16, 1, 16000, 2048, 0, 2), (BF16, 1, 2048, 8192, 0, 2), (BF16, 1, 16384, 2048, 1, 2), (F32, 1, 4096, 1024, 0, 2), (F32, 1, 16000, 4096, 1, 2),
+    (BF16, 1, 512, 2048, 0, 1), (BF16, 4, 16000, 2048, 0, 0), (BF16, 1, 2048, 2044, 0, 0),
+    (F32, 300, 1024, 4096, 0, 4), (F32, 600, 1024, 512, 0, 4), (F32, 64, 4096, 2048, 0, 4),
+    (F32, 600, 640, 512, 0, 6), (F32, 300, 4096, 512, 0, 6), (F32, 64, 16000, 512, 0, 6), (F32, 600, 4096, 4096, 0, 6), (F32, 300, 1024, 4096, 1, 6),
+    (BF16, 64, 128, 64, 0, 3), (BF16, 63, 128, 64, 0, 5), (BF16, 64, 128, 60, 0, 6)])
+def test_stack_product_kernel(dtype, T, N, K, glu, want):
+    """which kernel a layer stack's product takes: 0 a warp per row, 1 a block per row, 2 a block per eight rows with x in registers, 3 tcgen05, 4 float32
+    tiles in K parts, 5 mma.sync, 6 float32 tiles; the sizes on both sides of each line are among those measured"""
+    assert _lib.lib().b200_stack_product_kernel(dtype, T, N, K, glu, 148) == want
