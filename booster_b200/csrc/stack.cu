@@ -1259,7 +1259,7 @@ bool simt_big_enabled() {
     return on;
 }
 constexpr int GEMV_FEW_ROWS = 512;
-constexpr int GX_MIN_K = 1024;                // shorter rows leave most of a block's lanes without an entry: k_gemv, a warp per row
+constexpr int GX_MIN_K = 1024;
 // what the tcgen05 product needs beside its operands: room for the activations rounded to bfloat16 and the error flag its
 // bounded waits raise
 struct UmmaScratch { __nv_bfloat16 * xb = nullptr; size_t elems = 0; int * err = nullptr; float * part = nullptr; int sm_count = 148; };
@@ -1280,11 +1280,27 @@ int f32_k_parts(int T, int N, int K, int sm_count) {
     return cut < 0.97f * whole ? parts : 1;
 }
 
+// 16-byte chunks of a row that a lane of k_gemv_x takes: 1, 2 or 4 (0: the row is too long)
+int gx_chunks(int chunks) { return chunks <= GX_WARPS * 32 ? 1 : chunks <= 2 * GX_WARPS * 32 ? 2 : chunks <= 4 * GX_WARPS * 32 ? 4 : 0; }
+// one token: whether k_gemv_x is faster than k_gemv. A row has to fill most of a block's lanes (in sixteenths, by chunks per lane): 8192 x 1024 in bf16, half of them, takes 9.8 us
+// against 8.6, 2048 x 3072 (three quarters) 9.8 and 8.5, 2048 x 2048 6.2 and 6.2, 16000 x 2048 16.4 and 20.6. Of a gated unit, k_gemv's blocks hold sixteen rows and not eight, and waves decide: one
+// of its waves against two here loses (8192 x 4096 17.4 us with k_gemv, 18.9 here), two against two or three do not (10240 x 4096 0.77 of its time). With eight chunks a lane no row was
+// faster here (bf16 16000 x 16384: 179 us and 128). Measured: 514 to 28672 rows of 1024 to 16384 (float32: to 8192), cold.
+bool gx_pays(bool f32, int chunks, int N, int batch, bool glu, int sm_count) {
+    static const int plain[2][3] = {{12, 13, 13}, {12, 12, 15}}, resident[2][3] = {{8, 5, 4}, {7, 6, 5}};      // resident: blocks per SM, by their registers
+    const int ch = gx_chunks(chunks);
+    if (!ch) return false;
+    const int c = ch >> 1, full = ch * GX_WARPS * 32;
+    if (!glu) return 16 * chunks >= plain[f32][c] * full;
+    const auto waves = [&](int rows, int per_sm) { return ((long long) ((N + rows - 1) / rows) * batch + sm_count * per_sm - 1) / (sm_count * per_sm); };
+    const long long here = waves(GX_ROWS, resident[f32][c]), there = waves(16, 4);
+    return 2 * here <= 3 * there && 16 * chunks >= (here == 1 && ch > 1 ? 12 : 14) * full;
+}
 // the kernel a product goes to: mat-vecs of few tokens, then tile kernels
 enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG, LIN_ROWS_X, LIN_UMMA, LIN_F32_PARTS, LIN_MMA, LIN_SIMT };
 // vec: LinArgs::vec; x_elems: entries of X; xb_elems, part: what the scratch has room for
 LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu, bool seg, size_t x_elems, size_t xb_elems, bool part, int sm_count) {
-    if (T == 1 && vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && K / (dtype == STACK_F32 ? 4 : 8) <= 8 * GX_WARPS * 32) return LIN_ROWS_X;
+    if (T == 1 && vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && gx_pays(dtype == STACK_F32, K / (dtype == STACK_F32 ? 4 : 8), N, batch, glu, sm_count)) return LIN_ROWS_X;
     if (T <= GEMV_MAX_T) return !glu && batch == 1 && N <= GEMV_FEW_ROWS && K >= 1024 ? LIN_ROWS_LONG : LIN_ROWS;      // few, long rows: a block each
     if (dtype == STACK_BF16 && vec && umma_enabled() && T >= 64 && N >= 128 && K >= 64 && x_elems <= xb_elems) return LIN_UMMA;
     if (dtype == STACK_F32 && vec && batch == 1 && !glu && !seg && part && f32_k_parts(T, N, K, sm_count) > 1) return LIN_F32_PARTS;
@@ -1335,14 +1351,13 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
     if (launches) (*launches)++;
     const LinRoute route = lin_route(dtype, T, N, K, batch, a.vec != 0, a.glu != 0, a.seg != nullptr, (size_t) xbatch * T * K, us && us->xb ? us->elems : 0, us && us->part, us ? us->sm_count : 148);
     if (route == LIN_ROWS_X) {
-        const int gx_chunks = (K + GX_WARPS * 32 * vecw - 1) / (GX_WARPS * 32 * vecw);
+        const int ch = gx_chunks(K / vecw);
         const dim3 grid((unsigned) ((N + GX_ROWS - 1) / GX_ROWS), 1, (unsigned) batch);
         const auto go = [&](auto wt) {
             using WT = decltype(wt);
-            if (gx_chunks <= 1) k_gemv_x<WT, 1><<<grid, GX_WARPS * 32, 0, st>>>(a);
-            else if (gx_chunks <= 2) k_gemv_x<WT, 2><<<grid, GX_WARPS * 32, 0, st>>>(a);
-            else if (gx_chunks <= 4) k_gemv_x<WT, 4><<<grid, GX_WARPS * 32, 0, st>>>(a);
-            else k_gemv_x<WT, 8><<<grid, GX_WARPS * 32, 0, st>>>(a);
+            if (ch == 1) k_gemv_x<WT, 1><<<grid, GX_WARPS * 32, 0, st>>>(a);
+            else if (ch == 2) k_gemv_x<WT, 2><<<grid, GX_WARPS * 32, 0, st>>>(a);
+            else k_gemv_x<WT, 4><<<grid, GX_WARPS * 32, 0, st>>>(a);
         };
         if (dtype == STACK_F32) go(0.f); else go(__nv_bfloat16());
     } else if (route == LIN_ROWS_LONG) {

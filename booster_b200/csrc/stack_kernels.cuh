@@ -296,10 +296,10 @@ __global__ void __launch_bounds__(256) k_gemv(const LinArgs a) {
 }
 
 // one token against long rows: a block = GX_ROWS rows, its 8 warps cut K among them, and a lane keeps its entries of x in registers for all rows.
-// k_gemv reads 32 bytes of x for every 16 bytes of a row, which made the first-level cache its bound and left 2 KB of a row in flight per warp; here
-// nothing but weights is read in the loop, four rows at a time (2 KB CH per warp in flight). A warp's eight sums are folded by halving (9 shuffles), the
-// warps' parts added in order. CH: 16-byte chunks of a row per lane, K <= 8 x 32 x VEC x CH. Measured (bf16, cold rows): 16000 x 2048 21.8 us with
-// k_gemv, 15.2 here; 16384 x 2048 with the gated unit 17.6 and 15.8; 2048 x 2048 and 2048 x 8192 together 26.7 and 21.7.
+// k_gemv reads 32 bytes of x for every 16 bytes of a row, which makes the first-level cache its bound and leaves 2 KB of a row in flight per warp; here
+// nothing but weights is read in the loop, up to eight rows at a time. A warp's eight sums are folded by halving (9 shuffles), the
+// warps' parts added in order. CH: 16-byte chunks of a row per lane, K <= 8 x 32 x VEC x CH. bf16, cold rows: 16000 x 2048 20.6 us with
+// k_gemv, 16.4 here; 16384 x 2048 with the gated unit 18.4 and 16.5; 2048 x 8192 16.6 and 14.8. Where it does not pay: gx_pays.
 constexpr int GX_ROWS = 8, GX_WARPS = 8;
 template <typename WT, int CH>
 __global__ void __launch_bounds__(GX_WARPS * 32) k_gemv_x(const LinArgs a) {

@@ -70,6 +70,10 @@ BF16, F32 = 0, 1
 
 @pytest.mark.parametrize("dtype,T,N,K,glu,want", [
     (BF16, 1, 16000, 2048, 0, 2), (BF16, 1, 2048, 8192, 0, 2), (BF16, 1, 16384, 2048, 1, 2), (F32, 1, 4096, 1024, 0, 2), (F32, 1, 16000, 4096, 1, 2),
+    (BF16, 1, 2048, 1536, 0, 2), (BF16, 1, 2048, 1536, 1, 0), (BF16, 1, 2048, 3072, 1, 2), (BF16, 1, 2048, 3072, 0, 0),      # three quarters of a block's lanes
+    (BF16, 1, 5120, 4096, 1, 2), (BF16, 1, 8192, 4096, 1, 0), (BF16, 1, 10240, 4096, 1, 2), (F32, 1, 8192, 4096, 1, 0),     # a gated unit's waves
+    (BF16, 1, 2048, 1024, 0, 0), (BF16, 1, 8192, 3072, 1, 0), (F32, 1, 2048, 3072, 0, 0),          # lanes without entries: 1.2 times as long
+    (BF16, 1, 16000, 16384, 0, 0), (F32, 1, 16000, 8192, 0, 0),                  # eight chunks a lane: 1.4 and 1.2 times
     (BF16, 1, 512, 2048, 0, 1), (BF16, 4, 16000, 2048, 0, 0), (BF16, 1, 2048, 2044, 0, 0),
     (F32, 300, 1024, 4096, 0, 4), (F32, 600, 1024, 512, 0, 4), (F32, 64, 4096, 2048, 0, 4),
     (F32, 600, 640, 512, 0, 6), (F32, 300, 4096, 512, 0, 6), (F32, 64, 16000, 512, 0, 6), (F32, 600, 4096, 4096, 0, 6), (F32, 300, 1024, 4096, 1, 6),

@@ -427,9 +427,10 @@ def test_products_pick_their_kernel_and_agree_with_numpy(dtype, T, N, K, glu):
 @pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
 @pytest.mark.parametrize("T,N,K,glu", [
     (1, 513, 1024, False), (1, 1001, 2056, False), (1, 2048, 4096, True), (1, 600, 8192, False), (1, 530, 16384, False), (1, 514, 1032, True), (1, 512, 1024, False),
+    (1, 1001, 2040, False), (1, 1001, 4088, False), (1, 530, 8184, False), (1, 514, 2040, True), (1, 518, 4088, True), (1, 1030, 8192, True),
     (64, 128, 64, False), (65, 257, 72, False), (130, 300, 4096, False), (200, 2056, 1000, False), (129, 514, 264, True), (300, 130, 2064, False)])
 def test_products_where_their_rules_change(dtype, T, N, K, glu):
-    """one token: eight rows a block and each number of chunks per lane, rows and K that end inside a block; portions: TMA tiles that end inside T, N and K,
+    """one token: eight rows a block and each number of chunks per lane, rows and K that end inside a block or fill too little of one; portions: TMA tiles that end inside T, N and K,
     and float32 products in K parts. Bound: a sum of K float32 products in any order is off by at most (K + 8) 2^-24 sum |x w|."""
     rng = np.random.default_rng(T * 7 + N + K)
     x = rng.standard_normal((T, K)).astype(np.float32)
