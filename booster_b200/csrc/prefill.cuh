@@ -135,7 +135,8 @@ __global__ void __launch_bounds__(256) k_attn_softmax_rows(const AttnArgs a, int
 // sums of 16 meet in shared memory and one warp adds them in k_attn_softmax_rows' order, bit for bit. A warp per row reads a long row three times
 // and writes it twice, mostly past the L1: 288 tokens x 32 heads x 6288 keys 119 us against 225.
 static constexpr int SMX_THREADS = 256, SMX_MAX_G = 4;        // rows of up to 256 * 16 * 4 = 16384 scores
-static constexpr int SMX_MIN_ROW = 2048;                      // (shorter rows: most of a block would idle)
+static constexpr int SMX_MIN_ROW = 2048;                      // shorter rows leave most of a block idle: 256 tokens x 32 heads, two layers, rows of 1256 985 us with a warp each
+                                                              // and 993 here, of 2056 1258 and 1236, of 8256 3514 and 3418
 template <int G>
 __global__ void __launch_bounds__(SMX_THREADS) k_attn_softmax_block(const AttnArgs a, int nz) {
     __shared__ float wmax[SMX_THREADS / 32], gsum[G * SMX_THREADS];
@@ -213,7 +214,8 @@ __global__ void __launch_bounds__(SMX_THREADS) k_attn_softmax_block(const AttnAr
 }
 
 // packed fp32 pairs: each half is the IEEE operation of the scalar instruction (a packed multiply whose only use is a packed add is
-// contracted by the compiler: products that are added are not formed with these)
+// contracted by the compiler: products that are added are not formed with these). In place of float2 and its intrinsics, with which k_attn_pv_batch needs more
+// than its 128 registers (8 bytes spilled; 120 registers here).
 __device__ __forceinline__ uint64_t pair_of(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
 __device__ __forceinline__ float2 unpair(uint64_t p) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p)); return r; }
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
@@ -285,8 +287,7 @@ __global__ void __launch_bounds__(SCB_KEYS, 3) k_attn_scores_batch(const AttnArg
 
 // P.V of a prompt batch: CTA = (KV head, 8 (token, head) rows), all 128 dims, two CTAs per SM. A half-warp is one of tinyBLAS' 16 chains (positions
 // c, c + 16, ...), a lane 8 rows x 8 dims: 32 packed fmas per position on one 16-byte load of V (f16, converted in registers) and two of p.
-// Bound by the fp32 pipe, with the loads close behind. What was tried on the way (512 tokens x 32 heads x 6256 keys): a thread = chain x dim, 32 rows, a load
-// of p per fma 1.90 ms; lane = 4 rows x 16 dims on V staged as fp32 1.06 ms (shared-memory pipe 79 %), now 0.88 ms.
+// Bound by the fp32 pipe, with the loads close behind. 512 tokens x 32 heads x 6256 keys: 0.88 ms (1.90 with a thread per chain and dim, a load of p per fma).
 static constexpr int PVB_CHUNK = 64;           // positions staged at a time
 static constexpr int PVB_STAGES = 3;
 static constexpr int PVB_THREADS = 256;
