@@ -1,9 +1,8 @@
 #!/usr/bin/env python
-"""bench.py — BASELINE.json's metric on BASELINE.json's configs.
+"""bench.py — decode tokens/s of the reference's own models.
 
 metric : decode tokens/sec, single stream. `--config` picks the workload; the default is the configuration the metric is
-         quoted on (configs[1]: LLaMA-3-8B Q4_K_M, ctx 2048, 1 x B200). The others are the remaining GPU configs of
-         BASELINE.json (configs[2..4]); configs[0] is the reference's own CPU case and is what `--impl reference` runs.
+         quoted on (LLaMA-3-8B Q4_K_M, ctx 2048, 1 x B200). `--impl reference` runs the reference's own CPU case (the same file, ctx 512).
 
            8b-q4km-2048        LLaMA-3-8B Q4_K_M, single-stream decode at the end of ctx 2048            (default)
            8b-q8_0-prefill512  LLaMA-3-8B Q8_0: one 512-token prompt batch, then 1024 generated tokens
@@ -26,11 +25,11 @@ roofline: dominant kernel = the ffn gate|up mat-vec (47 % of the bytes of an 8B 
          bytes of one launch / its mean device time, measured live with a CUDA-event pair around every launch of an
          un-graphed token (b200_profile_token); peak = MEASURED_PEAKS.json hbm_gbs.
 cpu_baseline / --impl reference: the reference's own CPU llama_decode (oracle/_ref, unmodified sources) on the
-         host cores, same 8B GGUF, on a bounded sample (BASELINE.json configs[0]: ctx 512).
+         host cores, same 8B GGUF, on a bounded sample (ctx 512).
 
 N > 1 (torchrun, one rank per GPU): layers are split across ranks (stage r = layers [r*L/N, (r+1)*L/N)); one hand-off
 of the residual stream per boundary per token plus the 4-byte token hand-back; single stream, so stages run one after
-the other — value is NOT expected to rise with N (SURVEY.md §8e), "scaling": "strong".
+the other — value is NOT expected to rise with N, "scaling": "strong".
 """
 import argparse
 import ctypes as C
@@ -117,14 +116,14 @@ class ClockSampler:
 
 def cpu_reference_run(path, steps, warmup, sample_tokens=None, n_prompt=64):
     """the reference's own CPU llama_decode on the host cores; returns (tokens/s, info). A step is `sample_tokens` greedy
-    decode tokens (default: up to 32, capped so that the whole run stays inside ctx 512 — BASELINE.md §2: 64-token prompt,
+    decode tokens (default: up to 32, capped so that the whole run stays inside ctx 512: 64-token prompt,
     then >= 128 decode steps when the step count allows)"""
     if sample_tokens is None:
         sample_tokens = max(1, min(32, 400 // max(1, steps)))
     from oracle import ref
     cores = os.cpu_count() or 1
     best = None
-    # "threads = host cores" (BASELINE.json configs[0]); OpenMP barriers can make fewer threads faster on big hosts,
+    # "threads = host cores"; OpenMP barriers can make fewer threads faster on big hosts,
     # so give the reference its best of {cores, cores/2 (physical), 32} — all the host threads it can use well
     cands = sorted({cores, max(1, cores // 2), min(cores, 32)}, reverse=True)
     prompt = np.random.default_rng(42).integers(0, G.CONFIGS[CFG_NAME].n_vocab, size=n_prompt).tolist()
@@ -169,7 +168,7 @@ def bridge_e2e(path, ctx, n_prompt, n_gen, reps):
     """decode tokens/s through the nine bridge symbols: doInference on a host text prompt of token ids, generated tokens
     counted by a status() poller (the Go server's streaming loop, pkg/server/server.go:842-863); the timed region runs
     from the first generated token's appearance to the last one's. Sampler arguments: Janus at scale = hi = lo = 1.0,
-    i.e. the reference's deterministic setting (SURVEY.md §8c)."""
+    i.e. the reference's deterministic setting."""
     from booster_b200 import _lib
     L = _lib.lib()
     L.init(b"", b"")
@@ -489,13 +488,13 @@ def main():
     if args.impl == "reference":
         if rank != 0:
             return 0
-        # the reference's CPU path on BASELINE.json configs[0]: the 8B Q4_K_M file, ctx 512 — the config says what ran
+        # the reference's CPU path: the 8B Q4_K_M file, ctx 512 — the config says what ran
         path = model_path()
         tps, info = cpu_reference_run(path, args.steps, args.warmup)
         c8 = G.CONFIGS[CFG_NAME]
         config = {"workload": f"LLaMA-3-8B-shaped synthetic GGUF, {FTYPE}, single-stream greedy decode on the host CPU, ctx=512, "
                               f"{info['tokens_per_step']} tokens per step at n_kv {info['n_kv_first']}..{info['n_kv_last']}, threads={info['cores']} "
-                              f"(BASELINE.json configs[0]; the GPU arm's ctx-2048 positions would take the CPU minutes per step)",
+                              f"(the GPU arm's ctx-2048 positions would take the CPU minutes per step)",
                   "n_layer": c8.n_layer, "n_embd": c8.n_embd, "n_vocab": c8.n_vocab, "ctx": 512, "burst": info["tokens_per_step"],
                   "parallelism": f"{info['cores']} host threads (OpenMP)", "l2": "n/a (CPU)"}
         line = {"impl": "reference", "metric": "decode tokens/sec", "value": tps, "unit": "tokens/s", "n_gpus": args.gpus,
@@ -717,7 +716,7 @@ def main():
                                         "frac": gu_bytes / (iso_ms * 1e-3) / 1e9 / peak,
                                         "what": "gate|up launches of every layer back to back (distinct weights per launch, PDL), one CUDA-event pair"}
         line["kernel_ms_per_token"] = {k: round(v[0] / reps, 4) for k, v in acc.items()}
-        # ---- the reference's CPU llama_decode on this host, bounded sample (always BASELINE.json configs[0]: 8B Q4_K_M)
+        # ---- the reference's CPU llama_decode on this host, bounded sample (always the 8B Q4_K_M file)
         try:
             if args.no_cpu:
                 raise RuntimeError("skipped (--no-cpu)")

@@ -1,20 +1,20 @@
 // bridge.cpp — the nine cgo entry points of include/bridge.h on top of the B200 engine.
 //
 // Host-side mirror of cpp/bridge.cpp's operator interface for the hot path: same symbols, same argument
-// meaning, same return codes (SURVEY.md §8b). The generation loop follows the reference's control flow
+// meaning, same return codes. The generation loop follows the reference's control flow
 // (cpp/bridge.cpp:175-658: tokenize -> reject if > n_ctx-4 -> clear KV -> prompt in n_batch chunks ->
 // sample/decode one token at a time until EOG / n_predict / n_ctx-4 / stop flag -> per-token timings), but every
-// llama_decode is the CUDA engine. Differences, all documented in DESIGN.md / INTEGRATION.md:
+// llama_decode is the CUDA engine. Differences:
 //   * sampler: the reference's Janus sampler restated on the host (janus.hpp; logits come back once per token), or — with
 //     janus = 0, a setting the reference ignores — the standard chain; temperature <= 0 / top_k = 1 there is greedy
 //     arg-max on the device;
 //   * tokenizer: models with tokenizer.ggml.model == "no_vocab" take prompts that are white-space separated
-//     token ids and render pieces as "<id> "; text tokenizers (BPE/SPM) are row f-1, see tokenizer.hpp;
+//     token ids and render pieces as "<id> "; text tokenizers (BPE/SPM): tokenizer.hpp;
 //   * context shift (cpp/bridge.cpp:487-507): same branch, same unreachability (the loop ends at n_ctx - 4 first); the KV
 //     operations behind it are b200_kv_seq_rm / b200_kv_seq_add (engine.cu), bit-exact against the reference. Self-Extend
 //     (ga_n > 1, :509-524) cannot be switched on through initContext in the reference either and is not built;
 //   * status() returns a per-thread snapshot instead of a pointer into a string another thread appends to
-//     (the reference race).
+//     (a race in the reference).
 #include "../../include/bridge.h"
 #include "../../include/booster_b200.h"
 #include "tokenizer.hpp"

@@ -655,7 +655,7 @@ extern "C" int b200_n_ctx(const b200_ctx * c) { return c ? c->n_ctx : 0; }
 extern "C" int64_t b200_kernel_launches(const b200_ctx * c) { return !c ? 0 : c->stack ? b200::stack_ctx_launches(c->stack) : c->launches; }
 
 enum { KIND_EMBED = 0, KIND_QKV, KIND_ATTN, KIND_WO, KIND_GATEUP, KIND_DOWN, KIND_HEAD, KIND_ATTN_PV, KIND_COUNT };
-// (thread_local: up to 8 pods run doInference concurrently, each on its own OS thread — SURVEY §8b threading)
+// (thread_local: up to 8 pods run doInference concurrently, each on its own OS thread)
 static thread_local int g_kind = KIND_EMBED;   // set by enqueue_forward before each launch group
 static thread_local int g_only_kind = -1;       // b200_profile_kind: enqueue_forward launches only this kind (-1: everything)
 // function attributes (dynamic shared-memory opt-in) are raised lazily, per device, from whichever pod's thread gets
@@ -1022,7 +1022,7 @@ static void token_kernel_prepare(b200_ctx * c, size_t smem) {
 }
 // Which path decodes a token: 0 = one kernel per operator joined by programmatic dependent launch (default: measured
 // faster, 546 vs 371 tok/s on the 8B Q4_K_M config — the grid barrier costs 3 us against ~2 us for a PDL kernel boundary
-// and does not overlap the way the next kernel's early CTAs do; DESIGN.md §4), 1 = the persistent per-token kernel.
+// and does not overlap the way the next kernel's early CTAs do), 1 = the persistent per-token kernel.
 // BOOSTER_B200_TOKEN_KERNEL=1 or b200_set_token_kernel(1) selects it for contexts created afterwards.
 static int g_token_kernel = -1;
 extern "C" void b200_set_token_kernel(int on) { g_token_kernel = on ? 1 : 0; }
@@ -2678,7 +2678,7 @@ extern "C" int b200_stage_argmax(b200_ctx * c, int32_t * token_out) {
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// tokenizer entry points (host side, SURVEY.md §8 f-1): llama_tokenize / llama_token_to_piece / llama_token_is_eog
+// tokenizer entry points (host side): llama_tokenize / llama_token_to_piece / llama_token_is_eog
 // ------------------------------------------------------------------------------------------------------------
 struct b200_tokenizer { std::unique_ptr<b200::Tokenizer> t; };
 extern "C" b200_tokenizer * b200_tokenizer_load(const char * gguf_path) {

@@ -1,4 +1,4 @@
-// janus.hpp — host-side samplers behind doInference (SURVEY.md §8 row f-2).
+// janus.hpp — host-side samplers behind doInference.
 //
 // The reference's bridge samples EVERY token with its "Janus" sampler (cpp/bridge.cpp:586-596; the standard sampling
 // chain is commented out there): per-token repetition scales derived from the token TEXT (cpp/janus.cpp initJanus

@@ -1,5 +1,5 @@
 // prefill_mma.cuh — prompt batches of K-quant matrices (Q4_K / Q5_K / Q6_K x Q8_K) on the tensor cores, BIT-EXACT with the
-// reference's CPU arithmetic (SURVEY.md §8 row N-1; the counterpart of ggml-cuda's mul_mat_q, cpp/ggml/src/ggml-cuda/mmq.cuh).
+// reference's CPU arithmetic (the counterpart of ggml-cuda's mul_mat_q, cpp/ggml/src/ggml-cuda/mmq.cuh).
 //
 // What has to be reproduced (cpp/ggml/src/ggml-quants.c:6914-6977, 7487-7560, 8145-8220): per output element (row, token) and
 // per 256-weight super-block b, the AVX2 code forms EIGHT 32-bit integers — lane m sums scale[g] * w * a over bytes 4m..4m+3 of

@@ -1,4 +1,4 @@
-// tokenizer.hpp — host-side text <-> token-id interface used by bridge.cpp (SURVEY.md §8 row f-1).
+// tokenizer.hpp — host-side text <-> token-id interface used by bridge.cpp.
 // Replaces the reference's llama_tokenize / llama_token_to_piece / llama_token_is_eog calls
 // (cpp/bridge.cpp:275-278, 630, 640; implementation cpp/src/llama-vocab.cpp, cpp/src/unicode.cpp; vocabulary
 // loading cpp/src/llama.cpp:5250-5760).

@@ -1,7 +1,7 @@
 """Minimal GGUF v3 writer/reader (numpy) and synthetic LLaMA-shaped model generator.
 
-No model file exists offline, so tests and bench fabricate GGUFs with the exact
-hyper-parameters of the BASELINE.json configs. Two sources of weights:
+No model file exists offline, so tests and bench fabricate GGUFs with the exact hyper-parameters of
+LLaMA-3-8B, LLaMA-3-70B and Mistral-7B. Two sources of weights:
 
 * ``synth_llama(..., source="blocks")`` writes random *quantized blocks* directly (valid fp16 scales,
   random packed quants) following the reference's tensor-type mixture for the file type
@@ -195,7 +195,7 @@ class LlamaConfig:
 
 
 CONFIGS = {
-    # BASELINE.json configs (SURVEY.md §8 model constants)
+    # the models that bench.py measures
     "llama3-8b": LlamaConfig(),
     "mistral-7b": LlamaConfig(n_vocab=32000, rope_freq_base=10000.0, n_ctx_train=32768, name="synthetic-mistral-7b"),
     "llama3-70b": LlamaConfig(n_layer=80, n_embd=8192, n_head=64, n_head_kv=8, n_ff=28672, name="synthetic-llama3-70b"),
@@ -330,7 +330,7 @@ def synth_llama(path: str, cfg: LlamaConfig, ftype: str = "Q4_K_M", seed: int = 
 
 
 def weight_bytes_per_token(cfg: LlamaConfig, ftype: str) -> int:
-    """Algorithmic weight bytes one decoded token reads (SURVEY.md §8d): all per-layer matrices + output +
+    """Algorithmic weight bytes one decoded token reads: all per-layer matrices + output +
     norm vectors; token_embd excluded (one row)."""
     types = tensor_types(cfg, ftype)
     E, KV, FF, V = cfg.n_embd, cfg.n_head_kv * cfg.head_dim, cfg.n_ff, cfg.n_vocab

@@ -3,7 +3,7 @@
  * include/bridge.h is the boundary Booster's Go server binds. The entry points below sit one seam
  * lower — the llama.h calls cpp/bridge.cpp makes on the hot path — so that the CUDA path can be
  * parity-tested against the reference's CPU path on token ids and logits, without tokenizer or
- * sampler in between (SURVEY.md §8b "inner seams"). Every function cites the reference interface it
+ * sampler in between (its inner seams). Every function cites the reference interface it
  * replaces. Plain C, host pointers and sizes only; all device memory is owned by the library.
  *
  * Error convention: functions returning int return 0 on success, non-zero on failure;
@@ -62,7 +62,7 @@ enum { B200_INFO_N_VOCAB = 0, B200_INFO_N_EMBD, B200_INFO_N_LAYER, B200_INFO_N_H
        B200_INFO_FTYPE, B200_INFO_COUNT = 16 };
 int     b200_model_info(const b200_model * m, int32_t info[B200_INFO_COUNT]);
 /* algorithmic HBM bytes one decoded token reads from this stage's matrices + norm vectors
- * (token_embd excluded: one row) — SURVEY.md §8(d) / BASELINE.md §3 */
+ * (token_embd excluded: one row) */
 int64_t b200_model_weight_bytes(const b200_model * m);
 
 b200_ctx * b200_ctx_new(b200_model * m, int n_ctx);
@@ -76,7 +76,7 @@ void       b200_kv_clear(b200_ctx * c);               /* llama_kv_cache_clear (c
 int b200_kv_write(b200_ctx * c, int layer, int pos0, int n, const uint16_t * k_rows, const uint16_t * v_rows);
 int b200_kv_read(b200_ctx * c, int layer, int pos0, int n, uint16_t * k_rows, uint16_t * v_rows);
 
-/* Context shift (SURVEY.md §8 f-3): llama_kv_cache_seq_rm(ctx, 0, p0, p1) and llama_kv_cache_seq_add(ctx, 0, p0, p1, delta)
+/* Context shift: llama_kv_cache_seq_rm(ctx, 0, p0, p1) and llama_kv_cache_seq_add(ctx, 0, p0, p1, delta)
  * (cpp/bridge.cpp:500-501; cpp/src/llama.cpp:3154-3206, 3268-3314). Cells keep their places, freed cells are re-used by the
  * next tokens (llama_kv_cache_find_slot, :3028-3125), attention masks by the cells' positions, and the cached K rows of the
  * moved cells are re-rotated by the accumulated delta at the next decode (build_k_shift, :8482-8510) — the same cell order
@@ -165,7 +165,7 @@ void b200_set_prefill_mma(int mode);
 void b200_set_prefill_attn_batch(int on);
 /* Decode path of contexts created AFTER the call: 0 (default) = one kernel per operator joined by programmatic dependent
  * launch, 1 = ONE persistent kernel per token (token_kernel.cuh: phase list + grid barriers; same arithmetic, bit-identical
- * results; measured slower on B200, kept selectable: DESIGN.md §4). Env BOOSTER_B200_TOKEN_KERNEL=1 sets the initial value. */
+ * results; measured slower on B200, kept selectable). Env BOOSTER_B200_TOKEN_KERNEL=1 sets the initial value. */
 void b200_set_token_kernel(int on);
 /* one token through the persistent per-token kernel with %globaltimer stamps (ns) at its phase boundaries:
  * out = [n_phases][n_ctas][4]: 0 the phase's dependent half starts | 1 it is done | 2 arrived at the grid barrier, next
@@ -179,7 +179,7 @@ int64_t b200_trace_phases(b200_ctx * c, int32_t token, int pos, int reps, uint64
  * whose integer-millisecond values read 0 on a B200) */
 int b200_job_timing_us(const char * jobID, double * prompt_us_per_token, double * gen_us_per_token);
 
-/* ---- layer-split pipeline over NCCL (SURVEY.md §8e; replaces ggml_backend_cuda_cpy_tensor_async,
+/* ---- layer-split pipeline over NCCL (replaces ggml_backend_cuda_cpy_tensor_async,
  * cpp/ggml/src/ggml-cuda.cu:2386-2407, invoked from cpp/ggml/src/ggml-backend.c:1782) ---------------------
  * One process per GPU. Rank r owns the stage its model was loaded with. Per token each boundary moves the
  * residual stream f32[n_embd] with ONE ncclSend/ncclRecv; the last stage returns the argmax token to
@@ -231,14 +231,14 @@ float * b200_stage_logits_view(b200_ctx * c);
 float * b200_decode_view(b200_ctx * c, int32_t token, int pos);
 
 /* launch shape (warps per CTA, warps sharing a 32-row unit, ring stages per warp) the engine picks for a mat-vec whose
- * segments have the given block types: pure host arithmetic, exposed so that tests pin the shapes (DESIGN.md §4) */
+ * segments have the given block types: pure host arithmetic, exposed so that tests pin the shapes */
 int b200_op_launch_shape(const int32_t * types, int n_types, int64_t n_units, int64_t k, int norm, int sm_count, int32_t wgs[3]);
 /* tokens per block of a prompt batch's score kernel: n tokens behind `past` cells (host arithmetic, as above) */
 int b200_op_score_tokens(int n_head_kv, int gqa, int past, int n, int sm_count);
 /* kernel of one prompt product of T tokens: 2 = tcgen05, 1 = mma.sync, 3 = Q8_0's mma.sync, 0 = dp4a, -1 = bad arguments (host arithmetic, as above) */
 int b200_op_prompt_kernel(const int32_t * types, int n_types, int64_t n_units, int64_t k, int T, int sm_count);
 
-/* ---- tokenizer (host side; SURVEY.md §8 f-1) ----------------------------------------------------------------------
+/* ---- tokenizer (host side) ----------------------------------------------------------------------
  * The vocabulary of a GGUF (tokenizer.ggml.model = "llama" (SPM), "gpt2" (byte-level BPE, LLaMA-3 pre-tokenizer) or
  * "no_vocab" (prompts are decimal ids)), loaded without the weights.
  * b200_tokenize        == llama_tokenize(model, text, text_len, tokens, n_max, add_special, parse_special)
@@ -260,7 +260,7 @@ int32_t b200_tokenize(const b200_tokenizer * t, const char * text, int32_t text_
 int32_t b200_token_to_piece(const b200_tokenizer * t, int32_t token, char * buf, int32_t length, int special);
 int     b200_token_is_eog(const b200_tokenizer * t, int32_t token);
 int32_t b200_token_nl(const b200_tokenizer * t);
-/* ---- samplers (host side; SURVEY.md §8 f-2) ----------------------------------------------------------------------------
+/* ---- samplers (host side) ----------------------------------------------------------------------------
  * What doInference does with the logits of every token, exposed on its own so that it can be pinned against the reference's
  * sampler on the reference's logits (no GPU involved): janus != 0 -> sample_janus_token (cpp/janus.cpp:191-331) with the
  * tables of initJanus (:405-700) built from the GGUF's vocabulary; janus == 0 -> llama_sampling_sample's default chain

@@ -1,8 +1,8 @@
 /* oracle/oracle_port.c — TEST INFRASTRUCTURE, NOT PRODUCT ("port" oracle).
  *
  * A plain-C restatement of the reference's CPU arithmetic for the quantized LLaMA decode path, written
- * from the reference sources under /root/reference/cpp (every function cites the file:line it follows).
- * It exists so that parity can be checked where /root/reference is absent (the GPU box) and so that the
+ * from the reference sources (cpp/; every function cites the file:line it follows).
+ * It exists so that parity can be checked where the reference is absent and so that the
  * algorithm is stated once in readable scalar code. It is PINNED against the real reference: tests/ compare
  * it with oracle/_ref (the unmodified reference compiled by oracle/Makefile) and with the golden vectors under
  * tests/golden/ that oracle/_ref generated (tests/golden/make_golden.py).

@@ -1,11 +1,11 @@
 """oracle/ref.py — TEST INFRASTRUCTURE, NOT PRODUCT.
 
 ctypes driver for oracle/_ref/libbooster_cpu_ref_<variant>.so: the UNMODIFIED reference CPU path
-(cpp/ggml + cpp/src/llama.cpp + cpp/bridge.cpp, built by oracle/Makefile from /root/reference where it lies)
+(cpp/ggml + cpp/src/llama.cpp + cpp/bridge.cpp, built by oracle/Makefile from the reference where it lies)
 plus the thin veneer oracle/ref_shim.cpp. Only tests/, __graft_entry__.smoke() and bench.py's CPU legs may
 import this module; the product (booster_b200/) never does.
 
-Variant choice: "native" was compiled with -march=native in the build container (Sapphire Rapids: AVX-512,
+Variant choice: "native" was compiled with -march=native where it was built (Sapphire Rapids: AVX-512,
 AMX, AVX512-FP16), as Booster's own CPU build would be (booster_cpu.go:4); "v3" is an x86-64-v3 build.
 If the host CPU lacks a flag the native build needs we fall back to v3 (the K-quant dot products are AVX2
 in both; only ggml.c's f32 vector width and tinyBLAS tile width differ).

@@ -1,7 +1,6 @@
-"""Generate the golden fixtures under tests/golden/ from the UNMODIFIED reference (oracle/_ref, built from
-/root/reference by oracle/Makefile). Run in the build container (needs oracle/_ref); the outputs are committed
-so that the GPU box — where /root/reference does not exist — can check both the port oracle and the CUDA path
-against vectors the reference itself produced.
+"""Generate the golden fixtures under tests/golden/ from the UNMODIFIED reference (oracle/_ref, built
+by oracle/Makefile). Needs oracle/_ref; the outputs are committed so that a machine without the reference can check
+both the port oracle and the CUDA path against vectors the reference itself produced.
 
     python tests/golden/make_golden.py
 
@@ -190,7 +189,7 @@ def make_standard():
 
 if __name__ == "__main__":
     if not ref.available():
-        sys.exit("oracle/_ref is not built: run `make -C oracle ref` in the build container")
+        sys.exit("oracle/_ref is not built: run `make -C oracle ref`")
     print("reference variant:", ref.variant())
     only = sys.argv[1:]            # e.g. `make_golden.py tiny-gqa4-yarn`: (re)generate only the named models
     if only == ["janus"]:

@@ -1,4 +1,4 @@
-"""Regenerate the tokenizer golden fixtures from the REAL reference tokenizer (oracle/_ref, built from /root/reference):
+"""Regenerate the tokenizer golden fixtures from the REAL reference tokenizer (oracle/_ref):
     python tests/golden/make_tokenizer_golden.py
 writes tests/golden/vocab_{spm,bpe}.gguf (vocab-only synthetic GGUFs, tests/tokenizer_fixtures.py) and
 tests/golden/tokenizer_{spm,bpe}.json = for every test string the reference's llama_tokenize output for

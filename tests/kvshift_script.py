@@ -1,4 +1,4 @@
-"""The context-shift scenario of SURVEY §8 f-3, written once and run against any runner with the llama.h-shaped interface
+"""The context-shift scenario, written once and run against any runner with the llama.h-shaped interface
 (kv_clear / decode(tokens, pos0) -> logits / kv_seq_rm / kv_seq_add): the reference (oracle/ref.py RefModel, which makes
 tests/golden/kvshift_*.npz) and the CUDA engine (booster_b200.engine.Context).
 

@@ -81,7 +81,7 @@ def test_bad_model_path_returns_null():
 
 @pytest.mark.parametrize("kind", ["spm", "bpe"])
 def test_do_inference_with_text_prompt(kind, tmp_path):
-    """text in, text out through the nine symbols with a real vocabulary (SURVEY §8 f-1): the prompt is tokenized as
+    """text in, text out through the nine symbols with a real vocabulary: the prompt is tokenized as
     llama_tokenize(model, prompt, add_special=false, parse_special=true) (cpp/bridge.cpp:275-278), status() is the
     concatenation of llama_token_to_piece of prompt and generated tokens (cpp/bridge.cpp:628-632), generation stops at
     an end-of-generation token (cpp/bridge.cpp:640)."""
@@ -120,7 +120,7 @@ def test_do_inference_with_text_prompt(kind, tmp_path):
 
 
 def test_two_pods_concurrently_equal_sequential(golden_dir):
-    """the Go server runs one doInference per pod, up to 8 pods at once, each on its own OS thread (SURVEY §8b):
+    """the Go server runs one doInference per pod, up to 8 pods at once, each on its own OS thread:
     two pods decoding at the same time on one GPU give exactly what each gives alone"""
     path = os.path.join(golden_dir, "tiny_Q4_K_M.gguf")
     g = np.load(os.path.join(golden_dir, "tiny_Q4_K_M.npz"))
@@ -150,7 +150,7 @@ def test_two_pods_concurrently_equal_sequential(golden_dir):
 
 @pytest.mark.parametrize("kind", ["spm", "bpe"])
 def test_do_inference_janus_sampler_equals_reference_golden(kind, tmp_path, golden_dir):
-    """SURVEY §8 f-2 through the nine symbols: with the seed fixed, doInference generates the token ids the reference's own
+    """the samplers through the nine symbols: with the seed fixed, doInference generates the token ids the reference's own
     bridge loop generates with its Janus sampler (tests/golden/janus.json, made by the unmodified cpp/janus.cpp) — logits
     bit-identical, sampler arithmetic identical, same std::mt19937 draws. Three settings: the reference's deterministic one,
     its defaults, and a wide short list (real random draws)."""

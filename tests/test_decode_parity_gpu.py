@@ -3,11 +3,11 @@
   * the port oracle (itself bit-identical to the reference) on seeded random-block twins with the real 8B / 70B
     per-layer shapes,
   * the reference itself (oracle/_ref, AVX-512 build) when it loads on this host,
-plus size-independent properties at BASELINE.json's full sizes (determinism, graph == un-graphed, device-greedy
+plus size-independent properties at the models' full sizes (determinism, graph == un-graphed, device-greedy
 == host-greedy, stage split == single stage).
 
 Bitwise equality is the only meaningful criterion here: activations are re-quantized to int8 before every
-mat-mul, so any 1-ulp deviation eventually flips a quant and cascades to ~1e-2 (DESIGN.md "why bit-exact").
+mat-mul, so any 1-ulp deviation eventually flips a quant and cascades to ~1e-2.
 It also makes greedy decoding token-id-exact by construction."""
 import os
 
@@ -118,13 +118,13 @@ def test_long_context_bitwise(model_dir):
 
 
 @pytest.mark.parametrize("cfg,ftype,n_ctx,n_kv0", [
-    ("llama3-8b-2l", "Q4_K_M", 2048, 2040),      # BASELINE config 2: 8B shapes at the end of ctx 2048
-    ("llama3-8b-2l", "Q5_K_M", 8192, 8186),      # config 4: Mistral-7B shapes (same as 8B, GQA 4), Q5_K_M, ctx 8192
-    ("llama3-8b-2l", "Q8_0", 1536, 1530),        # config 3: Q8_0 after 512 prefill + 1K generated
-    ("llama3-70b-1l", "Q4_K_M", 4096, 4090),     # config 5: 70B shapes (GQA 8), ctx 4096
+    ("llama3-8b-2l", "Q4_K_M", 2048, 2040),      # 8B shapes at the end of ctx 2048
+    ("llama3-8b-2l", "Q5_K_M", 8192, 8186),      # Mistral-7B shapes (same as 8B, GQA 4), Q5_K_M, ctx 8192
+    ("llama3-8b-2l", "Q8_0", 1536, 1530),        # Q8_0 after 512 prefill + 1K generated
+    ("llama3-70b-1l", "Q4_K_M", 4096, 4090),     # 70B shapes (GQA 8), ctx 4096
 ])
 def test_fullshape_decode_at_full_context_vs_port_bitwise(model_dir, cfg, ftype, n_ctx, n_kv0):
-    """the real per-layer shapes decoding at the END of each BASELINE config's context. Both sides start from the same
+    """the real per-layer shapes decoding at the END of each model's context. Both sides start from the same
     KV cache (N(0,1) f16 rows for positions < n_kv0, injected through b200_kv_write / the port's cache arrays — a
     prefill of thousands of tokens through the scalar port would take minutes) and then decode real tokens: the new
     K/V rows, the attention over all n_kv0+ positions and the logits must be bit-identical, and stay so token after token."""
@@ -153,7 +153,7 @@ def test_fullshape_decode_at_full_context_vs_port_bitwise(model_dir, cfg, ftype,
 
 @pytest.mark.parametrize("model", ["tiny-gqa4_Q4_K_M", "tiny-gqa4-yarn_Q4_K_M"])
 def test_context_shift_bitwise_golden(golden_dir, model):
-    """SURVEY §8 f-3: llama_kv_cache_seq_rm + seq_add (cpp/bridge.cpp:487-507), the K-shift re-rotation of the cached K rows
+    """llama_kv_cache_seq_rm + seq_add (cpp/bridge.cpp:487-507), the K-shift re-rotation of the cached K rows
     (build_k_shift, cpp/src/llama.cpp:8482-8510) and the reference's cell bookkeeping (find_slot re-uses the freed cells in the
     middle of the cache) — every logit of the scenario in tests/kvshift_script.py equals the reference's, bit for bit.
     The YaRN model scales cos/sin by the attention factor, so its K-shift touches every cell (as the reference's does)."""
@@ -175,7 +175,7 @@ def test_context_shift_bitwise_golden(golden_dir, model):
 
 @pytest.mark.parametrize("model", ["tiny-gqa4_Q4_K_M", "tiny-gqa4-yarn_Q4_K_M"])
 def test_self_extend_bitwise_golden(golden_dir, model):
-    """SURVEY §8 f-3, Self-Extend (cpp/bridge.cpp:509-524, grp_attn_n = 2, grp_attn_w = 16): llama_kv_cache_seq_add / seq_div /
+    """Self-Extend (cpp/bridge.cpp:509-524, grp_attn_n = 2, grp_attn_w = 16): llama_kv_cache_seq_add / seq_div /
     seq_add before every decode — prompt chunks and generated tokens — compress whole windows of positions; cells keep their
     places, several cells share a position, every window is re-rotated by its own delta. Every logit of
     tests/kvshift_script.py::run_self_extend equals the reference's, bit for bit."""
@@ -256,7 +256,7 @@ def test_prompt_batch_attention_in_launch_groups(tmp_path, heads, kv_heads, n_ct
 @pytest.mark.parametrize("cfg,ftype,n_prompt", [("llama3-8b-2l", "Q4_K_M", 200), ("llama3-8b-2l", "Q8_0", 130), ("llama3-8b-2l", "Q5_K_M", 70),
                                                 ("llama3-70b-1l", "Q4_K_M", 65), ("tiny-gqa4", "Q4_K_M", 450)])
 def test_prompt_batch_kernels_equal_token_by_token_bitwise(model_dir, cfg, ftype, n_prompt):
-    """SURVEY §8 a-4 / N-1: a prompt batch through the batched kernels (prefill.cuh: weight tiles fetched once per 64 tokens,
+    """a prompt batch through the batched kernels (prefill.cuh: weight tiles fetched once per 64 tokens,
     attention with the token in blockIdx.z) gives the logits AND the KV cache of the token-by-token path, bit for bit —
     partial last chunks of 64, two passes of 512 for the long prompt, every block type, GQA 4 and 8, then decode continues
     on the cache the batch wrote."""

@@ -32,7 +32,7 @@ def test_mixture_matches_reference_rules():
 
 
 def test_algorithmic_bytes_match_survey_table():
-    # SURVEY.md §8d / BASELINE.md §3
+    # all per-layer matrices, output and norm vectors, without token_embd
     assert round(G.weight_bytes_per_token(G.CONFIGS["llama3-8b"], "Q4_K_M") / 1e6, 1) == 4617.4
     assert round(G.weight_bytes_per_token(G.CONFIGS["llama3-8b"], "Q8_0") / 1e6, 1) == 7974.8
     assert round(G.weight_bytes_per_token(G.CONFIGS["mistral-7b"], "Q5_K_M") / 1e6, 1) == 5040.6

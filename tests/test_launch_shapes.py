@@ -1,6 +1,6 @@
-"""The launch shape the engine picks for every mat-vec of the BASELINE.json models (warps per CTA, warps sharing a 32-row
+"""The launch shape the engine picks for every mat-vec of the 8B, 70B and 7B models (warps per CTA, warps sharing a 32-row
 unit, ring stages per warp) — pure host arithmetic (b200_op_launch_shape), pinned here so that a change of the selection
-rule or of the shared-memory budget shows up as a deliberate diff. DESIGN.md §4 explains the half-occupied Q6_K shapes."""
+rule or of the shared-memory budget shows up as a deliberate diff. Q6_K tiles of 6.7 KB halve the warps that fit."""
 import ctypes as C
 
 import pytest
@@ -15,7 +15,7 @@ SHAPES = [
     ("8B wo",                        [Q4_K],        128,  4096, 0, (16, 16, 2)),
     ("8B gate|up",                   [Q4_K],        896,  4096, 1, (14, 2, 3)),
     ("8B ffn_down Q4_K",             [Q4_K],        128, 14336, 0, (14, 14, 2)),
-    ("8B ffn_down Q6_K",             [Q6_K],        128, 14336, 0, (8, 8, 3)),      # round-2 item 1
+    ("8B ffn_down Q6_K",             [Q6_K],        128, 14336, 0, (8, 8, 3)),
     ("8B output Q6_K",               [Q6_K],       4008,  4096, 1, (16, 1, 2)),
     ("70B qkv, attn_v Q5_K",         [Q4_K, Q5_K],  320,  8192, 1, (12, 4, 3)),
     ("70B gate|up",                  [Q4_K],       1792,  8192, 1, (14, 1, 3)),

@@ -49,7 +49,7 @@ def test_vec_dot_bit_exact(ops, name):
 # V.p, ggml_vec_dot_f16 for batch > 1, the ggml_v_expf polynomial in silu/softmax, double row sums — so whole-model
 # logits are BIT-IDENTICAL to the reference's, step after step. Bitwise equality is the criterion: with quantized
 # activations anything weaker is meaningless, because a 1-ulp upstream difference eventually flips an int8 of a
-# Q8_K block and the deviation cascades to ~1e-2 and persists through the KV cache (DESIGN.md "why bit-exact").
+# Q8_K block and the deviation cascades to ~1e-2 and persists through the KV cache.
 @pytest.mark.parametrize("model", ["tiny_Q4_K_M", "tiny_Q5_K_M", "tiny_Q8_0", "tiny-gqa4_Q4_K_M", "tiny-gqa4-yarn_Q4_K_M"])
 def test_model_logits_vs_golden_bitwise(golden_dir, model):
     g = np.load(os.path.join(golden_dir, model + ".npz"))
@@ -73,7 +73,7 @@ def test_model_logits_vs_golden_bitwise(golden_dir, model):
 @pytest.mark.parametrize("model", ["tiny-gqa4_Q4_K_M", "tiny-gqa4-yarn_Q4_K_M"])
 @pytest.mark.parametrize("scenario", ["kvshift", "selfextend"])
 def test_port_kv_cells_vs_golden_bitwise(golden_dir, model, scenario):
-    """SURVEY §8 f-3 restated on the CPU: struct llama_kv_cache's cell bookkeeping (find_slot, seq_rm, seq_add, seq_div), the
+    """the KV cells restated on the CPU: struct llama_kv_cache's cell bookkeeping (find_slot, seq_rm, seq_add, seq_div), the
     K-shift of the cached f16 K rows by each cell's accumulated delta (build_k_shift) and attention masked by the cells'
     positions — the port reproduces every logit of the reference's context-shift scenario (cpp/bridge.cpp:487-507) and of its
     Self-Extend scenario (:509-524), bit for bit, incl. the YaRN model whose K-shift rescales every cell."""

@@ -1,4 +1,4 @@
-"""N > 1 host-side logic on CPU: world_size-2 `gloo` process group (SURVEY.md §8e): stage ranges partition the layers the
+"""N > 1 host-side logic on CPU: world_size-2 `gloo` process group: stage ranges partition the layers the
 way the reference's split does, the NCCL id reaches every rank, timings reduce to the slowest rank."""
 import os
 import socket
@@ -50,7 +50,7 @@ def _worker(rank, world, port, q):
         lb, le = P.stage_range(32, rank, world)
         slowest = P.max_over_ranks(dist, 1.0 + rank)
         launches = P.sum_over_ranks(dist, 100 * (rank + 1))
-        # the residual-stream hand-off, stood in for by gloo send/recv of f32[n_embd] (NCCL does it on the GPU box)
+        # the residual-stream hand-off, stood in for by gloo send/recv of f32[n_embd] (NCCL does it between GPUs)
         x = torch.full((4096,), float(rank), dtype=torch.float32)
         if rank == 0:
             dist.send(x, dst=1)

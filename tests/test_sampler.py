@@ -1,4 +1,4 @@
-"""the samplers behind doInference, pinned on the CPU against the reference's own sampler.
+"""The samplers behind doInference, pinned on the CPU against the reference's own sampler.
 
 Janus (booster_b200/csrc/janus.cpp) restates initJanus + sample_janus_token (cpp/janus.cpp:191-331, 405-700). The reference's
 janus.cpp is compiled UNMODIFIED into oracle/_ref; oracle/ref_shim.cpp runs the bridge's generation loop with it

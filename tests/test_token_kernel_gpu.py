@@ -1,6 +1,6 @@
 """The persistent per-token kernel (booster_b200/csrc/token_kernel.cuh: one launch per token, phases joined by grid
 barriers) computes with the same device code as the per-operator kernels: logits BIT-IDENTICAL to the reference's golden
-vectors, to the port oracle on the full 8B / 70B per-layer shapes at the end of the BASELINE contexts, and to the default
+vectors, to the port oracle on the full 8B / 70B per-layer shapes at the end of their contexts, and to the default
 path. It is selectable (b200_set_token_kernel / BOOSTER_B200_TOKEN_KERNEL=1), not the default — measured slower."""
 import os
 

@@ -1,4 +1,4 @@
-"""Tokenizer parity (SURVEY.md §8 f-1): booster_b200's llama_tokenize / llama_token_to_piece / llama_token_is_eog against
+"""Tokenizer parity: booster_b200's llama_tokenize / llama_token_to_piece / llama_token_is_eog against
 the reference's own tokenizer on synthetic SPM and byte-level-BPE (LLaMA-3 pre-tokenizer) vocabularies — token-id exact.
 Host-side code: no GPU needed. Golden vectors come from oracle/_ref (tests/golden/make_tokenizer_golden.py); where the
 reference library is present the comparison is also made live on further random strings, and the codepoint classes behind
@@ -158,7 +158,7 @@ def test_truncated_and_corrupted_gguf_fail_without_crashing(tmp_path):
 
 
 def test_crafted_gguf_headers_are_errors_not_crashes(tmp_path):
-    """the four crafted failures of the round-1 review: a 2^64-1 string length (pointer wrap), a huge array count
+    """four crafted failures: a 2^64-1 string length (pointer wrap), a huge array count
     (reserve -> length_error / bad_alloc), general.alignment = 0 (SIGFPE) and tensor sizes / offsets that overflow 64 bits"""
     import struct
 
