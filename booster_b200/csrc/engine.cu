@@ -1819,15 +1819,24 @@ static void pb_matmul(b200_ctx * c, const MatvecArgs & mv, int epi, int T, int p
     c->launches++;
 }
 // tokens per block of k_attn_scores_batch for nz tokens, the first of which sees n_kv cells. A block walks its tokens x GQA rows one after the other on
-// keys that it loads once: many rows save loads, few keep the SMs busy to the end. Halved from 16 until there are six blocks of 64 rows per SM, or as many more
-// as they are shorter (measured with 1, 2, 4, 8 and 16 tokens, 8 to 512 tokens at 0 to 8000, 8 heads on 1 key head to 64 on 8: within 5 % of the best of them, and
-// 16 heads on 2 key heads, 512 tokens at 0, two layers: 797 us with 16 tokens, 704 with four; 32 on 8, 512 at 8000: 7.1 ms with 16, 7.9 with four).
+// keys that it loads once, at the price of a dozen rows. An SM's share of all rows and a quarter of a block at the end, or one block where there are fewer than SMs, is
+// what a launch takes. Measured with 1, 2, 4, 8 and 16 tokens, 8 to 512 tokens at 0 to 8000, 8 heads on 1 key head to 64 on 8: nowhere slower than 16 throughout. 16 heads on 2 key
+// heads, 16 tokens at 0, two layers: 294 us with 16 tokens, 227 with one; 64 on 8, 256 tokens at 0: 2343 us with 16, 2195 with eight; 32 on 8, 64 tokens at 1000: 470 us with 16,
+// 482 with eight.
 static int scb_tokens(int n_head_kv, int gqa, int n_kv, int nz, int sm_count) {
-    for (int tq = SCB_TQ; ; tq /= 2) {
-        int64_t blocks = 0;                                // those with keys that a token of theirs sees
-        for (int z = 0; z < nz; z += tq) blocks += ((n_kv + std::min(z + tq, nz) - 1 + 31) / 32 * 32 + SCB_KEYS - 1) / SCB_KEYS;
-        if (tq == 1 || blocks * n_head_kv * 64 >= (int64_t) 6 * sm_count * tq * gqa) return tq;
+    int best = SCB_TQ;
+    int64_t least = INT64_MAX;
+    for (int tq = SCB_TQ; tq >= 1; tq /= 2) {
+        int64_t rows = 0;                                  // of the blocks with keys that a token of theirs sees
+        for (int z = 0; z < nz; z += tq) {
+            const int n = std::min(tq, nz - z);
+            rows += (int64_t) (((n_kv + z + n - 1 + 31) / 32 * 32 + SCB_KEYS - 1) / SCB_KEYS * n_head_kv) * (n * gqa + 12);
+        }
+        const int one = std::min(tq, nz) * gqa;
+        const int64_t cost = std::max(4 * (int64_t) sm_count * (one + 12), 4 * rows + (int64_t) sm_count * one);
+        if (cost < least) { least = cost; best = tq; }
     }
+    return best;
 }
 extern "C" int b200_op_score_tokens(int n_head_kv, int gqa, int past, int n, int sm_count) {
     return n_head_kv > 0 && gqa > 0 && past >= 0 && n > 0 && sm_count > 0 ? scb_tokens(n_head_kv, gqa, past + 1, n, sm_count) : 0;

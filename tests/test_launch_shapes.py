@@ -47,9 +47,9 @@ def test_launch_shape_rejects_oversized_vectors():
 
 
 @pytest.mark.parametrize("kv,gqa,past,n,want", [
-    (8, 4, 6000, 512, 16), (8, 4, 0, 512, 8), (8, 4, 1234, 77, 8), (16, 1, 0, 512, 16),   # many keys or heads: whole tiles
-    (2, 8, 0, 16, 1), (2, 8, 300, 64, 1), (8, 4, 0, 16, 1), (8, 8, 0, 256, 4),            # few: 16 tokens x 8 heads in two blocks took 24 us a layer more
-    (1, 8, 8000, 128, 8), (1, 8, 0, 1, 1)])
+    (8, 4, 6000, 512, 16), (8, 4, 0, 512, 16), (8, 4, 1234, 77, 16), (16, 1, 0, 512, 16), (8, 8, 8000, 74, 16),   # many keys or heads: whole tiles
+    (2, 8, 0, 16, 1), (2, 8, 300, 64, 2), (8, 4, 0, 16, 1), (2, 8, 0, 512, 8),             # few: 16 tokens x 8 heads in two blocks took 24 us a layer more
+    (8, 8, 0, 256, 8), (1, 8, 8000, 128, 16), (8, 4, 1000, 64, 16)])
 def test_score_tile(kv, gqa, past, n, want):
     """tokens per block of a prompt batch's score kernel: few enough that the grid fills 148 SMs"""
     assert _lib.lib().b200_op_score_tokens(kv, gqa, past, n, 148) == want
