@@ -1265,21 +1265,16 @@ constexpr int GX_MIN_K = 1024;
 struct UmmaScratch { __nv_bfloat16 * xb = nullptr; size_t elems = 0; int * err = nullptr; float * part = nullptr; int sm_count = 148; };
 size_t umma_part_floats(int sm_count) { return (size_t) sm_count * UM_BM * UM_BN; }      // one K part of an output tile per SM
 
-// K parts of a float32 product with few output tiles: two blocks of 128 x 128 per SM, 256 k each at least, where that is faster than 64 x 64 tiles (else 1). (All
-// parts together hold no more than two tiles per SM, which is what umma_part_floats has room for.)
-// The two times in us, from T = 64 to 600, N = 128 to 16000, K = 512 to 4096 on 148 SMs: a thin wave of 64 x 64 tiles takes 0.0725 per k, a fuller one more with its blocks per
-// SM (more still on weights that do not fit the L2); a part takes 0.137 per k with an SM to itself, 0.208 beside a second one. At K = 512 it goes either way: 600 x 1024 50
-// us whole and 44 in two parts, 600 x 640 41 and 44; so it does where half of each tile's rows are empty: 64 x 16000 x 1024 118 and 121. Long sums gain most: 300 x 1024 x 4096 355 and 88.
+// K parts of a float32 product with few output tiles (1: whole, in 64 x 64 tiles): two blocks of 128 x 128 per SM, 256 k each at least. (All parts together hold no
+// more than two tiles per SM, which is what umma_part_floats has room for.) In whole models of width 512 and 1024, where weights come from memory, no product of 64
+// to 600 tokens was faster whole (a pass of 64 tokens, the 512 x 512 products alone: 1959 us whole, 1861 in two parts; 1024 x 4096 2736 and 1398). Alone, 64 x 16000 is, up to
+// k = 1024: half of each tile's rows are empty, and there is room for two parts only (k = 512: 62 us whole, 68 in two parts; k = 2048: 234 and 226).
 int f32_k_parts(int T, int N, int K, int sm_count) {
     if (T < 64 || N < SG_BN || !split_k_enabled() || !simt_big_enabled()) return 1;
-    const int tiles = ((N + SG_BN - 1) / SG_BN) * ((T + SG_BM - 1) / SG_BM), parts = std::min(2 * sm_count / tiles, (K + SG_BK - 1) / SG_BK / 16);
-    if (parts <= 1) return 1;
-    const float per_sm = (float) (((N + 63) / 64) * ((T + 63) / 64)) / (float) sm_count;
-    const float whole = 4.f + (float) K * (per_sm <= 0.7f ? 0.0725f : 0.075f + 0.024f * per_sm);
-    const float cut = tiles * parts > sm_count ? 15.f + 0.208f * (float) K / (float) parts : 6.f + 0.137f * (float) K / (float) parts;
-    return cut < 0.97f * whole ? parts : 1;
+    const int room = 2 * sm_count / (((N + SG_BN - 1) / SG_BN) * ((T + SG_BM - 1) / SG_BM));
+    if (T <= 64 && room == 2 && K <= 1024) return 1;
+    return std::min(room, (K + SG_BK - 1) / SG_BK / 16);
 }
-
 // 16-byte chunks of a row that a lane of k_gemv_x takes: 1, 2 or 4 (0: the row is too long)
 int gx_chunks(int chunks) { return chunks <= GX_WARPS * 32 ? 1 : chunks <= 2 * GX_WARPS * 32 ? 2 : chunks <= 4 * GX_WARPS * 32 ? 4 : 0; }
 // one token: whether k_gemv_x is faster than k_gemv. A row has to fill most of a block's lanes (in sixteenths, by chunks per lane): 8192 x 1024 in bf16, half of them, takes 9.8 us

@@ -76,7 +76,8 @@ BF16, F32 = 0, 1
     (BF16, 1, 16000, 16384, 0, 0), (F32, 1, 16000, 8192, 0, 0),                  # eight chunks a lane: 1.4 and 1.2 times
     (BF16, 1, 512, 2048, 0, 1), (BF16, 4, 16000, 2048, 0, 0), (BF16, 1, 2048, 2044, 0, 0),
     (F32, 300, 1024, 4096, 0, 4), (F32, 600, 1024, 512, 0, 4), (F32, 64, 4096, 2048, 0, 4),
-    (F32, 600, 640, 512, 0, 6), (F32, 300, 4096, 512, 0, 6), (F32, 64, 16000, 512, 0, 6), (F32, 600, 4096, 4096, 0, 6), (F32, 300, 1024, 4096, 1, 6),
+    (F32, 64, 512, 512, 0, 4), (F32, 64, 16000, 512, 0, 6), (F32, 64, 16000, 2048, 0, 4), (F32, 100, 16000, 512, 0, 4), (F32, 600, 4096, 4096, 0, 6),
+    (F32, 64, 512, 256, 0, 6), (F32, 300, 1024, 4096, 1, 6),
     (BF16, 64, 128, 64, 0, 3), (BF16, 63, 128, 64, 0, 5), (BF16, 64, 128, 60, 0, 6)])
 def test_stack_product_kernel(dtype, T, N, K, glu, want):
     """which kernel a layer stack's product takes: 0 a warp per row, 1 a block per row, 2 a block per eight rows with x in registers, 3 tcgen05, 4 float32
