@@ -47,6 +47,7 @@
 #include <cstring>
 #include <memory>
 #include <stdexcept>
+#include <utility>
 #include <vector>
 
 namespace b200 {
@@ -178,6 +179,7 @@ struct RunSpec {                         // one execution of a layer within a st
 
 struct StackModel {
     int device = 0, dtype = STACK_BF16;
+    std::vector<std::pair<int, int>> mats;      // (N, K) of every matrix that is not one of a batch
     std::string design;
     int vocab = 0, E = 0, groups = 1;
     float eps = 1e-6f;
@@ -275,8 +277,8 @@ struct StackCtx {
     int sm_count = 148;
     __nv_bfloat16 * xb = nullptr;         // activations of a prompt pass rounded to bfloat16 (operand of the tcgen05 product)
     size_t xb_elems = 0;
-    float * xpart = nullptr;              // sums of the K parts of a product with few output tiles; a float32 context has it from the first such product on
-    bool no_xpart = false;                // ... or could not get it: its products stay whole
+    float * xpart = nullptr;              // sums of the K parts of a product with few output tiles
+    size_t xpart_floats = 0;
     int * d_err = nullptr, * h_err = nullptr;   // raised by a kernel whose bounded wait ran out
     bool taps = false;
     std::vector<float> tap_data;
@@ -323,6 +325,7 @@ DMat up_mat(StackModel & m, const std::vector<float> & w, int N, int K, const st
     }
     if (bias) { d.bias = up_f32(m, *bias); d.bytes += (int64_t) bias->size() * 4; }
     m.weight_bytes += d.bytes;
+    if (batch == 1) m.mats.emplace_back(N, K);
     return d;
 }
 void append(std::vector<float> & a, const std::vector<float> & b) { a.insert(a.end(), b.begin(), b.end()); }
@@ -1262,7 +1265,7 @@ constexpr int GEMV_FEW_ROWS = 512;
 constexpr int GX_MIN_K = 1024;
 // what the tcgen05 product needs beside its operands: room for the activations rounded to bfloat16 and the error flag its
 // bounded waits raise
-struct UmmaScratch { __nv_bfloat16 * xb = nullptr; size_t elems = 0; int * err = nullptr; float * part = nullptr; int sm_count = 148; };
+struct UmmaScratch { __nv_bfloat16 * xb = nullptr; size_t elems = 0; int * err = nullptr; float * part = nullptr; size_t part_floats = 0; int sm_count = 148; };
 size_t umma_part_floats(int sm_count) { return (size_t) sm_count * UM_BM * UM_BN; }      // one K part of an output tile per SM
 
 // K parts of a float32 product with few output tiles (1: whole, in 64 x 64 tiles): two blocks of 128 x 128 per SM, 256 k each at least. (All parts together hold no
@@ -1274,6 +1277,16 @@ int f32_k_parts(int T, int N, int K, int sm_count) {
     const int room = 2 * sm_count / (((N + SG_BN - 1) / SG_BN) * ((T + SG_BM - 1) / SG_BM));
     if (T <= 64 && room == 2 && K <= 1024) return 1;
     return std::min(room, (K + SG_BK - 1) / SG_BK / 16);
+}
+// room for the parts of every product that a float32 model runs on portions of up to cap tokens
+size_t f32_part_floats(const StackModel & m, int cap, int sm_count) {
+    size_t most = 0;
+    for (const auto & nk : m.mats)
+        for (int t = SG_BM; t - SG_BM < cap; t += SG_BM) {
+            const int T = std::min(t, cap), parts = f32_k_parts(T, nk.first, nk.second, sm_count);
+            if (parts > 1) most = std::max(most, (size_t) parts * T * nk.first);
+        }
+    return most;
 }
 // 16-byte chunks of a row that a lane of k_gemv_x takes: 1, 2 or 4 (0: the row is too long)
 int gx_chunks(int chunks) { return chunks <= GX_WARPS * 32 ? 1 : chunks <= 2 * GX_WARPS * 32 ? 2 : chunks <= 4 * GX_WARPS * 32 ? 4 : 0; }
@@ -1293,12 +1306,15 @@ bool gx_pays(bool f32, int chunks, int N, int batch, bool glu, int sm_count) {
 }
 // the kernel a product goes to: mat-vecs of few tokens, then tile kernels
 enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG, LIN_ROWS_X, LIN_UMMA, LIN_F32_PARTS, LIN_MMA, LIN_SIMT };
-// vec: LinArgs::vec; x_elems: entries of X; xb_elems, part: what the scratch has room for
-LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu, bool seg, size_t x_elems, size_t xb_elems, bool part, int sm_count) {
+// vec: LinArgs::vec; x_elems: entries of X; xb_elems, part_floats: what the scratch has room for
+LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu, bool seg, size_t x_elems, size_t xb_elems, size_t part_floats, int sm_count) {
     if (T == 1 && vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && gx_pays(dtype == STACK_F32, K / (dtype == STACK_F32 ? 4 : 8), N, batch, glu, sm_count)) return LIN_ROWS_X;
     if (T <= GEMV_MAX_T) return !glu && batch == 1 && N <= GEMV_FEW_ROWS && K >= 1024 ? LIN_ROWS_LONG : LIN_ROWS;      // few, long rows: a block each
     if (dtype == STACK_BF16 && vec && umma_enabled() && T >= 64 && N >= 128 && K >= 64 && x_elems <= xb_elems) return LIN_UMMA;
-    if (dtype == STACK_F32 && vec && batch == 1 && !glu && !seg && part && f32_k_parts(T, N, K, sm_count) > 1) return LIN_F32_PARTS;
+    if (dtype == STACK_F32 && vec && batch == 1 && !glu && !seg) {
+        const int parts = f32_k_parts(T, N, K, sm_count);
+        if (parts > 1 && (size_t) parts * T * N <= part_floats) return LIN_F32_PARTS;
+    }
     return dtype == STACK_BF16 && vec && mma_enabled() ? LIN_MMA : LIN_SIMT;
 }
 
@@ -1344,7 +1360,7 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
     const auto al16 = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
     a.vec = K % vecw == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % vecw == 0 && al16(X) && al16(W);
     if (launches) (*launches)++;
-    const LinRoute route = lin_route(dtype, T, N, K, batch, a.vec != 0, a.glu != 0, a.seg != nullptr, (size_t) xbatch * T * K, us && us->xb ? us->elems : 0, us && us->part, us ? us->sm_count : 148);
+    const LinRoute route = lin_route(dtype, T, N, K, batch, a.vec != 0, a.glu != 0, a.seg != nullptr, (size_t) xbatch * T * K, us && us->xb ? us->elems : 0, us && us->part ? us->part_floats : 0, us ? us->sm_count : 148);
     if (route == LIN_ROWS_X) {
         const int ch = gx_chunks(K / vecw);
         const dim3 grid((unsigned) ((N + GX_ROWS - 1) / GX_ROWS), 1, (unsigned) batch);
@@ -1398,12 +1414,7 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
 
 void linear(StackCtx * c, const float * X, int ldx, const DMat & W, float * Y, int ldy, int T, int batch = 1, long long sX = 0, long long sY = 0, bool glu = false, float glu_limit = 0.f,
             const LinOpt * opt = nullptr) {
-    // (never inside a capture: only products of 64 tokens and more are cut along K)
-    if (c->m->dtype == STACK_F32 && batch == 1 && !glu && f32_k_parts(T, W.N, W.K, c->sm_count) > 1 && !c->xpart && !c->no_xpart && cudaMalloc(&c->xpart, umma_part_floats(c->sm_count) * 4) != cudaSuccess) {
-        cudaGetLastError();
-        c->xpart = nullptr; c->no_xpart = true;
-    }
-    const UmmaScratch us{c->xb, c->xb_elems, c->d_err, c->xpart, c->sm_count};
+    const UmmaScratch us{c->xb, c->xb_elems, c->d_err, c->xpart, c->xpart_floats, c->sm_count};
     linear_on(c->st, c->m->dtype, &c->launches, X, ldx, W.w, W.bias, Y, ldy, T, W.N, W.K, batch, sX, (long long) W.N * W.K, sY, glu, glu_limit, &us, opt);
 }
 
@@ -2563,8 +2574,9 @@ StackCtx * stack_ctx_new(StackModel * m, int n_ctx) {
         if (m->dtype == STACK_BF16) {
             c->xb_elems = std::max(cap * (size_t) std::max({ 2 * m->E, m->maxA, m->maxOL, m->maxP, m->max_dense, m->side_dim }), moe_rows * (size_t) std::max(m->E, m->max_eff));
             SCU(cudaMalloc(&c->xb, c->xb_elems * 2));
-            SCU(cudaMalloc(&c->xpart, umma_part_floats(c->sm_count) * 4));
-        }
+            c->xpart_floats = umma_part_floats(c->sm_count);
+        } else c->xpart_floats = f32_part_floats(*m, c->cap, c->sm_count);
+        if (c->xpart_floats) SCU(cudaMalloc(&c->xpart, c->xpart_floats * 4));
         SCU(cudaMalloc(&c->d_err, 4)); SCU(cudaMemsetAsync(c->d_err, 0, 4, c->st));
         SCU(cudaMallocHost(&c->h_err, 4)); *c->h_err = 0;
         c->caches.assign((size_t) m->n_caches, nullptr);
@@ -2821,7 +2833,7 @@ int32_t stack_argmax(StackCtx * c) {
 }
 
 int stack_product_kernel(int dtype, int T, int N, int K, bool glu, int sm_count) {
-    return lin_route(dtype, T, N, K, 1, K % (dtype == STACK_F32 ? 4 : 8) == 0, glu, false, 0, 0, true, sm_count);
+    return lin_route(dtype, T, N, K, 1, K % (dtype == STACK_F32 ? 4 : 8) == 0, glu, false, 0, 0, SIZE_MAX, sm_count);
 }
 
 float stack_time_linear(int device, int dtype, int T, int N, int K, int reps) {
@@ -2838,7 +2850,7 @@ float stack_time_linear(int device, int dtype, int T, int N, int K, int reps) {
         SCU(cudaMalloc(&X, (size_t) T * K * 4)); SCU(cudaMalloc(&Y, (size_t) T * N * 4)); SCU(cudaMalloc(&W, wbytes * copies));
         SCU(cudaMemset(X, 0, (size_t) T * K * 4)); SCU(cudaMemset(W, 0, wbytes * copies));
         us.elems = (size_t) T * K;
-        SCU(cudaMalloc(&us.xb, us.elems * 2)); SCU(cudaMalloc(&us.part, umma_part_floats(us.sm_count) * 4)); SCU(cudaMalloc(&us.err, 4)); SCU(cudaMemset(us.err, 0, 4));
+        SCU(cudaMalloc(&us.xb, us.elems * 2)); us.part_floats = umma_part_floats(us.sm_count); SCU(cudaMalloc(&us.part, us.part_floats * 4)); SCU(cudaMalloc(&us.err, 4)); SCU(cudaMemset(us.err, 0, 4));
         SCU(cudaStreamCreate(&st)); SCU(cudaEventCreate(&e0)); SCU(cudaEventCreate(&e1));
         for (int i = 0; i < 3; i++) linear_on(st, dtype, nullptr, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
         SCU(cudaStreamSynchronize(st));
@@ -2873,7 +2885,7 @@ void stack_linear(int device, int dtype, int T, int N, int K, const float * x, c
         SCU(cudaMalloc(&X, (size_t) T * K * 4)); SCU(cudaMalloc(&Y, (size_t) T * ny * 4));
         SCU(cudaMemcpy(X, x, (size_t) T * K * 4, cudaMemcpyHostToDevice));
         us.elems = (size_t) T * K;
-        SCU(cudaMalloc(&us.xb, us.elems * 2)); SCU(cudaMalloc(&us.part, umma_part_floats(us.sm_count) * 4)); SCU(cudaMalloc(&us.err, 4)); SCU(cudaMemset(us.err, 0, 4));
+        SCU(cudaMalloc(&us.xb, us.elems * 2)); us.part_floats = umma_part_floats(us.sm_count); SCU(cudaMalloc(&us.part, us.part_floats * 4)); SCU(cudaMalloc(&us.err, 4)); SCU(cudaMemset(us.err, 0, 4));
         linear_on(nullptr, dtype, nullptr, X, K, d.w, d.bias, Y, ny, T, N, K, 1, 0, 0, 0, glu != 0, limit, &us);
         SCU(cudaDeviceSynchronize());
         SCU(cudaMemcpy(y, Y, (size_t) T * ny * 4, cudaMemcpyDeviceToHost));

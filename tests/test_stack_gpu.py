@@ -453,8 +453,8 @@ def test_products_where_their_rules_change(dtype, T, N, K, glu):
 
 
 def test_float32_contexts_hold_no_room_for_products_they_never_run(tmp_path):
-    """a float32 context has the 19 MB for products cut along K from its first portion of 64 tokens on, and not before: sixteen small contexts stay well below
-    what that room alone would take, and one that does run such a portion decodes the same rows afterwards"""
+    """a float32 context has room for the K parts of its own model's products and no more (19 MB would hold any): sixteen small contexts stay well below what
+    that alone would take, and a portion that is cut into parts decodes the oracle's rows"""
     torch = pytest.importorskip("torch")
     p = Pair(tmp_path, config([mingru(width=200)], width=1056), n_ctx=160)      # 600 x 1056: four K parts
     free = torch.cuda.mem_get_info()[0]
