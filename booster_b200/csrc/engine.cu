@@ -2815,8 +2815,8 @@ extern "C" int b200_op_mul_mat_vec(int type, const void * w, int64_t n_rows, int
     } catch (const std::exception & e) { return set_err(e.what()); }
 }
 
-// the batched mat-mul of a prompt batch as an operator: y[T][n_rows] = W x[t] for T <= 512 tokens, through k_quant_batch(_mma) +
-// k_mma_batch / k_matmul_batch exactly as prefill_batch() launches them (tests: worst-case magnitudes, ragged T)
+// the batched mat-mul of a prompt batch as an operator: y[T][n_rows] = W x[t] for T <= 512 tokens, through k_quant_batch(_mma) and
+// the kernel that pb_mma_mode picks, as prefill_batch() launches them (tests: worst-case magnitudes, ragged T)
 extern "C" int b200_op_mul_mat(int type, const void * w, int64_t n_rows, int64_t k, const float * x, int64_t T, float * y) {
     try {
         require_gpu();

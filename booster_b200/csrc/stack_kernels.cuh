@@ -482,8 +482,8 @@ __global__ void __launch_bounds__(256) k_gemm_simt(const LinArgs a) {
 // half-warp stay free of bank conflicts), twice the FMAs per shared-memory read of the 64 x 64 kernel, the next K slice
 // of both operands in registers while the current one is multiplied. float32 operands with 16-byte aligned rows only (a.vec); no gated unit, no segments.
 // Products of float32 models whose tiles leave SMs idle run here too, cut along K like k_gemm_bf16_umma's (ksplit > 1: blockIdx.z is the part, sums to
-// part [ksplit][T][N], k_split_sum adds them): 300 tokens x 1024 x 4096 as 80 blocks of 64 x 64 took 234 us, in twelve parts 83. Packed fmas
-// (pairs of columns) were tried and gain nothing: the shared-memory reads are the bound.
+// part [ksplit][T][N], k_split_sum adds them): 300 tokens, 1024 rows, k = 4096: 355 us as 80 blocks of 64 x 64, 88 in twelve parts. Bound by the
+// shared-memory reads.
 constexpr int SG_BM = 128, SG_BN = 128, SG_BK = 16;
 __global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a, int ksplit = 1, float * __restrict__ part = nullptr) {
     __shared__ __align__(16) float Xs[SG_BK][SG_BM + 4];

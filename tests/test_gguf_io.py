@@ -31,7 +31,7 @@ def test_mixture_matches_reference_rules():
     assert set(t70[f"blk.{i}.attn_v.weight"] for i in range(80)) == {G.Q5_K, G.Q6_K}   # 70B: Q4_K attn_v -> Q5_K
 
 
-def test_algorithmic_bytes_match_survey_table():
+def test_algorithmic_bytes_of_the_measured_models():
     # all per-layer matrices, output and norm vectors, without token_embd
     assert round(G.weight_bytes_per_token(G.CONFIGS["llama3-8b"], "Q4_K_M") / 1e6, 1) == 4617.4
     assert round(G.weight_bytes_per_token(G.CONFIGS["llama3-8b"], "Q8_0") / 1e6, 1) == 7974.8
