@@ -26,7 +26,7 @@
 #include "token_kernel.cuh"
 #include "prefill.cuh"
 #include "prefill_mma.cuh"
-#include "prefill_umma.cuh"
+#include "prefill_umma_q80.cuh"
 
 #include <algorithm>
 #include <array>
@@ -1696,7 +1696,7 @@ static void prefill_alloc(b200_ctx * c) {
     c->pb.cap = T;
 }
 static bool has_q6k(const TMat * seg, int n_seg) { for (int i = 0; i < n_seg; i++) if (seg[i].type == T_Q6_K) return true; return false; }
-// K-quant launches run on the tensor cores: tcgen05 (prefill_umma.cuh), or mma.sync (prefill_mma.cuh) for few and short rows
+// Launches run on the tensor cores: tcgen05 (prefill_umma.cuh, prefill_umma_q80.cuh), or mma.sync (prefill_mma.cuh) for few and short rows of K-quants
 static int g_prefill_mma = -1;         // 2 (default): tcgen05 (k_umma_batch) where it is the faster one, 1: mma.sync (k_mma_batch), 0: the dp4a kernel
 extern "C" void b200_set_prefill_mma(int mode) { g_prefill_mma = mode < 0 ? 0 : mode > 2 ? 2 : mode; }
 // Where the two K-quant products part. Both run one block per SM; k_mma_batch's tiles are 64 rows x 32 tokens, k_umma_batch's twice as many rows, and a
@@ -1705,13 +1705,13 @@ extern "C" void b200_set_prefill_mma(int mode) { g_prefill_mma = mode < 0 ? 0 : 
 // 2 us of 21 to 40 from k = 2048 on, on weights that come from memory (4096 x 4096, 32 tokens: 32 and 30 us); shorter rows lose what the longer pipeline
 // costs, 1 to 3 us a launch (k = 512 and 768, 8 tokens, 16 launches: 350 and 389 us). Q5_K expands slowest and is behind at every k (4096 x 4096, 32 tokens: 34 and 37 us).
 static constexpr int UM_MIN_K = 2048;
-// record layout / kernel of a launch: 3 = k_mma_batch_q80, 2 = k_umma_batch, 1 = k_mma_batch (segments of an even number of units), 0 = dp4a
+// record layout / kernel of a launch: 3 = k_umma_batch_q80, 2 = k_umma_batch, 1 = k_mma_batch (segments of an even number of units), 0 = dp4a
 static int pb_mma_mode(const MatvecArgs & mv, int T, int sm_count) {
     if (g_prefill_mma < 0) { const char * e = getenv("BOOSTER_B200_PREFILL_MMA"); g_prefill_mma = e ? std::max(0, std::min(2, atoi(e))) : 2; }
     if (g_prefill_mma == 0) return 0;
     bool even = true;
     for (int i = 0; i < mv.n_seg; i++) even = even && !(mv.seg[i].n_units & 1);
-    if (mv.act_q8_0) {   // Q8_0 x Q8_0: block-diagonal HMMA (k_mma_batch_q80)
+    if (mv.act_q8_0) {   // Q8_0 x Q8_0: block-diagonal MMAs (k_umma_batch_q80)
         for (int i = 0; i < mv.n_seg; i++) if (mv.seg[i].type != T_Q8_0) return 0;
         return even ? 3 : 0;
     }
@@ -1766,18 +1766,15 @@ static void pb_matmul(b200_ctx * c, const MatvecArgs & mv, int epi, int T, int p
     const int mma_mode = pb_mma_mode(mv, T, c->sm_count);
     bool q4 = false, q5 = false, q6 = false;
     for (int i = 0; i < mv.n_seg; i++) { q4 |= mv.seg[i].type == T_Q4_K; q5 |= mv.seg[i].type == T_Q5_K; q6 |= mv.seg[i].type == T_Q6_K; }
+    if (mma_mode >= 2) {
+        a.um_tok_tiles = (T + UM_NT - 1) / UM_NT;
+        for (int i = 0; i < mv.n_seg; i++) a.um_row_tiles += (mv.seg[i].n_units + 3) / 4;
+        a.err = c->pb.err;
+    }
     if (mma_mode == 3) {
-        a.mb_a_bytes = (uint32_t) Q80_A_BYTES;
-        a.mb_raw_stride = (uint32_t) ((8 * sb + 127) / 128 * 128);
-        a.mb_rec_copy = (uint32_t) Q80_REC_BYTES;
-        a.mb_stage_bytes = 2 * a.mb_raw_stride + (a.mb_rec_copy + 127) / 128 * 128;
-        a.mb_stages = (int) std::min<size_t>(MB_MAX_STAGES, ((size_t) 226 * 1024 - 2 * a.mb_a_bytes) / a.mb_stage_bytes);
-        if (a.mb_stages < 2) throw std::runtime_error("k_mma_batch_q80: shared memory layout does not fit");
-        const size_t smem_q = (size_t) 2 * a.mb_a_bytes + (size_t) a.mb_stages * a.mb_stage_bytes;
         static size_t attr_q[64] = {0};
-        raise_smem(k_mma_batch_q80, smem_q, attr_q, c->device);
-        const dim3 grid_q((unsigned) ((T + MB_NT - 1) / MB_NT), (unsigned) (a.n_units / 2));
-        k_mma_batch_q80<<<grid_q, MB_WARPS * 32, smem_q, c->st>>>(a);
+        raise_smem(k_umma_batch_q80, (size_t) UQ_SMEM, attr_q, c->device);
+        k_umma_batch_q80<<<(unsigned) std::min(c->sm_count, a.um_row_tiles * a.um_tok_tiles), UM_THREADS, UQ_SMEM, c->st>>>(a);
         c->launches++;
         return;
     }
@@ -1785,9 +1782,6 @@ static void pb_matmul(b200_ctx * c, const MatvecArgs & mv, int epi, int T, int p
         a.mb_raw_stride = (uint32_t) sb;
         a.mb_stage_bytes = (4 * a.mb_raw_stride + UM_REC_BYTES + 127) / 128 * 128;
         a.mb_stages = (int) std::min<size_t>(UM_MAX_STAGES, ((size_t) 226 * 1024 - UM_FIXED_SMEM) / a.mb_stage_bytes);
-        a.um_tok_tiles = (T + UM_NT - 1) / UM_NT;
-        for (int i = 0; i < mv.n_seg; i++) a.um_row_tiles += (mv.seg[i].n_units + 3) / 4;
-        a.err = c->pb.err;
         const size_t smem_u = (size_t) UM_FIXED_SMEM + (size_t) a.mb_stages * a.mb_stage_bytes;   // (more than half an SM's: one CTA per SM)
         static size_t attr_u[64] = {0};
         raise_smem(k_umma_batch, smem_u, attr_u, c->device);

@@ -167,8 +167,24 @@ __device__ __forceinline__ void um_write_records(const ActSmem & A, int n256, ui
     }
 }
 
+static constexpr int UQ_BLOCK_REC = UM_NT * 64 + UM_NT * 4;    // records of one (32-token chunk, 32-weight block): [8-byte piece c (4)][token][8 fp16] | f32 d[32]
+static constexpr int UQ_OFF_DX = UM_NT * 64;
+// k_quant_batch_mma, layout 3: token t's Q8_0 image (natural order) -> its pieces of the chunk's record blocks
+__device__ __forceinline__ void uq_write_records(const ActSmem & A, int n256, uint8_t * rec, int t, int lane, int warp, int W) {
+    const int chunk = t / UM_NT, j = t % UM_NT, blk = lane >> 2, c = lane & 3;
+    for (int b = warp; b < n256; b += W) {
+        uint8_t * r = rec + (((size_t) chunk * n256 + b) * 8 + blk) * UQ_BLOCK_REC;
+        const uint2 w = *reinterpret_cast<const uint2 *>(A.q + (size_t) b * 256 + 8 * lane);
+        uint4 o;
+        o.x = h2_ints(sbyte_of(w.x, 0), sbyte_of(w.x, 1)); o.y = h2_ints(sbyte_of(w.x, 2), sbyte_of(w.x, 3));
+        o.z = h2_ints(sbyte_of(w.y, 0), sbyte_of(w.y, 1)); o.w = h2_ints(sbyte_of(w.y, 2), sbyte_of(w.y, 3));
+        *reinterpret_cast<uint4 *>(r + c * (UM_NT * 16) + j * 16) = o;
+        if (c == 0) *reinterpret_cast<float *>(r + UQ_OFF_DX + j * 4) = A.dx[b * 8 + blk];
+    }
+}
+
 // k_quant_batch with the tensor-core record layouts (one CTA per token: the decode path's prologue, then the image is written out
-// for k_mma_batch (layout 1) or k_umma_batch (layout 2))
+// for k_mma_batch (layout 1), k_umma_batch (layout 2) or k_umma_batch_q80 (layout 3))
 __global__ void __launch_bounds__(512) k_quant_batch_mma(const QuantBatchArgs a) {
     extern __shared__ __align__(16) uint8_t qb_smem[];
     __shared__ double red_smem[MV_MAX_WARPS];
@@ -185,7 +201,7 @@ __global__ void __launch_bounds__(512) k_quant_batch_mma(const QuantBatchArgs a)
     }
     prologue_quantize<false, true>(a.X + (size_t) t * a.k, norm, a.eps, a.k, a.inv_k, a.act_q8_0, A, red_smem, ww, []() {}, W);
     __syncthreads();
-    if (a.layout == 3) q80_write_records(A, a.k / 256, a.rec, t, lane, warp, W);
+    if (a.layout == 3) uq_write_records(A, a.k / 256, a.rec, t, lane, warp, W);
     else if (a.layout == 2) um_write_records(A, a.k / 256, a.rec, t, lane, warp, W);
     else mb_write_records(A, a.k / 256, a.rec, t, lane, warp, W);
 }

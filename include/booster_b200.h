@@ -159,7 +159,7 @@ int64_t b200_trace_token(b200_ctx * c, int32_t token, int pos, int reps, uint64_
 void b200_set_prefill_batch(int on);
 /* K-quant prompt batches: 2 (default) = tcgen05.mma with operands and accumulators in TMEM (k_umma_batch), mma.sync where one wave of
    its smaller tiles is enough and rows are short or Q5_K;
-   1 = mma.sync HMMA (k_mma_batch); 0 = the dp4a batch kernel; all three are bit-identical */
+   1 = mma.sync HMMA (k_mma_batch); 0 = the dp4a batch kernel; all three are bit-identical. Q8_0: k_umma_batch_q80 in modes 1 and 2 */
 void b200_set_prefill_mma(int mode);
 /* 1 (default): prompt-batch attention through k_attn_softmax_rows + k_attn_pv_batch; 0: the per-token kernels over blockIdx.z */
 void b200_set_prefill_attn_batch(int on);
@@ -235,7 +235,7 @@ float * b200_decode_view(b200_ctx * c, int32_t token, int pos);
 int b200_op_launch_shape(const int32_t * types, int n_types, int64_t n_units, int64_t k, int norm, int sm_count, int32_t wgs[3]);
 /* tokens per block of a prompt batch's score kernel: n tokens behind `past` cells (host arithmetic, as above) */
 int b200_op_score_tokens(int n_head_kv, int gqa, int past, int n, int sm_count);
-/* kernel of one prompt product of T tokens: 2 = tcgen05, 1 = mma.sync, 3 = Q8_0's mma.sync, 0 = dp4a, -1 = bad arguments (host arithmetic, as above) */
+/* kernel of one prompt product of T tokens: 2 = tcgen05, 1 = mma.sync, 3 = Q8_0's tcgen05, 0 = dp4a, -1 = bad arguments (host arithmetic, as above) */
 int b200_op_prompt_kernel(const int32_t * types, int n_types, int64_t n_units, int64_t k, int T, int sm_count);
 
 /* ---- tokenizer (host side) ----------------------------------------------------------------------

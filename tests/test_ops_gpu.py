@@ -221,6 +221,25 @@ def test_mul_mat_batch_tcgen05_edges(name, shape, prefill_mma):
         assert np.array_equal(y[i], yr), f"token {i}: max abs diff {np.abs(y[i] - yr).max()}"
 
 
+@pytest.mark.parametrize("shape", [(64, 256, 1), (64, 512, 33), (192, 256, 31), (320, 4352, 32), (19072, 256, 40), (128, 14336, 65)])
+def test_mul_mat_batch_q8_0_edges(shape):
+    """k_umma_batch_q80 where its tiles and rings end: half of a 128-row tile, two to 112 stages of four blocks (the first fewer than the ring has), one token past a
+    tile and one short of it, more tiles than SMs — the reference's bits, on the largest weights, zero blocks and scales at the end of fp16's range"""
+    n, k, T = shape
+    rng = np.random.default_rng(n + k + T)
+    w = _extreme_blocks("Q8_0", n, k, rng).reshape(n, -1)
+    w[1::4, :34] = 0                                                       # a block of zeros with a scale of zero
+    w[2::4, 0:2] = np.array([6e-8], np.float16).view(np.uint8)             # a sub-normal scale
+    x = (rng.standard_normal((T, k)) * rng.choice([1e-6, 0.01, 1.0, 30.0], size=(T, 1))).astype(np.float32)
+    x[0], x[-1] = 3.0, -3.0
+    x[T // 2, :32] = 0.0
+    w = w.reshape(-1)
+    y = engine.op_mul_mat(TYPES["Q8_0"], w, n, k, x)
+    for i in sorted({0, T // 2, T - 1}):
+        yr = port.mul_mat_vec(TYPES["Q8_0"], w, n, k, x[i])
+        assert np.array_equal(y[i], yr), f"token {i}: max abs diff {np.abs(y[i] - yr).max()}"
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0"])
 def test_mul_mat_batch_kernel_variants(name, mode, prefill_mma):
