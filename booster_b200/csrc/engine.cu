@@ -687,15 +687,19 @@ static bool pdl_enabled() {
     if (v < 0) { const char * e = getenv("BOOSTER_B200_NO_PDL"); v = (e && e[0] == '1') ? 0 : 1; }
     return v == 1;
 }
-template <typename Arg>
-static void launch_fwd(void (*kern)(Arg), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Arg & arg, bool pdl = true) {
+template <typename... P, typename... A>
+static void launch_joined(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const A &... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = (pdl && pdl_enabled()) ? 1 : 0;
-    CU(cudaLaunchKernelEx(&cfg, kern, arg));
+    CU(cudaLaunchKernelEx(&cfg, kern, args...));
+}
+template <typename Arg>
+static void launch_fwd(void (*kern)(Arg), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Arg & arg, bool pdl = true) {
+    launch_joined(kern, grid, block, smem, st, pdl, arg);
 }
 
 static constexpr int TRACE_CTAS = 512, TRACE_MAX_LAUNCHES = 1024;
@@ -1747,9 +1751,9 @@ static void pb_quant(b200_ctx * c, const float * X, int k, int T, const float * 
     if (mma) {
         static size_t attr_m[64] = {0};
         if (smem > 48 * 1024) raise_smem(k_quant_batch_mma, smem, attr_m, c->device);
-        k_quant_batch_mma<<<(unsigned) T, 512, smem, c->st>>>(a);
+        launch_joined(k_quant_batch_mma, dim3((unsigned) T), dim3(512), smem, c->st, true, a);
     } else {
-        k_quant_batch<<<(unsigned) T, 512, smem, c->st>>>(a);
+        launch_joined(k_quant_batch, dim3((unsigned) T), dim3(512), smem, c->st, true, a);
     }
     c->launches++;
 }
@@ -1774,7 +1778,7 @@ static void pb_matmul(b200_ctx * c, const MatvecArgs & mv, int epi, int T, int p
     if (mma_mode == 3) {
         static size_t attr_q[64] = {0};
         raise_smem(k_umma_batch_q80, (size_t) UQ_SMEM, attr_q, c->device);
-        k_umma_batch_q80<<<(unsigned) std::min(c->sm_count, a.um_row_tiles * a.um_tok_tiles), UM_THREADS, UQ_SMEM, c->st>>>(a);
+        launch_joined(k_umma_batch_q80, dim3((unsigned) std::min(c->sm_count, a.um_row_tiles * a.um_tok_tiles)), dim3(UM_THREADS), UQ_SMEM, c->st, true, a);
         c->launches++;
         return;
     }
@@ -1785,7 +1789,7 @@ static void pb_matmul(b200_ctx * c, const MatvecArgs & mv, int epi, int T, int p
         const size_t smem_u = (size_t) UM_FIXED_SMEM + (size_t) a.mb_stages * a.mb_stage_bytes;   // (more than half an SM's: one CTA per SM)
         static size_t attr_u[64] = {0};
         raise_smem(k_umma_batch, smem_u, attr_u, c->device);
-        k_umma_batch<<<(unsigned) std::min(c->sm_count, a.um_row_tiles * a.um_tok_tiles), UM_THREADS, smem_u, c->st>>>(a);
+        launch_joined(k_umma_batch, dim3((unsigned) std::min(c->sm_count, a.um_row_tiles * a.um_tok_tiles)), dim3(UM_THREADS), smem_u, c->st, true, a);
         c->launches++;
         return;
     }
@@ -1801,7 +1805,7 @@ static void pb_matmul(b200_ctx * c, const MatvecArgs & mv, int epi, int T, int p
         static size_t attr_m[64] = {0};
         raise_smem(k_mma_batch, smem_m, attr_m, c->device);
         const dim3 grid_m((unsigned) ((T + MB_NT - 1) / MB_NT), (unsigned) (a.n_units / 2));
-        k_mma_batch<<<grid_m, MB_WARPS * 32, smem_m, c->st>>>(a);
+        launch_joined(k_mma_batch, grid_m, dim3(MB_WARPS * 32), smem_m, c->st, true, a);
         c->launches++;
         return;
     }
@@ -1809,7 +1813,7 @@ static void pb_matmul(b200_ctx * c, const MatvecArgs & mv, int epi, int T, int p
     static size_t attr[64] = {0};
     raise_smem(k_matmul_batch, smem, attr, c->device);
     const dim3 grid((unsigned) ((T + PB_CHUNK - 1) / PB_CHUNK), (unsigned) a.n_units);
-    k_matmul_batch<<<grid, PB_WARPS * 32, smem, c->st>>>(a, sb);
+    launch_joined(k_matmul_batch, grid, dim3(PB_WARPS * 32), smem, c->st, true, a, sb);
     c->launches++;
 }
 // tokens per block of k_attn_scores_batch for nz tokens, the first of which sees n_kv cells. A block walks its tokens x GQA rows one after the other on
@@ -1858,17 +1862,17 @@ static void pb_attention(b200_ctx * c, int li, int T, int pos0) {
         const size_t smem_sc = (size_t) tq * GQA * 128 * 4;
         static size_t attr_sc[64] = {0};
         if (smem_sc > 48 * 1024) raise_smem(k_attn_scores_batch<GQA>, smem_sc, attr_sc, c->device);
-        k_attn_scores_batch<GQA><<<gs, SCB_KEYS, smem_sc, c->st>>>(a, nz, tq);
+        launch_joined(k_attn_scores_batch<GQA>, gs, dim3(SCB_KEYS), smem_sc, c->st, true, a, nz, tq);
         const unsigned rows = (unsigned) (nz * a.n_head);
         const int groups = (n_pad_max / 16 + SMX_THREADS - 1) / SMX_THREADS;
-        if (n_pad_max < SMX_MIN_ROW || groups > SMX_MAX_G) k_attn_softmax_rows<<<(rows + 7) / 8, 256, 0, c->st>>>(a, nz);
-        else if (groups == 1) k_attn_softmax_block<1><<<rows, SMX_THREADS, 0, c->st>>>(a, nz);
-        else if (groups == 2) k_attn_softmax_block<2><<<rows, SMX_THREADS, 0, c->st>>>(a, nz);
-        else k_attn_softmax_block<SMX_MAX_G><<<rows, SMX_THREADS, 0, c->st>>>(a, nz);
+        if (n_pad_max < SMX_MIN_ROW || groups > SMX_MAX_G) launch_joined(k_attn_softmax_rows, dim3((rows + 7) / 8), dim3(256), 0, c->st, true, a, nz);
+        else if (groups == 1) launch_joined(k_attn_softmax_block<1>, dim3(rows), dim3(SMX_THREADS), 0, c->st, true, a, nz);
+        else if (groups == 2) launch_joined(k_attn_softmax_block<2>, dim3(rows), dim3(SMX_THREADS), 0, c->st, true, a, nz);
+        else launch_joined(k_attn_softmax_block<SMX_MAX_G>, dim3(rows), dim3(SMX_THREADS), 0, c->st, true, a, nz);
         static size_t attr_pvb[64] = {0};
         raise_smem(k_attn_pv_batch<GQA>, PVB_SMEM, attr_pvb, c->device);
         constexpr int TQ = PVB_ROWS / GQA;
-        k_attn_pv_batch<GQA><<<dim3((unsigned) a.n_head_kv, (unsigned) ((nz + TQ - 1) / TQ)), PVB_THREADS, PVB_SMEM, c->st>>>(a, nz);
+        launch_joined(k_attn_pv_batch<GQA>, dim3((unsigned) a.n_head_kv, (unsigned) ((nz + TQ - 1) / TQ)), dim3(PVB_THREADS), PVB_SMEM, c->st, true, a, nz);
         c->launches += 3;
     }
 }

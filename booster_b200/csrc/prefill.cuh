@@ -31,6 +31,7 @@ __host__ __device__ __forceinline__ int pb_record_bytes(int act_q8_0, int with_a
 
 __global__ void k_embed_batch(int type, const uint8_t * __restrict__ rows, size_t row_bytes, int k, const int32_t * __restrict__ tokens,
                               float * __restrict__ X) {
+    pdl_launch_dependents();
     const uint8_t * row = rows + (size_t) tokens[blockIdx.y] * row_bytes;
     float * out = X + (size_t) blockIdx.y * k;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) out[i] = dequant_elem(type, row, i);
@@ -52,6 +53,7 @@ struct QuantBatchArgs {
 __global__ void __launch_bounds__(512) k_quant_batch(const QuantBatchArgs a) {
     extern __shared__ __align__(16) uint8_t qb_smem[];
     __shared__ double red_smem[MV_MAX_WARPS];
+    pdl_launch_dependents();
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, W = blockDim.x >> 5;
     const ActSmem A = act_smem_carve(qb_smem, a.k, a.act_q8_0);
     const bool norm = a.norm_w != nullptr;
@@ -63,6 +65,7 @@ __global__ void __launch_bounds__(512) k_quant_batch(const QuantBatchArgs a) {
             if (b < a.k / 256) ldg8(a.norm_w + b * 256 + lane * 8, ww[u]);
         }
     }
+    pdl_wait();
     prologue_quantize<false, true>(a.X + (size_t) t * a.k, norm, a.eps, a.k, a.inv_k, a.act_q8_0, A, red_smem, ww, []() {}, W);
     __syncthreads();
     const int n256 = a.k / 256, rb = pb_record_bytes(a.act_q8_0, a.with_as);
@@ -91,6 +94,8 @@ __global__ void __launch_bounds__(512) k_quant_batch(const QuantBatchArgs a) {
 // ------------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_attn_softmax_rows(const AttnArgs a, int nz) {
     const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+    pdl_launch_dependents();
+    pdl_wait();
     if (row >= nz * a.n_head) return;
     const int z = row / a.n_head, h = row - z * a.n_head;
     const int n_pad = (a.n_kv_override + z + 31) / 32 * 32, n16 = n_pad / 16;
@@ -142,6 +147,8 @@ __global__ void __launch_bounds__(SMX_THREADS) k_attn_softmax_block(const AttnAr
     __shared__ float wmax[SMX_THREADS / 32], gsum[G * SMX_THREADS];
     __shared__ float inv_s;
     const int tid = threadIdx.x, lane = tid & 31, row = blockIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     const int z = row / a.n_head, h = row - z * a.n_head;
     const int n_pad = (a.n_kv_override + z + 31) / 32 * 32, n16 = n_pad / 16;
     float * S = a.S + (size_t) z * a.zs + (size_t) h * a.s_stride;
@@ -234,6 +241,8 @@ __global__ void __launch_bounds__(SCB_KEYS, 3) k_attn_scores_batch(const AttnArg
     constexpr int HD = 128;
     extern __shared__ __align__(16) uint8_t scb_dyn[];
     float * qs = reinterpret_cast<float *>(scb_dyn);                          // [tq * GQA][HD]
+    pdl_launch_dependents();
+    pdl_wait();
     const int g = blockIdx.x, tile = blockIdx.y, z0 = blockIdx.z * tq, tid = threadIdx.x;
     const int ntok = min(tq, nz - z0);
     const int n_kv_last = a.n_kv_override + z0 + ntok - 1;
@@ -300,6 +309,8 @@ template <int GQA>
 __global__ void __launch_bounds__(PVB_THREADS, 2) k_attn_pv_batch(const AttnArgs a, int nz) {
     constexpr int HD = 128, TQ = PVB_ROWS / GQA;
     extern __shared__ __align__(16) uint8_t pvb_dyn[];
+    pdl_launch_dependents();
+    pdl_wait();
     const int g = blockIdx.x, z0 = blockIdx.y * TQ, tid = threadIdx.x, c = tid >> 4, dg = tid & 15;     // dims 8 dg .. 8 dg + 7
     const int ntok = min(TQ, nz - z0);
     const int n_kv_last = a.n_kv_override + z0 + ntok - 1;     // cells attended by the CTA's last token
@@ -467,6 +478,8 @@ __global__ void __launch_bounds__(PB_WARPS * 32, 1) k_matmul_batch(const __grid_
     __shared__ __align__(8) uint64_t bars[2 * PB_STAGES];      // full[stage], empty[stage]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int chunk = blockIdx.x, unit = blockIdx.y;
+    pdl_launch_dependents();
+    pdl_wait();
     const int rb = pb_record_bytes(a.act_q8_0, a.with_as), st_tiles = pb_step_tiles(a.act_q8_0);
     const size_t w_bytes = ((size_t) max_tile_bytes * st_tiles + 127) / 128 * 128;
     const size_t stage_bytes = w_bytes + (size_t) PB_CHUNK * rb;

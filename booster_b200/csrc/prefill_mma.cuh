@@ -321,6 +321,8 @@ __device__ __forceinline__ void mb_mma_mins5(const uint8_t * As, uint32_t mins_o
 __global__ void __launch_bounds__(MB_WARPS * 32, 1) k_mma_batch(const __grid_constant__ MatmulBatchArgs a) {
     extern __shared__ __align__(128) uint8_t mb_smem[];
     __shared__ __align__(8) uint64_t bars[MB_MAX_STAGES];
+    pdl_launch_dependents();
+    pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int chunk = blockIdx.x, unit0 = 2 * blockIdx.y;
     const UnitDesc ud = pb_describe_unit(a, unit0), ud1 = pb_describe_unit(a, unit0 + 1);   // same segment (host: even unit counts)

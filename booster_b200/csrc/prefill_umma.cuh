@@ -188,6 +188,7 @@ __device__ __forceinline__ void uq_write_records(const ActSmem & A, int n256, ui
 __global__ void __launch_bounds__(512) k_quant_batch_mma(const QuantBatchArgs a) {
     extern __shared__ __align__(16) uint8_t qb_smem[];
     __shared__ double red_smem[MV_MAX_WARPS];
+    pdl_launch_dependents();
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, W = blockDim.x >> 5;
     const ActSmem A = act_smem_carve(qb_smem, a.k, a.act_q8_0);
     const bool norm = a.norm_w != nullptr;
@@ -199,6 +200,7 @@ __global__ void __launch_bounds__(512) k_quant_batch_mma(const QuantBatchArgs a)
             if (b < a.k / 256) ldg8(a.norm_w + b * 256 + lane * 8, ww[u]);
         }
     }
+    pdl_wait();
     prologue_quantize<false, true>(a.X + (size_t) t * a.k, norm, a.eps, a.k, a.inv_k, a.act_q8_0, A, red_smem, ww, []() {}, W);
     __syncthreads();
     if (a.layout == 3) uq_write_records(A, a.k / 256, a.rec, t, lane, warp, W);
@@ -388,6 +390,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch(const __grid_const
     float * outs = reinterpret_cast<float *>(um_smem + 2 * UM_A_MINS);
     uint8_t * stages = um_smem + UM_FIXED_SMEM;
     const int n_steps = a.tiles_unit, n_stages = a.mb_stages, n_tiles = a.um_row_tiles * a.um_tok_tiles;
+    pdl_launch_dependents();
     const uint32_t b_full = smem_u32(&bars[0]), b_empty = b_full + 8 * UM_MAX_STAGES, b_afull = b_empty + 8 * UM_MAX_STAGES, b_dfull = b_afull + 16, b_dfree = b_dfull + 16;
     if (tid == 0) {
         failed_s = 0;
@@ -400,27 +403,38 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch(const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (warp != 12) pdl_wait();                 // (warp 12 waits behind its first copies)
 
     if (warp >= 12) {
         regs_dec<24>();
         if (warp == 12) {                       // bulk copies: super-block after super-block, over all tiles of the CTA
             uint32_t s = 0, par = 1;            // (a stage's first use waits for nothing)
+            // one super-block of a tile -> stage s: the raw tiles and (a later call for those copied ahead) the records
+            auto copy = [&](const UmTile & t, int tt, int step, uint32_t s, bool raw, bool recs) {
+                const uint32_t rc = (uint32_t) um_rec_copy_bytes(t.type), dst = smem_u32(stages) + s * a.mb_stage_bytes, bar = b_full + 8 * s;
+                if (raw) {
+                    const uint8_t * src = t.tiles + (size_t) step * t.bytes;
+                    mbar_expect_tx(bar, (uint32_t) t.n_units * t.bytes + rc);
+                    for (int u = 0; u < t.n_units; u++) bulk_g2s(dst + u * a.mb_raw_stride, src + (size_t) u * n_steps * t.bytes, t.bytes, bar);
+                }
+                if (recs) bulk_g2s(dst + 4 * a.mb_raw_stride, a.rec + ((size_t) tt * n_steps + step) * UM_REC_BYTES, rc, bar);
+            };
+            const int early = min(n_stages, n_steps);
             for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
                 const int rt = tile / a.um_tok_tiles, tt = tile - rt * a.um_tok_tiles;
                 const UmTile t = um_tile(a, rt);
-                const uint32_t rc = (uint32_t) um_rec_copy_bytes(t.type), us = (uint32_t) n_steps * t.bytes;
-                const uint8_t * src = t.tiles, * rec = a.rec + (size_t) tt * n_steps * UM_REC_BYTES;
+                const bool first = tile == (int) blockIdx.x;
+                if (first) {                    // weights wait for nobody; the records are the previous kernel's
+                    if (elect_one()) { for (int i = 0; i < early; i++) copy(t, tt, i, i, true, false); }
+                    __syncwarp();
+                    pdl_wait();
+                }
 #pragma unroll 1
                 for (int step = 0; step < n_steps; step++) {
-                    um_wait(b_empty + 8 * s, par, failed, a.err);
-                    if (elect_one() && !*failed) {
-                        const uint32_t dst = smem_u32(stages) + s * a.mb_stage_bytes, bar = b_full + 8 * s;
-                        mbar_expect_tx(bar, (uint32_t) t.n_units * t.bytes + rc);
-                        for (int u = 0; u < t.n_units; u++) bulk_g2s(dst + u * a.mb_raw_stride, src + (size_t) u * us, t.bytes, bar);
-                        bulk_g2s(dst + 4 * a.mb_raw_stride, rec, rc, bar);
-                    }
+                    const bool ahead = first && step < early;
+                    if (!ahead) um_wait(b_empty + 8 * s, par, failed, a.err);
+                    if (elect_one() && !*failed) copy(t, tt, step, s, !ahead, true);
                     __syncwarp();
-                    src += t.bytes; rec += UM_REC_BYTES;
                     if (++s == (uint32_t) n_stages) { s = 0; par ^= 1u; }
                 }
             }

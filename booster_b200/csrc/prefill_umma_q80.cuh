@@ -77,15 +77,18 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch_q80(const __grid_c
     const uint32_t b_full = smem_u32(&bars[0]), b_empty = b_full + 8 * UQ_STAGES, b_pfull = b_empty + 8 * UQ_STAGES, b_pempty = b_pfull + 8 * UQ_SLOTS;
     const uint32_t b_dfull = b_pempty + 8 * UQ_SLOTS, b_dfree = b_dfull + 24;
     // four blocks of a tile -> stage s
-    auto copy = [&](const UmTile & t, int tt, int step, uint32_t s) {
+    auto copy = [&](const UmTile & t, int tt, int step, uint32_t s, bool raw, bool recs) {
         const uint32_t dst = smem_u32(stages) + s * UQ_STAGE, bar = b_full + 8 * s;
-        const uint8_t * src = t.tiles + (size_t) step * UQ_RAW;
-        mbar_expect_tx(bar, (uint32_t) t.n_units * UQ_RAW + UQ_STAGE_BLOCKS * UQ_BLOCK_REC);
-        for (int u = 0; u < t.n_units; u++) bulk_g2s(dst + u * UQ_RAW, src + (size_t) u * a.tiles_unit * 1088, UQ_RAW, bar);
-        bulk_g2s(dst + 4 * UQ_RAW, a.rec + ((size_t) tt * a.tiles_unit + step * UQ_STAGE_BLOCKS) * UQ_BLOCK_REC, UQ_STAGE_BLOCKS * UQ_BLOCK_REC, bar);
+        if (raw) {
+            const uint8_t * src = t.tiles + (size_t) step * UQ_RAW;
+            mbar_expect_tx(bar, (uint32_t) t.n_units * UQ_RAW + UQ_STAGE_BLOCKS * UQ_BLOCK_REC);
+            for (int u = 0; u < t.n_units; u++) bulk_g2s(dst + u * UQ_RAW, src + (size_t) u * a.tiles_unit * 1088, UQ_RAW, bar);
+        }
+        if (recs) bulk_g2s(dst + 4 * UQ_RAW, a.rec + ((size_t) tt * a.tiles_unit + step * UQ_STAGE_BLOCKS) * UQ_BLOCK_REC, UQ_STAGE_BLOCKS * UQ_BLOCK_REC, bar);
     };
     const int early = min(UQ_STAGES, n_steps);
-    if (tid == 12 * 32) {                       // the first tile's first copies are on their way while the operand is cleared
+    pdl_launch_dependents();
+    if (tid == 12 * 32) {                       // the first tile's first weights are on their way while the operand is cleared; they wait for nobody
         failed_s = 0;
         for (int s = 0; s < UQ_STAGES; s++) { mbar_init(b_full + 8 * s, 1); mbar_init(b_empty + 8 * s, 13); }
         for (int s = 0; s < UQ_SLOTS; s++) { mbar_init(b_pfull + 8 * s, 5); mbar_init(b_pempty + 8 * s, 2); }
@@ -94,7 +97,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch_q80(const __grid_c
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         const int rt = blockIdx.x / a.um_tok_tiles;
         const UmTile t = um_tile(a, rt);
-        for (int s = 0; s < early; s++) copy(t, blockIdx.x - rt * a.um_tok_tiles, s, s);
+        for (int s = 0; s < early; s++) copy(t, blockIdx.x - rt * a.um_tok_tiles, s, s, true, false);
     }
     for (int i = tid; i < UQ_SLOTS * UQ_B_SLOT / 16; i += UM_THREADS) reinterpret_cast<uint4 *>(bop)[i] = make_uint4(0u, 0u, 0u, 0u);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -102,6 +105,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch_q80(const __grid_c
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();
 
     if (warp >= 12) {
         regs_dec<24>();
@@ -112,11 +116,10 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch_q80(const __grid_c
                 const UmTile t = um_tile(a, rt);
 #pragma unroll 1
                 for (int step = 0; step < n_steps; step++) {
-                    if (tile != blockIdx.x || step >= early) {
-                        um_wait(b_empty + 8 * s, par, failed, a.err);
-                        if (elect_one() && !*failed) copy(t, tt, step, s);
-                        __syncwarp();
-                    }
+                    const bool ahead = tile == (int) blockIdx.x && step < early;
+                    if (!ahead) um_wait(b_empty + 8 * s, par, failed, a.err);
+                    if (elect_one() && !*failed) copy(t, tt, step, s, !ahead, true);
+                    __syncwarp();
                     if (++s == UQ_STAGES) { s = 0; par ^= 1u; }
                 }
             }
