@@ -24,6 +24,7 @@
 #define B200_TOKEN_KERNEL 1      // 0: build without the persistent per-token kernel (A/B: code size of the module)
 #endif
 #include "token_kernel.cuh"
+#include "matvec_q80.cuh"
 #include "prefill.cuh"
 #include "prefill_mma.cuh"
 #include "prefill_umma_q80.cuh"
@@ -714,6 +715,7 @@ static unsigned long long * trace_slot(b200_ctx * c, int ctas) {
 // combination with the most concurrently active warps (every unit resident in as few waves as possible), then the
 // deepest ring that still fits the shared memory. Pure host arithmetic (b200_op_launch_shape exposes it to the tests).
 static constexpr size_t MV_SMEM_BUDGET = 227 * 1024 - 512;    // dynamic shared memory of k_matvec
+static constexpr size_t QV_SMEM_BUDGET = 227 * 1024 - 1024;   // of k_matvec_q80, beside its barriers
 static void pick_launch_shape(int n_units, int tiles_unit, int k, bool norm, int act_q8_0, int stage_bytes, int nv, int sm_count,
                               int & bestW, int & bestG, int & bestS, size_t budget = MV_SMEM_BUDGET) {
     const size_t act_bytes = act_smem_bytes(k, act_q8_0);
@@ -774,9 +776,40 @@ static size_t shape_matvec(MatvecArgs & a, int epi, int sm_count, size_t budget)
     return smem;
 }
 
+// one token's product with a Q8_0 matrix on k_matvec_q80: every row of it in Q8_0, and with a norm a vector that one pass of the block's warps holds
+static bool matvec_q80_takes(const MatvecArgs & a) {
+    for (int i = 0; i < a.n_seg; i++) if (a.seg[i].type != T_Q8_0) return false;
+    return a.act_q8_0 && (a.norm_w == nullptr || a.k <= PRO_U * QV_WARPS * 256) && (size_t) qv_fixed_bytes(a.k) + (size_t) QV_TEAMS * 2 * 8 * 1088 <= QV_SMEM_BUDGET;
+}
+template <int NB>
+static void launch_matvec_q80_t(b200_ctx * c, MatvecArgs & a) {
+    const int grid = std::max(1, std::min(a.n_units, c->sm_count));
+    a.groups_per_cta = a.n_units > grid ? QV_TEAMS : 1;       // one unit per block: one team has the whole ring
+    a.stages = (int) std::min<size_t>(QV_MAX_STAGES, (QV_SMEM_BUDGET - qv_fixed_bytes(a.k)) / ((size_t) a.groups_per_cta * NB * 1088));
+    const size_t smem = (size_t) qv_fixed_bytes(a.k) + (size_t) a.groups_per_cta * a.stages * NB * 1088;
+    static size_t attr[64] = {0}, attr_t[64] = {0};
+    raise_smem(k_matvec_q80<NB, false>, smem, attr, c->device);
+    raise_smem(k_matvec_q80<NB, true>, smem, attr_t, c->device);
+    a.trace = trace_slot(c, grid);
+    launch_fwd(a.trace ? k_matvec_q80<NB, true> : k_matvec_q80<NB, false>, dim3((unsigned) grid), dim3(QV_THREADS), smem, c->st, a);
+    c->launches++;
+}
+static void launch_matvec_q80(b200_ctx * c, MatvecArgs a, int epi) {
+    a.epi = epi;
+    a.tiles_unit = a.seg[0].tiles_unit;
+    for (int i = 0; i < a.n_seg; i++)
+        if (a.seg[i].tiles_unit != a.tiles_unit) throw std::runtime_error("segments of one launch must share the unit shape");
+    a.inv_k = (a.k & (a.k - 1)) == 0 ? 1.0 / (double) a.k : 0.0;
+    a.err = c->pb.err;
+    // stages of 16 blocks where k allows it: waits and arrivals are paid half as often as with 8 (whole token of an 8B model's 8 layers: 521 and 607 us); 32 leave
+    // the large matrices a shorter ring (533 us)
+    if (a.tiles_unit % 16 == 0) launch_matvec_q80_t<16>(c, a);
+    else launch_matvec_q80_t<8>(c, a);
+}
 static void launch_matvec(b200_ctx * c, const MatvecArgs & a_in, int epi) {
     ProfScope ps(c);
     MatvecArgs a = a_in;
+    if (matvec_q80_takes(a)) return launch_matvec_q80(c, a, epi);
     const size_t smem = shape_matvec(a, epi, c->sm_count, MV_SMEM_BUDGET);
     static int prefill_env = -1;
     if (prefill_env < 0) { const char * e = getenv("BOOSTER_B200_PREFILL"); prefill_env = e ? atoi(e) : 0; }
@@ -2796,8 +2829,10 @@ extern "C" int b200_op_mul_mat_vec(int type, const void * w, int64_t n_rows, int
         const DevMat & d = om.d;
         DBuf dx((size_t) k * 4), dy((size_t) rows_pad * 4);
         CU(cudaMemcpyAsync(dx.p, x, (size_t) k * 4, cudaMemcpyHostToDevice, st));
-        b200_ctx tmp;   // only st / sm_count / launches are used by launch_matvec
+        b200_ctx tmp;   // only st / sm_count / launches / pb.err are used by launch_matvec
         tmp.st = st;
+        const std::shared_ptr<int32_t> flag = pinned_token_and_flag();
+        tmp.pb.err = flag.get() + 1;
         int dev = 0; CU(cudaGetDevice(&dev));
         cudaDeviceProp prop; CU(cudaGetDeviceProperties(&prop, dev));
         tmp.sm_count = prop.multiProcessorCount;
@@ -2809,6 +2844,7 @@ extern "C" int b200_op_mul_mat_vec(int type, const void * w, int64_t n_rows, int
         CU(cudaGetLastError());
         CU(cudaMemcpyAsync(y, dy.p, (size_t) n_rows * 4, cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
+        pb_check(&tmp);
         return 0;
     } catch (const std::exception & e) { return set_err(e.what()); }
 }

@@ -128,6 +128,7 @@ struct MatvecArgs {
     PfRange pf[PF_RANGES];     // L2 look-ahead for the kernels that follow (bytes == 0: unused)
     const float * warm_x;      // B200_WARM: constant vector of k floats for the dry run of the prologue (nullptr: no dry run)
     unsigned long long * trace; // nullptr unless b200_trace_token is running
+    int * err;                 // raised when a bounded wait ran out (the host reads it after its synchronisation)
 };
 
 static constexpr int MV_MAX_WARPS = 16;                     // one persistent CTA per SM, 8..16 warps (host picks)
@@ -525,6 +526,22 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
     } while (!ok);
 }
 // global -> shared bulk copy (TMA engine, no registers, no per-lane addressing); completes `bytes` on `bar`
+// mbarrier wait with an iteration limit: past it *failed is raised (every other wait of the CTA then gives up too), *err tells the host, and
+// the kernel runs to its end without storing
+__device__ __forceinline__ bool um_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void um_wait(uint32_t bar, uint32_t parity, volatile int * failed, int * err) {
+    if (um_try(bar, parity)) return;
+#pragma unroll 1
+    for (uint32_t spins = 0; spins < (1u << 22); spins++)
+        if (um_try(bar, parity) || *failed) return;
+    *failed = 1;
+    atomicExch_system(err, 1);
+}
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");

@@ -107,22 +107,6 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 __device__ __forceinline__ void tmem_ld8_ready(uint32_t (&r)[8]) {
     asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
 }
-// mbarrier wait with an iteration limit: past it *failed is raised (every other wait of the CTA then gives up too), *err tells the host, and
-// the kernel runs to its end without storing
-__device__ __forceinline__ bool um_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ void um_wait(uint32_t bar, uint32_t parity, volatile int * failed, int * err) {
-    if (um_try(bar, parity)) return;
-#pragma unroll 1
-    for (uint32_t spins = 0; spins < (1u << 22); spins++)
-        if (um_try(bar, parity) || *failed) return;
-    *failed = 1;
-    atomicExch_system(err, 1);
-}
 template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(N)); }
 template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(N)); }
 

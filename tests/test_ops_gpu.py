@@ -240,6 +240,22 @@ def test_mul_mat_batch_q8_0_edges(shape):
         assert np.array_equal(y[i], yr), f"token {i}: max abs diff {np.abs(y[i] - yr).max()}"
 
 
+@pytest.mark.parametrize("shape", [(32, 256), (96, 768), (4736, 512), (4768, 256), (9504, 768), (14240, 1280), (64, 14336), (160, 17408)])
+def test_mul_mat_vec_q8_0_edges(shape):
+    """k_matvec_q80 where its teams and rings end: one stage, stages of eight and of 16 blocks, as many units of 32 rows as SMs and one more (a block's second team), more
+    than both teams take at once, a ring that goes round, a vector of more than one pass of the quantizer — the reference's bits"""
+    n, k = shape
+    rng = np.random.default_rng(n + k)
+    w = _extreme_blocks("Q8_0", n, k, rng).reshape(n, -1)
+    w[1::4, :34] = 0
+    w[2::4, 0:2] = np.array([6e-8], np.float16).view(np.uint8)
+    x = (rng.standard_normal(k) * rng.choice([1e-6, 1.0, 30.0], size=k)).astype(np.float32)
+    x[32:64] = 0.0
+    y = engine.op_mul_mat_vec(TYPES["Q8_0"], w.reshape(-1), n, k, x)
+    yr = port.mul_mat_vec(TYPES["Q8_0"], w.reshape(-1), n, k, x)
+    assert np.array_equal(y, yr), f"max abs diff {np.abs(y - yr).max()}"
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0"])
 def test_mul_mat_batch_kernel_variants(name, mode, prefill_mma):
