@@ -516,6 +516,18 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch(const __grid_const
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
             const int rt = tile / a.um_tok_tiles, tt = tile - rt * a.um_tok_tiles;
             const UmTile t = um_tile(a, rt);
+            if (tt * UM_NT + 16 * th >= a.T) {                       // no tokens in this half: only the hand-overs
+#pragma unroll 1
+                for (int step = 0; step < n_steps; step++, it++) {
+                    for (int h = 0; h < 2; h++) {
+                        um_wait(b_dfull + 8 * h, it & 1, failed, a.err);
+                        if (lane == 0) mbar_arrive(b_dfree + 8 * h);
+                    }
+                    if (lane == 0) mbar_arrive(b_empty + 8 * st);
+                    if (++st == (uint32_t) n_stages) { st = 0; fpar ^= 1u; }
+                }
+                continue;
+            }
             auto run = [&](auto tag) {
                 constexpr int TYPE = decltype(tag)::value;
                 constexpr int NM = TYPE == T_Q4_K ? 4 : TYPE == T_Q5_K ? 1 : 0;
