@@ -25,6 +25,7 @@
 #endif
 #include "token_kernel.cuh"
 #include "matvec_q80.cuh"
+#include "matvec_kq.cuh"
 #include "prefill.cuh"
 #include "prefill_mma.cuh"
 #include "prefill_umma_q80.cuh"
@@ -716,6 +717,7 @@ static unsigned long long * trace_slot(b200_ctx * c, int ctas) {
 // deepest ring that still fits the shared memory. Pure host arithmetic (b200_op_launch_shape exposes it to the tests).
 static constexpr size_t MV_SMEM_BUDGET = 227 * 1024 - 512;    // dynamic shared memory of k_matvec
 static constexpr size_t QV_SMEM_BUDGET = 227 * 1024 - 1024;   // of k_matvec_q80, beside its barriers
+static constexpr size_t KV_SMEM_BUDGET = 227 * 1024 - 2560;   // of k_matvec_kq, beside its barriers
 static void pick_launch_shape(int n_units, int tiles_unit, int k, bool norm, int act_q8_0, int stage_bytes, int nv, int sm_count,
                               int & bestW, int & bestG, int & bestS, size_t budget = MV_SMEM_BUDGET) {
     const size_t act_bytes = act_smem_bytes(k, act_q8_0);
@@ -794,22 +796,69 @@ static void launch_matvec_q80_t(b200_ctx * c, MatvecArgs & a) {
     launch_fwd(a.trace ? k_matvec_q80<NB, true> : k_matvec_q80<NB, false>, dim3((unsigned) grid), dim3(QV_THREADS), smem, c->st, a);
     c->launches++;
 }
-static void launch_matvec_q80(b200_ctx * c, MatvecArgs a, int epi) {
+// what k_matvec_q80 and k_matvec_kq share of a launch's derived fields
+static void matvec_lanes_args(const b200_ctx * c, MatvecArgs & a, int epi) {
     a.epi = epi;
     a.tiles_unit = a.seg[0].tiles_unit;
     for (int i = 0; i < a.n_seg; i++)
         if (a.seg[i].tiles_unit != a.tiles_unit) throw std::runtime_error("segments of one launch must share the unit shape");
     a.inv_k = (a.k & (a.k - 1)) == 0 ? 1.0 / (double) a.k : 0.0;
     a.err = c->pb.err;
+}
+static void launch_matvec_q80(b200_ctx * c, MatvecArgs a, int epi) {
+    matvec_lanes_args(c, a, epi);
     // stages of 16 blocks where k allows it: waits and arrivals are paid half as often as with 8 (whole token of an 8B model's 8 layers: 521 and 607 us); 32 leave
     // the large matrices a shorter ring (533 us)
     if (a.tiles_unit % 16 == 0) launch_matvec_q80_t<16>(c, a);
     else launch_matvec_q80_t<8>(c, a);
 }
+// one token's product with K-quant matrices on k_matvec_kq: with a norm a vector that one pass of the block's warps holds, and room for two stages per team
+static bool matvec_kq_q6(const MatvecArgs & a) {
+    for (int i = 0; i < a.n_seg; i++) if (a.seg[i].type == T_Q6_K) return true;
+    return false;
+}
+static int matvec_kq_tile(const MatvecArgs & a) {
+    int sb = 0;
+    for (int i = 0; i < a.n_seg; i++) sb = std::max(sb, tile_bytes_of(a.seg[i].type));
+    return sb;
+}
+// rows per thread: with more units of 32 rows per SM than the teams of one row per thread are, two: the vector's words are then read once for both (gate|up 14.9 us, with one
+// 16.7). With fewer units two rows per thread halve the warps at work.
+static int matvec_kq_rows(const MatvecArgs & a, int sm_count) { return a.n_units > kv_teams(1) * sm_count ? 2 : 1; }
+static bool matvec_kq_takes(const MatvecArgs & a) {
+    for (int i = 0; i < a.n_seg; i++) if (a.seg[i].type != T_Q4_K && a.seg[i].type != T_Q5_K && a.seg[i].type != T_Q6_K) return false;
+    return !a.act_q8_0 && (a.norm_w == nullptr || a.k <= PRO_U * KV_WARPS * 256)
+        && (size_t) kv_act_bytes(a.k, matvec_kq_q6(a)) + (size_t) kv_teams(2) * 2 * ((matvec_kq_tile(a) + 127) / 128 * 128) <= KV_SMEM_BUDGET;
+}
+template <int U, int R, int NB>
+static void launch_matvec_kq_t(b200_ctx * c, MatvecArgs & a) {
+    const int grid = std::max(1, std::min(a.n_units, c->sm_count));
+    const size_t fixed = (size_t) kv_act_bytes(a.k, matvec_kq_q6(a));
+    a.groups_per_cta = std::min(kv_teams(R), (a.n_units + grid - 1) / grid);      // teams that have a unit share the ring's memory
+    a.stage_bytes = (NB * matvec_kq_tile(a) + 127) / 128 * 128;
+    // no more shared memory and warps than the launch uses: its blocks then start beside those of the kernel before (wo beside soft-max . V) and have weights on their way
+    const int steps = (a.n_units + grid * a.groups_per_cta - 1) / (grid * a.groups_per_cta) * (a.tiles_unit / NB);
+    a.stages = (int) std::min<size_t>(std::min(KV_MAX_STAGES, steps), (KV_SMEM_BUDGET - fixed) / ((size_t) a.groups_per_cta * a.stage_bytes));
+    const size_t smem = fixed + (size_t) a.groups_per_cta * a.stages * a.stage_bytes;
+    static size_t attr[64] = {0}, attr_t[64] = {0};
+    raise_smem(k_matvec_kq<U, R, NB, false>, smem, attr, c->device);
+    raise_smem(k_matvec_kq<U, R, NB, true>, smem, attr_t, c->device);
+    a.trace = trace_slot(c, grid);
+    launch_fwd(a.trace ? k_matvec_kq<U, R, NB, true> : k_matvec_kq<U, R, NB, false>, dim3((unsigned) grid), dim3((unsigned) (KV_WARPS + a.groups_per_cta) * 32), smem, c->st, a);
+    c->launches++;
+}
+static void launch_matvec_kq(b200_ctx * c, MatvecArgs a, int epi) {
+    matvec_lanes_args(c, a, epi);
+    const bool one = a.k <= KV_WARPS * 256;                     // a warp has one block of the vector
+    if (matvec_kq_rows(a, c->sm_count) == 2) { if (one) launch_matvec_kq_t<1, 2, 1>(c, a); else launch_matvec_kq_t<PRO_U, 2, 1>(c, a); }
+    else if (a.tiles_unit % 2 == 0) { if (one) launch_matvec_kq_t<1, 1, 2>(c, a); else launch_matvec_kq_t<PRO_U, 1, 2>(c, a); }
+    else { if (one) launch_matvec_kq_t<1, 1, 1>(c, a); else launch_matvec_kq_t<PRO_U, 1, 1>(c, a); }
+}
 static void launch_matvec(b200_ctx * c, const MatvecArgs & a_in, int epi) {
     ProfScope ps(c);
     MatvecArgs a = a_in;
     if (matvec_q80_takes(a)) return launch_matvec_q80(c, a, epi);
+    if (matvec_kq_takes(a)) return launch_matvec_kq(c, a, epi);
     const size_t smem = shape_matvec(a, epi, c->sm_count, MV_SMEM_BUDGET);
     static int prefill_env = -1;
     if (prefill_env < 0) { const char * e = getenv("BOOSTER_B200_PREFILL"); prefill_env = e ? atoi(e) : 0; }

@@ -794,8 +794,9 @@ __device__ __forceinline__ UnitDesc describe_unit(const MatvecArgs & a, int unit
 // The code of a unit is specialised on the unit's block type.
 // ------------------------------------------------------------------------------------------------------------
 // the row's epilogue (one call per unit; out of line: four block types share one copy)
-__device__ __noinline__ void matvec_epilogue(const MatvecArgs & a, float val, int row, int lane, float pre0, float pre1, int cell) {
+__device__ __noinline__ void matvec_epilogue(const MatvecArgs & a, float val, int row, int lane, float pre0, float pre1, int cell, bool own = true) {
     const float oth = __shfl_xor_sync(0xffffffffu, val, 1);    // partner row (2i <-> 2i+1)
+    if (!own) return;
     if (a.epi == EPI_STORE) {
         a.out[row] = val;
     } else if (a.epi == EPI_RESID) {

@@ -38,6 +38,59 @@ __device__ __forceinline__ void qv_quantize(const float (&v)[8], int lane, int b
     if ((lane & 3) == 0) dx[b] = __half2float(__float2half_rn(d));
 }
 
+// um_wait for a warp that has time: between two looks it sleeps, and leaves its scheduler's issue slots to the warps that add
+__device__ __forceinline__ void um_wait_asleep(uint32_t bar, uint32_t parity, volatile int * failed, int * err) {
+#pragma unroll 1
+    for (uint32_t looks = 0; looks < (1u << 22); looks++) {
+        if (um_try(bar, parity) || *failed) return;
+        __nanosleep(150);
+    }
+    *failed = 1;
+    atomicExch_system(err, 1);
+}
+// The copying warp of a team: its units' blocks, NB to a stage, into the team's ring from before the dependency wait on; weights wait for nobody. Passes the block's
+// barrier when the ring is full or nothing is left to copy: the consumers may start. full: one arrival and the stage's bytes; empty: one arrival per consuming warp.
+template <int NB, int TW>       // TW: consuming warps
+__device__ __forceinline__ void qv_copy(const MatvecArgs & a, int lane, bool has_team, int first, int stride, int S, uint32_t slot_bytes, uint32_t dst,
+                                        uint32_t b_full, uint32_t b_empty, volatile int * failed) {
+    if (lane == 0 && has_team) {
+        for (int s = 0; s < S; s++) { mbar_init(b_full + 8 * s, 1); mbar_init(b_empty + 8 * s, TW); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    const int n_steps = a.tiles_unit / NB;
+    int s = 0, n = 0;
+    uint32_t par = 1;
+    const uint64_t pol = l2_policy_evict_first();
+    bool synced = false;
+    if (has_team) {
+        for (int u = first; u < a.n_units; u += stride) {
+            const UnitDesc ud = describe_unit(a, u);
+            const uint32_t bytes = NB * ud.bytes;
+            const uint8_t * src = ud.tiles;
+#pragma unroll 1
+            for (int st = 0; st < n_steps; st++) {
+                if (n >= S) {
+                    if (!synced) { __syncthreads(); synced = true; }
+                    um_wait_asleep(b_empty + 8 * s, par, failed, a.err);
+                }
+                if (lane == 0 && !(n >= S && *failed)) {
+                    mbar_expect_tx(b_full + 8 * s, bytes);
+                    bulk_g2s_hint(dst + (uint32_t) s * slot_bytes, src, bytes, b_full + 8 * s, pol);
+                }
+                __syncwarp();
+                src += bytes;
+                n++;
+                if (++s == S) { s = 0; par ^= 1u; }
+            }
+        }
+    }
+    if (!synced) __syncthreads();
+    pdl_wait();
+    if (*failed) { for (int i = 0; i < 1000; i++) __nanosleep(1000); }      // copies nobody waited for end before the block does
+}
+
 // NB: blocks per stage of the ring
 template <int NB, bool TR>
 __global__ void __launch_bounds__(QV_THREADS, 1) k_matvec_q80(const __grid_constant__ MatvecArgs a) {
@@ -60,42 +113,8 @@ __global__ void __launch_bounds__(QV_THREADS, 1) k_matvec_q80(const __grid_const
     if (tid == 0) failed_s = 0;                                 // (first read behind the block's barrier)
     trace_mark<TR>(a.trace, 0);
     pdl_launch_dependents();
-    if (warp >= QV_WARPS) {                                     // the team's copies, stage after stage over its units; weights wait for nobody
-        if (lane == 0 && team < n_teams) {
-            for (int s = 0; s < S; s++) { mbar_init(b_full + 8 * s, 1); mbar_init(b_empty + 8 * s, 8); }
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        }
-        __syncwarp();
-        int s = 0, n = 0;
-        uint32_t par = 1;
-        const uint64_t pol = l2_policy_evict_first();
-        const uint32_t dst = smem_u32(slots);
-        bool synced = false;
-        if (team < n_teams) {
-            for (int u = first; u < a.n_units; u += stride) {
-                const UnitDesc ud = describe_unit(a, u);
-#pragma unroll 1
-                for (int st = 0; st < n_steps; st++) {
-                    if (n >= S) {
-                        if (!synced) { __syncthreads(); synced = true; }     // (the ring is full: the consumers may start)
-                        um_wait(b_empty + 8 * s, par, failed, a.err);
-                    }
-                    if (lane == 0 && !(n >= S && *failed)) {
-                        mbar_expect_tx(b_full + 8 * s, STAGE);
-                        bulk_g2s_hint(dst + (uint32_t) s * STAGE, ud.tiles + (size_t) st * STAGE, STAGE, b_full + 8 * s, pol);
-                    }
-                    __syncwarp();
-                    n++;
-                    if (++s == S) { s = 0; par ^= 1u; }
-                }
-            }
-        }
-        if (!synced) __syncthreads();
-        pdl_wait();
-        if (*failed) { for (int i = 0; i < 1000; i++) __nanosleep(1000); }      // copies nobody waited for end before the block does
-        return;
-    }
+    if (warp >= QV_WARPS)
+        return qv_copy<NB, 8>(a, lane, team < n_teams, first, stride, S, STAGE, smem_u32(slots), b_full, b_empty, failed);
     // ---- the vector: norm weights are constants and requested ahead of the wait; four blocks of 256 per warp and pass, their loads together
     const bool norm = a.norm_w != nullptr;
     const int n256 = a.k / 256;

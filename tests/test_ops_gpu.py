@@ -256,6 +256,24 @@ def test_mul_mat_vec_q8_0_edges(shape):
     assert np.array_equal(y, yr), f"max abs diff {np.abs(y - yr).max()}"
 
 
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K"])
+@pytest.mark.parametrize("shape", [(32, 256), (96, 768), (4736, 512), (4768, 256), (9504, 768), (14240, 1280), (64, 14336), (160, 17408), (4768, 9216)])
+def test_mul_mat_vec_k_quant_edges(name, shape):
+    """k_matvec_kq where its teams and rings end: one block of K, stages of one and of two blocks, as many units of 32 rows as SMs and one more (a block's second team),
+    more than both teams take at once, rings that go round, vectors of one and of several blocks per warp and of more than one pass, worst-case weights — the
+    reference's bits"""
+    n, k = shape
+    rng = np.random.default_rng(n + k)
+    w = _extreme_blocks(name, n, k, rng)
+    x = (rng.standard_normal(k) * rng.choice([1e-6, 1.0, 30.0], size=k)).astype(np.float32)
+    x[:256] = np.where(rng.random(256) < 0.5, 30.0, -30.0).astype(np.float32)
+    if k > 256:
+        x[256:512] = 0.0
+    y = engine.op_mul_mat_vec(TYPES[name], w.reshape(-1), n, k, x)
+    yr = port.mul_mat_vec(TYPES[name], w.reshape(-1), n, k, x)
+    assert np.array_equal(y, yr), f"max abs diff {np.abs(y - yr).max()}"
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0"])
 def test_mul_mat_batch_kernel_variants(name, mode, prefill_mma):
