@@ -117,6 +117,7 @@ struct MatvecArgs {
     int epi;                   // EPI_*: ONE kernel serves every mat-vec of the layer, so its code stays in the instruction cache
     // epilogue
     float * out;
+    float * out_host;          // EPI_STORE: the rows once more, into pinned host memory (nullptr: not)
     const float * resid;
     // EPI_QKV
     float * q_out;
@@ -799,6 +800,7 @@ __device__ __noinline__ void matvec_epilogue(const MatvecArgs & a, float val, in
     if (!own) return;
     if (a.epi == EPI_STORE) {
         a.out[row] = val;
+        if (a.out_host) a.out_host[row] = val;
     } else if (a.epi == EPI_RESID) {
         a.out[row] = __fadd_rn(val, pre0);                     // ggml_add(cur, inpSA / ffn_inp): llama.cpp:8865, 8901
     } else if (a.epi == EPI_SILU) {
@@ -1405,9 +1407,18 @@ __device__ __forceinline__ float dequant_elem(int type, const uint8_t * row, int
         default: return 0.f;
     }
 }
+// from_host: the step's scalars in pinned host memory; every block reads them there, block 0 puts them where the token's other kernels look (st). A copy node in front
+// of the kernels, and one behind them for the logits, cost a token 4 us (toy model: 80 -> 76): the copy engine starts behind the graph's dependency, not beside the kernels.
 __global__ void k_embed(int type, const uint8_t * __restrict__ rows, size_t row_bytes, int k,
-                        const DecodeState * __restrict__ st, int token_override, float * __restrict__ out) {
-    const int token = st ? st->token : token_override;
+                        DecodeState * st, const DecodeState * from_host, int token_override, float * __restrict__ out) {
+    __shared__ int32_t token_s;
+    if (from_host && threadIdx.x < 2) {
+        const int4 v = __ldcv(reinterpret_cast<const int4 *>(from_host) + threadIdx.x);
+        if (blockIdx.x == 0) reinterpret_cast<int4 *>(st)[threadIdx.x] = v;
+        if (threadIdx.x == 0) token_s = v.x;
+    }
+    if (from_host) __syncthreads();
+    const int token = from_host ? token_s : st ? st->token : token_override;
     const uint8_t * row = rows + (size_t) token * row_bytes;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) out[i] = dequant_elem(type, row, i);
 }
@@ -1661,15 +1672,14 @@ __global__ void __launch_bounds__(PV_DIMS * 16) k_attn_pv(const AttnArgs a) {
 //   grid (n_head_kv, HD / PVS_DIMS), block GQA * pvs_th(GQA) threads (16 chains x dim groups per head); shared: ps [GQA][n_pad] f32 | vs [v_chunk][8] f16
 // ------------------------------------------------------------------------------------------------------------
 static constexpr int PVS_DIMS = 8;            // dims per CTA: 8 halfs = one 16-byte cp.async per position
-// dims per thread: 1 (128 threads per head) up to GQA 4, 2 (64 threads per head) for GQA 8 — at most 512 threads
-__host__ __device__ constexpr int pvs_dpt(int gqa) { return gqa >= 8 ? 2 : 1; }
-__host__ __device__ constexpr int pvs_th(int gqa) { return 16 * (PVS_DIMS / pvs_dpt(gqa)); }
+static constexpr int PVS_SLOTS = 4;           // V slots of p_chunk positions each
+__host__ __device__ constexpr int pvs_th(int gqa) { return gqa >= 8 ? 64 : 128; }      // soft-max threads per head: at most 512 in all
+__host__ __device__ constexpr int pvs_hpt(int gqa) { return gqa >= 2 ? 2 : 1; }        // P.V: heads and dim pairs of a thread
 
 template <int GQA, bool TR>
 __global__ void __launch_bounds__(GQA * pvs_th(GQA)) k_attn_softmax_pv(const AttnArgs a) {
     constexpr int HD = 128;
-    constexpr int DPT = pvs_dpt(GQA);
-    constexpr int TH = pvs_th(GQA);                            // threads per head: 16 chains x (8 / DPT) dim groups
+    constexpr int TH = pvs_th(GQA);
     constexpr int NT = GQA * TH;
     constexpr int NW = TH / 32;
     extern __shared__ __align__(16) uint8_t sp_dyn[];
@@ -1678,27 +1688,26 @@ __global__ void __launch_bounds__(GQA * pvs_th(GQA)) k_attn_softmax_pv(const Att
     __shared__ float  red[GQA][16][PVS_DIMS + 1];
     const int g = blockIdx.x, slice = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
     const int h = tid / TH, ht = tid % TH;                     // head of the group, thread within the head
-    const int c = ht / (PVS_DIMS / DPT), dp = ht % (PVS_DIMS / DPT);   // chain, dim group
     const int w = ht >> 5;                                     // warp within the head
 
     trace_mark<TR>(a.trace, 0);
     pdl_launch_dependents();
     const int n_kv = attn_n_kv(a);                             // DecodeState is written by the previous TOKEN's last kernel
     const int n_pad = (n_kv + 31) / 32 * 32;
-    const int VCH = a.p_chunk;                                 // positions of V staged at a time (multiple of 32)
+    const int VCH = a.p_chunk;                                 // positions of V in a slot (multiple of 32)
     float * ps = reinterpret_cast<float *>(sp_dyn);            // [GQA][n_pad]
     __half (*vs)[PVS_DIMS] = reinterpret_cast<__half (*)[PVS_DIMS]>(sp_dyn + (size_t) GQA * n_pad * 4);
     const __half * vbase = a.v_cache + g * HD + slice * PVS_DIMS;
     // V rows of one chunk; rows in [n_kv, n_pad) are zero-filled: p == 0 there and the product must be 0, never NaN
-    auto stage_v = [&](int t0) {
+    auto stage_v = [&](int t0, int slot) {
         const int len = min(VCH, n_pad - t0);
         for (int i = tid; i < len; i += NT) {
-            if (t0 + i < n_kv) cp_async16(&vs[i][0], vbase + (size_t) (t0 + i) * a.kv_dim);
-            else *reinterpret_cast<uint4 *>(&vs[i][0]) = make_uint4(0u, 0u, 0u, 0u);
+            if (t0 + i < n_kv) cp_async16(&vs[slot * VCH + i][0], vbase + (size_t) (t0 + i) * a.kv_dim);
+            else *reinterpret_cast<uint4 *>(&vs[slot * VCH + i][0]) = make_uint4(0u, 0u, 0u, 0u);
         }
         cp_async_commit();
     };
-    stage_v(0);
+    for (int i = 0; i < PVS_SLOTS; i++) stage_v(i * VCH, i);
 #if B200_LOOKAHEAD
     if (lane == 0 && a.pf2[0].bytes)
         issue_l2_lookahead(a.pf2, (tid >> 5) * (gridDim.x * gridDim.y) + slice * gridDim.x + g, (NT / 32) * gridDim.x * gridDim.y, n_kv - 1);
@@ -1774,36 +1783,42 @@ __global__ void __launch_bounds__(GQA * pvs_th(GQA)) k_attn_softmax_pv(const Att
     __syncthreads();                                           // all rows normalised, every thread's V copies landed
     trace_mark<TR>(a.trace, 3);
 
-    // P.V: chain c of (head h, dims 2dp, 2dp+1): acc = fma(V[t][d], p[t], acc) over t = c, c+16, ...
-    float acc0 = 0.f, acc1 = 0.f;
-    for (int t0 = 0; t0 < n_pad; t0 += VCH) {
+    // P.V: acc = fma(V[t][d], p[t], acc) over t = c, c+16, ... A thread has chain c of two heads and two dims: three loads for four fmas. (A thread per head, chain and dim
+    // loads twice per fma: two thirds of this kernel's time at 8000 positions was this loop's shared-memory reads.)
+    constexpr int HPT = pvs_hpt(GQA);
+    const int dp = tid & 3, c = (tid >> 2) & 15, h0 = (tid >> 6) * HPT;
+    float acc[HPT][2] = {};
+    for (int t0 = 0, k = 0; t0 < n_pad; t0 += VCH, k++) {
         const int len = min(VCH, n_pad - t0);
-        if (t0) {
-            __syncthreads();
-            stage_v(t0);
-            cp_async_wait<0>();
+        if (k >= PVS_SLOTS) {
+            cp_async_wait<PVS_SLOTS - 1>();                     // (one group per chunk, the empty ones at the end too)
             __syncthreads();
         }
-        const int steps = len / 16;
-        const float * pr = row + t0 + c;
-        if (DPT == 2) {
-            const __half2 * vr = reinterpret_cast<const __half2 *>(&vs[c][2 * dp]);
+        if (h0 < GQA) {
+            const int steps = len / 16;
+            const float * pr = ps + (size_t) h0 * n_pad + t0 + c;
+            const __half2 * vr = reinterpret_cast<const __half2 *>(&vs[(k & (PVS_SLOTS - 1)) * VCH + c][2 * dp]);
 #pragma unroll 8
             for (int s = 0; s < steps; s++) {
                 const float2 v = __half22float2(vr[(size_t) s * 16 * (PVS_DIMS / 2)]);
-                const float p = pr[16 * s];
-                acc0 = __fmaf_rn(v.x, p, acc0);
-                acc1 = __fmaf_rn(v.y, p, acc1);
+#pragma unroll
+                for (int j = 0; j < HPT; j++) {
+                    const float p = pr[(size_t) j * n_pad + 16 * s];
+                    acc[j][0] = __fmaf_rn(v.x, p, acc[j][0]);
+                    acc[j][1] = __fmaf_rn(v.y, p, acc[j][1]);
+                }
             }
-        } else {
-            const __half * vr = &vs[c][dp];
-#pragma unroll 8
-            for (int s = 0; s < steps; s++)
-                acc0 = __fmaf_rn(__half2float(vr[(size_t) s * 16 * PVS_DIMS]), pr[16 * s], acc0);
+        }
+        if (n_pad > PVS_SLOTS * VCH) {
+            __syncthreads();                                    // the slot is read
+            if (t0 + PVS_SLOTS * VCH < n_pad) stage_v(t0 + PVS_SLOTS * VCH, k & (PVS_SLOTS - 1));
+            else cp_async_commit();
         }
     }
-    if (DPT == 2) { red[h][c][2 * dp] = acc0; red[h][c][2 * dp + 1] = acc1; }
-    else          red[h][c][dp] = acc0;
+    if (h0 < GQA) {
+#pragma unroll
+        for (int j = 0; j < HPT; j++) { red[h0 + j][c][2 * dp] = acc[j][0]; red[h0 + j][c][2 * dp + 1] = acc[j][1]; }
+    }
     __syncthreads();
     trace_mark<TR>(a.trace, 4);
     if (tid < GQA * PVS_DIMS) {
