@@ -36,6 +36,7 @@
 #include "stack.hpp"
 #include "safetensors.hpp"
 #include "stack_kernels.cuh"
+#include "stack_kernels_f32.cuh"
 #include "stack_kernels_mix.cuh"
 #include "stack_kernels_hyper.cuh"
 #include "stack_kernels_scan.cuh"
@@ -1304,6 +1305,14 @@ bool gx_pays(bool f32, int chunks, int N, int batch, bool glu, int sm_count) {
     const long long here = waves(GX_ROWS, resident[f32][c]), there = waves(16, 4);
     return 2 * here <= 3 * there && 16 * chunks >= (here == 1 && ch > 1 ? 12 : 14) * full;
 }
+// float32 tiles on the tensor cores (k_gemm_f32_umma) instead of the fp32 pipe: 64 tokens x 512 x 64 take 8.5 us here and 8.6 there, everything above is faster (600 x 16000 x 1024:
+// 694 and 156 us, 300 x 1024 x 4096 88 and 34). With less than half a tile's rows, columns or slice, the fp32 pipe's 64 x 64 tiles waste less.
+bool f32_umma_takes(bool vec, int T, int N, int K, const int * err) { return vec && err && umma_enabled() && T >= 64 && N >= 64 && K >= 64; }
+void launch_f32_umma(cudaStream_t st, const LinArgs & a, int * err, int batch, int parts = 1, float * part = nullptr) {
+    static const bool attr = [] { return cudaFuncSetAttribute(k_gemm_f32_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, F3_SMEM) == cudaSuccess; }();
+    if (!attr) throw std::runtime_error("cannot reserve shared memory for k_gemm_f32_umma");
+    k_gemm_f32_umma<<<dim3((unsigned) ((a.N + F3_BN - 1) / F3_BN), (unsigned) ((a.T + F3_BM - 1) / F3_BM), (unsigned) (parts > 1 ? parts : batch)), F3_THREADS, F3_SMEM, st>>>(a, err, parts, part);
+}
 // the kernel a product goes to: mat-vecs of few tokens, then tile kernels
 enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG, LIN_ROWS_X, LIN_UMMA, LIN_F32_PARTS, LIN_MMA, LIN_SIMT };
 // vec: LinArgs::vec; x_elems: entries of X; xb_elems, part_floats: what the scratch has room for
@@ -1398,10 +1407,16 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
         else k_gemm_bf16_umma<<<grid, 256, UM_SMEM, st>>>(mx, mw, a, us->err);
         if (launches) (*launches)++;
     } else if (route == LIN_F32_PARTS) {      // (a gated unit needs its sums whole: k_gemm_simt, 193 us against 236 in 128 x 128 tiles)
-        const int f32_parts = f32_k_parts(T, N, K, us->sm_count);
-        k_gemm_simt_big<<<dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((T + SG_BM - 1) / SG_BM), (unsigned) f32_parts), 256, 0, st>>>(a, f32_parts, us->part);
-        k_split_sum<<<dim3((unsigned) ((N + 255) / 256), (unsigned) T), 256, 0, st>>>(us->part, f32_parts, T, N, bias, Y, ldy);
+        int f32_parts = f32_k_parts(T, N, K, us->sm_count);
+        const int tiles = ((N + F3_BN - 1) / F3_BN) * ((T + F3_BM - 1) / F3_BM);
+        if (f32_umma_takes(a.vec != 0, T, N, K, us->err)) {     // one block per SM
+            f32_parts = std::min(f32_parts, std::max(1, us->sm_count / tiles));
+            launch_f32_umma(st, a, us->err, 1, f32_parts, us->part);
+        } else k_gemm_simt_big<<<dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((T + SG_BM - 1) / SG_BM), (unsigned) f32_parts), 256, 0, st>>>(a, f32_parts, us->part);
+        if (f32_parts > 1) k_split_sum<<<dim3((unsigned) ((N + 255) / 256), (unsigned) T), 256, 0, st>>>(us->part, f32_parts, T, N, bias, Y, ldy);
         if (launches) (*launches)++;
+    } else if (dtype == STACK_F32 && us && f32_umma_takes(a.vec != 0, T, N, K, us->err)) {
+        launch_f32_umma(st, a, us->err, batch);
     } else if (route == LIN_MMA) {
         const dim3 grid((unsigned) ((N + MM_BN - 1) / MM_BN), (unsigned) ((T + MM_BM - 1) / MM_BM), (unsigned) batch);
         k_gemm_bf16_mma<<<grid, 256, 0, st>>>(a);
@@ -1496,7 +1511,8 @@ void gemm_f32(StackCtx * c, const float * X, int ldx, long long sX, const float 
     LinArgs a{X, W, nullptr, Y, M, N, K, ldx, ldy, sX, sW, sY, 0, 0, 0.f, 0.f, w_kn, ldw, nz2, sX2, sW2, sY2};
     a.vec = K % 4 == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % 4 == 0 && sX2 % 4 == 0 && sW2 % 4 == 0 && ldw % 4 == 0 && al16(X) && al16(W);
     a.accum = accum; a.see_rows = see.rows; a.see_pos = see.pos; a.see_step = see.step;
-    if (a.vec && M >= SG_BM && N >= SG_BN && simt_big_enabled())       // operands that fill 128 x 128 tiles
+    if (f32_umma_takes(a.vec != 0, M, N, K, c->d_err)) launch_f32_umma(c->st, a, c->d_err, batch * nz2);
+    else if (a.vec && M >= SG_BM && N >= SG_BN && simt_big_enabled())       // operands that fill 128 x 128 tiles
         k_gemm_simt_big<<<dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((M + SG_BM - 1) / SG_BM), (unsigned) (batch * nz2)), 256, 0, c->st>>>(a);
     else k_gemm_simt<float><<<dim3((unsigned) ((N + 63) / 64), (unsigned) ((M + 63) / 64), (unsigned) (batch * nz2)), 256, 0, c->st>>>(a);
     c->launches++;
@@ -2897,7 +2913,7 @@ void stack_linear(int device, int dtype, int T, int N, int K, const float * x, c
     }
     cudaFree(X); cudaFree(Y); cudaFree(us.xb); cudaFree(us.part); cudaFree(us.err);
     for (void * p : tmp.allocs) cudaFree(p);
-    if (herr) throw std::runtime_error("k_gemm_bf16_umma gave up waiting for its pipeline");
+    if (herr) throw std::runtime_error("a tensor-core product gave up waiting for its pipeline");
 }
 
 }  // namespace b200

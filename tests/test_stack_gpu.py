@@ -468,3 +468,34 @@ def test_float32_contexts_hold_no_room_for_products_they_never_run(tmp_path):
     for c in more:
         c.close()
     p.close()
+
+
+@pytest.mark.parametrize("T,N,K,glu", [(64, 64, 64, False), (65, 66, 68, False), (127, 130, 132, True), (128, 128, 256, False), (129, 257, 196, False), (300, 1030, 4096, False),
+                                       (600, 300, 1024, True)])
+def test_float32_products_on_the_tensor_cores(T, N, K, glu):
+    """k_gemm_f32_umma at the edges of its tiles and slices, whole and in K parts, on numbers of 24 bits and of many magnitudes. Bound: a slice of 64 k is an accumulator added to 24
+    times, cut short each time (2^-23 of sum |x w|), the slices' sums are added in float32, and the products that are left out are below 2^-25. Rows with an infinity or a
+    NaN are what fmaf gives, their neighbours untouched."""
+    rng = np.random.default_rng(T + N + K)
+    x = (rng.standard_normal((T, K)) * np.exp(2.0 * rng.standard_normal((T, K)))).astype(np.float32)
+    w = (rng.standard_normal((N, K)) / np.sqrt(K)).astype(np.float32)
+    y, z = (np.zeros((T, N // 2 if glu else N), np.float32) for _ in range(2))
+    f32p = C.POINTER(C.c_float)
+    L = _lib.lib()
+
+    def product(x, y):
+        rc = L.b200_stack_linear(0, 1, T, N, K, x.ctypes.data_as(f32p), w.ctypes.data_as(f32p), None, int(glu), 7.0, y.ctypes.data_as(f32p))
+        assert rc == 0, _lib.last_error()
+    product(x, y)
+    xe, we = x.astype(np.float64), w.astype(np.float64)
+    ref, off = xe @ we.T, (K / 64 + 48 + 2) * 2.0 ** -24 * (np.abs(xe) @ np.abs(we).T)
+    if glu:      # slopes as in the test above
+        g, u = np.minimum(ref[:, 0::2], 7.0), np.clip(ref[:, 1::2], -7.0, 7.0)
+        ref = g * so.sigmoid(1.702 * g) * (u + 1.0)
+        off = 1.13 * off[:, 0::2] * (np.abs(u) + 1.0) + off[:, 1::2] * (np.abs(g) + 1.0) + 1e-5 * np.abs(ref) + 1e-30
+    assert (np.abs(y - ref) <= off + 1e-30).all(), float((np.abs(y - ref) / (off + 1e-30)).max())
+    x[5, 3], x[9, 0] = np.inf, np.nan
+    product(x, z)
+    if not glu:  # (the unit's clamps take them in)
+        assert np.isnan(z[9]).all() and np.isinf(z[5]).all() and np.array_equal(np.sign(z[5]), np.sign(w[:, 3]))
+    assert np.abs(np.delete(z, [5, 9], 0) - np.delete(ref, [5, 9], 0)).max() <= (K + 8) * 2.0 ** -22 * np.abs(ref).max() + off.max()
