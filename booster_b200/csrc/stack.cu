@@ -1456,7 +1456,9 @@ void launch_delta_scan(StackCtx * c, const LayerSpec & L, int T, int C, float * 
 // mixers: c->in [T][E] -> c->out [T][E]; R names the run's state
 void mixer_mingru(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     linear(c, c->in, c->m->E, L.zxg, c->P, 3 * L.width, T);
-    k_mingru_scan<<<(L.width + 127) / 128, 128, 0, c->st>>>(c->P, T, L.width, c->rec + R.off_rec, c->A);
+    // (a few tokens have no tile to share)
+    if (T > 8) k_mingru_tiles<<<(L.width + 31) / 32, MG_WARPS * 32, 0, c->st>>>(c->P, T, L.width, c->rec + R.off_rec, c->A);
+    else k_mingru_scan<<<(L.width + 127) / 128, 128, 0, c->st>>>(c->P, T, L.width, c->rec + R.off_rec, c->A);
     c->launches++;
     linear(c, c->A, L.width, L.o, c->out, c->m->E, T);
 }

@@ -884,6 +884,51 @@ __global__ void k_mingru_scan(const float * __restrict__ P, int T, int width, fl
     }
     state[c] = s;
 }
+// The same for prompt portions: a block has 32 channels, its 16 warps compute gates and candidates of MG_TB tokens, one walks the tile (two shared-memory reads and an fma a
+// token), all of them write it. k_mingru_scan's thread per channel fills 16 SMs at width 2048 and has the exponentials in its chain: 512 tokens 165 us, here 27.
+constexpr int MG_TB = 64, MG_WARPS = 16;
+__global__ void __launch_bounds__(MG_WARPS * 32) k_mingru_tiles(const float * __restrict__ P, int T, int width, float * __restrict__ state, float * __restrict__ A) {
+    constexpr int PER = MG_TB / MG_WARPS;
+    __shared__ float keep[MG_TB][32], add[MG_TB][32];          // 1 - z, then the state; z * cand
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane, ld = 3 * width;
+    const bool ok = c < width;
+    float s = warp == 0 && ok ? state[c] : 0.f;
+    float zp[PER], up[PER], gp[PER];
+    const auto fetch = [&](int t0) {
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int t = t0 + warp + MG_WARPS * i;
+            const float * p = P + (size_t) t * ld + c;
+            const bool in = ok && t < T;
+            zp[i] = in ? p[0] : 0.f; up[i] = in ? p[width] : 0.f; gp[i] = in ? p[2 * width] : 0.f;
+        }
+    };
+    fetch(0);
+    for (int t0 = 0; t0 < T; t0 += MG_TB) {
+        float g[PER];
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int k = warp + MG_WARPS * i;
+            const float z = sigmoidf_(zp[i]), cand = up[i] >= 0.f ? up[i] + 0.5f : sigmoidf_(up[i]);
+            keep[k][lane] = 1.0f - z; add[k][lane] = z * cand;
+            g[i] = siluf_(gp[i]);
+        }
+        __syncthreads();
+        if (t0 + MG_TB < T) fetch(t0 + MG_TB);
+        if (warp == 0) {
+            const int n = min(MG_TB, T - t0);
+#pragma unroll 8
+            for (int k = 0; k < n; k++) { s = fmaf(keep[k][lane], s, add[k][lane]); keep[k][lane] = s; }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int k = warp + MG_WARPS * i;
+            if (ok && t0 + k < T) A[(size_t) (t0 + k) * width + c] = keep[k][lane] * g[i];      // (its own entry, which it is also the next to write)
+        }
+    }
+    if (warp == 0 && ok) state[c] = s;
+}
 
 // ---- rotary positions on the first `dims` entries of a vector: pair i is (i, i + dims/2) ('rotate half') or, with
 // adjacent = 1, the neighbours (2i, 2i + 1) -------------------------------------------------------------------------------
