@@ -1313,6 +1313,12 @@ void launch_f32_umma(cudaStream_t st, const LinArgs & a, int * err, int batch, i
     if (!attr) throw std::runtime_error("cannot reserve shared memory for k_gemm_f32_umma");
     k_gemm_f32_umma<<<dim3((unsigned) ((a.N + F3_BN - 1) / F3_BN), (unsigned) ((a.T + F3_BM - 1) / F3_BM), (unsigned) (parts > 1 ? parts : batch)), F3_THREADS, F3_SMEM, st>>>(a, err, parts, part);
 }
+void split_sum(cudaStream_t st, const float * part, int parts, int T, int N, const float * bias, float * Y, int ldy) {
+    const bool wide = N % 4 == 0 && ldy % 4 == 0 && ((uintptr_t) Y & 15) == 0;
+    const dim3 grid((unsigned) ((N / (wide ? 4 : 1) + 255) / 256), (unsigned) T);
+    if (wide) k_split_sum<4><<<grid, 256, 0, st>>>(part, parts, T, N, bias, Y, ldy);
+    else k_split_sum<1><<<grid, 256, 0, st>>>(part, parts, T, N, bias, Y, ldy);
+}
 // the kernel a product goes to: mat-vecs of few tokens, then tile kernels
 enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG, LIN_ROWS_X, LIN_UMMA, LIN_F32_PARTS, LIN_MMA, LIN_SIMT };
 // vec: LinArgs::vec; x_elems: entries of X; xb_elems, part_floats: what the scratch has room for
@@ -1394,14 +1400,14 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
         // tensor memory path: activations to bfloat16 once, then tcgen05.mma over TMA-fed stages (a.vec: rows and batch strides are multiples of 16 bytes)
         static const bool attr = [] { return cudaFuncSetAttribute(k_gemm_bf16_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM) == cudaSuccess; }();
         if (!attr) throw std::runtime_error("cannot reserve shared memory for k_gemm_bf16_umma");
-        k_to_bf16<<<dim3((unsigned) std::min((K + 255) / 256, 64), (unsigned) T, (unsigned) xbatch), 256, 0, st>>>(X, ldx, T, K, sX, us->xb, (long long) T * K);
+        k_to_bf16<<<dim3((unsigned) std::min<long long>(((long long) T * (K / 8) + 255) / 256, 2048), (unsigned) xbatch), 256, 0, st>>>(X, ldx, T, K, sX, us->xb, (long long) T * K);
         const dim3 grid((unsigned) ((N + UM_BN - 1) / UM_BN), (unsigned) ((T + UM_BM - 1) / UM_BM), (unsigned) batch);
         const CUtensorMap mx = map_bf16(us->xb, K, T, xbatch, K, (long long) T * K, UM_BM), mw = map_bf16(W, K, N, batch, K, sW, UM_BN);
         const int tiles = (int) (grid.x * grid.y), nk = (K + UM_BK - 1) / UM_BK;
         const int ksplit = batch == 1 && !a.glu && !a.seg && us->part && split_k_enabled() ? std::min(us->sm_count / tiles, nk / 4) : 1;
         if (ksplit > 1) {
             k_gemm_bf16_umma<<<dim3(grid.x, grid.y, (unsigned) ksplit), 256, UM_SMEM, st>>>(mx, mw, a, us->err, ksplit, us->part);
-            k_split_sum<<<dim3((unsigned) ((N + 255) / 256), (unsigned) T), 256, 0, st>>>(us->part, ksplit, T, N, bias, Y, ldy);
+            split_sum(st, us->part, ksplit, T, N, bias, Y, ldy);
             if (launches) (*launches)++;
         }
         else k_gemm_bf16_umma<<<grid, 256, UM_SMEM, st>>>(mx, mw, a, us->err);
@@ -1413,7 +1419,7 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
             f32_parts = std::min(f32_parts, std::max(1, us->sm_count / tiles));
             launch_f32_umma(st, a, us->err, 1, f32_parts, us->part);
         } else k_gemm_simt_big<<<dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((T + SG_BM - 1) / SG_BM), (unsigned) f32_parts), 256, 0, st>>>(a, f32_parts, us->part);
-        if (f32_parts > 1) k_split_sum<<<dim3((unsigned) ((N + 255) / 256), (unsigned) T), 256, 0, st>>>(us->part, f32_parts, T, N, bias, Y, ldy);
+        if (f32_parts > 1) split_sum(st, us->part, f32_parts, T, N, bias, Y, ldy);
         if (launches) (*launches)++;
     } else if (dtype == STACK_F32 && us && f32_umma_takes(a.vec != 0, T, N, K, us->err)) {
         launch_f32_umma(st, a, us->err, batch);

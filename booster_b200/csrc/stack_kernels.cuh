@@ -16,6 +16,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 namespace b200 {
 namespace stk {
@@ -689,10 +690,17 @@ __global__ void __launch_bounds__(256) k_gemm_bf16_mma(const LinArgs a) {
 // Products with too few output tiles to fill the SMs are cut along K (ksplit > 1: blockIdx.z is the part): every part leaves its sums
 // in part [ksplit][T][N] and k_split_sum adds them in order, with the bias.
 // Every wait on an mbarrier is bounded: on a timeout the CTA raises *err, skips what is left and still frees its tensor memory.
-__global__ void k_to_bf16(const float * __restrict__ X, int ldx, int T, int K, long long sX, __nv_bfloat16 * __restrict__ Xb, long long sXb) {
-    const float * x = X + (size_t) blockIdx.z * sX + (size_t) blockIdx.y * ldx;
-    __nv_bfloat16 * o = Xb + (size_t) blockIdx.z * sXb + (size_t) blockIdx.y * K;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) o[k] = __float2bfloat16_rn(x[k]);
+// vec: rows and bases allow 16-byte loads (then K is a multiple of 8: LinArgs::vec of a bf16 product): eight entries a thread, over all rows of a batch entry at once.
+// 512 x 2048 5.6 us with an entry a thread, 4.0 now; 512 x 8192 13.6 and 6.2.
+__global__ void __launch_bounds__(256) k_to_bf16(const float * __restrict__ X, int ldx, int T, int K, long long sX, __nv_bfloat16 * __restrict__ Xb, long long sXb) {
+    const float * x = X + (size_t) blockIdx.y * sX;
+    __nv_bfloat16 * o = Xb + (size_t) blockIdx.y * sXb;
+    const int chunks = K / 8;
+    for (long long i = (long long) blockIdx.x * blockDim.x + threadIdx.x; i < (long long) T * chunks; i += (long long) gridDim.x * blockDim.x) {
+        const int t = (int) (i / chunks), k = (int) (i - (long long) t * chunks) * 8;
+        const float4 u = *reinterpret_cast<const float4 *>(x + (size_t) t * ldx + k), v = *reinterpret_cast<const float4 *>(x + (size_t) t * ldx + k + 4);
+        *reinterpret_cast<uint4 *>(o + (size_t) t * K + k) = make_uint4(pack_bf16(u.x, u.y), pack_bf16(u.z, u.w), pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    }
 }
 constexpr int UM_BM = 128, UM_BN = 256, UM_BK = 64, UM_STAGES = 4;
 constexpr int UM_A_BYTES = UM_BM * UM_BK * 2, UM_B_BYTES = UM_BN * UM_BK * 2, UM_STAGE_BYTES = UM_A_BYTES + UM_B_BYTES;
@@ -840,20 +848,33 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
     }
 }
 
-// Y[t][n] = bias[n] + the parts' sums, in order
-__global__ void k_split_sum(const float * __restrict__ part, int ksplit, int T, int N, const float * __restrict__ bias, float * __restrict__ Y, int ldy) {
-    const int t = blockIdx.y, n = blockIdx.x * blockDim.x + threadIdx.x;
+// Y[t][n] = bias[n] + the parts' sums, in order. NV entries a thread (four where N, ldy and the bases allow 16-byte accesses: 4 x 512 x 2048 7.9 -> 5.6 us)
+template <int NV>
+__global__ void __launch_bounds__(256) k_split_sum(const float * __restrict__ part, int ksplit, int T, int N, const float * __restrict__ bias, float * __restrict__ Y, int ldy) {
+    using V = typename std::conditional<NV == 4, float4, float>::type;
+    const int t = blockIdx.y, n = (blockIdx.x * blockDim.x + threadIdx.x) * NV;
     if (n >= N) return;
     const float * p = part + (size_t) t * N + n;
     const size_t plane = (size_t) T * N;
-    float v = bias ? bias[n] : 0.f;
+    __align__(16) float v[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i++) v[i] = bias ? bias[n + i] : 0.f;
     int z = 0;
     for (; z + 4 <= ksplit; z += 4) {
-        const float p0 = p[(size_t) z * plane], p1 = p[(size_t) (z + 1) * plane], p2 = p[(size_t) (z + 2) * plane], p3 = p[(size_t) (z + 3) * plane];
-        v = (((v + p0) + p1) + p2) + p3;
+        V q[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) q[j] = *reinterpret_cast<const V *>(p + (size_t) (z + j) * plane);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int i = 0; i < NV; i++) v[i] += reinterpret_cast<const float *>(&q[j])[i];
     }
-    for (; z < ksplit; z++) v += p[(size_t) z * plane];
-    Y[(size_t) t * ldy + n] = v;
+    for (; z < ksplit; z++) {
+        const V q = *reinterpret_cast<const V *>(p + (size_t) z * plane);
+#pragma unroll
+        for (int i = 0; i < NV; i++) v[i] += reinterpret_cast<const float *>(&q)[i];
+    }
+    *reinterpret_cast<V *>(Y + (size_t) t * ldy + n) = *reinterpret_cast<const V *>(v);
 }
 
 // ---- minGRU: S_t = (1 - z) S_(t-1) + z * cand, gates from the current token only ----------------------------------------
