@@ -705,7 +705,7 @@ def main():
                 traffic = tj["dram_bytes_read"] + tj["dram_bytes_write"]
         except Exception:
             pass
-        line["roofline"] = {"bound": "hbm", "kernel": "k_matvec<EPI_SILU> (ffn gate|up, fused RMSNorm + activation quant + SiLU*mul)",
+        line["roofline"] = {"bound": "hbm", "kernel": "k_matvec_kq / k_matvec_q80, EPI_SILU (ffn gate|up, fused RMSNorm + activation quant + SiLU*mul)",
                             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                             "peak_source": peak_src, "bytes_per_launch": float(gu_bytes), "ms_per_launch": gu_ms,
                             "share_of_token_time": acc["gate_up"][0] / reps / tot_ms}

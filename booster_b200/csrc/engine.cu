@@ -5,13 +5,13 @@
 // 6 fused kernels per layer, captured once into a CUDA graph and replayed per token; the per-token scalars
 // (token, pos) live in device memory (DecodeState) so the graph never needs re-instantiation.
 //
-//   per layer:  k_matvec<QKV>   [RMSNorm(attn_norm)+Q8_K quant] -> wq|wk|wv -> RoPE -> q (f32), K/V (f16 cache)
+//   per layer:  qkv    (k_matvec_kq, k_matvec_q80) [RMSNorm(attn_norm)+Q8_K quant] -> wq|wk|wv -> RoPE -> q (f32), K/V (f16 cache)
 //               k_attn_scores      raw K.q scores of the f16 cache (GQA group per CTA, 64 positions each)
 //               k_attn_softmax_pv  soft-max of the score rows + P.V -> kqv_merged_cont
-//               k_matvec<RESID> [quant] -> wo -> + residual                          (ffn_inp)
-//               k_matvec<SILU>  [RMSNorm(ffn_norm)+quant] -> gate|up -> silu(g)*u    (ffn_gate_par)
-//               k_matvec<RESID> [quant] -> down -> + residual                        (l_out)
-//   head:       k_matvec<STORE> [RMSNorm(output_norm)+quant] -> output -> logits
+//               wo              [quant] -> wo -> + residual                          (ffn_inp)
+//               gate|up         [RMSNorm(ffn_norm)+quant] -> gate|up -> silu(g)*u    (ffn_gate_par)
+//               down            [quant] -> down -> + residual                        (l_out)
+//   head:       output          [RMSNorm(output_norm)+quant] -> output -> logits
 //
 // There is no CPU fallback: every entry point fails with an error when no CUDA device is present.
 #include "../../include/booster_b200.h"
