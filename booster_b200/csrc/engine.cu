@@ -2128,8 +2128,8 @@ extern "C" int b200_decode(b200_ctx * c, const int32_t * tokens, int n, int pos0
             }
             if (!c->g_logits) {
                 c->g_logits = capture(c, [&]() {
-                    enqueue_forward(c, true, true);
-                    if (c->token_state > 0) CU(cudaMemcpyAsync(c->h_logits, c->logits, (size_t) m.n_vocab * 4, cudaMemcpyDeviceToHost, c->st));   // (its phases' arguments are fixed)
+                    enqueue_forward(c, true);
+                    CU(cudaMemcpyAsync(c->h_logits, c->logits, (size_t) m.n_vocab * 4, cudaMemcpyDeviceToHost, c->st));
                 }, &c->n_logits);
             }
             CU(cudaGraphLaunch(c->g_logits, c->st));
