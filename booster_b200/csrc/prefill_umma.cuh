@@ -521,6 +521,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch(const __grid_const
                 for (int step = 0; step < n_steps; step++, it++) {
                     for (int h = 0; h < 2; h++) {
                         um_wait(b_dfull + 8 * h, it & 1, failed, a.err);
+                        __syncwarp();                                // (a lane still at this phase would miss it, were the next one let in)
                         if (lane == 0) mbar_arrive(b_dfree + 8 * h);
                     }
                     if (lane == 0) mbar_arrive(b_empty + 8 * st);

@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch_q80(const __grid_c
 #pragma unroll 1
                     for (int b = 0; b < 2 * UQ_STAGE_BLOCKS; b++) {
                         um_wait(b_dfull + 8 * d, dpar, failed, a.err);
+                        __syncwarp();                            // (a lane still at this phase would miss it, were the next one let in)
                         mbar_arrive_if(b_dfree + 8 * d, one);
                         if (++d == 3) { d = 0; dpar ^= 1u; }
                     }

@@ -1,0 +1,34 @@
+"""Rules that every kernel of booster_b200/csrc keeps and that no run shows reliably when one is broken: read from the source."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "booster_b200" / "csrc"
+WAIT = re.compile(r"\b(um_wait|um_wait_asleep|mbar_wait|mbar_wait_limited)\(")
+ARRIVE = re.compile(r"if \(lane == 0\).*\bmbar_arrive\(|\bmbar_arrive_if\(")      # one lane of the warp
+JOINED = re.compile(r"__syncwarp\(\)|__syncthreads\(\)|tmem_ld_wait\(\)|tmem_st_wait\(\)|\.sync\b")
+
+
+def _code(path):
+    return [line.split("//")[0] for line in path.read_text().splitlines()]
+
+
+@pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("*.cuh")))
+def test_a_warp_is_whole_before_one_lane_arrives_for_it(name):
+    """All lanes of a warp wait for a barrier's phase, one lane arrives for the warp. Were it let on while another lane still looks for that phase, the barrier could complete the
+    next one, whose parity that lane then waits out. Between the wait and the arrival the lanes have to meet."""
+    code, bad = _code(CSRC / name), []
+    for i, line in enumerate(code):
+        if not ARRIVE.search(line) or "__device__" in line:
+            continue
+        for back in range(i, max(-1, i - 80), -1):
+            text = code[back]
+            if back == i:
+                text = text[:ARRIVE.search(text).start()]
+            if JOINED.search(text) or "__device__" in text or "__global__" in text:
+                break
+            if WAIT.search(text):
+                bad.append(f"{name}:{i + 1} (waits at {back + 1})")
+                break
+    assert not bad, bad

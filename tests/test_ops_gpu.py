@@ -221,6 +221,22 @@ def test_mul_mat_batch_tcgen05_edges(name, shape, prefill_mma):
         assert np.array_equal(y[i], yr), f"token {i}: max abs diff {np.abs(y[i] - yr).max()}"
 
 
+@pytest.mark.parametrize("name", list(TYPES))
+@pytest.mark.parametrize("T", [1, 16, 48])
+def test_mul_mat_batch_halves_without_tokens(name, T, prefill_mma):
+    """tile halves without tokens, whose warps only hand super-blocks on: over rings that go round many times and several tiles per CTA, the last tile's half alone and every
+    tile's — the reference's bits"""
+    n, k = 20480, 4096
+    rng = np.random.default_rng(T)
+    w = G.random_blocks(rng, TYPES[name], n, k).reshape(-1)
+    x = rng.standard_normal((T, k)).astype(np.float32)
+    prefill_mma(2)
+    y = engine.op_mul_mat(TYPES[name], w, n, k, x)
+    for i in sorted({0, T - 1}):
+        yr = port.mul_mat_vec(TYPES[name], w, n, k, x[i])
+        assert np.array_equal(y[i], yr), f"token {i}: max abs diff {np.abs(y[i] - yr).max()}"
+
+
 @pytest.mark.parametrize("shape", [(64, 256, 1), (64, 512, 33), (192, 256, 31), (320, 4352, 32), (19072, 256, 40), (128, 14336, 65)])
 def test_mul_mat_batch_q8_0_edges(shape):
     """k_umma_batch_q80 where its tiles and rings end: half of a 128-row tile, two to 112 stages of four blocks (the first fewer than the ring has), one token past a
