@@ -1324,14 +1324,14 @@ static cudaGraphExec_t capture(b200_ctx * c, const std::function<void()> & body,
 }
 
 extern "C" void b200_ctx_free(b200_ctx * c);
-// [0] a token handed back by the device, [1] the error flag of the prompt kernels
+// [0] a token handed back by the device, [1] the error flag of the kernels whose waits are bounded: products of prompt batches and of single tokens
 static std::shared_ptr<int32_t> pinned_token_and_flag() {
     int32_t * p = nullptr;
     CU(cudaMallocHost(&p, 2 * sizeof(int32_t)));
     p[0] = p[1] = 0;
     return std::shared_ptr<int32_t>(p, [](int32_t * q) { cudaFreeHost(q); });
 }
-// whether a prompt kernel of this context or of the stages it took rows from has given up; the flags are clear afterwards
+// whether a kernel of this context or of the stages it took rows from has given up; the flags are clear afterwards
 static bool pb_take_flags(b200_ctx * c) {
     bool failed = false;
     const auto take = [&](volatile int32_t * flag) { if (*flag) { *flag = 0; failed = true; } };
@@ -1756,9 +1756,18 @@ static bool prefill_batch_usable(const b200_ctx * c, int n) {
     if (m.n_ff % 256 || m.n_embd % 256 || std::max(m.n_ff, m.n_embd) / 256 > 4 * 16 * 4) return false;
     return true;
 }
-// after a synchronisation: a batch whose kernel gave up waiting left no result, here or on a stage before this one
+// after a synchronisation: a kernel that gave up waiting left no result, here or on a stage before this one
 static void pb_check(b200_ctx * c) {
-    if (pb_take_flags(c)) throw std::runtime_error("a prompt kernel's bounded wait ran out");
+    if (pb_take_flags(c)) throw std::runtime_error("a matrix product's bounded wait ran out");
+}
+// c takes rows of prev: what prev's kernels raise, or those of a stage before it, is this context's failure too
+static void pb_note_upstream(b200_ctx * c, const b200_ctx * prev) {
+    const auto note = [&](const std::shared_ptr<int32_t> & f) {
+        auto & u = c->pb.upstream;
+        if (std::find(u.begin(), u.end(), f) == u.end()) u.push_back(f);
+    };
+    note(prev->pinned);
+    for (const auto & f : prev->pb.upstream) note(f);
 }
 static void prefill_alloc(b200_ctx * c) {
     if (c->pb.cap) return;
@@ -2038,12 +2047,7 @@ extern "C" int b200_stage_forward_batch(b200_ctx * c, const int32_t * tokens, in
             CU(cudaMemcpyPeerAsync(c->pb.X, m.device, prev->pb.X, prev->m->device, (size_t) n * m.n_embd * 4, c->st));
             CU(cudaEventRecord(prev->ev_taken, c->st));
             prev->taken_pending = true;
-            const auto note = [&](const std::shared_ptr<int32_t> & f) {
-                auto & u = c->pb.upstream;
-                if (std::find(u.begin(), u.end(), f) == u.end()) u.push_back(f);
-            };
-            note(prev->pinned);
-            for (const auto & f : prev->pb.upstream) note(f);
+            pb_note_upstream(c, prev);
         } else {
             prefill_embed(c, tokens, n);
         }
@@ -2123,6 +2127,7 @@ extern "C" int b200_decode(b200_ctx * c, const int32_t * tokens, int n, int pos0
                 CU(cudaMemcpyAsync(c->d_state, c->h_state, sizeof(DecodeState), cudaMemcpyHostToDevice, c->st));
                 enqueue_forward(c);
                 CU(cudaStreamSynchronize(c->st));
+                pb_check(c);
                 if (last && logits_out) CU(cudaMemcpy(logits_out, c->logits, (size_t) m.n_vocab * 4, cudaMemcpyDeviceToHost));
                 continue;
             }
@@ -2288,6 +2293,7 @@ extern "C" int b200_profile_token(b200_ctx * c, int32_t token, int pos, float ms
             cudaEventDestroy(pe.second.first); cudaEventDestroy(pe.second.second);
         }
         c->prof_ev.clear();
+        pb_check(c);
         return 0;
     } catch (const std::exception & e) { if (c) c->prof = false; return set_err(e.what()); }
 }
@@ -2320,6 +2326,7 @@ extern "C" int b200_profile_kind(b200_ctx * c, int kind, int pos, int reps, floa
         g_only_kind = -1;
         (void) l0;
         CU(cudaStreamSynchronize(c->st));
+        pb_check(c);
         CU(cudaEventElapsedTime(ms_total, c->ev_t0, c->ev_t1));
         return 0;
     } catch (const std::exception & e) { g_only_kind = -1; return set_err(e.what()); }
@@ -2356,6 +2363,7 @@ extern "C" int64_t b200_trace_token(b200_ctx * c, int32_t token, int pos, int re
             CU(cudaStreamSynchronize(c->st));
         }
         cudaGraphExecDestroy(ge);
+        pb_check(c);
         const int64_t nl = c->trace_seq;
         const int64_t need = nl * TRACE_CTAS * TRACE_PHASES;
         if (out && cap_words >= need) CU(cudaMemcpy(out, c->d_trace, (size_t) need * 8, cudaMemcpyDeviceToHost));
@@ -2389,6 +2397,7 @@ extern "C" int64_t b200_trace_phases(b200_ctx * c, int32_t token, int pos, int r
             c->ttracing = false;
             CU(cudaStreamSynchronize(c->st));
         }
+        pb_check(c);
         if (out && cap_words >= (int64_t) words) CU(cudaMemcpy(out, c->d_ttrace, words * 8, cudaMemcpyDeviceToHost));
         if (kinds) {
             std::vector<Phase> plan((size_t) c->n_phases);
@@ -2628,6 +2637,7 @@ extern "C" int b200_pipeline_generate_greedy(b200_ctx * c, int32_t first_token, 
         NC(g_nccl.GroupEnd());
         if (out_tokens) CU(cudaMemcpyAsync(out_tokens, c->d_out_tokens, (size_t) n_steps * 4, cudaMemcpyDeviceToHost, c->st));
         CU(cudaStreamSynchronize(c->st));
+        pb_check(c);                   // (behind the burst's last exchange: no rank is left waiting for this one)
         CU(cudaEventElapsedTime(&c->last_device_ms, c->ev_t0, c->ev_t1));
         return 0;
     } catch (const std::exception & e) { return set_err(e.what()); }
@@ -2652,6 +2662,7 @@ extern "C" int b200_pipeline_decode(b200_ctx * c, const int32_t * tokens, int n,
             enqueue_stage_step(c, false);
             CU(cudaStreamSynchronize(c->st));
         }
+        pb_check(c);                   // (behind the batch's last exchange, as above)
         if (c->rank == c->world - 1 && logits_out) CU(cudaMemcpy(logits_out, c->logits, (size_t) m.n_vocab * 4, cudaMemcpyDeviceToHost));
         return 0;
     } catch (const std::exception & e) { return set_err(e.what()); }
@@ -2686,6 +2697,7 @@ extern "C" int b200_stage_forward(b200_ctx * c, int32_t token, int pos, int batc
             CU(cudaMemcpyPeerAsync(c->x, m.device, prev->x, prev->m->device, (size_t) m.n_embd * 4, c->st));
             CU(cudaEventRecord(prev->ev_taken, c->st));
             prev->taken_pending = true;
+            pb_note_upstream(c, prev);
         }
         const BatchPlace place = place_batch(c, pos, 1);
         note_positions(c, pos + 1);
@@ -2697,7 +2709,7 @@ extern "C" int b200_stage_forward(b200_ctx * c, int32_t token, int pos, int batc
         return 0;
     } catch (const std::exception & e) { return set_err(e.what()); }
 }
-// what a prompt kernel of this stage does when a bounded wait runs out, from the host
+// what a kernel of this stage does when a bounded wait runs out, from the host
 extern "C" int b200_stage_raise(b200_ctx * c) {
     if (!c || !c->pb.err) return set_err("not a context of the GGUF LLaMA path");
     *(volatile int32_t *) c->pb.err = 1;

@@ -2769,7 +2769,7 @@ void stack_decode(StackCtx * c, const int32_t * tokens, int n, int pos0, const i
         SCU(cudaMemcpyAsync(c->h_err, c->d_err, 4, cudaMemcpyDeviceToHost, c->st));
         SCU(cudaEventRecord(c->ev1, c->st));
         SCU(cudaStreamSynchronize(c->st));
-        if (*c->h_err) throw std::runtime_error("a tensor-core product gave up waiting for its pipeline (k_gemm_bf16_umma); the step's results are invalid");
+        if (*c->h_err) throw std::runtime_error("a tensor-core product gave up waiting for its pipeline; the step's results are invalid");
         if (row_off) { c->d_last_row = row_off - 1; c->h_last = c->h_logits + (size_t) (row_off - 1) * m.vocab; }
     }
     cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1);

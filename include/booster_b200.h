@@ -217,9 +217,10 @@ int b200_stage_forward(b200_ctx * c, int32_t token, int pos, int batch_gt1, b200
    stage of a pod); b200_stage_forward_batch returns 2 without doing anything when they cannot. */
 int b200_stage_batch_usable(b200_ctx * c, int n);
 int b200_stage_forward_batch(b200_ctx * c, const int32_t * tokens, int n, int pos0, b200_ctx * prev);
-/* Waits inside the prompt kernels are bounded: one that runs out raises a flag of its stage, its results are missing, and the next
-   b200_stage_sync / _logits / _logits_view / _argmax fails on that stage or on a later one that took its rows, which clears the flags of
-   the chain. b200_stage_raise raises stage `c`'s flag from the host (tests). */
+/* Waits inside the matrix products, of prompt batches and of single tokens, are bounded: one that runs out raises a flag of its stage, its
+   results are missing, and the next b200_stage_sync / _logits / _logits_view / _argmax fails on that stage or on a later one that took its
+   rows (b200_stage_forward, _batch), which clears the flags of the chain; calls that synchronise themselves (b200_decode, the pipeline's)
+   fail where they run. b200_stage_raise raises stage `c`'s flag from the host (tests). */
 int b200_stage_raise(b200_ctx * c);
 int b200_stage_sync(b200_ctx * c);    /* wait for everything enqueued on this stage (llama_synchronize, cpp/src/llama.cpp:18536) */
 int b200_stage_logits(b200_ctx * c, float * logits_out);

@@ -442,6 +442,16 @@ def test_stage_chain_reports_an_earlier_stage_that_gave_up(tmp_path):
             assert read(cs[2]) != 0 and b"bounded wait" in L.b200_last_error()
             for c in cs:                                    # reported once, by the call that hit it
                 assert L.b200_stage_sync(c.h) == 0
+    def chain_of_one():
+        for i, c in enumerate(cs):
+            engine.check(L.b200_stage_forward(c.h, 7, 20, 0, cs[i - 1].h if i else None), f"stage {i}")
+    for stage in range(3):                                  # the same of a single token's products
+        for read in reads:
+            chain_of_one()
+            engine.check(L.b200_stage_raise(cs[stage].h), "raise")
+            assert read(cs[2]) != 0 and b"bounded wait" in L.b200_last_error()
+            for c in cs:
+                assert L.b200_stage_sync(c.h) == 0
     chain()
     engine.check(L.b200_stage_raise(cs[0].h), "raise")
     for c in cs:                                            # a sequence that is given up takes its failure with it
@@ -451,3 +461,20 @@ def test_stage_chain_reports_an_earlier_stage_that_gave_up(tmp_path):
     _same(out, want, "logits after the failures")
     for x in cs + ms:
         x.close()
+
+
+def test_steps_with_taps_report_a_product_that_gave_up(tmp_path):
+    """the step that hands out intermediate values runs its kernels one by one: it looks at the error flag as the replayed one does"""
+    path = str(tmp_path / "m.gguf")
+    G.synth_llama(path, G.LlamaConfig(n_layer=1, n_embd=512, n_head=4, n_head_kv=1, n_ff=768, n_vocab=256, n_ctx_train=256), "Q4_K_M", seed=5)
+    m = engine.Model(path)
+    c = engine.Context(m, 64)
+    for taps in (True, False):
+        c.set_taps(taps)
+        want = c.decode([5], 0)
+        for tokens in ([5], [5, 6, 7]):
+            engine.check(m.L.b200_stage_raise(c.h), "raise")
+            with pytest.raises(engine.B200Error, match="bounded wait"):
+                c.decode(tokens, 0)
+        _same(c.decode([5], 0), want, "logits after the failure")
+    c.close(); m.close()

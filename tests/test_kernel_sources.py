@@ -32,3 +32,16 @@ def test_a_warp_is_whole_before_one_lane_arrives_for_it(name):
                 bad.append(f"{name}:{i + 1} (waits at {back + 1})")
                 break
     assert not bad, bad
+
+
+def test_every_call_that_runs_products_reads_their_error_flag():
+    """a product whose bounded wait runs out stores nothing and raises a flag: each entry point that runs one and synchronises looks at it before it reports success"""
+    text = (CSRC / "engine.cu").read_text()
+    calls, bad = re.split(r'(?m)^(?=extern "C" )', text)[1:], []
+    for call in calls:
+        body = "\n".join(line.split("//")[0] for line in call.splitlines())
+        name = re.search(r"(b200_\w+)\(", body).group(1)
+        runs = re.search(r"\b(enqueue_forward|enqueue_stage_step|cudaGraphLaunch|launch_matvec|pb_matmul)\(", body)
+        if runs and "cudaStreamSynchronize(" in body and "pb_check(" not in body[body.rindex("cudaStreamSynchronize("):]:
+            bad.append(name)
+    assert not bad, bad
