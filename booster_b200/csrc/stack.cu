@@ -47,6 +47,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <utility>
 #include <vector>
@@ -290,6 +291,19 @@ struct StackCtx {
 };
 
 namespace {
+
+// A kernel's limit of dynamic shared memory is set per device and only ever grows; models on several devices, and contexts on several threads, come here with the same kernels.
+// have: what it was raised to on each device so far.
+template <typename K>
+void raise_smem(K kern, size_t smem, size_t (&have)[64]) {
+    static std::mutex mu;
+    int device = 0;
+    SCU(cudaGetDevice(&device));
+    std::lock_guard<std::mutex> lk(mu);
+    if (smem <= have[device & 63]) return;
+    SCU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    have[device & 63] = smem;
+}
 
 // ---- uploads --------------------------------------------------------------------------------------------------
 void * dev_alloc(StackModel & m, size_t bytes) {
@@ -1309,8 +1323,8 @@ bool gx_pays(bool f32, int chunks, int N, int batch, bool glu, int sm_count) {
 // 694 and 156 us, 300 x 1024 x 4096 88 and 34). With less than half a tile's rows, columns or slice, the fp32 pipe's 64 x 64 tiles waste less.
 bool f32_umma_takes(bool vec, int T, int N, int K, const int * err) { return vec && err && umma_enabled() && T >= 64 && N >= 64 && K >= 64; }
 void launch_f32_umma(cudaStream_t st, const LinArgs & a, int * err, int batch, int parts = 1, float * part = nullptr) {
-    static const bool attr = [] { return cudaFuncSetAttribute(k_gemm_f32_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, F3_SMEM) == cudaSuccess; }();
-    if (!attr) throw std::runtime_error("cannot reserve shared memory for k_gemm_f32_umma");
+    static size_t have[64] = {0};
+    raise_smem(k_gemm_f32_umma, F3_SMEM, have);
     k_gemm_f32_umma<<<dim3((unsigned) ((a.N + F3_BN - 1) / F3_BN), (unsigned) ((a.T + F3_BM - 1) / F3_BM), (unsigned) (parts > 1 ? parts : batch)), F3_THREADS, F3_SMEM, st>>>(a, err, parts, part);
 }
 void split_sum(cudaStream_t st, const float * part, int parts, int T, int N, const float * bias, float * Y, int ldy) {
@@ -1398,8 +1412,8 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
         }
     } else if (route == LIN_UMMA) {
         // tensor memory path: activations to bfloat16 once, then tcgen05.mma over TMA-fed stages (a.vec: rows and batch strides are multiples of 16 bytes)
-        static const bool attr = [] { return cudaFuncSetAttribute(k_gemm_bf16_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM) == cudaSuccess; }();
-        if (!attr) throw std::runtime_error("cannot reserve shared memory for k_gemm_bf16_umma");
+        static size_t have[64] = {0};
+        raise_smem(k_gemm_bf16_umma, UM_SMEM, have);
         k_to_bf16<<<dim3((unsigned) std::min<long long>(((long long) T * (K / 8) + 255) / 256, 2048), (unsigned) xbatch), 256, 0, st>>>(X, ldx, T, K, sX, us->xb, (long long) T * K);
         const dim3 grid((unsigned) ((N + UM_BN - 1) / UM_BN), (unsigned) ((T + UM_BM - 1) / UM_BM), (unsigned) batch);
         const CUtensorMap mx = map_bf16(us->xb, K, T, xbatch, K, (long long) T * K, UM_BM), mw = map_bf16(W, K, N, batch, K, sW, UM_BN);
@@ -2577,13 +2591,9 @@ StackCtx * stack_ctx_new(StackModel * m, int n_ctx) {
         if (m->max_scan_state > 0 && c->cap >= SCAN_CHUNK_MIN_T) {
             const size_t nch = (size_t) (c->cap + RC - 1) / RC;
             fl(&c->scan_sb, nch * m->max_scan_state); fl(&c->scan_ac, nch * (size_t) m->max_scan_heads);
-            static size_t attr = 48 * 1024;
+            static size_t have_64[64] = {0}, have_128[64] = {0};
             const size_t need = outer_chunk_smem(m->max_scan_dim, 128);
-            if (need > attr) {
-                SCU(cudaFuncSetAttribute(k_outer_chunk_out<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) need));
-                SCU(cudaFuncSetAttribute(k_outer_chunk_out<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) need));
-                attr = need;
-            }
+            if (need > 48 * 1024) { raise_smem(k_outer_chunk_out<64>, need, have_64); raise_smem(k_outer_chunk_out<128>, need, have_128); }
         }
         size_t moe_rows = 0;
         if (m->max_slots > 0) {
@@ -2661,14 +2671,11 @@ StackCtx * stack_ctx_new(StackModel * m, int n_ctx) {
         fl(&c->att_part, part); fl(&c->att_ml, ml);
         if (da_part) { fl(&c->da_part, da_part); fl((float **) &c->da_counter, da_cnt); }
         if (c->att_scores_floats) fl(&c->att_scores, c->att_scores_floats);
-        {   // the opt-in limit is a property of the kernel, not of a context: it only ever grows
-            static size_t attr = 48 * 1024;
-            if (smem > attr) {
-                SCU(cudaFuncSetAttribute(k_latent_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-                SCU(cudaFuncSetAttribute(k_latent_attn_staged<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-                SCU(cudaFuncSetAttribute(k_latent_attn_staged<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-                attr = smem;
-            }
+        if (smem > 48 * 1024) {
+            static size_t have_plain[64] = {0}, have_v[64] = {0}, have_s[64] = {0};
+            raise_smem(k_latent_attn, smem, have_plain);
+            raise_smem(k_latent_attn_staged<true>, smem, have_v);
+            raise_smem(k_latent_attn_staged<false>, smem, have_s);
         }
         SCU(cudaMalloc(&c->d_step, sizeof(StepDev)));
         SCU(cudaMemsetAsync(c->d_step, 0, sizeof(StepDev), c->st));

@@ -45,3 +45,10 @@ def test_every_call_that_runs_products_reads_their_error_flag():
         if runs and "cudaStreamSynchronize(" in body and "pb_check(" not in body[body.rindex("cudaStreamSynchronize("):]:
             bad.append(name)
     assert not bad, bad
+
+
+@pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("*.cu")))
+def test_shared_memory_limits_are_kept_per_device(name):
+    """a kernel's limit of dynamic shared memory holds on the device it was set on: what remembers that it was raised is an array over devices"""
+    once = [line.strip() for line in _code(CSRC / name) if re.search(r"static (const )?(bool|size_t) \w+ = ", line) and ("cudaFuncSetAttribute" in line or "attr" in line)]
+    assert not once, once
