@@ -1528,11 +1528,11 @@ AttnPlan plan_attention(const LayerSpec & L, int n_ctx, int T, int sm_count) {
 // A second batch level (nz2 products per first-level index, strides sX2 / sW2 / sY2) serves operands that are cut twice: tiles x heads.
 struct See { int rows = 0, pos = 0, step = 0; };      // LinArgs::see_*
 void gemm_f32(StackCtx * c, const float * X, int ldx, long long sX, const float * W, int w_kn, int ldw, long long sW, float * Y, int ldy, long long sY,
-              int M, int N, int K, int batch, int nz2 = 1, long long sX2 = 0, long long sW2 = 0, long long sY2 = 0, int accum = 0, See see = See()) {
+              int M, int N, int K, int batch, int nz2 = 1, long long sX2 = 0, long long sW2 = 0, long long sY2 = 0, int accum = 0, See see = See(), int rows_all = 0) {
     const auto al16 = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
     LinArgs a{X, W, nullptr, Y, M, N, K, ldx, ldy, sX, sW, sY, 0, 0, 0.f, 0.f, w_kn, ldw, nz2, sX2, sW2, sY2};
     a.vec = K % 4 == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % 4 == 0 && sX2 % 4 == 0 && sW2 % 4 == 0 && ldw % 4 == 0 && al16(X) && al16(W);
-    a.accum = accum; a.see_rows = see.rows; a.see_pos = see.pos; a.see_step = see.step;
+    a.accum = accum; a.see_rows = see.rows; a.see_pos = see.pos; a.see_step = see.step; a.rows_all = rows_all;
     if (f32_umma_takes(a.vec != 0, M, N, K, c->d_err)) launch_f32_umma(c->st, a, c->d_err, batch * nz2);
     else if (a.vec && M >= SG_BM && N >= SG_BN && simt_big_enabled())       // operands that fill 128 x 128 tiles
         k_gemm_simt_big<<<dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((M + SG_BM - 1) / SG_BM), (unsigned) (batch * nz2)), 256, 0, c->st>>>(a);
@@ -1582,10 +1582,10 @@ void mixer_latent(StackCtx * c, const LayerSpec & L, const RunSpec & Rn, int T) 
             const long long jlo = L.window > 0 ? (long long) pos0 + (long long) g0 * TQ - span + 1 : 0;     // may be negative: the cache has a zero margin in front
             const float * keys = cache + jlo * W;
             const long long sK = L.window > 0 ? (long long) TQ * W : 0;
-            gemm_f32(c, c->QK + (size_t) g0 * M * W, W, (long long) M * W, keys, 0, 0, sK, c->att_scores, nk, (long long) M * nk, M, nk, W, ng);
-            const int rows = (std::min(T, (g0 + ng) * TQ) - g0 * TQ) * H;
+            const int rows = (std::min(T, (g0 + ng) * TQ) - g0 * TQ) * H;          // (rows past the last token hold what an earlier pass left)
+            gemm_f32(c, c->QK + (size_t) g0 * M * W, W, (long long) M * W, keys, 0, 0, sK, c->att_scores, nk, (long long) M * nk, M, nk, W, ng, 1, 0, 0, 0, 0, See(), rows);
             k_latent_softmax_rows<<<(rows + 7) / 8, 256, 0, c->st>>>(c->att_scores, rows, H, TQ, nk, L.window, span, L.sink, &c->d_step->st, L.scale, g0);
-            gemm_f32(c, c->att_scores, nk, (long long) M * nk, keys, 1, W, sK, c->OL + (size_t) g0 * M * rank, rank, (long long) M * rank, M, rank, nk, ng);
+            gemm_f32(c, c->att_scores, nk, (long long) M * nk, keys, 1, W, sK, c->OL + (size_t) g0 * M * rank, rank, (long long) M * rank, M, rank, nk, ng, 1, 0, 0, 0, 0, See(), rows);
             c->launches++;
         }
         c->launches++;

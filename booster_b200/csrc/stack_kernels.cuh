@@ -181,6 +181,7 @@ struct LinArgs {
     // z1 see_step + m / see_rows only. Positions are the columns (w_kn = 0: tiles beyond their rows' last one are left alone) or the inner
     // dimension (w_kn = 1: the sum ends with the tile's last one, rounded up to 4; what lies up to there counts)
     int see_rows = 0, see_pos = 0, see_step = 0;
+    int rows_all = 0;   // k_gemm_f32_umma, > 0: rows of X and Y over all first-level entries of T each (the last one's may be fewer); others are neither read nor written
 };
 // the last position a tile of rows m0 .. m0 + rows - 1 sees
 __device__ __forceinline__ int tile_sees(const LinArgs & a, int z1, int m0, int rows) { return a.see_pos + z1 * a.see_step + (min(m0 + rows, a.T) - 1) / a.see_rows; }

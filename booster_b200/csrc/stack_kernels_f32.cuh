@@ -1,6 +1,6 @@
 // stack_kernels_f32.cuh — float32 products on the tensor cores (sm_100a, tcgen05): Y = X W^T (+ bias), the operand layouts of k_gemm_simt_big.
 //
-// A float32 number is the sum of three bfloat16 ones, exactly: hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid (24 bits are 8 + 8 + 8; below 2^-110 the last ones go).
+// A float32 number is the sum of three bfloat16 ones, exactly: hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid (24 bits are 8 + 8 + 8; a number below 2^-110 loses what is below 2^-134).
 // A product of two takes six MMAs (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi; what is left out is below 2^-26 of it). The tensor cores add in float32 without rounding to
 // nearest, so an accumulator holds 64 terms of a sum only: the small products first, hi hi last, then it is added to registers. Against 64 bits that is as close as a
 // chain of fmaf or closer (2-norm, random operands of nine shapes, k 64 to 8192: 0.8e-7 to 1.6e-7 here, 1.2e-7 to 5.7e-7 by fmaf; a whole float32 model's logits 4.5e-7 and 1.1e-6).
@@ -9,7 +9,8 @@
 //   MMA warp  24 tcgen05.mma of 128 x 128 x 16 per slice of 64 k
 // What bounds it: the MMAs, 65 clocks each (375 TFLOP/s of float32 products on all SMs); the fp32 pipe's tiles in k_gemm_simt_big reach 42.
 // Measured (B200): 600 x 16000 x 1024 694 -> 156 us, 300 x 4096 x 1024 91 -> 35, 64 x 512 x 512 40 -> 16; scores of 512 tokens x 16 heads over windows of 1152 rows of 576: 260 -> 92.
-// A tile that meets an infinity or a NaN (whose halves would be NaN) is done again by fmaf.
+// Rows and columns of a tile that three parts do not hold (an infinity or a NaN, whose parts would be NaN; nothing but numbers below 2^-100, whose last part would be gone) are
+// done again by fmaf, and they alone: what an output is does not depend on the rows beside it. In every other row the parts that are gone are below 2^-33 of its largest number.
 #pragma once
 
 namespace b200 {
@@ -18,27 +19,33 @@ namespace stk {
 constexpr int F3_BM = 128, F3_BN = 128, F3_BK = 64, F3_WORKERS = 512, F3_THREADS = F3_WORKERS + 32;
 constexpr int F3_PLANE = 128 * F3_BK * 2, F3_STAGE = 6 * F3_PLANE, F3_SMEM = 2 * F3_STAGE + 1024;       // X hi, mid, lo | W hi, mid, lo; + alignment slack
 
-// two numbers into a word of each plane; bad turns NaN with a number that is not finite
-__device__ __forceinline__ void f3_split(float x, float y, uint32_t & hi, uint32_t & mid, uint32_t & lo, float & bad) {
+// the largest magnitude met so far; NaN once there was one
+__device__ __forceinline__ void f3_top(float & top, float x) { asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(x))); }
+// whether three parts do not hold a row with this largest number: it becomes an infinity as bfloat16, or is below 2^-100 (a row of zeros is held)
+__device__ __forceinline__ bool f3_off(float top) { const uint32_t t = __float_as_uint(top); return t >= 0x7f7f8000u || (t > 0u && t < 0x0d800000u); }
+// two numbers into a word of each plane
+__device__ __forceinline__ void f3_split(float x, float y, uint32_t & hi, uint32_t & mid, uint32_t & lo, float & top) {
     hi = pack_bf16(x, y);
     const float rx = x - __uint_as_float(hi << 16), ry = y - __uint_as_float(hi & 0xffff0000u);
     mid = pack_bf16(rx, ry);
     const float lx = rx - __uint_as_float(mid << 16), ly = ry - __uint_as_float(mid & 0xffff0000u);
     lo = __byte_perm(__float_as_uint(lx), __float_as_uint(ly), 0x7632u);
-    bad = fmaf(lx, 0.f, fmaf(ly, 0.f, bad));
+    f3_top(top, x); f3_top(top, y);
 }
 
 __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a, int * err, int ksplit = 1, float * __restrict__ part = nullptr) {
     extern __shared__ uint8_t f3_raw[];
     __shared__ __align__(8) uint64_t full[2], done[2];
     __shared__ uint32_t tmem_base_s;
-    __shared__ int failed_s, bad_s;
+    __shared__ int failed_s;
+    __shared__ float x_top[F3_BM];             // largest magnitudes of the tile's rows of X and of W
+    __shared__ uint32_t w_top[F3_BN];
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t smem0 = (smem_addr(f3_raw) + 1023u) & ~1023u;
     uint8_t * const sm = f3_raw + (smem0 - smem_addr(f3_raw));
     const int m0 = blockIdx.y * F3_BM, n0 = blockIdx.x * F3_BN;
     const int zb = ksplit > 1 ? 0 : blockIdx.z, z1 = zb / a.nz2, z2 = zb - z1 * a.nz2;
-    const int r0 = a.seg ? a.seg[zb] : 0, T = a.seg ? a.seg[zb + 1] - r0 : a.T;
+    const int r0 = a.seg ? a.seg[zb] : 0, T = a.seg ? a.seg[zb + 1] - r0 : a.rows_all > 0 ? min(a.T, a.rows_all - z1 * a.T) : a.T;
     if (m0 >= T) return;                      // (the whole block, before anything is allocated)
     const float * X = a.X + (a.seg ? (size_t) r0 * a.ldx : (size_t) z1 * a.sX + (size_t) z2 * a.sX2);
     const float * W = reinterpret_cast<const float *>(a.W) + (size_t) z1 * a.sW + (size_t) z2 * a.sW2;
@@ -58,7 +65,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
     const int nk = (K - kbeg + F3_BK - 1) / F3_BK;      // at least one: ksplit <= slices
     volatile int * failed = &failed_s;
     if (tid == 0) {
-        failed_s = 0; bad_s = 0;
+        failed_s = 0;
         for (int s = 0; s < 2; s++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_addr(&full[s])), "r"(F3_WORKERS / 32) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&done[s])) : "memory");
@@ -66,6 +73,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    if (tid < F3_BN) w_top[tid] = 0u;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_addr(&tmem_base_s)), "r"(256u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -105,7 +113,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
         // ---- slices. Rows of X (and of W [N][K]): 16 threads a row, four rows a thread, 4 k each; a W [K][N]: a thread a column, 16 k
         float4 xr[4];
         float wr[16];
-        float bad = 0.f;
+        float xt[4] = {}, wt[4] = {};                           // of the rows (W [K][N]: of the column) this thread splits
         const int lr = tid >> 4, lk = tid & 15, wn = tid & 127, wk = (tid >> 7) * 16;
         const auto fetch = [&](int k0) {
             const int k = k0 + 4 * lk;
@@ -123,10 +131,10 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
                 for (int i = 0; i < 16; i++) wr[i] = n0 + wn < a.N && k0 + wk + i < K ? W[(size_t) (k0 + wk + i) * ldw + n0 + wn] : 0.f;
             }
         };
-        const auto store4 = [&](uint8_t * plane0, int row, float x, float y, float z, float w) {
+        const auto store4 = [&](uint8_t * plane0, int row, float x, float y, float z, float w, float & top) {
             uint32_t h[2], m[2], l[2];
-            f3_split(x, y, h[0], m[0], l[0], bad);
-            f3_split(z, w, h[1], m[1], l[1], bad);
+            f3_split(x, y, h[0], m[0], l[0], top);
+            f3_split(z, w, h[1], m[1], l[1], top);
             uint8_t * p = plane0 + row * 128 + (((lk >> 1) ^ (row & 7)) << 4) + (lk & 1) * 8;
             *reinterpret_cast<uint2 *>(p) = make_uint2(h[0], h[1]);
             *reinterpret_cast<uint2 *>(p + F3_PLANE) = make_uint2(m[0], m[1]);
@@ -158,15 +166,15 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
             uint8_t * st = sm + (c & 1) * F3_STAGE;             // free: slice c - 2 was drained
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                store4(st, lr + 32 * i, xr[i].x, xr[i].y, xr[i].z, xr[i].w);
-                if (!a.w_kn) store4(st + 3 * F3_PLANE, lr + 32 * i, wr[4 * i], wr[4 * i + 1], wr[4 * i + 2], wr[4 * i + 3]);
+                store4(st, lr + 32 * i, xr[i].x, xr[i].y, xr[i].z, xr[i].w, xt[i]);
+                if (!a.w_kn) store4(st + 3 * F3_PLANE, lr + 32 * i, wr[4 * i], wr[4 * i + 1], wr[4 * i + 2], wr[4 * i + 3], wt[i]);
             }
             if (a.w_kn) {
 #pragma unroll
                 for (int g = 0; g < 2; g++) {
                     uint32_t h[4], m[4], l[4];
 #pragma unroll
-                    for (int i = 0; i < 4; i++) f3_split(wr[8 * g + 2 * i], wr[8 * g + 2 * i + 1], h[i], m[i], l[i], bad);
+                    for (int i = 0; i < 4; i++) f3_split(wr[8 * g + 2 * i], wr[8 * g + 2 * i + 1], h[i], m[i], l[i], wt[0]);
                     uint8_t * p = st + 3 * F3_PLANE + wn * 128 + ((((wk >> 3) + g) ^ (wn & 7)) << 4);
                     *reinterpret_cast<uint4 *>(p) = make_uint4(h[0], h[1], h[2], h[3]);
                     *reinterpret_cast<uint4 *>(p + F3_PLANE) = make_uint4(m[0], m[1], m[2], m[3]);
@@ -180,23 +188,51 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
             if (c > 0) drain(c - 1);
         }
         drain(nk - 1);
-        if (bad != 0.f) bad_s = 1;                              // (NaN compares unequal)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {                           // 16 lanes share a row
+#pragma unroll
+            for (int o = 8; o; o >>= 1) {
+                f3_top(xt[i], __shfl_xor_sync(0xffffffffu, xt[i], o));
+                if (!a.w_kn) f3_top(wt[i], __shfl_xor_sync(0xffffffffu, wt[i], o));
+            }
+            if (lk == 0) {
+                x_top[lr + 32 * i] = xt[i];
+                if (!a.w_kn) w_top[lr + 32 * i] = __float_as_uint(wt[i]);
+            }
+        }
+        if (a.w_kn) atomicMax(&w_top[wn], __float_as_uint(wt[0]));      // (magnitudes and NaN are ordered as their bits)
         asm volatile("bar.sync 1, %0;" :: "n"(F3_WORKERS) : "memory");
-        const int m = m0 + 32 * (warp & 3) + lane, nb = n0 + (warp >> 2) * 32;
+        const int mw = m0 + 32 * (warp & 3), m = mw + lane, nb = n0 + (warp >> 2) * 32;
+        const uint32_t x_off = __ballot_sync(0xffffffffu, f3_off(x_top[32 * (warp & 3) + lane])), w_off = __ballot_sync(0xffffffffu, f3_off(__uint_as_float(w_top[(warp >> 2) * 32 + lane])));
+        if (x_off | w_off) {                                    // a row: lane = column, a column: lane = row; through the slices' memory, which the MMAs are done with
+            float * again = reinterpret_cast<float *>(sm) + warp * (32 * 33);
+            const auto chain = [&](int m, int n) {
+                float v = 0.f;
+                if (m >= T || n >= a.N) return v;
+                const float * x = X + (size_t) m * a.ldx;
+#pragma unroll 4
+                for (int k = kbeg; k < K; k += 4) {             // (K is a multiple of 4)
+                    const float4 u = *reinterpret_cast<const float4 *>(x + k);
+                    float4 w;
+                    if (a.w_kn) { const float * p = W + (size_t) k * ldw + n; w = make_float4(p[0], p[ldw], p[2 * (size_t) ldw], p[3 * (size_t) ldw]); }
+                    else w = *reinterpret_cast<const float4 *>(W + (size_t) n * ldw + k);
+                    v = fmaf(u.w, w.w, fmaf(u.z, w.z, fmaf(u.y, w.y, fmaf(u.x, w.x, v))));
+                }
+                return v;
+            };
+#pragma unroll 1
+            for (int i = 0; i < 32; i++) {
+                if (x_off >> i & 1) again[i * 33 + lane] = chain(mw + i, nb + lane);
+                if (w_off >> i & 1) again[lane * 33 + i] = chain(m, nb + i);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 32; j++) if ((x_off >> lane | w_off >> j) & 1) acc[j] = again[lane * 33 + j];
+        }
         if (m < T && !*failed) {
             const int ldy = ksplit > 1 ? a.N : a.ldy;
             const float * bias = ksplit > 1 ? nullptr : a.bias;
             float * Y = (ksplit > 1 ? part + (size_t) blockIdx.z * T * a.N : a.seg ? a.Y + (size_t) r0 * ldy : a.Y + (size_t) z1 * a.sY + (size_t) z2 * a.sY2) + (size_t) m * ldy;
-            if (bad_s) {
-#pragma unroll 1
-                for (int j = 0; j < 32; j++) {
-                    float v = 0.f;
-                    if (nb + j < a.N)
-                        for (int k = kbeg; k < K; k++) v = fmaf(X[(size_t) m * a.ldx + k], a.w_kn ? W[(size_t) k * ldw + nb + j] : W[(size_t) (nb + j) * ldw + k], v);
-#pragma unroll
-                    for (int i = 0; i < 32; i++) if (i == j) acc[i] = v;
-                }
-            }
             if (a.glu) {
 #pragma unroll
                 for (int j = 0; j < 32; j += 2)

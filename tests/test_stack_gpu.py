@@ -499,3 +499,53 @@ def test_float32_products_on_the_tensor_cores(T, N, K, glu):
     if not glu:  # (the unit's clamps take them in)
         assert np.isnan(z[9]).all() and np.isinf(z[5]).all() and np.array_equal(np.sign(z[5]), np.sign(w[:, 3]))
     assert np.abs(np.delete(z, [5, 9], 0) - np.delete(ref, [5, 9], 0)).max() <= (K + 8) * 2.0 ** -22 * np.abs(ref).max() + off.max()
+
+
+@pytest.mark.parametrize("T,N,K", [(65, 66, 68), (129, 257, 196), (300, 1030, 4096)])
+def test_float32_products_leave_rows_beside_odd_ones_alone(T, N, K):
+    """k_gemm_f32_umma, whole and in K parts: rows and columns that three bfloat16 parts do not hold (an infinity, a NaN, nothing but numbers around 2^-113) are what fmaf gives, and
+    every other output has the bits it has without them. Bound: (K + 8) 2^-24 sum |x w|, and half the smallest number for each sum in its range."""
+    rng = np.random.default_rng(T + N + K)
+    x, w = rng.standard_normal((T, K)).astype(np.float32), (rng.standard_normal((N, K)) / np.sqrt(K)).astype(np.float32)
+    f32p = C.POINTER(C.c_float)
+
+    def product(x, w):
+        y = np.zeros((T, N), np.float32)
+        rc = _lib.lib().b200_stack_linear(0, 1, T, N, K, x.ctypes.data_as(f32p), w.ctypes.data_as(f32p), None, 0, 7.0, y.ctypes.data_as(f32p))
+        assert rc == 0, _lib.last_error()
+        return y
+    y = product(x, w)
+    x[3, K // 2], x[40, 1] = np.inf, np.nan
+    x[64] *= np.float32(2.0 ** -113)
+    w[7, K - 1] = np.nan
+    w[33] *= np.float32(2.0 ** -111)
+    z = product(x, w)
+    rows, cols = np.setdiff1d(np.arange(T), [3, 40, 64]), np.setdiff1d(np.arange(N), [7, 33])
+    assert np.array_equal(z[np.ix_(rows, cols)], y[np.ix_(rows, cols)])
+    assert np.isnan(z[40]).all() and np.isnan(z[:, 7]).all() and not np.isfinite(z[3]).any()
+    tiny = np.ones((T, N), bool)
+    tiny[[3, 40]], tiny[:, 7] = False, False
+    tiny[np.ix_(rows, cols)] = False
+    xe, we = np.nan_to_num(x.astype(np.float64), posinf=0.0), np.nan_to_num(w.astype(np.float64))
+    off = (K + 8) * (2.0 ** -24 * (np.abs(xe) @ np.abs(we).T) + 2.0 ** -149)
+    assert (np.abs(z - xe @ we.T) <= off)[tiny].all()
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_attention_tiles_do_not_depend_on_rows_past_the_last_token(tmp_path, dtype):
+    """the last tile of 16 tokens has rows that no token of the portion fills. They hold an earlier pass's queries, here infinite ones of a token whose queries overflow (its cached
+    rows do not), and the portion's logits are those of a context that never saw it, bit for bit"""
+    def edit(w):
+        w["embed"][:, 0] = 0.0
+        w["embed"][60, 0] = 1.0
+        w["l0.mix.q"][:, 0] = 3e38
+        w["l0.mix.dkv"][:, 0] = 0.0
+    p = Pair(tmp_path, config([latent(heads=8, dim=8, rot_dim=16, vdim=8, kv_rank=64, window=0)]), dtype=dtype, n_ctx=96, edit=edit)
+    toks = [t % 60 for t in p.tokens(70)]
+    want = p.run(toks)
+    other = engine.Context(p.model, 96)
+    other.decode_rows(toks[:66] + [60] * 14, 0, [0])
+    got = p.run(toks, ctx=other)
+    assert np.isfinite(want).all() and np.array_equal(got, want)
+    other.close()
+    p.close()
