@@ -890,13 +890,12 @@ static bool launch_attention_2k(b200_ctx * c, const AttnArgs & a_in, int n_ctx_p
     const size_t row_bytes = (size_t) GQA * n_ctx_pad * 4;
     const size_t budget = 200 * 1024;
     if (row_bytes + (size_t) PV_BATCH * 16 > budget) return false;
-    // PVS_SLOTS slots of V, the whole context in them where it fits
-    const int vch = std::min((int) ((budget - row_bytes) / 16) / PVS_SLOTS / 32 * 32, (n_ctx_pad + 32 * PVS_SLOTS - 1) / (32 * PVS_SLOTS) * 32);
-    a.p_chunk = vch;
-    size_t smem = row_bytes + (size_t) PVS_SLOTS * vch * 16;
+    // the whole context's V beside the rows where it fits
+    size_t smem = std::min(PVS_SMEM, row_bytes + (size_t) n_ctx_pad * 16);
     // at most one CTA per SM: the block scheduler then spreads the (n_head_kv x 16) CTAs over distinct SMs even when
     // they are launched early (PDL) next to the tail of the previous kernel
     if ((int) a.n_head_kv * (128 / PVS_DIMS) <= c->sm_count) smem = std::max(smem, (size_t) 116 * 1024);
+    a.p_chunk = (int) (smem / 16);
     static size_t attr[64] = {0};
     const int dv = c->device & 63;
     std::unique_lock<std::mutex> attr_lock(g_attr_mu);

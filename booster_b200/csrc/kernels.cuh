@@ -1452,7 +1452,7 @@ struct AttnArgs {
     const DecodeState * st;
     int n_kv_override;        // >0: use instead of st->pos+1 (operator-level test)
     int round_q_override;     // operator-level test of the batch>1 arithmetic
-    int p_chunk;              // positions of p staged in shared memory by k_attn_pv (multiple of PV_BATCH)
+    int p_chunk;              // k_attn_pv: positions of p staged in shared memory (multiple of PV_BATCH); k_attn_softmax_pv: its shared memory in units of 16 bytes
     PfRange pf[PF_RANGES];    // L2 look-ahead issued by k_attn_scores
     PfRange pf2[PF_RANGES];   // ... and by k_attn_softmax_pv
     const int32_t * cell_pos; // [n_ctx] position held by each KV cell (-1: empty); read only when st->managed
@@ -1669,12 +1669,16 @@ __global__ void __launch_bounds__(PV_DIMS * 16) k_attn_pv(const AttnArgs a) {
 // with exactly k_attn_softmax's arithmetic, on a shared-memory copy; then thread (h, c, dl) runs chain c of output
 // dim dl of head h. The CTA's V slice is independent of the scores and is put in flight BEFORE griddepcontrol.wait
 // (k_attn_scores waits for the QKV kernel before it lets this kernel launch, so K/V/q are already visible).
-//   grid (n_head_kv, HD / PVS_DIMS), block GQA * pvs_th(GQA) threads (16 chains x dim groups per head); shared: ps [GQA][n_pad] f32 | vs [v_chunk][8] f16
+//   grid (n_head_kv, HD / PVS_DIMS), block GQA * pvs_th(GQA) threads; shared: ps [GQA][n_pad] f32 | vs [slot][position][8] f16
 // ------------------------------------------------------------------------------------------------------------
 static constexpr int PVS_DIMS = 8;            // dims per CTA: 8 halfs = one 16-byte cp.async per position
-static constexpr int PVS_SLOTS = 4;           // V slots of p_chunk positions each
+static constexpr int PVS_SLOTS = 4;           // V slots; all of V in them where it fits beside the score rows
+static constexpr size_t PVS_SMEM = 222 * 1024;   // dynamic shared memory at most, beside up to 5 KB of sums
 __host__ __device__ constexpr int pvs_th(int gqa) { return gqa >= 8 ? 64 : 128; }      // soft-max threads per head: at most 512 in all
-__host__ __device__ constexpr int pvs_hpt(int gqa) { return gqa >= 2 ? 2 : 1; }        // P.V: heads and dim pairs of a thread
+// P.V: heads and dims of a thread, so that four warps and more are at work whatever the heads (two dims of one head at 1: two warps, 5 to 10 % more per launch between 500 and 8000
+// positions; at 2, one dim of two heads 2 %, one of one head 3 % more than two dims of one)
+__host__ __device__ constexpr int pvs_hpt(int gqa) { return gqa >= 4 ? 2 : 1; }
+__host__ __device__ constexpr int pvs_dpt(int gqa) { return gqa >= 2 ? 2 : 1; }
 
 template <int GQA, bool TR>
 __global__ void __launch_bounds__(GQA * pvs_th(GQA)) k_attn_softmax_pv(const AttnArgs a) {
@@ -1694,20 +1698,22 @@ __global__ void __launch_bounds__(GQA * pvs_th(GQA)) k_attn_softmax_pv(const Att
     pdl_launch_dependents();
     const int n_kv = attn_n_kv(a);                             // DecodeState is written by the previous TOKEN's last kernel
     const int n_pad = (n_kv + 31) / 32 * 32;
-    const int VCH = a.p_chunk;                                 // positions of V in a slot (multiple of 32)
+    // positions of V that the rows of THIS token leave room for: all of them, or slots of a multiple of 32. One barrier a slot (scores and this kernel, per launch of the two, one
+    // 32-head layer: at the end of the longest context of 1, 2, 4 and 8 heads per key head 545, 141, 44 and 28 us with one slot of 256 positions, 242, 72, 25 and 20 here;
+    // at 2000 of such a context 33, 13, 7.8 and 10.7, now 26, 10, 5.9 and 8.8)
+    const int room = a.p_chunk - GQA * n_pad / 4, VCH = n_pad <= room ? n_pad : room / PVS_SLOTS / 32 * 32;
     float * ps = reinterpret_cast<float *>(sp_dyn);            // [GQA][n_pad]
     __half (*vs)[PVS_DIMS] = reinterpret_cast<__half (*)[PVS_DIMS]>(sp_dyn + (size_t) GQA * n_pad * 4);
     const __half * vbase = a.v_cache + g * HD + slice * PVS_DIMS;
     // V rows of one chunk; rows in [n_kv, n_pad) are zero-filled: p == 0 there and the product must be 0, never NaN
-    auto stage_v = [&](int t0, int slot) {
-        const int len = min(VCH, n_pad - t0);
+    auto stage_v = [&](int t0, int len, int at) {
         for (int i = tid; i < len; i += NT) {
-            if (t0 + i < n_kv) cp_async16(&vs[slot * VCH + i][0], vbase + (size_t) (t0 + i) * a.kv_dim);
-            else *reinterpret_cast<uint4 *>(&vs[slot * VCH + i][0]) = make_uint4(0u, 0u, 0u, 0u);
+            if (t0 + i < n_kv) cp_async16(&vs[at + i][0], vbase + (size_t) (t0 + i) * a.kv_dim);
+            else *reinterpret_cast<uint4 *>(&vs[at + i][0]) = make_uint4(0u, 0u, 0u, 0u);
         }
         cp_async_commit();
     };
-    for (int i = 0; i < PVS_SLOTS; i++) stage_v(i * VCH, i);
+    stage_v(0, min(n_pad, PVS_SLOTS * VCH), 0);
 #if B200_LOOKAHEAD
     if (lane == 0 && a.pf2[0].bytes)
         issue_l2_lookahead(a.pf2, (tid >> 5) * (gridDim.x * gridDim.y) + slice * gridDim.x + g, (NT / 32) * gridDim.x * gridDim.y, n_kv - 1);
@@ -1783,41 +1789,42 @@ __global__ void __launch_bounds__(GQA * pvs_th(GQA)) k_attn_softmax_pv(const Att
     __syncthreads();                                           // all rows normalised, every thread's V copies landed
     trace_mark<TR>(a.trace, 3);
 
-    // P.V: acc = fma(V[t][d], p[t], acc) over t = c, c+16, ... A thread has chain c of two heads and two dims: three loads for four fmas. (A thread per head, chain and dim
-    // loads twice per fma: two thirds of this kernel's time at 8000 positions was this loop's shared-memory reads.)
-    constexpr int HPT = pvs_hpt(GQA);
-    const int dp = tid & 3, c = (tid >> 2) & 15, h0 = (tid >> 6) * HPT;
-    float acc[HPT][2] = {};
+    // P.V: acc = fma(V[t][d], p[t], acc) over t = c, c+16, ... A thread has chain c of HPT heads and DPT dims. From four heads on two of each: three loads for four fmas. (A thread
+    // per head, chain and dim loads twice per fma: two thirds of this kernel's time at 8000 positions was this loop's shared-memory reads.)
+    constexpr int HPT = pvs_hpt(GQA), DPT = pvs_dpt(GQA), DG = PVS_DIMS / DPT;
+    const int dp = tid % DG, c = tid / DG % 16, h0 = tid / (16 * DG) * HPT;
+    float acc[HPT][DPT] = {};
     for (int t0 = 0, k = 0; t0 < n_pad; t0 += VCH, k++) {
         const int len = min(VCH, n_pad - t0);
-        if (k >= PVS_SLOTS) {
-            cp_async_wait<PVS_SLOTS - 1>();                     // (one group per chunk, the empty ones at the end too)
+        if (k > 0) {                                            // the chunk before is read by all threads, this one is there: the slot of the one takes the chunk three after the other
+            cp_async_wait<PVS_SLOTS - 2>();                     // (one group per chunk from the fifth on, the empty ones at the end too)
             __syncthreads();
+            const int t1 = t0 + (PVS_SLOTS - 1) * VCH;
+            stage_v(t1, min(VCH, n_pad - t1), (k - 1) % PVS_SLOTS * VCH);
         }
         if (h0 < GQA) {
             const int steps = len / 16;
             const float * pr = ps + (size_t) h0 * n_pad + t0 + c;
-            const __half2 * vr = reinterpret_cast<const __half2 *>(&vs[(k & (PVS_SLOTS - 1)) * VCH + c][2 * dp]);
+            const __half * vr = &vs[k % PVS_SLOTS * VCH + c][DPT * dp];
 #pragma unroll 8
             for (int s = 0; s < steps; s++) {
-                const float2 v = __half22float2(vr[(size_t) s * 16 * (PVS_DIMS / 2)]);
+                float v[DPT];
+                if (DPT == 2) { const float2 u = __half22float2(*reinterpret_cast<const __half2 *>(vr + (size_t) s * 16 * PVS_DIMS)); v[0] = u.x; v[DPT - 1] = u.y; }
+                else v[0] = __half2float(vr[(size_t) s * 16 * PVS_DIMS]);
 #pragma unroll
                 for (int j = 0; j < HPT; j++) {
                     const float p = pr[(size_t) j * n_pad + 16 * s];
-                    acc[j][0] = __fmaf_rn(v.x, p, acc[j][0]);
-                    acc[j][1] = __fmaf_rn(v.y, p, acc[j][1]);
+#pragma unroll
+                    for (int i = 0; i < DPT; i++) acc[j][i] = __fmaf_rn(v[i], p, acc[j][i]);
                 }
             }
-        }
-        if (n_pad > PVS_SLOTS * VCH) {
-            __syncthreads();                                    // the slot is read
-            if (t0 + PVS_SLOTS * VCH < n_pad) stage_v(t0 + PVS_SLOTS * VCH, k & (PVS_SLOTS - 1));
-            else cp_async_commit();
         }
     }
     if (h0 < GQA) {
 #pragma unroll
-        for (int j = 0; j < HPT; j++) { red[h0 + j][c][2 * dp] = acc[j][0]; red[h0 + j][c][2 * dp + 1] = acc[j][1]; }
+        for (int j = 0; j < HPT; j++)
+#pragma unroll
+            for (int i = 0; i < DPT; i++) red[h0 + j][c][DPT * dp + i] = acc[j][i];
     }
     __syncthreads();
     trace_mark<TR>(a.trace, 4);

@@ -478,3 +478,18 @@ def test_steps_with_taps_report_a_product_that_gave_up(tmp_path):
                 c.decode(tokens, 0)
         _same(c.decode([5], 0), want, "logits after the failure")
     c.close(); m.close()
+
+
+@pytest.mark.parametrize("n_head,n_head_kv,longest", [(4, 4, 50176), (4, 2, 25088), (4, 1, 12544), (8, 1, 6272)])
+def test_a_token_early_in_the_longest_context(tmp_path, n_head, n_head_kv, longest):
+    """a context reserves shared memory for its longest score rows; a token that needs less of it decodes the bits of a small context"""
+    path = str(tmp_path / "m.gguf")
+    G.synth_llama(path, G.LlamaConfig(n_layer=1, n_embd=128 * n_head, n_head=n_head, n_head_kv=n_head_kv, n_ff=768, n_vocab=256, n_ctx_train=65536), "Q4_K_M", seed=5)
+    m = engine.Model(path)
+    small, large = engine.Context(m, 96), engine.Context(m, longest)
+    toks = np.random.default_rng(2).integers(0, 256, size=70).tolist()
+    for c in (small, large):
+        c.decode(toks[:60], 0)
+    for i in range(60, 70):
+        _same(large.decode([toks[i]], i), small.decode([toks[i]], i), f"token {i}")
+    small.close(); large.close(); m.close()

@@ -121,6 +121,12 @@ def test_attention_long_context_route_bit_exact(cfg, round_q):
         engine.set_attention_route(0)
 
 
+@pytest.mark.parametrize("cfg", [(2, 2, 50176), (2, 2, 12000), (4, 2, 25088), (8, 2, 12544), (8, 1, 6272), (8, 2, 7200), (2, 2, 14208), (2, 2, 11360), (2, 2, 11361)])
+def test_attention_where_v_goes_round_its_slots(cfg):
+    """soft-max . V of one token: the longest context of each number of heads per key head (slots of 96 to 352 positions), and V that just fits its four slots and just does not"""
+    _attention_case(cfg, False)
+
+
 def _attention_case(cfg, round_q):
     n_head, n_head_kv, n_kv = cfg
     hd = 128
