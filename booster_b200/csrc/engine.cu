@@ -1200,8 +1200,9 @@ static bool token_kernel_build(b200_ctx *) { return false; }
 template <int GQA> static void token_kernel_launch(b200_ctx *) { throw std::runtime_error("built without the per-token kernel"); }
 #endif
 // enqueue the layers of this stage (+ embedding on the first stage, + head on the last) for ONE token whose
-// scalars are in c->d_state (host_state, single-stage contexts: in c->h_state, from where k_embed takes them)
-static void enqueue_forward(b200_ctx * c, bool host_state = false) {
+// scalars are in c->d_state. Single-stage contexts: host_state, the scalars come from c->h_state; host_logits, the
+// logits go to c->h_logits as well
+static void enqueue_forward(b200_ctx * c, bool host_state = false, bool host_logits = false) {
     b200_model & m = *c->m;
     const int E = m.n_embd, HD = m.head_dim, KVD = m.n_head_kv * HD, QD = m.n_head * HD, FF = m.n_ff;
     if (m.has_embd() && want(KIND_EMBED)) {
@@ -1295,6 +1296,7 @@ static void enqueue_forward(b200_ctx * c, bool host_state = false) {
     if (m.has_head() && want(KIND_HEAD)) {
         g_kind = KIND_HEAD;
         MatvecArgs a = args_head(c);
+        if (host_logits) a.out_host = c->h_logits;
         launch_matvec(c, a, EPI_STORE);
         tap(c, "result_output", -1, c->logits, (size_t) m.n_vocab);
     }

@@ -117,6 +117,7 @@ struct MatvecArgs {
     int epi;                   // EPI_*: ONE kernel serves every mat-vec of the layer, so its code stays in the instruction cache
     // epilogue
     float * out;
+    float * out_host;          // EPI_STORE: the rows once more, into pinned host memory (nullptr: not)
     const float * resid;
     // EPI_QKV
     float * q_out;
@@ -799,6 +800,7 @@ __device__ __noinline__ void matvec_epilogue(const MatvecArgs & a, float val, in
     if (!own) return;
     if (a.epi == EPI_STORE) {
         a.out[row] = val;
+        if (a.out_host) a.out_host[row] = val;
     } else if (a.epi == EPI_RESID) {
         a.out[row] = __fadd_rn(val, pre0);                     // ggml_add(cur, inpSA / ffn_inp): llama.cpp:8865, 8901
     } else if (a.epi == EPI_SILU) {
