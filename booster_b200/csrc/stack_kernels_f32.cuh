@@ -1,5 +1,6 @@
 // stack_kernels_f32.cuh — float32 products on the tensor cores (sm_100a, tcgen05): Y = X W^T (+ bias), the operand layouts of k_gemm_simt_big.
 //
+// The method is that of Henry, Tang and Heinecke (Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations, 2019).
 // A float32 number is the sum of three bfloat16 ones, exactly: hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid (24 bits are 8 + 8 + 8; a number below 2^-110 loses what is below 2^-134).
 // A product of two takes six MMAs (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi; what is left out is below 2^-26 of it). The tensor cores add in float32 without rounding to
 // nearest, so an accumulator holds 64 terms of a sum only: the small products first, hi hi last, then it is added to registers. Against 64 bits that is as close as a
@@ -11,6 +12,7 @@
 // Measured (B200): 600 x 16000 x 1024 694 -> 156 us, 300 x 4096 x 1024 91 -> 35, 64 x 512 x 512 40 -> 16; scores of 512 tokens x 16 heads over windows of 1152 rows of 576: 260 -> 92.
 // Rows and columns of a tile that three parts do not hold (an infinity or a NaN, whose parts would be NaN; nothing but numbers below 2^-100, whose last part would be gone) are
 // done again by fmaf, and they alone: what an output is does not depend on the rows beside it. In every other row the parts that are gone are below 2^-33 of its largest number.
+// The loop only gathers the bits that have no plane; a tile that has any looks for its odd rows then (largest magnitudes kept per row in the loop: 4 us a tile more).
 #pragma once
 
 namespace b200 {
@@ -19,27 +21,66 @@ namespace stk {
 constexpr int F3_BM = 128, F3_BN = 128, F3_BK = 64, F3_WORKERS = 512, F3_THREADS = F3_WORKERS + 32;
 constexpr int F3_PLANE = 128 * F3_BK * 2, F3_STAGE = 6 * F3_PLANE, F3_SMEM = 2 * F3_STAGE + 1024;       // X hi, mid, lo | W hi, mid, lo; + alignment slack
 
-// the largest magnitude met so far; NaN once there was one
-__device__ __forceinline__ void f3_top(float & top, float x) { asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(x))); }
-// whether three parts do not hold a row with this largest number: it becomes an infinity as bfloat16, or is below 2^-100 (a row of zeros is held)
-__device__ __forceinline__ bool f3_off(float top) { const uint32_t t = __float_as_uint(top); return t >= 0x7f7f8000u || (t > 0u && t < 0x0d800000u); }
-// two numbers into a word of each plane
-__device__ __forceinline__ void f3_split(float x, float y, uint32_t & hi, uint32_t & mid, uint32_t & lo, float & top) {
+// two numbers into a word of each plane; lost takes the bits that have no plane (a number that is not finite as bfloat16 leaves the NaN of a subtraction, all ones)
+__device__ __forceinline__ void f3_split(float x, float y, uint32_t & hi, uint32_t & mid, uint32_t & lo, uint32_t & lost) {
     hi = pack_bf16(x, y);
     const float rx = x - __uint_as_float(hi << 16), ry = y - __uint_as_float(hi & 0xffff0000u);
     mid = pack_bf16(rx, ry);
     const float lx = rx - __uint_as_float(mid << 16), ly = ry - __uint_as_float(mid & 0xffff0000u);
     lo = __byte_perm(__float_as_uint(lx), __float_as_uint(ly), 0x7632u);
-    f3_top(top, x); f3_top(top, y);
+    lost |= __float_as_uint(lx) | __float_as_uint(ly);
+}
+
+// What a warp of a tile with odd numbers does for its 32 rows from mw and 32 columns from nb: rows and columns that three parts do not hold (a largest magnitude that is no
+// finite bfloat16 number, or below 2^-100 and not zero) are formed by fmaf, a lane per output, into again [row][33]. Returns their masks.
+__device__ __noinline__ uint2 f3_again(const float * X, int ldx, const float * W, int ldw, bool w_kn, int T, int N, int kbeg, int K, int mw, int nb, float * again) {
+    const int lane = threadIdx.x & 31;
+    const auto off = [](uint32_t top) { return top >= 0x7f7f8000u || (top > 0u && top < 0x0d800000u); };
+    const auto bits = [](float v) { return __float_as_uint(v) & 0x7fffffffu; };        // magnitudes and NaN are ordered as their bits
+    uint32_t x_off = 0, w_off = 0;
+#pragma unroll 1
+    for (int i = 0; i < 32; i++) {
+        uint32_t x = 0, w = 0;
+        for (int k = kbeg + lane; k < K; k += 32) {
+            if (mw + i < T) x = max(x, bits(X[(size_t) (mw + i) * ldx + k]));
+            if (nb + i < N && !w_kn) w = max(w, bits(W[(size_t) (nb + i) * ldw + k]));
+        }
+        if (off(__reduce_max_sync(0xffffffffu, x))) x_off |= 1u << i;
+        if (off(__reduce_max_sync(0xffffffffu, w))) w_off |= 1u << i;
+    }
+    if (w_kn) {
+        uint32_t w = 0;
+        if (nb + lane < N) for (int k = kbeg; k < K; k++) w = max(w, bits(W[(size_t) k * ldw + nb + lane]));
+        w_off = __ballot_sync(0xffffffffu, off(w));
+    }
+    const auto chain = [&](int m, int n) {
+        float v = 0.f;
+        if (m >= T || n >= N) return v;
+        const float * x = X + (size_t) m * ldx;
+#pragma unroll 4
+        for (int k = kbeg; k < K; k += 4) {             // (K is a multiple of 4)
+            const float4 u = *reinterpret_cast<const float4 *>(x + k);
+            float4 w;
+            if (w_kn) { const float * p = W + (size_t) k * ldw + n; w = make_float4(p[0], p[ldw], p[2 * (size_t) ldw], p[3 * (size_t) ldw]); }
+            else w = *reinterpret_cast<const float4 *>(W + (size_t) n * ldw + k);
+            v = fmaf(u.w, w.w, fmaf(u.z, w.z, fmaf(u.y, w.y, fmaf(u.x, w.x, v))));
+        }
+        return v;
+    };
+#pragma unroll 1
+    for (int i = 0; i < 32; i++) {                      // a row: lane = column, a column: lane = row
+        if (x_off >> i & 1) again[i * 33 + lane] = chain(mw + i, nb + lane);
+        if (w_off >> i & 1) again[lane * 33 + i] = chain(mw + lane, nb + i);
+    }
+    __syncwarp();
+    return make_uint2(x_off, w_off);
 }
 
 __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a, int * err, int ksplit = 1, float * __restrict__ part = nullptr) {
     extern __shared__ uint8_t f3_raw[];
     __shared__ __align__(8) uint64_t full[2], done[2];
     __shared__ uint32_t tmem_base_s;
-    __shared__ int failed_s;
-    __shared__ float x_top[F3_BM];             // largest magnitudes of the tile's rows of X and of W
-    __shared__ uint32_t w_top[F3_BN];
+    __shared__ int failed_s, odd_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t smem0 = (smem_addr(f3_raw) + 1023u) & ~1023u;
     uint8_t * const sm = f3_raw + (smem0 - smem_addr(f3_raw));
@@ -65,7 +106,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
     const int nk = (K - kbeg + F3_BK - 1) / F3_BK;      // at least one: ksplit <= slices
     volatile int * failed = &failed_s;
     if (tid == 0) {
-        failed_s = 0;
+        failed_s = 0; odd_s = 0;
         for (int s = 0; s < 2; s++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_addr(&full[s])), "r"(F3_WORKERS / 32) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&done[s])) : "memory");
@@ -73,7 +114,6 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (tid < F3_BN) w_top[tid] = 0u;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_addr(&tmem_base_s)), "r"(256u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -113,7 +153,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
         // ---- slices. Rows of X (and of W [N][K]): 16 threads a row, four rows a thread, 4 k each; a W [K][N]: a thread a column, 16 k
         float4 xr[4];
         float wr[16];
-        float xt[4] = {}, wt[4] = {};                           // of the rows (W [K][N]: of the column) this thread splits
+        uint32_t lost = 0;
         const int lr = tid >> 4, lk = tid & 15, wn = tid & 127, wk = (tid >> 7) * 16;
         const auto fetch = [&](int k0) {
             const int k = k0 + 4 * lk;
@@ -131,10 +171,10 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
                 for (int i = 0; i < 16; i++) wr[i] = n0 + wn < a.N && k0 + wk + i < K ? W[(size_t) (k0 + wk + i) * ldw + n0 + wn] : 0.f;
             }
         };
-        const auto store4 = [&](uint8_t * plane0, int row, float x, float y, float z, float w, float & top) {
+        const auto store4 = [&](uint8_t * plane0, int row, float x, float y, float z, float w) {
             uint32_t h[2], m[2], l[2];
-            f3_split(x, y, h[0], m[0], l[0], top);
-            f3_split(z, w, h[1], m[1], l[1], top);
+            f3_split(x, y, h[0], m[0], l[0], lost);
+            f3_split(z, w, h[1], m[1], l[1], lost);
             uint8_t * p = plane0 + row * 128 + (((lk >> 1) ^ (row & 7)) << 4) + (lk & 1) * 8;
             *reinterpret_cast<uint2 *>(p) = make_uint2(h[0], h[1]);
             *reinterpret_cast<uint2 *>(p + F3_PLANE) = make_uint2(m[0], m[1]);
@@ -166,15 +206,15 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
             uint8_t * st = sm + (c & 1) * F3_STAGE;             // free: slice c - 2 was drained
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                store4(st, lr + 32 * i, xr[i].x, xr[i].y, xr[i].z, xr[i].w, xt[i]);
-                if (!a.w_kn) store4(st + 3 * F3_PLANE, lr + 32 * i, wr[4 * i], wr[4 * i + 1], wr[4 * i + 2], wr[4 * i + 3], wt[i]);
+                store4(st, lr + 32 * i, xr[i].x, xr[i].y, xr[i].z, xr[i].w);
+                if (!a.w_kn) store4(st + 3 * F3_PLANE, lr + 32 * i, wr[4 * i], wr[4 * i + 1], wr[4 * i + 2], wr[4 * i + 3]);
             }
             if (a.w_kn) {
 #pragma unroll
                 for (int g = 0; g < 2; g++) {
                     uint32_t h[4], m[4], l[4];
 #pragma unroll
-                    for (int i = 0; i < 4; i++) f3_split(wr[8 * g + 2 * i], wr[8 * g + 2 * i + 1], h[i], m[i], l[i], wt[0]);
+                    for (int i = 0; i < 4; i++) f3_split(wr[8 * g + 2 * i], wr[8 * g + 2 * i + 1], h[i], m[i], l[i], lost);
                     uint8_t * p = st + 3 * F3_PLANE + wn * 128 + ((((wk >> 3) + g) ^ (wn & 7)) << 4);
                     *reinterpret_cast<uint4 *>(p) = make_uint4(h[0], h[1], h[2], h[3]);
                     *reinterpret_cast<uint4 *>(p + F3_PLANE) = make_uint4(m[0], m[1], m[2], m[3]);
@@ -188,46 +228,14 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
             if (c > 0) drain(c - 1);
         }
         drain(nk - 1);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {                           // 16 lanes share a row
-#pragma unroll
-            for (int o = 8; o; o >>= 1) {
-                f3_top(xt[i], __shfl_xor_sync(0xffffffffu, xt[i], o));
-                if (!a.w_kn) f3_top(wt[i], __shfl_xor_sync(0xffffffffu, wt[i], o));
-            }
-            if (lk == 0) {
-                x_top[lr + 32 * i] = xt[i];
-                if (!a.w_kn) w_top[lr + 32 * i] = __float_as_uint(wt[i]);
-            }
-        }
-        if (a.w_kn) atomicMax(&w_top[wn], __float_as_uint(wt[0]));      // (magnitudes and NaN are ordered as their bits)
+        if (lost & 0xffffu) odd_s = 1;
         asm volatile("bar.sync 1, %0;" :: "n"(F3_WORKERS) : "memory");
         const int mw = m0 + 32 * (warp & 3), m = mw + lane, nb = n0 + (warp >> 2) * 32;
-        const uint32_t x_off = __ballot_sync(0xffffffffu, f3_off(x_top[32 * (warp & 3) + lane])), w_off = __ballot_sync(0xffffffffu, f3_off(__uint_as_float(w_top[(warp >> 2) * 32 + lane])));
-        if (x_off | w_off) {                                    // a row: lane = column, a column: lane = row; through the slices' memory, which the MMAs are done with
+        if (odd_s) {                                            // through the slices' memory, which the MMAs are done with
             float * again = reinterpret_cast<float *>(sm) + warp * (32 * 33);
-            const auto chain = [&](int m, int n) {
-                float v = 0.f;
-                if (m >= T || n >= a.N) return v;
-                const float * x = X + (size_t) m * a.ldx;
-#pragma unroll 4
-                for (int k = kbeg; k < K; k += 4) {             // (K is a multiple of 4)
-                    const float4 u = *reinterpret_cast<const float4 *>(x + k);
-                    float4 w;
-                    if (a.w_kn) { const float * p = W + (size_t) k * ldw + n; w = make_float4(p[0], p[ldw], p[2 * (size_t) ldw], p[3 * (size_t) ldw]); }
-                    else w = *reinterpret_cast<const float4 *>(W + (size_t) n * ldw + k);
-                    v = fmaf(u.w, w.w, fmaf(u.z, w.z, fmaf(u.y, w.y, fmaf(u.x, w.x, v))));
-                }
-                return v;
-            };
-#pragma unroll 1
-            for (int i = 0; i < 32; i++) {
-                if (x_off >> i & 1) again[i * 33 + lane] = chain(mw + i, nb + lane);
-                if (w_off >> i & 1) again[lane * 33 + i] = chain(m, nb + i);
-            }
-            __syncwarp();
+            const uint2 off = f3_again(X, a.ldx, W, ldw, a.w_kn != 0, T, a.N, kbeg, K, mw, nb, again);
 #pragma unroll
-            for (int j = 0; j < 32; j++) if ((x_off >> lane | w_off >> j) & 1) acc[j] = again[lane * 33 + j];
+            for (int j = 0; j < 32; j++) if ((off.x >> lane | off.y >> j) & 1) acc[j] = again[lane * 33 + j];
         }
         if (m < T && !*failed) {
             const int ldy = ksplit > 1 ? a.N : a.ldy;
