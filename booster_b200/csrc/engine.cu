@@ -784,7 +784,7 @@ static bool matvec_q80_takes(const MatvecArgs & a) {
     return a.act_q8_0 && (a.norm_w == nullptr || a.k <= PRO_U * QV_WARPS * 256) && (size_t) qv_fixed_bytes(a.k) + (size_t) QV_TEAMS * 2 * 8 * 1088 <= QV_SMEM_BUDGET;
 }
 template <int NB>
-static void launch_matvec_q80_t(b200_ctx * c, MatvecArgs & a, bool pdl) {
+static void launch_matvec_q80_t(b200_ctx * c, MatvecArgs & a) {
     const int grid = std::max(1, std::min(a.n_units, c->sm_count));
     a.groups_per_cta = a.n_units > grid ? QV_TEAMS : 1;       // one unit per block: one team has the whole ring
     a.stages = (int) std::min<size_t>(QV_MAX_STAGES, (QV_SMEM_BUDGET - qv_fixed_bytes(a.k)) / ((size_t) a.groups_per_cta * NB * 1088));
@@ -793,7 +793,7 @@ static void launch_matvec_q80_t(b200_ctx * c, MatvecArgs & a, bool pdl) {
     raise_smem(k_matvec_q80<NB, false>, smem, attr, c->device);
     raise_smem(k_matvec_q80<NB, true>, smem, attr_t, c->device);
     a.trace = trace_slot(c, grid);
-    launch_fwd(a.trace ? k_matvec_q80<NB, true> : k_matvec_q80<NB, false>, dim3((unsigned) grid), dim3(QV_THREADS), smem, c->st, a, pdl);
+    launch_fwd(a.trace ? k_matvec_q80<NB, true> : k_matvec_q80<NB, false>, dim3((unsigned) grid), dim3(QV_THREADS), smem, c->st, a);
     c->launches++;
 }
 // what k_matvec_q80 and k_matvec_kq share of a launch's derived fields
@@ -805,12 +805,12 @@ static void matvec_lanes_args(const b200_ctx * c, MatvecArgs & a, int epi) {
     a.inv_k = (a.k & (a.k - 1)) == 0 ? 1.0 / (double) a.k : 0.0;
     a.err = c->pb.err;
 }
-static void launch_matvec_q80(b200_ctx * c, MatvecArgs a, int epi, bool pdl) {
+static void launch_matvec_q80(b200_ctx * c, MatvecArgs a, int epi) {
     matvec_lanes_args(c, a, epi);
     // stages of 16 blocks where k allows it: waits and arrivals are paid half as often as with 8 (whole token of an 8B model's 8 layers: 521 and 607 us); 32 leave
     // the large matrices a shorter ring (533 us)
-    if (a.tiles_unit % 16 == 0) launch_matvec_q80_t<16>(c, a, pdl);
-    else launch_matvec_q80_t<8>(c, a, pdl);
+    if (a.tiles_unit % 16 == 0) launch_matvec_q80_t<16>(c, a);
+    else launch_matvec_q80_t<8>(c, a);
 }
 // one token's product with K-quant matrices on k_matvec_kq: with a norm a vector that one pass of the block's warps holds, and room for two stages per team
 static bool matvec_kq_q6(const MatvecArgs & a) {
@@ -831,7 +831,7 @@ static bool matvec_kq_takes(const MatvecArgs & a) {
         && (size_t) kv_act_bytes(a.k, matvec_kq_q6(a)) + (size_t) kv_teams(2) * 2 * ((matvec_kq_tile(a) + 127) / 128 * 128) <= KV_SMEM_BUDGET;
 }
 template <int U, int R, int NB>
-static void launch_matvec_kq_t(b200_ctx * c, MatvecArgs & a, bool pdl) {
+static void launch_matvec_kq_t(b200_ctx * c, MatvecArgs & a) {
     const int grid = std::max(1, std::min(a.n_units, c->sm_count));
     const size_t fixed = (size_t) kv_act_bytes(a.k, matvec_kq_q6(a));
     a.groups_per_cta = std::min(kv_teams(R), (a.n_units + grid - 1) / grid);      // teams that have a unit share the ring's memory
@@ -845,21 +845,21 @@ static void launch_matvec_kq_t(b200_ctx * c, MatvecArgs & a, bool pdl) {
     raise_smem(k_matvec_kq<U, R, NB, false>, smem, attr, c->device);
     raise_smem(k_matvec_kq<U, R, NB, true>, smem, attr_t, c->device);
     a.trace = trace_slot(c, grid);
-    launch_fwd(a.trace ? k_matvec_kq<U, R, NB, true> : k_matvec_kq<U, R, NB, false>, dim3((unsigned) grid), dim3((unsigned) (KV_WARPS + a.groups_per_cta) * 32), smem, c->st, a, pdl);
+    launch_fwd(a.trace ? k_matvec_kq<U, R, NB, true> : k_matvec_kq<U, R, NB, false>, dim3((unsigned) grid), dim3((unsigned) (KV_WARPS + a.groups_per_cta) * 32), smem, c->st, a);
     c->launches++;
 }
-static void launch_matvec_kq(b200_ctx * c, MatvecArgs a, int epi, bool pdl) {
+static void launch_matvec_kq(b200_ctx * c, MatvecArgs a, int epi) {
     matvec_lanes_args(c, a, epi);
     const bool one = a.k <= KV_WARPS * 256;                     // a warp has one block of the vector
-    if (matvec_kq_rows(a, c->sm_count) == 2) { if (one) launch_matvec_kq_t<1, 2, 1>(c, a, pdl); else launch_matvec_kq_t<PRO_U, 2, 1>(c, a, pdl); }
-    else if (a.tiles_unit % 2 == 0) { if (one) launch_matvec_kq_t<1, 1, 2>(c, a, pdl); else launch_matvec_kq_t<PRO_U, 1, 2>(c, a, pdl); }
-    else { if (one) launch_matvec_kq_t<1, 1, 1>(c, a, pdl); else launch_matvec_kq_t<PRO_U, 1, 1>(c, a, pdl); }
+    if (matvec_kq_rows(a, c->sm_count) == 2) { if (one) launch_matvec_kq_t<1, 2, 1>(c, a); else launch_matvec_kq_t<PRO_U, 2, 1>(c, a); }
+    else if (a.tiles_unit % 2 == 0) { if (one) launch_matvec_kq_t<1, 1, 2>(c, a); else launch_matvec_kq_t<PRO_U, 1, 2>(c, a); }
+    else { if (one) launch_matvec_kq_t<1, 1, 1>(c, a); else launch_matvec_kq_t<PRO_U, 1, 1>(c, a); }
 }
-static void launch_matvec(b200_ctx * c, const MatvecArgs & a_in, int epi, bool pdl = true) {
+static void launch_matvec(b200_ctx * c, const MatvecArgs & a_in, int epi) {
     ProfScope ps(c);
     MatvecArgs a = a_in;
-    if (matvec_q80_takes(a)) return launch_matvec_q80(c, a, epi, pdl);
-    if (matvec_kq_takes(a)) return launch_matvec_kq(c, a, epi, pdl);
+    if (matvec_q80_takes(a)) return launch_matvec_q80(c, a, epi);
+    if (matvec_kq_takes(a)) return launch_matvec_kq(c, a, epi);
     const size_t smem = shape_matvec(a, epi, c->sm_count, MV_SMEM_BUDGET);
     static int prefill_env = -1;
     if (prefill_env < 0) { const char * e = getenv("BOOSTER_B200_PREFILL"); prefill_env = e ? atoi(e) : 0; }
@@ -876,7 +876,7 @@ static void launch_matvec(b200_ctx * c, const MatvecArgs & a_in, int epi, bool p
     }
     const int grid = std::max(1, std::min(a.n_units, c->sm_count));
     a.trace = trace_slot(c, grid);
-    launch_fwd(a.trace ? k_matvec<true> : k_matvec<false>, dim3((unsigned) grid), dim3((unsigned) (W * 32)), smem, c->st, a, pdl);
+    launch_fwd(a.trace ? k_matvec<true> : k_matvec<false>, dim3((unsigned) grid), dim3((unsigned) (W * 32)), smem, c->st, a);
     c->launches++;
 }
 
@@ -1200,16 +1200,16 @@ static bool token_kernel_build(b200_ctx *) { return false; }
 template <int GQA> static void token_kernel_launch(b200_ctx *) { throw std::runtime_error("built without the per-token kernel"); }
 #endif
 // enqueue the layers of this stage (+ embedding on the first stage, + head on the last) for ONE token whose
-// scalars are in c->d_state. Single-stage contexts: host_state, the scalars come from c->h_state; host_logits, the
-// logits go to c->h_logits as well
-static void enqueue_forward(b200_ctx * c, bool host_state = false, bool host_logits = false) {
+// scalars are in c->d_state. host_logits: the head's rows go to c->h_logits as well (not from the persistent kernel, whose
+// phases' arguments are fixed)
+static void enqueue_forward(b200_ctx * c, bool host_logits = false) {
     b200_model & m = *c->m;
     const int E = m.n_embd, HD = m.head_dim, KVD = m.n_head_kv * HD, QD = m.n_head * HD, FF = m.n_ff;
     if (m.has_embd() && want(KIND_EMBED)) {
         const int thr = 256;
         g_kind = KIND_EMBED;
         ProfScope ps(c);
-        k_embed<<<(E + thr - 1) / thr, thr, 0, c->st>>>(m.embd_type, m.embd_rows, m.embd_row_bytes, E, c->d_state, host_state ? c->h_state : nullptr, 0, c->x);
+        k_embed<<<(E + thr - 1) / thr, thr, 0, c->st>>>(m.embd_type, m.embd_rows, m.embd_row_bytes, E, c->d_state, 0, c->x);
         c->launches++;
     }
     // the persistent kernel runs everything after the embedding row; taps, per-launch profiling and the per-kernel phase
@@ -1240,7 +1240,7 @@ static void enqueue_forward(b200_ctx * c, bool host_state = false, bool host_log
                 pf_push(a.pf, pf_slice(L.wo.m.p0, tiled_bytes(L.wo.m), 0.0, pp.kvwo));
             }
 #endif
-            launch_matvec(c, a, EPI_QKV, !(host_state && li == 0));   // (the kernels behind it read the scalars ahead of their dependency wait: k_embed is over by then)
+            launch_matvec(c, a, EPI_QKV);
             tap(c, "Qcur", il, c->q, (size_t) QD);
         }
         if (want(KIND_ATTN) || want(KIND_ATTN_PV)) {   // attention
@@ -1296,7 +1296,7 @@ static void enqueue_forward(b200_ctx * c, bool host_state = false, bool host_log
     if (m.has_head() && want(KIND_HEAD)) {
         g_kind = KIND_HEAD;
         MatvecArgs a = args_head(c);
-        if (host_logits) a.out_host = c->h_logits;
+        if (host_logits) a.out_host = c->h_logits;      // (a matrix has whole units of 32 rows, so no row is past the vocabulary)
         launch_matvec(c, a, EPI_STORE);
         tap(c, "result_output", -1, c->logits, (size_t) m.n_vocab);
     }
@@ -2132,8 +2132,9 @@ extern "C" int b200_decode(b200_ctx * c, const int32_t * tokens, int n, int pos0
             }
             if (!c->g_logits) {
                 c->g_logits = capture(c, [&]() {
+                    CU(cudaMemcpyAsync(c->d_state, c->h_state, sizeof(DecodeState), cudaMemcpyHostToDevice, c->st));
                     enqueue_forward(c, true);
-                    CU(cudaMemcpyAsync(c->h_logits, c->logits, (size_t) m.n_vocab * 4, cudaMemcpyDeviceToHost, c->st));
+                    if (c->token_state > 0) CU(cudaMemcpyAsync(c->h_logits, c->logits, (size_t) m.n_vocab * 4, cudaMemcpyDeviceToHost, c->st));
                 }, &c->n_logits);
             }
             CU(cudaGraphLaunch(c->g_logits, c->st));
@@ -2231,7 +2232,8 @@ extern "C" int b200_step_greedy(b200_ctx * c, int32_t token, int pos, int32_t * 
         } else {
             if (!c->g_step) {
                 c->g_step = capture(c, [&]() {
-                    enqueue_forward(c, true);
+                    CU(cudaMemcpyAsync(c->d_state, c->h_state, sizeof(DecodeState), cudaMemcpyHostToDevice, c->st));
+                    enqueue_forward(c);
                     enqueue_argmax(c, 0);
                     CU(cudaMemcpyAsync(c->h_tok, c->d_out_tokens, 4, cudaMemcpyDeviceToHost, c->st));
                 }, &c->n_step);
@@ -2865,7 +2867,7 @@ extern "C" int b200_op_dequantize_row(int type, const void * w, int64_t k, float
         if (rb == 0) throw std::runtime_error("unsupported type");
         DBuf dw(rb), dy((size_t) k * 4);
         CU(cudaMemcpy(dw.p, w, rb, cudaMemcpyHostToDevice));
-        k_embed<<<(unsigned) ((k + 255) / 256), 256>>>(type, dw.as<uint8_t>(), rb, (int) k, nullptr, nullptr, 0, dy.as<float>());
+        k_embed<<<(unsigned) ((k + 255) / 256), 256>>>(type, dw.as<uint8_t>(), rb, (int) k, nullptr, 0, dy.as<float>());
         CU(cudaGetLastError());
         CU(cudaMemcpy(y, dy.p, (size_t) k * 4, cudaMemcpyDeviceToHost));
         return 0;

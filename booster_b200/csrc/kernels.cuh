@@ -800,6 +800,7 @@ __device__ __noinline__ void matvec_epilogue(const MatvecArgs & a, float val, in
     if (!own) return;
     if (a.epi == EPI_STORE) {
         a.out[row] = val;
+        // a copy node behind the head cost a token of an 8B model's 8 layers 5 us with a quarter of its vocabulary and 18 with all of it, a toy model's 3
         if (a.out_host) a.out_host[row] = val;
     } else if (a.epi == EPI_RESID) {
         a.out[row] = __fadd_rn(val, pre0);                     // ggml_add(cur, inpSA / ffn_inp): llama.cpp:8865, 8901
@@ -1407,18 +1408,11 @@ __device__ __forceinline__ float dequant_elem(int type, const uint8_t * row, int
         default: return 0.f;
     }
 }
-// from_host: the step's scalars in pinned host memory; every block reads them there, block 0 puts them where the token's other kernels look (st). A copy node in front
-// of the kernels, and one behind them for the logits, cost a token 4 us (toy model: 80 -> 76): the copy engine starts behind the graph's dependency, not beside the kernels.
+// (The step's scalars come by a copy node in front. Read by this kernel in pinned memory, with the first qkv joined to it plainly so that attention could read them ahead of its
+// wait, a toy model's token took as long and an 8B model's 8 layers 10 to 12 us more: the first kernels no longer overlapped.)
 __global__ void k_embed(int type, const uint8_t * __restrict__ rows, size_t row_bytes, int k,
-                        DecodeState * st, const DecodeState * from_host, int token_override, float * __restrict__ out) {
-    __shared__ int32_t token_s;
-    if (from_host && threadIdx.x < 2) {
-        const int4 v = __ldcv(reinterpret_cast<const int4 *>(from_host) + threadIdx.x);
-        if (blockIdx.x == 0) reinterpret_cast<int4 *>(st)[threadIdx.x] = v;
-        if (threadIdx.x == 0) token_s = v.x;
-    }
-    if (from_host) __syncthreads();
-    const int token = from_host ? token_s : st ? st->token : token_override;
+                        const DecodeState * __restrict__ st, int token_override, float * __restrict__ out) {
+    const int token = st ? st->token : token_override;
     const uint8_t * row = rows + (size_t) token * row_bytes;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) out[i] = dequant_elem(type, row, i);
 }

@@ -493,3 +493,16 @@ def test_a_token_early_in_the_longest_context(tmp_path, n_head, n_head_kv, longe
     for i in range(60, 70):
         _same(large.decode([toks[i]], i), small.decode([toks[i]], i), f"token {i}")
     small.close(); large.close(); m.close()
+
+
+@pytest.mark.parametrize("n_vocab", [32, 4128])
+def test_logits_written_by_the_head_are_those_it_keeps(tmp_path, n_vocab):
+    """a replayed step's head writes its rows to the host's buffer too: they are the rows that the step with taps copies from the device"""
+    path = str(tmp_path / "m.gguf")
+    G.synth_llama(path, G.LlamaConfig(n_layer=1, n_embd=512, n_head=4, n_head_kv=1, n_ff=768, n_vocab=n_vocab, n_ctx_train=256), "Q4_K_M", seed=5)
+    m = engine.Model(path)
+    a, b = engine.Context(m, 64), engine.Context(m, 64)
+    b.set_taps(True)
+    for pos, tok in enumerate([3, n_vocab - 1, 17]):
+        _same(a.decode([tok], pos), b.decode([tok], pos), f"token {pos}")
+    a.close(); b.close(); m.close()
