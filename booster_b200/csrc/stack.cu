@@ -1283,22 +1283,23 @@ constexpr int GX_MIN_K = 1024;
 struct UmmaScratch { __nv_bfloat16 * xb = nullptr; size_t elems = 0; int * err = nullptr; float * part = nullptr; size_t part_floats = 0; int sm_count = 148; };
 size_t umma_part_floats(int sm_count) { return (size_t) sm_count * UM_BM * UM_BN; }      // one K part of an output tile per SM
 
-// K parts of a float32 product with few output tiles (1: whole, in 64 x 64 tiles): two blocks of 128 x 128 per SM, 256 k each at least. (All parts together hold no
-// more than two tiles per SM, which is what umma_part_floats has room for.) In whole models of width 512 and 1024, where weights come from memory, no product of 64
-// to 600 tokens was faster whole (a pass of 64 tokens, the 512 x 512 products alone: 1959 us whole, 1861 in two parts; 1024 x 4096 2736 and 1398). Alone, 64 x 16000 is, up to
-// k = 1024: half of each tile's rows are empty, and there is room for two parts only (k = 512: 62 us whole, 68 in two parts; k = 2048: 234 and 226).
+// float32 tiles on the tensor cores (k_gemm_f32_umma) instead of the fp32 pipe: 64 tokens x 512 x 64 take 8.5 us here and 8.6 there, everything above is faster (600 x 16000 x 1024:
+// 694 and 156 us, 300 x 1024 x 4096 88 and 31). With less than half a tile's rows, columns or slice, the fp32 pipe's 64 x 64 tiles waste less.
+bool f32_umma_takes(bool vec, int T, int N, int K) { return vec && umma_enabled() && T >= 64 && N >= 64 && K >= 64; }
+// K parts of such a product (1: whole): as many as there are SMs for its tiles, one block each, of 256 k and more. Of 98 products of 64 to 600 tokens, 64 to 16000 rows and k = 512 to
+// 8192 none is slower so than whole, and whole they take up to five times as long (64 x 512 x 512 22.8 us whole, 20.6 in two parts; 300 x 1024 x 4096 110 and 35; where
+// the tiles fill the SMs there is one part: 64 x 16000 x 1024 39).
 int f32_k_parts(int T, int N, int K, int sm_count) {
-    if (T < 64 || N < SG_BN || !split_k_enabled() || !simt_big_enabled()) return 1;
-    const int room = 2 * sm_count / (((N + SG_BN - 1) / SG_BN) * ((T + SG_BM - 1) / SG_BM));
-    if (T <= 64 && room == 2 && K <= 1024) return 1;
-    return std::min(room, (K + SG_BK - 1) / SG_BK / 16);
+    if (N < F3_BN || !split_k_enabled()) return 1;
+    const int tiles = ((N + F3_BN - 1) / F3_BN) * ((T + F3_BM - 1) / F3_BM);
+    return std::max(1, std::min(sm_count / tiles, (K + 15) / 256));
 }
 // room for the parts of every product that a float32 model runs on portions of up to cap tokens
 size_t f32_part_floats(const StackModel & m, int cap, int sm_count) {
     size_t most = 0;
     for (const auto & nk : m.mats)
-        for (int t = SG_BM; t - SG_BM < cap; t += SG_BM) {
-            const int T = std::min(t, cap), parts = f32_k_parts(T, nk.first, nk.second, sm_count);
+        for (int t = F3_BM; t - F3_BM < cap; t += F3_BM) {
+            const int T = std::min(t, cap), parts = f32_umma_takes(nk.second % 4 == 0, T, nk.first, nk.second) ? f32_k_parts(T, nk.first, nk.second, sm_count) : 1;
             if (parts > 1) most = std::max(most, (size_t) parts * T * nk.first);
         }
     return most;
@@ -1319,9 +1320,6 @@ bool gx_pays(bool f32, int chunks, int N, int batch, bool glu, int sm_count) {
     const long long here = waves(GX_ROWS, resident[f32][c]), there = waves(16, 4);
     return 2 * here <= 3 * there && 16 * chunks >= (here == 1 && ch > 1 ? 12 : 14) * full;
 }
-// float32 tiles on the tensor cores (k_gemm_f32_umma) instead of the fp32 pipe: 64 tokens x 512 x 64 take 8.5 us here and 8.6 there, everything above is faster (600 x 16000 x 1024:
-// 694 and 156 us, 300 x 1024 x 4096 88 and 34). With less than half a tile's rows, columns or slice, the fp32 pipe's 64 x 64 tiles waste less.
-bool f32_umma_takes(bool vec, int T, int N, int K, const int * err) { return vec && err && umma_enabled() && T >= 64 && N >= 64 && K >= 64; }
 void launch_f32_umma(cudaStream_t st, const LinArgs & a, int * err, int batch, int parts = 1, float * part = nullptr) {
     static size_t have[64] = {0};
     raise_smem(k_gemm_f32_umma, F3_SMEM, have);
@@ -1334,15 +1332,15 @@ void split_sum(cudaStream_t st, const float * part, int parts, int T, int N, con
     else k_split_sum<1><<<grid, 256, 0, st>>>(part, parts, T, N, bias, Y, ldy);
 }
 // the kernel a product goes to: mat-vecs of few tokens, then tile kernels
-enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG, LIN_ROWS_X, LIN_UMMA, LIN_F32_PARTS, LIN_MMA, LIN_SIMT };
-// vec: LinArgs::vec; x_elems: entries of X; xb_elems, part_floats: what the scratch has room for
-LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu, bool seg, size_t x_elems, size_t xb_elems, size_t part_floats, int sm_count) {
+enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG, LIN_ROWS_X, LIN_UMMA, LIN_F32_PARTS, LIN_MMA, LIN_SIMT, LIN_F32_UMMA };
+// vec: LinArgs::vec; scratch: whether there is any (an error flag); x_elems: entries of X; xb_elems, part_floats: what the scratch has room for
+LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu, bool seg, bool scratch, size_t x_elems, size_t xb_elems, size_t part_floats, int sm_count) {
     if (T == 1 && vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && gx_pays(dtype == STACK_F32, K / (dtype == STACK_F32 ? 4 : 8), N, batch, glu, sm_count)) return LIN_ROWS_X;
     if (T <= GEMV_MAX_T) return !glu && batch == 1 && N <= GEMV_FEW_ROWS && K >= 1024 ? LIN_ROWS_LONG : LIN_ROWS;      // few, long rows: a block each
     if (dtype == STACK_BF16 && vec && umma_enabled() && T >= 64 && N >= 128 && K >= 64 && x_elems <= xb_elems) return LIN_UMMA;
-    if (dtype == STACK_F32 && vec && batch == 1 && !glu && !seg) {
-        const int parts = f32_k_parts(T, N, K, sm_count);
-        if (parts > 1 && (size_t) parts * T * N <= part_floats) return LIN_F32_PARTS;
+    if (dtype == STACK_F32 && scratch && f32_umma_takes(vec, T, N, K)) {
+        const int parts = batch == 1 && !glu && !seg ? f32_k_parts(T, N, K, sm_count) : 1;      // (a gated unit needs its sums whole)
+        return parts > 1 && (size_t) parts * T * N <= part_floats ? LIN_F32_PARTS : LIN_F32_UMMA;
     }
     return dtype == STACK_BF16 && vec && mma_enabled() ? LIN_MMA : LIN_SIMT;
 }
@@ -1389,7 +1387,7 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
     const auto al16 = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
     a.vec = K % vecw == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % vecw == 0 && al16(X) && al16(W);
     if (launches) (*launches)++;
-    const LinRoute route = lin_route(dtype, T, N, K, batch, a.vec != 0, a.glu != 0, a.seg != nullptr, (size_t) xbatch * T * K, us && us->xb ? us->elems : 0, us && us->part ? us->part_floats : 0, us ? us->sm_count : 148);
+    const LinRoute route = lin_route(dtype, T, N, K, batch, a.vec != 0, a.glu != 0, a.seg != nullptr, us && us->err, (size_t) xbatch * T * K, us && us->xb ? us->elems : 0, us && us->part ? us->part_floats : 0, us ? us->sm_count : 148);
     if (route == LIN_ROWS_X) {
         const int ch = gx_chunks(K / vecw);
         const dim3 grid((unsigned) ((N + GX_ROWS - 1) / GX_ROWS), 1, (unsigned) batch);
@@ -1426,16 +1424,12 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
         }
         else k_gemm_bf16_umma<<<grid, 256, UM_SMEM, st>>>(mx, mw, a, us->err);
         if (launches) (*launches)++;
-    } else if (route == LIN_F32_PARTS) {      // (a gated unit needs its sums whole: k_gemm_simt, 193 us against 236 in 128 x 128 tiles)
-        int f32_parts = f32_k_parts(T, N, K, us->sm_count);
-        const int tiles = ((N + F3_BN - 1) / F3_BN) * ((T + F3_BM - 1) / F3_BM);
-        if (f32_umma_takes(a.vec != 0, T, N, K, us->err)) {     // one block per SM
-            f32_parts = std::min(f32_parts, std::max(1, us->sm_count / tiles));
-            launch_f32_umma(st, a, us->err, 1, f32_parts, us->part);
-        } else k_gemm_simt_big<<<dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((T + SG_BM - 1) / SG_BM), (unsigned) f32_parts), 256, 0, st>>>(a, f32_parts, us->part);
-        if (f32_parts > 1) split_sum(st, us->part, f32_parts, T, N, bias, Y, ldy);
+    } else if (route == LIN_F32_PARTS) {
+        const int parts = f32_k_parts(T, N, K, us->sm_count);
+        launch_f32_umma(st, a, us->err, 1, parts, us->part);
+        split_sum(st, us->part, parts, T, N, bias, Y, ldy);
         if (launches) (*launches)++;
-    } else if (dtype == STACK_F32 && us && f32_umma_takes(a.vec != 0, T, N, K, us->err)) {
+    } else if (route == LIN_F32_UMMA) {
         launch_f32_umma(st, a, us->err, batch);
     } else if (route == LIN_MMA) {
         const dim3 grid((unsigned) ((N + MM_BN - 1) / MM_BN), (unsigned) ((T + MM_BM - 1) / MM_BM), (unsigned) batch);
@@ -1533,7 +1527,7 @@ void gemm_f32(StackCtx * c, const float * X, int ldx, long long sX, const float 
     LinArgs a{X, W, nullptr, Y, M, N, K, ldx, ldy, sX, sW, sY, 0, 0, 0.f, 0.f, w_kn, ldw, nz2, sX2, sW2, sY2};
     a.vec = K % 4 == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % 4 == 0 && sX2 % 4 == 0 && sW2 % 4 == 0 && ldw % 4 == 0 && al16(X) && al16(W);
     a.accum = accum; a.see_rows = see.rows; a.see_pos = see.pos; a.see_step = see.step; a.rows_all = rows_all;
-    if (f32_umma_takes(a.vec != 0, M, N, K, c->d_err)) launch_f32_umma(c->st, a, c->d_err, batch * nz2);
+    if (f32_umma_takes(a.vec != 0, M, N, K)) launch_f32_umma(c->st, a, c->d_err, batch * nz2);
     else if (a.vec && M >= SG_BM && N >= SG_BN && simt_big_enabled())       // operands that fill 128 x 128 tiles
         k_gemm_simt_big<<<dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((M + SG_BM - 1) / SG_BM), (unsigned) (batch * nz2)), 256, 0, c->st>>>(a);
     else k_gemm_simt<float><<<dim3((unsigned) ((N + 63) / 64), (unsigned) ((M + 63) / 64), (unsigned) (batch * nz2)), 256, 0, c->st>>>(a);
@@ -2864,7 +2858,7 @@ int32_t stack_argmax(StackCtx * c) {
 }
 
 int stack_product_kernel(int dtype, int T, int N, int K, bool glu, int sm_count) {
-    return lin_route(dtype, T, N, K, 1, K % (dtype == STACK_F32 ? 4 : 8) == 0, glu, false, 0, 0, SIZE_MAX, sm_count);
+    return lin_route(dtype, T, N, K, 1, K % (dtype == STACK_F32 ? 4 : 8) == 0, glu, false, true, 0, 0, SIZE_MAX, sm_count);
 }
 
 float stack_time_linear(int device, int dtype, int T, int N, int K, int reps) {

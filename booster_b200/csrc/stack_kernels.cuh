@@ -162,9 +162,9 @@ struct LinArgs {
     int vec;            // 1: K, ldx and all bases allow 16-byte loads
     int glu;            // GLU_*: rows of W are interleaved (2i: gate_i, 2i + 1: up_i); the epilogue writes a gated unit to Y[t][i] (N / 2 wide)
     float limit, alpha; //    GLU_SIGMOID: y_i = g sigmoid(alpha g) (u + up_shift), g = min(gate_i, limit), u = clamp(up_i, -limit, limit); GLU_GELU: gelu(gate_i) up_i
-    int w_kn, ldw;      // k_gemm_simt only. w_kn = 1: W is given [K][N] with row stride ldw (the attention's weights x cached rows);
+    int w_kn, ldw;      // float32 tile kernels. w_kn = 1: W is given [K][N] with row stride ldw (the attention's weights x cached rows);
                         // w_kn = 0 and ldw > 0: W is [N][K] with row stride ldw (keys inside wider cached rows)
-    int nz2 = 1;        // k_gemm_simt only: blockIdx.z = z1 * nz2 + z2, a second batch level with the strides below
+    int nz2 = 1;        // float32 tile kernels: blockIdx.z = z1 * nz2 + z2, a second batch level with the strides below
     long long sX2 = 0, sW2 = 0, sY2 = 0;
     float up_shift = 1.0f;
     // tile kernels: batch entry z works on rows seg[z] .. seg[z + 1] - 1 of X and Y (rows sorted by the matrix they meet: a routed
@@ -176,7 +176,7 @@ struct LinArgs {
     int x_share = 1;
     // k_gemv: entry z's input row is x_scale[z] times the row it reads (a routed expert that runs on a weighted input); no bias then
     const float * x_scale = nullptr;
-    int accum = 0;      // k_gemm_simt only: Y += the product (a second set of keys joining a weighted sum)
+    int accum = 0;      // float32 tile kernels: Y += the product (a second set of keys joining a weighted sum)
     // float32 tile kernels, see_rows > 0 (every earlier position is seen): row m of first-level entry z1 concerns positions 0 .. see_pos +
     // z1 see_step + m / see_rows only. Positions are the columns (w_kn = 0: tiles beyond their rows' last one are left alone) or the inner
     // dimension (w_kn = 1: the sum ends with the tile's last one, rounded up to 4; what lies up to there counts)
@@ -483,16 +483,14 @@ __global__ void __launch_bounds__(256) k_gemm_simt(const LinArgs a) {
 // heads): 256 threads with 8 x 8 outputs each (two 4 x 4 quarters 64 apart, so that the 16-byte shared-memory reads of a
 // half-warp stay free of bank conflicts), twice the FMAs per shared-memory read of the 64 x 64 kernel, the next K slice
 // of both operands in registers while the current one is multiplied. float32 operands with 16-byte aligned rows only (a.vec); no gated unit, no segments.
-// Products of float32 models whose tiles leave SMs idle run here too, cut along K like k_gemm_bf16_umma's (ksplit > 1: blockIdx.z is the part, sums to
-// part [ksplit][T][N], k_split_sum adds them): 300 tokens, 1024 rows, k = 4096: 355 us as 80 blocks of 64 x 64, 88 in twelve parts. Bound by the
-// shared-memory reads.
+// Bound by the shared-memory reads. (Where k is 64 and more as well k_gemm_f32_umma takes its place: this one is left for shorter ones.)
 constexpr int SG_BM = 128, SG_BN = 128, SG_BK = 16;
-__global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a, int ksplit = 1, float * __restrict__ part = nullptr) {
+__global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a) {
     __shared__ __align__(16) float Xs[SG_BK][SG_BM + 4];
     __shared__ __align__(16) float Ws[SG_BK][SG_BN + 4];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int m0 = blockIdx.y * SG_BM, n0 = blockIdx.x * SG_BN;
-    const int zb = ksplit > 1 ? 0 : blockIdx.z, z1 = zb / a.nz2, z2 = zb - z1 * a.nz2;
+    const int z1 = blockIdx.z / a.nz2, z2 = blockIdx.z - z1 * a.nz2;
     const float * X = a.X + (size_t) z1 * a.sX + (size_t) z2 * a.sX2;
     const float * W = reinterpret_cast<const float *>(a.W) + (size_t) z1 * a.sW + (size_t) z2 * a.sW2;
     const int ldw = a.ldw > 0 ? a.ldw : a.K;
@@ -501,12 +499,6 @@ __global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a, int k
         const int last = tile_sees(a, z1, m0, SG_BM);
         if (a.w_kn) K = min(K, (last + 4) / 4 * 4);
         else if (n0 > last) return;
-    }
-    int kbeg = 0;
-    if (ksplit > 1) {
-        const int nk = (K + SG_BK - 1) / SG_BK;
-        kbeg = (int) ((long long) nk * blockIdx.z / ksplit) * SG_BK;
-        K = min(K, (int) ((long long) nk * (blockIdx.z + 1) / ksplit) * SG_BK);
     }
     float acc[8][8];
 #pragma unroll
@@ -538,8 +530,8 @@ __global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a, int k
             }
         }
     };
-    fetch(kbeg);
-    for (int k0 = kbeg; k0 < K; k0 += SG_BK) {
+    fetch(0);
+    for (int k0 = 0; k0 < K; k0 += SG_BK) {
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const float xv[4] = { xr[h].x, xr[h].y, xr[h].z, xr[h].w };
@@ -566,9 +558,7 @@ __global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a, int k
         }
         __syncthreads();
     }
-    const int ldy = ksplit > 1 ? a.N : a.ldy;
-    const float * bias = ksplit > 1 ? nullptr : a.bias;
-    float * Y = ksplit > 1 ? part + (size_t) blockIdx.z * a.T * a.N : a.Y + (size_t) z1 * a.sY + (size_t) z2 * a.sY2;
+    float * Y = a.Y + (size_t) z1 * a.sY + (size_t) z2 * a.sY2;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
@@ -576,7 +566,7 @@ __global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a, int k
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const int n = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
-            if (n < a.N) Y[(size_t) m * ldy + n] = acc[i][j] + (bias ? bias[n] : 0.f) + (a.accum ? Y[(size_t) m * ldy + n] : 0.f);
+            if (n < a.N) Y[(size_t) m * a.ldy + n] = acc[i][j] + (a.bias ? a.bias[n] : 0.f) + (a.accum ? Y[(size_t) m * a.ldy + n] : 0.f);
         }
     }
 }

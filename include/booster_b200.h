@@ -125,7 +125,7 @@ void b200_reset_timings(b200_ctx * c);
  * negative on error. bench.py's per-kernel roofline of the family. */
 float b200_stack_time_linear(int device, int dtype, int T, int N, int K, int reps);
 /* the kernel such a product takes (glu: gate and up rows interleaved): 0 a warp per row, 1 a block per row, 2 a block per eight rows with x in
- * registers, 3 tcgen05, 4 float32 tiles in K parts, 5 mma.sync, 6 float32 tiles, -1 bad arguments (host arithmetic, tests) */
+ * registers, 3 tcgen05 (bfloat16), 4 tcgen05 (float32) in K parts, 5 mma.sync, 6 tiles on the fp32 pipe, 7 tcgen05 (float32) whole, -1 bad arguments (host arithmetic, tests) */
 int b200_stack_product_kernel(int dtype, int T, int N, int K, int glu, int sm_count);
 /* operator-level parity entry of the same products: y[T][N] = x[T][K] . w[N][K]^T (+ bias[N]); glu != 0: the rows of w are
  * interleaved (gate_i, up_i) and y is [T][N / 2], the clamped gated unit g sigmoid(1.702 g) (u + 1) with g = min(gate, limit),

@@ -61,7 +61,7 @@ def test_score_tile(kv, gqa, past, n, want):
     ([Q5_K], 4096, 4096, 32, 1), ([Q5_K, Q6_K], 2560, 2048, 33, 1), ([Q4_K], 768, 512, 100, 1), ([Q4_K], 4096, 1792, 8, 1),
     ([Q8_0], 4096, 4096, 32, 3), ([Q4_K], 96, 4096, 512, 0), ([Q4_K, Q8_0], 128, 4096, 32, 0)])
 def test_prompt_product_kernel(types, rows, k, T, want):
-    """which kernel a prompt product takes (2 tcgen05, 1 mma.sync, 3 Q8_0's mma.sync, 0 dp4a); an odd number of 32-row units goes to dp4a"""
+    """which kernel a prompt product takes (2 tcgen05, 1 mma.sync, 3 Q8_0's tcgen05, 0 dp4a); an odd number of 32-row units goes to dp4a"""
     assert _lib.lib().b200_op_prompt_kernel((C.c_int32 * len(types))(*types), len(types), rows // 32, k, T, 148) == want
 
 
@@ -76,10 +76,11 @@ BF16, F32 = 0, 1
     (BF16, 1, 16000, 16384, 0, 0), (F32, 1, 16000, 8192, 0, 0),                  # eight chunks a lane: 1.4 and 1.2 times
     (BF16, 1, 512, 2048, 0, 1), (BF16, 4, 16000, 2048, 0, 0), (BF16, 1, 2048, 2044, 0, 0),
     (F32, 300, 1024, 4096, 0, 4), (F32, 600, 1024, 512, 0, 4), (F32, 64, 4096, 2048, 0, 4),
-    (F32, 64, 512, 512, 0, 4), (F32, 64, 16000, 512, 0, 6), (F32, 64, 16000, 2048, 0, 4), (F32, 100, 16000, 512, 0, 4), (F32, 600, 4096, 4096, 0, 6),
-    (F32, 64, 512, 256, 0, 6), (F32, 300, 1024, 4096, 1, 6),
+    (F32, 64, 512, 512, 0, 4), (F32, 64, 512, 496, 0, 7), (F32, 64, 9472, 1024, 0, 4), (F32, 64, 9600, 1024, 0, 7), (F32, 64, 16000, 2048, 0, 7), (F32, 600, 4096, 4096, 0, 7),      # two blocks' worth of k, two SMs a tile
+    (F32, 64, 512, 256, 0, 7), (F32, 300, 1024, 4096, 1, 7), (F32, 64, 64, 64, 0, 7), (F32, 64, 64, 4096, 0, 7), (F32, 64, 128, 4096, 0, 4),
+    (F32, 63, 512, 512, 0, 6), (F32, 64, 63, 512, 0, 6), (F32, 64, 512, 60, 0, 6), (F32, 64, 512, 510, 0, 6),
     (BF16, 64, 128, 64, 0, 3), (BF16, 63, 128, 64, 0, 5), (BF16, 64, 128, 60, 0, 6)])
 def test_stack_product_kernel(dtype, T, N, K, glu, want):
-    """which kernel a layer stack's product takes: 0 a warp per row, 1 a block per row, 2 a block per eight rows with x in registers, 3 tcgen05, 4 float32
-    tiles in K parts, 5 mma.sync, 6 float32 tiles; the sizes on both sides of each line are among those measured"""
+    """which kernel a layer stack's product takes: 0 a warp per row, 1 a block per row, 2 a block per eight rows with x in registers, 3 tcgen05 (bfloat16), 4 and 7
+    tcgen05 (float32) in K parts and whole, 5 mma.sync, 6 tiles on the fp32 pipe; the sizes on both sides of each line are among those measured"""
     assert _lib.lib().b200_stack_product_kernel(dtype, T, N, K, glu, 148) == want
