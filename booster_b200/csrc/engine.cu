@@ -778,88 +778,106 @@ static size_t shape_matvec(MatvecArgs & a, int epi, int sm_count, size_t budget)
     return smem;
 }
 
-// one token's product with a Q8_0 matrix on k_matvec_q80: every row of it in Q8_0, and with a norm a vector that one pass of the block's warps holds
-static bool matvec_q80_takes(const MatvecArgs & a) {
-    for (int i = 0; i < a.n_seg; i++) if (a.seg[i].type != T_Q8_0) return false;
-    return a.act_q8_0 && (a.norm_w == nullptr || a.k <= PRO_U * QV_WARPS * 256) && (size_t) qv_fixed_bytes(a.k) + (size_t) QV_TEAMS * 2 * 8 * 1088 <= QV_SMEM_BUDGET;
+// Which kernel one token's product takes, and its launch there. k_matvec_q80: every row in Q8_0; k_matvec_kq: every row in a K-quant type; either where one pass of the block's
+// warps holds a vector that is normed (up to 16384 entries, which is as far as k_matvec goes too) and two stages per team fit beside the vector. k_matvec has what is left:
+// vectors without a norm of more than 58 368 entries with Q6_K, 143 616 with the other K-quants and 171 008 in Q8_0.
+enum MatvecKernel { MV_WARPS = 0, MV_Q80 = 1, MV_KQ = 2 };
+struct LanesShape {
+    int kernel = MV_WARPS;
+    int rows = 1, nb = 1;                   // rows per thread; tiles per stage of a ring
+    int teams = 1, stages = 0, stage_bytes = 0, grid = 0;
+    size_t smem = 0;
+};
+static LanesShape lanes_shape(const int * types, int n_types, int n_units, int k, bool norm, int epi, int sm_count) {
+    LanesShape s;
+    bool q80 = true, kq = true, q6 = false;
+    int tile = 0;
+    for (int i = 0; i < n_types; i++) {
+        q80 = q80 && types[i] == T_Q8_0;
+        kq = kq && (types[i] == T_Q4_K || types[i] == T_Q5_K || types[i] == T_Q6_K);
+        q6 = q6 || types[i] == T_Q6_K;
+        tile = std::max(tile, tile_bytes_of(types[i]));
+    }
+    s.grid = std::max(1, std::min(n_units, sm_count));
+    if (q80) {
+        const size_t fixed = (size_t) qv_fixed_bytes(k);
+        if ((norm && k > PRO_U * QV_WARPS * 256) || fixed + (size_t) QV_TEAMS * 2 * 8 * tile > QV_SMEM_BUDGET) return s;
+        s.kernel = MV_Q80;
+        // stages of 16 blocks where k allows it: waits and arrivals are paid half as often as with 8 (whole token of an 8B model's 8 layers: 521 and 607 us); 32 leave
+        // the large matrices a shorter ring (533 us)
+        s.nb = k / 32 % 16 == 0 ? 16 : 8;
+        s.teams = n_units > s.grid ? QV_TEAMS : 1;            // one unit per block: one team has the whole ring
+        s.stage_bytes = s.nb * tile;
+        s.stages = (int) std::min<size_t>(QV_MAX_STAGES, (QV_SMEM_BUDGET - fixed) / ((size_t) s.teams * s.stage_bytes));
+        s.smem = fixed + (size_t) s.teams * s.stages * s.stage_bytes;
+    } else if (kq) {
+        const size_t fixed = (size_t) kv_act_bytes(k, q6);
+        if ((norm && k > PRO_U * KV_WARPS * 256) || fixed + (size_t) kv_teams(2) * 2 * ((tile + 127) / 128 * 128) > KV_SMEM_BUDGET) return s;
+        s.kernel = MV_KQ;
+        // with more units of 32 rows per SM than the teams of one row per thread are, two rows: the vector's words are then read once for both (gate|up 14.9 us, with one
+        // 16.7). With fewer units two rows per thread halve the warps at work.
+        s.rows = n_units > kv_teams(1) * sm_count ? 2 : 1;
+        s.nb = s.rows == 1 && k / 256 % 2 == 0 ? 2 : 1;
+        s.teams = std::min(kv_teams(s.rows), (n_units + s.grid - 1) / s.grid);            // teams that have a unit share the ring's memory
+        s.stage_bytes = (s.nb * tile + 127) / 128 * 128;
+        // no more shared memory and warps than the launch uses: its blocks then start beside those of the kernel before (wo beside soft-max . V) and have weights on their way
+        const int steps = (n_units + s.grid * s.teams - 1) / (s.grid * s.teams) * (k / 256 / s.nb);
+        const size_t budget = KV_SMEM_BUDGET - (epi == EPI_QKV ? 8 * 1024 : 0);            // behind qkv a block of k_attn_scores fits beside it
+        s.stages = (int) std::min<size_t>(std::min(KV_MAX_STAGES, steps), (budget - fixed) / ((size_t) s.teams * s.stage_bytes));
+        s.smem = fixed + (size_t) s.teams * s.stages * s.stage_bytes;
+    }
+    return s;
+}
+// out: kernel (MatvecKernel), rows per thread, tiles per stage, teams, stages, blocks, dynamic shared memory (host arithmetic)
+extern "C" int b200_op_lanes_shape(const int32_t * types, int n_types, int64_t n_units, int64_t k, int norm, int qkv, int sm_count, int32_t out[7]) {
+    if (!types || n_types <= 0 || !out || n_units <= 0 || k <= 0 || k % 256 || sm_count <= 0) return set_err("bad arguments");
+    const LanesShape s = lanes_shape(types, n_types, (int) n_units, (int) k, norm != 0, qkv ? EPI_QKV : EPI_STORE, sm_count);
+    const int v[7] = {s.kernel, s.rows, s.nb, s.teams, s.stages, s.grid, (int) s.smem};
+    std::copy(v, v + 7, out);
+    return 0;
 }
 template <int NB>
-static void launch_matvec_q80_t(b200_ctx * c, MatvecArgs & a) {
-    const int grid = std::max(1, std::min(a.n_units, c->sm_count));
-    a.groups_per_cta = a.n_units > grid ? QV_TEAMS : 1;       // one unit per block: one team has the whole ring
-    a.stages = (int) std::min<size_t>(QV_MAX_STAGES, (QV_SMEM_BUDGET - qv_fixed_bytes(a.k)) / ((size_t) a.groups_per_cta * NB * 1088));
-    const size_t smem = (size_t) qv_fixed_bytes(a.k) + (size_t) a.groups_per_cta * a.stages * NB * 1088;
+static void launch_matvec_q80(b200_ctx * c, MatvecArgs & a, const LanesShape & s) {
     static size_t attr[64] = {0}, attr_t[64] = {0};
-    raise_smem(k_matvec_q80<NB, false>, smem, attr, c->device);
-    raise_smem(k_matvec_q80<NB, true>, smem, attr_t, c->device);
-    a.trace = trace_slot(c, grid);
-    launch_fwd(a.trace ? k_matvec_q80<NB, true> : k_matvec_q80<NB, false>, dim3((unsigned) grid), dim3(QV_THREADS), smem, c->st, a);
-    c->launches++;
-}
-// what k_matvec_q80 and k_matvec_kq share of a launch's derived fields
-static void matvec_lanes_args(const b200_ctx * c, MatvecArgs & a, int epi) {
-    a.epi = epi;
-    a.tiles_unit = a.seg[0].tiles_unit;
-    for (int i = 0; i < a.n_seg; i++)
-        if (a.seg[i].tiles_unit != a.tiles_unit) throw std::runtime_error("segments of one launch must share the unit shape");
-    a.inv_k = (a.k & (a.k - 1)) == 0 ? 1.0 / (double) a.k : 0.0;
-    a.err = c->pb.err;
-}
-static void launch_matvec_q80(b200_ctx * c, MatvecArgs a, int epi) {
-    matvec_lanes_args(c, a, epi);
-    // stages of 16 blocks where k allows it: waits and arrivals are paid half as often as with 8 (whole token of an 8B model's 8 layers: 521 and 607 us); 32 leave
-    // the large matrices a shorter ring (533 us)
-    if (a.tiles_unit % 16 == 0) launch_matvec_q80_t<16>(c, a);
-    else launch_matvec_q80_t<8>(c, a);
-}
-// one token's product with K-quant matrices on k_matvec_kq: with a norm a vector that one pass of the block's warps holds, and room for two stages per team
-static bool matvec_kq_q6(const MatvecArgs & a) {
-    for (int i = 0; i < a.n_seg; i++) if (a.seg[i].type == T_Q6_K) return true;
-    return false;
-}
-static int matvec_kq_tile(const MatvecArgs & a) {
-    int sb = 0;
-    for (int i = 0; i < a.n_seg; i++) sb = std::max(sb, tile_bytes_of(a.seg[i].type));
-    return sb;
-}
-// rows per thread: with more units of 32 rows per SM than the teams of one row per thread are, two: the vector's words are then read once for both (gate|up 14.9 us, with one
-// 16.7). With fewer units two rows per thread halve the warps at work.
-static int matvec_kq_rows(const MatvecArgs & a, int sm_count) { return a.n_units > kv_teams(1) * sm_count ? 2 : 1; }
-static bool matvec_kq_takes(const MatvecArgs & a) {
-    for (int i = 0; i < a.n_seg; i++) if (a.seg[i].type != T_Q4_K && a.seg[i].type != T_Q5_K && a.seg[i].type != T_Q6_K) return false;
-    return !a.act_q8_0 && (a.norm_w == nullptr || a.k <= PRO_U * KV_WARPS * 256)
-        && (size_t) kv_act_bytes(a.k, matvec_kq_q6(a)) + (size_t) kv_teams(2) * 2 * ((matvec_kq_tile(a) + 127) / 128 * 128) <= KV_SMEM_BUDGET;
+    raise_smem(k_matvec_q80<NB, false>, s.smem, attr, c->device);
+    raise_smem(k_matvec_q80<NB, true>, s.smem, attr_t, c->device);
+    a.trace = trace_slot(c, s.grid);
+    launch_fwd(a.trace ? k_matvec_q80<NB, true> : k_matvec_q80<NB, false>, dim3((unsigned) s.grid), dim3(QV_THREADS), s.smem, c->st, a);
 }
 template <int U, int R, int NB>
-static void launch_matvec_kq_t(b200_ctx * c, MatvecArgs & a) {
-    const int grid = std::max(1, std::min(a.n_units, c->sm_count));
-    const size_t fixed = (size_t) kv_act_bytes(a.k, matvec_kq_q6(a));
-    a.groups_per_cta = std::min(kv_teams(R), (a.n_units + grid - 1) / grid);      // teams that have a unit share the ring's memory
-    a.stage_bytes = (NB * matvec_kq_tile(a) + 127) / 128 * 128;
-    // no more shared memory and warps than the launch uses: its blocks then start beside those of the kernel before (wo beside soft-max . V) and have weights on their way
-    const int steps = (a.n_units + grid * a.groups_per_cta - 1) / (grid * a.groups_per_cta) * (a.tiles_unit / NB);
-    const size_t budget = KV_SMEM_BUDGET - (a.epi == EPI_QKV ? 8 * 1024 : 0);      // behind qkv a block of k_attn_scores fits beside it
-    a.stages = (int) std::min<size_t>(std::min(KV_MAX_STAGES, steps), (budget - fixed) / ((size_t) a.groups_per_cta * a.stage_bytes));
-    const size_t smem = fixed + (size_t) a.groups_per_cta * a.stages * a.stage_bytes;
+static void launch_matvec_kq(b200_ctx * c, MatvecArgs & a, const LanesShape & s) {
     static size_t attr[64] = {0}, attr_t[64] = {0};
-    raise_smem(k_matvec_kq<U, R, NB, false>, smem, attr, c->device);
-    raise_smem(k_matvec_kq<U, R, NB, true>, smem, attr_t, c->device);
-    a.trace = trace_slot(c, grid);
-    launch_fwd(a.trace ? k_matvec_kq<U, R, NB, true> : k_matvec_kq<U, R, NB, false>, dim3((unsigned) grid), dim3((unsigned) (KV_WARPS + a.groups_per_cta) * 32), smem, c->st, a);
-    c->launches++;
+    raise_smem(k_matvec_kq<U, R, NB, false>, s.smem, attr, c->device);
+    raise_smem(k_matvec_kq<U, R, NB, true>, s.smem, attr_t, c->device);
+    a.trace = trace_slot(c, s.grid);
+    launch_fwd(a.trace ? k_matvec_kq<U, R, NB, true> : k_matvec_kq<U, R, NB, false>, dim3((unsigned) s.grid), dim3((unsigned) (KV_WARPS + s.teams) * 32), s.smem, c->st, a);
 }
-static void launch_matvec_kq(b200_ctx * c, MatvecArgs a, int epi) {
-    matvec_lanes_args(c, a, epi);
+// false: k_matvec's
+static bool launch_matvec_lanes(b200_ctx * c, MatvecArgs a, int epi) {
+    int types[3];
+    for (int i = 0; i < a.n_seg; i++) {
+        types[i] = a.seg[i].type;
+        if (a.seg[i].tiles_unit != a.seg[0].tiles_unit) throw std::runtime_error("segments of one launch must share the unit shape");
+    }
+    const LanesShape s = lanes_shape(types, a.n_seg, a.n_units, a.k, a.norm_w != nullptr, epi, c->sm_count);
+    if (s.kernel == MV_WARPS || (s.kernel == MV_Q80) != (a.act_q8_0 != 0)) return false;
+    a.epi = epi;
+    a.tiles_unit = a.seg[0].tiles_unit;
+    a.inv_k = (a.k & (a.k - 1)) == 0 ? 1.0 / (double) a.k : 0.0;
+    a.err = c->pb.err;
+    a.groups_per_cta = s.teams; a.stages = s.stages; a.stage_bytes = s.stage_bytes;
     const bool one = a.k <= KV_WARPS * 256;                     // a warp has one block of the vector
-    if (matvec_kq_rows(a, c->sm_count) == 2) { if (one) launch_matvec_kq_t<1, 2, 1>(c, a); else launch_matvec_kq_t<PRO_U, 2, 1>(c, a); }
-    else if (a.tiles_unit % 2 == 0) { if (one) launch_matvec_kq_t<1, 1, 2>(c, a); else launch_matvec_kq_t<PRO_U, 1, 2>(c, a); }
-    else { if (one) launch_matvec_kq_t<1, 1, 1>(c, a); else launch_matvec_kq_t<PRO_U, 1, 1>(c, a); }
+    if (s.kernel == MV_Q80) { if (s.nb == 16) launch_matvec_q80<16>(c, a, s); else launch_matvec_q80<8>(c, a, s); }
+    else if (s.rows == 2) { if (one) launch_matvec_kq<1, 2, 1>(c, a, s); else launch_matvec_kq<PRO_U, 2, 1>(c, a, s); }
+    else if (s.nb == 2) { if (one) launch_matvec_kq<1, 1, 2>(c, a, s); else launch_matvec_kq<PRO_U, 1, 2>(c, a, s); }
+    else { if (one) launch_matvec_kq<1, 1, 1>(c, a, s); else launch_matvec_kq<PRO_U, 1, 1>(c, a, s); }
+    c->launches++;
+    return true;
 }
 static void launch_matvec(b200_ctx * c, const MatvecArgs & a_in, int epi) {
     ProfScope ps(c);
     MatvecArgs a = a_in;
-    if (matvec_q80_takes(a)) return launch_matvec_q80(c, a, epi);
-    if (matvec_kq_takes(a)) return launch_matvec_kq(c, a, epi);
+    if (launch_matvec_lanes(c, a, epi)) return;
     const size_t smem = shape_matvec(a, epi, c->sm_count, MV_SMEM_BUDGET);
     static int prefill_env = -1;
     if (prefill_env < 0) { const char * e = getenv("BOOSTER_B200_PREFILL"); prefill_env = e ? atoi(e) : 0; }

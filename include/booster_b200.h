@@ -231,8 +231,11 @@ int b200_stage_argmax(b200_ctx * c, int32_t * token_out);
 float * b200_stage_logits_view(b200_ctx * c);
 float * b200_decode_view(b200_ctx * c, int32_t token, int pos);
 
-/* launch shape (warps per CTA, warps sharing a 32-row unit, ring stages per warp) the engine picks for a mat-vec whose
- * segments have the given block types: pure host arithmetic, exposed so that tests pin the shapes */
+/* kernel and launch of one token's product whose segments have the given block types: out = kernel (0 k_matvec, 1 k_matvec_q80, 2 k_matvec_kq), rows per thread,
+ * tiles per stage, teams, stages, blocks, dynamic shared memory; n_units = rows / 32 (host arithmetic, exposed so that tests pin the shapes) */
+int b200_op_lanes_shape(const int32_t * types, int n_types, int64_t n_units, int64_t k, int norm, int qkv, int sm_count, int32_t out[7]);
+/* launch shape (warps per CTA, warps sharing a 32-row unit, ring stages per warp) of k_matvec, for the vectors that the two kernels above do not
+ * hold, and of the persistent per-token kernel's phases, whose shared memory is smaller: host arithmetic, as above */
 int b200_op_launch_shape(const int32_t * types, int n_types, int64_t n_units, int64_t k, int norm, int sm_count, int32_t wgs[3]);
 /* tokens per block of a prompt batch's score kernel: n tokens behind `past` cells (host arithmetic, as above) */
 int b200_op_score_tokens(int n_head_kv, int gqa, int past, int n, int sm_count);

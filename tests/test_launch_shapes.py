@@ -1,6 +1,8 @@
-"""The launch shape the engine picks for every mat-vec of the 8B, 70B and 7B models (warps per CTA, warps sharing a 32-row
-unit, ring stages per warp) — pure host arithmetic (b200_op_launch_shape), pinned here so that a change of the selection
-rule or of the shared-memory budget shows up as a deliberate diff. Q6_K tiles of 6.7 KB halve the warps that fit."""
+"""The launch shapes that the engine picks: pure host arithmetic, pinned here so that a change of a rule or of a shared-memory budget shows up as a deliberate diff.
+
+One token's products (b200_op_lanes_shape): every mat-vec of the 8B, 70B, 405B and 7B models goes to k_matvec_q80 or k_matvec_kq. k_matvec's own shapes (b200_op_launch_shape: warps
+per CTA, warps sharing a 32-row unit, ring stages per warp; the persistent per-token kernel's phases follow the same rule) are pinned at the same sizes. Q6_K tiles of 6.7 KB
+halve the warps that fit."""
 import ctypes as C
 
 import pytest
@@ -23,6 +25,62 @@ SHAPES = [
     ("Mistral-7B Q5_K_M gate|up",    [Q5_K],        896,  4096, 1, (16, 2, 2)),
     ("8B Q8_0 gate|up",              [Q8_0],        896,  4096, 1, (16, 2, 4)),
 ]
+
+
+LANES = [
+    # name,                    types,        units, k,    norm, qkv, (kernel, rows per thread, tiles per stage, teams, stages, blocks)
+    ("8B qkv, all Q4_K",       [Q4_K],        192,  4096, 1, 1, (2, 1, 2, 2, 8, 148)),
+    ("8B qkv, attn_v Q6_K",    [Q4_K, Q6_K],  192,  4096, 1, 1, (2, 1, 2, 2, 7, 148)),
+    ("8B wo",                  [Q4_K],        128,  4096, 0, 0, (2, 1, 2, 1, 8, 128)),        # as many stages as the walk has
+    ("8B gate|up",             [Q4_K],        896,  4096, 1, 0, (2, 2, 1, 7, 6, 148)),
+    ("8B ffn_down Q4_K",       [Q4_K],        128, 14336, 0, 0, (2, 1, 2, 1, 16, 128)),
+    ("8B ffn_down Q6_K",       [Q6_K],        128, 14336, 0, 0, (2, 1, 2, 1, 14, 128)),
+    ("8B output Q6_K",         [Q6_K],       4008,  4096, 1, 0, (2, 2, 1, 8, 4, 148)),
+    ("70B qkv, attn_v Q5_K",   [Q4_K, Q5_K],  320,  8192, 1, 1, (2, 1, 2, 3, 6, 148)),
+    ("70B ffn_down Q6_K",      [Q6_K],        256, 28672, 0, 0, (2, 1, 2, 2, 6, 148)),
+    ("405B qkv, attn_v Q6_K",  [Q4_K, Q6_K],  576, 16384, 1, 1, (2, 1, 2, 4, 3, 148)),
+    ("405B ffn_down Q6_K",     [Q6_K],        512, 53248, 0, 0, (2, 1, 2, 4, 2, 148)),
+    ("Mistral gate|up Q5_K",   [Q5_K],        896,  4096, 1, 0, (2, 2, 1, 7, 5, 148)),
+    ("8B Q8_0 gate|up",        [Q8_0],        896,  4096, 1, 0, (1, 1, 16, 2, 6, 148)),
+    ("8B Q8_0 ffn_down",       [Q8_0],        128, 14336, 0, 0, (1, 1, 16, 1, 12, 128)),
+    ("toy ffn_down",           [Q4_K],         16,   768, 0, 0, (2, 1, 1, 1, 3, 16)),         # an odd number of blocks: one to a stage
+    ("toy Q8_0 ffn_down",      [Q8_0],         16,   768, 0, 0, (1, 1, 8, 1, 24, 16)),
+    ("four teams' units",      [Q4_K],        592,  4096, 1, 0, (2, 1, 2, 4, 6, 148)),
+    ("one more",               [Q4_K],        593,  4096, 1, 0, (2, 2, 1, 5, 9, 148)),
+    ("longest Q6_K vector",    [Q6_K],        593, 58368, 0, 0, (2, 2, 1, 5, 3, 148)),
+    ("one block more",         [Q6_K],        593, 58624, 0, 0, (0, 1, 1, 1, 0, 148)),
+    ("longest normed vector",  [Q6_K],        192, 16384, 1, 1, (2, 1, 2, 2, 6, 148)),
+    ("Q8_0 beside a K-quant",  [Q4_K, Q8_0],  192,  4096, 0, 0, (0, 1, 1, 1, 0, 148)),
+]
+
+
+@pytest.mark.parametrize("name,types,units,k,norm,qkv,want", LANES, ids=[s[0] for s in LANES])
+def test_lanes_shape(name, types, units, k, norm, qkv, want):
+    out = (C.c_int32 * 7)()
+    assert _lib.lib().b200_op_lanes_shape((C.c_int32 * len(types))(*types), len(types), units, k, norm, qkv, 148, out) == 0
+    assert tuple(out[:6]) == want
+
+
+@pytest.mark.parametrize("sm_count", [1, 20, 132, 148])
+@pytest.mark.parametrize("types", [[Q4_K], [Q5_K], [Q6_K], [Q4_K, Q6_K], [Q5_K, Q6_K], [Q8_0]], ids=str)
+def test_every_lanes_shape_is_one_the_kernel_takes(types, sm_count):
+    """what the kernels assume of a launch, over rows of 1 to 5000 units and vectors of one block to past the longest: stages that divide the vector, a stage and a unit for every team,
+    rings and teams within the barriers' arrays, shared memory within a block's, and a normed vector in one pass"""
+    L, out = _lib.lib(), (C.c_int32 * 7)()
+    q80 = types[0] == Q8_0
+    for k in list(range(256, 6400, 256)) + [8192, 14336, 16384, 16640, 28672, 53248, 57088, 58112, 58368, 143616, 171008, 171264]:
+        for units in (1, 2, 15, 16, 17, 19, 20, 21, 64, 131, 132, 133, 148, 149, 296, 297, 591, 592, 593, 896, 1184, 1185, 4008, 5000):
+            for norm in (0, 1):
+                assert L.b200_op_lanes_shape((C.c_int32 * len(types))(*types), len(types), units, k, norm, 1, sm_count, out) == 0
+                kernel, rows, nb, teams, stages, blocks, smem = out
+                if kernel == 0:
+                    assert (norm and k > 16384) or k > 50000
+                    continue
+                assert kernel == (1 if q80 else 2) and not (norm and k > 16384)
+                assert blocks == min(units, sm_count) and 1 <= teams and (teams - 1) * blocks < units
+                assert (k // (32 if q80 else 256)) % nb == 0
+                assert teams <= (2 if q80 else 4 * rows) and 1 <= stages <= (24 if q80 else 16)
+                assert smem + (1024 if q80 else 2560) <= 227 * 1024
 
 
 @pytest.mark.parametrize("name,types,units,k,norm,want", SHAPES, ids=[s[0] for s in SHAPES])

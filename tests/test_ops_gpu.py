@@ -279,11 +279,12 @@ def test_mul_mat_vec_q8_0_edges(shape):
 
 
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K"])
-@pytest.mark.parametrize("shape", [(32, 256), (96, 768), (4736, 512), (4768, 256), (9504, 768), (14240, 1280), (64, 14336), (160, 17408), (4768, 9216)])
+@pytest.mark.parametrize("shape", [(32, 256), (96, 768), (4736, 512), (4768, 256), (9504, 768), (14240, 1280), (64, 14336), (160, 17408), (4768, 9216),
+                                   (18944, 512), (18976, 512), (18976, 4352), (37888, 256), (37920, 256), (37952, 2304)])
 def test_mul_mat_vec_k_quant_edges(name, shape):
-    """k_matvec_kq where its teams and rings end: one block of K, stages of one and of two blocks, as many units of 32 rows as SMs and one more (a block's second team),
-    more than both teams take at once, rings that go round, vectors of one and of several blocks per warp and of more than one pass, worst-case weights — the
-    reference's bits"""
+    """k_matvec_kq where its teams and rings end: one block of K, stages of one and of two blocks, as many units of 32 rows as SMs and one more (a block's second team), as many as
+    the four teams of one row per thread and one more (two rows per thread from there), as many as their eight teams and one more (a team's second unit, taken by some), rings
+    that go round, vectors of one and of several blocks per warp and of more than one pass, worst-case weights — the reference's bits"""
     n, k = shape
     rng = np.random.default_rng(n + k)
     w = _extreme_blocks(name, n, k, rng)
@@ -294,6 +295,19 @@ def test_mul_mat_vec_k_quant_edges(name, shape):
     y = engine.op_mul_mat_vec(TYPES[name], w.reshape(-1), n, k, x)
     yr = port.mul_mat_vec(TYPES[name], w.reshape(-1), n, k, x)
     assert np.array_equal(y, yr), f"max abs diff {np.abs(y - yr).max()}"
+
+
+@pytest.mark.parametrize("name,shape", [("Q6_K", (64, 58368)), ("Q6_K", (64, 58624)), ("Q6_K", (4800, 60160)), ("Q8_0", (64, 171008)), ("Q8_0", (64, 171264))])
+def test_mul_mat_vec_long_vectors(name, shape):
+    """the longest vectors that the kernels with a chain per thread hold, and longer ones, which k_matvec takes — the reference's bits"""
+    n, k = shape
+    out = (C.c_int32 * 7)()
+    assert _lib.lib().b200_op_lanes_shape((C.c_int32 * 1)(TYPES[name]), 1, n // 32, k, 0, 0, 148, out) == 0
+    assert (out[0] == 0) == (k > (58368 if name == "Q6_K" else 171008))
+    rng = np.random.default_rng(k)
+    w = G.random_blocks(rng, TYPES[name], n, k).reshape(-1)
+    x = rng.standard_normal(k).astype(np.float32)
+    assert np.array_equal(engine.op_mul_mat_vec(TYPES[name], w, n, k, x), port.mul_mat_vec(TYPES[name], w, n, k, x))
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
