@@ -567,7 +567,6 @@ struct b200_ctx {
     float * q = nullptr;        // [n_head*hd]
     float * att = nullptr;      // kqv_merged_cont [n_head*hd]
     float * ffh = nullptr;      // silu(gate)*up [n_ff]
-    float * warm_x = nullptr;   // constant vector [max(n_ff, n_embd)] read by the prologue's dry run (B200_WARM)
     float * logits = nullptr;   // [n_vocab]
     float * S = nullptr;        // attention scores / probabilities [n_head][n_ctx]
     unsigned int * tickets = nullptr;
@@ -1007,43 +1006,6 @@ static void tap(b200_ctx * c, const std::string & name, int il, const float * dp
     c->tapstore.v[name + "-" + std::to_string(il)] = std::move(h);
 }
 
-// L2 look-ahead plan (kernels.cuh PfRange): which later kernel's bytes each kernel of a layer prefetches into L2.
-//   QKV      -> this layer's K and V rows 0..pos, wo                      (consumed by scores, softmax+P.V, wo)
-//   scores   -> gate|up, first part        softmax+P.V -> gate|up, middle        wo -> gate|up, rest
-//   gate|up  -> down                       down        -> the next layer's QKV stack (or the head's first tiles)
-// The short kernels between two big mat-vecs are latency-bound and leave HBM idle; with the plan HBM streams the whole
-// time and the big mat-vecs find (most of) their tiles in L2. BOOSTER_B200_PF="kvwo,gu_scores,gu_pv,gu_wo,down,next"
-// (fractions of the consumer's bytes, 0 = off) tunes it; BOOSTER_B200_PF=0 disables the look-ahead.
-struct PfPlan { float kvwo = 1.f, gu_scores = 0.f, gu_pv = 0.f, gu_wo = 0.f, down = 0.f, next = 1.f; };
-static const PfPlan & pf_plan() {
-    static PfPlan p; static bool init = false;
-    if (!init) {
-        init = true;
-        if (const char * e = getenv("BOOSTER_B200_PF")) {
-            float v[6] = {0, 0, 0, 0, 0, 0};
-            const int n = sscanf(e, "%f,%f,%f,%f,%f,%f", &v[0], &v[1], &v[2], &v[3], &v[4], &v[5]);
-            if (n == 1 && v[0] == 0.f) { p = PfPlan{0, 0, 0, 0, 0, 0}; }
-            else if (n == 6) { p = PfPlan{v[0], v[1], v[2], v[3], v[4], v[5]}; }
-        }
-    }
-    return p;
-}
-static size_t tiled_bytes(const TMat & m) { return (size_t) m.n_units * m.tiles_unit * m.tile_bytes; }
-static size_t tiled_bytes(const DevStack & s) { size_t n = 0; for (int i = 0; i < s.n_seg; i++) n += tiled_bytes(s.seg[i]); return n; }
-// bytes [from, to) (fractions) of a tiled matrix as a look-ahead range, cut at tile-size-independent 16-byte multiples
-static PfRange pf_slice(const uint8_t * base, size_t total, double from, double to) {
-    PfRange r{nullptr, 0, 0};
-    from = std::min(1.0, std::max(0.0, from)); to = std::min(1.0, std::max(from, to));
-    const size_t b0 = (size_t) (total * from) / 8192 * 8192, b1 = to >= 1.0 ? total : (size_t) (total * to) / 8192 * 8192;
-    if (b1 <= b0) return r;
-    r.p = base + b0; r.bytes = (uint32_t) std::min<size_t>(b1 - b0, 0xfffffff0u);
-    return r;
-}
-static void pf_push(PfRange (&pf)[PF_RANGES], const PfRange & r) {
-    if (!r.bytes) return;
-    for (int i = 0; i < PF_RANGES; i++) if (!pf[i].bytes) { pf[i] = r; return; }
-}
-
 // arguments of the mat-vecs of one layer / of the head (shared by the per-kernel path and the persistent kernel's plan)
 static MatvecArgs args_qkv(b200_ctx * c, int li) {
     b200_model & m = *c->m; LayerW & L = m.layers[(size_t) li];
@@ -1241,23 +1203,12 @@ static void enqueue_forward(b200_ctx * c, bool host_logits = false) {
         }
         return;
     }
-    const PfPlan & pp = pf_plan();
     for (int li = 0; li < (int) m.layers.size(); li++) {
         LayerW & L = m.layers[(size_t) li];
         const int il = m.layer_begin + li;
-        const size_t gu_bytes = tiled_bytes(L.gateup.m);
-        (void) pp; (void) gu_bytes;
         if (want(KIND_QKV)) {   // QKV
             g_kind = KIND_QKV;
             MatvecArgs a = args_qkv(c, li);
-#if B200_LOOKAHEAD
-            if (pp.kvwo > 0.f) {
-                const uint32_t row = (uint32_t) KVD * 2, all = (uint32_t) std::min<size_t>((size_t) c->n_ctx * row, 0xfffffff0u);
-                pf_push(a.pf, PfRange{(const uint8_t *) c->kc[(size_t) li], all, row});
-                pf_push(a.pf, PfRange{(const uint8_t *) c->vc[(size_t) li], all, row});
-                pf_push(a.pf, pf_slice(L.wo.m.p0, tiled_bytes(L.wo.m), 0.0, pp.kvwo));
-            }
-#endif
             launch_matvec(c, a, EPI_QKV);
             tap(c, "Qcur", il, c->q, (size_t) QD);
         }
@@ -1269,44 +1220,24 @@ static void enqueue_forward(b200_ctx * c, bool host_logits = false) {
             a.n_head = m.n_head; a.n_head_kv = m.n_head_kv; a.head_dim = HD; a.kv_dim = KVD;
             a.scale = 1.0f / sqrtf((float) HD);
             a.st = c->d_state; a.n_kv_override = 0; a.round_q_override = 0; a.cell_pos = c->d_cell_pos;
-#if B200_LOOKAHEAD
-            pf_push(a.pf,  pf_slice(L.gateup.m.p0, gu_bytes, 0.0, pp.gu_scores));
-            pf_push(a.pf2, pf_slice(L.gateup.m.p0, gu_bytes, pp.gu_scores, pp.gu_scores + pp.gu_pv));
-#endif
             launch_attention(c, a, c->n_ctx);
             tap(c, "kqv_merged_cont", il, c->att, (size_t) QD);
         }
         if (want(KIND_WO)) {   // wo + residual
             g_kind = KIND_WO;
             MatvecArgs a = args_wo(c, li);
-#if B200_LOOKAHEAD
-            pf_push(a.pf, pf_slice(L.gateup.m.p0, gu_bytes, pp.gu_scores + pp.gu_pv, pp.gu_scores + pp.gu_pv + pp.gu_wo));
-#endif
             launch_matvec(c, a, EPI_RESID);
             tap(c, "ffn_inp", il, c->x, (size_t) E);
         }
         if (want(KIND_GATEUP)) {   // gate/up (interleaved virtual matrix) + SiLU*mul
             g_kind = KIND_GATEUP;
             MatvecArgs a = args_gateup(c, li);
-#if B200_LOOKAHEAD
-            pf_push(a.pf, pf_slice(L.down.m.p0, tiled_bytes(L.down.m), 0.0, pp.down));
-#endif
             launch_matvec(c, a, EPI_SILU);
             tap(c, "ffn_gate_par", il, c->ffh, (size_t) FF);
         }
         if (want(KIND_DOWN)) {   // down + residual
             g_kind = KIND_DOWN;
             MatvecArgs a = args_down(c, li);
-#if B200_LOOKAHEAD
-            if (li + 1 < (int) m.layers.size()) {
-                const DevStack & nq = m.layers[(size_t) li + 1].qkv;
-                pf_push(a.pf, pf_slice(nq.seg[0].p0, tiled_bytes(nq), 0.0, pp.next));
-            } else if (m.has_head()) {
-                // the head is 431 MB: only its first tiles (what the layer stack's look-ahead depth allows)
-                const size_t hb = tiled_bytes(m.output.m);
-                pf_push(a.pf, pf_slice(m.output.m.p0, hb, 0.0, pp.next * std::min(1.0, 32.0e6 / (double) hb)));
-            }
-#endif
             launch_matvec(c, a, EPI_RESID);
             tap(c, "l_out", il, c->x, (size_t) E);
         }
@@ -1383,12 +1314,6 @@ extern "C" b200_ctx * b200_ctx_new(b200_model * m, int n_ctx) {
         CU(cudaMalloc(&c->q, (size_t) QD * 4));
         CU(cudaMalloc(&c->att, (size_t) QD * 4));
         CU(cudaMalloc(&c->ffh, (size_t) m->n_ff * 4));
-        {
-            std::vector<float> w((size_t) std::max(m->n_ff, m->n_embd));
-            for (size_t i = 0; i < w.size(); i++) w[i] = 0.25f + 0.001f * (float) (i % 97);
-            CU(cudaMalloc(&c->warm_x, w.size() * 4));
-            CU(cudaMemcpy(c->warm_x, w.data(), w.size() * 4, cudaMemcpyHostToDevice));
-        }
         CU(cudaMalloc(&c->logits, (size_t) m->n_vocab * 4));
         CU(cudaMalloc(&c->S, (size_t) m->n_head * c->n_ctx * 4));
         CU(cudaMalloc(&c->tickets, (size_t) m->n_head_kv * 4));
@@ -1446,7 +1371,7 @@ extern "C" void b200_ctx_free(b200_ctx * c) {
     cudaFree(c->inbox); cudaFree(c->p2p_counts);
     for (auto p : c->kc) cudaFree(p);
     for (auto p : c->vc) cudaFree(p);
-    cudaFree(c->x); cudaFree(c->q); cudaFree(c->att); cudaFree(c->ffh); cudaFree(c->warm_x); cudaFree(c->logits);
+    cudaFree(c->x); cudaFree(c->q); cudaFree(c->att); cudaFree(c->ffh); cudaFree(c->logits);
     cudaFree(c->d_cell_pos);
     cudaFree(c->pb.X); cudaFree(c->pb.Q); cudaFree(c->pb.ATT); cudaFree(c->pb.FFH); cudaFree(c->pb.S); cudaFree(c->pb.rec); cudaFree(c->pb.tokens);
     cudaFree(c->d_trace); cudaFree(c->d_plan); cudaFree(c->d_bar); cudaFree(c->S_T); cudaFree(c->d_ttrace);

@@ -38,12 +38,6 @@
 #ifndef B200_CHAIN_UNROLL
 #define B200_CHAIN_UNROLL 1
 #endif
-#ifndef B200_LOOKAHEAD
-#define B200_LOOKAHEAD 0     // L2 look-ahead prefetches (PfRange): measured neutral-to-negative on B200
-#endif
-#ifndef B200_WARM
-#define B200_WARM 0          // dry run of the prologue before griddepcontrol.wait (instruction-cache warm-up)
-#endif
 
 namespace b200 {
 
@@ -79,15 +73,6 @@ struct alignas(16) DecodeState {
 };
 
 enum { EPI_STORE = 0, EPI_RESID = 1, EPI_QKV = 2, EPI_SILU = 3 };
-
-// L2 look-ahead: a byte range of HBM that a LATER kernel of the token will stream (its weight tiles, this layer's K/V
-// rows). Every kernel of the forward pass carries up to PF_RANGES of them and turns them into bulk L2 prefetches in its
-// data-independent prologue, so that HBM keeps streaming while the (short, latency-bound) kernels in between wait on
-// each other; the consumer then finds its tiles in the 126 MB L2. per_pos != 0: the range grows with the position
-// (K/V rows 0..pos): bytes = min(bytes, (pos + 1) * per_pos).
-static constexpr int PF_RANGES = 3;
-static constexpr uint32_t PF_CHUNK = 8192;
-struct PfRange { const uint8_t * p; uint32_t bytes; uint32_t per_pos; };
 
 struct MatvecArgs {
     TMat seg[3];
@@ -126,8 +111,6 @@ struct MatvecArgs {
     int n_q, n_k, head_dim, kv_dim;
     const float2 * rope;       // [n_ctx][head_dim/2] (cos, sin)
     const DecodeState * st;
-    PfRange pf[PF_RANGES];     // L2 look-ahead for the kernels that follow (bytes == 0: unused)
-    const float * warm_x;      // B200_WARM: constant vector of k floats for the dry run of the prologue (nullptr: no dry run)
     unsigned long long * trace; // nullptr unless b200_trace_token is running
     int * err;                 // raised when a bounded wait ran out (the host reads it after its synchronisation)
 };
@@ -526,7 +509,6 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
 #endif
     } while (!ok);
 }
-// global -> shared bulk copy (TMA engine, no registers, no per-lane addressing); completes `bytes` on `bar`
 // mbarrier wait with an iteration limit: past it *failed is raised (every other wait of the CTA then gives up too), *err tells the host, and
 // the kernel runs to its end without storing
 __device__ __forceinline__ bool um_try(uint32_t bar, uint32_t parity) {
@@ -543,13 +525,14 @@ __device__ __forceinline__ void um_wait(uint32_t bar, uint32_t parity, volatile 
     *failed = 1;
     atomicExch_system(err, 1);
 }
+// global -> shared bulk copy (TMA engine, no registers, no per-lane addressing); completes `bytes` on `bar`
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
 // the same copy with an L2 evict-first hint: a tile is read exactly once per token, so after the copy its lines are the
-// preferred victims and the look-ahead data that has NOT been consumed yet stays resident
+// preferred victims
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
     uint64_t pol;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
@@ -558,24 +541,6 @@ __device__ __forceinline__ uint64_t l2_policy_evict_first() {
 __device__ __forceinline__ void bulk_g2s_hint(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar, uint64_t pol) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
                  :: "r"(dst), "l"(src), "r"(bytes), "r"(bar), "l"(pol) : "memory");
-}
-
-// L2 look-ahead (PfRange): lane 0 of warp `wid` (of `n_w` issuing warps in the whole grid) prefetches chunks wid,
-// wid + n_w, ... of every range — the ranges arrive front first, in the order their consumer walks them
-__device__ __forceinline__ void l2_prefetch_bulk(const void * p, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(p), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void issue_l2_lookahead(const PfRange (&pf)[PF_RANGES], int wid, int n_w, int pos) {
-#pragma unroll 1
-    for (int r = 0; r < PF_RANGES; r++) {
-        uint32_t bytes = pf[r].bytes;
-        if (bytes == 0) continue;
-        if (pf[r].per_pos) bytes = min(bytes, (uint32_t) (pos + 1) * pf[r].per_pos);
-        bytes &= ~15u;
-#pragma unroll 1
-        for (uint32_t off = (uint32_t) wid * PF_CHUNK; off < bytes; off += (uint32_t) n_w * PF_CHUNK)
-            l2_prefetch_bulk(pf[r].p + off, min(PF_CHUNK, bytes - off));
-    }
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -1153,12 +1118,6 @@ __global__ void __launch_bounds__(MV_MAX_WARPS * 32, 1) k_matvec(const __grid_co
         }
     }
 
-    // L2 look-ahead for the kernels that follow (after this CTA's own first tiles are requested). DecodeState is
-    // written by the previous TOKEN's last kernel, so pos may be read before the wait.
-#if B200_LOOKAHEAD
-    if (lane == 0 && a.pf[0].bytes) issue_l2_lookahead(a.pf, warp * gridDim.x + blockIdx.x, W * gridDim.x, a.st ? a.st->pos : 0);
-#endif
-
     trace_mark<TR>(a.trace, 1);
     pdl_wait();                                                // x (and everything else the previous kernels wrote) is visible
     trace_mark<TR>(a.trace, 2);
@@ -1447,8 +1406,6 @@ struct AttnArgs {
     int n_kv_override;        // >0: use instead of st->pos+1 (operator-level test)
     int round_q_override;     // operator-level test of the batch>1 arithmetic
     int p_chunk;              // k_attn_pv: positions of p staged in shared memory (multiple of PV_BATCH); k_attn_softmax_pv: its shared memory in units of 16 bytes
-    PfRange pf[PF_RANGES];    // L2 look-ahead issued by k_attn_scores
-    PfRange pf2[PF_RANGES];   // ... and by k_attn_softmax_pv
     const int32_t * cell_pos; // [n_ctx] position held by each KV cell (-1: empty); read only when st->managed
     // prompt batches: blockIdx.z = token of the batch; token z uses q + z*zq, S + z*zs, out + z*zq and attends
     // n_kv_override + z cells (its own position included). All zero for a single token.
@@ -1489,10 +1446,6 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attn_scores(const AttnArgs a) {
 #pragma unroll
         for (int s = 0; s < 8; s++) kv[s] = __ldg(kr + s * 4);            // 4 halfs at element 16s + 4c4
     }
-#if B200_LOOKAHEAD
-    if ((tid & 31) == 0 && a.pf[0].bytes)
-        issue_l2_lookahead(a.pf, (tid >> 5) * (gridDim.x * gridDim.y) + tile * gridDim.x + g, (ATT_THREADS / 32) * gridDim.x * gridDim.y, n_kv - 1);
-#endif
     pdl_wait();                                               // q and this token's K row come from the QKV kernel
     pdl_launch_dependents();                                  // AFTER the wait: the next kernel may touch K/V/q before ITS wait
     trace_mark<TR>(a.trace, 1);
@@ -1708,10 +1661,6 @@ __global__ void __launch_bounds__(GQA * pvs_th(GQA)) k_attn_softmax_pv(const Att
         cp_async_commit();
     };
     stage_v(0, min(n_pad, PVS_SLOTS * VCH), 0);
-#if B200_LOOKAHEAD
-    if (lane == 0 && a.pf2[0].bytes)
-        issue_l2_lookahead(a.pf2, (tid >> 5) * (gridDim.x * gridDim.y) + slice * gridDim.x + g, (NT / 32) * gridDim.x * gridDim.y, n_kv - 1);
-#endif
     pdl_wait();                                               // the raw scores are complete
     trace_mark<TR>(a.trace, 1);
     float * row = ps + (size_t) h * n_pad;
