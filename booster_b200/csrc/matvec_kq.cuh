@@ -5,11 +5,13 @@
 // registers, a row's are in four neighbouring threads, and nothing is exchanged before the row is finished, then by shuffles. A warp is 8 R rows, its weight words are 128
 // consecutive bytes of the tile; 32 rows are a team of 4 / R warps with a ring and a copying warp of its own.
 // Scales go in pairs: two four-byte sums fit 16 bits each (<= 4 * 32 * 127), one dp2a multiplies both by their scales.
-// What bounds it: with several units of 32 rows per SM HBM (gate|up of an 8B model, 66 MB: 11.3 us, 5.9 TB/s, 2.5 of them before the vector is quantized), with one unit
-// the team's four warps, one per scheduler: 300 clocks a super-block of which 105 issue (down 8.7 us behind the quantizer). Copies are 9 KB where two super-blocks make a
-// stage: a bulk copy costs 210 to 230 clocks of the copy engine however small it is, 4.6 KB ones end at 20 bytes a clock and SM.
-// Measured (B200, token of an 8B model's 8 layers at 2000): 508 us with k_matvec (a thread = a row, K split over warps that exchange the integers), 476 here; gate|up
-// 16.7 -> 12.9, qkv 9.0 -> 6.7, down 15.6 -> 13.2. One lane per thread (eight warps a unit): 507. Four teams taking a unit's super-blocks in turn and four warps for the
+// What bounds it: with several units of 32 rows per SM the issue slots (gate|up of an 8B model, 66 MB: 67 % of them busy, DRAM at 46 %, alone and cold under ncu), with one unit
+// the team's four warps, one per scheduler: 300 clocks a super-block of which 105 issue. Copies are 9 KB where two super-blocks make a stage: a bulk copy costs 210 to 230
+// clocks of the copy engine however small it is, 4.6 KB ones end at 20 bytes a clock and SM.
+// Measured (B200, an 8B model's 8 layers at 2000; launches of one kind back to back, k_matvec, a thread = a row, K split over warps that exchange the integers, and this one): qkv
+// 8.5 and 7.3 us, wo 5.2 and 5.5, gate|up 15.8 and 14.9 (4.4 TB/s), down 15.2 and 13.3, head 20.9 and 20.0; the token 509 and 467. Models of width 512 to 8192: tokens 0.77 to
+// 0.95 of the time; alone two rows per thread are behind k_matvec at k of 3072 and more (gate|up up to 9 %) and a Q6_K head of 4096 rows at k = 5120 and 6144 (3 to 8 %).
+// One lane per thread (eight warps a unit): 507 us a token against 485 when it was tried. Four teams taking a unit's super-blocks in turn and four warps for the
 // chains: 521. The next super-block's words read ahead into registers: 510.
 #pragma once
 #include "matvec_q80.cuh"

@@ -6,7 +6,8 @@
 // gives a thread all eight lanes of a row and splits K over warps, which hand the chains over after every 32 weights: a bulk copy, a wait and a hand-over per 1088 bytes.)
 // 32 rows are 256 threads, a team: warp = eight rows x four lanes, so that a warp's weights are 128 consecutive bytes of the tile.
 // What bounds it: HBM where there are several units of 32 rows per SM, else the instructions of the eight warps that a unit has, 9 per weight word.
-// Measured (B200, 8 layers of an 8B model, token at 333): 967 us with k_matvec, 521 us here; gate|up (125 MB) 22 us of which 18 behind the wait, down (62 MB) 12.
+// Measured (B200, 8 layers of an 8B model, token at 333): 968 us with k_matvec, 515 here; launches of one kind back to back gate|up (125 MB) 37.6 and 22.4 us, down (62 MB)
+// 36.1 and 13.1, wo 12.2 and 5.8. Alone and cold under ncu gate|up has DRAM at 57 % and 47 % of the issue slots busy.
 // Reading a stage's words ahead of adding the one before: 630 against 607 with stages of eight blocks.
 #pragma once
 #include "kernels.cuh"

@@ -8,8 +8,10 @@
 //   workers   16 warps: float32 slices of both operands from global memory (the next one's loads in flight), split, 16-bit planes into shared memory in the 128-byte swizzle;
 //             then the sums of the slice before last out of tensor memory (two accumulators) into registers
 //   MMA warp  24 tcgen05.mma of 128 x 128 x 16 per slice of 64 k
-// What bounds it: the MMAs, 65 clocks each (375 TFLOP/s of float32 products on all SMs); the fp32 pipe's tiles in k_gemm_simt_big reach 42.
-// Measured (B200): 600 x 16000 x 1024 694 -> 156 us, 300 x 4096 x 1024 91 -> 35, 64 x 512 x 512 40 -> 16; scores of 512 tokens x 16 heads over windows of 1152 rows of 576: 260 -> 92.
+// What bounds it: one block per SM whose slice is a chain (load, split and store, hand-over, MMAs, drain) that two stages overlap in part only: under ncu 50 % of the issue slots and
+// 23 to 31 % of the tensor pipe are busy (512 x 8192 x 1024 in 84 us). The MMAs alone, 65 clocks each, would allow 375 TFLOP/s of float32 products; 600 x 16000 x 1024 reach 126.
+// Measured (B200), the fp32 pipe's tiles and this: 600 x 16000 x 1024 694 and 156 us, 300 x 4096 x 1024 91 and 35, 64 x 512 x 512 40 and 16; scores of 512 tokens x 16 heads over
+// windows of 1152 rows of 576 260 and 92. A long sum in one block is where the odd rows' check shows: 64 x 64 x 4096 97 us without it, 103 with.
 // Rows and columns of a tile that three parts do not hold (an infinity or a NaN, whose parts would be NaN; nothing but numbers below 2^-100, whose last part would be gone) are
 // done again by fmaf, and they alone: what an output is does not depend on the rows beside it. In every other row the parts that are gone are below 2^-33 of its largest number.
 // The loop only gathers the bits that have no plane; a tile that has any looks for its odd rows then (largest magnitudes kept per row in the loop: 4 us a tile more).
