@@ -640,13 +640,13 @@ def main():
             pc.close()
             pm = float(np.mean(pms[1:]))
             line["prompt_batch"] = {"tokens": 512, "ms": pm, "tokens_per_s": 512e3 / pm,
-                                    "kernels": ("k_quant_batch_mma + k_mma_batch_q80 (block-diagonal fp16 HMMA: exact 4-byte lane sums)" if ftype == "Q8_0" else
+                                    "kernels": ("k_quant_batch_mma + k_umma_batch_q80 (block-diagonal fp16 tcgen05 products: exact 4-byte lane sums)" if ftype == "Q8_0" else
                                                 "k_quant_batch_mma + k_umma_batch (exact fp16 tcgen05 products per AVX2 lane-slice, A operand in tensor memory)") +
                                                " + k_attn_scores_batch / k_attn_softmax_rows / k_attn_pv_batch",
                                     "what": "b200_decode of one 512-token batch at positions 0..511, wall clock incl. the final synchronisation"}
-            try:   # tensor-pipe utilisation of the batch mat-mul kernel from the committed ncu --set full capture
+            try:   # tensor-pipe utilisation of the batch mat-mul kernel from the committed ncu capture
                 with open(os.path.join(ROOT, "profiles", "prefill_tensor.json")) as f:
-                    line["prompt_batch"]["tensor_pipe"] = json.load(f)["k_mma_batch_q80" if ftype == "Q8_0" else "k_umma_batch"]
+                    line["prompt_batch"]["tensor_pipe"] = json.load(f)["k_umma_batch_q80" if ftype == "Q8_0" else "k_umma_batch"]
             except Exception:
                 pass
         except Exception as e:
@@ -695,17 +695,17 @@ def main():
         gu_ms = acc["gate_up"][0] / acc["gate_up"][1]
         achieved = gu_bytes / (gu_ms * 1e-3) / 1e9
         tot_ms = sum(v[0] for v in acc.values()) / reps
-        # DRAM traffic of one gate|up launch from the committed ncu --set full capture (profiles/traffic.json, written by
-        # scripts/ncu_summary.py): dram__bytes_read.sum + dram__bytes_write.sum (8B Q4_K_M shapes)
+        # DRAM traffic of one gate|up launch from the committed ncu capture (profiles/traffic.json): dram__bytes_read.sum + dram__bytes_write.sum (8B Q4_K_M shapes)
+        gu_kernel = "k_matvec_q80" if ftype == "Q8_0" else "k_matvec_kq"
         traffic = None
         try:
             with open(os.path.join(ROOT, "profiles", "traffic.json")) as f:
                 tj = json.load(f)["gate_up"]
-            if args.config == DEFAULT_CONFIG:
+            if args.config == DEFAULT_CONFIG and tj["kernel"] == gu_kernel:
                 traffic = tj["dram_bytes_read"] + tj["dram_bytes_write"]
         except Exception:
             pass
-        line["roofline"] = {"bound": "hbm", "kernel": "k_matvec_kq / k_matvec_q80, EPI_SILU (ffn gate|up, fused RMSNorm + activation quant + SiLU*mul)",
+        line["roofline"] = {"bound": "hbm", "kernel": gu_kernel + ", EPI_SILU (ffn gate|up, fused RMSNorm + activation quant + SiLU*mul)",
                             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                             "peak_source": peak_src, "bytes_per_launch": float(gu_bytes), "ms_per_launch": gu_ms,
                             "share_of_token_time": acc["gate_up"][0] / reps / tot_ms}

@@ -1,5 +1,7 @@
 """Print the key metrics of an .ncu-rep (read here, no GPU needed): python scripts/ncu_summary.py file.ncu-rep"""
 import csv
+import os
+import re
 import subprocess
 import sys
 
@@ -38,7 +40,7 @@ if len(sys.argv) > 2:
     scale = {"byte": 1.0, "Kbyte": 1e3, "Mbyte": 1e6, "Gbyte": 1e9}
     out_j = {}
     for name, row in zip(names, rows[2:]):
-        out_j[name] = {"kernel": row[hdr.index('Kernel Name')], "dram_bytes_read": float(row[ir]) * scale[units[ir]],
+        out_j[name] = {"kernel": re.match(r"(?:void )?(\w+)", row[hdr.index('Kernel Name')]).group(1), "dram_bytes_read": float(row[ir]) * scale[units[ir]],
                        "dram_bytes_write": float(row[iw]) * scale[units[iw]], "ncu_duration_us": float(row[it]),
-                       "source": sys.argv[1]}
+                       "source": os.path.basename(sys.argv[1])}
     json.dump(out_j, open(sys.argv[2], "w"), indent=1)
