@@ -488,6 +488,12 @@ def main():
     if args.impl == "reference":
         if rank != 0:
             return 0
+        try:
+            from oracle import ref
+            ref.lib()
+        except Exception:
+            print(json.dumps({"impl": "reference", "unavailable": "the reference's CPU library is not built (make -C oracle ref needs the reference's sources)"}))
+            return 0
         # the reference's CPU path: the 8B Q4_K_M file, ctx 512 — the config says what ran
         path = model_path()
         tps, info = cpu_reference_run(path, args.steps, args.warmup)
