@@ -1809,6 +1809,11 @@ static void pb_matmul(b200_ctx * c, const MatvecArgs & mv, int epi, int T, int p
     if (mma_mode >= 2) {
         a.um_tok_tiles = (T + UM_NT - 1) / UM_NT;
         for (int i = 0; i < mv.n_seg; i++) a.um_row_tiles += (mv.seg[i].n_units + 3) / 4;
+        // Q8_0: while every half of a token tile can have an SM of its own it gets one (17 to 32 tokens, 4 layers of width 4096 with as wide a feed-forward: 971 us with the
+        // mma.sync kernel of 64-row tiles before, 1018 in whole tiles, 900 in halves; 64 tokens 1050 and 996; whole models of width 512 to 8192, 17 to 256 tokens: 0.89 to
+        // 0.99 of the time). A second wave costs more than it saves.
+        const int halves = (T + UM_NT / 2 - 1) / (UM_NT / 2);
+        if (mma_mode == 3 && T > UM_NT / 2 && a.um_row_tiles * halves <= c->sm_count) { a.um_halves = 1; a.um_tok_tiles = halves; }
         a.err = c->pb.err;
     }
     if (mma_mode == 3) {

@@ -424,6 +424,7 @@ struct MatmulBatchArgs {
     uint32_t mb_a_bytes, mb_raw_stride, mb_stage_bytes, mb_rec_copy;
     int mb_stages;
     int um_row_tiles, um_tok_tiles;       // k_umma_batch: 128-row tiles (of every segment by itself), 32-token tiles
+    int um_halves;                        // k_umma_batch_q80: 1: um_tok_tiles counts halves of 16 tokens
     int * err;                            // raised by a kernel whose bounded wait ran out
 };
 

@@ -14,7 +14,8 @@
 // Measured (B200, 8 layers of an 8B model, 512 tokens): 32.0 ms of products with mma.sync (64 x 32 tiles, fragments through shared memory), 20.2 ms here.
 //
 // Persistent, one CTA per SM, four warpgroups (setmaxnreg: 2 x 224 + 40 + 24 registers x 128 threads = the launch's 512 x 128):
-//   warps 0-7   consume: one output row and 16 tokens per thread; its eight chains per token are 128 registers
+//   warps 0-7   consume: one output row and 16 tokens per thread; its eight chains per token are 128 registers. A half of a tile without tokens, or whose tokens another
+//               block has (um_halves), is only handed over
 //   warps 8-11  expand: lane = row of a 32-row unit, int8 -> fp16 -> tcgen05.st, two blocks at a time (pfull)
 //   warp 12     bulk copies of raw tiles and activation records into a ring of stages of four blocks (full / empty)
 //   warps 13,15 MMAs of half 0 / 1 of each block (dfull), once its operands are there and the consumers have drained the buffer (dfree). One issuer for both: 23.4 ms.
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch_q80(const __grid_c
             mbar_expect_tx(bar, (uint32_t) t.n_units * UQ_RAW + UQ_STAGE_BLOCKS * UQ_BLOCK_REC);
             for (int u = 0; u < t.n_units; u++) bulk_g2s(dst + u * UQ_RAW, src + (size_t) u * a.tiles_unit * 1088, UQ_RAW, bar);
         }
-        if (recs) bulk_g2s(dst + 4 * UQ_RAW, a.rec + ((size_t) tt * a.tiles_unit + step * UQ_STAGE_BLOCKS) * UQ_BLOCK_REC, UQ_STAGE_BLOCKS * UQ_BLOCK_REC, bar);
+        if (recs) bulk_g2s(dst + 4 * UQ_RAW, a.rec + ((size_t) (tt >> a.um_halves) * a.tiles_unit + step * UQ_STAGE_BLOCKS) * UQ_BLOCK_REC, UQ_STAGE_BLOCKS * UQ_BLOCK_REC, bar);
     };
     const int early = min(UQ_STAGES, n_steps);
     pdl_launch_dependents();
@@ -223,7 +224,8 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch_q80(const __grid_c
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
             const int rt = tile / a.um_tok_tiles, tt = tile - rt * a.um_tok_tiles;
             const UmTile t = um_tile(a, rt);
-            if (tt * UM_NT + 16 * th >= a.T) {                   // no tokens in this half: only the hand-overs
+            const int tok0 = (tt >> a.um_halves) * UM_NT + 16 * th;
+            if (tok0 >= a.T || (a.um_halves && (tt & 1) != th)) { // this half has no tokens, or another block has them: only the hand-overs
 #pragma unroll 1
                 for (int step = 0; step < n_steps; step++) {
 #pragma unroll 1
@@ -289,7 +291,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma_batch_q80(const __grid_c
                 out[(2 * i + 1) * UM_OUT_STRIDE + lane] = finish_row<T_Q8_0>(c1);
             }
             __syncwarp();
-            if (q < t.n_units && !*failed) um_epilogue(a, out, t.row0 + 32 * q, tt * UM_NT + 16 * th, lane);
+            if (q < t.n_units && !*failed) um_epilogue(a, out, t.row0 + 32 * q, tok0, lane);
             __syncwarp();
         }
     }

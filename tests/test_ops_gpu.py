@@ -262,6 +262,20 @@ def test_mul_mat_batch_q8_0_edges(shape):
         assert np.array_equal(y[i], yr), f"token {i}: max abs diff {np.abs(y[i] - yr).max()}"
 
 
+@pytest.mark.parametrize("shape", [(9472, 512, 17), (9472, 512, 32), (9536, 512, 32), (9536, 512, 17), (6272, 256, 33), (6272, 256, 48), (6336, 256, 48), (128, 4096, 49), (640, 768, 250), (192, 256, 512)])
+def test_mul_mat_batch_q8_0_halves(shape):
+    """k_umma_batch_q80 with a block per half of a token tile: as many of them as SMs and one row tile more (whole tiles), two, three and four halves, a half with one token, an odd
+    number of units — the reference's bits at both ends of every half"""
+    n, k, T = shape
+    rng = np.random.default_rng(n + k + T)
+    w = G.random_blocks(rng, TYPES["Q8_0"], n, k).reshape(-1)
+    x = rng.standard_normal((T, k)).astype(np.float32)
+    y = engine.op_mul_mat(TYPES["Q8_0"], w, n, k, x)
+    for i in sorted({t for h in range(0, T, 16) for t in (h, min(h + 15, T - 1))}):
+        yr = port.mul_mat_vec(TYPES["Q8_0"], w, n, k, x[i])
+        assert np.array_equal(y[i], yr), f"token {i}: max abs diff {np.abs(y[i] - yr).max()}"
+
+
 @pytest.mark.parametrize("shape", [(32, 256), (96, 768), (4736, 512), (4768, 256), (9504, 768), (14240, 1280), (64, 14336), (160, 17408)])
 def test_mul_mat_vec_q8_0_edges(shape):
     """k_matvec_q80 where its teams and rings end: one stage, stages of eight and of 16 blocks, as many units of 32 rows as SMs and one more (a block's second team), more
