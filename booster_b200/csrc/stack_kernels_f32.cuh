@@ -1,7 +1,7 @@
 // stack_kernels_f32.cuh — float32 products on the tensor cores (sm_100a, tcgen05): Y = X W^T (+ bias), the operand layouts of k_gemm_simt_big.
 //
 // The method is that of Henry, Tang and Heinecke (Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations, 2019).
-// A float32 number is the sum of three bfloat16 ones, exactly: hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid (24 bits are 8 + 8 + 8; a number below 2^-110 loses what is below 2^-134).
+// A float32 number is the sum of three bfloat16 ones, exactly: hi = bf16(x), mid = bf16(x - hi), lo = x - hi - mid (24 bits are 8 + 8 + 8; a number below 2^-110 loses what is below 2^-133).
 // A product of two takes six MMAs (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi; what is left out is below 2^-26 of it). The tensor cores add in float32 without rounding to
 // nearest, so an accumulator holds 64 terms of a sum only: the small products first, hi hi last, then it is added to registers. Against 64 bits that is as close as a
 // chain of fmaf or closer (2-norm, random operands of nine shapes, k 64 to 8192: 0.8e-7 to 1.6e-7 here, 1.2e-7 to 5.7e-7 by fmaf; a whole float32 model's logits 4.5e-7 and 1.1e-6).
@@ -11,10 +11,10 @@
 // What bounds it: one block per SM whose slice is a chain (load, split and store, hand-over, MMAs, drain) that two stages overlap in part only: under ncu 50 % of the issue slots and
 // 23 to 31 % of the tensor pipe are busy (512 x 8192 x 1024 in 84 us). The MMAs alone, 65 clocks each, would allow 375 TFLOP/s of float32 products; 600 x 16000 x 1024 reach 126.
 // Measured (B200), the fp32 pipe's tiles and this: 600 x 16000 x 1024 694 and 156 us, 300 x 4096 x 1024 91 and 35, 64 x 512 x 512 40 and 16; scores of 512 tokens x 16 heads over
-// windows of 1152 rows of 576 260 and 92. A long sum in one block is where the odd rows' check shows: 64 x 64 x 4096 97 us without it, 103 with.
-// Rows and columns of a tile that three parts do not hold (an infinity or a NaN, whose parts would be NaN; nothing but numbers below 2^-100, whose last part would be gone) are
-// done again by fmaf, and they alone: what an output is does not depend on the rows beside it. In every other row the parts that are gone are below 2^-33 of its largest number.
-// The loop only gathers the bits that have no plane; a tile that has any looks for its odd rows then (largest magnitudes kept per row in the loop: 4 us a tile more).
+// windows of 1152 rows of 576 260 and 92.
+// Rows and columns of a tile with an infinity or a NaN (whose parts would be NaN) are done again by fmaf, and they alone: what an output is does not depend on the rows beside it.
+// The loop only notices that there is one; a tile that has one looks for its rows then (largest magnitudes kept per row in the loop: 4 us a tile more). What a number below
+// 2^-110 loses, less than 2^-133, is left: attention weights of far keys are such numbers, and beside their row's others it is nothing.
 #pragma once
 
 namespace b200 {
@@ -23,21 +23,21 @@ namespace stk {
 constexpr int F3_BM = 128, F3_BN = 128, F3_BK = 64, F3_WORKERS = 512, F3_THREADS = F3_WORKERS + 32;
 constexpr int F3_PLANE = 128 * F3_BK * 2, F3_STAGE = 6 * F3_PLANE, F3_SMEM = 2 * F3_STAGE + 1024;       // X hi, mid, lo | W hi, mid, lo; + alignment slack
 
-// two numbers into a word of each plane; lost takes the bits that have no plane (a number that is not finite as bfloat16 leaves the NaN of a subtraction, all ones)
-__device__ __forceinline__ void f3_split(float x, float y, uint32_t & hi, uint32_t & mid, uint32_t & lo, uint32_t & lost) {
+// two numbers into a word of each plane; odd turns NaN with a number that is not finite as bfloat16
+__device__ __forceinline__ void f3_split(float x, float y, uint32_t & hi, uint32_t & mid, uint32_t & lo, float & odd) {
     hi = pack_bf16(x, y);
     const float rx = x - __uint_as_float(hi << 16), ry = y - __uint_as_float(hi & 0xffff0000u);
     mid = pack_bf16(rx, ry);
     const float lx = rx - __uint_as_float(mid << 16), ly = ry - __uint_as_float(mid & 0xffff0000u);
     lo = __byte_perm(__float_as_uint(lx), __float_as_uint(ly), 0x7632u);
-    lost |= __float_as_uint(lx) | __float_as_uint(ly);
+    odd = fmaf(lx, 0.f, fmaf(ly, 0.f, odd));
 }
 
-// What a warp of a tile with odd numbers does for its 32 rows from mw and 32 columns from nb: rows and columns that three parts do not hold (a largest magnitude that is no
-// finite bfloat16 number, or below 2^-100 and not zero) are formed by fmaf, a lane per output, into again [row][33]. Returns their masks.
+// What a warp of a tile with odd numbers does for its 32 rows from mw and 32 columns from nb: rows and columns with a number that is not
+// finite as bfloat16 are formed by fmaf, a lane per output, into again [row][33]. Returns their masks.
 __device__ __noinline__ uint2 f3_again(const float * X, int ldx, const float * W, int ldw, bool w_kn, int T, int N, int kbeg, int K, int mw, int nb, float * again) {
     const int lane = threadIdx.x & 31;
-    const auto off = [](uint32_t top) { return top >= 0x7f7f8000u || (top > 0u && top < 0x0d800000u); };
+    const auto off = [](uint32_t top) { return top >= 0x7f7f8000u; };                  // (from there on rounding gives infinity)
     const auto bits = [](float v) { return __float_as_uint(v) & 0x7fffffffu; };        // magnitudes and NaN are ordered as their bits
     uint32_t x_off = 0, w_off = 0;
 #pragma unroll 1
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
         // ---- slices. Rows of X (and of W [N][K]): 16 threads a row, four rows a thread, 4 k each; a W [K][N]: a thread a column, 16 k
         float4 xr[4];
         float wr[16];
-        uint32_t lost = 0;
+        float odd = 0.f;
         const int lr = tid >> 4, lk = tid & 15, wn = tid & 127, wk = (tid >> 7) * 16;
         const auto fetch = [&](int k0) {
             const int k = k0 + 4 * lk;
@@ -175,8 +175,8 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
         };
         const auto store4 = [&](uint8_t * plane0, int row, float x, float y, float z, float w) {
             uint32_t h[2], m[2], l[2];
-            f3_split(x, y, h[0], m[0], l[0], lost);
-            f3_split(z, w, h[1], m[1], l[1], lost);
+            f3_split(x, y, h[0], m[0], l[0], odd);
+            f3_split(z, w, h[1], m[1], l[1], odd);
             uint8_t * p = plane0 + row * 128 + (((lk >> 1) ^ (row & 7)) << 4) + (lk & 1) * 8;
             *reinterpret_cast<uint2 *>(p) = make_uint2(h[0], h[1]);
             *reinterpret_cast<uint2 *>(p + F3_PLANE) = make_uint2(m[0], m[1]);
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
                 for (int g = 0; g < 2; g++) {
                     uint32_t h[4], m[4], l[4];
 #pragma unroll
-                    for (int i = 0; i < 4; i++) f3_split(wr[8 * g + 2 * i], wr[8 * g + 2 * i + 1], h[i], m[i], l[i], lost);
+                    for (int i = 0; i < 4; i++) f3_split(wr[8 * g + 2 * i], wr[8 * g + 2 * i + 1], h[i], m[i], l[i], odd);
                     uint8_t * p = st + 3 * F3_PLANE + wn * 128 + ((((wk >> 3) + g) ^ (wn & 7)) << 4);
                     *reinterpret_cast<uint4 *>(p) = make_uint4(h[0], h[1], h[2], h[3]);
                     *reinterpret_cast<uint4 *>(p + F3_PLANE) = make_uint4(m[0], m[1], m[2], m[3]);
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
             if (c > 0) drain(c - 1);
         }
         drain(nk - 1);
-        if (lost & 0xffffu) odd_s = 1;
+        if (odd != 0.f) odd_s = 1;                              // (NaN compares unequal)
         asm volatile("bar.sync 1, %0;" :: "n"(F3_WORKERS) : "memory");
         const int mw = m0 + 32 * (warp & 3), m = mw + lane, nb = n0 + (warp >> 2) * 32;
         if (odd_s) {                                            // through the slices' memory, which the MMAs are done with

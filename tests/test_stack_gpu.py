@@ -503,8 +503,9 @@ def test_float32_products_on_the_tensor_cores(T, N, K, glu):
 
 @pytest.mark.parametrize("T,N,K", [(65, 66, 68), (129, 257, 196), (300, 1030, 4096)])
 def test_float32_products_leave_rows_beside_odd_ones_alone(T, N, K):
-    """k_gemm_f32_umma, whole and in K parts: rows and columns that three bfloat16 parts do not hold (an infinity, a NaN, nothing but numbers around 2^-113) are what fmaf gives, and
-    every other output has the bits it has without them. Bound: (K + 8) 2^-24 sum |x w|, and half the smallest number for each sum in its range."""
+    """k_gemm_f32_umma, whole and in K parts: rows and columns with an infinity or a NaN are what fmaf gives, rows of nothing but numbers around 2^-113 lose what three bfloat16 parts
+    cannot hold of them, and every other output has the bits it has without them. Bound: (K + 8) 2^-24 sum |x w|; a part below 2^-133 is gone from each x (times |w|) and each w
+    (times |x|), and each of six products and sums can end below the smallest float32 number, 2^-149."""
     rng = np.random.default_rng(T + N + K)
     x, w = rng.standard_normal((T, K)).astype(np.float32), (rng.standard_normal((N, K)) / np.sqrt(K)).astype(np.float32)
     f32p = C.POINTER(C.c_float)
@@ -527,7 +528,7 @@ def test_float32_products_leave_rows_beside_odd_ones_alone(T, N, K):
     tiny[[3, 40]], tiny[:, 7] = False, False
     tiny[np.ix_(rows, cols)] = False
     xe, we = np.nan_to_num(x.astype(np.float64), posinf=0.0), np.nan_to_num(w.astype(np.float64))
-    off = (K + 8) * (2.0 ** -24 * (np.abs(xe) @ np.abs(we).T) + 2.0 ** -149)
+    off = (K + 8) * (2.0 ** -24 * (np.abs(xe) @ np.abs(we).T) + 6 * 2.0 ** -149) + 2.0 ** -133 * (np.abs(we).sum(1)[None, :] + np.abs(xe).sum(1)[:, None])
     assert (np.abs(z - xe @ we.T) <= off)[tiny].all()
 
 
