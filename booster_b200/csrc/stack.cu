@@ -1283,9 +1283,11 @@ constexpr int GX_MIN_K = 1024;
 struct UmmaScratch { __nv_bfloat16 * xb = nullptr; size_t elems = 0; int * err = nullptr; float * part = nullptr; size_t part_floats = 0; int sm_count = 148; };
 size_t umma_part_floats(int sm_count) { return (size_t) sm_count * UM_BM * UM_BN; }      // one K part of an output tile per SM
 
-// float32 tiles on the tensor cores (k_gemm_f32_umma) instead of the fp32 pipe: 64 tokens x 512 x 64 take 8.5 us here and 8.6 there, everything above is faster (600 x 16000 x 1024:
-// 694 and 156 us, 300 x 1024 x 4096 88 and 31). With less than half a tile's rows, columns or slice, the fp32 pipe's 64 x 64 tiles waste less.
-bool f32_umma_takes(bool vec, int T, int N, int K) { return vec && umma_enabled() && T >= 64 && N >= 64 && K >= 64; }
+// float32 tiles on the tensor cores (k_gemm_f32_umma) instead of the fp32 pipe: 600 x 16000 x 1024 take 694 us there and 156 here, 300 x 1024 x 4096 88 and 31. With less than half a
+// tile's rows, columns or slice, the fp32 pipe's 64 x 64 tiles waste less. One slice (k below 128) takes 11 us here, 9 in 64 x 64 tiles and 13 in 128 x 128 ones, which
+// products of 128 rows and columns would go to (64 to 512 rows, 64 to 2048 columns, k = 64 to 2048, batches of 1 to 128, W in both layouts: of 6858 products with two slices and
+// more 5 are slower here, by 2 to 11 %; of those with one, 263 of 1152, by up to 40 %, all of them with fewer rows or columns).
+bool f32_umma_takes(bool vec, int T, int N, int K) { return vec && umma_enabled() && T >= 64 && N >= 64 && (K >= 2 * F3_BK || (K >= F3_BK && T >= F3_BM && N >= F3_BN)); }
 // K parts of such a product (1: whole): as many as there are SMs for its tiles, one block each, of 256 k and more. Of 98 products of 64 to 600 tokens, 64 to 16000 rows and k = 512 to
 // 8192 none is slower so than whole, and whole they take up to five times as long (64 x 512 x 512 22.8 us whole, 20.6 in two parts; 300 x 1024 x 4096 110 and 35; where
 // the tiles fill the SMs there is one part: 64 x 16000 x 1024 39).

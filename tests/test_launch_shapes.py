@@ -135,7 +135,7 @@ BF16, F32 = 0, 1
     (BF16, 1, 512, 2048, 0, 1), (BF16, 4, 16000, 2048, 0, 0), (BF16, 1, 2048, 2044, 0, 0),
     (F32, 300, 1024, 4096, 0, 4), (F32, 600, 1024, 512, 0, 4), (F32, 64, 4096, 2048, 0, 4),
     (F32, 64, 512, 512, 0, 4), (F32, 64, 512, 496, 0, 7), (F32, 64, 9472, 1024, 0, 4), (F32, 64, 9600, 1024, 0, 7), (F32, 64, 16000, 2048, 0, 7), (F32, 600, 4096, 4096, 0, 7),      # two blocks' worth of k, two SMs a tile
-    (F32, 64, 512, 256, 0, 7), (F32, 300, 1024, 4096, 1, 7), (F32, 64, 64, 64, 0, 7), (F32, 64, 64, 4096, 0, 7), (F32, 64, 128, 4096, 0, 4),
+    (F32, 64, 512, 256, 0, 7), (F32, 300, 1024, 4096, 1, 7), (F32, 64, 64, 128, 0, 7), (F32, 64, 64, 124, 0, 6), (F32, 127, 512, 64, 0, 6), (F32, 128, 128, 64, 0, 7), (F32, 128, 127, 64, 0, 6), (F32, 64, 64, 4096, 0, 7), (F32, 64, 128, 4096, 0, 4),
     (F32, 63, 512, 512, 0, 6), (F32, 64, 63, 512, 0, 6), (F32, 64, 512, 60, 0, 6), (F32, 64, 512, 510, 0, 6),
     (BF16, 64, 128, 64, 0, 3), (BF16, 63, 128, 64, 0, 5), (BF16, 64, 128, 60, 0, 6)])
 def test_stack_product_kernel(dtype, T, N, K, glu, want):
