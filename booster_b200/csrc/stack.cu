@@ -236,6 +236,7 @@ struct StackCtx {
     int n_ctx = 0, n_past = 0, cap = 0;
     int32_t last_token = -1;              // the sequence's newest token (-1: none yet)
     cudaStream_t st = nullptr;
+    bool cold = true;                     // Lane::cold of the stream that launches go to
     cudaStream_t st2 = nullptr;           // BLOCK_SHARED, few-token steps: the feed-forward beside the mixer
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     float * F = nullptr, * SZ = nullptr;  // BLOCK_SHARED: units of a dense feed-forward [cap][max_dense]; the token input's gate [cap][side_dim]
@@ -291,6 +292,27 @@ struct StackCtx {
 };
 
 namespace {
+
+// where a pass's launches go. cold: the next one waits for all before it as a whole (it may have to wait for another stream as well); nullptr: every one does (a product by itself)
+struct Lane { cudaStream_t st = nullptr; bool * cold = nullptr; };
+// a launch that may become resident while the kernel before it runs (stack_kernels.cuh: pdl_wait)
+template <typename... P, typename... A>
+void pdl(const Lane & l, dim3 grid, dim3 block, size_t smem, void (*kern)(P...), A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = l.st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = l.cold && !*l.cold ? 1 : 0;
+    if (l.cold) *l.cold = false;
+    SCU(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+}
+template <typename... P, typename... A>
+void pdl(StackCtx * c, dim3 grid, dim3 block, size_t smem, void (*kern)(P...), A... args) { pdl(Lane{c->st, &c->cold}, grid, block, smem, kern, args...); }
+
+// in front of a walk over a portion's tokens: its few blocks are chains of instructions, and let in while the kernel before still fills most SMs they crowd on the first that are
+// free (512 tokens of the delta rule, 128 blocks: 128 us one to an SM, 340 so). They wait for that kernel to end; a token's step is too short for that.
+void spread(StackCtx * c, int T) { if (T > 8) c->cold = true; }
 
 // A kernel's limit of dynamic shared memory is set per device and only ever grows; models on several devices, and contexts on several threads, come here with the same kernels.
 // have: what it was raised to on each device so far.
@@ -1322,16 +1344,16 @@ bool gx_pays(bool f32, int chunks, int N, int batch, bool glu, int sm_count) {
     const long long here = waves(GX_ROWS, resident[f32][c]), there = waves(16, 4);
     return 2 * here <= 3 * there && 16 * chunks >= (here == 1 && ch > 1 ? 12 : 14) * full;
 }
-void launch_f32_umma(cudaStream_t st, const LinArgs & a, int * err, int batch, int parts = 1, float * part = nullptr) {
+void launch_f32_umma(const Lane & lane, const LinArgs & a, int * err, int batch, int parts = 1, float * part = nullptr) {
     static size_t have[64] = {0};
     raise_smem(k_gemm_f32_umma, F3_SMEM, have);
-    k_gemm_f32_umma<<<dim3((unsigned) ((a.N + F3_BN - 1) / F3_BN), (unsigned) ((a.T + F3_BM - 1) / F3_BM), (unsigned) (parts > 1 ? parts : batch)), F3_THREADS, F3_SMEM, st>>>(a, err, parts, part);
+    pdl(lane, dim3((unsigned) ((a.N + F3_BN - 1) / F3_BN), (unsigned) ((a.T + F3_BM - 1) / F3_BM), (unsigned) (parts > 1 ? parts : batch)), F3_THREADS, F3_SMEM, k_gemm_f32_umma, a, err, parts, part);
 }
-void split_sum(cudaStream_t st, const float * part, int parts, int T, int N, const float * bias, float * Y, int ldy) {
+void split_sum(const Lane & lane, const float * part, int parts, int T, int N, const float * bias, float * Y, int ldy) {
     const bool wide = N % 4 == 0 && ldy % 4 == 0 && ((uintptr_t) Y & 15) == 0;
     const dim3 grid((unsigned) ((N / (wide ? 4 : 1) + 255) / 256), (unsigned) T);
-    if (wide) k_split_sum<4><<<grid, 256, 0, st>>>(part, parts, T, N, bias, Y, ldy);
-    else k_split_sum<1><<<grid, 256, 0, st>>>(part, parts, T, N, bias, Y, ldy);
+    if (wide) pdl(lane, grid, 256, 0, k_split_sum<4>, part, parts, T, N, bias, Y, ldy);
+    else pdl(lane, grid, 256, 0, k_split_sum<1>, part, parts, T, N, bias, Y, ldy);
 }
 // the kernel a product goes to: mat-vecs of few tokens, then tile kernels
 enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG, LIN_ROWS_X, LIN_UMMA, LIN_F32_PARTS, LIN_MMA, LIN_SIMT, LIN_F32_UMMA };
@@ -1345,6 +1367,35 @@ LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu
         return parts > 1 && (size_t) parts * T * N <= part_floats ? LIN_F32_PARTS : LIN_F32_UMMA;
     }
     return dtype == STACK_BF16 && vec && mma_enabled() ? LIN_MMA : LIN_SIMT;
+}
+
+// One token's product in a pass goes to k_gemv_ring where a row's 16-byte pieces fit a block's registers: four (bf16) or eight (float32) a lane. Longer rows, and products of rows that
+// are no multiple of 16 bytes, go where they go by themselves: lin_route's lines are those of cold products, whose first bytes nobody has asked for.
+bool ring_takes(int K) { return K <= 8192; }
+template <typename WT, int TEAM, int CH>
+void launch_ring_as(const Lane & lane, const LinArgs & a, int batch, int sm_count) {
+    constexpr int RS = gr_rows(CH) * (GR_THREADS / 32 / TEAM);
+    // a block per SM (of the batch), in rounds where it would have more than 256 rows; an even number of rows, since a gated unit's come in pairs
+    const long long all = (long long) a.N * batch, rounds = (all + 256LL * sm_count - 1) / (256LL * sm_count);
+    const int gx = (int) std::max<long long>(1, rounds * sm_count / batch), rpb = std::min(256, ((a.N + gx - 1) / gx + 1) / 2 * 2);
+    const size_t smem = (size_t) GR_PIECES * GR_THREADS * 16 + (size_t) ((rpb + RS - 1) / RS * RS) * TEAM * 4;
+    static size_t have[64] = {0};
+    raise_smem(k_gemv_ring<WT, TEAM, CH>, (size_t) GR_PIECES * GR_THREADS * 16 + 288 * 8 * 4, have);
+    pdl(lane, dim3((unsigned) ((a.N + rpb - 1) / rpb), 1, (unsigned) batch), GR_THREADS, smem, k_gemv_ring<WT, TEAM, CH>, a, rpb);
+}
+void launch_ring(const Lane & lane, const LinArgs & a, int dtype, int batch, int sm_count) {
+    const auto go = [&](auto wt) {
+        using WT = decltype(wt);
+        const int chunks = (a.K + 16 / (int) sizeof(WT) - 1) / (16 / (int) sizeof(WT));
+        if (chunks <= 32) launch_ring_as<WT, 1, 1>(lane, a, batch, sm_count);
+        else if (chunks <= 64) launch_ring_as<WT, 2, 1>(lane, a, batch, sm_count);
+        else if (chunks <= 128) launch_ring_as<WT, 4, 1>(lane, a, batch, sm_count);
+        else if (chunks <= 256) launch_ring_as<WT, 8, 1>(lane, a, batch, sm_count);
+        else if (chunks <= 512) launch_ring_as<WT, 8, 2>(lane, a, batch, sm_count);
+        else if (chunks <= 1024) launch_ring_as<WT, 8, 4>(lane, a, batch, sm_count);
+        else if constexpr (sizeof(WT) == 4) launch_ring_as<WT, 8, 8>(lane, a, batch, sm_count);
+    };
+    if (dtype == STACK_F32) go(0.f); else go(__nv_bfloat16());
 }
 
 // tensor map of a bf16 matrix batch [nz][rows][K] (strides in elements): boxes of 64 columns, one 128-byte swizzled row each, by box_rows
@@ -1378,7 +1429,7 @@ struct LinOpt {
     int x_share = 1;
     const float * x_scale = nullptr;        // mat-vec: entry z runs on x_scale[z] times its input row
 };
-void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, int ldx, const void * W, const float * bias, float * Y, int ldy,
+void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X, int ldx, const void * W, const float * bias, float * Y, int ldy,
                int T, int N, int K, int batch = 1, long long sX = 0, long long sW = 0, long long sY = 0, bool glu = false, float glu_limit = 0.f,
                const UmmaScratch * us = nullptr, const LinOpt * opt = nullptr) {
     if (T <= 0 || N <= 0) return;
@@ -1390,55 +1441,56 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
     a.vec = K % vecw == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % vecw == 0 && al16(X) && al16(W);
     if (launches) (*launches)++;
     const LinRoute route = lin_route(dtype, T, N, K, batch, a.vec != 0, a.glu != 0, a.seg != nullptr, us && us->err, (size_t) xbatch * T * K, us && us->xb ? us->elems : 0, us && us->part ? us->part_floats : 0, us ? us->sm_count : 148);
-    if (route == LIN_ROWS_X) {
+    if (T == 1 && a.vec && lane.cold && ring_takes(K)) launch_ring(lane, a, dtype, batch, us ? us->sm_count : 148);
+    else if (route == LIN_ROWS_X) {
         const int ch = gx_chunks(K / vecw);
         const dim3 grid((unsigned) ((N + GX_ROWS - 1) / GX_ROWS), 1, (unsigned) batch);
         const auto go = [&](auto wt) {
             using WT = decltype(wt);
-            if (ch == 1) k_gemv_x<WT, 1><<<grid, GX_WARPS * 32, 0, st>>>(a);
-            else if (ch == 2) k_gemv_x<WT, 2><<<grid, GX_WARPS * 32, 0, st>>>(a);
-            else k_gemv_x<WT, 4><<<grid, GX_WARPS * 32, 0, st>>>(a);
+            if (ch == 1) pdl(lane, grid, GX_WARPS * 32, 0, k_gemv_x<WT, 1>, a);
+            else if (ch == 2) pdl(lane, grid, GX_WARPS * 32, 0, k_gemv_x<WT, 2>, a);
+            else pdl(lane, grid, GX_WARPS * 32, 0, k_gemv_x<WT, 4>, a);
         };
         if (dtype == STACK_F32) go(0.f); else go(__nv_bfloat16());
     } else if (route == LIN_ROWS_LONG) {
-        if (dtype == STACK_F32) k_gemv<float, 1, 8><<<(unsigned) N, 256, 0, st>>>(a); else k_gemv<__nv_bfloat16, 1, 8><<<(unsigned) N, 256, 0, st>>>(a);
+        if (dtype == STACK_F32) pdl(lane, (unsigned) N, 256, 0, k_gemv<float, 1, 8>, a); else pdl(lane, (unsigned) N, 256, 0, k_gemv<__nv_bfloat16, 1, 8>, a);
     } else if (route == LIN_ROWS) {
         if (a.glu) {
             const dim3 grid((unsigned) ((N / 2 + 7) / 8), 1, (unsigned) batch);
-            if (dtype == STACK_F32) k_gemv<float, 2><<<grid, 256, 0, st>>>(a); else k_gemv<__nv_bfloat16, 2><<<grid, 256, 0, st>>>(a);
+            if (dtype == STACK_F32) pdl(lane, grid, 256, 0, k_gemv<float, 2>, a); else pdl(lane, grid, 256, 0, k_gemv<__nv_bfloat16, 2>, a);
         } else {
             const dim3 grid((unsigned) ((N + 7) / 8), 1, (unsigned) batch);
-            if (dtype == STACK_F32) k_gemv<float, 1><<<grid, 256, 0, st>>>(a); else k_gemv<__nv_bfloat16, 1><<<grid, 256, 0, st>>>(a);
+            if (dtype == STACK_F32) pdl(lane, grid, 256, 0, k_gemv<float, 1>, a); else pdl(lane, grid, 256, 0, k_gemv<__nv_bfloat16, 1>, a);
         }
     } else if (route == LIN_UMMA) {
         // tensor memory path: activations to bfloat16 once, then tcgen05.mma over TMA-fed stages (a.vec: rows and batch strides are multiples of 16 bytes)
         static size_t have[64] = {0};
         raise_smem(k_gemm_bf16_umma, UM_SMEM, have);
-        k_to_bf16<<<dim3((unsigned) std::min<long long>(((long long) T * (K / 8) + 255) / 256, 2048), (unsigned) xbatch), 256, 0, st>>>(X, ldx, T, K, sX, us->xb, (long long) T * K);
+        pdl(lane, dim3((unsigned) std::min<long long>(((long long) T * (K / 8) + 255) / 256, 2048), (unsigned) xbatch), 256, 0, k_to_bf16, X, ldx, T, K, sX, us->xb, (long long) T * K);
         const dim3 grid((unsigned) ((N + UM_BN - 1) / UM_BN), (unsigned) ((T + UM_BM - 1) / UM_BM), (unsigned) batch);
         const CUtensorMap mx = map_bf16(us->xb, K, T, xbatch, K, (long long) T * K, UM_BM), mw = map_bf16(W, K, N, batch, K, sW, UM_BN);
         const int tiles = (int) (grid.x * grid.y), nk = (K + UM_BK - 1) / UM_BK;
         const int ksplit = batch == 1 && !a.glu && !a.seg && us->part && split_k_enabled() ? std::min(us->sm_count / tiles, nk / 4) : 1;
         if (ksplit > 1) {
-            k_gemm_bf16_umma<<<dim3(grid.x, grid.y, (unsigned) ksplit), 256, UM_SMEM, st>>>(mx, mw, a, us->err, ksplit, us->part);
-            split_sum(st, us->part, ksplit, T, N, bias, Y, ldy);
+            pdl(lane, dim3(grid.x, grid.y, (unsigned) ksplit), 256, UM_SMEM, k_gemm_bf16_umma, mx, mw, a, us->err, ksplit, us->part);
+            split_sum(lane, us->part, ksplit, T, N, bias, Y, ldy);
             if (launches) (*launches)++;
         }
-        else k_gemm_bf16_umma<<<grid, 256, UM_SMEM, st>>>(mx, mw, a, us->err);
+        else pdl(lane, grid, 256, UM_SMEM, k_gemm_bf16_umma, mx, mw, a, us->err, 1, nullptr);
         if (launches) (*launches)++;
     } else if (route == LIN_F32_PARTS) {
         const int parts = f32_k_parts(T, N, K, us->sm_count);
-        launch_f32_umma(st, a, us->err, 1, parts, us->part);
-        split_sum(st, us->part, parts, T, N, bias, Y, ldy);
+        launch_f32_umma(lane, a, us->err, 1, parts, us->part);
+        split_sum(lane, us->part, parts, T, N, bias, Y, ldy);
         if (launches) (*launches)++;
     } else if (route == LIN_F32_UMMA) {
-        launch_f32_umma(st, a, us->err, batch);
+        launch_f32_umma(lane, a, us->err, batch);
     } else if (route == LIN_MMA) {
         const dim3 grid((unsigned) ((N + MM_BN - 1) / MM_BN), (unsigned) ((T + MM_BM - 1) / MM_BM), (unsigned) batch);
-        k_gemm_bf16_mma<<<grid, 256, 0, st>>>(a);
+        pdl(lane, grid, 256, 0, k_gemm_bf16_mma, a);
     } else {
         const dim3 grid((unsigned) ((N + 63) / 64), (unsigned) ((T + 63) / 64), (unsigned) batch);
-        if (dtype == STACK_F32) k_gemm_simt<float><<<grid, 256, 0, st>>>(a); else k_gemm_simt<__nv_bfloat16><<<grid, 256, 0, st>>>(a);
+        if (dtype == STACK_F32) pdl(lane, grid, 256, 0, k_gemm_simt<float>, a); else pdl(lane, grid, 256, 0, k_gemm_simt<__nv_bfloat16>, a);
     }
     SCU(cudaGetLastError());
 }
@@ -1446,19 +1498,19 @@ void linear_on(cudaStream_t st, int dtype, int64_t * launches, const float * X, 
 void linear(StackCtx * c, const float * X, int ldx, const DMat & W, float * Y, int ldy, int T, int batch = 1, long long sX = 0, long long sY = 0, bool glu = false, float glu_limit = 0.f,
             const LinOpt * opt = nullptr) {
     const UmmaScratch us{c->xb, c->xb_elems, c->d_err, c->xpart, c->xpart_floats, c->sm_count};
-    linear_on(c->st, c->m->dtype, &c->launches, X, ldx, W.w, W.bias, Y, ldy, T, W.N, W.K, batch, sX, (long long) W.N * W.K, sY, glu, glu_limit, &us, opt);
+    linear_on(Lane{c->st, &c->cold}, c->m->dtype, &c->launches, X, ldx, W.w, W.bias, Y, ldy, T, W.N, W.K, batch, sX, (long long) W.N * W.K, sY, glu, glu_limit, &us, opt);
 }
 
 // end of a sub-layer: X += norm(Y) * w_post; Hn = norm(X) * w_next when another sub-layer follows
 void post_norm_add(StackCtx * c, const float * w_post, const float * w_next, int T) {
     const StackModel & m = *c->m;
-    k_post_norm_add<<<T, std::min(256, 32 * m.groups), 0, c->st>>>(c->Y, w_post, c->X, w_next, c->Hn, m.E, m.groups, m.eps);
+    pdl(c, T, std::min(256, 32 * m.groups), 0, k_post_norm_add, c->Y, w_post, c->X, w_next, c->Hn, m.E, m.groups, m.eps);
     c->launches++;
 }
 
 void norm(StackCtx * c, const float * X, int ldx, const int32_t * rows, const float * w, int n, int groups, float * Y, int ldy, int T, bool accumulate) {
     const int threads = std::min(256, 32 * groups);
-    k_group_norm<<<T, threads, 0, c->st>>>(X, ldx, rows, w, n, groups, c->m->eps, Y, ldy, accumulate ? 1 : 0);
+    pdl(c, T, threads, 0, k_group_norm, X, ldx, rows, w, n, groups, c->m->eps, Y, ldy, accumulate ? 1 : 0);
     c->launches++;
     SCU(cudaGetLastError());
 }
@@ -1466,15 +1518,17 @@ void norm(StackCtx * c, const float * X, int ldx, const int32_t * rows, const fl
 template <int DMAX>
 void launch_delta_scan(StackCtx * c, const LayerSpec & L, int T, int C, float * S) {
     const dim3 grid((unsigned) L.H, (unsigned) ((L.V + DSCAN_COLS - 1) / DSCAN_COLS));
-    k_delta_scan<DMAX><<<grid, 128, 0, c->st>>>(c->CV, C, c->BG, T, L.H, L.KH, L.D, L.V, S, c->O);
+    spread(c, T);
+    pdl(c, grid, 128, 0, k_delta_scan<DMAX>, c->CV, C, c->BG, T, L.H, L.KH, L.D, L.V, S, c->O);
 }
 
 // mixers: c->in [T][E] -> c->out [T][E]; R names the run's state
 void mixer_mingru(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     linear(c, c->in, c->m->E, L.zxg, c->P, 3 * L.width, T);
     // (a few tokens have no tile to share)
-    if (T > 8) k_mingru_tiles<<<(L.width + 31) / 32, MG_WARPS * 32, 0, c->st>>>(c->P, T, L.width, c->rec + R.off_rec, c->A);
-    else k_mingru_scan<<<(L.width + 127) / 128, 128, 0, c->st>>>(c->P, T, L.width, c->rec + R.off_rec, c->A);
+    spread(c, T);
+    if (T > 8) pdl(c, (L.width + 31) / 32, MG_WARPS * 32, 0, k_mingru_tiles, c->P, T, L.width, c->rec + R.off_rec, c->A);
+    else pdl(c, (L.width + 127) / 128, 128, 0, k_mingru_scan, c->P, T, L.width, c->rec + R.off_rec, c->A);
     c->launches++;
     linear(c, c->A, L.width, L.o, c->out, c->m->E, T);
 }
@@ -1529,10 +1583,10 @@ void gemm_f32(StackCtx * c, const float * X, int ldx, long long sX, const float 
     LinArgs a{X, W, nullptr, Y, M, N, K, ldx, ldy, sX, sW, sY, 0, 0, 0.f, 0.f, w_kn, ldw, nz2, sX2, sW2, sY2};
     a.vec = K % 4 == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % 4 == 0 && sX2 % 4 == 0 && sW2 % 4 == 0 && ldw % 4 == 0 && al16(X) && al16(W);
     a.accum = accum; a.see_rows = see.rows; a.see_pos = see.pos; a.see_step = see.step; a.rows_all = rows_all;
-    if (f32_umma_takes(a.vec != 0, M, N, K)) launch_f32_umma(c->st, a, c->d_err, batch * nz2);
+    if (f32_umma_takes(a.vec != 0, M, N, K)) launch_f32_umma(Lane{c->st, &c->cold}, a, c->d_err, batch * nz2);
     else if (a.vec && M >= SG_BM && N >= SG_BN && simt_big_enabled())       // operands that fill 128 x 128 tiles
-        k_gemm_simt_big<<<dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((M + SG_BM - 1) / SG_BM), (unsigned) (batch * nz2)), 256, 0, c->st>>>(a);
-    else k_gemm_simt<float><<<dim3((unsigned) ((N + 63) / 64), (unsigned) ((M + 63) / 64), (unsigned) (batch * nz2)), 256, 0, c->st>>>(a);
+        pdl(c, dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((M + SG_BM - 1) / SG_BM), (unsigned) (batch * nz2)), 256, 0, k_gemm_simt_big, a);
+    else pdl(c, dim3((unsigned) ((N + 63) / 64), (unsigned) ((M + 63) / 64), (unsigned) (batch * nz2)), 256, 0, k_gemm_simt<float>, a);
     c->launches++;
 }
 constexpr int ATT_TQ = 16;                 // tokens per tile of the prompt attention
@@ -1542,7 +1596,7 @@ constexpr size_t ATT_SCORE_BYTES = (size_t) 256 << 20;
 void latent_values_out(StackCtx * c, const LayerSpec & L, int T, int ldp, int gate_off) {
     const int H = L.H, V = L.V, rank = L.rank;
     linear(c, c->OL, H * rank, L.uv, c->A, H * V, T, H, rank, V);
-    if (L.head_gate) { k_head_gate<<<dim3((unsigned) T, T <= 16 ? (unsigned) ((H * V + 255) / 256) : 1u), 256, 0, c->st>>>(c->A, c->P + gate_off, ldp, H, V, L.gate_rows == H ? 0 : 1); c->launches++; }
+    if (L.head_gate) { pdl(c, dim3((unsigned) T, T <= 16 ? (unsigned) ((H * V + 255) / 256) : 1u), 256, 0, k_head_gate, c->A, c->P + gate_off, ldp, H, V, L.gate_rows == H ? 0 : 1); c->launches++; }
     linear(c, c->A, H * V, L.o, c->out, c->m->E, T);
 }
 
@@ -1556,12 +1610,12 @@ void mixer_latent(StackCtx * c, const LayerSpec & L, const RunSpec & Rn, int T) 
     if (L.q_rank > 0) {
         // P[t] = [ query latent | down-projection | head gates ]: norm of the query latent in place, q = W_uq c_q into A, cache row, absorbed queries from A
         gate_off = L.q_rank + rank;
-        k_latent_prep<<<dim3((unsigned) T, T <= 16 ? (unsigned) ((H + 4) / 4) : 1u), 128, 0, c->st>>>(c->P, ldp, H, D, 0, rank, L.cnorm, c->m->eps, rope, &c->d_step->st, cache, c->QK, L.q_rank, L.qnorm, L.q_rank);
+        pdl(c, dim3((unsigned) T, T <= 16 ? (unsigned) ((H + 4) / 4) : 1u), 128, 0, k_latent_prep, c->P, ldp, H, D, 0, rank, L.cnorm, c->m->eps, rope, &c->d_step->st, cache, c->QK, L.q_rank, L.qnorm, L.q_rank);
         linear(c, c->P, ldp, L.uq, c->A, H * D, T);
         linear(c, c->A, H * D, L.ukT, c->QK, H * W, T, H, D, W);
     } else {
         gate_off = H * (D + R) + W;
-        k_latent_prep<<<dim3((unsigned) T, T <= 16 ? (unsigned) ((H + 4) / 4) : 1u), 128, 0, c->st>>>(c->P, ldp, H, D, R, rank, L.cnorm, c->m->eps, rope, &c->d_step->st, cache, c->QK, H * (D + R), nullptr, 0);
+        pdl(c, dim3((unsigned) T, T <= 16 ? (unsigned) ((H + 4) / 4) : 1u), 128, 0, k_latent_prep, c->P, ldp, H, D, R, rank, L.cnorm, c->m->eps, rope, &c->d_step->st, cache, c->QK, H * (D + R), nullptr, 0);
         // absorbed queries, one product per head: QK[t][h][0..rank) = W_uk,h^T q[t][h][0..D)
         linear(c, c->P, ldp, L.ukT, c->QK, H * W, T, H, D + R, W);
     }
@@ -1580,7 +1634,7 @@ void mixer_latent(StackCtx * c, const LayerSpec & L, const RunSpec & Rn, int T) 
             const long long sK = L.window > 0 ? (long long) TQ * W : 0;
             const int rows = (std::min(T, (g0 + ng) * TQ) - g0 * TQ) * H;          // (rows past the last token hold what an earlier pass left)
             gemm_f32(c, c->QK + (size_t) g0 * M * W, W, (long long) M * W, keys, 0, 0, sK, c->att_scores, nk, (long long) M * nk, M, nk, W, ng, 1, 0, 0, 0, 0, See(), rows);
-            k_latent_softmax_rows<<<(rows + 7) / 8, 256, 0, c->st>>>(c->att_scores, rows, H, TQ, nk, L.window, span, L.sink, &c->d_step->st, L.scale, g0);
+            pdl(c, (rows + 7) / 8, 256, 0, k_latent_softmax_rows, c->att_scores, rows, H, TQ, nk, L.window, span, L.sink, &c->d_step->st, L.scale, g0);
             gemm_f32(c, c->att_scores, nk, (long long) M * nk, keys, 1, W, sK, c->OL + (size_t) g0 * M * rank, rank, (long long) M * rank, M, rank, nk, ng, 1, 0, 0, 0, 0, See(), rows);
             c->launches++;
         }
@@ -1591,10 +1645,10 @@ void mixer_latent(StackCtx * c, const LayerSpec & L, const RunSpec & Rn, int T) 
     const AttnPlan ap = plan_attention(L, c->n_ctx, T, c->sm_count);
     const LatAttnArgs aa{c->QK, cache, L.sink, &c->d_step->st, c->OL, c->att_part, c->att_ml, T, H, rank, R, L.window, L.scale, ap.TQ, ap.HQ, ap.nsplit, ap.smax};
     const dim3 grid((unsigned) ((T + ap.TQ - 1) / ap.TQ), (unsigned) ((H + ap.HQ - 1) / ap.HQ), (unsigned) ap.nsplit);
-    if (!ap.staged) k_latent_attn<<<grid, 256, ap.smem, c->st>>>(aa);
-    else if (W % 4 == 0) k_latent_attn_staged<true><<<grid, 256, ap.smem, c->st>>>(aa);
-    else k_latent_attn_staged<false><<<grid, 256, ap.smem, c->st>>>(aa);
-    if (ap.nsplit > 1) { k_latent_combine<<<dim3((unsigned) T, (unsigned) H, (unsigned) ((rank + 63) / 64)), 256, 0, c->st>>>(aa); c->launches++; }
+    if (!ap.staged) pdl(c, grid, 256, ap.smem, k_latent_attn, aa);
+    else if (W % 4 == 0) pdl(c, grid, 256, ap.smem, k_latent_attn_staged<true>, aa);
+    else pdl(c, grid, 256, ap.smem, k_latent_attn_staged<false>, aa);
+    if (ap.nsplit > 1) { pdl(c, dim3((unsigned) T, (unsigned) H, (unsigned) ((rank + 63) / 64)), 256, 0, k_latent_combine, aa); c->launches++; }
     c->launches += 2;
     latent_values_out(c, L, T, ldp, gate_off);
 }
@@ -1602,9 +1656,9 @@ void mixer_latent(StackCtx * c, const LayerSpec & L, const RunSpec & Rn, int T) 
 // causal convolution of a portion's rows with the history a sequence keeps (k_causal_conv), then the history moves on
 void causal_conv(StackCtx * c, ConvArgs a, int batch = 1) {
     a.fuse_hist = a.T == 1 ? 1 : 0;
-    k_causal_conv<<<dim3((unsigned) ((a.C + 127) / 128), (unsigned) a.T, (unsigned) batch), 128, 0, c->st>>>(a);
+    pdl(c, dim3((unsigned) ((a.C + 127) / 128), (unsigned) a.T, (unsigned) batch), 128, 0, k_causal_conv, a);
     c->launches++;
-    if (a.taps > 1 && !a.fuse_hist) { k_causal_conv_hist<<<dim3((unsigned) ((a.C + 127) / 128), 1, (unsigned) batch), 128, 0, c->st>>>(a); c->launches++; }
+    if (a.taps > 1 && !a.fuse_hist) { pdl(c, dim3((unsigned) ((a.C + 127) / 128), 1, (unsigned) batch), 128, 0, k_causal_conv_hist, a); c->launches++; }
 }
 
 void mixer_delta(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
@@ -1612,12 +1666,12 @@ void mixer_delta(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     float * S = c->rec + R.off_rec, * hist = S + (size_t) H * D * V;
     linear(c, c->in, E, L.proj, c->P, ldp, T);
     causal_conv(c, ConvArgs{c->P, ldp, 0, L.wconv, 0, hist, 0, c->CV, C, 0, T, C, L.taps, 1, 0, nullptr, nullptr, 0, 0, 0});
-    k_delta_gates<<<T, 128, 0, c->st>>>(c->CV, C, c->P, ldp, H, KH, D, V, L.A_log, L.dt_bias, c->BG);
+    pdl(c, T, 128, 0, k_delta_gates, c->CV, C, c->P, ldp, H, KH, D, V, L.A_log, L.dt_bias, c->BG);
     if (D <= 32) launch_delta_scan<32>(c, L, T, C, S);
     else if (D <= 64) launch_delta_scan<64>(c, L, T, C, S);
     else if (D <= 128) launch_delta_scan<128>(c, L, T, C, S);
     else launch_delta_scan<256>(c, L, T, C, S);
-    k_delta_out<<<dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, c->st>>>(c->O, c->P, ldp, C + 2 * H, H, V, L.dnorm, 0, 0, c->m->eps, c->A);
+    pdl(c, dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, k_delta_out, c->O, c->P, ldp, C + 2 * H, H, V, L.dnorm, 0, 0, c->m->eps, c->A);
     c->launches += 3;
     linear(c, c->A, H * V, L.o, c->out, E, T);
 }
@@ -1630,7 +1684,8 @@ void launch_gdelta_scan(StackCtx * c, const LayerSpec & L, int T, int ldp, float
     while (ncols > 16 && L.H * ((L.V + ncols - 1) / ncols) < c->sm_count) ncols = (ncols / 2 + 7) / 8 * 8;
     const int threads = GD_RG * ncols, HD = L.H * L.D;
     const dim3 grid((unsigned) L.H, (unsigned) ((L.V + ncols - 1) / ncols));
-    k_gdelta_scan<DMAX><<<grid, threads, 0, c->st>>>(c->P, ldp, 0, HD, 2 * HD, c->CV, T, L.H, L.D, L.V, S, c->O);
+    spread(c, T);
+    pdl(c, grid, threads, 0, k_gdelta_scan<DMAX>, c->P, ldp, 0, HD, 2 * HD, c->CV, T, L.H, L.D, L.V, S, c->O);
 }
 
 // generalized delta rule: P[t] = [ r | k | v | gate | removal logit | decay latent ]
@@ -1639,13 +1694,13 @@ void mixer_gdelta(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     float * S = c->rec + R.off_rec;
     linear(c, c->in, E, L.proj, c->P, ldp, T);
     const dim3 pgrid((unsigned) T, (unsigned) H);
-    if (c->m->dtype == STACK_F32) k_gdelta_prep<float><<<pgrid, 128, (size_t) (L.lora + D) * 4, c->st>>>(c->P, ldp, HD, 2 * HD + 2 * HV, lat_off, L.lora, (const float *) L.w2.w, L.w2.bias, H, D, c->CV);
-    else k_gdelta_prep<__nv_bfloat16><<<pgrid, 128, (size_t) (L.lora + D) * 4, c->st>>>(c->P, ldp, HD, 2 * HD + 2 * HV, lat_off, L.lora, (const __nv_bfloat16 *) L.w2.w, L.w2.bias, H, D, c->CV);
+    if (c->m->dtype == STACK_F32) pdl(c, pgrid, 128, (size_t) (L.lora + D) * 4, k_gdelta_prep<float>, c->P, ldp, HD, 2 * HD + 2 * HV, lat_off, L.lora, (const float *) L.w2.w, L.w2.bias, H, D, c->CV);
+    else pdl(c, pgrid, 128, (size_t) (L.lora + D) * 4, k_gdelta_prep<__nv_bfloat16>, c->P, ldp, HD, 2 * HD + 2 * HV, lat_off, L.lora, (const __nv_bfloat16 *) L.w2.w, L.w2.bias, H, D, c->CV);
     if (D <= 32) launch_gdelta_scan<32>(c, L, T, ldp, S);
     else if (D <= 64) launch_gdelta_scan<64>(c, L, T, ldp, S);
     else if (D <= 128) launch_gdelta_scan<128>(c, L, T, ldp, S);
     else launch_gdelta_scan<256>(c, L, T, ldp, S);
-    k_delta_out<<<dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, c->st>>>(c->O, c->P, ldp, 2 * HD + HV, H, V, L.dnorm, V, 1, c->m->eps, c->A);
+    pdl(c, dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, k_delta_out, c->O, c->P, ldp, 2 * HD + HV, H, V, L.dnorm, V, 1, c->m->eps, c->A);
     c->launches += 3;
     linear(c, c->A, HV, L.o, c->out, E, T);
 }
@@ -1669,7 +1724,7 @@ void mixer_diffattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T)
         // prompt portion: float32 products over tiles of ATT_TQ tokens, one batch entry per (tile, key/value head, map)
         const int TQ = ATT_TQ, Rh = H / G, M = TQ * Rh, ntile = (T + TQ - 1) / TQ, Tpad = ntile * TQ;
         const int pos0 = c->h_step->st.pos0;
-        k_diff_q_layout<<<Tpad, 256, 0, c->st>>>(Q, ldq, T, Tpad, H, G, D, c->QK);
+        pdl(c, Tpad, 256, 0, k_diff_q_layout, Q, ldq, T, Tpad, H, G, D, c->QK);
         const int span = L.window > 0 ? std::min(L.window, pos0 + Tpad) : 0;
         const int nk = ((L.window > 0 ? span + TQ - 1 : pos0 + Tpad) + 3) / 4 * 4;
         const int per_group = (int) std::max<size_t>(1, c->att_scores_floats / ((size_t) 2 * G * M * nk));
@@ -1682,12 +1737,12 @@ void mixer_diffattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T)
             gemm_f32(c, c->QK + (size_t) g0 * M * D, D, (long long) M * D, keys, 0, row, sK, c->att_scores, nk, (long long) M * nk, M, nk, D, ng,
                      2 * G, (long long) Tpad * Rh * D, D, grp);
             const int rows = ng * M * G;
-            k_diff_softmax_rows<<<(rows + 7) / 8, 256, 0, c->st>>>(c->att_scores, ng * M, G, Rh, TQ, nk, L.window, span, &c->d_step->st, L.scale, L.lambda, g0, T);
+            pdl(c, (rows + 7) / 8, 256, 0, k_diff_softmax_rows, c->att_scores, ng * M, G, Rh, TQ, nk, L.window, span, &c->d_step->st, L.scale, L.lambda, g0, T);
             gemm_f32(c, c->att_scores, nk, (long long) M * nk, keys + (size_t) G * 2 * D, 1, row, sK, c->OL + (size_t) g0 * M * V, V, (long long) M * V, M, V, nk, ng,
                      G, 2 * grp, V, (long long) Tpad * Rh * V);
             c->launches++;
         }
-        k_diff_norm_out<<<dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, c->st>>>(c->OL, Tpad, H, G, V, c->m->eps, 1.0f - L.diff, c->A);
+        pdl(c, dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, k_diff_norm_out, c->OL, Tpad, H, G, V, c->m->eps, 1.0f - L.diff, c->A);
         c->launches += 2;
         linear(c, c->A, H * V, L.o, c->out, E, T);
         return;
@@ -1700,10 +1755,10 @@ void mixer_diffattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T)
                    (D % 4 == 0 && row % 4 == 0 && ((uintptr_t) cache & 15) == 0) ? 1 : 0, nsplit, c->da_part, c->da_counter};
     const dim3 grid((unsigned) ((T + TQ - 1) / TQ), (unsigned) H, (unsigned) nsplit);
     const size_t smem = diffattn_smem(L, TQ);
-    if (V <= 32) k_diff_attn<1><<<grid, 256, smem, c->st>>>(a);
-    else if (V <= 64) k_diff_attn<2><<<grid, 256, smem, c->st>>>(a);
-    else if (V <= 128) k_diff_attn<4><<<grid, 256, smem, c->st>>>(a);
-    else k_diff_attn<8><<<grid, 256, smem, c->st>>>(a);
+    if (V <= 32) pdl(c, grid, 256, smem, k_diff_attn<1>, a);
+    else if (V <= 64) pdl(c, grid, 256, smem, k_diff_attn<2>, a);
+    else if (V <= 128) pdl(c, grid, 256, smem, k_diff_attn<4>, a);
+    else pdl(c, grid, 256, smem, k_diff_attn<8>, a);
     c->launches++;
     linear(c, c->A, H * V, L.o, c->out, E, T);
 }
@@ -1721,7 +1776,8 @@ void launch_outer_walk(StackCtx * c, const OuterScan & s) {
     const int cols = s.V + (s.norm ? 1 : 0);
     int ncols = std::min(128, (cols + 7) / 8 * 8);
     while (ncols > 16 && s.H * ((cols + ncols - 1) / ncols) < c->sm_count) ncols = (ncols / 2 + 7) / 8 * 8;
-    k_outer_scan<DMAX><<<dim3((unsigned) s.H, (unsigned) ((cols + ncols - 1) / ncols)), GD_RG * ncols, 0, c->st>>>(s);
+    spread(c, s.T);
+    pdl(c, dim3((unsigned) s.H, (unsigned) ((cols + ncols - 1) / ncols)), GD_RG * ncols, 0, k_outer_scan<DMAX>, s);
     c->launches++;
 }
 template <int NC>
@@ -1731,9 +1787,9 @@ void launch_outer_chunks(StackCtx * c, const OuterScan & s) {
     const dim3 grid((unsigned) s.H, (unsigned) nch, (unsigned) ((s.V + NC - 1) / NC));
     const auto al16 = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
     const int vec = ((s.ldq | s.ldk | s.ldv | s.D | s.V) & 3) == 0 && al16(s.Q) && al16(s.K) && al16(s.Vv) ? 1 : 0;
-    k_outer_chunk_kv<NC><<<grid, 256, 0, c->st>>>(s, vec, c->scan_sb, c->scan_ac);
-    k_outer_chunk_state<<<dim3((unsigned) s.H, (unsigned) ((n + 255) / 256)), 256, 0, c->st>>>(n, s.head_stride, nch, c->scan_ac, s.S, c->scan_sb);
-    k_outer_chunk_out<NC><<<grid, 128, outer_chunk_smem(s.D, NC), c->st>>>(s, vec, c->scan_sb);
+    pdl(c, grid, 256, 0, k_outer_chunk_kv<NC>, s, vec, c->scan_sb, c->scan_ac);
+    pdl(c, dim3((unsigned) s.H, (unsigned) ((n + 255) / 256)), 256, 0, k_outer_chunk_state, n, s.head_stride, nch, c->scan_ac, s.S, c->scan_sb);
+    pdl(c, grid, 128, outer_chunk_smem(s.D, NC), k_outer_chunk_out<NC>, s, vec, c->scan_sb);
     c->launches += 3;
 }
 // the outer-product recurrence over a portion: long ones chunk by chunk, short ones token by token
@@ -1750,10 +1806,10 @@ template <int KIND>
 void launch_outer_token(StackCtx * c, const OuterToken & t) {
     const int threads = GD_RG * std::min(128, (t.V + 7) / 8 * 8);
     const size_t sm = (size_t) (t.V + 1) * 4;
-    if (t.D <= 32) k_outer_token<32, KIND><<<t.H, threads, sm, c->st>>>(t);
-    else if (t.D <= 64) k_outer_token<64, KIND><<<t.H, threads, sm, c->st>>>(t);
-    else if (t.D <= 128) k_outer_token<128, KIND><<<t.H, threads, sm, c->st>>>(t);
-    else k_outer_token<256, KIND><<<t.H, threads, sm, c->st>>>(t);
+    if (t.D <= 32) pdl(c, t.H, threads, sm, k_outer_token<32, KIND>, t);
+    else if (t.D <= 64) pdl(c, t.H, threads, sm, k_outer_token<64, KIND>, t);
+    else if (t.D <= 128) pdl(c, t.H, threads, sm, k_outer_token<128, KIND>, t);
+    else pdl(c, t.H, threads, sm, k_outer_token<256, KIND>, t);
     c->launches++;
 }
 
@@ -1772,12 +1828,12 @@ void mixer_retention(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T
         linear(c, c->A, HV, L.o, c->out, E, T);
         return;
     }
-    k_retention_prep<<<dim3((unsigned) T, (unsigned) ((2 * H + 3) / 4)), 128, 0, c->st>>>(c->P, ldp, 0, HD, H, D, RopeArgs{L.rope_freq, L.rope_dims, 1.0f}, L.k_scale, &c->d_step->st);
+    pdl(c, dim3((unsigned) T, (unsigned) ((2 * H + 3) / 4)), 128, 0, k_retention_prep, c->P, ldp, 0, HD, H, D, RopeArgs{L.rope_freq, L.rope_dims, 1.0f}, L.k_scale, &c->d_step->st);
     OuterScan s{};
     s.Q = c->P; s.K = c->P + HD; s.Vv = c->P + 2 * HD; s.ldq = s.ldk = s.ldv = ldp;
     s.T = T; s.H = H; s.share = 1; s.D = D; s.V = V; s.kind = SCAN_CONST; s.decay = L.decay; s.S = S; s.head_stride = (long long) L.head_stride; s.O = c->O;
     outer_scan(c, s);
-    k_delta_out<<<dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, c->st>>>(c->O, c->P, ldp, 2 * HD + HV, H, V, nullptr, 0, 0, c->m->eps, c->A);
+    pdl(c, dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, k_delta_out, c->O, c->P, ldp, 2 * HD + HV, H, V, nullptr, 0, 0, c->m->eps, c->A);
     c->launches += 2;
     linear(c, c->A, HV, L.o, c->out, E, T);
 }
@@ -1798,13 +1854,13 @@ void mixer_mlstm(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
         linear(c, c->A, HV, L.o, c->out, E, T);
         return;
     }
-    k_mlstm_gates<<<H, 256, (size_t) 3 * T * 4, c->st>>>(c->P, ldp, gi, gi + H, L.gate_cap, T, H, m_state, c->BG, ldg);
+    pdl(c, H, 256, (size_t) 3 * T * 4, k_mlstm_gates, c->P, ldp, gi, gi + H, L.gate_cap, T, H, m_state, c->BG, ldg);
     OuterScan s{};
     s.Q = c->P; s.K = c->P + HD; s.Vv = c->P + 2 * HD; s.ldq = s.ldk = s.ldv = ldp;
     s.T = T; s.H = H; s.share = 1; s.D = D; s.V = V; s.kind = SCAN_TABLE; s.ab = c->BG; s.ld_ab = ldg; s.S = S; s.head_stride = (long long) L.head_stride;
     s.norm = 1; s.O = c->O; s.den = c->den;
     outer_scan(c, s);
-    k_mlstm_out<<<dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, c->st>>>(c->O, c->den, c->BG, ldg, q_scale, c->P, ldp, 2 * HD + HV, H, V, L.dnorm, c->m->eps, c->A);
+    pdl(c, dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, k_mlstm_out, c->O, c->den, c->BG, ldg, q_scale, c->P, ldp, 2 * HD + HV, H, V, L.dnorm, c->m->eps, c->A);
     c->launches += 2;
     linear(c, c->A, HV, L.o, c->out, E, T);
 }
@@ -1821,13 +1877,13 @@ void mixer_ssd(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     s.T = T; s.H = H; s.share = H / G; s.D = N; s.V = V; s.S = S; s.head_stride = (long long) L.head_stride; s.O = c->O;
     if (T == 1) { s.kind = SCAN_STEP; s.ab = c->P + inner + C; s.ld_ab = ldp; s.dt_bias = L.dt_bias; s.A_log = L.A_log; }
     else {
-        k_step_table<<<T, H >= 128 ? 128 : 32, 0, c->st>>>(c->P + inner + C, ldp, L.dt_bias, L.A_log, H, c->BG, 2 * H);
+        pdl(c, T, H >= 128 ? 128 : 32, 0, k_step_table, c->P + inner + C, ldp, L.dt_bias, L.A_log, H, c->BG, 2 * H);
         c->launches++;
         s.kind = SCAN_TABLE; s.ab = c->BG; s.ld_ab = 2 * H;
     }
     outer_scan(c, s);
     const int n = inner / L.norm_parts, nt = T > 16 ? 256 : std::min(1024, std::max(128, (n + 63) / 64 * 32));
-    k_gated_part_norm<<<dim3((unsigned) T, (unsigned) L.norm_parts), nt, 0, c->st>>>(c->O, c->CV, C, L.skip, c->P, ldp, inner, V, L.norm_parts, L.dnorm, c->m->eps, c->A);
+    pdl(c, dim3((unsigned) T, (unsigned) L.norm_parts), nt, 0, k_gated_part_norm, c->O, c->CV, C, L.skip, c->P, ldp, inner, V, L.norm_parts, L.dnorm, c->m->eps, c->A);
     c->launches++;
     linear(c, c->A, inner, L.o, c->out, E, T);
 }
@@ -1838,13 +1894,13 @@ void launch_selective(StackCtx * c, const LayerSpec & L, const SelScan & s) {
     const int nblk = (s.inner + 256 / LANES - 1) / (256 / LANES);
     if (s.T >= SCAN_CHUNK_MIN_T && s.L && scan_chunks_enabled()) {
         const unsigned rest = (unsigned) ((s.T + s.seg - 1) / s.seg - 1);
-        k_selective_scan<LANES, NS, SEL_FIRST><<<dim3((unsigned) nblk, rest), 256, 0, c->st>>>(s);
-        k_selective_scan<LANES, NS, SEL_REST><<<dim3((unsigned) nblk, rest), 256, 0, c->st>>>(s);
+        pdl(c, dim3((unsigned) nblk, rest), 256, 0, k_selective_scan<LANES, NS, SEL_FIRST>, s);
+        pdl(c, dim3((unsigned) nblk, rest), 256, 0, k_selective_scan<LANES, NS, SEL_REST>, s);
         c->launches++;
     }
-    else if (s.T > 1) k_selective_scan<LANES, NS, SEL_WHOLE><<<nblk, 256, 0, c->st>>>(s);
-    else if (c->m->dtype == STACK_F32) k_selective_token<float, LANES, NS><<<nblk, 256, (size_t) L.dt_rank * 4, c->st>>>(s, (const float *) L.wdt.w, L.wdt.bias, L.dt_rank);
-    else k_selective_token<__nv_bfloat16, LANES, NS><<<nblk, 256, (size_t) L.dt_rank * 4, c->st>>>(s, (const __nv_bfloat16 *) L.wdt.w, L.wdt.bias, L.dt_rank);
+    else if (s.T > 1) pdl(c, nblk, 256, 0, k_selective_scan<LANES, NS, SEL_WHOLE>, s);
+    else if (c->m->dtype == STACK_F32) pdl(c, nblk, 256, (size_t) L.dt_rank * 4, k_selective_token<float, LANES, NS>, s, (const float *) L.wdt.w, L.wdt.bias, L.dt_rank);
+    else pdl(c, nblk, 256, (size_t) L.dt_rank * 4, k_selective_token<__nv_bfloat16, LANES, NS>, s, (const __nv_bfloat16 *) L.wdt.w, L.wdt.bias, L.dt_rank);
     c->launches++;
 }
 // selective scan: P[t] = [ x | z ] -> convolution of x -> [ step latent | B | C ] from it -> step sizes -> scan with skip and gate -> output product
@@ -1873,13 +1929,13 @@ void mixer_sigattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) 
     const int E = c->m->E, H = L.H, G = L.KH, D = L.D, V = L.V, nq = H * D, row = (int) L.cache_row;
     float * cache = c->caches[(size_t) R.cache_index];
     linear(c, c->in, E, L.proj, c->P, L.proj.N, T);
-    k_sigattn_prep<<<T, 256, 0, c->st>>>(c->P, L.proj.N, H, G, D, V, L.qw, L.kw, c->m->eps, L.t_coef, L.t_every, &c->d_step->st, c->CV, cache);
+    pdl(c, T, 256, 0, k_sigattn_prep, c->P, L.proj.N, H, G, D, V, L.qw, L.kw, c->m->eps, L.t_coef, L.t_every, &c->d_step->st, c->CV, cache);
     c->launches++;
     if (T >= 8) {
         // prompt portion: float32 products over tiles of ATT_TQ tokens, one batch entry per (tile, key/value head)
         const int TQ = ATT_TQ, Rh = H / G, M = TQ * Rh, ntile = (T + TQ - 1) / TQ, Tpad = ntile * TQ;
         const int pos0 = c->h_step->st.pos0;
-        k_group_q_layout<<<Tpad, 256, 0, c->st>>>(c->CV, nq, T, Tpad, H, G, D, c->QK);
+        pdl(c, Tpad, 256, 0, k_group_q_layout, c->CV, nq, T, Tpad, H, G, D, c->QK);
         const size_t nk_max = (size_t) (pos0 + Tpad + 3) / 4 * 4;
         const int per_group = (int) std::max<size_t>(1, c->att_scores_floats / ((size_t) G * M * nk_max));
         for (int g0 = 0; g0 < ntile; g0 += per_group) {
@@ -1889,12 +1945,12 @@ void mixer_sigattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) 
             gemm_f32(c, c->QK + (size_t) g0 * M * D, D, (long long) M * D, cache, 0, row, 0, c->att_scores, nk, (long long) M * nk, M, nk, D, ng,
                      G, (long long) Tpad * Rh * D, D, grp);
             const int rows = ng * M * G;
-            k_sig_weight_rows<<<(rows + 7) / 8, 256, 0, c->st>>>(c->att_scores, ng * M, G, Rh, TQ, nk, &c->d_step->st, L.scale, L.slope, L.pb, g0, T);
+            pdl(c, (rows + 7) / 8, 256, 0, k_sig_weight_rows, c->att_scores, ng * M, G, Rh, TQ, nk, &c->d_step->st, L.scale, L.slope, L.pb, g0, T);
             gemm_f32(c, c->att_scores, nk, (long long) M * nk, cache + (size_t) G * D, 1, row, 0, c->OL + (size_t) g0 * M * V, V, (long long) M * V, M, V, nk, ng,
                      G, grp, V, (long long) Tpad * Rh * V);
             c->launches++;
         }
-        k_group_o_layout<<<T, 256, 0, c->st>>>(c->OL, Tpad, H, G, V, c->A);
+        pdl(c, T, 256, 0, k_group_o_layout, c->OL, Tpad, H, G, V, c->A, nullptr, 0, 0);
         c->launches += 2;
         linear(c, c->A, H * V, L.o, c->out, E, T);
         return;
@@ -1907,10 +1963,10 @@ void mixer_sigattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) 
     const dim3 grid((unsigned) ((T + TQ - 1) / TQ), (unsigned) H, (unsigned) nsplit);
     const int VPL = sig_vpl(L);
     const size_t smem = ((size_t) TQ * D + (size_t) 8 * 32 * VPL) * 4;
-    if (VPL == 1) k_sig_attn<1><<<grid, 256, smem, c->st>>>(a);
-    else if (VPL == 2) k_sig_attn<2><<<grid, 256, smem, c->st>>>(a);
-    else if (VPL == 4) k_sig_attn<4><<<grid, 256, smem, c->st>>>(a);
-    else k_sig_attn<8><<<grid, 256, smem, c->st>>>(a);
+    if (VPL == 1) pdl(c, grid, 256, smem, k_sig_attn<1>, a);
+    else if (VPL == 2) pdl(c, grid, 256, smem, k_sig_attn<2>, a);
+    else if (VPL == 4) pdl(c, grid, 256, smem, k_sig_attn<4>, a);
+    else pdl(c, grid, 256, smem, k_sig_attn<8>, a);
     c->launches++;
     linear(c, c->A, H * V, L.o, c->out, E, T);
 }
@@ -1946,9 +2002,9 @@ void mixer_gqattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     linear(c, c->in, E, L.proj, c->P, ldp, T);
     const GqaPrepArgs pa{c->P, ldp, H, G, D, V, L.qw, L.kw, c->m->eps, RopeArgs{L.rope_freq, L.rope_dims, L.rope_mag, L.rope_adjacent ? 1 : 0}, st, c->CV, cache, row,
                          c->VF, L.vmode, L.vlambda, L.unit_qk ? 1 : 0};
-    k_gqa_prep<<<dim3((unsigned) T, T <= 16 ? (unsigned) ((H + G + 7) / 8) : 1u), 256, 0, c->st>>>(pa);      // few tokens: a token's heads over several blocks
+    pdl(c, dim3((unsigned) T, T <= 16 ? (unsigned) ((H + G + 7) / 8) : 1u), 256, 0, k_gqa_prep, pa);      // few tokens: a token's heads over several blocks
     c->launches++;
-    if (L.pool > 0) { k_pool_rows<<<dim3((unsigned) (T / L.pool + 1), (unsigned) ((row + 127) / 128)), 128, 0, c->st>>>(cache, row, pool, L.pool, st); c->launches++; }
+    if (L.pool > 0) { pdl(c, dim3((unsigned) (T / L.pool + 1), (unsigned) ((row + 127) / 128)), 128, 0, k_pool_rows, cache, row, pool, L.pool, st); c->launches++; }
     const float * gate = L.head_gate ? c->P + nq + row : nullptr;
     const int gate_per_entry = L.head_gate && L.gate_rows == H * V && V > 1 ? 1 : 0;
     const GqaMask mask{L.mask_kind, L.window, L.pool};
@@ -1958,7 +2014,7 @@ void mixer_gqattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
         // are [ block means | tokens ]; the token columns of a masked layer start `span` - 1 positions before the tile
         const int TQ = ATT_TQ, Rh = H / G, M = TQ * Rh, ntile = (T + TQ - 1) / TQ, Tpad = ntile * TQ;
         const int pos0 = c->h_step->st.pos0;
-        k_group_q_layout<<<Tpad, 256, 0, c->st>>>(c->CV, nq, T, Tpad, H, G, D, c->QK);
+        pdl(c, Tpad, 256, 0, k_group_q_layout, c->CV, nq, T, Tpad, H, G, D, c->QK);
         const bool masked = L.mask_kind != MASK_CAUSAL;
         const int span = masked ? std::min(L.window, pos0 + Tpad) : 0;
         const size_t nk_max = (size_t) ((masked ? span + TQ - 1 : pos0 + Tpad) + 3) / 4 * 4;
@@ -1979,14 +2035,14 @@ void mixer_gqattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
             if (npc) gemm_f32(c, c->QK + (size_t) g0 * M * D, D, (long long) M * D, pool, 0, row, 0, c->att_scores, ld, (long long) M * ld, M, npc, D, ng,
                               G, (long long) Tpad * Rh * D, D, grp);
             const int rows = ng * M * G;
-            k_gqa_softmax_rows<<<(rows + 7) / 8, 256, 0, c->st>>>(c->att_scores, ng * M, G, Rh, TQ, npc, nk, span, mask, sc, L.r1, L.r2, L.sink, st, g0, T);
+            pdl(c, (rows + 7) / 8, 256, 0, k_gqa_softmax_rows, c->att_scores, ng * M, G, Rh, TQ, npc, nk, span, mask, sc, L.r1, L.r2, L.sink, st, g0, T);
             gemm_f32(c, c->att_scores + npc, ld, (long long) M * ld, keys + (size_t) G * D, 1, row, sK, c->OL + (size_t) g0 * M * V, V, (long long) M * V, M, V, nk, ng,
                      G, grp, V, (long long) Tpad * Rh * V, 0, masked ? See() : See{Rh, pos0 + g0 * TQ, TQ});
             if (npc) gemm_f32(c, c->att_scores, ld, (long long) M * ld, pool + (size_t) G * D, 1, row, 0, c->OL + (size_t) g0 * M * V, V, (long long) M * V, M, V, npc, ng,
                               G, grp, V, (long long) Tpad * Rh * V, 1);
             c->launches++;
         }
-        k_group_o_layout<<<T, 256, 0, c->st>>>(c->OL, Tpad, H, G, V, c->A, gate, ldp, gate_per_entry);      // the gates ride on the regrouping
+        pdl(c, T, 256, 0, k_group_o_layout, c->OL, Tpad, H, G, V, c->A, gate, ldp, gate_per_entry);      // the gates ride on the regrouping
         c->launches += 2;
         linear(c, c->A, H * V, L.o, c->out, E, T);
         return;
@@ -1999,10 +2055,10 @@ void mixer_gqattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
         const dim3 grid((unsigned) T, (unsigned) (G * ngrp), (unsigned) nsplit);
         const size_t smem = gqg_smem(RT, V);
         const bool wide = D > 128 || V > 128;
-        if (RT == 1) { if (wide) k_gqa_attn_group<1, 2><<<grid, 256, smem, c->st>>>(a); else k_gqa_attn_group<1, 1><<<grid, 256, smem, c->st>>>(a); }
-        else if (RT == 2) { if (wide) k_gqa_attn_group<2, 2><<<grid, 256, smem, c->st>>>(a); else k_gqa_attn_group<2, 1><<<grid, 256, smem, c->st>>>(a); }
-        else if (RT == 4) { if (wide) k_gqa_attn_group<4, 2><<<grid, 256, smem, c->st>>>(a); else k_gqa_attn_group<4, 1><<<grid, 256, smem, c->st>>>(a); }
-        else k_gqa_attn_group<8, 1><<<grid, 256, smem, c->st>>>(a);
+        if (RT == 1) { if (wide) pdl(c, grid, 256, smem, k_gqa_attn_group<1, 2>, a); else pdl(c, grid, 256, smem, k_gqa_attn_group<1, 1>, a); }
+        else if (RT == 2) { if (wide) pdl(c, grid, 256, smem, k_gqa_attn_group<2, 2>, a); else pdl(c, grid, 256, smem, k_gqa_attn_group<2, 1>, a); }
+        else if (RT == 4) { if (wide) pdl(c, grid, 256, smem, k_gqa_attn_group<4, 2>, a); else pdl(c, grid, 256, smem, k_gqa_attn_group<4, 1>, a); }
+        else pdl(c, grid, 256, smem, k_gqa_attn_group<8, 1>, a);
         c->launches++;
         linear(c, c->A, H * V, L.o, c->out, E, T);
         return;
@@ -2015,10 +2071,10 @@ void mixer_gqattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     const dim3 grid((unsigned) ((T + TQ - 1) / TQ), (unsigned) H, (unsigned) nsplit);
     const int VPL = gqa_vpl(L);
     const size_t smem = ((size_t) TQ * D + (size_t) 8 * (2 + 32 * VPL)) * 4;
-    if (VPL == 1) k_gqa_attn<1><<<grid, 256, smem, c->st>>>(a);
-    else if (VPL == 2) k_gqa_attn<2><<<grid, 256, smem, c->st>>>(a);
-    else if (VPL == 4) k_gqa_attn<4><<<grid, 256, smem, c->st>>>(a);
-    else k_gqa_attn<8><<<grid, 256, smem, c->st>>>(a);
+    if (VPL == 1) pdl(c, grid, 256, smem, k_gqa_attn<1>, a);
+    else if (VPL == 2) pdl(c, grid, 256, smem, k_gqa_attn<2>, a);
+    else if (VPL == 4) pdl(c, grid, 256, smem, k_gqa_attn<4>, a);
+    else pdl(c, grid, 256, smem, k_gqa_attn<8>, a);
     c->launches++;
     linear(c, c->A, H * V, L.o, c->out, E, T);
 }
@@ -2066,8 +2122,8 @@ void enqueue_layers_sequential(StackCtx * c, int T) {
     const int E = m.E;
     const int nthreads = std::min(256, std::max(128, 32 * m.groups));
     const float * w0 = m.layers[(size_t) m.runs[0].layer].norm1;
-    if (m.dtype == STACK_F32) k_embed_rows<float><<<T, nthreads, 0, c->st>>>((const float *) m.embed, c->d_step->tokens, E, m.vocab, c->X, w0, m.groups, m.eps, c->Hn);
-    else k_embed_rows<__nv_bfloat16><<<T, nthreads, 0, c->st>>>((const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, c->X, w0, m.groups, m.eps, c->Hn);
+    if (m.dtype == STACK_F32) pdl(c, T, nthreads, 0, k_embed_rows<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, c->X, w0, m.groups, m.eps, c->Hn);
+    else pdl(c, T, nthreads, 0, k_embed_rows<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, c->X, w0, m.groups, m.eps, c->Hn);
     c->launches++;
     c->in = c->Hn; c->out = c->Y;
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
@@ -2093,8 +2149,8 @@ void enqueue_layers_parallel(StackCtx * c, int T) {
     const int E = m.E, ct = m.canon_taps;
     const size_t plane = (size_t) c->cap * E;
     const bool looped = m.loop_step != nullptr;
-    if (m.dtype == STACK_F32) k_embed_plain<float><<<T, 128, 0, c->st>>>((const float *) m.embed, c->d_step->tokens, E, m.vocab, c->X, looped ? c->XC + E : nullptr, 2 * E);
-    else k_embed_plain<__nv_bfloat16><<<T, 128, 0, c->st>>>((const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, c->X, looped ? c->XC + E : nullptr, 2 * E);
+    if (m.dtype == STACK_F32) pdl(c, T, 128, 0, k_embed_plain<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, c->X, looped ? c->XC + E : nullptr, 2 * E, 1.0f);
+    else pdl(c, T, 128, 0, k_embed_plain<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, c->X, looped ? c->XC + E : nullptr, 2 * E, 1.0f);
     c->launches++;
     const float * ya = nullptr, * yb = nullptr;        // outputs of the layer before, not yet added to X
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
@@ -2103,7 +2159,7 @@ void enqueue_layers_parallel(StackCtx * c, int T) {
         float * H1 = c->Hn, * H2 = c->Hn + plane;
         if (R.pass >= 0) {
             // x <- W_in [x; x0] + step[pass]: the finished x goes to the left half of XC (x0 is in the right half since the embedding)
-            k_add_norm2<<<T, 256, 0, c->st>>>(c->X, ya, yb, c->XC, 2 * E, nullptr, nullptr, nullptr, nullptr, E, m.eps);
+            pdl(c, T, 256, 0, k_add_norm2, c->X, ya, yb, c->XC, 2 * E, nullptr, nullptr, nullptr, nullptr, E, m.eps);
             c->launches++;
             ya = yb = nullptr;
             DMat w = m.loop_in;
@@ -2114,11 +2170,11 @@ void enqueue_layers_parallel(StackCtx * c, int T) {
         const float * u1 = H1, * u2 = H2;
         float * hist = c->rec + R.off_rec + (L.n_rec - (size_t) nsub * std::max(ct - 1, 0) * E);
         if (T == 1 && ct > 0) {                        // one token: sum, both norms, both input convolutions and their history in one launch
-            k_add_norm2_canon1<<<CANON1_CTAS, 256, 0, c->st>>>(c->X, ya, yb, L.norm1, L.has_mlp ? L.norm2 : nullptr, L.canon, hist, c->U, (long long) plane, E, ct, m.eps);
+            pdl(c, CANON1_CTAS, 256, 0, k_add_norm2_canon1, c->X, ya, yb, L.norm1, L.has_mlp ? L.norm2 : nullptr, L.canon, hist, c->U, (long long) plane, E, ct, m.eps);
             c->launches++;
             u1 = c->U; u2 = c->U + plane;
         } else {
-            k_add_norm2<<<T, 256, 0, c->st>>>(c->X, ya, yb, nullptr, 0, L.norm1, L.has_mlp ? L.norm2 : nullptr, H1, H2, E, m.eps);
+            pdl(c, T, 256, 0, k_add_norm2, c->X, ya, yb, nullptr, 0, L.norm1, L.has_mlp ? L.norm2 : nullptr, H1, H2, E, m.eps);
             c->launches++;
         }
         if (ct > 0 && T > 1) {
@@ -2131,13 +2187,13 @@ void enqueue_layers_parallel(StackCtx * c, int T) {
         ya = c->Y; yb = nullptr;
         if (L.has_mlp) {
             linear(c, u2, E, L.gateup, c->A, L.ff, T);
-            k_polynorm<<<T, 256, 0, c->st>>>(c->A, L.ff, L.act, m.eps);
+            pdl(c, T, 256, 0, k_polynorm, c->A, L.ff, L.act, m.eps);
             c->launches++;
             linear(c, c->A, L.ff, L.down, c->Y2, E, T);
             yb = c->Y2;
         }
         if (c->taps || ri + 1 == m.runs.size()) {      // the residual stream itself is wanted now
-            k_add_norm2<<<T, 256, 0, c->st>>>(c->X, ya, yb, nullptr, 0, nullptr, nullptr, nullptr, nullptr, E, m.eps);
+            pdl(c, T, 256, 0, k_add_norm2, c->X, ya, yb, nullptr, 0, nullptr, nullptr, nullptr, nullptr, E, m.eps);
             c->launches++;
             ya = yb = nullptr;
             if (c->taps) tap_layer(c, ri, T);
@@ -2152,7 +2208,7 @@ void enqueue_layers_parallel(StackCtx * c, int T) {
 void mixture_ff(StackCtx * c, const LayerSpec & L, const float * h, int T, const int32_t ** slot_of) {
     const int E = c->m->E, top = L.top, ff = L.e_ff, slots = T * top, n = L.n_exp + L.n_ident;
     const RouteArgs ra{h, E, E, L.router, L.w_sg, n, top, L.n_groups, L.keep_groups, L.r_scale, c->r_sel, c->r_wt, c->r_sg, c->r_z, c->r_counter, L.route_fn, T <= 16 ? 8 : 1, L.corr, L.norm_w ? 1 : 0, L.r_bias};
-    k_moe_route<<<dim3((unsigned) T, (unsigned) ((n + (L.w_sg ? 1 : 0) + 8 / ra.wpr - 1) / (8 / ra.wpr))), 256, (size_t) (2 * n + L.n_groups) * 4, c->st>>>(ra);
+    pdl(c, dim3((unsigned) T, (unsigned) ((n + (L.w_sg ? 1 : 0) + 8 / ra.wpr - 1) / (8 / ra.wpr))), 256, (size_t) (2 * n + L.n_groups) * 4, k_moe_route, ra);
     c->launches++;
     LinOpt o;
     o.glu_kind = L.act_kind; o.alpha = L.act_alpha; o.shift = L.act_shift;
@@ -2170,9 +2226,9 @@ void mixture_ff(StackCtx * c, const LayerSpec & L, const float * h, int T, const
         while (tpe * 2 * n <= 1024 && tpe * 2 <= slots) tpe *= 2;
         const size_t cnt_bytes = (size_t) n * tpe * 4;
         const int in_smem = (size_t) slots * 4 + cnt_bytes <= 40 * 1024 ? 1 : 0;
-        k_moe_sort<<<1, 1024, cnt_bytes + (in_smem ? (size_t) slots * 4 : 0), c->st>>>(c->r_sel, slots, top, n, tpe, in_smem, c->r_seg, c->r_slot, c->r_src);
-        if (L.scale_input) k_spread_rows<<<slots, 128, 0, c->st>>>(h, E, c->r_slot, c->r_wt, top, E, c->Xp);
-        else k_gather_rows<<<slots, 128, 0, c->st>>>(h, E, c->r_src, E, c->Xp);
+        pdl(c, 1, 1024, cnt_bytes + (in_smem ? (size_t) slots * 4 : 0), k_moe_sort, c->r_sel, slots, top, n, tpe, in_smem, c->r_seg, c->r_slot, c->r_src);
+        if (L.scale_input) pdl(c, slots, 128, 0, k_spread_rows, h, E, c->r_slot, c->r_wt, top, E, c->Xp);
+        else pdl(c, slots, 128, 0, k_gather_rows, h, E, c->r_src, E, c->Xp);
         c->launches += 2;
         o.seg = c->r_seg;
         linear(c, c->Xp, E, L.e_gateup, c->Ap, ff, slots, L.n_exp, 0, 0, true, L.e_limit, &o);      // rows of identity outputs sort behind the last matrix
@@ -2197,8 +2253,8 @@ void enqueue_layers_prenorm(StackCtx * c, int T) {
     {
         const LayerSpec & L0 = m.layers[(size_t) m.runs[0].layer];
         const DytW ne{m.embed_w, m.embed_b, m.embed_alpha}, n1{L0.norm1, L0.n1_b, L0.n1_alpha};
-        if (m.dtype == STACK_F32) k_embed_dyt<float><<<T, 256, 0, c->st>>>((const float *) m.embed, c->d_step->tokens, E, m.vocab, ne, n1, c->X, m.depth_avg ? c->keep : nullptr, c->Hn);
-        else k_embed_dyt<__nv_bfloat16><<<T, 256, 0, c->st>>>((const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, ne, n1, c->X, m.depth_avg ? c->keep : nullptr, c->Hn);
+        if (m.dtype == STACK_F32) pdl(c, T, 256, 0, k_embed_dyt<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, ne, n1, c->X, m.depth_avg ? c->keep : nullptr, c->Hn);
+        else pdl(c, T, 256, 0, k_embed_dyt<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, ne, n1, c->X, m.depth_avg ? c->keep : nullptr, c->Hn);
         c->launches++;
     }
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
@@ -2215,7 +2271,7 @@ void enqueue_layers_prenorm(StackCtx * c, int T) {
             if (N) { a.nw = N->norm1; a.nb = N->n1_b; a.alpha = N->n1_alpha; a.Hn = c->Hn; }
         };
         if (L.has_mlp) { j.nw = L.norm2; j.nb = L.n2_b; j.alpha = L.n2_alpha; j.Hn = c->Hn; } else layer_end(j);
-        k_join<<<jgrid, 256, 0, c->st>>>(j);
+        pdl(c, jgrid, 256, 0, k_join, j);
         c->launches++;
         if (L.has_mlp) {
             JoinArgs f{};
@@ -2224,7 +2280,7 @@ void enqueue_layers_prenorm(StackCtx * c, int T) {
             f.Yk = c->Yk; f.wt = c->r_wt; f.top = L.top;
             if (L.ff > 0) { f.Ysh = c->Y; f.sg = c->r_sg; }
             layer_end(f);
-            k_join<<<jgrid, 256, 0, c->st>>>(f);
+            pdl(c, jgrid, 256, 0, k_join, f);
             c->launches++;
         }
         if (c->taps) tap_layer(c, ri, T);
@@ -2241,8 +2297,8 @@ void enqueue_layers_hyper(StackCtx * c, int T) {
     const long long plane = (long long) c->cap * E;
     {
         const LayerSpec & L0 = m.layers[(size_t) m.runs[0].layer];
-        if (m.dtype == STACK_F32) k_hc_embed<float><<<T, hc_threads(T, E), 0, c->st>>>((const float *) m.embed, c->d_step->tokens, E, m.vocab, S, c->XS, plane, L0.hc[0], L0.g1, m.eps, c->Hn);
-        else k_hc_embed<__nv_bfloat16><<<T, hc_threads(T, E), 0, c->st>>>((const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, S, c->XS, plane, L0.hc[0], L0.g1, m.eps, c->Hn);
+        if (m.dtype == STACK_F32) pdl(c, T, hc_threads(T, E), 0, k_hc_embed<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, S, c->XS, plane, L0.hc[0], L0.g1, m.eps, c->Hn);
+        else pdl(c, T, hc_threads(T, E), 0, k_hc_embed<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, S, c->XS, plane, L0.hc[0], L0.g1, m.eps, c->Hn);
         c->launches++;
     }
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
@@ -2257,8 +2313,8 @@ void enqueue_layers_hyper(StackCtx * c, int T) {
             if (nw) { for (int s = 0; s < HC_MAX; s++) j.nin[s] = nw->in[s]; j.g = !last_sub ? L.g2 : N->g1; j.Hn = c->Hn; }
             else { for (int s = 0; s < S; s++) j.nin[s] = 1.f; j.g = m.final_g; j.Hn = c->Hn; }      // after the last layer: the model's norm of the sum of the streams
             if (last_sub && c->taps) j.Xsum = c->X;
-            if (E % 4 == 0) k_hc_join<4><<<T, hc_threads(T, E, 4, 512), 0, c->st>>>(j);      // every buffer of a context is 16-byte aligned and its rows are E floats apart
-            else k_hc_join<1><<<T, hc_threads(T, E), 0, c->st>>>(j);
+            if (E % 4 == 0) pdl(c, T, hc_threads(T, E, 4, 512), 0, k_hc_join<4>, j);      // every buffer of a context is 16-byte aligned and its rows are E floats apart
+            else pdl(c, T, hc_threads(T, E), 0, k_hc_join<1>, j);
             c->launches++;
         };
         c->in = c->Hn; c->out = c->Y;
@@ -2283,8 +2339,8 @@ void enqueue_layers_hyper(StackCtx * c, int T) {
 void enqueue_layers_postnorm(StackCtx * c, int T) {
     StackModel & m = *c->m;
     const int E = m.E;
-    if (m.dtype == STACK_F32) k_embed_plain<float><<<T, hc_threads(T, E), 0, c->st>>>((const float *) m.embed, c->d_step->tokens, E, m.vocab, c->X, nullptr, 0, m.embed_scale);
-    else k_embed_plain<__nv_bfloat16><<<T, hc_threads(T, E), 0, c->st>>>((const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, c->X, nullptr, 0, m.embed_scale);
+    if (m.dtype == STACK_F32) pdl(c, T, hc_threads(T, E), 0, k_embed_plain<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, c->X, nullptr, 0, m.embed_scale);
+    else pdl(c, T, hc_threads(T, E), 0, k_embed_plain<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, c->X, nullptr, 0, m.embed_scale);
     c->launches++;
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
         const RunSpec & R = m.runs[ri];
@@ -2293,8 +2349,8 @@ void enqueue_layers_postnorm(StackCtx * c, int T) {
         const auto join = [&](PostJoinArgs & j, const float * w, bool end) {
             j.X = c->X; j.E = E; j.eps = m.eps; j.mult = m.residual_mult; j.w = w; j.scratch = c->Hn;
             if (end && last) { j.fw = m.final_norm; j.Hn = c->Hn; }
-            if (E % 4 == 0) k_post_join<4><<<T, hc_threads(T, E, 4), 0, c->st>>>(j);      // every buffer of a context is 16-byte aligned and its rows are E floats apart
-            else k_post_join<1><<<T, hc_threads(T, E), 0, c->st>>>(j);
+            if (E % 4 == 0) pdl(c, T, hc_threads(T, E, 4), 0, k_post_join<4>, j);      // every buffer of a context is 16-byte aligned and its rows are E floats apart
+            else pdl(c, T, hc_threads(T, E), 0, k_post_join<1>, j);
             c->launches++;
         };
         c->in = c->X; c->out = c->Y;
@@ -2334,8 +2390,8 @@ bool side_fused_enabled() {
 // while it lives, launches go to the context's second stream
 struct SideStream {
     StackCtx * c; bool on;
-    SideStream(StackCtx * c_, bool on_) : c(c_), on(on_) { if (on) std::swap(c->st, c->st2); }
-    ~SideStream() { if (on) std::swap(c->st, c->st2); }
+    SideStream(StackCtx * c_, bool on_) : c(c_), on(on_) { if (on) { std::swap(c->st, c->st2); c->cold = true; } }
+    ~SideStream() { if (on) { std::swap(c->st, c->st2); c->cold = true; } }
 };
 
 // end of a layer of a shared-input block: X += Ya + Yb (or the mixture's choices), then the token's own input, then the norm nw -> Hn
@@ -2352,8 +2408,8 @@ void layer_end(StackCtx * c, const LayerSpec & L, SumArgs a, const float * nw, i
         a.nw = nw;
         const dim3 g1((unsigned) ((dim + SIDE_ROWS - 1) / SIDE_ROWS), (unsigned) T), g2((unsigned) ((E + side_rows_per_block(lpr) - 1) / side_rows_per_block(lpr)), (unsigned) T);
         const auto go = [&](auto in, auto out) {
-            in<<<g1, SIDE_THREADS, (size_t) E * 4, c->st>>>(a, s, c->d_step->tokens, m.vocab, E % vecw == 0 ? 1 : 0, c->XE, c->SZ);
-            out<<<g2, SIDE_THREADS, (size_t) dim * 4, c->st>>>(a, s, c->XE, c->SZ, c->Y, c->end_counter, dim % vecw == 0 ? 1 : 0, lpr);      // Y: the mixer's output has been summed by then
+            pdl(c, g1, SIDE_THREADS, (size_t) E * 4, in, a, s, c->d_step->tokens, m.vocab, E % vecw == 0 ? 1 : 0, c->XE, c->SZ);
+            pdl(c, g2, SIDE_THREADS, (size_t) dim * 4, out, a, s, c->XE, c->SZ, c->Y, c->end_counter, dim % vecw == 0 ? 1 : 0, lpr);      // Y: the mixer's output has been summed by then
         };
         if (m.dtype == STACK_F32) { if (E % 4 == 0) go(k_side_in<float>, k_side_out<float, 4>); else go(k_side_in<float>, k_side_out<float, 1>); }
         else if (E % 4 == 0) go(k_side_in<__nv_bfloat16>, k_side_out<__nv_bfloat16, 4>);
@@ -2361,19 +2417,19 @@ void layer_end(StackCtx * c, const LayerSpec & L, SumArgs a, const float * nw, i
         c->launches += 2;
         return;
     }
-    if (E % 4 == 0) k_sum_join<4><<<T, nt, 0, c->st>>>(a);      // every buffer of a context is 16-byte aligned and its rows are E floats apart
-    else k_sum_join<1><<<T, hc_threads(T, E), 0, c->st>>>(a);
+    if (E % 4 == 0) pdl(c, T, nt, 0, k_sum_join<4>, a);      // every buffer of a context is 16-byte aligned and its rows are E floats apart
+    else pdl(c, T, hc_threads(T, E), 0, k_sum_join<1>, a);
     c->launches++;
     if (dim <= 0) return;
     linear(c, c->X, E, L.side_gate, c->SZ, dim, T);
     const dim3 zgrid((unsigned) T, (unsigned) ((dim + 127) / 128));
-    if (m.dtype == STACK_F32) k_side_gate<float><<<zgrid, 128, 0, c->st>>>(c->SZ, s, c->d_step->tokens, m.vocab);
-    else k_side_gate<__nv_bfloat16><<<zgrid, 128, 0, c->st>>>(c->SZ, s, c->d_step->tokens, m.vocab);
+    if (m.dtype == STACK_F32) pdl(c, zgrid, 128, 0, k_side_gate<float>, c->SZ, s, c->d_step->tokens, m.vocab);
+    else pdl(c, zgrid, 128, 0, k_side_gate<__nv_bfloat16>, c->SZ, s, c->d_step->tokens, m.vocab);
     linear(c, c->SZ, dim, L.side_proj, c->Y, E, T);
     PostJoinArgs j{};
     j.X = c->X; j.E = E; j.eps = m.eps; j.mult = 1.f; j.w = L.side_norm; j.scratch = c->Hn; j.Ya = c->Y; j.fw = nw; j.Hn = c->Hn;
-    if (E % 4 == 0) k_post_join<4><<<T, nt, 0, c->st>>>(j);
-    else k_post_join<1><<<T, hc_threads(T, E), 0, c->st>>>(j);
+    if (E % 4 == 0) pdl(c, T, nt, 0, k_post_join<4>, j);
+    else pdl(c, T, hc_threads(T, E), 0, k_post_join<1>, j);
     c->launches += 2;
 }
 
@@ -2385,8 +2441,8 @@ void enqueue_layers_shared(StackCtx * c, int T) {
     const int E = m.E, nt = hc_threads(T, E);
     const float * w0 = m.layers[(size_t) m.runs[0].layer].norm1;
     const PairTable pt{m.pair_table, (unsigned long long) m.pair_mul_prev, (unsigned long long) m.pair_mul_cur, (unsigned long long) m.pair_buckets};
-    if (m.dtype == STACK_F32) k_embed_pair<float><<<T, nt, 0, c->st>>>((const float *) m.embed, pt, &c->d_step->st, c->d_step->tokens, E, m.vocab, w0, m.eps, c->X, c->Hn);
-    else k_embed_pair<__nv_bfloat16><<<T, nt, 0, c->st>>>((const __nv_bfloat16 *) m.embed, pt, &c->d_step->st, c->d_step->tokens, E, m.vocab, w0, m.eps, c->X, c->Hn);
+    if (m.dtype == STACK_F32) pdl(c, T, nt, 0, k_embed_pair<float>, (const float *) m.embed, pt, &c->d_step->st, c->d_step->tokens, E, m.vocab, w0, m.eps, c->X, c->Hn);
+    else pdl(c, T, nt, 0, k_embed_pair<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, pt, &c->d_step->st, c->d_step->tokens, E, m.vocab, w0, m.eps, c->X, c->Hn);
     c->launches++;
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
         const RunSpec & R = m.runs[ri];
@@ -2420,6 +2476,7 @@ void enqueue_layers_shared(StackCtx * c, int T) {
 
 // the layers over the T tokens whose header (positions, ids) is already on the device
 void enqueue_layers(StackCtx * c, int T) {
+    c->cold = true;
     if (c->m->block == BLOCK_PARALLEL) enqueue_layers_parallel(c, T);
     else if (c->m->block == BLOCK_PRENORM) enqueue_layers_prenorm(c, T);
     else if (c->m->block == BLOCK_HYPER) enqueue_layers_hyper(c, T);
@@ -2435,14 +2492,14 @@ void enqueue_head(StackCtx * c, int n_rows, int64_t row_off, bool one_token = fa
     const float * hn = c->Hn;
     if (normed) {
         // the last join left the normed residual (the sum of the streams) in Hn for every row of the pass: the wanted rows are gathered for the head
-        if (!one_token) { k_gather_rows<<<n_rows, 128, 0, c->st>>>(c->Hn, m.E, c->d_step->rows, m.E, c->Y); c->launches++; hn = c->Y; }
+        if (!one_token) { pdl(c, n_rows, 128, 0, k_gather_rows, c->Hn, m.E, c->d_step->rows, m.E, c->Y); c->launches++; hn = c->Y; }
     }
-    else if (m.dyt) { k_dyt_rows<<<n_rows, 256, 0, c->st>>>(c->X, m.E, c->d_step->rows, DytW{m.final_norm, m.final_b, m.final_alpha}, m.E, c->Hn, m.E); c->launches++; }
+    else if (m.dyt) { pdl(c, n_rows, 256, 0, k_dyt_rows, c->X, m.E, c->d_step->rows, DytW{m.final_norm, m.final_b, m.final_alpha}, m.E, c->Hn, m.E); c->launches++; }
     else norm(c, c->X, m.E, c->d_step->rows, m.final_norm, m.E, m.groups, c->Hn, m.E, n_rows, false);
     linear(c, hn, m.E, m.head, c->d_logits + row_off * m.vocab, m.vocab, n_rows);
     if (m.softcap > 0.f) {
         const size_t n = (size_t) n_rows * m.vocab;
-        k_softcap<<<(unsigned) ((n + 255) / 256), 256, 0, c->st>>>(c->d_logits + row_off * m.vocab, n, m.softcap);
+        pdl(c, (unsigned) ((n + 255) / 256), 256, 0, k_softcap, c->d_logits + row_off * m.vocab, n, m.softcap);
         c->launches++;
     }
 }
@@ -2802,7 +2859,7 @@ void stack_generate_greedy(StackCtx * c, int32_t first_token, int pos0, int n_st
     const auto body = [&]() {
         enqueue_layers(c, 1);
         enqueue_head(c, 1, 0, true);
-        k_argmax_advance<<<1, 1024, 0, c->st>>>(c->d_logits, m.vocab, &c->d_step->st, c->d_step->tokens, c->d_out_tokens, c->d_counter);
+        pdl(c, 1, 1024, 0, k_argmax_advance, c->d_logits, m.vocab, &c->d_step->st, c->d_step->tokens, c->d_out_tokens, c->d_counter);
         c->launches++;
     };
     if (!c->g_greedy) {
@@ -2852,7 +2909,7 @@ float * stack_logits_view(StackCtx * c) {
 int32_t stack_argmax(StackCtx * c) {
     if (c->d_last_row < 0) throw std::runtime_error("no logits yet: the last step asked for none");
     SCU(cudaSetDevice(c->m->device));
-    k_argmax_row<<<1, 1024, 0, c->st>>>(c->d_logits + (size_t) c->d_last_row * c->m->vocab, c->m->vocab, c->d_arg);
+    pdl(c, 1, 1024, 0, k_argmax_row, c->d_logits + (size_t) c->d_last_row * c->m->vocab, c->m->vocab, c->d_arg);
     c->launches++;
     SCU(cudaMemcpyAsync(c->h_arg, c->d_arg, 4, cudaMemcpyDeviceToHost, c->st));
     SCU(cudaStreamSynchronize(c->st));
@@ -2879,10 +2936,10 @@ float stack_time_linear(int device, int dtype, int T, int N, int K, int reps) {
         us.elems = (size_t) T * K;
         SCU(cudaMalloc(&us.xb, us.elems * 2)); us.part_floats = umma_part_floats(us.sm_count); SCU(cudaMalloc(&us.part, us.part_floats * 4)); SCU(cudaMalloc(&us.err, 4)); SCU(cudaMemset(us.err, 0, 4));
         SCU(cudaStreamCreate(&st)); SCU(cudaEventCreate(&e0)); SCU(cudaEventCreate(&e1));
-        for (int i = 0; i < 3; i++) linear_on(st, dtype, nullptr, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
+        for (int i = 0; i < 3; i++) linear_on(Lane{st}, dtype, nullptr, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
         SCU(cudaStreamSynchronize(st));
         SCU(cudaEventRecord(e0, st));
-        for (int i = 0; i < reps; i++) linear_on(st, dtype, nullptr, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
+        for (int i = 0; i < reps; i++) linear_on(Lane{st}, dtype, nullptr, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
         SCU(cudaEventRecord(e1, st));
         SCU(cudaStreamSynchronize(st));
         cudaEventElapsedTime(&ms, e0, e1);
@@ -2896,7 +2953,7 @@ float stack_time_linear(int device, int dtype, int T, int N, int K, int reps) {
     return ms / (float) std::max(reps, 1);
 }
 
-void stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y) {
+void stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y, bool in_pass) {
     SCU(cudaSetDevice(device));
     StackModel tmp;                      // owns the device copies
     tmp.device = device; tmp.dtype = dtype;
@@ -2913,7 +2970,8 @@ void stack_linear(int device, int dtype, int T, int N, int K, const float * x, c
         SCU(cudaMemcpy(X, x, (size_t) T * K * 4, cudaMemcpyHostToDevice));
         us.elems = (size_t) T * K;
         SCU(cudaMalloc(&us.xb, us.elems * 2)); us.part_floats = umma_part_floats(us.sm_count); SCU(cudaMalloc(&us.part, us.part_floats * 4)); SCU(cudaMalloc(&us.err, 4)); SCU(cudaMemset(us.err, 0, 4));
-        linear_on(nullptr, dtype, nullptr, X, K, d.w, d.bias, Y, ny, T, N, K, 1, 0, 0, 0, glu != 0, limit, &us);
+        bool cold = true;
+        for (int i = 0; i < (in_pass ? 2 : 1); i++) linear_on(Lane{nullptr, in_pass ? &cold : nullptr}, dtype, nullptr, X, K, d.w, d.bias, Y, ny, T, N, K, 1, 0, 0, 0, glu != 0, limit, &us);
         SCU(cudaDeviceSynchronize());
         SCU(cudaMemcpy(y, Y, (size_t) T * ny * 4, cudaMemcpyDeviceToHost));
         SCU(cudaMemcpy(&herr, us.err, 4, cudaMemcpyDeviceToHost));

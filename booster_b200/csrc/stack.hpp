@@ -57,6 +57,6 @@ float   stack_time_linear(int device, int dtype, int T, int N, int K, int reps);
 int     stack_product_kernel(int dtype, int T, int N, int K, bool glu, int sm_count);
 // one product y[T][N] = x[T][K] w[N][K]^T (+ bias; glu: rows of w interleaved gate/up, y[T][N/2] = the clamped gated unit)
 // through the kernel the family would pick for that shape (parity tests)
-void    stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y);
+void    stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y, bool in_pass = false);
 
 }  // namespace b200

@@ -21,6 +21,15 @@
 namespace b200 {
 namespace stk {
 
+// Programmatic dependent launch: a pass's kernels are launched so that one may become resident while the one before it still runs. pdl_launch_dependents() lets the next
+// kernel's blocks in as soon as there is room, pdl_wait() returns when the kernel before has completed and its writes are visible. Every kernel here waits before it reads
+// anything another kernel writes and before it writes anything: what may come first are its own set-up and reads of weights. A kernel that waits for its predecessor thereby
+// waits for all before it, since that one has waited too: no path through a kernel leaves out the wait. Without the launch attribute both are no-ops.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel is let in behind the wait and not in front of it: earlier, several kernels queue up on the SMs one behind the other, and a large one finds some SMs with room for
+// two of its blocks and others full (a gated unit of 16384 x 2048 in bf16, one block per SM: 11 us alone on the SMs and 16 behind such a queue).
+__device__ __forceinline__ void pdl_enter() { pdl_wait(); pdl_launch_dependents(); }
 
 __device__ __forceinline__ float wf(const float * p, size_t i) { return p[i]; }
 __device__ __forceinline__ float wf(const __nv_bfloat16 * p, size_t i) { return __bfloat162float(p[i]); }
@@ -56,7 +65,7 @@ struct StepState {
 };
 
 // ---- RMS norm of one group by one warp: y = x / sqrt(mean(x^2) + eps) * w ------------------------------------------------
-__device__ __forceinline__ void warp_group_norm(const float * __restrict__ x, const float * __restrict__ w, int gs, float eps, float * __restrict__ y, int lane) {
+__device__ __forceinline__ void warp_group_norm(const float * x, const float * __restrict__ w, int gs, float eps, float * y, int lane) {
     float ss = 0.f;
     for (int i = lane; i < gs; i += 32) { const float v = x[i]; ss = fmaf(v, v, ss); }
     ss = warp_sum(ss);
@@ -64,39 +73,62 @@ __device__ __forceinline__ void warp_group_norm(const float * __restrict__ x, co
     for (int i = lane; i < gs; i += 32) y[i] = x[i] * r * w[i];
 }
 
+constexpr int POST_NPL = 16;       // elements per lane that k_embed_rows and k_post_norm_add keep in registers (groups of up to 512)
 // ---- embedding fused with the first layer's input norm: X[t] = embed[token[t]], Hn[t] = norm(X[t]) * w ---------------------
 template <typename WT>
-__global__ void k_embed_rows(const WT * __restrict__ embed, const int32_t * __restrict__ tokens, int E, int n_vocab, float * __restrict__ X,
-                             const float * __restrict__ w, int groups, float eps, float * __restrict__ Hn) {
+__global__ void k_embed_rows(const WT * __restrict__ embed, const int32_t * tokens, int E, int n_vocab, float * X,
+                             const float * __restrict__ w, int groups, float eps, float * Hn) {
+    pdl_enter();
     const int t = blockIdx.x;
     int tok = tokens[t];
     tok = tok < 0 ? 0 : tok >= n_vocab ? n_vocab - 1 : tok;      // ids are validated on the host; never read outside the table
-    for (int i = threadIdx.x; i < E; i += blockDim.x) X[(size_t) t * E + i] = wf(embed, (size_t) tok * E + i);
-    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, gs = E / groups;
-    for (int g = warp; g < groups; g += nw) warp_group_norm(X + (size_t) t * E + g * gs, w + g * gs, gs, eps, Hn + (size_t) t * E + g * gs, lane);
+    const WT * e = embed + (size_t) tok * E;
+    for (int g = warp; g < groups; g += nw) {
+        const size_t b = (size_t) t * E + (size_t) g * gs;
+        if (gs <= 32 * POST_NPL) {            // the group in registers, its weights asked for with it: one round trip behind the token's
+            float xv[POST_NPL], wv[POST_NPL], ss = 0.f;
+#pragma unroll
+            for (int k = 0; k < POST_NPL; k++) { const int i = lane + 32 * k; xv[k] = i < gs ? wf(e, (size_t) g * gs + i) : 0.f; wv[k] = i < gs ? w[g * gs + i] : 0.f; }
+#pragma unroll
+            for (int k = 0; k < POST_NPL; k++) ss = fmaf(xv[k], xv[k], ss);
+            ss = warp_sum(ss);
+            const float r = 1.0f / sqrtf(ss / (float) gs + eps);
+#pragma unroll
+            for (int k = 0; k < POST_NPL; k++) { const int i = lane + 32 * k; if (i < gs) { X[b + i] = xv[k]; Hn[b + i] = xv[k] * r * wv[k]; } }
+            continue;
+        }
+        for (int i = lane; i < gs; i += 32) X[b + i] = wf(e, (size_t) g * gs + i);
+        __syncwarp();
+        warp_group_norm(X + b, w + g * gs, gs, eps, Hn + b, lane);
+    }
 }
 
 // ---- end of a sub-layer, fused: X[t] += norm(Y[t]) * w_post, then (w_next != nullptr) Hn[t] = norm(X[t]) * w_next, the input
 // norm of the sub-layer that follows. Same groups for both; one block per row, one warp per group.
-constexpr int POST_NPL = 16;       // elements per lane k_post_norm_add keeps in registers (groups of up to 512)
-__global__ void k_post_norm_add(const float * __restrict__ Y, const float * __restrict__ w_post, float * __restrict__ X,
-                                const float * __restrict__ w_next, float * __restrict__ Hn, int n, int groups, float eps) {
+__global__ void k_post_norm_add(const float * Y, const float * __restrict__ w_post, float * X,
+                                const float * __restrict__ w_next, float * Hn, int n, int groups, float eps) {
     const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, gs = n / groups;
+    bool waited = false;
     for (int g = warp; g < groups; g += nw) {
         const size_t b = (size_t) row * n + (size_t) g * gs;
         const float * y = Y + b;
         float * x = X + b;
         if (gs <= 32 * POST_NPL) {
-            // the group lives in registers, and both weights are asked for with it: one round trip to memory instead of three dependent ones
-            // (a decode step is latency-bound: one token of 2048 entries in 8 groups 9.1 us while the weights came after the sums, now 4.0)
+            // the group lives in registers, and both weights are asked for ahead of the wait: one round trip to memory instead of three dependent ones
+            // (a decode step is latency-bound: one token of 2048 entries in 8 groups 9.1 us while the weights came after the sums, 4.0 with the group)
             float yv[POST_NPL], xv[POST_NPL], wp[POST_NPL], wn[POST_NPL];
             float ss = 0.f;
 #pragma unroll
             for (int k = 0; k < POST_NPL; k++) {
                 const int i = lane + 32 * k;
-                yv[k] = i < gs ? y[i] : 0.f; xv[k] = i < gs ? x[i] : 0.f;
                 wp[k] = i < gs ? w_post[g * gs + i] : 0.f; wn[k] = w_next && i < gs ? w_next[g * gs + i] : 0.f;
+            }
+            if (!waited) { pdl_enter(); waited = true; }
+#pragma unroll
+            for (int k = 0; k < POST_NPL; k++) {
+                const int i = lane + 32 * k;
+                yv[k] = i < gs ? y[i] : 0.f; xv[k] = i < gs ? x[i] : 0.f;
             }
 #pragma unroll
             for (int k = 0; k < POST_NPL; k++) ss = fmaf(yv[k], yv[k], ss);
@@ -116,6 +148,7 @@ __global__ void k_post_norm_add(const float * __restrict__ Y, const float * __re
             }
             continue;
         }
+        if (!waited) { pdl_enter(); waited = true; }
         float ss = 0.f;
         for (int i = lane; i < gs; i += 32) ss = fmaf(y[i], y[i], ss);
         ss = warp_sum(ss);
@@ -128,13 +161,15 @@ __global__ void k_post_norm_add(const float * __restrict__ Y, const float * __re
             for (int i = lane; i < gs; i += 32) Hn[b + i] = x[i] * r2 * w_next[g * gs + i];     // each lane re-reads what it wrote
         }
     }
+    if (!waited) pdl_enter();      // (a warp without a group)
 }
 
 // ---- RMS norm in `groups` equal consecutive parts; eps inside the root ----------------------------------------------
 // one block per row, one warp per group (round robin). rows != nullptr gathers input rows (the head's wanted rows).
 // accumulate == 0: Y[row] = norm(X[row]) * w;  accumulate == 1: Y[row] += norm(X[row]) * w  (the residual sum)
-__global__ void k_group_norm(const float * __restrict__ X, int ldx, const int32_t * __restrict__ rows, const float * __restrict__ w,
-                             int n, int groups, float eps, float * __restrict__ Y, int ldy, int accumulate) {
+__global__ void k_group_norm(const float * X, int ldx, const int32_t * rows, const float * __restrict__ w,
+                             int n, int groups, float eps, float * Y, int ldy, int accumulate) {
+    pdl_enter();
     const int row = blockIdx.x, src = rows ? rows[row] : row;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int gs = n / groups;
@@ -201,6 +236,7 @@ constexpr int GEMV_MAX_T = 4;
 // few rows to fill the SMs): the block's 8 warps share one row and add their sums in a fixed order
 template <typename WT, int RPW, int WPR = 1>
 __global__ void __launch_bounds__(256) k_gemv(const LinArgs a) {
+    pdl_enter();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n = (WPR > 1 ? (int) blockIdx.x : blockIdx.x * (blockDim.x >> 5) + warp) * RPW;      // RPW = 2: a (gate, up) pair per warp
     const int part = WPR > 1 ? warp : 0;
@@ -305,6 +341,7 @@ __global__ void __launch_bounds__(256) k_gemv(const LinArgs a) {
 constexpr int GX_ROWS = 8, GX_WARPS = 8;
 template <typename WT, int CH>
 __global__ void __launch_bounds__(GX_WARPS * 32) k_gemv_x(const LinArgs a) {
+    pdl_enter();
     constexpr int VEC = 16 / (int) sizeof(WT), RB = CH >= 4 ? 2 : CH == 2 ? 4 : 8;      // rows whose loads are in flight together
     __shared__ float sums[GX_WARPS][GX_ROWS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.x * GX_ROWS;
@@ -381,10 +418,120 @@ __global__ void __launch_bounds__(GX_WARPS * 32) k_gemv_x(const LinArgs a) {
     }
 }
 
+// one token's product inside a pass: a block has `rpb` consecutive rows, which its threads copy through a ring in shared memory (each its own 16-byte pieces: nobody else reads
+// them, so that no barrier stands between a copy and its use), and x in registers. The first GR_STAGES - 1 stages, up to 80 KB a block and 12 MB on the whole GPU, are asked for
+// before pdl_wait(): memory is busy while the kernels in front of this one normalise, rotate or drain, and what a layer's smaller products need is there when x is.
+// One block per SM with everything in flight: a gated unit of 16384 x 2048 in bf16 takes 12.4 us of a token's time and the 2048 x 8192 behind it 6.6 (5.5 and 5.1 TB/s, the second's
+// first 12 MB read under the first), where k_gemv_x started cold took 16.5 and 14.8; 2048 x 2048 2.5 us and not 7.3. A token of Matulorn (width 2048, four layers) 340 us before, 226 now.
+// TEAM warps cut a row's K among them (8 / TEAM rows at a time), CH: 16-byte pieces of a row per lane, K <= TEAM x 32 x VEC x CH.
+constexpr int GR_THREADS = 256, GR_PIECES = 24;                // pieces of a thread's in the ring
+__host__ __device__ constexpr int gr_rows(int ch) { return ch >= 4 ? 1 : 4 / ch; }                       // a team's rows per stage
+__host__ __device__ constexpr int gr_stages(int ch) { return GR_PIECES / (gr_rows(ch) * ch); }
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void * src, uint32_t bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void * src, uint32_t bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+template <typename WT, int TEAM, int CH>
+__global__ void __launch_bounds__(GR_THREADS, 2) k_gemv_ring(const LinArgs a, int rpb) {
+    constexpr int VEC = 16 / (int) sizeof(WT), RPT = gr_rows(CH), TEAMS = GR_THREADS / 32 / TEAM, RS = RPT * TEAMS, PIECES = RPT * CH, STAGES = gr_stages(CH);
+    extern __shared__ __align__(16) uint4 gr_ring[];           // [STAGES][PIECES][threads] | sums of [row][warp of its team]
+    float * sums = reinterpret_cast<float *>(gr_ring + GR_PIECES * GR_THREADS);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, team = warp / TEAM, tw = warp % TEAM;
+    const int n0 = blockIdx.x * rpb, rows = min(rpb, a.N - n0), n = (rows + RS - 1) / RS;
+    if (a.w_index) { pdl_wait(); pdl_launch_dependents(); }    // which matrix: an earlier kernel's choice
+    const int wi = a.w_index ? a.w_index[blockIdx.z] : (int) blockIdx.z;
+    if (a.n_w > 0 && wi >= a.n_w) return;                      // (only a choice can name none)
+    const WT * w = reinterpret_cast<const WT *>(a.W) + (size_t) wi * a.sW + (size_t) n0 * a.K;
+    const uint32_t ring = (uint32_t) __cvta_generic_to_shared(gr_ring + tid);
+    const auto copy = [&](int i, int slot) {
+        if (i < n) {
+#pragma unroll
+            for (int r = 0; r < RPT; r++) {
+                const int row = i * RS + r * TEAMS + team;
+#pragma unroll
+                for (int c = 0; c < CH; c++) {
+                    const int k = ((c * TEAM + tw) * 32 + lane) * VEC;
+                    const bool in = row < rows && k < a.K;     // otherwise zeros
+                    cp_async16(ring + (uint32_t) ((slot * PIECES + r * CH + c) * GR_THREADS * 16), in ? w + (size_t) row * a.K + k : w, in ? 16u : 0u);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; i++) copy(i, i);
+    if (!a.w_index) { pdl_wait(); pdl_launch_dependents(); }
+    const float * x = a.X + (size_t) (blockIdx.z / a.x_share) * a.sX;
+    float xv[CH][VEC];
+#pragma unroll
+    for (int c = 0; c < CH; c++) {
+        const int k = ((c * TEAM + tw) * 32 + lane) * VEC;
+#pragma unroll
+        for (int i = 0; i < VEC; i += 4) {
+            const float4 f = k < a.K ? *reinterpret_cast<const float4 *>(x + k + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            xv[c][i] = f.x; xv[c][i + 1] = f.y; xv[c][i + 2] = f.z; xv[c][i + 3] = f.w;
+        }
+    }
+    int slot = 0;
+    for (int i = 0; i < n; i++) {
+        asm volatile("cp.async.wait_group %0;" :: "n"(STAGES - 2) : "memory");
+        copy(i + STAGES - 1, slot == 0 ? STAGES - 1 : slot - 1);      // where the stage before was, whose numbers this thread has used
+        float acc[RPT];
+#pragma unroll
+        for (int r = 0; r < RPT; r++) {
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+            for (int c = 0; c < CH; c++) {
+                const uint4 raw = gr_ring[(slot * PIECES + r * CH + c) * GR_THREADS + tid];
+                const uint32_t uu[4] = { raw.x, raw.y, raw.z, raw.w };
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    if constexpr (sizeof(WT) == 2) {
+                        s0 = fmaf(__uint_as_float(uu[j] << 16), xv[c][2 * j], s0);
+                        s1 = fmaf(__uint_as_float(uu[j] & 0xffff0000u), xv[c][2 * j + 1], s1);
+                    } else if (j & 1) s1 = fmaf(__uint_as_float(uu[j]), xv[c][j], s1);
+                    else s0 = fmaf(__uint_as_float(uu[j]), xv[c][j], s0);
+                }
+            }
+            acc[r] = s0 + s1;
+        }
+        // RPT sums over 32 lanes: each halving sends half of the values to the other half of the lanes
+        int at = 0, off = 16;                                  // the row this lane ends with
+#pragma unroll
+        for (int half = RPT / 2; half >= 1; half >>= 1, off >>= 1) {
+            const bool up = lane & off;
+#pragma unroll
+            for (int j = 0; j < half; j++) {
+                const float keep = up ? acc[half + j] : acc[j], send = up ? acc[j] : acc[half + j];
+                acc[j] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+            }
+            at = 2 * at + (up ? 1 : 0);
+        }
+#pragma unroll
+        for (int o = 16 / RPT; o >= 1; o >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+        if (lane % (32 / RPT) == 0) sums[(i * RS + at * TEAMS + team) * TEAM + tw] = acc[0];
+        if (++slot == STAGES) slot = 0;
+    }
+    __syncthreads();
+    const float scale = a.x_scale ? a.x_scale[blockIdx.z] : 1.0f;
+    const auto total = [&](int r) {
+        float v = 0.f;
+#pragma unroll
+        for (int j = 0; j < TEAM; j++) v += sums[r * TEAM + j];
+        return v * scale + (a.bias ? a.bias[n0 + r] : 0.f);
+    };
+    float * y = a.Y + (size_t) blockIdx.z * a.sY;
+    if (a.glu) { for (int r = 2 * tid; r + 1 < rows; r += 2 * GR_THREADS) y[(n0 + r) >> 1] = gated_unit(a, total(r), total(r + 1)); }
+    else for (int r = tid; r < rows; r += GR_THREADS) y[n0 + r] = total(r);
+}
+
 // prompt portions in true float32 (and every shape the tensor-core kernel does not take): 64 x 64 x 16 tiles on the CUDA
 // cores, 256 threads with 4 x 4 outputs each
 template <typename WT>
 __global__ void __launch_bounds__(256) k_gemm_simt(const LinArgs a) {
+    pdl_enter();
     __shared__ __align__(16) float Xs[16][64 + 4];
     __shared__ __align__(16) float Ws[16][64 + 4];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -486,6 +633,7 @@ __global__ void __launch_bounds__(256) k_gemm_simt(const LinArgs a) {
 // Bound by the shared-memory reads. (Where k is 64 and more as well k_gemm_f32_umma takes its place: this one is left for shorter ones.)
 constexpr int SG_BM = 128, SG_BN = 128, SG_BK = 16;
 __global__ void __launch_bounds__(256, 2) k_gemm_simt_big(const LinArgs a) {
+    pdl_enter();
     __shared__ __align__(16) float Xs[SG_BK][SG_BM + 4];
     __shared__ __align__(16) float Ws[SG_BK][SG_BN + 4];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -588,6 +736,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 __global__ void __launch_bounds__(256) k_gemm_bf16_mma(const LinArgs a) {
+    pdl_enter();
     __shared__ __align__(16) __nv_bfloat16 As[2][MM_BM][MM_LD];
     __shared__ __align__(16) __nv_bfloat16 Bs[2][MM_BN][MM_LD];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -683,7 +832,8 @@ __global__ void __launch_bounds__(256) k_gemm_bf16_mma(const LinArgs a) {
 // Every wait on an mbarrier is bounded: on a timeout the CTA raises *err, skips what is left and still frees its tensor memory.
 // vec: rows and bases allow 16-byte loads (then K is a multiple of 8: LinArgs::vec of a bf16 product): eight entries a thread, over all rows of a batch entry at once.
 // 512 x 2048 5.6 us with an entry a thread, 4.0 now; 512 x 8192 13.6 and 6.2.
-__global__ void __launch_bounds__(256) k_to_bf16(const float * __restrict__ X, int ldx, int T, int K, long long sX, __nv_bfloat16 * __restrict__ Xb, long long sXb) {
+__global__ void __launch_bounds__(256) k_to_bf16(const float * X, int ldx, int T, int K, long long sX, __nv_bfloat16 * Xb, long long sXb) {
+    pdl_enter();
     const float * x = X + (size_t) blockIdx.y * sX;
     __nv_bfloat16 * o = Xb + (size_t) blockIdx.y * sXb;
     const int chunks = K / 8;
@@ -696,9 +846,6 @@ __global__ void __launch_bounds__(256) k_to_bf16(const float * __restrict__ X, i
 constexpr int UM_BM = 128, UM_BN = 256, UM_BK = 64, UM_STAGES = 4;
 constexpr int UM_A_BYTES = UM_BM * UM_BK * 2, UM_B_BYTES = UM_BN * UM_BK * 2, UM_STAGE_BYTES = UM_A_BYTES + UM_B_BYTES;
 constexpr int UM_SMEM = UM_STAGES * UM_STAGE_BYTES + 1024;                 // + alignment slack
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void * src, uint32_t bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap * map, int x, int y, int z, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
@@ -716,7 +863,8 @@ __device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity,
     return false;
 }
 // maps: X as bf16 [xbatch][T][K] (box 64 x 128), W [batch][N][K] (box 64 x 256)
-__global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const LinArgs a, int * err, int ksplit = 1, float * __restrict__ part = nullptr) {
+__global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const LinArgs a, int * err, int ksplit = 1, float * part = nullptr) {
+    pdl_enter();
     extern __shared__ uint8_t um_raw[];
     __shared__ __align__(8) uint64_t full[UM_STAGES], empty[UM_STAGES], done;
     __shared__ uint32_t tmem_base_s;
@@ -841,7 +989,8 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
 
 // Y[t][n] = bias[n] + the parts' sums, in order. NV entries a thread (four where N, ldy and the bases allow 16-byte accesses: 4 x 512 x 2048 7.9 -> 5.6 us)
 template <int NV>
-__global__ void __launch_bounds__(256) k_split_sum(const float * __restrict__ part, int ksplit, int T, int N, const float * __restrict__ bias, float * __restrict__ Y, int ldy) {
+__global__ void __launch_bounds__(256) k_split_sum(const float * part, int ksplit, int T, int N, const float * __restrict__ bias, float * Y, int ldy) {
+    pdl_enter();
     using V = typename std::conditional<NV == 4, float4, float>::type;
     const int t = blockIdx.y, n = (blockIdx.x * blockDim.x + threadIdx.x) * NV;
     if (n >= N) return;
@@ -871,7 +1020,8 @@ __global__ void __launch_bounds__(256) k_split_sum(const float * __restrict__ pa
 // ---- minGRU: S_t = (1 - z) S_(t-1) + z * cand, gates from the current token only ----------------------------------------
 // P[t] = [ z pre-activation | candidate pre-activation u | output-gate pre-activation ] (3 * width, biases included);
 // cand = u + 1/2 for u >= 0, sigmoid(u) below. A[t] = S_t * silu(gate). One thread per channel walks the portion in order.
-__global__ void k_mingru_scan(const float * __restrict__ P, int T, int width, float * __restrict__ state, float * __restrict__ A) {
+__global__ void k_mingru_scan(const float * P, int T, int width, float * state, float * A) {
+    pdl_enter();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= width) return;
     float s = state[c];
@@ -899,7 +1049,8 @@ __global__ void k_mingru_scan(const float * __restrict__ P, int T, int width, fl
 // The same for prompt portions: a block has 32 channels, its 16 warps compute gates and candidates of MG_TB tokens, one walks the tile (two shared-memory reads and an fma a
 // token), all of them write it. k_mingru_scan's thread per channel fills 16 SMs at width 2048 and has the exponentials in its chain: 512 tokens 165 us, here 27.
 constexpr int MG_TB = 64, MG_WARPS = 16;
-__global__ void __launch_bounds__(MG_WARPS * 32) k_mingru_tiles(const float * __restrict__ P, int T, int width, float * __restrict__ state, float * __restrict__ A) {
+__global__ void __launch_bounds__(MG_WARPS * 32) k_mingru_tiles(const float * P, int T, int width, float * state, float * A) {
+    pdl_enter();
     constexpr int PER = MG_TB / MG_WARPS;
     __shared__ float keep[MG_TB][32], add[MG_TB][32];          // 1 - z, then the state; z * cand
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane, ld = 3 * width;
@@ -952,9 +1103,13 @@ struct RopeArgs {
 };
 __device__ __forceinline__ int rope_lo(const RopeArgs & r, int i) { return r.adjacent ? 2 * i : i; }
 __device__ __forceinline__ int rope_hi(const RopeArgs & r, int i) { return r.adjacent ? 2 * i + 1 : i + r.dims / 2; }
-__device__ __forceinline__ void rope_pair(const RopeArgs & r, int pos, int i, float u, float v, float & ou, float & ov) {
+__device__ __forceinline__ void rope_angle(const RopeArgs & r, int pos, int i, float & c, float & s) {
     const float ang = (float) pos * r.freq[i];
-    const float c = cosf(ang) * r.mag, s = sinf(ang) * r.mag;
+    c = cosf(ang) * r.mag; s = sinf(ang) * r.mag;
+}
+__device__ __forceinline__ void rope_pair(const RopeArgs & r, int pos, int i, float u, float v, float & ou, float & ov) {
+    float c, s;
+    rope_angle(r, pos, i, c, s);
     ou = u * c - v * s;
     ov = v * c + u * s;
 }
@@ -967,17 +1122,36 @@ __device__ __forceinline__ void rope_pair(const RopeArgs & r, int pos, int i, fl
 // dkv_off: where the down-projection starts in a row of P (H (D + R) in the layout above; a design whose queries pass a
 // latent of their own keeps [ query latent | down-projection | ... ] there and has no rotated parts: R = 0).
 // qnorm != nullptr: the first q_rank entries of the row (the query latent) are RMS-normed in place with that weight by a warp of their own.
-__global__ void k_latent_prep(float * __restrict__ P, int ldp, int H, int D, int R, int rank, const float * __restrict__ cnorm, float eps,
-                              RopeArgs rope, const StepState * __restrict__ st, float * __restrict__ cache, float * __restrict__ QK, int dkv_off,
+// What a token's chain waits for stands behind pdl_wait(): positions, angles and weights come first (the step's header is written before the pass's first launch), and
+// the latent is read once (up to LAT_NPL entries a lane in registers; a loop over each of two passes took 8.5 us of a token's layer).
+constexpr int LAT_NPL = 16;
+__global__ void k_latent_prep(float * P, int ldp, int H, int D, int R, int rank, const float * __restrict__ cnorm, float eps,
+                              RopeArgs rope, const StepState * st, float * cache, float * QK, int dkv_off,
                               const float * __restrict__ qnorm, int q_rank) {
     const int t = blockIdx.x, pos = st->pos0 + t, bk = blockIdx.y, nblk = gridDim.y;      // grid (T, blocks): the rotated vectors are dealt over the blocks of a token
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     float * p = P + (size_t) t * ldp;
     const float * dkv = p + dkv_off;
-    if (qnorm && bk == 0 && warp == (nw > 1 ? 1 : 0)) warp_group_norm(p, qnorm, q_rank, eps, p, lane);
     float * row = cache + (size_t) pos * (rank + R);
     const int half = rope.dims / 2;
-    if (warp == 0 && bk == nblk - 1) {
+    const bool norms = warp == 0 && bk == nblk - 1, fits = rank <= 32 * LAT_NPL;
+    float cw[LAT_NPL], cs = 0.f, sn = 0.f;
+#pragma unroll
+    for (int k = 0; k < LAT_NPL; k++) cw[k] = norms && fits && lane + 32 * k < rank ? cnorm[lane + 32 * k] : 0.f;
+    if (lane < half) rope_angle(rope, pos, lane, cs, sn);
+    pdl_enter();
+    if (qnorm && bk == 0 && warp == (nw > 1 ? 1 : 0)) warp_group_norm(p, qnorm, q_rank, eps, p, lane);
+    if (norms && fits) {
+        float x[LAT_NPL], ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < LAT_NPL; k++) x[k] = lane + 32 * k < rank ? dkv[lane + 32 * k] : 0.f;
+#pragma unroll
+        for (int k = 0; k < LAT_NPL; k++) ss = fmaf(x[k], x[k], ss);
+        ss = warp_sum(ss);
+        const float r = 1.0f / sqrtf(ss / (float) rank + eps);
+#pragma unroll
+        for (int k = 0; k < LAT_NPL; k++) if (lane + 32 * k < rank) row[lane + 32 * k] = x[k] * r * cw[k];
+    } else if (norms) {
         float ss = 0.f;
         for (int i = lane; i < rank; i += 32) ss = fmaf(dkv[i], dkv[i], ss);
         ss = warp_sum(ss);
@@ -989,7 +1163,13 @@ __global__ void k_latent_prep(float * __restrict__ P, int ldp, int H, int D, int
         const float * src = v == H ? dkv + rank : p + (size_t) v * (D + R) + D;
         float * dst = v == H ? row + rank : QK + ((size_t) t * H + v) * (rank + R) + rank;
         for (int i = lane; i < R; i += 32) {
-            if (i < half) { const int lo = rope_lo(rope, i), hi = rope_hi(rope, i); float a, b; rope_pair(rope, pos, i, src[lo], src[hi], a, b); dst[lo] = a; dst[hi] = b; }
+            if (i < half) {
+                const int lo = rope_lo(rope, i), hi = rope_hi(rope, i);
+                if (i >= 32) rope_angle(rope, pos, i, cs, sn);
+                const float u = src[lo], w = src[hi];
+                dst[lo] = u * cs - w * sn; dst[hi] = w * cs + u * sn;
+                if (half > 32 && i + 32 >= half) rope_angle(rope, pos, lane, cs, sn);      // (for the next vector)
+            }
             if (i >= rope.dims) dst[i] = src[i];
         }
     }
@@ -1015,6 +1195,7 @@ struct LatAttnArgs {
 };
 constexpr int LAT_NQ_MAX = 16, LAT_RPT = 2;
 __global__ void __launch_bounds__(256) k_latent_attn(const LatAttnArgs a) {
+    pdl_enter();
     extern __shared__ float sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int W = a.rank + a.R, NQ = a.TQ * a.HQ;
@@ -1141,12 +1322,24 @@ __global__ void __launch_bounds__(256) k_latent_attn_staged(const LatAttnArgs a)
     {   // the slice's cached rows and the block's queries: every copy is issued before any is waited for
         const float * src = a.cache + (size_t) jb * W;
         const uint32_t dst = (uint32_t) __cvta_generic_to_shared(keys), qdst = (uint32_t) __cvta_generic_to_shared(q);
-        if (VEC) {
-            const int w4 = W >> 2;
-            for (int i = tid; i < nk * w4; i += 256) {
-                const int j = i / w4, e = (i - j * w4) << 2;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + (uint32_t) (j * WP + e) * 4u), "l"(src + (size_t) j * W + e) : "memory");
+        const int w4 = W >> 2, mine = max(0, min(nk, a.st->pos0 - jb));      // rows that earlier passes left come ahead of the wait
+        const auto rows = [&](int j0, int j1) {
+            if (VEC) {
+                for (int i = j0 * w4 + tid; i < j1 * w4; i += 256) {
+                    const int j = i / w4, e = (i - j * w4) << 2;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + (uint32_t) (j * WP + e) * 4u), "l"(src + (size_t) j * W + e) : "memory");
+                }
+            } else {
+                for (int i = j0 * W + tid; i < j1 * W; i += 256) {
+                    const int j = i / W, e = i - j * W;
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst + (uint32_t) (j * WP + e) * 4u), "l"(src + (size_t) j * W + e) : "memory");
+                }
             }
+        };
+        rows(0, mine);
+        pdl_enter();
+        rows(mine, nk);
+        if (VEC) {
             for (int i = tid; i < NQ * w4; i += 256) {
                 const int qi = i / w4, e = (i - qi * w4) << 2, tq = qi / a.HQ, h = h0 + qi % a.HQ;
                 if (tq < nt && h < a.H)
@@ -1154,10 +1347,6 @@ __global__ void __launch_bounds__(256) k_latent_attn_staged(const LatAttnArgs a)
                 else *reinterpret_cast<float4 *>(q + (size_t) qi * W + e) = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         } else {
-            for (int i = tid; i < nk * W; i += 256) {
-                const int j = i / W, e = i - j * W;
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst + (uint32_t) (j * WP + e) * 4u), "l"(src + (size_t) j * W + e) : "memory");
-            }
             for (int i = tid; i < NQ * W; i += 256) {
                 const int qi = i / W, e = i - qi * W, tq = qi / a.HQ, h = h0 + qi % a.HQ;
                 if (tq < nt && h < a.H)
@@ -1261,26 +1450,32 @@ __global__ void __launch_bounds__(256) k_latent_attn_staged(const LatAttnArgs a)
 }
 
 // merge of the key slices of one (token, head): weights exp(m_z - M) with M the largest maximum (the sink included)
+// Every slice's numbers are asked for before any is used: a thread's parts of the sums, and two slices' maxima a lane.
 __global__ void __launch_bounds__(256) k_latent_combine(const LatAttnArgs a) {       // grid (T, H, ceil(rank / 64)): 64 latent entries x 4 groups of slices
-    const int t = blockIdx.x, h = blockIdx.y;
+    pdl_enter();
+    const int t = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31;
     const size_t th = (size_t) t * a.H + h;
     const float * ml = a.ml + th * a.nsplit * 2;
-    const float snk = a.sink ? a.sink[h] : -INFINITY;
-    float M = snk;
-    for (int z = 0; z < a.nsplit; z++) M = fmaxf(M, ml[2 * z]);
-    float den = snk == -INFINITY ? 0.f : expf(snk - M);
-    for (int z = 0; z < a.nsplit; z++) if (ml[2 * z] != -INFINITY) den += ml[2 * z + 1] * expf(ml[2 * z] - M);
-    const float inv = den > 0.f ? 1.0f / den : 0.f;
     __shared__ float wz[64];            // nsplit <= 64
     __shared__ float red[4][64];
-    if (threadIdx.x < a.nsplit) wz[threadIdx.x] = ml[2 * threadIdx.x] != -INFINITY ? expf(ml[2 * threadIdx.x] - M) * inv : 0.f;
-    __syncthreads();
     const int r = blockIdx.z * 64 + (threadIdx.x & 63), g = threadIdx.x >> 6;
+    float pv[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) { const int z = g + 4 * k; pv[k] = z < a.nsplit && r < a.rank ? a.part[(th * a.nsplit + z) * a.rank + r] : 0.f; }
+    float m[2], l[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) { const int z = lane + 32 * k; m[k] = z < a.nsplit ? ml[2 * z] : -INFINITY; l[k] = z < a.nsplit ? ml[2 * z + 1] : 0.f; }
+    const float snk = a.sink ? a.sink[h] : -INFINITY, M = fmaxf(snk, warp_max(fmaxf(m[0], m[1])));
+    float e[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) e[k] = m[k] != -INFINITY ? expf(m[k] - M) : 0.f;
+    const float den = warp_sum(e[0] * l[0] + e[1] * l[1]) + (snk == -INFINITY ? 0.f : expf(snk - M));
+    const float inv = den > 0.f ? 1.0f / den : 0.f;
+    if (threadIdx.x < 32) { wz[lane] = e[0] * inv; wz[lane + 32] = e[1] * inv; }
+    __syncthreads();
     float acc = 0.f;
-    if (r < a.rank) {
-#pragma unroll 8
-        for (int z = g; z < a.nsplit; z += 4) acc = fmaf(a.part[(th * a.nsplit + z) * a.rank + r], wz[z], acc);     // empty slices wrote zeros
-    }
+#pragma unroll
+    for (int k = 0; k < 16; k++) acc = fmaf(pv[k], wz[g + 4 * k], acc);       // (slices without keys, and none, have weight 0)
     red[g][threadIdx.x & 63] = acc;
     __syncthreads();
     if (g == 0 && r < a.rank) a.OL[th * a.rank + r] = (red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x]);
@@ -1290,8 +1485,9 @@ __global__ void __launch_bounds__(256) k_latent_combine(const LatAttnArgs a) {  
 // weights stay 32-bit): per tile of TQ tokens, S = QK_tile (TQ H rows) x cached rows [jlo, jlo + nk)^T, then this kernel, then
 // OL_tile = S x cached latents. Row (t, h) of tile i = t / TQ sees key jlo_i + n, jlo_i = pos0 + i TQ - span + 1 (window > 0)
 // or 0; keys outside 0 <= p - j < window (or j < 0) get weight 0. One warp per row; the sink joins maximum and denominator.
-__global__ void k_latent_softmax_rows(float * __restrict__ S, int n_rows, int H, int TQ, int nk, int window, int span, const float * __restrict__ sink,
-                                      const StepState * __restrict__ st, float scale, int tile0) {
+__global__ void k_latent_softmax_rows(float * S, int n_rows, int H, int TQ, int nk, int window, int span, const float * __restrict__ sink,
+                                      const StepState * st, float scale, int tile0) {
+    pdl_enter();
     const int lane = threadIdx.x & 31, row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);      // row = (t - tile0 TQ) H + h
     if (row >= n_rows) return;
     const int tl = row / H, h = row % H, t = tile0 * TQ + tl, p = st->pos0 + t;
@@ -1333,6 +1529,7 @@ struct ConvArgs {
     const float * bias = nullptr;
 };
 __global__ void k_causal_conv(const ConvArgs a) {
+    pdl_enter();
     const int c = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y, z = blockIdx.z;
     if (c >= a.C) return;
     const float * X = a.X + (size_t) z * a.sX;
@@ -1356,6 +1553,7 @@ __global__ void k_causal_conv(const ConvArgs a) {
 }
 // afterwards: the history becomes the last taps - 1 inputs of (history ++ portion)
 __global__ void k_causal_conv_hist(const ConvArgs a) {
+    pdl_enter();
     const int c = blockIdx.x * blockDim.x + threadIdx.x, z = blockIdx.z;
     if (c >= a.C) return;
     const float * X = a.X + (size_t) z * a.sX;
@@ -1367,8 +1565,9 @@ __global__ void k_causal_conv_hist(const ConvArgs a) {
 }
 // Step 2, per token: q and k become unit vectors per head (x / sqrt(sum x^2 + 1e-6)), q is also scaled by D^(-1/2);
 // beta = sigmoid(beta logit); decay g = exp(-exp(A_log) * softplus(decay input + dt_bias)). BG[t] = [ beta: H | g: H ].
-__global__ void k_delta_gates(float * __restrict__ CV, int C, const float * __restrict__ P, int ldp, int H, int KH, int D, int V,
-                              const float * __restrict__ A_log, const float * __restrict__ dt_bias, float * __restrict__ BG) {
+__global__ void k_delta_gates(float * CV, int C, const float * P, int ldp, int H, int KH, int D, int V,
+                              const float * __restrict__ A_log, const float * __restrict__ dt_bias, float * BG) {
+    pdl_enter();
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     float * cv = CV + (size_t) t * C;
     for (int v = warp; v < 2 * KH; v += nw) {     // q heads, then k heads
@@ -1395,47 +1594,64 @@ __global__ void k_delta_gates(float * __restrict__ CV, int C, const float * __re
 // register tile (rows beyond D stay zero).
 constexpr int DSCAN_LANES = 8, DSCAN_COLS = 16, DSCAN_TT = 8;
 template <int DMAX>
-__global__ void __launch_bounds__(128) k_delta_scan(const float * __restrict__ CV, int C, const float * __restrict__ BG, int T, int H, int KH, int D, int V,
-                                                    float * __restrict__ S, float * __restrict__ O) {
-    constexpr int TT = DSCAN_TT, NJ = DMAX / 32, NL = TT * DMAX / 128;
-    __shared__ __align__(16) float ks[TT][DMAX], qs[TT][DMAX];
-    __shared__ float bg[TT][2], vs[TT][DSCAN_COLS], kq[TT];
+__global__ void __launch_bounds__(128) k_delta_scan(const float * CV, int C, const float * BG, int T, int H, int KH, int D, int V,
+                                                    float * S, float * O) {
+    constexpr int TT = DSCAN_TT, NJ = DMAX / 32;
+    __shared__ __align__(16) float ks2[2][TT][DMAX], qs2[2][TT][DMAX];      // a tile being walked, the next one on its way
+    __shared__ float bg2[2][TT][2], vs2[2][TT][DSCAN_COLS], kq[TT];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane & 7, cl = warp * 4 + (lane >> 3);
     const int h = blockIdx.x, col = blockIdx.y * DSCAN_COLS + cl, kh = h / (H / KH);
     const bool live = col < V;
     float * Sh = S + (size_t) h * D * V;
     float2 s[NJ][2];
 #pragma unroll
-    for (int j = 0; j < NJ; j++) {
+    for (int j = 0; j < NJ; j++) {                             // (an earlier pass left the state: it is there ahead of the wait)
         float x[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) { const int d = 32 * j + 4 * r + i; x[i] = (live && d < D) ? Sh[(size_t) d * V + col] : 0.f; }
         s[j][0] = make_float2(x[0], x[1]); s[j][1] = make_float2(x[2], x[3]);
     }
-    float kr[NL], qr[NL], vr = 0.f, br = 0.f;
-    const auto fetch = [&](int t0) {
+    pdl_enter();
+    const bool wide = D % 4 == 0 && C % 4 == 0;                // rows of q and k in 16-byte pieces
+    const auto fetch = [&](int t0, int buf) {
+        const float * q = CV + (size_t) kh * D, * k = CV + (size_t) (KH + kh) * D;
+        const uint32_t kd = (uint32_t) __cvta_generic_to_shared(&ks2[buf][0][0]), qd = (uint32_t) __cvta_generic_to_shared(&qs2[buf][0][0]);
+        if (wide) {
 #pragma unroll
-        for (int i = 0; i < NL; i++) {
-            const int idx = tid + 128 * i, t = t0 + idx / DMAX, d = idx % DMAX;
-            const float * cv = CV + (size_t) t * C;
-            const bool on = t < T && d < D;
-            qr[i] = on ? cv[(size_t) kh * D + d] : 0.f;
-            kr[i] = on ? cv[(size_t) (KH + kh) * D + d] : 0.f;
+            for (int i = 0; i < (TT * DMAX + 511) / 512; i++) {
+                const int at = 4 * (tid + 128 * i), t = t0 + at / DMAX, d = at % DMAX;
+                if (at >= TT * DMAX) break;
+                const bool on = t < T && d < D;
+                const size_t o = on ? (size_t) t * C + d : 0;
+                cp_async16(kd + at * 4u, k + o, on ? 16u : 0u);
+                cp_async16(qd + at * 4u, q + o, on ? 16u : 0u);
+            }
+        } else {
+            for (int i = 0; i < TT * DMAX / 128; i++) {
+                const int at = tid + 128 * i, t = t0 + at / DMAX, d = at % DMAX;
+                const bool on = t < T && d < D;
+                const size_t o = on ? (size_t) t * C + d : 0;
+                cp_async4(kd + at * 4u, k + o, on ? 4u : 0u);
+                cp_async4(qd + at * 4u, q + o, on ? 4u : 0u);
+            }
         }
         const int t = t0 + tid / DSCAN_COLS, c = blockIdx.y * DSCAN_COLS + tid % DSCAN_COLS;
-        vr = (t < T && c < V) ? CV[(size_t) t * C + (size_t) 2 * KH * D + (size_t) h * V + c] : 0.f;
-        if (tid < 2 * TT) br = t0 + (tid >> 1) < T ? BG[(size_t) (t0 + (tid >> 1)) * 2 * H + (tid & 1) * H + h] : 0.f;
+        const bool on = t < T && c < V;
+        cp_async4((uint32_t) __cvta_generic_to_shared(&vs2[buf][0][0]) + tid * 4u, on ? CV + (size_t) t * C + (size_t) 2 * KH * D + (size_t) h * V + c : CV, on ? 4u : 0u);
+        if (tid < 2 * TT) {
+            const bool in = t0 + (tid >> 1) < T;
+            cp_async4((uint32_t) __cvta_generic_to_shared(&bg2[buf][0][0]) + tid * 4u, in ? BG + (size_t) (t0 + (tid >> 1)) * 2 * H + (tid & 1) * H + h : BG, in ? 4u : 0u);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    fetch(0);
-    for (int t0 = 0; t0 < T; t0 += TT) {
+    fetch(0, 0);
+    for (int t0 = 0, buf = 0; t0 < T; t0 += TT, buf ^= 1) {
         const int nt = min(TT, T - t0);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < NL; i++) { const int idx = tid + 128 * i; ks[idx / DMAX][idx % DMAX] = kr[i]; qs[idx / DMAX][idx % DMAX] = qr[i]; }
-        vs[tid / DSCAN_COLS][tid % DSCAN_COLS] = vr;
-        if (tid < 2 * TT) bg[tid >> 1][tid & 1] = br;
-        __syncthreads();
-        if (t0 + TT < T) fetch(t0 + TT);
+        if (t0 + TT < T) fetch(t0 + TT, buf ^ 1);
+        const float (*ks)[DMAX] = ks2[buf], (*qs)[DMAX] = qs2[buf];
+        const float (*bg)[2] = bg2[buf], (*vs)[DSCAN_COLS] = vs2[buf];
         {   // k.q of the tile's tokens: 16 lanes each
             const int tt = tid >> 4;
             float x = 0.f;
@@ -1482,8 +1698,9 @@ __global__ void __launch_bounds__(128) k_delta_scan(const float * __restrict__ C
 }
 // Step 4: each head's read-out over its root mean square (eps inside the root), times a weight (w_stride 0: one [V] shared by
 // the heads; V: [H][V]), times the activated output gate (silu, or sigmoid when gate_sigmoid). One warp per (token, head).
-__global__ void k_delta_out(const float * __restrict__ O, const float * __restrict__ P, int ldp, int gate_off, int H, int V,
-                            const float * __restrict__ normw, int w_stride, int gate_sigmoid, float eps, float * __restrict__ A) {
+__global__ void k_delta_out(const float * O, const float * P, int ldp, int gate_off, int H, int V,
+                            const float * normw, int w_stride, int gate_sigmoid, float eps, float * A) {
+    pdl_enter();
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int h = blockIdx.y * nw + warp; h < H; h += gridDim.y * nw) {
         const float * o = O + (size_t) t * H * V + (size_t) h * V;
@@ -1508,8 +1725,9 @@ constexpr float GDELTA_DECAY_RATE = 0.60653065971263342f;      // e^(-1/2)
 // The decay logits are a low-rank product computed here: logit = w0 + W2 tanh(latent), latent = the last `lora` entries of the
 // row (lat_off), W2 [H D][lora] in the model's storage type; the block keeps tanh(latent) in shared memory.
 template <typename WT>
-__global__ void k_gdelta_prep(const float * __restrict__ P, int ldp, int k_off, int a_off, int lat_off, int lora, const WT * __restrict__ W2, const float * __restrict__ w0,
-                              int H, int D, float * __restrict__ G) {
+__global__ void k_gdelta_prep(const float * P, int ldp, int k_off, int a_off, int lat_off, int lora, const WT * __restrict__ W2, const float * __restrict__ w0,
+                              int H, int D, float * G) {
+    pdl_enter();
     extern __shared__ float sm_prep[];
     float * lat = sm_prep, * wl = sm_prep + lora;            // tanh(latent) [lora], decay logits of this head [D]
     const int t = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -1561,8 +1779,9 @@ __device__ __forceinline__ void cp_async4(float * dst, const float * src, bool r
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src), "r"(real ? 4u : 0u) : "memory");
 }
 template <int DMAX>
-__global__ void __launch_bounds__(512) k_gdelta_scan(const float * __restrict__ P, int ldp, int r_off, int k_off, int v_off, const float * __restrict__ G,
-                                                     int T, int H, int D, int V, float * __restrict__ S, float * __restrict__ O) {
+__global__ void __launch_bounds__(512) k_gdelta_scan(const float * P, int ldp, int r_off, int k_off, int v_off, const float * G,
+                                                     int T, int H, int D, int V, float * S, float * O) {
+    pdl_enter();
     // two buffers of GD_TT tokens: asynchronous copies fill one while the other is walked
     constexpr int TT = DMAX > 128 ? 2 : 4, DR = DMAX / GD_RG, ROW = GD_RG * (DR + GD_PAD);
     __shared__ __align__(16) float rs[2][TT][ROW], ks[2][TT][ROW], ws[2][TT][ROW], us[2][TT][ROW], bs[2][TT][ROW], vs[2][TT][128];
@@ -1651,6 +1870,7 @@ struct DiffAttnArgs {
 };
 template <int VPL>
 __global__ void __launch_bounds__(256) k_diff_attn(const DiffAttnArgs a) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int WPQ = 8 / a.TQ, qi = warp / WPQ, wq = warp % WPQ;
@@ -1683,7 +1903,7 @@ __global__ void __launch_bounds__(256) k_diff_attn(const DiffAttnArgs a) {
                 if (a.vec) {
 #pragma unroll 8
                     for (int e = 0; e < a.D; e += 4) {                // unrolled: the loads of several steps are in flight together
-                        const float4 ka = __ldg(reinterpret_cast<const float4 *>(k1 + e)), kb = __ldg(reinterpret_cast<const float4 *>(k2 + e));
+                        const float4 ka = *reinterpret_cast<const float4 *>(k1 + e), kb = *(reinterpret_cast<const float4 *>(k2 + e));
                         const float4 qa = *reinterpret_cast<const float4 *>(q1 + e), qb = *reinterpret_cast<const float4 *>(q2 + e);
                         x0 = fmaf(qa.x, ka.x, x0); x1 = fmaf(qa.y, ka.y, x1); x0 = fmaf(qa.z, ka.z, x0); x1 = fmaf(qa.w, ka.w, x1);
                         y0 = fmaf(qb.x, kb.x, y0); y1 = fmaf(qb.y, kb.y, y1); y0 = fmaf(qb.z, kb.z, y0); y1 = fmaf(qb.w, kb.w, y1);
@@ -1707,7 +1927,7 @@ __global__ void __launch_bounds__(256) k_diff_attn(const DiffAttnArgs a) {
 #pragma unroll
                 for (int i = 0; i < VPL; i++) {
                     const int vi = lane + 32 * i;
-                    const float v = vi < a.V ? __ldg(vrow + (size_t) kk * a.ldc + vi) : 0.f;
+                    const float v = vi < a.V ? *(vrow + (size_t) kk * a.ldc + vi) : 0.f;
                     acc1[i] = fmaf(w1, v, acc1[i]); acc2[i] = fmaf(w2, v, acc2[i]);
                 }
             }
@@ -1781,7 +2001,8 @@ __global__ void __launch_bounds__(256) k_diff_attn(const DiffAttnArgs a) {
 // k_diff_softmax_rows turns the pair of score rows into ONE row of weights P = softmax(S_1) - lambda softmax(S_2) (both maps
 // weigh the same values, so the difference can be taken on the weights), then O = P V_g, then k_diff_norm_out.
 // k_diff_q_layout: queries [T][H][2][D] -> Qr[g][m][Tpad][R][D] (rows of one group and map contiguous; rows past T zero)
-__global__ void k_diff_q_layout(const float * __restrict__ Q, int ldq, int T, int Tpad, int H, int G, int D, float * __restrict__ Qr) {
+__global__ void k_diff_q_layout(const float * Q, int ldq, int T, int Tpad, int H, int G, int D, float * Qr) {
+    pdl_enter();
     const int t = blockIdx.x, R = H / G, nq = H * 2 * D;
     for (int i = threadIdx.x; i < nq; i += blockDim.x) {
         const int h = i / (2 * D), m = (i / D) & 1, d = i % D, g = h / R, hq = h - g * R;
@@ -1790,8 +2011,9 @@ __global__ void k_diff_q_layout(const float * __restrict__ Q, int ldq, int T, in
 }
 // S holds, for a group of ng tiles starting at tile0, [g][m][ng TQ R rows][nk]; row (tile, token, head) sees key jlo + n with
 // jlo = pos0 + tile TQ - span + 1 (window > 0) or 0, as in k_latent_softmax_rows. The weights replace map 1's row.
-__global__ void k_diff_softmax_rows(float * __restrict__ S, int n_rows, int G, int R, int TQ, int nk, int window, int span,
-                                    const StepState * __restrict__ st, float scale, float lambda, int tile0, int T) {
+__global__ void k_diff_softmax_rows(float * S, int n_rows, int G, int R, int TQ, int nk, int window, int span,
+                                    const StepState * st, float scale, float lambda, int tile0, int T) {
+    pdl_enter();
     const int lane = threadIdx.x & 31, id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (id >= n_rows * G) return;
     const int g = id / n_rows, r = id - g * n_rows;
@@ -1811,7 +2033,8 @@ __global__ void k_diff_softmax_rows(float * __restrict__ S, int n_rows, int G, i
     for (int n = lane; n < nk; n += 32) s1[n] = (n >= n_lo && n <= n_hi) ? expf(s1[n] * scale - m1) * i1 - expf(s2[n] * scale - m2) * i2 : 0.f;
 }
 // Or[g][Tpad][R][V] -> A[t][h][V]: each head's vector over its root mean square (eps inside the root), times out_scale
-__global__ void k_diff_norm_out(const float * __restrict__ Or, int Tpad, int H, int G, int V, float eps, float out_scale, float * __restrict__ A) {
+__global__ void k_diff_norm_out(const float * Or, int Tpad, int H, int G, int V, float eps, float out_scale, float * A) {
+    pdl_enter();
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, R = H / G;
     for (int h = blockIdx.y * nw + warp; h < H; h += gridDim.y * nw) {
         const int g = h / R, hq = h - g * R;
@@ -1828,8 +2051,9 @@ __global__ void k_diff_norm_out(const float * __restrict__ Or, int Tpad, int H, 
 // End of one layer and start of the next in one pass over a row: X[t] += Ya[t] + Yb[t] (either may be absent), the new row also
 // goes to Xc (row stride ldc; the input of a product that follows) when given, then H1[t] = X^ w1 and H2[t] = X^ w2 with
 // X^ = X / sqrt(mean(X^2) + eps): both norms share the root mean square, the weights arrive as 1 + w. One block per row.
-__global__ void __launch_bounds__(256) k_add_norm2(float * __restrict__ X, const float * __restrict__ Ya, const float * __restrict__ Yb, float * __restrict__ Xc, int ldc,
-                                                   const float * __restrict__ w1, const float * __restrict__ w2, float * __restrict__ H1, float * __restrict__ H2, int n, float eps) {
+__global__ void __launch_bounds__(256) k_add_norm2(float * X, const float * Ya, const float * Yb, float * Xc, int ldc,
+                                                   const float * w1, const float * w2, float * H1, float * H2, int n, float eps) {
+    pdl_enter();
     __shared__ float red[8];
     const int row = blockIdx.x, tid = threadIdx.x;
     float * x = X + (size_t) row * n;
@@ -1863,8 +2087,9 @@ __global__ void __launch_bounds__(256) k_add_norm2(float * __restrict__ X, const
 // cluster through distributed shared memory, so that no block reads an entry of X another block rewrites.
 constexpr int CANON1_CTAS = 8;
 __global__ void __cluster_dims__(CANON1_CTAS, 1, 1) __launch_bounds__(256)
-k_add_norm2_canon1(float * __restrict__ X, const float * __restrict__ Ya, const float * __restrict__ Yb, const float * __restrict__ w1, const float * __restrict__ w2,
-                   const float * __restrict__ cw, float * __restrict__ hist, float * __restrict__ U, long long plane, int n, int taps, float eps) {
+k_add_norm2_canon1(float * X, const float * Ya, const float * Yb, const float * w1, const float * w2,
+                   const float * cw, float * hist, float * U, long long plane, int n, int taps, float eps) {
+    pdl_enter();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ float red[8];
@@ -1904,7 +2129,8 @@ k_add_norm2_canon1(float * __restrict__ X, const float * __restrict__ Ya, const 
 
 // embedding without a norm: X[t] = scale * embed[token[t]]; X0 (row stride ld0), when given, keeps the same row for later layers
 template <typename WT>
-__global__ void k_embed_plain(const WT * __restrict__ embed, const int32_t * __restrict__ tokens, int E, int n_vocab, float * __restrict__ X, float * __restrict__ X0, int ld0, float scale = 1.0f) {
+__global__ void k_embed_plain(const WT * __restrict__ embed, const int32_t * tokens, int E, int n_vocab, float * X, float * X0, int ld0, float scale = 1.0f) {
+    pdl_enter();
     const int t = blockIdx.x;
     int tok = tokens[t];
     tok = tok < 0 ? 0 : tok >= n_vocab ? n_vocab - 1 : tok;
@@ -1917,7 +2143,8 @@ __global__ void k_embed_plain(const WT * __restrict__ embed, const int32_t * __r
 
 // ---- polynomial activation with norms: y = a N(z) + b N(z^2) + c N(z^3) + e, powers element by element, N divides a row by its
 // root mean square (eps inside the root); coef = [a, b, c, e]. One block per row, in place, float32.
-__global__ void __launch_bounds__(256) k_polynorm(float * __restrict__ Z, int n, const float * __restrict__ coef, float eps) {
+__global__ void __launch_bounds__(256) k_polynorm(float * Z, int n, const float * __restrict__ coef, float eps) {
+    pdl_enter();
     __shared__ float red[3][8];
     float * z = Z + (size_t) blockIdx.x * n;
     const int tid = threadIdx.x;
@@ -1936,18 +2163,21 @@ __global__ void __launch_bounds__(256) k_polynorm(float * __restrict__ Z, int n,
 // ---- small element-wise steps ---------------------------------------------------------------------------------------------------
 // output gate: A[t][h][0..V) *= sigmoid(gate[t][h]) (one number per head), or with per_entry = 1 A[t][i] *= sigmoid(gate[t][i])
 // (one number per entry); gate rows of stride ldg. grid (T, slices of a row)
-__global__ void k_head_gate(float * __restrict__ A, const float * __restrict__ gate, int ldg, int H, int V, int per_entry) {
+__global__ void k_head_gate(float * A, const float * gate, int ldg, int H, int V, int per_entry) {
+    pdl_enter();
     const int t = blockIdx.x;
     for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < H * V; i += blockDim.x * gridDim.y) A[(size_t) t * H * V + i] *= sigmoidf_(gate[(size_t) t * ldg + (per_entry ? i : i / V)]);
 }
 // soft cap on the logits: x <- cap tanh(x / cap)
-__global__ void k_softcap(float * __restrict__ x, size_t n, float cap) {
+__global__ void k_softcap(float * x, size_t n, float cap) {
+    pdl_enter();
     const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = cap * tanhf(x[i] / cap);
 }
 
 // ---- arg-max of one row of logits (lowest index wins ties) -----------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_argmax_row(const float * __restrict__ x, int n, int32_t * __restrict__ out) {
+__global__ void __launch_bounds__(1024) k_argmax_row(const float * x, int n, int32_t * out) {
+    pdl_enter();
     __shared__ float bv[32];
     __shared__ int bi[32];
     float best = -INFINITY; int idx = 0x7fffffff;
@@ -1966,8 +2196,9 @@ __global__ void __launch_bounds__(1024) k_argmax_row(const float * __restrict__ 
 
 // the device-resident greedy loop's last kernel: arg-max of the token's logits becomes the next step's token at the next
 // position (header in device memory), and is appended to the list the host reads after the burst
-__global__ void __launch_bounds__(1024) k_argmax_advance(const float * __restrict__ x, int n, StepState * st, int32_t * token_slot,
-                                                         int32_t * __restrict__ out, int32_t * counter) {
+__global__ void __launch_bounds__(1024) k_argmax_advance(const float * x, int n, StepState * st, int32_t * token_slot,
+                                                         int32_t * out, int32_t * counter) {
+    pdl_enter();
     __shared__ float bv[32];
     __shared__ int bi[32];
     float best = -INFINITY; int idx = 0x7fffffff;

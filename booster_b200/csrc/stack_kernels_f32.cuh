@@ -78,7 +78,8 @@ __device__ __noinline__ uint2 f3_again(const float * X, int ldx, const float * W
     return make_uint2(x_off, w_off);
 }
 
-__global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a, int * err, int ksplit = 1, float * __restrict__ part = nullptr) {
+__global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a, int * err, int ksplit = 1, float * part = nullptr) {
+    pdl_enter();
     extern __shared__ uint8_t f3_raw[];
     __shared__ __align__(8) uint64_t full[2], done[2];
     __shared__ uint32_t tmem_base_s;

@@ -40,8 +40,9 @@ inline int hc_threads(int T, int E, int per_thread = 2, int most = 1024) {
 // embedding into all S streams, fused with the first sub-layer's read-in and norm:
 // XS[s][t] = embed[token[t]]; Hn[t] = u / sqrt(mean(u^2) + eps) * g with u = sum_s in[s] XS[s][t]
 template <typename WT>
-__global__ void __launch_bounds__(1024) k_hc_embed(const WT * __restrict__ embed, const int32_t * __restrict__ tokens, int E, int n_vocab, int S,
-                                                  float * __restrict__ XS, long long plane, HcW w, float g, float eps, float * __restrict__ Hn) {
+__global__ void __launch_bounds__(1024) k_hc_embed(const WT * __restrict__ embed, const int32_t * tokens, int E, int n_vocab, int S,
+                                                  float * XS, long long plane, HcW w, float g, float eps, float * Hn) {
+    pdl_enter();
     __shared__ float red[32];
     const int t = blockIdx.x, nt = blockDim.x;
     int tok = tokens[t];
@@ -78,6 +79,7 @@ struct HcJoinArgs {
 constexpr int HC_OWN = 2;              // read-in chunks a thread keeps in registers until the row's sum of squares is known
 template <int VEC>
 __global__ void __launch_bounds__(VEC == 4 ? 512 : 1024) k_hc_join(const HcJoinArgs a) {
+    pdl_enter();
     __shared__ float red[32];
     const int t = blockIdx.x, S = a.S, nt = blockDim.x, nchunk = a.E / VEC;
     const size_t row = (size_t) t * a.E;
@@ -171,6 +173,10 @@ __global__ void __launch_bounds__(256) k_gqa_prep(const GqaPrepArgs a) {
     float * row = a.cache + (size_t) pos * a.ldc;
     const int half = a.rope.dims / 2;
     const int nblk = gridDim.y, bk = blockIdx.y;
+    float cs[2], sn[2];                                        // angles of pairs lane and lane + 32, ahead of the wait (the step's header is written before the pass's first launch)
+#pragma unroll
+    for (int k = 0; k < 2; k++) if (lane + 32 * k < half) rope_angle(a.rope, pos, lane + 32 * k, cs[k], sn[k]);
+    pdl_enter();
     for (int vec = bk * 8 + warp; vec < a.H + a.G; vec += 8 * nblk) {
         const bool is_q = vec < a.H;
         const float * src = is_q ? q + (size_t) vec * a.D : k + (size_t) (vec - a.H) * a.D;
@@ -183,12 +189,12 @@ __global__ void __launch_bounds__(256) k_gqa_prep(const GqaPrepArgs a) {
             ss = warp_sum(ss);
             r = 1.0f / sqrtf(ss / (float) a.D + a.eps);
         }
-        for (int i = lane; i < half; i += 32) {
+        for (int i = lane, k = 0; i < half; i += 32, k++) {
             const int lo = rope_lo(a.rope, i), hi = rope_hi(a.rope, i);
             const float x = src[lo] * r * (w ? w[lo] : 1.0f), y = src[hi] * r * (w ? w[hi] : 1.0f);
-            float ox, oy;
-            rope_pair(a.rope, pos, i, x, y, ox, oy);
-            dst[lo] = ox; dst[hi] = oy;
+            float c = k ? cs[1] : cs[0], s = k ? sn[1] : sn[0];
+            if (k > 1) rope_angle(a.rope, pos, i, c, s);
+            dst[lo] = x * c - y * s; dst[hi] = y * c + x * s;
         }
         for (int i = a.rope.dims + lane; i < a.D; i += 32) dst[i] = src[i] * r * (w ? w[i] : 1.0f);
     }
@@ -202,7 +208,8 @@ __global__ void __launch_bounds__(256) k_gqa_prep(const GqaPrepArgs a) {
 
 // means of whole blocks of P cached rows: pool[b] = (1 / P) sum_(j < P) cache[b P + j], for every block whose last position
 // b P + P - 1 lies in this step (its rows are all in the cache then). grid (n_tokens / P + 1, slices of the row).
-__global__ void k_pool_rows(const float * __restrict__ cache, int ldc, float * __restrict__ pool, int P, const StepState * __restrict__ st) {
+__global__ void k_pool_rows(const float * cache, int ldc, float * pool, int P, const StepState * st) {
+    pdl_enter();
     const int b = st->pos0 / P + blockIdx.x;
     if ((long long) (b + 1) * P > (long long) st->pos0 + st->n_tokens) return;
     const float * src = cache + (size_t) b * P * ldc;
@@ -252,6 +259,7 @@ struct GqaAttnArgs {
 };
 template <int VPL>
 __global__ void __launch_bounds__(256) k_gqa_attn(const GqaAttnArgs a) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int WPQ = 8 / a.TQ, qi = warp / WPQ, wq = warp % WPQ;
@@ -295,7 +303,7 @@ __global__ void __launch_bounds__(256) k_gqa_attn(const GqaAttnArgs a) {
                 if (a.vec) {
 #pragma unroll 8
                     for (int e = 0; e < a.D; e += 4) {
-                        const float4 ka = __ldg(reinterpret_cast<const float4 *>(k1 + e));
+                        const float4 ka = *reinterpret_cast<const float4 *>(k1 + e);
                         const float4 qa = *reinterpret_cast<const float4 *>(q1 + e);
                         x0 = fmaf(qa.x, ka.x, x0); x1 = fmaf(qa.y, ka.y, x1); x0 = fmaf(qa.z, ka.z, x0); x1 = fmaf(qa.w, ka.w, x1);
                     }
@@ -319,7 +327,7 @@ __global__ void __launch_bounds__(256) k_gqa_attn(const GqaAttnArgs a) {
 #pragma unroll
                 for (int i = 0; i < VPL; i++) {
                     const int vi = lane + 32 * i;
-                    const float v = vi < a.V ? __ldg(vrow + vi) : 0.f;
+                    const float v = vi < a.V ? *(vrow + vi) : 0.f;
                     acc[i] = fmaf(wk, v, acc[i]);
                 }
             }
@@ -397,6 +405,30 @@ __global__ void __launch_bounds__(256) k_gqa_attn_group(const GqaAttnArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = blockIdx.x, R = a.H / a.G, ngrp = (R + RT - 1) / RT;
     const int g = blockIdx.y / ngrp, h0 = g * R + (blockIdx.y - g * ngrp) * RT, nh = min(RT, (g + 1) * R - h0), V = a.V, MG = 2 + V;
     const int pos0 = a.st->pos0, p = pos0 + t;
+    const int jlo = gqa_first_token(a.mask, p), nb = gqa_blocks_seen(a.mask, p), ntot = nb + p - jlo + 1, nstrip = (ntot + KS - 1) / KS;
+    const int ns = min((int) gridDim.z, (nstrip + 7) / 8), z = blockIdx.z;
+    if (z >= ns) { pdl_enter(); return; }
+    const float * tokens = a.cache + ((long long) jlo - nb) * a.ldc;
+    const size_t koff = (size_t) g * a.D, voff = (size_t) a.G * a.D + (size_t) g * V;
+    float4 k[KS][CH], v[KS][CH];
+    const auto rows = [&](int n0) {
+#pragma unroll
+        for (int i = 0; i < KS; i++) {
+            const int n = min(n0 + i, ntot - 1);               // past the end: the last row again, with weight 0
+            const float * row = n < nb ? a.pool + (size_t) n * a.ldc : tokens + (long long) n * a.ldc;
+#pragma unroll
+            for (int c = 0; c < CH; c++) {
+                const int e = 4 * lane + 128 * c;
+                k[i][c] = e < a.D ? *reinterpret_cast<const float4 *>(row + koff + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[i][c] = e < V ? *reinterpret_cast<const float4 *>(row + voff + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+    };
+    // a warp's first rows come ahead of the wait where all of them are tokens of earlier passes (this one's, and the means it moves on, are written by the kernels in front)
+    const int s0 = z * 8 + warp;
+    const bool early = nb == 0 && s0 < nstrip && jlo + s0 * KS + KS - 1 < pos0;
+    if (early) rows(s0 * KS);
+    pdl_enter();
     float4 q[RT][CH];
 #pragma unroll
     for (int h = 0; h < RT; h++)
@@ -405,34 +437,18 @@ __global__ void __launch_bounds__(256) k_gqa_attn_group(const GqaAttnArgs a) {
             const int e = 4 * lane + 128 * c;
             q[h][c] = h < nh && e < a.D ? *reinterpret_cast<const float4 *>(a.Q + (size_t) t * a.ldq + (size_t) (h0 + h) * a.D + e) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-    const int jlo = gqa_first_token(a.mask, p), nb = gqa_blocks_seen(a.mask, p), ntot = nb + p - jlo + 1, nstrip = (ntot + KS - 1) / KS;
-    const int ns = min((int) gridDim.z, (nstrip + 7) / 8), z = blockIdx.z;
-    if (z >= ns) return;
     const int hh = lane / REP / KS, kk = lane / REP % KS;      // this lane's (head, key) of a strip
     const bool mine = hh < nh;
     const float r1 = a.r1 && mine ? a.r1[h0 + hh] : 0.f, r2 = a.r1 && mine ? a.r2[h0 + hh] : 0.f;
-    const float * tokens = a.cache + ((long long) jlo - nb) * a.ldc;
-    const size_t koff = (size_t) g * a.D, voff = (size_t) a.G * a.D + (size_t) g * V;
     float4 acc[RT][CH];
     float m = -INFINITY, l = 0.f;
 #pragma unroll
     for (int h = 0; h < RT; h++)
 #pragma unroll
         for (int c = 0; c < CH; c++) acc[h][c] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = z * 8 + warp; s < nstrip; s += 8 * ns) {
+    for (int s = s0; s < nstrip; s += 8 * ns) {
         const int n0 = s * KS;
-        float4 k[KS][CH], v[KS][CH];
-#pragma unroll
-        for (int i = 0; i < KS; i++) {
-            const int n = min(n0 + i, ntot - 1);               // past the end: the last row again, with weight 0
-            const float * row = n < nb ? a.pool + (size_t) n * a.ldc : tokens + (long long) n * a.ldc;
-#pragma unroll
-            for (int c = 0; c < CH; c++) {
-                const int e = 4 * lane + 128 * c;
-                k[i][c] = e < a.D ? __ldg(reinterpret_cast<const float4 *>(row + koff + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                v[i][c] = e < V ? __ldg(reinterpret_cast<const float4 *>(row + voff + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-        }
+        if (s != s0 || !early) rows(n0);
         float d[NV];
 #pragma unroll
         for (int h = 0; h < RT; h++)
@@ -570,9 +586,10 @@ __global__ void __launch_bounds__(256) k_gqa_attn_group(const GqaAttnArgs a) {
 // than the sequence so far; the cache has a zero margin in front) or 0 when the products start at position 0 (span == 0).
 // S holds [g][n_rows = ng TQ R][npc + nk] for a group of ng tiles starting at tile0. One warp per row. Without a mask (span == 0) columns
 // past the row's tile are neither computed nor read: weights are written up to the tile's last position, rounded up to 4.
-__global__ void k_gqa_softmax_rows(float * __restrict__ S, int n_rows, int G, int R, int TQ, int npc, int nk, int span, GqaMask mask, GqaScore sc,
+__global__ void k_gqa_softmax_rows(float * S, int n_rows, int G, int R, int TQ, int npc, int nk, int span, GqaMask mask, GqaScore sc,
                                    const float * __restrict__ r1v, const float * __restrict__ r2v, const float * __restrict__ sink,
-                                   const StepState * __restrict__ st, int tile0, int T) {
+                                   const StepState * st, int tile0, int T) {
+    pdl_enter();
     const int lane = threadIdx.x & 31, id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (id >= n_rows * G) return;
     const int g = id / n_rows, r = id - g * n_rows, h = g * R + r % R;

@@ -18,8 +18,9 @@ __device__ __forceinline__ float dytf_(float x, const DytW & n, int i) { return 
 // embedding under that norm: X[t] = dyt_e(embed[token[t]]) (also kept as plane 0 of the depth history when given),
 // Hn[t] = dyt_1(X[t]) for the first layer
 template <typename WT>
-__global__ void k_embed_dyt(const WT * __restrict__ embed, const int32_t * __restrict__ tokens, int E, int n_vocab, DytW ne, DytW n1,
-                            float * __restrict__ X, float * __restrict__ keep0, float * __restrict__ Hn) {
+__global__ void k_embed_dyt(const WT * __restrict__ embed, const int32_t * tokens, int E, int n_vocab, DytW ne, DytW n1,
+                            float * X, float * keep0, float * Hn) {
+    pdl_enter();
     const int t = blockIdx.x;
     int tok = tokens[t];
     tok = tok < 0 ? 0 : tok >= n_vocab ? n_vocab - 1 : tok;
@@ -31,7 +32,8 @@ __global__ void k_embed_dyt(const WT * __restrict__ embed, const int32_t * __res
     }
 }
 // the head's input: Y[r] = dyt(X[rows[r]]) on the wanted rows
-__global__ void k_dyt_rows(const float * __restrict__ X, int ldx, const int32_t * __restrict__ rows, DytW n, int E, float * __restrict__ Y, int ldy) {
+__global__ void k_dyt_rows(const float * X, int ldx, const int32_t * rows, DytW n, int E, float * Y, int ldy) {
+    pdl_enter();
     const int r = blockIdx.x, src = rows ? rows[r] : r;
     for (int i = threadIdx.x; i < E; i += blockDim.x) Y[(size_t) r * ldy + i] = dytf_(X[(size_t) src * ldx + i], n, i);
 }
@@ -56,6 +58,7 @@ struct JoinArgs {
     const float * nw; const float * nb; float alpha; float * Hn;                            // nw != nullptr: the next norm
 };
 __global__ void __launch_bounds__(256) k_join(const JoinArgs a) {
+    pdl_enter();
     __shared__ float red[2][8];
     const int t = blockIdx.x, tid = threadIdx.x;
     const size_t row = (size_t) t * a.E;
@@ -123,6 +126,7 @@ template <int NV> __device__ __forceinline__ void block_sums(float (&v)[NV], flo
 }
 template <int VEC>
 __global__ void __launch_bounds__(1024) k_post_join(const PostJoinArgs a) {
+    pdl_enter();
     __shared__ float red[2][32];
     const int t = blockIdx.x, nt = blockDim.x, nchunk = a.E / VEC;
     const size_t row = (size_t) t * a.E;
@@ -222,7 +226,8 @@ __global__ void __launch_bounds__(1024) k_post_join(const PostJoinArgs a) {
 // P[t] = [ q: H x D | k: H x D | v: H x V | output-gate pre-activation: H x V ].
 // Step 1, per token, in place: the first rope.dims entries of every q and k head are rotated by the token's position
 // ('rotate half' pairs), then k is scaled by k_scale (D^(-1/2)). grid (T, ceil(2 H / warps per block)): a warp per head.
-__global__ void k_retention_prep(float * __restrict__ P, int ldp, int q_off, int k_off, int H, int D, RopeArgs rope, float k_scale, const StepState * __restrict__ st) {
+__global__ void k_retention_prep(float * P, int ldp, int q_off, int k_off, int H, int D, RopeArgs rope, float k_scale, const StepState * st) {
+    pdl_enter();
     const int t = blockIdx.x, pos = st->pos0 + t;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, half = rope.dims / 2;
     for (int v = blockIdx.y * nw + warp; v < 2 * H; v += gridDim.y * nw) {
@@ -244,8 +249,9 @@ __global__ void k_retention_prep(float * __restrict__ P, int ldp, int q_off, int
 // the root) and multiplied by plain weights; q is also multiplied by the position's temperature
 // 1 + coef ln(floor((p + 1) / every) + 1); every value head is divided by its own root mean square (no weight). Queries go to
 // Q[t] (H x D), keys and values to the cache row of the position: [ k: G x D | v: G x V ]. One block per token.
-__global__ void __launch_bounds__(256) k_sigattn_prep(const float * __restrict__ P, int ldp, int H, int G, int D, int V, const float * __restrict__ qw, const float * __restrict__ kw,
-                                                      float eps, float t_coef, int t_every, const StepState * __restrict__ st, float * __restrict__ Q, float * __restrict__ cache) {
+__global__ void __launch_bounds__(256) k_sigattn_prep(const float * P, int ldp, int H, int G, int D, int V, const float * qw, const float * kw,
+                                                      float eps, float t_coef, int t_every, const StepState * st, float * Q, float * cache) {
+    pdl_enter();
     __shared__ float red[2][8];
     const int t = blockIdx.x, pos = st->pos0 + t, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nq = H * D, nk = G * D;
@@ -291,6 +297,7 @@ struct SigAttnArgs {
 };
 template <int VPL>
 __global__ void __launch_bounds__(256) k_sig_attn(const SigAttnArgs a) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int WPQ = 8 / a.TQ, qi = warp / WPQ, wq = warp % WPQ;
@@ -327,7 +334,7 @@ __global__ void __launch_bounds__(256) k_sig_attn(const SigAttnArgs a) {
                 if (a.vec) {
 #pragma unroll 8
                     for (int e = 0; e < a.D; e += 4) {
-                        const float4 ka = __ldg(reinterpret_cast<const float4 *>(k1 + e));
+                        const float4 ka = *reinterpret_cast<const float4 *>(k1 + e);
                         const float4 qa = *reinterpret_cast<const float4 *>(q1 + e);
                         x0 = fmaf(qa.x, ka.x, x0); x1 = fmaf(qa.y, ka.y, x1); x0 = fmaf(qa.z, ka.z, x0); x1 = fmaf(qa.w, ka.w, x1);
                     }
@@ -343,7 +350,7 @@ __global__ void __launch_bounds__(256) k_sig_attn(const SigAttnArgs a) {
 #pragma unroll
                 for (int i = 0; i < VPL; i++) {
                     const int vi = lane + 32 * i;
-                    const float v = vi < a.V ? __ldg(vrow + (size_t) kk * a.ldc + vi) : 0.f;
+                    const float v = vi < a.V ? *(vrow + (size_t) kk * a.ldc + vi) : 0.f;
                     acc[i] = fmaf(wk, v, acc[i]);
                 }
             }
@@ -384,7 +391,8 @@ __global__ void __launch_bounds__(256) k_sig_attn(const SigAttnArgs a) {
 // family: per tile of TQ tokens and key/value head g, S = Q_g K_g^T (rows: the tile's tokens x the R = H / G query heads of the
 // group), k_sig_weight_rows turns scores into weights, then O = W V_g.
 // queries [T][H][D] -> Qr[g][Tpad][R][D] (rows past T are zero)
-__global__ void k_group_q_layout(const float * __restrict__ Q, int ldq, int T, int Tpad, int H, int G, int D, float * __restrict__ Qr) {
+__global__ void k_group_q_layout(const float * Q, int ldq, int T, int Tpad, int H, int G, int D, float * Qr) {
+    pdl_enter();
     const int t = blockIdx.x, R = H / G, nq = H * D;
     for (int i = threadIdx.x; i < nq; i += blockDim.x) {
         const int h = i / D, d = i - h * D, g = h / R, hq = h - g * R;
@@ -393,8 +401,9 @@ __global__ void k_group_q_layout(const float * __restrict__ Q, int ldq, int T, i
 }
 // S holds [g][n_rows = ng TQ R][nk] for a group of ng tiles starting at tile0; column n is key n (no window: the products
 // start at position 0). One warp per row.
-__global__ void k_sig_weight_rows(float * __restrict__ S, int n_rows, int G, int R, int TQ, int nk, const StepState * __restrict__ st, float scale,
-                                  const float * __restrict__ slope, const float * __restrict__ pb, int tile0, int T) {
+__global__ void k_sig_weight_rows(float * S, int n_rows, int G, int R, int TQ, int nk, const StepState * st, float scale,
+                                  const float * slope, const float * pb, int tile0, int T) {
+    pdl_enter();
     const int lane = threadIdx.x & 31, id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (id >= n_rows * G) return;
     const int g = id / n_rows, r = id - g * n_rows, h = g * R + r % R;
@@ -405,7 +414,8 @@ __global__ void k_sig_weight_rows(float * __restrict__ S, int n_rows, int G, int
 }
 // Or[g][Tpad][R][V] -> A[t][h][V], times sigmoid(gate[t][h]) when a gate is given (one number per head, or per_entry = 1: one per entry of
 // A[t]; rows of stride ldg)
-__global__ void k_group_o_layout(const float * __restrict__ Or, int Tpad, int H, int G, int V, float * __restrict__ A, const float * __restrict__ gate = nullptr, int ldg = 0, int per_entry = 0) {
+__global__ void k_group_o_layout(const float * Or, int Tpad, int H, int G, int V, float * A, const float * gate = nullptr, int ldg = 0, int per_entry = 0) {
+    pdl_enter();
     const int t = blockIdx.x, R = H / G;
     for (int i = threadIdx.x; i < H * V; i += blockDim.x) {
         const int h = i / V, d = i - h * V, g = h / R, hq = h - g * R;
@@ -448,15 +458,24 @@ __global__ void __launch_bounds__(256) k_moe_route(const RouteArgs a) {
     const int wpr = a.wpr, kw = warp % wpr;
     const int rows = a.n + (a.w_sg ? 1 : 0), e = blockIdx.y * (8 / wpr) + warp / wpr;
     float * z = a.z + (size_t) t * (a.n + 1);
+    constexpr int AHEAD = 4;                                // a row's pieces that a lane asks for ahead of the wait
+    const float * w = e < a.n ? a.Wr + (size_t) e * a.E : a.w_sg;
+    const bool wide = e < rows && (a.E & 3) == 0 && (a.ld & 3) == 0 && (((uintptr_t) w | (uintptr_t) h) & 15) == 0;
+    float4 wv[AHEAD];
+#pragma unroll
+    for (int j = 0; j < AHEAD; j++) { const int i = ((j * wpr + kw) * 32 + lane) * 4; wv[j] = wide && i < a.E ? *reinterpret_cast<const float4 *>(w + i) : make_float4(0.f, 0.f, 0.f, 0.f); }
+    pdl_enter();
     if (e < rows) {
-        const float * w = e < a.n ? a.Wr + (size_t) e * a.E : a.w_sg;
         float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f, acc3 = 0.f;
-        if ((a.E & 3) == 0 && (a.ld & 3) == 0 && (((uintptr_t) w | (uintptr_t) h) & 15) == 0) {
+        const auto add = [&](int i, const float4 & y) {
+            const float4 x = *reinterpret_cast<const float4 *>(h + i);
+            acc0 = fmaf(x.x, y.x, acc0); acc1 = fmaf(x.y, y.y, acc1); acc2 = fmaf(x.z, y.z, acc2); acc3 = fmaf(x.w, y.w, acc3);
+        };
+        if (wide) {
+#pragma unroll
+            for (int j = 0; j < AHEAD; j++) { const int i = ((j * wpr + kw) * 32 + lane) * 4; if (i < a.E) add(i, wv[j]); }
 #pragma unroll 4
-            for (int i = (kw * 32 + lane) * 4; i < a.E; i += 128 * wpr) {
-                const float4 x = *reinterpret_cast<const float4 *>(h + i), y = __ldg(reinterpret_cast<const float4 *>(w + i));
-                acc0 = fmaf(x.x, y.x, acc0); acc1 = fmaf(x.y, y.y, acc1); acc2 = fmaf(x.z, y.z, acc2); acc3 = fmaf(x.w, y.w, acc3);
-            }
+            for (int i = ((AHEAD * wpr + kw) * 32 + lane) * 4; i < a.E; i += 128 * wpr) add(i, *reinterpret_cast<const float4 *>(w + i));
         } else {
             for (int i = kw * 32 + lane; i < a.E; i += 32 * wpr) acc0 = fmaf(w[i], h[i], acc0);
         }
@@ -547,8 +566,9 @@ __global__ void __launch_bounds__(256) k_moe_route(const RouteArgs a) {
 // 1024 threads: `tpe` threads per expert (a power of two) each count one contiguous part of the slots, a block-wide prefix sum
 // over (expert, part) gives every thread its first row, a second walk places the slots. Dynamic shared memory: the slots'
 // experts when they fit (in_smem), then n tpe counters.
-__global__ void __launch_bounds__(1024) k_moe_sort(const int32_t * __restrict__ sel, int n_slots, int top, int n, int tpe, int in_smem,
-                                                   int32_t * __restrict__ seg, int32_t * __restrict__ slot_of, int32_t * __restrict__ src_row) {
+__global__ void __launch_bounds__(1024) k_moe_sort(const int32_t * sel, int n_slots, int top, int n, int tpe, int in_smem,
+                                                   int32_t * seg, int32_t * slot_of, int32_t * src_row) {
+    pdl_enter();
     extern __shared__ int ssm[];
     __shared__ int wsum[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -592,7 +612,8 @@ __global__ void __launch_bounds__(1024) k_moe_sort(const int32_t * __restrict__ 
     }
 }
 // Y[r] = X[src_row[r]]
-__global__ void k_gather_rows(const float * __restrict__ X, int ldx, const int32_t * __restrict__ src_row, int E, float * __restrict__ Y) {
+__global__ void k_gather_rows(const float * X, int ldx, const int32_t * src_row, int E, float * Y) {
+    pdl_enter();
     const int r = blockIdx.x;
     const float * x = X + (size_t) src_row[r] * ldx;
     if ((E & 3) == 0 && (ldx & 3) == 0) {
@@ -604,7 +625,8 @@ __global__ void k_gather_rows(const float * __restrict__ X, int ldx, const int32
 
 // Y[slot_of[s]] = wt[s] X[s / top]: every (token, choice) slot's input row, weighted by the choice's score, at the row the sort
 // gave the slot (an expert that runs on the weighted input)
-__global__ void k_spread_rows(const float * __restrict__ X, int ldx, const int32_t * __restrict__ slot_of, const float * __restrict__ wt, int top, int E, float * __restrict__ Y) {
+__global__ void k_spread_rows(const float * X, int ldx, const int32_t * slot_of, const float * wt, int top, int E, float * Y) {
+    pdl_enter();
     const int s = blockIdx.x;
     const float * x = X + (size_t) (s / top) * ldx;
     float * y = Y + (size_t) slot_of[s] * E;

@@ -43,7 +43,8 @@ __device__ __forceinline__ void outer_ab(const OuterScan & s, int t, int h, floa
     else { a = s.ab[(size_t) t * s.ld_ab + h]; b = s.ab[(size_t) t * s.ld_ab + s.H + h]; }
 }
 // the table of a and b from step sizes, for portions of several tokens: AB[t] = [ a: H | b: H ]
-__global__ void k_step_table(const float * __restrict__ raw, int ldr, const float * __restrict__ dt_bias, const float * __restrict__ A_log, int H, float * __restrict__ AB, int ld_ab) {
+__global__ void k_step_table(const float * raw, int ldr, const float * __restrict__ dt_bias, const float * __restrict__ A_log, int H, float * AB, int ld_ab) {
+    pdl_enter();
     const int t = blockIdx.x;
     for (int h = threadIdx.x; h < H; h += blockDim.x) {
         const float dt = step_size(raw + (size_t) t * ldr, dt_bias, h);
@@ -58,6 +59,7 @@ __global__ void k_step_table(const float * __restrict__ raw, int ldr, const floa
 // four lanes' reads fall into different banks. A head's columns are spread over gridDim.y blocks.
 template <int DMAX>
 __global__ void __launch_bounds__(512) k_outer_scan(const OuterScan a) {
+    pdl_enter();
     constexpr int TT = DMAX > 128 ? 4 : 8, DR = DMAX / GD_RG, ROW = GD_RG * (DR + GD_PAD);
     __shared__ __align__(16) float qs[2][TT][ROW], ks[2][TT][ROW], vs[2][TT][128], gs[2][TT][2];
     const int h = blockIdx.x, hq = h / a.share, tid = threadIdx.x, lane = tid & 31, rg = lane & 3, ncols = blockDim.x / GD_RG;
@@ -154,7 +156,8 @@ __device__ __forceinline__ void async_copies_done() {
 // grid (H, chunks, ceil(V / NC)), 256 threads: thread (ty, tx) owns 8 x NC / 16 of a 128 x NC tile of U_c; keys and values of the
 // chunk are staged in shared memory
 template <int NC>
-__global__ void __launch_bounds__(256, NC == 128 ? 2 : 1) k_outer_chunk_kv(const OuterScan a, int vec, float * __restrict__ SB, float * __restrict__ AC) {
+__global__ void __launch_bounds__(256, NC == 128 ? 2 : 1) k_outer_chunk_kv(const OuterScan a, int vec, float * SB, float * AC) {
+    pdl_enter();
     constexpr int CW = NC / 16;
     __shared__ __align__(16) float Ks[RC][128], Vs[RC][NC];
     __shared__ float pw[RC];
@@ -211,7 +214,8 @@ __global__ void __launch_bounds__(256, NC == 128 ? 2 : 1) k_outer_chunk_kv(const
     }
 }
 // grid (H, ceil(entries / 256)): a thread owns one entry of the state (matrix and normaliser alike) and walks the chunks
-__global__ void k_outer_chunk_state(int n, long long head_stride, int nch, const float * __restrict__ AC, float * __restrict__ S, float * __restrict__ SB) {
+__global__ void k_outer_chunk_state(int n, long long head_stride, int nch, const float * AC, float * S, float * SB) {
+    pdl_enter();
     const int h = blockIdx.x, e = blockIdx.y * blockDim.x + threadIdx.x;
     if (e >= n) return;
     const float * ac = AC + (size_t) h * nch;
@@ -234,7 +238,8 @@ __global__ void k_outer_chunk_state(int n, long long head_stride, int nch, const
 // grid (H, chunks, ceil(V / NC)), 128 threads: warp w owns tokens 8 w .. 8 w + 7 of the chunk, a lane NC / 32 value channels.
 // Dynamic shared memory: q and k of the chunk [RC][D + 4] each, the weighted scores [RC][RC + 4], the values [RC][NC].
 template <int NC>
-__global__ void __launch_bounds__(128) k_outer_chunk_out(const OuterScan a, int vec_all, const float * __restrict__ SB) {
+__global__ void __launch_bounds__(128) k_outer_chunk_out(const OuterScan a, int vec_all, const float * SB) {
+    pdl_enter();
     extern __shared__ __align__(16) float csm[];
     constexpr int CW = NC / 32, AP = RC + 4;            // score rows padded to whole 16-byte chunks
     const int D = a.D, V = a.V, Dp = D + 4;
@@ -294,11 +299,11 @@ __global__ void __launch_bounds__(128) k_outer_chunk_out(const OuterScan a, int 
     const auto srow = [&](int d, float (&sv)[CW]) {
         const float * p = Sc + (size_t) d * V + v;
         if (vec) {
-            if constexpr (CW == 4) { const float4 f = __ldg(reinterpret_cast<const float4 *>(p)); sv[0] = f.x; sv[1] = f.y; sv[2] = f.z; sv[3] = f.w; }
-            else { const float2 f = __ldg(reinterpret_cast<const float2 *>(p)); sv[0] = f.x; sv[1] = f.y; }
+            if constexpr (CW == 4) { const float4 f = *(reinterpret_cast<const float4 *>(p)); sv[0] = f.x; sv[1] = f.y; sv[2] = f.z; sv[3] = f.w; }
+            else { const float2 f = *(reinterpret_cast<const float2 *>(p)); sv[0] = f.x; sv[1] = f.y; }
         } else {
 #pragma unroll
-            for (int b = 0; b < CW; b++) sv[b] = v + b < V ? __ldg(p + b) : 0.f;
+            for (int b = 0; b < CW; b++) sv[b] = v + b < V ? *(p + b) : 0.f;
         }
     };
 #pragma unroll 2
@@ -354,7 +359,7 @@ __global__ void __launch_bounds__(128) k_outer_chunk_out(const OuterScan a, int 
         const float * nc = Sc + (size_t) D * V;
         float dq[8] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
         for (int d = lane; d < D; d += 32) {
-            const float n = __ldg(nc + d);
+            const float n = *(nc + d);
 #pragma unroll
             for (int i = 0; i < 8; i++) dq[i] = fmaf(n, Qs[(warp * 8 + i) * Dp + d], dq[i]);
         }
@@ -379,8 +384,9 @@ __device__ __forceinline__ float mlstm_divisor(float nq, float m) { return fmaxf
 // portions of several tokens: AB[t] = [ a: H | b: H | m: H ]. One block per head: log gates of all tokens at once into shared memory
 // (3 T floats, dynamic), the maximum from token to token in order by one warp (two dependent operations each), then a and b of
 // all tokens at once. m_state [H] is part of the sequence's state.
-__global__ void __launch_bounds__(256) k_mlstm_gates(const float * __restrict__ P, int ldp, int i_off, int f_off, float cap, int T, int H,
-                                                     float * __restrict__ m_state, float * __restrict__ AB, int ld_ab) {
+__global__ void __launch_bounds__(256) k_mlstm_gates(const float * P, int ldp, int i_off, int f_off, float cap, int T, int H,
+                                                     float * m_state, float * AB, int ld_ab) {
+    pdl_enter();
     extern __shared__ float msm[];
     float * li = msm, * lf = msm + T, * mx = msm + 2 * T;
     const int h = blockIdx.x;
@@ -433,6 +439,7 @@ struct OuterToken {
 };
 template <int DMAX, int KIND>
 __global__ void __launch_bounds__(512) k_outer_token(const OuterToken a) {
+    pdl_enter();
     constexpr int DR = DMAX / GD_RG, ROW = GD_RG * (DR + GD_PAD);
     extern __shared__ float o_s[];                      // [V] read-out, [V]: n . q
     __shared__ __align__(16) float qs[ROW], ks[ROW];
@@ -527,8 +534,9 @@ __global__ void __launch_bounds__(512) k_outer_token(const OuterToken a) {
 }
 // portions of several tokens, mLSTM's last step: each head's read-out (times the query's scale, over its divisor) over its root mean
 // square, times a weight [H][V], times sigmoid(gate). m sits in the third part of a row of the gate table. One warp per (token, head).
-__global__ void k_mlstm_out(const float * __restrict__ O, const float * __restrict__ den, const float * __restrict__ AB, int ld_ab, float q_scale, const float * __restrict__ P, int ldp, int gate_off,
-                            int H, int V, const float * __restrict__ w, float eps, float * __restrict__ A) {
+__global__ void k_mlstm_out(const float * O, const float * den, const float * AB, int ld_ab, float q_scale, const float * P, int ldp, int gate_off,
+                            int H, int V, const float * __restrict__ w, float eps, float * A) {
+    pdl_enter();
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int h = blockIdx.y * nw + warp; h < H; h += gridDim.y * nw) {
         const size_t at = (size_t) t * H * V + (size_t) h * V;
@@ -544,8 +552,9 @@ __global__ void k_mlstm_out(const float * __restrict__ O, const float * __restri
 
 // ---- state-space mixer's read-out: y = (o + skip[h] x) silu(z), then each of `parts` equal parts of the row over its own root mean
 // square (eps inside the root), times a weight. One block per (token, part).
-__global__ void __launch_bounds__(1024) k_gated_part_norm(const float * __restrict__ O, const float * __restrict__ X, int ldx, const float * __restrict__ skip, const float * __restrict__ Z, int ldz,
-                                                          int inner, int V, int parts, const float * __restrict__ w, float eps, float * __restrict__ A) {
+__global__ void __launch_bounds__(1024) k_gated_part_norm(const float * O, const float * X, int ldx, const float * skip, const float * Z, int ldz,
+                                                          int inner, int V, int parts, const float * __restrict__ w, float eps, float * A) {
+    pdl_enter();
     __shared__ float red[32];
     constexpr int OWN = 8;                              // entries a thread keeps in registers until the part's sum of squares is known
     const int t = blockIdx.x, n = inner / parts, i0 = blockIdx.y * n, nt = blockDim.x;
@@ -603,6 +612,7 @@ struct SelScan {
 };
 template <int LANES, int NS, int MODE>
 __global__ void __launch_bounds__(256) k_selective_scan(const SelScan a) {
+    pdl_enter();
     constexpr int NCH = 256 / LANES, NM = LANES * NS, TT = NM > 64 ? 8 : 16;
     __shared__ __align__(16) float xs[2][TT][NCH], ds[2][TT][NCH], zs[2][TT][NCH], bs[2][TT][NM], cs[2][TT][NM];
     const int tid = threadIdx.x, rg = tid % LANES, cl = tid / LANES, c0 = blockIdx.x * NCH, c = c0 + cl, N = a.N;
@@ -699,6 +709,7 @@ __global__ void __launch_bounds__(256) k_selective_scan(const SelScan a) {
 // one token: the step size's low-rank product (Wdt [inner][R], bias) is part of the same launch; the lanes of a channel share it
 template <typename WT, int LANES, int NS>
 __global__ void __launch_bounds__(256) k_selective_token(const SelScan a, const WT * __restrict__ Wdt, const float * __restrict__ bdt, int R) {
+    pdl_enter();
     constexpr int NCH = 256 / LANES;
     extern __shared__ float low[];                      // [R] the step size's low-rank input
     const int tid = threadIdx.x, rg = tid % LANES, cl = tid / LANES, c = blockIdx.x * NCH + cl, N = a.N;

@@ -15,8 +15,9 @@ namespace stk {
 // layer's input. One block per token (hc_threads threads).
 struct PairTable { const void * w; unsigned long long mul_prev, mul_cur, buckets; };      // w == nullptr: no such table
 template <typename WT>
-__global__ void __launch_bounds__(1024) k_embed_pair(const WT * __restrict__ embed, PairTable pt, const StepState * __restrict__ st, const int32_t * __restrict__ tokens,
-                                                    int E, int n_vocab, const float * __restrict__ w, float eps, float * __restrict__ X, float * __restrict__ Hn) {
+__global__ void __launch_bounds__(1024) k_embed_pair(const WT * __restrict__ embed, PairTable pt, const StepState * st, const int32_t * tokens,
+                                                    int E, int n_vocab, const float * __restrict__ w, float eps, float * X, float * Hn) {
+    pdl_enter();
     __shared__ float red[32];
     const int t = blockIdx.x, nt = blockDim.x;
     const auto id = [&](int i) { const int v = tokens[i]; return v < 0 ? 0 : v >= n_vocab ? n_vocab - 1 : v; };      // ids are validated on the host; never read outside the table
@@ -70,6 +71,7 @@ template <int VEC> __device__ __forceinline__ void sum_chunk(const SumArgs & a, 
 }
 template <int VEC>
 __global__ void __launch_bounds__(1024) k_sum_join(const SumArgs a) {
+    pdl_enter();
     __shared__ float red[32];
     const int t = blockIdx.x, nt = blockDim.x, nchunk = a.E / VEC;
     const size_t row = (size_t) t * a.E;
@@ -118,7 +120,8 @@ struct SideW {
 };
 // prompt portions, between the two products: Z[t][i] <- gelu(Z[t][i]) e_i. grid (T, slices of dim)
 template <typename WT>
-__global__ void k_side_gate(float * __restrict__ Z, SideW s, const int32_t * __restrict__ tokens, int n_vocab) {
+__global__ void k_side_gate(float * Z, SideW s, const int32_t * tokens, int n_vocab) {
+    pdl_enter();
     const int t = blockIdx.x, i = blockIdx.y * blockDim.x + threadIdx.x;
     if (i >= s.dim) return;
     int tok = tokens[t];
@@ -153,7 +156,7 @@ __device__ __forceinline__ uint4 ld_now(const void * p) {                 // sta
     return v;
 }
 template <typename WT>
-__global__ void __launch_bounds__(SIDE_THREADS) k_side_in(const SumArgs a, const SideW s, const int32_t * __restrict__ tokens, int n_vocab, int vec, float * __restrict__ Xs, float * __restrict__ G) {
+__global__ void __launch_bounds__(SIDE_THREADS) k_side_in(const SumArgs a, const SideW s, const int32_t * tokens, int n_vocab, int vec, float * Xs, float * G) {
     extern __shared__ __align__(16) float xs[];
     __shared__ float ps[SIDE_THREADS / 32];
     constexpr int VEC = 16 / (int) sizeof(WT), GP = 4, WPR = SIDE_THREADS / 32 / SIDE_ROWS;      // chunks per lane asked for ahead; warps per row
@@ -169,6 +172,7 @@ __global__ void __launch_bounds__(SIDE_THREADS) k_side_in(const SumArgs a, const
     int tok = tokens[t];
     tok = tok < 0 ? 0 : tok >= n_vocab ? n_vocab - 1 : tok;
     const float e = on ? wf(reinterpret_cast<const WT *>(s.table), (size_t) tok * s.ld + s.off + r) : 0.f;
+    pdl_enter();
     const auto sum = [&](int i, auto & v) {
         constexpr int N = sizeof(v) / sizeof(float);
         sum_chunk<N>(a, t, i, v);
@@ -202,7 +206,7 @@ __global__ void __launch_bounds__(SIDE_THREADS) k_side_in(const SumArgs a, const
 constexpr int SIDE_PER = 2;
 inline int side_rows_per_block(int lpr) { return SIDE_THREADS / lpr * SIDE_PER; }
 template <typename WT, int XV>
-__global__ void __launch_bounds__(SIDE_THREADS) k_side_out(const SumArgs a, const SideW s, const float * __restrict__ Xs, const float * __restrict__ G, float * __restrict__ Y, int * __restrict__ counter, int vec, int lpr) {
+__global__ void __launch_bounds__(SIDE_THREADS) k_side_out(const SumArgs a, const SideW s, const float * Xs, const float * G, float * Y, int * counter, int vec, int lpr) {
     extern __shared__ __align__(16) float g[];
     __shared__ float red[32];
     __shared__ int last_s;
@@ -214,6 +218,7 @@ __global__ void __launch_bounds__(SIDE_THREADS) k_side_out(const SumArgs a, cons
 #pragma unroll
         for (int j = 0; j < SIDE_PER; j++) { const int r = r0 + j * ngrp; wp[j] = r < E && sub * VEC < dim ? ld_now(Wp + (size_t) r * dim + sub * VEC) : make_uint4(0u, 0u, 0u, 0u); }
     }
+    pdl_enter();
     for (int i = tid; i < dim; i += SIDE_THREADS) g[i] = G[(size_t) t * dim + i];
     __syncthreads();
     const size_t row = (size_t) t * E;

@@ -124,7 +124,7 @@ void b200_reset_timings(b200_ctx * c);
  * T <= 4 takes the decode mat-vec, larger T the prompt kernels), CUDA events around `reps` launches over distinct weights;
  * negative on error. bench.py's per-kernel roofline of the family. */
 float b200_stack_time_linear(int device, int dtype, int T, int N, int K, int reps);
-/* the kernel such a product takes (glu: gate and up rows interleaved): 0 a warp per row, 1 a block per row, 2 a block per eight rows with x in
+/* the kernel such a product takes by itself (in a model's pass one token's products go to the ring kernel, b200_stack_linear_in_pass; glu: gate and up rows interleaved): 0 a warp per row, 1 a block per row, 2 a block per eight rows with x in
  * registers, 3 tcgen05 (bfloat16), 4 tcgen05 (float32) in K parts, 5 mma.sync, 6 tiles on the fp32 pipe, 7 tcgen05 (float32) whole, -1 bad arguments (host arithmetic, tests) */
 int b200_stack_product_kernel(int dtype, int T, int N, int K, int glu, int sm_count);
 /* operator-level parity entry of the same products: y[T][N] = x[T][K] . w[N][K]^T (+ bias[N]); glu != 0: the rows of w are
@@ -133,6 +133,8 @@ int b200_stack_product_kernel(int dtype, int T, int N, int K, int glu, int sm_co
  * T <= 4 the mat-vec, else (bfloat16) tcgen05.mma with TMEM accumulators for T >= 64, N >= 128, K >= 64, K % 8 == 0, mma.sync
  * for other 16-byte-aligned shapes, the CUDA-core product for float32 and odd shapes. */
 int b200_stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y);
+/* the same product as a model's pass launches it: one token's takes the kernel that asks for its rows ahead of the kernel in front of it, here the same product once more */
+int b200_stack_linear_in_pass(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y);
 /* number of kernels launched by this library's own code since the context was created */
 int64_t b200_kernel_launches(const b200_ctx * c);
 /* device time (CUDA events on the engine's stream) of the last b200_generate_greedy /

@@ -52,3 +52,21 @@ def test_shared_memory_limits_are_kept_per_device(name):
     """a kernel's limit of dynamic shared memory holds on the device it was set on: what remembers that it was raised is an array over devices"""
     once = [line.strip() for line in _code(CSRC / name) if re.search(r"static (const )?(bool|size_t) \w+ = ", line) and ("cudaFuncSetAttribute" in line or "attr" in line)]
     assert not once, once
+
+
+@pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("stack_kernels*.cuh")))
+def test_stack_kernels_wait_for_the_kernel_before_them(name):
+    """a pass's kernels become resident while the one before still runs: each waits before it reads what another wrote, and reads that coherently (no __ldg, no read-only pointer of
+    what a pass computes: the compiler may take such a load for one of a constant and move it ahead of the wait)"""
+    text = "\n".join(_code(CSRC / name))
+    bodies = re.split(r"__global__", text)[1:]
+    weights = {"embed", "w_post", "w_next", "cnorm", "qnorm", "W2", "w0", "coef", "sink", "dt_bias", "A_log", "w", "bias", "r1v", "r2v", "Wdt", "bdt"}
+    bad = []
+    for b in bodies:
+        kernel = re.search(r"\b(k_\w+)\s*\(", b).group(1)
+        signature = b[:b.index("{")]
+        if "pdl_enter()" not in b and "pdl_wait()" not in b:
+            bad.append(f"{kernel} does not wait")
+        bad += [f"{kernel}: {m}" for m in re.findall(r"\*\s*__restrict__\s*(\w+)", signature) if m not in weights]
+        bad += [f"{kernel}: __ldg of {m}" for m in re.findall(r"__ldg\((.*)", b) if "(w + i)" not in m]
+    assert not bad, bad

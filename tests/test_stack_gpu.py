@@ -452,6 +452,30 @@ def test_products_where_their_rules_change(dtype, T, N, K, glu):
     assert (np.abs(y - ref) <= off).all(), np.max(np.abs(y - ref) / off)
 
 
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("N,K,glu", [
+    (1, 8, False), (13, 256, False), (300, 264, True), (147, 504, False), (2, 520, True), (149, 1024, False), (1184, 1032, True), (297, 2040, False), (38000, 2048, False),
+    (40002, 64, True), (130, 2056, False), (606, 4096, True), (7, 4104, False), (301, 8192, False), (34, 8184, True), (301, 8200, False), (60, 1031, False)])
+def test_one_token_products_in_a_pass(dtype, N, K, glu):
+    """the ring kernel at the edges of its teams of warps and pieces per lane, with fewer and more rows than SMs and stages, in one round and several, behind itself; and what it leaves
+    to the kernels of products by themselves. Bound: test_products_where_their_rules_change"""
+    rng = np.random.default_rng(N + K)
+    x = rng.standard_normal((1, K)).astype(np.float32)
+    w = so.round_bf16((rng.standard_normal((N, K)) / np.sqrt(K)).astype(np.float32))
+    b = so.round_bf16(rng.standard_normal(N).astype(np.float32))
+    y = np.full(N // 2 if glu else N, np.nan, np.float32)
+    f32p = C.POINTER(C.c_float)
+    rc = _lib.lib().b200_stack_linear_in_pass(0, 0 if dtype == "bfloat16" else 1, 1, N, K, x.ctypes.data_as(f32p), w.ctypes.data_as(f32p), b.ctypes.data_as(f32p), int(glu), 7.0, y.ctypes.data_as(f32p))
+    assert rc == 0, _lib.last_error()
+    ref = (x.astype(np.float64) @ w.astype(np.float64).T + b)[0]
+    off = (K + 8) * 2.0 ** -24 * ((np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64)).T)[0] + np.abs(b))
+    if glu:
+        g, u = np.minimum(ref[0::2], 7.0), np.clip(ref[1::2], -7.0, 7.0)
+        ref = g * so.sigmoid(1.702 * g) * (u + 1.0)
+        off = 1.13 * np.abs(u + 1.0) * off[0::2] + (np.abs(g) + 1.0) * off[1::2] + 1e-5 * (1.0 + np.abs(ref))
+    assert (np.abs(y - ref) <= off).all(), np.nanmax(np.abs(y - ref) / off)
+
+
 def test_float32_contexts_hold_no_room_for_products_they_never_run(tmp_path):
     """a float32 context has room for the K parts of its own model's products and no more (19 MB would hold any): sixteen small contexts stay well below what
     that alone would take, and a portion that is cut into parts decodes the oracle's rows"""
