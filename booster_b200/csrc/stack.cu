@@ -37,6 +37,7 @@
 #include "safetensors.hpp"
 #include "stack_kernels.cuh"
 #include "stack_kernels_f32.cuh"
+#include "stack_kernels_pair.cuh"
 #include "stack_kernels_mix.cuh"
 #include "stack_kernels_hyper.cuh"
 #include "stack_kernels_scan.cuh"
@@ -279,6 +280,9 @@ struct StackCtx {
     int * da_counter = nullptr;           // per (token, head): slices done
     int sm_count = 148;
     __nv_bfloat16 * xb = nullptr;         // activations of a prompt pass rounded to bfloat16 (operand of the tcgen05 product)
+    __nv_bfloat16 * u16 = nullptr;        // gated units of a prompt pass as their product left them, rounded (as many entries as xb)
+    __nv_bfloat16 * h16 = nullptr;        // Hn rounded, where this pass's norms leave it so ...
+    bool h16_on = false;                  // ... and whether they do
     size_t xb_elems = 0;
     float * xpart = nullptr;              // sums of the K parts of a product with few output tiles
     size_t xpart_floats = 0;
@@ -1355,13 +1359,44 @@ void split_sum(const Lane & lane, const float * part, int parts, int T, int N, c
     if (wide) pdl(lane, grid, 256, 0, k_split_sum<4>, part, parts, T, N, bias, Y, ldy);
     else pdl(lane, grid, 256, 0, k_split_sum<1>, part, parts, T, N, bias, Y, ldy);
 }
+// bfloat16 products on pairs of SMs (k_gemm_bf16_pair): whole matrices, or rows sorted by expert, of at least half a pair's rows. Per-head products of a batch and narrower ones keep
+// a block per 128 tokens x 256 rows.
+bool pair_takes(int N, int n_seg) { return N >= 128 && n_seg <= PG_SEG_MAX; }
+// How a product is cut: tokens per tile (one or two accumulators) and K parts, by the clocks they cost. A slice takes as long as its MMAs (2 clocks a column) or its bytes out of L2 (40 a
+// clock and SM); a tile 3000 to fill the pipeline, and 10 a column to drain; parts 4000 for the launch that adds them and 500 each, and their sums' way (4 bytes at 16 a clock and SM).
+PairPlan pair_plan(int T, int N, int K, int n_seg, bool parts_ok, int sm_count, size_t part_floats) {
+    const int pairs = sm_count / 2, nk = (K + PG_BK - 1) / PG_BK, row_tiles = (N + PG_ROWS - 1) / PG_ROWS;
+    PairPlan best{1, 256, 1, 0, 2, n_seg};
+    if (!n_seg) {
+        double least = 1e30;
+        const int most = (T + 31) / 32 * 32;
+        for (int acc = 1; acc <= 2; acc++)
+            for (int tiles = 1; tiles <= 64; tiles++) {
+                const int n = ((T + tiles * acc - 1) / (tiles * acc) + 31) / 32 * 32;
+                if (n > 256) continue;
+                if (n < 64 && n < most) break;
+                const int tt = (T + acc * n - 1) / (acc * n);
+                for (int parts = 1; parts <= (parts_ok ? std::min(16, std::max(1, nk / 2)) : 1); parts++) {
+                    if (parts > 1 && (size_t) parts * T * N > part_floats) break;
+                    const int work = row_tiles * tt * parts, rounds = (work + pairs - 1) / pairs;
+                    const double slice = std::max(2.0 * acc * n, pg_stage_bytes(acc, n) / 40.0), drain = 10.0 * acc * n, form = slice * ((nk + parts - 1) / parts);
+                    const bool over = 2 * acc * n <= 512;
+                    const double cost = 3000 + (over ? rounds * std::max(form, drain) + drain : rounds * (form + drain)) + (parts > 1 ? 4000 + 500 * parts + (double) parts * T * N * 4 / (16.0 * sm_count) : 0);
+                    if (cost < least) { least = cost; best = PairPlan{acc, n, parts, 0, over ? 2 : 1, 0}; }
+                }
+            }
+    }
+    best.stages = std::min(PG_MAX_STAGES, PG_SMEM / pg_stage_bytes(best.acc, best.n));
+    return best;
+}
+
 // the kernel a product goes to: mat-vecs of few tokens, then tile kernels
 enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG, LIN_ROWS_X, LIN_UMMA, LIN_F32_PARTS, LIN_MMA, LIN_SIMT, LIN_F32_UMMA };
 // vec: LinArgs::vec; scratch: whether there is any (an error flag); x_elems: entries of X; xb_elems, part_floats: what the scratch has room for
 LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu, bool seg, bool scratch, size_t x_elems, size_t xb_elems, size_t part_floats, int sm_count) {
     if (T == 1 && vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && gx_pays(dtype == STACK_F32, K / (dtype == STACK_F32 ? 4 : 8), N, batch, glu, sm_count)) return LIN_ROWS_X;
     if (T <= GEMV_MAX_T) return !glu && batch == 1 && N <= GEMV_FEW_ROWS && K >= 1024 ? LIN_ROWS_LONG : LIN_ROWS;      // few, long rows: a block each
-    if (dtype == STACK_BF16 && vec && umma_enabled() && T >= 64 && N >= 128 && K >= 64 && x_elems <= xb_elems) return LIN_UMMA;
+    if (dtype == STACK_BF16 && vec && umma_enabled() && K >= 64 && x_elems <= xb_elems && ((T >= 64 && N >= 128) || (N >= 256 && (batch == 1 || seg) && pair_takes(N, seg ? batch : 0)))) return LIN_UMMA;      // (few tokens: a pair's columns are as few; half a pair's rows stay with mma.sync)
     if (dtype == STACK_F32 && scratch && f32_umma_takes(vec, T, N, K)) {
         const int parts = batch == 1 && !glu && !seg ? f32_k_parts(T, N, K, sm_count) : 1;      // (a gated unit needs its sums whole)
         return parts > 1 && (size_t) parts * T * N <= part_floats ? LIN_F32_PARTS : LIN_F32_UMMA;
@@ -1418,6 +1453,27 @@ CUtensorMap map_bf16(const void * base, int K, int rows, int nz, long long ld, l
     return m;
 }
 
+template <bool SEG, int ACC, int GLU, bool ROUND>
+void launch_pair_as(const Lane & lane, const CUtensorMap & mx, const CUtensorMap & mw, const LinArgs & a, const PairPlan & p, int work, int sm_count, int * err, float * part) {
+    static size_t have[64] = {0};
+    raise_smem(k_gemm_bf16_pair<SEG, ACC, GLU, ROUND>, PG_SMEM + 1024, have);
+    pdl(lane, 2 * std::min(sm_count / 2, work), PG_THREADS, (size_t) p.stages * pg_stage_bytes(ACC, p.n) + 1024, k_gemm_bf16_pair<SEG, ACC, GLU, ROUND>, mx, mw, a, p, err, part);
+}
+void launch_pair(const Lane & lane, const CUtensorMap & mx, const CUtensorMap & mw, const LinArgs & a, const PairPlan & p, int work, int sm_count, int * err, float * part) {
+    const auto go = [&](auto seg, auto acc) {
+        constexpr bool S = decltype(seg)::value;
+        constexpr int A = decltype(acc)::value;
+        if (a.glu == GLU_GELU && a.Yb) launch_pair_as<S, A, GLU_GELU, true>(lane, mx, mw, a, p, work, sm_count, err, part);
+        else if (a.glu == GLU_GELU) launch_pair_as<S, A, GLU_GELU, false>(lane, mx, mw, a, p, work, sm_count, err, part);
+        else if (a.glu && a.Yb) launch_pair_as<S, A, GLU_SIGMOID, true>(lane, mx, mw, a, p, work, sm_count, err, part);
+        else if (a.glu) launch_pair_as<S, A, GLU_SIGMOID, false>(lane, mx, mw, a, p, work, sm_count, err, part);
+        else launch_pair_as<S, A, GLU_NONE, false>(lane, mx, mw, a, p, work, sm_count, err, part);
+    };
+    if (a.seg) go(std::true_type(), std::integral_constant<int, 1>());
+    else if (p.acc == 1) go(std::false_type(), std::integral_constant<int, 1>());
+    else go(std::false_type(), std::integral_constant<int, 2>());
+}
+
 // what a product may ask for beyond its operands: the gated unit's kind and constants (y = g sigmoid(alpha g) (u + shift), g and u clamped
 // at +-limit, or gelu(g) u), rows sorted into segments per batch entry (tile kernels), an indexed batch (mat-vec)
 struct LinOpt {
@@ -1428,13 +1484,15 @@ struct LinOpt {
     int n_w = 0;                            // mat-vec: matrices in the indexed batch (0: every index is one)
     int x_share = 1;
     const float * x_scale = nullptr;        // mat-vec: entry z runs on x_scale[z] times its input row
+    const __nv_bfloat16 * x16 = nullptr;    // tcgen05 (bfloat16): X rounded, rows K apart, if it is there already
+    __nv_bfloat16 * y16 = nullptr;          // gated units of such a product on pairs of SMs (pairs()): rounded, here, instead of Y
 };
 void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X, int ldx, const void * W, const float * bias, float * Y, int ldy,
                int T, int N, int K, int batch = 1, long long sX = 0, long long sW = 0, long long sY = 0, bool glu = false, float glu_limit = 0.f,
                const UmmaScratch * us = nullptr, const LinOpt * opt = nullptr) {
     if (T <= 0 || N <= 0) return;
     LinArgs a{X, W, bias, Y, T, N, K, ldx, ldy, sX, sW, sY, 0, glu ? GLU_SIGMOID : GLU_NONE, glu_limit, GLU_ALPHA, 0, 0};
-    if (opt) { if (glu) a.glu = opt->glu_kind; a.n_w = opt->n_w; a.alpha = opt->alpha; a.up_shift = opt->shift; a.seg = opt->seg; a.w_index = opt->w_index; a.x_share = opt->x_share; a.x_scale = opt->x_scale; }
+    if (opt) { if (glu) a.glu = opt->glu_kind; a.n_w = opt->n_w; a.alpha = opt->alpha; a.up_shift = opt->shift; a.seg = opt->seg; a.w_index = opt->w_index; a.x_share = opt->x_share; a.x_scale = opt->x_scale; a.Yb = opt->y16; }
     const int xbatch = a.seg ? 1 : batch;      // segments: X is one matrix of T rows
     const int vecw = dtype == STACK_F32 ? 4 : 8;
     const auto al16 = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
@@ -1466,9 +1524,19 @@ void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X
         // tensor memory path: activations to bfloat16 once, then tcgen05.mma over TMA-fed stages (a.vec: rows and batch strides are multiples of 16 bytes)
         static size_t have[64] = {0};
         raise_smem(k_gemm_bf16_umma, UM_SMEM, have);
-        pdl(lane, dim3((unsigned) std::min<long long>(((long long) T * (K / 8) + 255) / 256, 2048), (unsigned) xbatch), 256, 0, k_to_bf16, X, ldx, T, K, sX, us->xb, (long long) T * K);
+        const __nv_bfloat16 * x16 = opt && opt->x16 ? opt->x16 : us->xb;
+        if (x16 == us->xb && !(opt && opt->x16)) pdl(lane, dim3((unsigned) std::min<long long>(((long long) T * (K / 8) + 255) / 256, 2048), (unsigned) xbatch), 256, 0, k_to_bf16, X, ldx, T, K, sX, us->xb, (long long) T * K);
+        if ((batch == 1 || a.seg) && pair_takes(N, a.seg ? batch : 0)) {
+            const PairPlan p = pair_plan(T, N, K, a.seg ? batch : 0, !a.glu && !a.seg && us->part && split_k_enabled(), us->sm_count, us->part_floats);
+            const CUtensorMap mx = map_bf16(x16, K, T, 1, K, (long long) T * K, a.seg ? 32 : p.n / 2), mw = map_bf16(W, K, N, batch, K, sW, 128);
+            const int row_tiles = (N + PG_ROWS - 1) / PG_ROWS, work = a.seg ? row_tiles * batch * ((T + 255) / 256) : row_tiles * ((T + p.acc * p.n - 1) / (p.acc * p.n)) * p.parts;
+            launch_pair(lane, mx, mw, a, p, work, us->sm_count, us->err, us->part);
+            if (p.parts > 1) { split_sum(lane, us->part, p.parts, T, N, bias, Y, ldy); if (launches) (*launches)++; }
+            if (launches) (*launches)++;
+            return;
+        }
         const dim3 grid((unsigned) ((N + UM_BN - 1) / UM_BN), (unsigned) ((T + UM_BM - 1) / UM_BM), (unsigned) batch);
-        const CUtensorMap mx = map_bf16(us->xb, K, T, xbatch, K, (long long) T * K, UM_BM), mw = map_bf16(W, K, N, batch, K, sW, UM_BN);
+        const CUtensorMap mx = map_bf16(x16, K, T, xbatch, K, (long long) T * K, UM_BM), mw = map_bf16(W, K, N, batch, K, sW, UM_BN);
         const int tiles = (int) (grid.x * grid.y), nk = (K + UM_BK - 1) / UM_BK;
         const int ksplit = batch == 1 && !a.glu && !a.seg && us->part && split_k_enabled() ? std::min(us->sm_count / tiles, nk / 4) : 1;
         if (ksplit > 1) {
@@ -1498,13 +1566,36 @@ void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X
 void linear(StackCtx * c, const float * X, int ldx, const DMat & W, float * Y, int ldy, int T, int batch = 1, long long sX = 0, long long sY = 0, bool glu = false, float glu_limit = 0.f,
             const LinOpt * opt = nullptr) {
     const UmmaScratch us{c->xb, c->xb_elems, c->d_err, c->xpart, c->xpart_floats, c->sm_count};
+    LinOpt rounded;
+    if (c->h16_on && X == c->Hn && batch == 1 && W.K == c->m->E && ldx == W.K) {       // the norm left its rows as bfloat16 too
+        if (opt) rounded = *opt;
+        rounded.x16 = c->h16;
+        opt = &rounded;
+    }
     linear_on(Lane{c->st, &c->cold}, c->m->dtype, &c->launches, X, ldx, W.w, W.bias, Y, ldy, T, W.N, W.K, batch, sX, (long long) W.N * W.K, sY, glu, glu_limit, &us, opt);
+}
+
+// whether a bfloat16 model's product of this pass goes to pairs of SMs (n_seg > 0: rows sorted by that many experts)
+bool pairs(const StackCtx * c, int T, const DMat & W, int n_seg = 0) {
+    return c->m->dtype == STACK_BF16 && W.K % 8 == 0 && pair_takes(W.N, n_seg) &&
+           lin_route(STACK_BF16, T, W.N, W.K, std::max(1, n_seg), true, false, n_seg > 0, true, (size_t) T * W.K, c->xb_elems, c->xpart_floats, c->sm_count) == LIN_UMMA;
+}
+// a feed-forward of gated units: F [T][ff] holds them, or u16 their rounded values where both products take those
+void gated_ff(StackCtx * c, const float * X, const DMat & gateup, float * F, const DMat & down, float * Y, int T, float limit, const LinOpt * opt = nullptr, int n_seg = 0) {
+    const int ff = down.K, batch = std::max(1, n_seg);
+    const bool both = pairs(c, T, gateup, n_seg) && pairs(c, T, down, n_seg);
+    LinOpt o, d;
+    if (opt) o = *opt;
+    d.seg = o.seg;
+    if (both) { o.y16 = c->u16; d.x16 = c->u16; }
+    linear(c, X, gateup.K, gateup, F, ff, T, batch, 0, 0, true, limit, &o);
+    linear(c, F, ff, down, Y, down.N, T, batch, 0, 0, false, 0.f, &d);
 }
 
 // end of a sub-layer: X += norm(Y) * w_post; Hn = norm(X) * w_next when another sub-layer follows
 void post_norm_add(StackCtx * c, const float * w_post, const float * w_next, int T) {
     const StackModel & m = *c->m;
-    pdl(c, T, std::min(256, 32 * m.groups), 0, k_post_norm_add, c->Y, w_post, c->X, w_next, c->Hn, m.E, m.groups, m.eps);
+    pdl(c, T, std::min(256, 32 * m.groups), 0, k_post_norm_add, c->Y, w_post, c->X, w_next, c->Hn, m.E, m.groups, m.eps, c->h16_on ? c->h16 : nullptr);
     c->launches++;
 }
 
@@ -2122,8 +2213,8 @@ void enqueue_layers_sequential(StackCtx * c, int T) {
     const int E = m.E;
     const int nthreads = std::min(256, std::max(128, 32 * m.groups));
     const float * w0 = m.layers[(size_t) m.runs[0].layer].norm1;
-    if (m.dtype == STACK_F32) pdl(c, T, nthreads, 0, k_embed_rows<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, c->X, w0, m.groups, m.eps, c->Hn);
-    else pdl(c, T, nthreads, 0, k_embed_rows<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, c->X, w0, m.groups, m.eps, c->Hn);
+    if (m.dtype == STACK_F32) pdl(c, T, nthreads, 0, k_embed_rows<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, c->X, w0, m.groups, m.eps, c->Hn, c->h16_on ? c->h16 : nullptr);
+    else pdl(c, T, nthreads, 0, k_embed_rows<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, c->X, w0, m.groups, m.eps, c->Hn, c->h16_on ? c->h16 : nullptr);
     c->launches++;
     c->in = c->Hn; c->out = c->Y;
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
@@ -2133,8 +2224,7 @@ void enqueue_layers_sequential(StackCtx * c, int T) {
         run_mixer(c, L, R, T);                         // Hn holds norm1(x)
         post_norm_add(c, L.norm1b, L.has_mlp ? L.norm2 : next_in, T);
         if (L.has_mlp) {
-            linear(c, c->Hn, E, L.gateup, c->A, L.ff, T, 1, 0, 0, true, L.limit);      // clamped gated unit in the epilogue
-            linear(c, c->A, L.ff, L.down, c->Y, E, T);
+            gated_ff(c, c->Hn, L.gateup, c->A, L.down, c->Y, T, L.limit);
             post_norm_add(c, L.norm2b, next_in, T);
         }
         if (c->taps) tap_layer(c, ri, T);
@@ -2228,11 +2318,11 @@ void mixture_ff(StackCtx * c, const LayerSpec & L, const float * h, int T, const
         const int in_smem = (size_t) slots * 4 + cnt_bytes <= 40 * 1024 ? 1 : 0;
         pdl(c, 1, 1024, cnt_bytes + (in_smem ? (size_t) slots * 4 : 0), k_moe_sort, c->r_sel, slots, top, n, tpe, in_smem, c->r_seg, c->r_slot, c->r_src);
         if (L.scale_input) pdl(c, slots, 128, 0, k_spread_rows, h, E, c->r_slot, c->r_wt, top, E, c->Xp);
+        else if (c->h16_on && h == c->Hn && E % 8 == 0 && pairs(c, slots, L.e_gateup, L.n_exp)) { pdl(c, slots, 128, 0, k_gather_rows16, c->h16, c->r_src, E, c->xb); o.x16 = c->xb; }
         else pdl(c, slots, 128, 0, k_gather_rows, h, E, c->r_src, E, c->Xp);
         c->launches += 2;
         o.seg = c->r_seg;
-        linear(c, c->Xp, E, L.e_gateup, c->Ap, ff, slots, L.n_exp, 0, 0, true, L.e_limit, &o);      // rows of identity outputs sort behind the last matrix
-        linear(c, c->Ap, ff, L.e_down, c->Yk, E, slots, L.n_exp, 0, 0, false, 0.f, &o);
+        gated_ff(c, c->Xp, L.e_gateup, c->Ap, L.e_down, c->Yk, slots, L.e_limit, &o, L.n_exp);      // rows of identity outputs sort behind the last matrix
         *slot_of = c->r_slot;
     }
     if (L.ff > 0) {
@@ -2398,7 +2488,7 @@ struct SideStream {
 void layer_end(StackCtx * c, const LayerSpec & L, SumArgs a, const float * nw, int T) {
     const StackModel & m = *c->m;
     const int E = m.E, dim = m.side_dim, nt = hc_threads(T, E, 4);
-    a.X = c->X; a.E = E; a.eps = m.eps; a.Hn = c->Hn;
+    a.X = c->X; a.E = E; a.eps = m.eps; a.Hn = c->Hn; a.H16 = c->h16_on ? c->h16 : nullptr;
     a.nw = dim > 0 ? nullptr : nw;
     const SideW s{m.side_table, (int) m.layers.size() * dim, L.side_off, dim, L.side_gate.w, L.side_proj.w, L.side_norm};
     if (dim > 0 && T <= GEMV_MAX_T && E <= SIDE_MOST && dim <= SIDE_MOST && side_fused_enabled()) {
@@ -2427,7 +2517,7 @@ void layer_end(StackCtx * c, const LayerSpec & L, SumArgs a, const float * nw, i
     else pdl(c, zgrid, 128, 0, k_side_gate<__nv_bfloat16>, c->SZ, s, c->d_step->tokens, m.vocab);
     linear(c, c->SZ, dim, L.side_proj, c->Y, E, T);
     PostJoinArgs j{};
-    j.X = c->X; j.E = E; j.eps = m.eps; j.mult = 1.f; j.w = L.side_norm; j.scratch = c->Hn; j.Ya = c->Y; j.fw = nw; j.Hn = c->Hn;
+    j.X = c->X; j.E = E; j.eps = m.eps; j.mult = 1.f; j.w = L.side_norm; j.scratch = c->Hn; j.Ya = c->Y; j.fw = nw; j.Hn = c->Hn; j.H16 = c->h16_on ? c->h16 : nullptr;
     if (E % 4 == 0) pdl(c, T, nt, 0, k_post_join<4>, j);
     else pdl(c, T, hc_threads(T, E), 0, k_post_join<1>, j);
     c->launches += 2;
@@ -2441,8 +2531,8 @@ void enqueue_layers_shared(StackCtx * c, int T) {
     const int E = m.E, nt = hc_threads(T, E);
     const float * w0 = m.layers[(size_t) m.runs[0].layer].norm1;
     const PairTable pt{m.pair_table, (unsigned long long) m.pair_mul_prev, (unsigned long long) m.pair_mul_cur, (unsigned long long) m.pair_buckets};
-    if (m.dtype == STACK_F32) pdl(c, T, nt, 0, k_embed_pair<float>, (const float *) m.embed, pt, &c->d_step->st, c->d_step->tokens, E, m.vocab, w0, m.eps, c->X, c->Hn);
-    else pdl(c, T, nt, 0, k_embed_pair<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, pt, &c->d_step->st, c->d_step->tokens, E, m.vocab, w0, m.eps, c->X, c->Hn);
+    if (m.dtype == STACK_F32) pdl(c, T, nt, 0, k_embed_pair<float>, (const float *) m.embed, pt, &c->d_step->st, c->d_step->tokens, E, m.vocab, w0, m.eps, c->X, c->Hn, c->h16_on ? c->h16 : nullptr);
+    else pdl(c, T, nt, 0, k_embed_pair<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, pt, &c->d_step->st, c->d_step->tokens, E, m.vocab, w0, m.eps, c->X, c->Hn, c->h16_on ? c->h16 : nullptr);
     c->launches++;
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
         const RunSpec & R = m.runs[ri];
@@ -2461,8 +2551,7 @@ void enqueue_layers_shared(StackCtx * c, int T) {
             } else {
                 LinOpt o;
                 o.glu_kind = L.act_kind; o.alpha = L.act_alpha; o.shift = L.act_shift;
-                linear(c, c->Hn, E, L.gateup, c->F, L.ff, T, 1, 0, 0, true, INFINITY, &o);
-                linear(c, c->F, L.ff, L.down, c->Y2, E, T);
+                gated_ff(c, c->Hn, L.gateup, c->F, L.down, c->Y2, T, INFINITY, &o);
                 a.Yb = c->Y2;
             }
             if (fork) SCU(cudaEventRecord(c->ev_join, c->st));
@@ -2477,6 +2566,7 @@ void enqueue_layers_shared(StackCtx * c, int T) {
 // the layers over the T tokens whose header (positions, ids) is already on the device
 void enqueue_layers(StackCtx * c, int T) {
     c->cold = true;
+    c->h16_on = c->h16 && T > GEMV_MAX_T && umma_enabled();
     if (c->m->block == BLOCK_PARALLEL) enqueue_layers_parallel(c, T);
     else if (c->m->block == BLOCK_PRENORM) enqueue_layers_prenorm(c, T);
     else if (c->m->block == BLOCK_HYPER) enqueue_layers_hyper(c, T);
@@ -2490,6 +2580,7 @@ void enqueue_head(StackCtx * c, int n_rows, int64_t row_off, bool one_token = fa
     StackModel & m = *c->m;
     const bool normed = m.block == BLOCK_HYPER || m.block == BLOCK_POSTNORM || m.block == BLOCK_SHARED;
     const float * hn = c->Hn;
+    c->h16_on = false;      // (what the head reads is no pass's row by row)
     if (normed) {
         // the last join left the normed residual (the sum of the streams) in Hn for every row of the pass: the wanted rows are gathered for the head
         if (!one_token) { pdl(c, n_rows, 128, 0, k_gather_rows, c->Hn, m.E, c->d_step->rows, m.E, c->Y); c->launches++; hn = c->Y; }
@@ -2601,7 +2692,7 @@ void stack_ctx_free(StackCtx * c) {
     for (float * p : { c->X, c->Hn, c->Y, c->P, c->A, c->QK, c->OL, c->CV, c->BG, c->O, c->rec, c->d_logits }) cudaFree(p);
     for (float * p : c->cache_allocs) cudaFree(p);
     cudaFree(c->att_scores); cudaFree(c->da_part); cudaFree(c->da_counter);
-    cudaFree(c->xb); cudaFree(c->xpart); cudaFree(c->d_err); cudaFreeHost(c->h_err);
+    cudaFree(c->xb); cudaFree(c->u16); cudaFree(c->h16); cudaFree(c->xpart); cudaFree(c->d_err); cudaFreeHost(c->h_err);
     cudaFree(c->d_step); cudaFree(c->d_arg); cudaFree(c->att_part); cudaFree(c->att_ml);
     cudaFreeHost(c->h_step); cudaFreeHost(c->h_logits); cudaFreeHost(c->h_arg);
     if (c->ev0) { cudaEventDestroy(c->ev0); cudaEventDestroy(c->ev1); }
@@ -2660,7 +2751,8 @@ StackCtx * stack_ctx_new(StackModel * m, int n_ctx) {
         fl(&c->rec, m->rec_floats);
         if (m->dtype == STACK_BF16) {
             c->xb_elems = std::max(cap * (size_t) std::max({ 2 * m->E, m->maxA, m->maxOL, m->maxP, m->max_dense, m->side_dim }), moe_rows * (size_t) std::max(m->E, m->max_eff));
-            SCU(cudaMalloc(&c->xb, c->xb_elems * 2));
+            SCU(cudaMalloc(&c->xb, c->xb_elems * 2)); SCU(cudaMalloc(&c->u16, c->xb_elems * 2));
+            if (m->block == BLOCK_SHARED || m->block == BLOCK_SEQUENTIAL) SCU(cudaMalloc(&c->h16, cap * m->E * 2));
             c->xpart_floats = umma_part_floats(c->sm_count);
         } else c->xpart_floats = f32_part_floats(*m, c->cap, c->sm_count);
         if (c->xpart_floats) SCU(cudaMalloc(&c->xpart, c->xpart_floats * 4));

@@ -57,6 +57,14 @@ template <int VEC> __device__ __forceinline__ void st_chunk(float * p, const flo
     else p[0] = v[0];
 }
 
+// the same chunk rounded to bfloat16 (8-byte aligned rows for VEC = 4)
+template <int VEC> __device__ __forceinline__ void st_chunk16(__nv_bfloat16 * p, const float (&v)[VEC]) {
+    if constexpr (VEC == 4) {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+        *reinterpret_cast<uint2 *>(p) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+    } else p[0] = __float2bfloat16_rn(v[0]);
+}
+
 // what a step works on: written by the host (or by a memcpy node of the replayed decode graph) before the launches
 struct StepState {
     int32_t pos0;       // position of the step's first token within its sequence
@@ -77,7 +85,7 @@ constexpr int POST_NPL = 16;       // elements per lane that k_embed_rows and k_
 // ---- embedding fused with the first layer's input norm: X[t] = embed[token[t]], Hn[t] = norm(X[t]) * w ---------------------
 template <typename WT>
 __global__ void k_embed_rows(const WT * __restrict__ embed, const int32_t * tokens, int E, int n_vocab, float * X,
-                             const float * __restrict__ w, int groups, float eps, float * Hn) {
+                             const float * __restrict__ w, int groups, float eps, float * Hn, __nv_bfloat16 * H16) {
     pdl_enter();
     const int t = blockIdx.x;
     int tok = tokens[t];
@@ -95,19 +103,20 @@ __global__ void k_embed_rows(const WT * __restrict__ embed, const int32_t * toke
             ss = warp_sum(ss);
             const float r = 1.0f / sqrtf(ss / (float) gs + eps);
 #pragma unroll
-            for (int k = 0; k < POST_NPL; k++) { const int i = lane + 32 * k; if (i < gs) { X[b + i] = xv[k]; Hn[b + i] = xv[k] * r * wv[k]; } }
+            for (int k = 0; k < POST_NPL; k++) { const int i = lane + 32 * k; if (i < gs) { X[b + i] = xv[k]; const float h = xv[k] * r * wv[k]; Hn[b + i] = h; if (H16) H16[b + i] = __float2bfloat16_rn(h); } }
             continue;
         }
         for (int i = lane; i < gs; i += 32) X[b + i] = wf(e, (size_t) g * gs + i);
         __syncwarp();
         warp_group_norm(X + b, w + g * gs, gs, eps, Hn + b, lane);
+        if (H16) for (int i = lane; i < gs; i += 32) H16[b + i] = __float2bfloat16_rn(Hn[b + i]);      // each lane what it wrote
     }
 }
 
 // ---- end of a sub-layer, fused: X[t] += norm(Y[t]) * w_post, then (w_next != nullptr) Hn[t] = norm(X[t]) * w_next, the input
-// norm of the sub-layer that follows. Same groups for both; one block per row, one warp per group.
+// norm of the sub-layer that follows. Same groups for both; one block per row, one warp per group. H16 != nullptr: Hn rounded to bfloat16 as well, the operand of the products that follow.
 __global__ void k_post_norm_add(const float * Y, const float * __restrict__ w_post, float * X,
-                                const float * __restrict__ w_next, float * Hn, int n, int groups, float eps) {
+                                const float * __restrict__ w_next, float * Hn, int n, int groups, float eps, __nv_bfloat16 * H16) {
     const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, gs = n / groups;
     bool waited = false;
     for (int g = warp; g < groups; g += nw) {
@@ -144,7 +153,7 @@ __global__ void k_post_norm_add(const float * Y, const float * __restrict__ w_po
                 s2 = warp_sum(s2);
                 const float r2 = 1.0f / sqrtf(s2 / (float) gs + eps);
 #pragma unroll
-                for (int k = 0; k < POST_NPL; k++) { const int i = lane + 32 * k; if (i < gs) Hn[b + i] = xv[k] * r2 * wn[k]; }
+                for (int k = 0; k < POST_NPL; k++) { const int i = lane + 32 * k; if (i < gs) { const float h = xv[k] * r2 * wn[k]; Hn[b + i] = h; if (H16) H16[b + i] = __float2bfloat16_rn(h); } }
             }
             continue;
         }
@@ -158,7 +167,7 @@ __global__ void k_post_norm_add(const float * Y, const float * __restrict__ w_po
         if (w_next) {
             s2 = warp_sum(s2);
             const float r2 = 1.0f / sqrtf(s2 / (float) gs + eps);
-            for (int i = lane; i < gs; i += 32) Hn[b + i] = x[i] * r2 * w_next[g * gs + i];     // each lane re-reads what it wrote
+            for (int i = lane; i < gs; i += 32) { const float h = x[i] * r2 * w_next[g * gs + i]; Hn[b + i] = h; if (H16) H16[b + i] = __float2bfloat16_rn(h); }     // each lane re-reads what it wrote
         }
     }
     if (!waited) pdl_enter();      // (a warp without a group)
@@ -216,6 +225,7 @@ struct LinArgs {
     // z1 see_step + m / see_rows only. Positions are the columns (w_kn = 0: tiles beyond their rows' last one are left alone) or the inner
     // dimension (w_kn = 1: the sum ends with the tile's last one, rounded up to 4; what lies up to there counts)
     int see_rows = 0, see_pos = 0, see_step = 0;
+    __nv_bfloat16 * Yb = nullptr;     // k_gemm_bf16_pair: gated units go here, rounded to bfloat16 (the operand of the next product), and not to Y
     int rows_all = 0;   // k_gemm_f32_umma, > 0: rows of X and Y over all first-level entries of T each (the last one's may be fewer); others are neither read nor written
 };
 // the last position a tile of rows m0 .. m0 + rows - 1 sees

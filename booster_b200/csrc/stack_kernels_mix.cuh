@@ -113,6 +113,7 @@ struct PostJoinArgs {
     const float * Yk; const float * wt; const int32_t * sel; const int32_t * slot_of; int top, n_real; const float * Ysh; const float * sg;
     const float * fw; float * Hn;           // fw != nullptr: the model's norm
     float * scratch;
+    __nv_bfloat16 * H16 = nullptr;          // Hn rounded to bfloat16 as well
 };
 constexpr int POST_OWN = 2;
 template <int NV> __device__ __forceinline__ void block_sums(float (&v)[NV], float (*red)[32]) {
@@ -219,6 +220,7 @@ __global__ void __launch_bounds__(1024) k_post_join(const PostJoinArgs a) {
 #pragma unroll
         for (int e = 0; e < VEC; e++) x[e] = x[e] * f * w[e];
         st_chunk<VEC>(a.Hn + row + c * VEC, x);
+        if (a.H16) st_chunk16<VEC>(a.H16 + row + c * VEC, x);
     }
 }
 
@@ -612,6 +614,13 @@ __global__ void __launch_bounds__(1024) k_moe_sort(const int32_t * sel, int n_sl
     }
 }
 // Y[r] = X[src_row[r]]
+// rows of 16-bit entries: E a multiple of 8, 16-byte aligned
+__global__ void k_gather_rows16(const __nv_bfloat16 * X, const int32_t * src_row, int E, __nv_bfloat16 * Y) {
+    pdl_enter();
+    const uint4 * x = reinterpret_cast<const uint4 *>(X + (size_t) src_row[blockIdx.x] * E);
+    uint4 * y = reinterpret_cast<uint4 *>(Y + (size_t) blockIdx.x * E);
+    for (int i = threadIdx.x; i < E / 8; i += blockDim.x) y[i] = x[i];
+}
 __global__ void k_gather_rows(const float * X, int ldx, const int32_t * src_row, int E, float * Y) {
     pdl_enter();
     const int r = blockIdx.x;

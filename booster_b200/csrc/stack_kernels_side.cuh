@@ -16,7 +16,7 @@ namespace stk {
 struct PairTable { const void * w; unsigned long long mul_prev, mul_cur, buckets; };      // w == nullptr: no such table
 template <typename WT>
 __global__ void __launch_bounds__(1024) k_embed_pair(const WT * __restrict__ embed, PairTable pt, const StepState * st, const int32_t * tokens,
-                                                    int E, int n_vocab, const float * __restrict__ w, float eps, float * X, float * Hn) {
+                                                    int E, int n_vocab, const float * __restrict__ w, float eps, float * X, float * Hn, __nv_bfloat16 * H16) {
     pdl_enter();
     __shared__ float red[32];
     const int t = blockIdx.x, nt = blockDim.x;
@@ -33,7 +33,11 @@ __global__ void __launch_bounds__(1024) k_embed_pair(const WT * __restrict__ emb
     }
     ss = block_sum(ss, red);
     const float r = 1.0f / sqrtf(ss / (float) E + eps);
-    for (int i = threadIdx.x; i < E; i += nt) Hn[row + i] = X[row + i] * r * w[i];        // what this thread wrote
+    for (int i = threadIdx.x; i < E; i += nt) {           // what this thread wrote
+        const float h = X[row + i] * r * w[i];
+        Hn[row + i] = h;
+        if (H16) H16[row + i] = __float2bfloat16_rn(h);
+    }
 }
 
 // ---- end of two sub-layers that read the same input: X[t] += Ya[t] + Yb[t] + sum_k wt[t][k] Yk[slot(t, k)] (Yb, Yk may be absent; slot_of ==
@@ -44,6 +48,7 @@ struct SumArgs {
     const float * Ya; const float * Yb;
     const float * Yk; const float * wt; const int32_t * slot_of; int top;
     const float * nw; float * Hn;
+    __nv_bfloat16 * H16 = nullptr;          // Hn rounded to bfloat16 as well
 };
 constexpr int SUM_OWN = 2;
 template <int VEC> __device__ __forceinline__ void sum_chunk(const SumArgs & a, int t, int i, float (&x)[VEC]) {
@@ -102,6 +107,7 @@ __global__ void __launch_bounds__(1024) k_sum_join(const SumArgs a) {
 #pragma unroll
         for (int e = 0; e < VEC; e++) x[e] = x[e] * r * w[e];
         st_chunk<VEC>(a.Hn + row + i, x);
+        if (a.H16) st_chunk16<VEC>(a.H16 + row + i, x);
     };
 #pragma unroll
     for (int k = 0; k < SUM_OWN; k++) { const int c = threadIdx.x + k * nt; if (c < nchunk) finish(c * VEC, own[k]); }

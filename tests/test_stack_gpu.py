@@ -476,6 +476,41 @@ def test_one_token_products_in_a_pass(dtype, N, K, glu):
     assert (np.abs(y - ref) <= off).all(), np.nanmax(np.abs(y - ref) / off)
 
 
+@pytest.mark.parametrize("T,N,K,glu", [
+    (5, 128, 64, False), (31, 130, 72, True), (33, 256, 1032, False), (63, 1000, 2048, False), (96, 258, 128, True), (257, 600, 64, False), (256, 514, 200, True), (300, 3000, 520, False),
+    (513, 2056, 264, True), (600, 256, 4096, False), (1100, 140, 96, False), (7, 20000, 64, True)])
+def test_bfloat16_products_on_pairs_of_sms(T, N, K, glu):
+    """few tokens and many, tiles that end inside T, N and K, one accumulator and two, K parts, more tiles than pairs. Bound: test_products_where_their_rules_change; the tensor cores
+    add without rounding to nearest, which at worst doubles it"""
+    rng = np.random.default_rng(T + N + K)
+    x = rng.standard_normal((T, K)).astype(np.float32)
+    w = so.round_bf16((rng.standard_normal((N, K)) / np.sqrt(K)).astype(np.float32))
+    b = so.round_bf16(rng.standard_normal(N).astype(np.float32))
+    y = np.full((T, N // 2 if glu else N), np.nan, np.float32)
+    f32p = C.POINTER(C.c_float)
+    rc = _lib.lib().b200_stack_linear(0, 0, T, N, K, x.ctypes.data_as(f32p), w.ctypes.data_as(f32p), b.ctypes.data_as(f32p), int(glu), 7.0, y.ctypes.data_as(f32p))
+    assert rc == 0, _lib.last_error()
+    xe, we = so.round_bf16(x).astype(np.float64), w.astype(np.float64)
+    ref = xe @ we.T + b
+    off = 2 * (K + 8) * 2.0 ** -24 * (np.abs(xe) @ np.abs(we).T + np.abs(b))
+    if glu:
+        g, u = np.minimum(ref[:, 0::2], 7.0), np.clip(ref[:, 1::2], -7.0, 7.0)
+        ref = g * so.sigmoid(1.702 * g) * (u + 1.0)
+        off = 1.13 * np.abs(u + 1.0) * off[:, 0::2] + (np.abs(g) + 1.0) * off[:, 1::2] + 1e-5 * (1.0 + np.abs(ref))
+    assert (np.abs(y - ref) <= off).all(), np.nanmax(np.abs(y - ref) / off)
+
+
+@pytest.mark.parametrize("cuts", [None, [5, 33, 262], [64, 1, 235]], ids=str)
+def test_bfloat16_portions_hand_rounded_rows_on(tmp_path, cuts):
+    """a model wide enough for pairs of SMs: norms and gated units leave their rows rounded for the products behind them, in portions of few tokens and many"""
+    cfg = config([mingru(width=136, mlp=ff(192)), delta(heads=4, kv_heads=2, dim=32, vdim=32, mlp=ff(200)), latent(heads=4, dim=32, rot_dim=16, vdim=32, kv_rank=64, window=40, mlp=ff(128))], width=128, groups=4, vocab=160)
+    p = Pair(tmp_path, cfg, dtype="bfloat16")
+    toks = p.tokens(300, seed=2)
+    e = row_errs(p.run(toks, cuts), p.expected(toks))
+    assert np.median(e) < 3e-2 and e.max() < 0.25, (float(np.median(e)), float(e.max()))      # 2^-9 relative per product input, as test_bfloat16_prompt_kernels_and_decode
+    p.close()
+
+
 def test_float32_contexts_hold_no_room_for_products_they_never_run(tmp_path):
     """a float32 context has room for the K parts of its own model's products and no more (19 MB would hold any): sixteen small contexts stay well below what
     that alone would take, and a portion that is cut into parts decodes the oracle's rows"""
