@@ -10,7 +10,7 @@ OBJS := $(OBJDIR)/engine.o $(OBJDIR)/stack.o $(OBJDIR)/safetensors.o $(OBJDIR)/g
 
 all: $(LIB)
 
-$(OBJDIR)/engine.o: $(CSRC)/engine.cu $(CSRC)/kernels.cuh $(CSRC)/token_kernel.cuh $(CSRC)/matvec_q80.cuh $(CSRC)/matvec_kq.cuh $(CSRC)/prefill.cuh $(CSRC)/prefill_mma.cuh $(CSRC)/prefill_umma.cuh $(CSRC)/prefill_umma_q80.cuh $(CSRC)/gguf.hpp $(CSRC)/tokenizer.hpp $(CSRC)/stack.hpp $(CSRC)/safetensors.hpp include/booster_b200.h
+$(OBJDIR)/engine.o: $(CSRC)/engine.cu $(CSRC)/kernels.cuh $(CSRC)/token_kernel.cuh $(CSRC)/attn_cluster.cuh $(CSRC)/matvec_q80.cuh $(CSRC)/matvec_kq.cuh $(CSRC)/prefill.cuh $(CSRC)/prefill_mma.cuh $(CSRC)/prefill_umma.cuh $(CSRC)/prefill_umma_q80.cuh $(CSRC)/gguf.hpp $(CSRC)/tokenizer.hpp $(CSRC)/stack.hpp $(CSRC)/safetensors.hpp include/booster_b200.h
 	@mkdir -p $(OBJDIR)
 	$(NVCC) $(NVCCFLAGS) -c $< -o $@ 2> $(OBJDIR)/engine.ptxas.log || (cat $(OBJDIR)/engine.ptxas.log; false)
 

@@ -6,6 +6,7 @@
 // (token, pos) live in device memory (DecodeState) so the graph never needs re-instantiation.
 //
 //   per layer:  qkv    (k_matvec_kq, k_matvec_q80) [RMSNorm(attn_norm)+Q8_K quant] -> wq|wk|wv -> RoPE -> q (f32), K/V (f16 cache)
+//               k_attn_cluster     short contexts of 4 and 8 heads per key head: all of a layer's attention, a cluster per KV head; else
 //               k_attn_scores      raw K.q scores of the f16 cache (GQA group per CTA, 64 positions each)
 //               k_attn_softmax_pv  soft-max of the score rows + P.V -> kqv_merged_cont
 //               wo              [quant] -> wo -> + residual                          (ffn_inp)
@@ -24,6 +25,7 @@
 #define B200_TOKEN_KERNEL 1      // 0: build without the persistent per-token kernel (A/B: code size of the module)
 #endif
 #include "token_kernel.cuh"
+#include "attn_cluster.cuh"
 #include "matvec_q80.cuh"
 #include "matvec_kq.cuh"
 #include "prefill.cuh"
@@ -938,8 +940,8 @@ static bool launch_attention_2k(b200_ctx * c, const AttnArgs & a_in, int n_ctx_p
     return true;
 }
 
-// attention route: 0 = automatic (two launches when the GQA score rows fit one CTA's shared memory, else the
-// long-context three-kernel route), 1 = always the long-context route (tests keep both covered at every size)
+// attention route: 0 = automatic (one launch where that pays, else two when the GQA score rows fit one CTA's shared memory, else the long-context three-kernel route), 1 = always the
+// long-context route, 2 = two launches where they fit, 3 = one launch where it fits (tests keep all covered at every size)
 static int g_attn_route = 0;
 extern "C" void b200_set_attention_route(int route) { g_attn_route = route; }
 static bool attn_2k_enabled() {
@@ -948,8 +950,69 @@ static bool attn_2k_enabled() {
     return v == 1 && g_attn_route != 1;
 }
 
+// one launch (k_attn_cluster): a cluster of CL blocks per KV head, all clusters on the GPU at once. False where the context's scores and weights leave no room for a ring, or the
+// clusters do not fit beside one another
+template <int GQA, int CL>
+static bool launch_attention_cluster_as(b200_ctx * c, const AttnArgs & a_in, int n_ctx_pad) {
+    const int n16 = n_ctx_pad / 16, need = (ac_own(n16, CL) + AC_ROWS - 1) / AC_ROWS + (n16 * (16 / CL) + AC_ROWS - 1) / AC_ROWS + 1;
+    const size_t beside = ac_beside(GQA, CL, n16);
+    int stages = 0;
+    for (int s : AC_STAGES) if ((size_t) s * AC_STAGE + beside <= AC_SMEM) { stages = s; if (s >= need) break; }
+    if (stages < std::min(need, 4)) return false;
+    const size_t smem = (size_t) stages * AC_STAGE + beside;
+    auto kern = k_attn_cluster<GQA, CL>;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(CL, (unsigned) a_in.n_head_kv); cfg.blockDim = dim3(AC_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = c->st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    static size_t attr[64] = {0};
+    static int clusters[64] = {0};                             // at once, with the shared memory in attr
+    const int dv = c->device & 63;
+    {
+        std::lock_guard<std::mutex> attr_lock(g_attr_mu);
+        if (smem > attr[dv]) {
+            if (CL > 8) CU(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+            attr[dv] = smem;
+            if (cudaOccupancyMaxActiveClusters(&clusters[dv], kern, &cfg) != cudaSuccess) { cudaGetLastError(); clusters[dv] = 0; }
+        }
+        if (clusters[dv] < a_in.n_head_kv) return false;
+    }
+    AttnArgs a = a_in;
+    g_kind = KIND_ATTN; ProfScope ps(c);
+    a.trace = trace_slot(c, CL * a.n_head_kv);
+    if (pdl_enabled()) cfg.numAttrs = 2;
+    CU(cudaLaunchKernelEx(&cfg, kern, a, n16, stages));
+    c->launches += 1;
+    return true;
+}
+// Where the one launch is the faster one. Behind Q8_0's qkv, and with eight heads per key head, whose K-quant qkv fills the SMs as well, no block of k_attn_scores finds room before qkv
+// ends, and a second launch is 2.5 us a layer; blocks of a long context have more to do than half of the SMs do in that time. Tokens of one launch in parts of two launches' (B200; three file
+// types, at the end and at an eighth of contexts of 256 to 2048): eight heads per key head 0.93 to 1.01 up to 1536, 1.02 at 2048; four behind Q8_0 0.96 to 0.98 up to 1024, 1.00 at 1536;
+// four behind K-quants 0.99 to 1.00 up to 512 and 1.02 from 768 on; one and two heads 0.94 to 1.10.
+static bool attn_cluster_pays(const b200_ctx * c, int gqa, int n_ctx_pad) {
+    if (g_attn_route == 3) return true;
+    if (gqa == 8) return n_ctx_pad <= 1536;
+    return gqa == 4 && n_ctx_pad <= 1024 && c->m && !c->m->layers.empty() && c->m->layers[0].qkv.seg[0].type == T_Q8_0;
+}
+template <int GQA>
+static bool launch_attention_cluster(b200_ctx * c, const AttnArgs & a, int n_ctx_pad) {
+    if constexpr (GQA >= 4) {
+        if (g_attn_route == 2 || !attn_cluster_pays(c, GQA, n_ctx_pad)) return false;
+        const int heads = a.n_head_kv, sms = c->sm_count;
+        if (heads * 16 <= sms && launch_attention_cluster_as<GQA, 16>(c, a, n_ctx_pad)) return true;
+        return heads * 8 <= sms && launch_attention_cluster_as<GQA, 8>(c, a, n_ctx_pad);
+    }
+    return false;
+}
+
 template <int GQA>
 static void launch_attention_t(b200_ctx * c, const AttnArgs & a_in, int n_ctx_pad) {
+    if (attn_2k_enabled() && launch_attention_cluster<GQA>(c, a_in, n_ctx_pad)) return;
     if (attn_2k_enabled() && launch_attention_2k<GQA>(c, a_in, n_ctx_pad)) return;
     // long-context route (the GQA score rows do not fit one CTA's shared memory): scores, softmax, chunked P.V
     AttnArgs a = a_in;

@@ -325,7 +325,7 @@ def set_prefill_mma(mode: int) -> None:
 
 
 def set_attention_route(route: int) -> None:
-    """0: automatic (cluster kernel when it fits), 1: always the long-context three-kernel route"""
+    """0: automatic, 1: always the long-context three-kernel route, 2: two launches a layer where they fit, 3: one launch where it fits"""
     _lib.lib().b200_set_attention_route(route)
 
 

@@ -121,6 +121,18 @@ def test_attention_long_context_route_bit_exact(cfg, round_q):
         engine.set_attention_route(0)
 
 
+# one launch per layer, a cluster of 16 or 8 blocks per KV head, against the two launches: fewer vectors than blocks, stages that end inside, more stages than the ring has, contexts it leaves
+@pytest.mark.parametrize("cfg", [(4, 1, 1), (4, 1, 17), (8, 1, 33), (32, 8, 130), (32, 8, 333), (64, 8, 1029), (64, 16, 700), (16, 4, 2050), (128, 16, 300), (64, 8, 4200), (8, 1, 9000), (8, 2, 20011)])
+@pytest.mark.parametrize("round_q", [False, True])
+@pytest.mark.parametrize("route", [2, 3])
+def test_attention_routes_bit_exact(cfg, round_q, route):
+    engine.set_attention_route(route)
+    try:
+        _attention_case(cfg, round_q)
+    finally:
+        engine.set_attention_route(0)
+
+
 @pytest.mark.parametrize("cfg", [(2, 2, 50176), (2, 2, 12000), (4, 2, 25088), (8, 2, 12544), (8, 1, 6272), (8, 2, 7200), (2, 2, 14208), (2, 2, 11360), (2, 2, 11361)])
 def test_attention_where_v_goes_round_its_slots(cfg):
     """soft-max . V of one token: the longest context of each number of heads per key head (slots of 96 to 352 positions), and V that just fits its four slots and just does not"""
