@@ -249,6 +249,7 @@ struct StackCtx {
     const float * in = nullptr;           // what the mixer being enqueued reads ([T][E]) ...
     float * out = nullptr;                // ... and writes
     float * X = nullptr, * Hn = nullptr, * Y = nullptr, * P = nullptr, * A = nullptr, * QK = nullptr, * OL = nullptr, * CV = nullptr, * BG = nullptr, * O = nullptr;
+    bool token_step = false;              // the pass being enqueued is a token's step and no portion of a prompt
     float * rec = nullptr;                // recurrent slab
     std::vector<float *> caches;          // per run of an attention layer: [n_ctx][cache_row]
     StepDev * d_step = nullptr, * h_step = nullptr;
@@ -1737,8 +1738,9 @@ void mixer_latent(StackCtx * c, const LayerSpec & L, const RunSpec & Rn, int T) 
     const LatAttnArgs aa{c->QK, cache, L.sink, &c->d_step->st, c->OL, c->att_part, c->att_ml, T, H, rank, R, L.window, L.scale, ap.TQ, ap.HQ, ap.nsplit, ap.smax};
     const dim3 grid((unsigned) ((T + ap.TQ - 1) / ap.TQ), (unsigned) ((H + ap.HQ - 1) / ap.HQ), (unsigned) ap.nsplit);
     if (!ap.staged) pdl(c, grid, 256, ap.smem, k_latent_attn, aa);
-    else if (W % 4 == 0) pdl(c, grid, 256, ap.smem, k_latent_attn_staged<true>, aa);
-    else pdl(c, grid, 256, ap.smem, k_latent_attn_staged<false>, aa);
+    else if (W % 4 == 0 && ap.TQ * ap.HQ <= 4) pdl(c, grid, 256, ap.smem, k_latent_attn_staged<true, 4>, aa);
+    else if (W % 4 == 0) pdl(c, grid, 256, ap.smem, k_latent_attn_staged<true, LAT_NQ_MAX>, aa);
+    else pdl(c, grid, 256, ap.smem, k_latent_attn_staged<false, LAT_NQ_MAX>, aa);
     if (ap.nsplit > 1) { pdl(c, dim3((unsigned) T, (unsigned) H, (unsigned) ((rank + 63) / 64)), 256, 0, k_latent_combine, aa); c->launches++; }
     c->launches += 2;
     latent_values_out(c, L, T, ldp, gate_off);
@@ -2220,7 +2222,7 @@ void enqueue_layers_sequential(StackCtx * c, int T) {
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
         const RunSpec & R = m.runs[ri];
         const LayerSpec & L = m.layers[(size_t) R.layer];
-        const float * next_in = ri + 1 < m.runs.size() ? m.layers[(size_t) m.runs[ri + 1].layer].norm1 : nullptr;     // the final norm runs on the wanted rows only
+        const float * next_in = ri + 1 < m.runs.size() ? m.layers[(size_t) m.runs[ri + 1].layer].norm1 : c->token_step ? m.final_norm : nullptr;     // a portion's final norm runs on the wanted rows only
         run_mixer(c, L, R, T);                         // Hn holds norm1(x)
         post_norm_add(c, L.norm1b, L.has_mlp ? L.norm2 : next_in, T);
         if (L.has_mlp) {
@@ -2315,8 +2317,9 @@ void mixture_ff(StackCtx * c, const LayerSpec & L, const float * h, int T, const
         int tpe = 1;
         while (tpe * 2 * n <= 1024 && tpe * 2 <= slots) tpe *= 2;
         const size_t cnt_bytes = (size_t) n * tpe * 4;
-        const int in_smem = (size_t) slots * 4 + cnt_bytes <= 40 * 1024 ? 1 : 0;
-        pdl(c, 1, 1024, cnt_bytes + (in_smem ? (size_t) slots * 4 : 0), k_moe_sort, c->r_sel, slots, top, n, tpe, in_smem, c->r_seg, c->r_slot, c->r_src);
+        const size_t slot_bytes = (size_t) (slots + slots / 32) * 4;
+        const int in_smem = slot_bytes + cnt_bytes <= 40 * 1024 ? 1 : 0;
+        pdl(c, 1, 1024, cnt_bytes + (in_smem ? slot_bytes : 0), k_moe_sort, c->r_sel, slots, top, n, tpe, in_smem, c->r_seg, c->r_slot, c->r_src);
         if (L.scale_input) pdl(c, slots, 128, 0, k_spread_rows, h, E, c->r_slot, c->r_wt, top, E, c->Xp);
         else if (c->h16_on && h == c->Hn && E % 8 == 0 && pairs(c, slots, L.e_gateup, L.n_exp)) { pdl(c, slots, 128, 0, k_gather_rows16, c->h16, c->r_src, E, c->xb); o.x16 = c->xb; }
         else pdl(c, slots, 128, 0, k_gather_rows, h, E, c->r_src, E, c->Xp);
@@ -2585,8 +2588,9 @@ void enqueue_head(StackCtx * c, int n_rows, int64_t row_off, bool one_token = fa
         // the last join left the normed residual (the sum of the streams) in Hn for every row of the pass: the wanted rows are gathered for the head
         if (!one_token) { pdl(c, n_rows, 128, 0, k_gather_rows, c->Hn, m.E, c->d_step->rows, m.E, c->Y); c->launches++; hn = c->Y; }
     }
-    else if (m.dyt) { pdl(c, n_rows, 256, 0, k_dyt_rows, c->X, m.E, c->d_step->rows, DytW{m.final_norm, m.final_b, m.final_alpha}, m.E, c->Hn, m.E); c->launches++; }
-    else norm(c, c->X, m.E, c->d_step->rows, m.final_norm, m.E, m.groups, c->Hn, m.E, n_rows, false);
+    else if (one_token && m.block == BLOCK_SEQUENTIAL) {}      // the last layer left it in Hn
+    else if (m.dyt) { pdl(c, n_rows, 256, 0, k_dyt_rows, c->X, m.E, one_token ? nullptr : c->d_step->rows, DytW{m.final_norm, m.final_b, m.final_alpha}, m.E, c->Hn, m.E); c->launches++; }
+    else norm(c, c->X, m.E, one_token ? nullptr : c->d_step->rows, m.final_norm, m.E, m.groups, c->Hn, m.E, n_rows, false);
     linear(c, hn, m.E, m.head, c->d_logits + row_off * m.vocab, m.vocab, n_rows);
     if (m.softcap > 0.f) {
         const size_t n = (size_t) n_rows * m.vocab;
@@ -2617,10 +2621,11 @@ bool graph_enabled() {
 
 // one token: header in, layers, head, logits out — the body of the replayed graph and of its un-captured twin
 void enqueue_token_step(StackCtx * c) {
+    c->token_step = true;
     SCU(cudaMemcpyAsync(c->d_step, c->h_step, sizeof(StepState) + sizeof(int32_t), cudaMemcpyHostToDevice, c->st));
-    SCU(cudaMemsetAsync(c->d_step->rows, 0, sizeof(int32_t), c->st));      // the wanted row is the token itself (a prompt pass leaves its own rows here)
     enqueue_layers(c, 1);
     enqueue_head(c, 1, 0, true);
+    c->token_step = false;
     SCU(cudaMemcpyAsync(c->h_logits, c->d_logits, (size_t) c->m->vocab * 4, cudaMemcpyDeviceToHost, c->st));
 }
 
@@ -2692,7 +2697,7 @@ void stack_ctx_free(StackCtx * c) {
     for (float * p : { c->X, c->Hn, c->Y, c->P, c->A, c->QK, c->OL, c->CV, c->BG, c->O, c->rec, c->d_logits }) cudaFree(p);
     for (float * p : c->cache_allocs) cudaFree(p);
     cudaFree(c->att_scores); cudaFree(c->da_part); cudaFree(c->da_counter);
-    cudaFree(c->xb); cudaFree(c->u16); cudaFree(c->h16); cudaFree(c->xpart); cudaFree(c->d_err); cudaFreeHost(c->h_err);
+    cudaFree(c->xb); cudaFree(c->xpart); cudaFree(c->d_err); cudaFreeHost(c->h_err);
     cudaFree(c->d_step); cudaFree(c->d_arg); cudaFree(c->att_part); cudaFree(c->att_ml);
     cudaFreeHost(c->h_step); cudaFreeHost(c->h_logits); cudaFreeHost(c->h_arg);
     if (c->ev0) { cudaEventDestroy(c->ev0); cudaEventDestroy(c->ev1); }
@@ -2751,8 +2756,11 @@ StackCtx * stack_ctx_new(StackModel * m, int n_ctx) {
         fl(&c->rec, m->rec_floats);
         if (m->dtype == STACK_BF16) {
             c->xb_elems = std::max(cap * (size_t) std::max({ 2 * m->E, m->maxA, m->maxOL, m->maxP, m->max_dense, m->side_dim }), moe_rows * (size_t) std::max(m->E, m->max_eff));
-            SCU(cudaMalloc(&c->xb, c->xb_elems * 2)); SCU(cudaMalloc(&c->u16, c->xb_elems * 2));
-            if (m->block == BLOCK_SHARED || m->block == BLOCK_SEQUENTIAL) SCU(cudaMalloc(&c->h16, cap * m->E * 2));
+            c->xb_elems = (c->xb_elems + 63) / 64 * 64;
+            const bool norms = m->block == BLOCK_SHARED || m->block == BLOCK_SEQUENTIAL;
+            SCU(cudaMalloc(&c->xb, (2 * c->xb_elems + (norms ? cap * m->E : 0)) * 2));      // one allocation: a context is made per sequence
+            c->u16 = c->xb + c->xb_elems;
+            if (norms) c->h16 = c->u16 + c->xb_elems;
             c->xpart_floats = umma_part_floats(c->sm_count);
         } else c->xpart_floats = f32_part_floats(*m, c->cap, c->sm_count);
         if (c->xpart_floats) SCU(cudaMalloc(&c->xpart, c->xpart_floats * 4));
@@ -2817,10 +2825,11 @@ StackCtx * stack_ctx_new(StackModel * m, int n_ctx) {
         if (da_part) { fl(&c->da_part, da_part); fl((float **) &c->da_counter, da_cnt); }
         if (c->att_scores_floats) fl(&c->att_scores, c->att_scores_floats);
         if (smem > 48 * 1024) {
-            static size_t have_plain[64] = {0}, have_v[64] = {0}, have_s[64] = {0};
+            static size_t have_plain[64] = {0}, have_v[64] = {0}, have_v4[64] = {0}, have_s[64] = {0};
             raise_smem(k_latent_attn, smem, have_plain);
-            raise_smem(k_latent_attn_staged<true>, smem, have_v);
-            raise_smem(k_latent_attn_staged<false>, smem, have_s);
+            raise_smem(k_latent_attn_staged<true, LAT_NQ_MAX>, smem, have_v);
+            raise_smem(k_latent_attn_staged<true, 4>, smem, have_v4);
+            raise_smem(k_latent_attn_staged<false, LAT_NQ_MAX>, smem, have_s);
         }
         SCU(cudaMalloc(&c->d_step, sizeof(StepDev)));
         SCU(cudaMemsetAsync(c->d_step, 0, sizeof(StepDev), c->st));
@@ -2914,6 +2923,7 @@ void stack_decode(StackCtx * c, const int32_t * tokens, int n, int pos0, const i
             while (ri < n_rows && rows[ri] < i0 + T) c->h_step->rows[nr++] = rows[ri++] - i0;
             SCU(cudaMemcpyAsync(c->d_step, c->h_step, sizeof(StepState) + (size_t) T * 4, cudaMemcpyHostToDevice, c->st));
             if (nr) SCU(cudaMemcpyAsync(c->d_step->rows, c->h_step->rows, (size_t) nr * 4, cudaMemcpyHostToDevice, c->st));
+            c->token_step = false;               // (a capture that failed may have left it)
             enqueue_layers(c, T);
             if (nr) { enqueue_head(c, nr, row_off); row_off += nr; }
         }
@@ -2949,8 +2959,10 @@ void stack_generate_greedy(StackCtx * c, int32_t first_token, int pos0, int n_st
     SCU(cudaStreamSynchronize(c->st));
     c->h_step->st = StepState{pos0, 1, c->last_token}; c->h_step->tokens[0] = first_token;
     const auto body = [&]() {
+        c->token_step = true;
         enqueue_layers(c, 1);
         enqueue_head(c, 1, 0, true);
+        c->token_step = false;
         pdl(c, 1, 1024, 0, k_argmax_advance, c->d_logits, m.vocab, &c->d_step->st, c->d_step->tokens, c->d_out_tokens, c->d_counter);
         c->launches++;
     };
@@ -2969,7 +2981,6 @@ void stack_generate_greedy(StackCtx * c, int32_t first_token, int pos0, int n_st
         if (!ok) { cudaGetLastError(); c->graph_failed = true; stack_generate_greedy(c, first_token, pos0, n_steps, out_tokens); return; }
     }
     SCU(cudaMemcpyAsync(c->d_step, c->h_step, sizeof(StepState) + sizeof(int32_t), cudaMemcpyHostToDevice, c->st));
-    SCU(cudaMemsetAsync(c->d_step->rows, 0, sizeof(int32_t), c->st));
     SCU(cudaMemsetAsync(c->d_counter, 0, 4, c->st));
     SCU(cudaEventRecord(c->ev0, c->st));
     for (int i = 0; i < n_steps; i++) SCU(cudaGraphLaunch(c->g_greedy, c->st));

@@ -832,7 +832,7 @@ __global__ void __launch_bounds__(256) k_gemm_bf16_mma(const LinArgs a) {
 // tcgen05.mma (kind::f16, bf16 x bf16 -> f32) with the accumulator in tensor memory: D[128 tokens][256 rows of W] per CTA.
 //   operands   both K-major, tiles of K = 64 in the 128-byte swizzle: one TMA copy per operand and stage, four stages (zero-fill past T, N and K); the
 //              activations were rounded to bfloat16 by k_to_bf16 beforehand
-//   warp 0     one lane issues the copies (full[stage] by bytes), warp 1 one lane the MMAs, four K = 16 steps per stage; tcgen05.commit frees
+//   warp 0     issues the copies (full[stage] by bytes), warp 1 the MMAs, four K = 16 steps per stage; tcgen05.commit frees
 //              the stage (empty) and, after the last, the accumulator (done)
 //   epilogue   warp w owns TMEM lanes 32 (w & 3) .. + 31 (= tokens) and column half w >> 2: tcgen05.ld, bias / gated unit, stores
 // What bounds it: a tile moves 48 KB of L2 per 4.2 MFLOP. With 12 cp.async per thread and stage and a block-wide barrier per stage the copies were the
@@ -872,6 +872,23 @@ __device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity,
     atomicExch(err, 1);
     return false;
 }
+// one lane of a whole warp, always the same one. A warp that feeds copies or MMAs walks its loop as one, so that their operands stay in uniform registers; in a loop of lane 0 alone an
+// instruction costs its issuer 100 to 130 clocks (a slice of k_gemm_bf16_pair for 64 tokens: 960 clocks so, 520 as a warp, 400 with the copies on two warps).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// a wait within limits; nothing more once one has run out
+__device__ __forceinline__ void tc_wait(uint32_t bar, uint32_t parity, bool & dead) {
+    for (uint32_t spins = 0; !dead; spins++) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) break;
+        if (spins >= (1u << 22)) dead = true;
+    }
+}
+
 // maps: X as bf16 [xbatch][T][K] (box 64 x 128), W [batch][N][K] (box 64 x 256)
 __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const LinArgs a, int * err, int ksplit = 1, float * part = nullptr) {
     pdl_enter();
@@ -908,30 +925,32 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
     const int nk = (ksplit > 1 ? (int) ((long long) nk_all * (blockIdx.z + 1) / ksplit) : nk_all) - kbeg;       // at least one: ksplit <= nk_all
     if (warp == 0) {
         const int zx = a.seg ? 0 : bz;
-        if (lane == 0) {
-            for (int kt = 0; kt < nk; kt++) {
-                const int slot = kt % UM_STAGES;
-                if (kt >= UM_STAGES) mbar_wait_limited(smem_addr(&empty[slot]), (uint32_t) ((kt / UM_STAGES - 1) & 1), failed, err);
-                if (*failed) break;
+        bool dead = false;
+        int slot = 0, turn = 0;
+        for (int kt = 0; kt < nk; kt++) {
+            if (turn > 0) tc_wait(smem_addr(&empty[slot]), (uint32_t) ((turn - 1) & 1), dead);
+            if (elect_one() && !dead) {
                 const uint32_t sa = smem0 + (uint32_t) slot * UM_STAGE_BYTES, bar = smem_addr(&full[slot]);
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"((uint32_t) UM_STAGE_BYTES) : "memory");
                 tma_load_3d(sa, &map_x, (kbeg + kt) * UM_BK, r0 + m0, zx, bar);
                 tma_load_3d(sa + UM_A_BYTES, &map_w, (kbeg + kt) * UM_BK, n0, bz, bar);
             }
-            if (*failed) for (int i = 0; i < 1000; i++) __nanosleep(1000);      // copies under way land before the block ends
+            __syncwarp();
+            if (++slot == UM_STAGES) { slot = 0; turn++; }
         }
+        if (dead) { *failed = 1; atomicExch(err, 1); for (int i = 0; i < 1000; i++) __nanosleep(1000); }      // copies under way land before the block ends
         __syncwarp();
     } else if (warp == 1) {
         // instruction descriptor: D f32, A and B bf16, both K-major, N = 256, M = 128
         constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (UM_BN >> 3) << 17) | ((uint32_t) (UM_BM >> 4) << 24);
         // K-major, 128-byte swizzle: start >> 4 | 8-row group stride 1024 B >> 4 << 32 | version 1 | layout 2; a K = 16 step is 32 bytes along the row
         constexpr uint64_t DESC = ((uint64_t) 1 << 16) | ((uint64_t) (1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
-        if (lane == 0) {
-            for (int kt = 0; kt < nk; kt++) {
-                const int slot = kt % UM_STAGES;
-                mbar_wait_limited(smem_addr(&full[slot]), (uint32_t) ((kt / UM_STAGES) & 1), failed, err);
-                if (*failed) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        bool dead = false;
+        int slot = 0, turn = 0;
+        for (int kt = 0; kt < nk; kt++) {
+            tc_wait(smem_addr(&full[slot]), (uint32_t) (turn & 1), dead);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one() && !dead) {
                 const uint32_t sa = smem0 + (uint32_t) slot * UM_STAGE_BYTES, sb = sa + UM_A_BYTES;
 #pragma unroll
                 for (int ks = 0; ks < UM_BK / 16; ks++) {
@@ -941,10 +960,12 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
                                  :: "r"(tmem), "l"(da), "l"(db), "r"(IDESC), "r"(accumulate) : "memory");
                 }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_addr(&empty[slot])) : "memory");
+                if (kt == nk - 1) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_addr(&done)) : "memory");
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_addr(&done)) : "memory");
-            if (*failed) for (int i = 0; i < 1000; i++) __nanosleep(1000);      // MMAs under way end before tensor memory is given back
+            __syncwarp();
+            if (++slot == UM_STAGES) { slot = 0; turn++; }
         }
+        if (dead) { *failed = 1; atomicExch(err, 1); for (int i = 0; i < 1000; i++) __nanosleep(1000); }      // MMAs under way end before tensor memory is given back
         __syncwarp();
     }
     const bool ok = mbar_wait_limited(smem_addr(&done), 0u, failed, err) && !*failed;
@@ -1311,9 +1332,9 @@ __global__ void __launch_bounds__(256) k_latent_attn(const LatAttnArgs a) {
 // The same step for decode when a block's key slice fits shared memory: asynchronous copies bring the slice's cached rows in
 // all at once (no chain of dependent loads), and scores and weighted sum read them from there. One to eight lanes own a
 // (query, key) score; the weighted sum keeps k_latent_attn's ownership (LAT_RPT latent entries, all queries). VEC: rows are
-// whole 16-byte chunks (rank + R a multiple of 4); otherwise 4-byte copies. Rows are padded so that the keys of a warp fall
+// whole 16-byte chunks (rank + R a multiple of 4); otherwise 4-byte copies. NQM: 4 or LAT_NQ_MAX queries at most. Rows are padded so that the keys of a warp fall
 // into different banks. Same results layout (OL, or part / ml for k_latent_combine) as k_latent_attn.
-template <bool VEC>
+template <bool VEC, int NQM>
 __global__ void __launch_bounds__(256) k_latent_attn_staged(const LatAttnArgs a) {
     extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1424,9 +1445,9 @@ __global__ void __launch_bounds__(256) k_latent_attn_staged(const LatAttnArgs a)
     __syncthreads();
     // weighted sum of the latents: a thread owns LAT_RPT entries of the latent for all NQ queries
     for (int rb = 0; rb < a.rank; rb += 256 * LAT_RPT) {
-        float acc[LAT_NQ_MAX][LAT_RPT];
+        float acc[NQM][LAT_RPT];
 #pragma unroll
-        for (int qi = 0; qi < LAT_NQ_MAX; qi++)
+        for (int qi = 0; qi < NQM; qi++)
 #pragma unroll
             for (int k = 0; k < LAT_RPT; k++) acc[qi][k] = 0.f;
         for (int j = 0; j < nk; j++) {
@@ -1435,7 +1456,7 @@ __global__ void __launch_bounds__(256) k_latent_attn_staged(const LatAttnArgs a)
 #pragma unroll
             for (int k = 0; k < LAT_RPT; k++) cv[k] = rb + tid + 256 * k < a.rank ? c[256 * k] : 0.f;
 #pragma unroll
-            for (int qi = 0; qi < LAT_NQ_MAX; qi++) {
+            for (int qi = 0; qi < NQM; qi++) {
                 if (qi < NQ) {
                     const float w = s[(size_t) qi * a.smax + j];
 #pragma unroll
@@ -1444,7 +1465,7 @@ __global__ void __launch_bounds__(256) k_latent_attn_staged(const LatAttnArgs a)
             }
         }
 #pragma unroll
-        for (int qi = 0; qi < LAT_NQ_MAX; qi++) {
+        for (int qi = 0; qi < NQM; qi++) {
             if (qi >= NQ) continue;
             const int tq = qi / a.HQ, h = h0 + qi % a.HQ;
             if (tq >= nt || h >= a.H) continue;

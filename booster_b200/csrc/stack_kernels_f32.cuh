@@ -129,12 +129,12 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
         // instruction descriptor: D f32, A and B bf16, both K-major, N = 128, M = 128; operands K-major in the 128-byte swizzle (as in k_gemm_bf16_umma)
         constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (F3_BN >> 3) << 17) | ((uint32_t) (F3_BM >> 4) << 24);
         constexpr uint64_t DESC = ((uint64_t) 1 << 16) | ((uint64_t) (1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
-        if (lane == 0) {
-            for (int c = 0; c < nk; c++) {
-                const int s = c & 1;
-                mbar_wait_limited(smem_addr(&full[s]), (uint32_t) ((c >> 1) & 1), failed, err);
-                if (*failed) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        bool dead = false;
+        for (int c = 0; c < nk; c++) {
+            const int s = c & 1;
+            tc_wait(smem_addr(&full[s]), (uint32_t) ((c >> 1) & 1), dead);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one() && !dead) {
                 const uint32_t sx = smem0 + (uint32_t) s * F3_STAGE, sw = sx + 3 * F3_PLANE;
 #pragma unroll
                 for (int q = 0; q < 6; q++) {
@@ -149,8 +149,9 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
                 }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_addr(&done[s])) : "memory");
             }
-            if (*failed) for (int i = 0; i < 1000; i++) __nanosleep(1000);      // MMAs under way end before tensor memory is given back
+            __syncwarp();
         }
+        if (dead) { *failed = 1; atomicExch(err, 1); for (int i = 0; i < 1000; i++) __nanosleep(1000); }      // MMAs under way end before tensor memory is given back
         __syncwarp();
     } else {
         // ---- slices. Rows of X (and of W [N][K]): 16 threads a row, four rows a thread, 4 k each; a W [K][N]: a thread a column, 16 k

@@ -44,28 +44,11 @@ __device__ __forceinline__ void pair_commit(uint32_t bar) {       // to the barr
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" :: "r"(bar), "h"((uint16_t) 3) : "memory");
 }
 
-// one lane of a whole warp, always the same one. (The warp walks its loop as one: operands of copies and MMAs stay in uniform registers. A loop of lane 0 alone took 960 clocks a slice of
-// 64 tokens, copies and MMAs in one warp each; so and with the copies in two warps 400.)
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
 __device__ __forceinline__ void pair_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
                    "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr) : "memory");
 }
-// a wait within limits; nothing more once one has run out
-__device__ __forceinline__ void pair_wait(uint32_t bar, uint32_t parity, bool & dead) {
-    for (uint32_t spins = 0; !dead; spins++) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) break;
-        if (spins >= (1u << 22)) dead = true;
-    }
-}
-
 // a piece of work of a pair: rows of W from n0, tokens from t0 of those r0 .. r0 + T - 1, slices kb .. kb + nk - 1
 struct PairTile { int n0, t0, r0, T, z, part, kb, nk; };
 
@@ -162,7 +145,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) k_gem
             const PairTile t = tile(v);
             for (int kt = 0; kt < t.nk; kt++, it++) {
                 if (it >= ahead) {
-                    if (turn > 0) pair_wait(smem_addr(&empty[slot]), (uint32_t) ((turn - 1) & 1), dead);
+                    if (turn > 0) tc_wait(smem_addr(&empty[slot]), (uint32_t) ((turn - 1) & 1), dead);
                     load(t, kt, slot);
                 }
                 if (++slot == p.stages) { slot = 0; turn++; }
@@ -177,7 +160,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) k_gem
             const PairTile t = tile(v);
             const int half = (SEG ? columns(t, 0) : p.n) / 2, y = t.r0 + t.t0 + (int) rank * half;
             for (int kt = 0; kt < t.nk; kt++) {
-                if (turn > 0) pair_wait(smem_addr(&empty[slot]), (uint32_t) ((turn - 1) & 1), dead);
+                if (turn > 0) tc_wait(smem_addr(&empty[slot]), (uint32_t) ((turn - 1) & 1), dead);
                 if (elect_one() && !dead) {
                     const uint32_t dst = smem0 + (uint32_t) slot * stage_bytes + PG_W_BYTES, bar = bars + 8u * (uint32_t) slot;
                     const int k = (t.kb + kt) * PG_BK;
@@ -202,12 +185,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) k_gem
             for (int v = first; v < total; v += step, i++) {
                 const PairTile t = tile(v);
                 const int set = p.sets == 2 ? i & 1 : 0, round = p.sets == 2 ? i >> 1 : i;
-                if (round > 0) pair_wait(smem_addr(&acc_empty[set]), (uint32_t) ((round - 1) & 1), dead);
+                if (round > 0) tc_wait(smem_addr(&acc_empty[set]), (uint32_t) ((round - 1) & 1), dead);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d0 = tmem + (uint32_t) (set * ACC * p.n), idesc = IDESC | ((uint32_t) ((SEG ? columns(t, 0) : p.n) >> 3) << 17);
                 const bool second = ACC > 1 && columns(t, 1) > 0;
                 for (int kt = 0; kt < t.nk; kt++) {
-                    pair_wait(smem_addr(&full[slot]), (uint32_t) (turn & 1), dead);
+                    tc_wait(smem_addr(&full[slot]), (uint32_t) (turn & 1), dead);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (elect_one() && !dead) {
                         const uint64_t dw = DESC | (uint64_t) ((smem0 + (uint32_t) slot * stage_bytes) >> 4), dx = dw + (PG_W_BYTES >> 4);
