@@ -293,6 +293,7 @@ struct StackCtx {
     int tap_T = 0;
     int64_t launches = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_header = nullptr;      // the step's header has been copied
     float last_ms = 0.f;
 };
 
@@ -1749,7 +1750,8 @@ void mixer_latent(StackCtx * c, const LayerSpec & L, const RunSpec & Rn, int T) 
 // causal convolution of a portion's rows with the history a sequence keeps (k_causal_conv), then the history moves on
 void causal_conv(StackCtx * c, ConvArgs a, int batch = 1) {
     a.fuse_hist = a.T == 1 ? 1 : 0;
-    pdl(c, dim3((unsigned) ((a.C + 127) / 128), (unsigned) a.T, (unsigned) batch), 128, 0, k_causal_conv, a);
+    if (a.T > 1 && a.taps <= CONV_TAPS) pdl(c, dim3((unsigned) ((a.C + 127) / 128), (unsigned) ((a.T + CONV_TT - 1) / CONV_TT), (unsigned) batch), 128, 0, k_causal_conv_rows, a);
+    else pdl(c, dim3((unsigned) ((a.C + 127) / 128), (unsigned) a.T, (unsigned) batch), 128, 0, k_causal_conv, a);
     c->launches++;
     if (a.taps > 1 && !a.fuse_hist) { pdl(c, dim3((unsigned) ((a.C + 127) / 128), 1, (unsigned) batch), 128, 0, k_causal_conv_hist, a); c->launches++; }
 }
@@ -1759,7 +1761,7 @@ void mixer_delta(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     float * S = c->rec + R.off_rec, * hist = S + (size_t) H * D * V;
     linear(c, c->in, E, L.proj, c->P, ldp, T);
     causal_conv(c, ConvArgs{c->P, ldp, 0, L.wconv, 0, hist, 0, c->CV, C, 0, T, C, L.taps, 1, 0, nullptr, nullptr, 0, 0, 0});
-    pdl(c, T, 128, 0, k_delta_gates, c->CV, C, c->P, ldp, H, KH, D, V, L.A_log, L.dt_bias, c->BG);
+    pdl(c, T, T <= 16 ? 512 : 128, 0, k_delta_gates, c->CV, C, c->P, ldp, H, KH, D, V, L.A_log, L.dt_bias, c->BG);
     if (D <= 32) launch_delta_scan<32>(c, L, T, C, S);
     else if (D <= 64) launch_delta_scan<64>(c, L, T, C, S);
     else if (D <= 128) launch_delta_scan<128>(c, L, T, C, S);
@@ -2701,6 +2703,7 @@ void stack_ctx_free(StackCtx * c) {
     cudaFree(c->d_step); cudaFree(c->d_arg); cudaFree(c->att_part); cudaFree(c->att_ml);
     cudaFreeHost(c->h_step); cudaFreeHost(c->h_logits); cudaFreeHost(c->h_arg);
     if (c->ev0) { cudaEventDestroy(c->ev0); cudaEventDestroy(c->ev1); }
+    if (c->ev_header) cudaEventDestroy(c->ev_header);
     if (c->st) cudaStreamDestroy(c->st);
     delete c;
 }
@@ -2838,7 +2841,7 @@ StackCtx * stack_ctx_new(StackModel * m, int n_ctx) {
         SCU(cudaMalloc(&c->d_out_tokens, (size_t) (n_ctx + 1) * 4)); SCU(cudaMalloc(&c->d_counter, 4));
         SCU(cudaMalloc(&c->d_arg, 4));
         SCU(cudaMallocHost(&c->h_arg, 4));
-        SCU(cudaEventCreate(&c->ev0)); SCU(cudaEventCreate(&c->ev1));
+        SCU(cudaEventCreate(&c->ev0)); SCU(cudaEventCreate(&c->ev1)); SCU(cudaEventCreateWithFlags(&c->ev_header, cudaEventDisableTiming));
         ensure_logit_rows(c.get(), 16);
         SCU(cudaMemsetAsync(c->rec, 0, std::max<size_t>(m->rec_floats, 4) * 4, c->st));
         SCU(cudaStreamSynchronize(c->st));
@@ -2916,13 +2919,14 @@ void stack_decode(StackCtx * c, const int32_t * tokens, int n, int pos0, const i
         int ri = 0;
         for (int i0 = 0; i0 < n; i0 += c->cap) {
             const int T = std::min(c->cap, n - i0);
-            SCU(cudaStreamSynchronize(c->st));              // the pinned header is free again
+            if (i0 == 0) SCU(cudaStreamSynchronize(c->st)); else SCU(cudaEventSynchronize(c->ev_header));      // the pinned header is free again: a portion is enqueued while the one before runs
             c->h_step->st = StepState{pos0 + i0, T, i0 ? tokens[i0 - 1] : c->last_token};
             std::memcpy(c->h_step->tokens, tokens + i0, (size_t) T * 4);
             int nr = 0;
             while (ri < n_rows && rows[ri] < i0 + T) c->h_step->rows[nr++] = rows[ri++] - i0;
             SCU(cudaMemcpyAsync(c->d_step, c->h_step, sizeof(StepState) + (size_t) T * 4, cudaMemcpyHostToDevice, c->st));
             if (nr) SCU(cudaMemcpyAsync(c->d_step->rows, c->h_step->rows, (size_t) nr * 4, cudaMemcpyHostToDevice, c->st));
+            SCU(cudaEventRecord(c->ev_header, c->st));
             c->token_step = false;               // (a capture that failed may have left it)
             enqueue_layers(c, T);
             if (nr) { enqueue_head(c, nr, row_off); row_off += nr; }

@@ -1582,6 +1582,38 @@ __global__ void k_causal_conv(const ConvArgs a) {
         h[(size_t) (a.taps - 2) * a.C + c] = X[c];
     }
 }
+// The same for portions: a thread takes CONV_TT tokens of its channel, whose inputs it asks for together (512 tokens x 4096 channels x 4 taps with a token a thread, 16384 blocks: 18 us).
+constexpr int CONV_TT = 8, CONV_TAPS = 8;                     // tokens; taps at most
+__global__ void __launch_bounds__(128) k_causal_conv_rows(const ConvArgs a) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, t0 = blockIdx.y * CONV_TT, z = blockIdx.z;
+    const int cc = min(c, a.C - 1), first = CONV_TAPS - a.taps;
+    const float * w = a.w + (size_t) z * a.sW + (size_t) cc * a.taps;
+    float wv[CONV_TAPS];
+#pragma unroll
+    for (int m = 0; m < CONV_TAPS; m++) wv[m] = m >= first ? w[m - first] : 0.f;
+    const float b = a.bias ? a.bias[cc] : 0.f;
+    pdl_enter();
+    if (c >= a.C) return;
+    const float * X = a.X + (size_t) z * a.sX, * hist = a.hist + (size_t) z * a.sH;
+    float in[CONV_TT + CONV_TAPS - 1];                         // of tokens t0 - CONV_TAPS + 1 ..
+#pragma unroll
+    for (int j = 0; j < CONV_TT + CONV_TAPS - 1; j++) {
+        const int tau = t0 - (CONV_TAPS - 1) + j;
+        in[j] = j < first || tau >= a.T ? 0.f : tau >= 0 ? X[(size_t) tau * a.ldx + c] : hist[(size_t) (a.taps - 1 + tau) * a.C + c];
+    }
+#pragma unroll
+    for (int i = 0; i < CONV_TT; i++) {
+        const int t = t0 + i;
+        if (t >= a.T) break;
+        float y = b;
+#pragma unroll
+        for (int m = 0; m < CONV_TAPS; m++) if (m >= first) y = fmaf(wv[m], in[i + m], y);
+        if (a.add_input) y += in[i + CONV_TAPS - 1];
+        if (a.act == 1) y = siluf_(y);
+        if (a.cache && c >= a.split) a.cache[(size_t) (a.st->pos0 + t) * a.ldc + (c - a.split)] = y;
+        else a.Y[(size_t) z * a.sY + (size_t) t * a.ldy + c] = y;
+    }
+}
 // afterwards: the history becomes the last taps - 1 inputs of (history ++ portion)
 __global__ void k_causal_conv_hist(const ConvArgs a) {
     pdl_enter();
@@ -1598,17 +1630,21 @@ __global__ void k_causal_conv_hist(const ConvArgs a) {
 // beta = sigmoid(beta logit); decay g = exp(-exp(A_log) * softplus(decay input + dt_bias)). BG[t] = [ beta: H | g: H ].
 __global__ void k_delta_gates(float * CV, int C, const float * P, int ldp, int H, int KH, int D, int V,
                               const float * __restrict__ A_log, const float * __restrict__ dt_bias, float * BG) {
-    pdl_enter();
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     float * cv = CV + (size_t) t * C;
+    pdl_enter();
     for (int v = warp; v < 2 * KH; v += nw) {     // q heads, then k heads
         float * x = cv + (size_t) v * D;
-        float ss = 0.f;
-        for (int i = lane; i < D; i += 32) ss = fmaf(x[i], x[i], ss);
+        float e[8], ss = 0.f;                     // D <= 256
+#pragma unroll
+        for (int k = 0; k < 8; k++) e[k] = lane + 32 * k < D ? x[lane + 32 * k] : 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; k++) ss = fmaf(e[k], e[k], ss);
         ss = warp_sum(ss);
         float r = 1.0f / sqrtf(ss + 1e-6f);
         if (v < KH) r *= 1.0f / sqrtf((float) D);
-        for (int i = lane; i < D; i += 32) x[i] *= r;
+#pragma unroll
+        for (int k = 0; k < 8; k++) if (lane + 32 * k < D) x[lane + 32 * k] = e[k] * r;
     }
     const float * p = P + (size_t) t * ldp + 2 * KH * D + H * V;
     for (int h = threadIdx.x; h < H; h += blockDim.x) {
@@ -1736,6 +1772,24 @@ __global__ void k_delta_out(const float * O, const float * P, int ldp, int gate_
     for (int h = blockIdx.y * nw + warp; h < H; h += gridDim.y * nw) {
         const float * o = O + (size_t) t * H * V + (size_t) h * V;
         const float * gp = P + (size_t) t * ldp + gate_off + (size_t) h * V;
+        if (V <= 128) {                            // everything asked for at once
+            float ov[4], gv[4], wv[4], ss = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int i = lane + 32 * k;
+                ov[k] = i < V ? o[i] : 0.f; gv[k] = i < V ? gp[i] : 0.f; wv[k] = i < V && normw ? normw[(size_t) h * w_stride + i] : 1.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) ss = fmaf(ov[k], ov[k], ss);
+            ss = warp_sum(ss);
+            const float r = 1.0f / sqrtf(ss / (float) V + eps);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int i = lane + 32 * k;
+                if (i < V) A[(size_t) t * H * V + (size_t) h * V + i] = ov[k] * r * wv[k] * (gate_sigmoid ? sigmoidf_(gv[k]) : siluf_(gv[k]));
+            }
+            continue;
+        }
         float ss = 0.f;
         for (int i = lane; i < V; i += 32) ss = fmaf(o[i], o[i], ss);
         ss = warp_sum(ss);

@@ -305,6 +305,17 @@ def test_a_step_longer_than_one_pass(tmp_path):
     p.close()
 
 
+@pytest.mark.parametrize("taps", [2, 8, 9])
+def test_convolution_of_portions_at_the_edges_of_its_tiles(tmp_path, taps):
+    """eight tokens of a channel to a thread up to eight taps, a token a thread above; the heads' vectors of every length a block holds in registers and one that it does not"""
+    p = Pair(tmp_path, config([delta(heads=2, kv_heads=1, dim=33, vdim=128, conv=taps), delta(heads=3, kv_heads=3, dim=43, vdim=130, conv=taps)]), seed=taps)
+    toks = p.tokens(60, seed=taps)
+    want = p.expected(toks)
+    for cuts in (None, [7, 8, 9, 16, 17], [2, 3, 1]):
+        assert err(p.run(toks, cuts), want) < TOL32
+    p.close()
+
+
 def row_errs(got, want):
     got, want = np.asarray(got, np.float64), np.asarray(want, np.float64)
     d = got - want
