@@ -993,11 +993,15 @@ static bool launch_attention_cluster_as(b200_ctx * c, const AttnArgs & a_in, int
 // Where the one launch is the faster one. Behind Q8_0's qkv, and with eight heads per key head, whose K-quant qkv fills the SMs as well, no block of k_attn_scores finds room before qkv
 // ends, and a second launch is 2.5 us a layer; blocks of a long context have more to do than half of the SMs do in that time. Tokens of one launch in parts of two launches' (B200; three file
 // types, at the end and at an eighth of contexts of 256 to 2048): eight heads per key head 0.93 to 1.01 up to 1536, 1.02 at 2048; four behind Q8_0 0.96 to 0.98 up to 1024, 1.00 at 1536;
-// four behind K-quants 0.99 to 1.00 up to 512 and 1.02 from 768 on; one and two heads 0.94 to 1.10.
+// four behind K-quants 0.99 to 1.00 up to 512 and 1.02 from 768 on; one and two heads 0.94 to 1.10. Where qkv leaves SMs to k_attn_scores two launches are as fast or faster: four heads per
+// key head on 1, 2, 4 and 6 key heads (24, 48, 96 and 144 units of qkv's rows) behind Q8_0 1.00 to 1.02, 1.00 to 1.02, 0.99 to 1.02 and 0.96 to 1.00; eight on 1, 2 and 4 (40, 80 and 160)
+// 0.99 to 1.01, 0.93 to 1.00 and 0.92 to 0.98.
 static bool attn_cluster_pays(const b200_ctx * c, int gqa, int n_ctx_pad) {
     if (g_attn_route == 3) return true;
-    if (gqa == 8) return n_ctx_pad <= 1536;
-    return gqa == 4 && n_ctx_pad <= 1024 && c->m && !c->m->layers.empty() && c->m->layers[0].qkv.seg[0].type == T_Q8_0;
+    if (!c->m || c->m->layers.empty()) return false;
+    const auto & qkv = c->m->layers[0].qkv;                    // units of 32 rows, a block each while there are SMs
+    if (gqa == 8) return n_ctx_pad <= 1536 && qkv.n_units >= c->sm_count / 2;
+    return gqa == 4 && n_ctx_pad <= 1024 && qkv.seg[0].type == T_Q8_0 && qkv.n_units >= c->sm_count * 3 / 4;
 }
 template <int GQA>
 static bool launch_attention_cluster(b200_ctx * c, const AttnArgs & a, int n_ctx_pad) {
