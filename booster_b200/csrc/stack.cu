@@ -1409,6 +1409,10 @@ LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu
 // One token's product in a pass goes to k_gemv_ring where a row's 16-byte pieces fit a block's registers: four (bf16) or eight (float32) a lane. Longer rows, and products of rows that
 // are no multiple of 16 bytes, go where they go by themselves: lin_route's lines are those of cold products, whose first bytes nobody has asked for.
 bool ring_takes(int K) { return K <= 8192; }
+// Two to four tokens are as many layers of its grid, a token's blocks each (k_gemv's warps read every token's x again for each row). All of them read the weights at once, so that two
+// tokens of a large matrix, 16384 x 2048 and more, stay with k_gemv: a pass of two of Matulorn (width 2048, bf16, four layers) 399 us behind k_gemv, 376 with every product here, 332 with
+// the line between 34 and 65 MB; Bozisun 497, 490 and 450; float32 at width 1024 300 and 250. Three and four tokens 479 and 555 us behind k_gemv, 408 and 462 here (Bozisun 556, 659; 541, 650).
+bool ring_takes_tokens(int dtype, int T, int N, int K) { return T > 2 || (size_t) N * K * (dtype == STACK_F32 ? 4 : 2) < (size_t) 48 << 20; }
 template <typename WT, int TEAM, int CH>
 void launch_ring_as(const Lane & lane, const LinArgs & a, int batch, int sm_count) {
     constexpr int RS = gr_rows(CH) * (GR_THREADS / 32 / TEAM);
@@ -1501,7 +1505,10 @@ void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X
     a.vec = K % vecw == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % vecw == 0 && al16(X) && al16(W);
     if (launches) (*launches)++;
     const LinRoute route = lin_route(dtype, T, N, K, batch, a.vec != 0, a.glu != 0, a.seg != nullptr, us && us->err, (size_t) xbatch * T * K, us && us->xb ? us->elems : 0, us && us->part ? us->part_floats : 0, us ? us->sm_count : 148);
-    if (T == 1 && a.vec && lane.cold && ring_takes(K)) launch_ring(lane, a, dtype, batch, us ? us->sm_count : 148);
+    if (a.vec && lane.cold && ring_takes(K) && (T == 1 || (T <= GEMV_MAX_T && batch == 1 && !a.seg && !a.w_index && !a.x_scale && ring_takes_tokens(dtype, T, N, K)))) {
+        if (T > 1) { a.sX = ldx; a.sW = 0; a.sY = ldy; a.T = 1; }
+        launch_ring(lane, a, dtype, T > 1 ? T : batch, us ? us->sm_count : 148);
+    }
     else if (route == LIN_ROWS_X) {
         const int ch = gx_chunks(K / vecw);
         const dim3 grid((unsigned) ((N + GX_ROWS - 1) / GX_ROWS), 1, (unsigned) batch);

@@ -487,6 +487,28 @@ def test_one_token_products_in_a_pass(dtype, N, K, glu):
     assert (np.abs(y - ref) <= off).all(), np.nanmax(np.abs(y - ref) / off)
 
 
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("T,N,K,glu", [(2, 1, 8, False), (3, 149, 520, False), (4, 302, 1032, True), (2, 16001, 2048, False), (3, 16001, 2048, False), (2, 5000, 2048, True), (4, 150, 8192, False), (3, 40002, 64, True), (4, 37, 8200, False)])
+def test_products_of_few_tokens_in_a_pass(dtype, T, N, K, glu):
+    """the ring kernel with a token to each layer of its grid: fewer rows than blocks, several rounds, odd tokens; and rows that it leaves alone. Bound: test_products_where_their_rules_change"""
+    rng = np.random.default_rng(T + N + K)
+    x = rng.standard_normal((T, K)).astype(np.float32)
+    w = so.round_bf16((rng.standard_normal((N, K)) / np.sqrt(K)).astype(np.float32))
+    b = so.round_bf16(rng.standard_normal(N).astype(np.float32))
+    y = np.full((T, N // 2 if glu else N), np.nan, np.float32)
+    f32p = C.POINTER(C.c_float)
+    rc = _lib.lib().b200_stack_linear_in_pass(0, 0 if dtype == "bfloat16" else 1, T, N, K, x.ctypes.data_as(f32p), w.ctypes.data_as(f32p), b.ctypes.data_as(f32p), int(glu), 7.0, y.ctypes.data_as(f32p))
+    assert rc == 0, _lib.last_error()
+    xe, we = x.astype(np.float64), w.astype(np.float64)
+    ref = xe @ we.T + b
+    off = (K + 8) * 2.0 ** -24 * (np.abs(xe) @ np.abs(we).T + np.abs(b))
+    if glu:
+        g, u = np.minimum(ref[:, 0::2], 7.0), np.clip(ref[:, 1::2], -7.0, 7.0)
+        ref = g * so.sigmoid(1.702 * g) * (u + 1.0)
+        off = 1.13 * np.abs(u + 1.0) * off[:, 0::2] + (np.abs(g) + 1.0) * off[:, 1::2] + 1e-5 * (1.0 + np.abs(ref))
+    assert (np.abs(y - ref) <= off).all(), np.nanmax(np.abs(y - ref) / off)
+
+
 @pytest.mark.parametrize("T,N,K,glu", [
     (5, 128, 64, False), (31, 130, 72, True), (33, 256, 1032, False), (63, 1000, 2048, False), (96, 258, 128, True), (257, 600, 64, False), (256, 514, 200, True), (300, 3000, 520, False),
     (513, 2056, 264, True), (600, 256, 4096, False), (1100, 140, 96, False), (7, 20000, 64, True)])
