@@ -2290,6 +2290,11 @@ extern "C" int b200_stack_linear_in_pass(int device, int dtype, int T, int N, in
         return 0;
     } catch (const std::exception & e) { cudaGetLastError(); return set_err(e.what()); }
 }
+extern "C" int b200_stack_latent_plan(int heads, int rank, int rot, int window, int n_ctx, int T, int sm_count, int32_t * out) {
+    if (heads <= 0 || rank <= 0 || rot < 0 || window < 0 || n_ctx <= 0 || T <= 0 || sm_count <= 0 || !out) return set_err("bad arguments");
+    b200::stack_latent_plan(heads, rank, rot, window, n_ctx, T, sm_count, out);
+    return 0;
+}
 extern "C" float b200_last_device_ms(const b200_ctx * c) { return c ? c->last_device_ms : 0.f; }
 
 // One token, un-graphed, with a CUDA-event pair around every launch on the engine's own stream:

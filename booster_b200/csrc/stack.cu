@@ -1645,7 +1645,7 @@ AttnPlan plan_attention(const LayerSpec & L, int n_ctx, int T, int sm_count) {
         p.HQ = std::min(L.H, std::max(1, LAT_NQ_MAX / p.TQ));
         int blocks = ((T + p.TQ - 1) / p.TQ) * ((L.H + p.HQ - 1) / p.HQ);
         const int WP = W % 4 == 0 ? W + 4 : (W | 1);
-        p.nsplit = std::max(1, std::min({ 2 * sm_count / blocks, (keys + 7) / 8, 64 }));
+        p.nsplit = std::max(1, std::min({ 2 * sm_count / blocks, (keys + 7) / 8, LAT_MAX_SPLIT }));
         while (blocks * p.nsplit < sm_count && p.HQ > 4) {      // SMs left idle: fewer heads per block (the rows come from L2 again)
             p.HQ = (p.HQ + 1) / 2;
             blocks = ((T + p.TQ - 1) / p.TQ) * ((L.H + p.HQ - 1) / p.HQ);
@@ -1653,8 +1653,8 @@ AttnPlan plan_attention(const LayerSpec & L, int n_ctx, int T, int sm_count) {
         for (;;) {
             p.smax = (keys + p.nsplit - 1) / p.nsplit;
             p.smem = ((size_t) p.TQ * p.HQ * (W + p.smax + 1) + (size_t) p.smax * WP + 8) * 4;
-            if (p.smem <= 160 * 1024 || p.nsplit >= 64) break;
-            p.nsplit = std::min(64, p.nsplit * 2);
+            if (p.smem <= 160 * 1024 || p.nsplit >= LAT_MAX_SPLIT) break;
+            p.nsplit = std::min(LAT_MAX_SPLIT, p.nsplit * 2);
         }
         if (p.smem <= 160 * 1024) return p;
     }
@@ -1663,14 +1663,17 @@ AttnPlan plan_attention(const LayerSpec & L, int n_ctx, int T, int sm_count) {
     if (T < 8) p.HQ = std::min(p.HQ, 4);
     const int blocks = ((T + p.TQ - 1) / p.TQ) * ((L.H + p.HQ - 1) / p.HQ);
     p.nsplit = 1;
-    if (blocks < sm_count) p.nsplit = std::max(1, std::min({ 2 * sm_count / blocks, (keys + 31) / 32, 64 }));
+    if (blocks < sm_count) p.nsplit = std::max(1, std::min({ 2 * sm_count / blocks, (keys + 31) / 32, LAT_MAX_SPLIT }));
     for (;;) {
         p.smax = (keys + p.nsplit - 1) / p.nsplit;
         p.smem = ((size_t) p.TQ * p.HQ * (W + p.smax + 1) + 8) * 4;
-        if (p.smem <= 200 * 1024 || p.nsplit >= 64) break;
-        p.nsplit *= 2;                    // slice the keys until the scores of a block fit
+        if (p.smem <= 200 * 1024 || p.nsplit >= LAT_MAX_SPLIT) break;
+        p.nsplit = std::min(LAT_MAX_SPLIT, p.nsplit * 2);      // slice the keys until the scores of a block fit
     }
-    while (p.smem > 200 * 1024 && p.HQ > 1) { p.HQ = (p.HQ + 1) / 2; p.smem = ((size_t) p.TQ * p.HQ * (W + p.smax + 1) + 8) * 4; }
+    while (p.smem > 200 * 1024 && p.TQ * p.HQ > 1) {           // then fewer heads, and at last fewer tokens, per block
+        (p.HQ > 1 ? p.HQ : p.TQ) = ((p.HQ > 1 ? p.HQ : p.TQ) + 1) / 2;
+        p.smem = ((size_t) p.TQ * p.HQ * (W + p.smax + 1) + 8) * 4;
+    }
     return p;
 }
 
@@ -3032,6 +3035,14 @@ int32_t stack_argmax(StackCtx * c) {
 
 int stack_product_kernel(int dtype, int T, int N, int K, bool glu, int sm_count) {
     return lin_route(dtype, T, N, K, 1, K % (dtype == STACK_F32 ? 4 : 8) == 0, glu, false, true, 0, 0, SIZE_MAX, sm_count);
+}
+
+void stack_latent_plan(int heads, int rank, int rot, int window, int n_ctx, int T, int sm_count, int32_t out[6]) {
+    LayerSpec L;
+    L.H = heads; L.rank = rank; L.R = rot; L.window = window;
+    const AttnPlan p = plan_attention(L, n_ctx, T, sm_count);
+    const int32_t v[6] = { p.TQ, p.HQ, p.nsplit, p.smax, (int32_t) std::min<size_t>(p.smem, INT32_MAX), p.staged ? 1 : 0 };
+    std::copy(v, v + 6, out);
 }
 
 float stack_time_linear(int device, int dtype, int T, int N, int K, int reps) {

@@ -59,4 +59,7 @@ int     stack_product_kernel(int dtype, int T, int N, int K, bool glu, int sm_co
 // through the kernel the family would pick for that shape (parity tests)
 void    stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y, bool in_pass = false);
 
+// launch shape of a latent layer's attention over a pass of T tokens: tokens and heads per block, key slices, score-row stride, shared memory, whether keys are staged (host arithmetic, tests)
+void    stack_latent_plan(int heads, int rank, int rot, int window, int n_ctx, int T, int sm_count, int32_t out[6]);
+
 }  // namespace b200

@@ -1225,6 +1225,7 @@ struct LatAttnArgs {
     int TQ, HQ, nsplit, smax;      // smax: score-row stride = the most keys one block can get
 };
 constexpr int LAT_NQ_MAX = 16, LAT_RPT = 2;
+constexpr int LAT_MAX_SPLIT = 64;      // key slices at most: what k_latent_combine's lanes read
 __global__ void __launch_bounds__(256) k_latent_attn(const LatAttnArgs a) {
     pdl_enter();
     extern __shared__ float sm[];
@@ -1487,12 +1488,12 @@ __global__ void __launch_bounds__(256) k_latent_combine(const LatAttnArgs a) {  
     const int t = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31;
     const size_t th = (size_t) t * a.H + h;
     const float * ml = a.ml + th * a.nsplit * 2;
-    __shared__ float wz[64];            // nsplit <= 64
+    __shared__ float wz[LAT_MAX_SPLIT];
     __shared__ float red[4][64];
     const int r = blockIdx.z * 64 + (threadIdx.x & 63), g = threadIdx.x >> 6;
-    float pv[16];
+    float pv[LAT_MAX_SPLIT / 4];
 #pragma unroll
-    for (int k = 0; k < 16; k++) { const int z = g + 4 * k; pv[k] = z < a.nsplit && r < a.rank ? a.part[(th * a.nsplit + z) * a.rank + r] : 0.f; }
+    for (int k = 0; k < LAT_MAX_SPLIT / 4; k++) { const int z = g + 4 * k; pv[k] = z < a.nsplit && r < a.rank ? a.part[(th * a.nsplit + z) * a.rank + r] : 0.f; }
     float m[2], l[2];
 #pragma unroll
     for (int k = 0; k < 2; k++) { const int z = lane + 32 * k; m[k] = z < a.nsplit ? ml[2 * z] : -INFINITY; l[k] = z < a.nsplit ? ml[2 * z + 1] : 0.f; }
@@ -1506,7 +1507,7 @@ __global__ void __launch_bounds__(256) k_latent_combine(const LatAttnArgs a) {  
     __syncthreads();
     float acc = 0.f;
 #pragma unroll
-    for (int k = 0; k < 16; k++) acc = fmaf(pv[k], wz[g + 4 * k], acc);       // (slices without keys, and none, have weight 0)
+    for (int k = 0; k < LAT_MAX_SPLIT / 4; k++) acc = fmaf(pv[k], wz[g + 4 * k], acc);       // (slices without keys, and none, have weight 0)
     red[g][threadIdx.x & 63] = acc;
     __syncthreads();
     if (g == 0 && r < a.rank) a.OL[th * a.rank + r] = (red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x]);

@@ -135,6 +135,9 @@ int b200_stack_product_kernel(int dtype, int T, int N, int K, int glu, int sm_co
 int b200_stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y);
 /* the same product as a model's pass launches it: one token's takes the kernel that asks for its rows ahead of the kernel in front of it, here the same product once more */
 int b200_stack_linear_in_pass(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y);
+/* launch shape of a latent-attention layer over a pass of T tokens (the decode kernels: T < 8): out = tokens per block, heads per block, key slices, score-row
+ * stride, bytes of shared memory, 1 where a block's keys are staged in it (host arithmetic, tests) */
+int b200_stack_latent_plan(int heads, int rank, int rot, int window, int n_ctx, int T, int sm_count, int32_t * out);
 /* number of kernels launched by this library's own code since the context was created */
 int64_t b200_kernel_launches(const b200_ctx * c);
 /* device time (CUDA events on the engine's stream) of the last b200_generate_greedy /

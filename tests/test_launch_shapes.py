@@ -123,6 +123,27 @@ def test_prompt_product_kernel(types, rows, k, T, want):
     assert _lib.lib().b200_op_prompt_kernel((C.c_int32 * len(types))(*types), len(types), rows // 32, k, T, 148) == want
 
 
+@pytest.mark.parametrize("heads", [1, 3, 4, 16, 32, 128])
+@pytest.mark.parametrize("rank,rot", [(32, 8), (256, 64), (512, 64), (1000, 3)])
+@pytest.mark.parametrize("window", [0, 1, 512, 8192])
+def test_latent_attention_plan(heads, rank, rot, window):
+    """what the kernels of a pass of few tokens assume: 16 queries a block and 64 key slices at most (k_latent_combine's lanes), slices and score rows that hold every key a tile can see,
+    and a block's shared memory. Contexts for which nothing fits are refused when they are made, each at every number of tokens alike: more tokens never need more than one"""
+    L, out = _lib.lib(), (C.c_int32 * 6)()
+    for n_ctx in (1, 31, 64, 512, 4096, 5000, 32768, 65536, 98304, 131072, 200000, 400000, 900000, 1000000):
+        for sm_count in (20, 132, 148):
+            one = None
+            for T in range(1, 8):
+                assert L.b200_stack_latent_plan(heads, rank, rot, window, n_ctx, T, sm_count, out) == 0
+                tq, hq, nsplit, smax, smem, staged = out
+                assert 1 <= tq <= min(T, 4) and 1 <= hq <= heads and tq * hq <= 16 and 1 <= nsplit <= 64, tuple(out)
+                keys = min(window + tq - 1, n_ctx) if window else n_ctx
+                assert smax * nsplit >= keys
+                if T == 1:
+                    one = smem <= 227 * 1024
+                assert (smem <= 227 * 1024) == one, (n_ctx, T, tuple(out))
+
+
 BF16, F32 = 0, 1
 
 

@@ -316,6 +316,15 @@ def test_convolution_of_portions_at_the_edges_of_its_tiles(tmp_path, taps):
     p.close()
 
 
+@pytest.mark.parametrize("heads,tokens", [(16, 7), (32, 3), (32, 4), (32, 7)])
+def test_few_tokens_a_step_in_the_longest_contexts(tmp_path, heads, tokens):
+    """an unmasked latent layer in a context whose score rows only fit a block in many key slices: every slice counts, the newest keys' among them, from one key to a slice to several"""
+    p = Pair(tmp_path, config([latent(heads=heads, dim=8, rot_dim=8, vdim=8, kv_rank=32, window=0)]), n_ctx=131072)
+    toks = p.tokens(50 + 20 * tokens)
+    assert err(p.run(toks, [50] + [tokens] * 20), p.expected(toks)) < TOL32
+    p.close()
+
+
 def row_errs(got, want):
     got, want = np.asarray(got, np.float64), np.asarray(want, np.float64)
     d = got - want
