@@ -879,6 +879,11 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
     return p != 0;
 }
+// the wait for a tcgen05.ld of 16 registers, with them as operands: nothing that uses them is moved in front of it
+__device__ __forceinline__ void tc_ld_ready(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                 "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]) :: "memory");
+}
 // a wait within limits; nothing more once one has run out
 __device__ __forceinline__ void tc_wait(uint32_t bar, uint32_t parity, bool & dead) {
     for (uint32_t spins = 0; !dead; spins++) {
@@ -978,14 +983,14 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
         float * Y = (ksplit > 1 ? part + (size_t) blockIdx.z * T * a.N : a.seg ? a.Y + (size_t) r0 * ldy : a.Y + (size_t) blockIdx.z * a.sY) + (size_t) m * ldy;
 #pragma unroll 1
         for (int c = 0; c < UM_BN / 2; c += 16) {
+            uint32_t r[16];
             float v[16];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                uint32_t r0, r1, r2, r3;
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(taddr + (uint32_t) (c + 4 * j)) : "memory");
-                v[4 * j] = __uint_as_float(r0); v[4 * j + 1] = __uint_as_float(r1); v[4 * j + 2] = __uint_as_float(r2); v[4 * j + 3] = __uint_as_float(r3);
-            }
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int j = 0; j < 16; j += 4)
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[j]), "=r"(r[j + 1]), "=r"(r[j + 2]), "=r"(r[j + 3]) : "r"(taddr + (uint32_t) (c + j)) : "memory");
+            tc_ld_ready(r);
+#pragma unroll
+            for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
             if (m < T) {
                 const int nb = n0 + cbase + c;
                 if (!a.glu && nb + 15 < a.N && (ldy & 3) == 0 && ((uintptr_t) (Y + nb) & 15) == 0) {       // whole 16-byte stores

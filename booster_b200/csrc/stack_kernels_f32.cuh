@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(F3_THREADS, 1) k_gemm_f32_umma(const LinArgs a
                 asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
                              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
                                "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(taddr + (uint32_t) (c & 1) * F3_BN + 16 * h) : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                tc_ld_ready(v);
 #pragma unroll
                 for (int j = 0; j < 16; j++) acc[16 * h + j] += __uint_as_float(v[j]);
             }

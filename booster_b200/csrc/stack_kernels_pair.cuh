@@ -243,7 +243,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) k_gem
 #pragma unroll 1
                 for (int j = lo; j < hi; j += 16) {
                     uint32_t r[16];
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    tc_ld_ready(next);
 #pragma unroll
                     for (int e = 0; e < 16; e++) r[e] = next[e];
                     if (j + 16 < hi) pair_ld16(taddr + (uint32_t) (j + 16), next);      // on its way while these are stored

@@ -54,6 +54,17 @@ def test_shared_memory_limits_are_kept_per_device(name):
     assert not once, once
 
 
+@pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("*.cuh")))
+def test_accumulators_are_read_behind_the_wait_for_them(name):
+    """tcgen05.ld returns before its registers hold anything: only what depends on tcgen05.wait::ld is safe from being moved in front of it. The wait has the registers as operands, or the
+    statement behind it has"""
+    text = "\n".join(_code(CSRC / name))
+    bad = [text[:m.start()].count("\n") + 1 for m in re.finditer(r"asm volatile\(\"tcgen05\.wait::ld[^;]*;\"([^;]*);", text)
+           if '"+r"' not in m.group(1) and "void tmem_ld_wait()" not in text[text.rfind("\n", 0, m.start()):m.start()]]
+    bad += [text[:m.start()].count("\n") + 1 for m in re.finditer(r"\btmem_ld_wait\(\);(\s*)(?!tmem_ld\d+_ready\()\S", text)]
+    assert not bad, bad
+
+
 @pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("stack_kernels*.cuh")))
 def test_stack_kernels_wait_for_the_kernel_before_them(name):
     """a pass's kernels become resident while the one before still runs: each waits before it reads what another wrote, and reads that coherently (no __ldg, no read-only pointer of
