@@ -2290,6 +2290,14 @@ extern "C" int b200_stack_linear_in_pass(int device, int dtype, int T, int N, in
         return 0;
     } catch (const std::exception & e) { cudaGetLastError(); return set_err(e.what()); }
 }
+extern "C" int b200_stack_products(int device, int dtype, int T, int N, int K, int batch, const int32_t * seg, const float * x, const float * w, int glu, float limit, int rounded, float * y) {
+    try {
+        require_gpu();
+        if (T <= 0 || N <= 0 || K <= 0 || batch <= 0 || !x || !w || !y || (dtype != 0 && dtype != 1) || glu < 0 || glu > 2 || (glu && N % 2)) throw std::runtime_error("bad arguments");
+        b200::stack_products(device, dtype, T, N, K, batch, seg, x, w, glu, limit, rounded != 0, y);
+        return 0;
+    } catch (const std::exception & e) { cudaGetLastError(); return set_err(e.what()); }
+}
 extern "C" int b200_stack_latent_plan(int heads, int rank, int rot, int window, int n_ctx, int T, int sm_count, int32_t * out) {
     if (heads <= 0 || rank <= 0 || rot < 0 || window < 0 || n_ctx <= 0 || T <= 0 || sm_count <= 0 || !out) return set_err("bad arguments");
     b200::stack_latent_plan(heads, rank, rot, window, n_ctx, T, sm_count, out);

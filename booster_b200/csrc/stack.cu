@@ -3078,36 +3078,70 @@ float stack_time_linear(int device, int dtype, int T, int N, int K, int reps) {
     return ms / (float) std::max(reps, 1);
 }
 
-void stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y, bool in_pass) {
+namespace {
+// products by themselves, on copies of the operands: y[batch][T][ny] = x[batch][T][K] w[batch][N][K]^T, or with seg the rows seg[z] .. seg[z + 1] - 1 of one x[T][K] on matrix z. What no kernel
+// stores is NaN. launches: how often (in_pass, as launches of a pass)
+void products(int device, int dtype, int T, int N, int K, int batch, const int32_t * seg, const float * x, const float * w, const float * bias, int glu, float limit, bool rounded, float * y, bool in_pass) {
     SCU(cudaSetDevice(device));
     StackModel tmp;                      // owns the device copies
     tmp.device = device; tmp.dtype = dtype;
     float * X = nullptr, * Y = nullptr;
+    int32_t * dseg = nullptr;
     UmmaScratch us;
     int herr = 0;
-    const int ny = glu ? N / 2 : N;
+    const int ny = glu ? N / 2 : N, planes = seg ? 1 : batch;
+    const size_t nx = (size_t) planes * T * K, n_out = (size_t) planes * T * ny;
+    const auto give_back = [&] {
+        cudaFree(X); cudaFree(Y); cudaFree(dseg); cudaFree(us.xb); cudaFree(us.part); cudaFree(us.err);
+        for (void * p : tmp.allocs) cudaFree(p);
+    };
     try {
-        const std::vector<float> wv(w, w + (size_t) N * K);
+        const std::vector<float> wv(w, w + (size_t) batch * N * K);
         std::vector<float> bv;
         if (bias) bv.assign(bias, bias + N);
-        const DMat d = up_mat(tmp, wv, N, K, bias ? &bv : nullptr);
-        SCU(cudaMalloc(&X, (size_t) T * K * 4)); SCU(cudaMalloc(&Y, (size_t) T * ny * 4));
-        SCU(cudaMemcpy(X, x, (size_t) T * K * 4, cudaMemcpyHostToDevice));
-        us.elems = (size_t) T * K;
+        const DMat d = up_mat(tmp, wv, N, K, bias ? &bv : nullptr, batch);
+        SCU(cudaMalloc(&X, nx * 4)); SCU(cudaMalloc(&Y, n_out * 4)); SCU(cudaMemset(Y, 0xff, n_out * 4));
+        SCU(cudaMemcpy(X, x, nx * 4, cudaMemcpyHostToDevice));
+        us.elems = nx;
         SCU(cudaMalloc(&us.xb, us.elems * 2)); us.part_floats = umma_part_floats(us.sm_count); SCU(cudaMalloc(&us.part, us.part_floats * 4)); SCU(cudaMalloc(&us.err, 4)); SCU(cudaMemset(us.err, 0, 4));
+        LinOpt o;
+        o.glu_kind = glu;
+        if (seg) {
+            SCU(cudaMalloc(&dseg, ((size_t) batch + 1) * 4)); SCU(cudaMemcpy(dseg, seg, ((size_t) batch + 1) * 4, cudaMemcpyHostToDevice));
+            o.seg = dseg;
+        }
+        if (rounded) {
+            const bool vec = K % 8 == 0;
+            if (!glu || dtype != STACK_BF16 || !(batch == 1 || seg) || !pair_takes(N, seg ? batch : 0) ||
+                lin_route(dtype, T, N, K, batch, vec, true, seg != nullptr, true, nx, us.elems, us.part_floats, us.sm_count) != LIN_UMMA) throw std::runtime_error("this product does not hand rounded units on");
+            o.y16 = reinterpret_cast<__nv_bfloat16 *>(Y);
+        }
         bool cold = true;
-        for (int i = 0; i < (in_pass ? 2 : 1); i++) linear_on(Lane{nullptr, in_pass ? &cold : nullptr}, dtype, nullptr, X, K, d.w, d.bias, Y, ny, T, N, K, 1, 0, 0, 0, glu != 0, limit, &us);
+        for (int i = 0; i < (in_pass ? 2 : 1); i++)
+            linear_on(Lane{nullptr, in_pass ? &cold : nullptr}, dtype, nullptr, X, K, d.w, d.bias, Y, ny, T, N, K, batch, seg ? 0 : (long long) T * K, (long long) N * K, (long long) T * ny, glu != 0, limit, &us, &o);
         SCU(cudaDeviceSynchronize());
-        SCU(cudaMemcpy(y, Y, (size_t) T * ny * 4, cudaMemcpyDeviceToHost));
+        if (rounded) {
+            std::vector<uint16_t> h(n_out);
+            SCU(cudaMemcpy(h.data(), Y, n_out * 2, cudaMemcpyDeviceToHost));
+            for (size_t i = 0; i < n_out; i++) { const uint32_t u = (uint32_t) h[i] << 16; std::memcpy(y + i, &u, 4); }
+        } else SCU(cudaMemcpy(y, Y, n_out * 4, cudaMemcpyDeviceToHost));
         SCU(cudaMemcpy(&herr, us.err, 4, cudaMemcpyDeviceToHost));
-    } catch (...) {
-        cudaFree(X); cudaFree(Y); cudaFree(us.xb); cudaFree(us.part); cudaFree(us.err);
-        for (void * p : tmp.allocs) cudaFree(p);
-        throw;
-    }
-    cudaFree(X); cudaFree(Y); cudaFree(us.xb); cudaFree(us.part); cudaFree(us.err);
-    for (void * p : tmp.allocs) cudaFree(p);
+    } catch (...) { give_back(); throw; }
+    give_back();
     if (herr) throw std::runtime_error("a tensor-core product gave up waiting for its pipeline");
+}
+}  // namespace
+
+void stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y, bool in_pass) {
+    products(device, dtype, T, N, K, 1, nullptr, x, w, bias, glu ? GLU_SIGMOID : GLU_NONE, limit, false, y, in_pass);
+}
+void stack_products(int device, int dtype, int T, int N, int K, int batch, const int32_t * seg, const float * x, const float * w, int glu, float limit, bool rounded, float * y) {
+    if (seg) {
+        if (T <= GEMV_MAX_T) throw std::runtime_error("few rows are not sorted by matrix");
+        for (int z = 0; z < batch; z++) if (seg[z] < 0 || seg[z] > seg[z + 1]) throw std::runtime_error("segments must not fall");
+        if (seg[0] != 0 || seg[batch] > T) throw std::runtime_error("segments must start at row 0 and end within the rows");
+    }
+    products(device, dtype, T, N, K, batch, seg, x, w, nullptr, glu, limit, rounded, y, false);
 }
 
 }  // namespace b200

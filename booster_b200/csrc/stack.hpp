@@ -59,6 +59,9 @@ int     stack_product_kernel(int dtype, int T, int N, int K, bool glu, int sm_co
 // through the kernel the family would pick for that shape (parity tests)
 void    stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y, bool in_pass = false);
 
+// a batch of such products, x[batch][T][K] on w[batch][N][K], or (seg: batch + 1 first rows) the rows of one x[T][K] sorted by matrix; glu: 1 clamped sigmoid units, 2 GELU units; rounded:
+// bfloat16 units as the pair kernel hands them to the product behind (an error where it does not take the product)
+void    stack_products(int device, int dtype, int T, int N, int K, int batch, const int32_t * seg, const float * x, const float * w, int glu, float limit, bool rounded, float * y);
 // launch shape of a latent layer's attention over a pass of T tokens: tokens and heads per block, key slices, score-row stride, shared memory, whether keys are staged (host arithmetic, tests)
 void    stack_latent_plan(int heads, int rank, int rot, int window, int n_ctx, int T, int sm_count, int32_t out[6]);
 

@@ -10,7 +10,7 @@
 //              one shuffle gives each lane one unit). They join K parts, segments and the tile after (a second set of accumulators where both fit 512 columns) to one loop
 // What bounds it: a pair's slice is 16 KB of W and 16 KB of X per block for 256 x 256 (1024 clocks of MMAs for 512 tokens: 47 bytes a clock and SM out of L2), and W itself from HBM.
 // Its predecessor for these shapes, one block per 128 tokens x 256 rows, read 94 bytes a clock and stored a token per lane, 4 bytes of each sector at a time for gated units.
-// Measured in a pass (B200, with and without the rounding of X that is now the norm's or the unit's): 512 x 16384 x 2048 gated 81 + 2.7 us then, 35 now; 512 x 2048 x 8192 18 + 4.5 + 3.7
+// Measured in a pass (B200, with and without the rounding of X that is now the norm's or the unit's): 512 x 16384 x 2048 gated 81 + 2.7 us then, 42 now (7 of them the units' exponentials and quotients, the same as every other product's); 512 x 2048 x 8192 18 + 4.5 + 3.7
 // (parts) and 17 + 3.1; 512 x 2048 x 2048 18 + 2.7 + 3.7 and 10 + 3.4; 2048 rows of 16 experts of 4096 x 2048 106 and 64 (268 MB of weights), 16 tokens x 2048 x 8192 by mma.sync 245, now
 // 23 by itself. The MMA loop is at the tensor cores' rate for 512 tokens (1020 clocks a slice); for 64 tokens a slice takes 400 clocks, half of them waits and votes between instructions.
 // Every wait on an mbarrier is bounded: on a timeout the block raises *err, skips what is left, and still meets its partner and frees its tensor memory.
@@ -52,12 +52,6 @@ __device__ __forceinline__ void pair_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 // a piece of work of a pair: rows of W from n0, tokens from t0 of those r0 .. r0 + T - 1, slices kb .. kb + nk - 1
 struct PairTile { int n0, t0, r0, T, z, part, kb, nk; };
 
-// a gated unit that is rounded to bfloat16 next: the exponential and the quotient may be a few units in their last place off (2^-20 of the unit at the clamps of a model; it is
-// rounded to 2^-9): an exact quotient is a call
-__device__ __forceinline__ float rounded_glu(float gate, float up, float limit, float alpha, float shift) {
-    const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
-    return __fdividef(g, 1.0f + __expf(-alpha * g)) * (u + shift);
-}
 // SEG: rows sorted by expert (one accumulator a tile). GLU: GLU_*; ROUND: its units go to Yb. map_x: X as bf16 [1][rows][K], box 64 x n / 2 (SEG: 64 x 32); map_w: W [batch][N][K], box 64 x 128
 template <bool SEG, int ACC, int GLU, bool ROUND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) k_gemm_bf16_pair(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
@@ -255,7 +249,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) k_gem
 #pragma unroll
                         for (int e = 0; e < 16; e += 2) {                      // (stores stand behind: between the units they would put them in a row)
                             const float mine = __uint_as_float(odd ? r[e + 1] : r[e]) + b, gate = odd ? u[e / 2] : mine, up = odd ? mine : u[e / 2];
-                            u[e / 2] = GLU == GLU_GELU ? gelu_tanhf_(gate) * up : ROUND ? rounded_glu(gate, up, a.limit, a.alpha, a.up_shift) : clamped_glu(gate, up, a.limit, a.alpha, a.up_shift);
+                            u[e / 2] = GLU == GLU_GELU ? gelu_tanhf_(gate) * up : clamped_glu(gate, up, a.limit, a.alpha, a.up_shift);
                         }
                         const size_t at = (size_t) (t.r0 + tok + odd) * ldy + (n >> 1);
                         const int most = in ? left - odd : 0;

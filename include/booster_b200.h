@@ -135,6 +135,10 @@ int b200_stack_product_kernel(int dtype, int T, int N, int K, int glu, int sm_co
 int b200_stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y);
 /* the same product as a model's pass launches it: one token's takes the kernel that asks for its rows ahead of the kernel in front of it, here the same product once more */
 int b200_stack_linear_in_pass(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y);
+/* a batch of products as a layer's heads run them, x[batch][T][K] on w[batch][N][K] -> y[batch][T][N], or as its experts do (seg: batch + 1 first rows, from 0): rows seg[z] to
+ * seg[z + 1] - 1 of x[T][K] on matrix z -> y[T][N]. glu: 1 clamped sigmoid units, 2 GELU units (y has N / 2 columns); rounded: the units as bfloat16, as the kernel on pairs of
+ * SMs hands them to the product behind it (an error where it does not take the product). Entries that no kernel stores are NaN */
+int b200_stack_products(int device, int dtype, int T, int N, int K, int batch, const int32_t * seg, const float * x, const float * w, int glu, float limit, int rounded, float * y);
 /* launch shape of a latent-attention layer over a pass of T tokens (the decode kernels: T < 8): out = tokens per block, heads per block, key slices, score-row
  * stride, bytes of shared memory, 1 where a block's keys are staged in it (host arithmetic, tests) */
 int b200_stack_latent_plan(int heads, int rank, int rot, int window, int n_ctx, int T, int sm_count, int32_t * out);

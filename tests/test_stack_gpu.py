@@ -542,6 +542,37 @@ def test_bfloat16_products_on_pairs_of_sms(T, N, K, glu):
     assert (np.abs(y - ref) <= off).all(), np.nanmax(np.abs(y - ref) / off)
 
 
+def run_products(x, w, seg=None, glu=0, limit=0.0, rounded=False):
+    """b200_stack_products: bfloat16 products of heads (x [batch][T][K]) or of rows sorted by matrix (x [T][K], seg)"""
+    i32p, f32p = C.POINTER(C.c_int32), C.POINTER(C.c_float)
+    batch, N, K = w.shape
+    T = x.shape[-2]
+    y = np.zeros(x.shape[:-1] + (N // 2 if glu else N,), np.float32)
+    s = None if seg is None else np.ascontiguousarray(seg, np.int32)
+    rc = _lib.lib().b200_stack_products(0, 0, T, N, K, batch, None if s is None else s.ctypes.data_as(i32p), x.ctypes.data_as(f32p), w.ctypes.data_as(f32p), glu, limit, int(rounded), y.ctypes.data_as(f32p))
+    assert rc == 0, _lib.last_error()
+    return y
+
+
+def sorted_rows(counts):
+    return np.concatenate([[0], np.cumsum(counts)])
+
+
+@pytest.mark.parametrize("counts,N,K,glu,limit", [
+    ([5], 256, 64, 1, 7.0), ([300], 514, 136, 1, np.inf), ([600], 1030, 520, 1, 3.0), ([70], 300, 2048, 2, 0.0),              # one matrix: few columns, one accumulator and two
+    ([0, 300, 7, 0, 33, 0], 512, 128, 1, np.inf), ([1, 2, 600], 258, 264, 1, 7.0), ([40, 0, 25], 320, 96, 2, 0.0)], ids=str)      # experts: empty ones, a second tile of tokens
+def test_gated_units_handed_on_are_the_units_rounded(counts, N, K, glu, limit):
+    """gates of every size, far beyond the clamps: what the product behind reads is the float32 unit of the same sums, rounded to bfloat16 once"""
+    rng = np.random.default_rng(sum(counts) + N + K)
+    x = (rng.standard_normal((sum(counts), K)) * rng.choice([0.05, 1.0, 40.0], size=(sum(counts), 1))).astype(np.float32)
+    w = so.round_bf16((rng.standard_normal((len(counts), N, K)) / np.sqrt(K)).astype(np.float32))
+    seg = sorted_rows(counts) if len(counts) > 1 else None
+    xs = x if seg is not None else x[None]
+    whole = run_products(xs, w, seg, glu, limit)
+    assert np.isfinite(whole).all()
+    assert np.array_equal(run_products(xs, w, seg, glu, limit, rounded=True), so.round_bf16(whole))
+
+
 @pytest.mark.parametrize("cuts", [None, [5, 33, 262], [64, 1, 235]], ids=str)
 def test_bfloat16_portions_hand_rounded_rows_on(tmp_path, cuts):
     """a model wide enough for pairs of SMs: norms and gated units leave their rows rounded for the products behind them, in portions of few tokens and many"""
