@@ -2298,6 +2298,11 @@ extern "C" int b200_stack_products(int device, int dtype, int T, int N, int K, i
         return 0;
     } catch (const std::exception & e) { cudaGetLastError(); return set_err(e.what()); }
 }
+extern "C" int b200_stack_product_plan(int dtype, int T, int N, int K, int batch, int seg, int glu, int sm_count, int32_t * out) {
+    if ((dtype != 0 && dtype != 1) || T <= 0 || N <= 0 || K <= 0 || batch <= 0 || sm_count <= 0 || !out || (glu && N % 2)) return set_err("bad arguments");
+    b200::stack_product_plan(dtype, T, N, K, batch, seg != 0, glu != 0, sm_count, out);
+    return 0;
+}
 extern "C" int b200_stack_latent_plan(int heads, int rank, int rot, int window, int n_ctx, int T, int sm_count, int32_t * out) {
     if (heads <= 0 || rank <= 0 || rot < 0 || window < 0 || n_ctx <= 0 || T <= 0 || sm_count <= 0 || !out) return set_err("bad arguments");
     b200::stack_latent_plan(heads, rank, rot, window, n_ctx, T, sm_count, out);

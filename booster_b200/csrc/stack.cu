@@ -1406,6 +1406,13 @@ LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu
     return dtype == STACK_BF16 && vec && mma_enabled() ? LIN_MMA : LIN_SIMT;
 }
 
+// whether tiles on the fp32 pipe start on empty SMs although they stand inside a pass. They are long chains of instructions with room for several of them on an SM: let in while the kernel
+// before still fills most SMs, the blocks of experts, of a grid of half the SMs and more, and of most of a tile's rows crowd on the first SMs that are free. Float32 passes at width 1024,
+// overlapped and so: of 6 to 12 tokens Rumurax 2.93 to 3.11 and 2.73 to 2.86 ms, Bozisun 4.42 to 4.70 and 4.17 to 4.41, Kogerax 3.83 to 4.08 and 3.73 to 3.89, the other designs within 1 %;
+// of 33 to 63 Rumurax 2.54 to 2.60 and 2.39 to 2.49, Tosevik 2.75 to 2.81 and 2.67 to 2.74, Kogerax 3.77 to 3.86 and 3.65 to 3.76, Matulorn 1 % less, Bozisun 1.4 and Dopilorn 0.8 % more.
+// Other grids of up to 32 tokens take 1 to 2 % longer so.
+bool simt_whole(bool seg, int T, int blocks, int sm_count) { return seg || 2 * blocks >= sm_count || (T > 32 && T < 64); }
+
 // One token's product in a pass goes to k_gemv_ring where a row's 16-byte pieces fit a block's registers: four (bf16) or eight (float32) a lane. Longer rows, and products of rows that
 // are no multiple of 16 bytes, go where they go by themselves: lin_route's lines are those of cold products, whose first bytes nobody has asked for.
 bool ring_takes(int K) { return K <= 8192; }
@@ -1567,6 +1574,7 @@ void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X
         pdl(lane, grid, 256, 0, k_gemm_bf16_mma, a);
     } else {
         const dim3 grid((unsigned) ((N + 63) / 64), (unsigned) ((T + 63) / 64), (unsigned) batch);
+        if (lane.cold && simt_whole(a.seg != nullptr, T, (int) (grid.x * grid.y * grid.z), us ? us->sm_count : 148)) *lane.cold = true;
         if (dtype == STACK_F32) pdl(lane, grid, 256, 0, k_gemm_simt<float>, a); else pdl(lane, grid, 256, 0, k_gemm_simt<__nv_bfloat16>, a);
     }
     SCU(cudaGetLastError());
@@ -2165,6 +2173,9 @@ void mixer_gqattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
         else if (RT == 4) { if (wide) pdl(c, grid, 256, smem, k_gqa_attn_group<4, 2>, a); else pdl(c, grid, 256, smem, k_gqa_attn_group<4, 1>, a); }
         else pdl(c, grid, 256, smem, k_gqa_attn_group<8, 1>, a);
         c->launches++;
+        // (this kernel has two blocks for every SM: the few blocks of a float32 product behind it would crowd on the first SMs that it leaves. Bozisun at width 1024, seven tokens at
+        // position 2000: 4.79 ms so and 4.36 whole)
+        if (T > GEMV_MAX_T && c->m->dtype == STACK_F32) c->cold = true;
         linear(c, c->A, H * V, L.o, c->out, E, T);
         return;
     }
@@ -3035,6 +3046,13 @@ int32_t stack_argmax(StackCtx * c) {
 
 int stack_product_kernel(int dtype, int T, int N, int K, bool glu, int sm_count) {
     return lin_route(dtype, T, N, K, 1, K % (dtype == STACK_F32 ? 4 : 8) == 0, glu, false, true, 0, 0, SIZE_MAX, sm_count);
+}
+
+void stack_product_plan(int dtype, int T, int N, int K, int batch, bool seg, bool glu, int sm_count, int32_t out[2]) {
+    const bool vec = K % (dtype == STACK_F32 ? 4 : 8) == 0;
+    const LinRoute route = lin_route(dtype, T, N, K, batch, vec, glu, seg, true, 0, 0, SIZE_MAX, sm_count);
+    out[0] = route;
+    out[1] = route == LIN_SIMT && simt_whole(seg, T, (N + 63) / 64 * ((T + 63) / 64) * batch, sm_count) ? 1 : 0;
 }
 
 void stack_latent_plan(int heads, int rank, int rot, int window, int n_ctx, int T, int sm_count, int32_t out[6]) {

@@ -163,3 +163,17 @@ def test_stack_product_kernel(dtype, T, N, K, glu, want):
     """which kernel a layer stack's product takes: 0 a warp per row, 1 a block per row, 2 a block per eight rows with x in registers, 3 tcgen05 (bfloat16), 4 and 7
     tcgen05 (float32) in K parts and whole, 5 mma.sync, 6 tiles on the fp32 pipe; the sizes on both sides of each line are among those measured"""
     assert _lib.lib().b200_stack_product_kernel(dtype, T, N, K, glu, 148) == want
+
+
+def product_plan(dtype, T, N, K, batch=1, seg=0, glu=0, sm_count=148):
+    out = (C.c_int32 * 2)()
+    assert _lib.lib().b200_stack_product_plan(dtype, T, N, K, batch, seg, glu, sm_count, out) == 0
+    return tuple(out)
+
+
+@pytest.mark.parametrize("dtype,T,N,K,batch,seg,glu,want", [
+    (F32, 24, 64, 1024, 16, 1, 0, 1), (F32, 24, 64, 1024, 2, 1, 1, 1),                                  # experts' rows, however few
+    (F32, 7, 4736, 1024, 1, 0, 0, 1), (F32, 7, 4672, 1024, 1, 0, 0, 0), (F32, 7, 64, 1024, 74, 0, 0, 1), (F32, 7, 64, 1024, 73, 0, 0, 0), (BF16, 7, 8192, 1020, 1, 0, 1, 1),      # 74 tiles of 64 rows
+    (F32, 32, 1024, 1024, 1, 0, 0, 0), (F32, 33, 1024, 1024, 1, 0, 0, 1), (F32, 63, 1024, 1024, 1, 0, 0, 1), (F32, 64, 63, 1024, 1, 0, 0, 0)])
+def test_large_grids_of_fp32_tiles_start_on_empty_sms(dtype, T, N, K, batch, seg, glu, want):
+    assert product_plan(dtype, T, N, K, batch, seg, glu) == (6, want)
