@@ -1398,7 +1398,10 @@ enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG, LIN_ROWS_X, LIN_UMMA, LIN_F32_PARTS
 LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu, bool seg, bool scratch, size_t x_elems, size_t xb_elems, size_t part_floats, int sm_count) {
     if (T == 1 && vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && gx_pays(dtype == STACK_F32, K / (dtype == STACK_F32 ? 4 : 8), N, batch, glu, sm_count)) return LIN_ROWS_X;
     if (T <= GEMV_MAX_T) return !glu && batch == 1 && N <= GEMV_FEW_ROWS && K >= 1024 ? LIN_ROWS_LONG : LIN_ROWS;      // few, long rows: a block each
-    if (dtype == STACK_BF16 && vec && umma_enabled() && K >= 64 && x_elems <= xb_elems && ((T >= 64 && N >= 128) || (N >= 256 && (batch == 1 || seg) && pair_takes(N, seg ? batch : 0)))) return LIN_UMMA;      // (few tokens: a pair's columns are as few; half a pair's rows stay with mma.sync)
+    // 5 to 63 tokens: a pair's columns are as few. Less than half of its rows, or than three slices of k, stay with mma.sync, which needs no rounding launch in front: 256 to 4096 rows of
+    // 5 to 63 tokens take 8.3 us there and 9.3 here at k = 64, 10.3 and 10.3 to 12.3 from 72 to 136, 12.3 and 11.5 at 192, 12.3 and 10 at 256
+    const bool few = K >= 3 * PG_BK && N >= PG_ROWS && (batch == 1 || seg) && pair_takes(N, seg ? batch : 0);
+    if (dtype == STACK_BF16 && vec && umma_enabled() && K >= 64 && x_elems <= xb_elems && ((T >= 64 && N >= 128) || few)) return LIN_UMMA;
     if (dtype == STACK_F32 && scratch && f32_umma_takes(vec, T, N, K)) {
         const int parts = batch == 1 && !glu && !seg ? f32_k_parts(T, N, K, sm_count) : 1;      // (a gated unit needs its sums whole)
         return parts > 1 && (size_t) parts * T * N <= part_floats ? LIN_F32_PARTS : LIN_F32_UMMA;

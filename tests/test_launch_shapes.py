@@ -177,3 +177,12 @@ def product_plan(dtype, T, N, K, batch=1, seg=0, glu=0, sm_count=148):
     (F32, 32, 1024, 1024, 1, 0, 0, 0), (F32, 33, 1024, 1024, 1, 0, 0, 1), (F32, 63, 1024, 1024, 1, 0, 0, 1), (F32, 64, 63, 1024, 1, 0, 0, 0)])
 def test_large_grids_of_fp32_tiles_start_on_empty_sms(dtype, T, N, K, batch, seg, glu, want):
     assert product_plan(dtype, T, N, K, batch, seg, glu) == (6, want)
+
+
+@pytest.mark.parametrize("T,N,K,batch,seg,want", [
+    (5, 256, 192, 1, 0, 3), (5, 256, 184, 1, 0, 5), (5, 255, 192, 1, 0, 5), (63, 256, 192, 1, 0, 3), (63, 4096, 64, 1, 0, 5), (63, 254, 4096, 1, 0, 5), (5, 256, 196, 1, 0, 6),
+    (5, 256, 192, 4, 1, 3), (63, 256, 192, 512, 1, 3), (63, 256, 192, 513, 1, 5), (63, 256, 192, 4, 0, 5),                       # experts, more of them than a block notes, heads
+    (64, 256, 64, 1, 0, 3), (64, 128, 64, 1, 0, 3), (64, 127, 64, 1, 0, 5), (64, 128, 64, 513, 1, 3), (64, 128, 64, 4, 0, 3), (64, 128, 56, 1, 0, 5)])
+def test_bfloat16_products_of_portions(T, N, K, batch, seg, want):
+    """few tokens go to the tensor memory from 256 rows and three slices of k on, 64 and more from 128 rows and one slice"""
+    assert product_plan(BF16, T, N, K, batch, seg)[0] == want

@@ -520,7 +520,8 @@ def test_products_of_few_tokens_in_a_pass(dtype, T, N, K, glu):
 
 @pytest.mark.parametrize("T,N,K,glu", [
     (5, 128, 64, False), (31, 130, 72, True), (33, 256, 1032, False), (63, 1000, 2048, False), (96, 258, 128, True), (257, 600, 64, False), (256, 514, 200, True), (300, 3000, 520, False),
-    (513, 2056, 264, True), (600, 256, 4096, False), (1100, 140, 96, False), (7, 20000, 64, True)])
+    (513, 2056, 264, True), (600, 256, 4096, False), (1100, 140, 96, False), (7, 20000, 64, True),
+    (5, 256, 192, False), (31, 386, 200, True), (7, 20000, 192, True)])
 def test_bfloat16_products_on_pairs_of_sms(T, N, K, glu):
     """few tokens and many, tiles that end inside T, N and K, one accumulator and two, K parts, more tiles than pairs. Bound: test_products_where_their_rules_change; the tensor cores
     add without rounding to nearest, which at worst doubles it"""
@@ -559,8 +560,8 @@ def sorted_rows(counts):
 
 
 @pytest.mark.parametrize("counts,N,K,glu,limit", [
-    ([5], 256, 64, 1, 7.0), ([300], 514, 136, 1, np.inf), ([600], 1030, 520, 1, 3.0), ([70], 300, 2048, 2, 0.0),              # one matrix: few columns, one accumulator and two
-    ([0, 300, 7, 0, 33, 0], 512, 128, 1, np.inf), ([1, 2, 600], 258, 264, 1, 7.0), ([40, 0, 25], 320, 96, 2, 0.0)], ids=str)      # experts: empty ones, a second tile of tokens
+    ([5], 256, 192, 1, 7.0), ([300], 514, 136, 1, np.inf), ([600], 1030, 520, 1, 3.0), ([70], 300, 2048, 2, 0.0),              # one matrix: few columns, one accumulator and two
+    ([0, 300, 7, 0, 33, 0], 512, 128, 1, np.inf), ([1, 2, 600], 258, 264, 1, 7.0), ([40, 0, 20], 320, 208, 2, 0.0)], ids=str)      # experts: empty ones, a second tile of tokens
 def test_gated_units_handed_on_are_the_units_rounded(counts, N, K, glu, limit):
     """gates of every size, far beyond the clamps: what the product behind reads is the float32 unit of the same sums, rounded to bfloat16 once"""
     rng = np.random.default_rng(sum(counts) + N + K)
