@@ -1305,7 +1305,6 @@ bool simt_big_enabled() {
     return on;
 }
 constexpr int GEMV_FEW_ROWS = 512;
-constexpr int GX_MIN_K = 1024;
 // what the tcgen05 product needs beside its operands: room for the activations rounded to bfloat16 and the error flag its
 // bounded waits raise
 struct UmmaScratch { __nv_bfloat16 * xb = nullptr; size_t elems = 0; int * err = nullptr; float * part = nullptr; size_t part_floats = 0; int sm_count = 148; };
@@ -1333,22 +1332,6 @@ size_t f32_part_floats(const StackModel & m, int cap, int sm_count) {
             if (parts > 1) most = std::max(most, (size_t) parts * T * nk.first);
         }
     return most;
-}
-// 16-byte chunks of a row that a lane of k_gemv_x takes: 1, 2 or 4 (0: the row is too long)
-int gx_chunks(int chunks) { return chunks <= GX_WARPS * 32 ? 1 : chunks <= 2 * GX_WARPS * 32 ? 2 : chunks <= 4 * GX_WARPS * 32 ? 4 : 0; }
-// one token: whether k_gemv_x is faster than k_gemv. A row has to fill most of a block's lanes (in sixteenths, by chunks per lane): 8192 x 1024 in bf16, half of them, takes 9.8 us
-// against 8.6, 2048 x 3072 (three quarters) 9.8 and 8.5, 2048 x 2048 6.2 and 6.2, 16000 x 2048 16.4 and 20.6. Of a gated unit, k_gemv's blocks hold sixteen rows and not eight, and waves decide: one
-// of its waves against two here loses (8192 x 4096 17.4 us with k_gemv, 18.9 here), two against two or three do not (10240 x 4096 0.77 of its time). With eight chunks a lane no row was
-// faster here (bf16 16000 x 16384: 179 us and 128). Measured: 514 to 28672 rows of 1024 to 16384 (float32: to 8192), cold.
-bool gx_pays(bool f32, int chunks, int N, int batch, bool glu, int sm_count) {
-    static const int plain[2][3] = {{12, 13, 13}, {12, 12, 15}}, resident[2][3] = {{8, 5, 4}, {7, 6, 5}};      // resident: blocks per SM, by their registers
-    const int ch = gx_chunks(chunks);
-    if (!ch) return false;
-    const int c = ch >> 1, full = ch * GX_WARPS * 32;
-    if (!glu) return 16 * chunks >= plain[f32][c] * full;
-    const auto waves = [&](int rows, int per_sm) { return ((long long) ((N + rows - 1) / rows) * batch + sm_count * per_sm - 1) / (sm_count * per_sm); };
-    const long long here = waves(GX_ROWS, resident[f32][c]), there = waves(16, 4);
-    return 2 * here <= 3 * there && 16 * chunks >= (here == 1 && ch > 1 ? 12 : 14) * full;
 }
 void launch_f32_umma(const Lane & lane, const LinArgs & a, int * err, int batch, int parts = 1, float * part = nullptr) {
     static size_t have[64] = {0};
@@ -1392,16 +1375,29 @@ PairPlan pair_plan(int T, int N, int K, int n_seg, bool parts_ok, int sm_count, 
     return best;
 }
 
+// One token's product goes to k_gemv_ring where a row's 16-byte pieces fit a block's registers: four (bf16) or eight (float32) a lane. Longer rows, and rows that are no multiple of 16
+// bytes, go to k_gemv.
+bool ring_takes(int K) { return K <= 8192; }
+// Two to four tokens are as many layers of its grid, a token's blocks each (k_gemv's warps read every token's x again for each row). All of them read the weights at once, so that two
+// tokens of a large matrix, 16384 x 2048 and more, stay with k_gemv: a pass of two of Matulorn (width 2048, bf16, four layers) 399 us behind k_gemv, 376 with every product here, 332 with
+// the line between 34 and 65 MB; Bozisun 497, 490 and 450; float32 at width 1024 300 and 250. Three and four tokens 479 and 555 us behind k_gemv, 408 and 462 here (Bozisun 556, 659; 541, 650).
+bool ring_takes_tokens(int dtype, int T, int N, int K) { return T > 2 || (size_t) N * K * (dtype == STACK_F32 ? 4 : 2) < (size_t) 48 << 20; }
+// pieces of work of a plan, at most (n_seg segments end inside their tiles of tokens)
+int pair_work(const PairPlan & p, int T, int N, int n_seg) {
+    const int row_tiles = (N + PG_ROWS - 1) / PG_ROWS;
+    return p.n_seg ? row_tiles * n_seg * ((T + 255) / 256) : row_tiles * ((T + p.acc * p.n - 1) / (p.acc * p.n)) * p.parts;
+}
+
 // the kernel a product goes to: mat-vecs of few tokens, then tile kernels
-enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG, LIN_ROWS_X, LIN_UMMA, LIN_F32_PARTS, LIN_MMA, LIN_SIMT, LIN_F32_UMMA };
-// vec: LinArgs::vec; scratch: whether there is any (an error flag); x_elems: entries of X; xb_elems, part_floats: what the scratch has room for
-LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu, bool seg, bool scratch, size_t x_elems, size_t xb_elems, size_t part_floats, int sm_count) {
-    if (T == 1 && vec && K >= GX_MIN_K && N > GEMV_FEW_ROWS && gx_pays(dtype == STACK_F32, K / (dtype == STACK_F32 ? 4 : 8), N, batch, glu, sm_count)) return LIN_ROWS_X;
+enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG = 1, LIN_RING = 2, LIN_UMMA = 3, LIN_F32_PARTS = 4, LIN_MMA = 5, LIN_SIMT = 6, LIN_F32_UMMA = 7, LIN_PAIR = 8 };
+// vec: LinArgs::vec; indexed: matrices or scales of the batch by index; scratch: whether there is any (an error flag); x_elems: entries of X; xb_elems, part_floats: what the scratch has room for
+LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu, bool seg, bool indexed, bool scratch, size_t x_elems, size_t xb_elems, size_t part_floats, int sm_count) {
+    if (vec && ring_takes(K) && (T == 1 || (T <= GEMV_MAX_T && batch == 1 && !seg && !indexed && ring_takes_tokens(dtype, T, N, K)))) return LIN_RING;
     if (T <= GEMV_MAX_T) return !glu && batch == 1 && N <= GEMV_FEW_ROWS && K >= 1024 ? LIN_ROWS_LONG : LIN_ROWS;      // few, long rows: a block each
     // 5 to 63 tokens: a pair's columns are as few. Less than half of its rows, or than three slices of k, stay with mma.sync, which needs no rounding launch in front: 256 to 4096 rows of
     // 5 to 63 tokens take 8.3 us there and 9.3 here at k = 64, 10.3 and 10.3 to 12.3 from 72 to 136, 12.3 and 11.5 at 192, 12.3 and 10 at 256
     const bool few = K >= 3 * PG_BK && N >= PG_ROWS && (batch == 1 || seg) && pair_takes(N, seg ? batch : 0);
-    if (dtype == STACK_BF16 && vec && umma_enabled() && K >= 64 && x_elems <= xb_elems && ((T >= 64 && N >= 128) || few)) return LIN_UMMA;
+    if (dtype == STACK_BF16 && vec && umma_enabled() && K >= 64 && x_elems <= xb_elems && ((T >= 64 && N >= 128) || few)) return (batch == 1 || seg) && pair_takes(N, seg ? batch : 0) ? LIN_PAIR : LIN_UMMA;
     if (dtype == STACK_F32 && scratch && f32_umma_takes(vec, T, N, K)) {
         const int parts = batch == 1 && !glu && !seg ? f32_k_parts(T, N, K, sm_count) : 1;      // (a gated unit needs its sums whole)
         return parts > 1 && (size_t) parts * T * N <= part_floats ? LIN_F32_PARTS : LIN_F32_UMMA;
@@ -1416,13 +1412,6 @@ LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu
 // Other grids of up to 32 tokens take 1 to 2 % longer so.
 bool simt_whole(bool seg, int T, int blocks, int sm_count) { return seg || 2 * blocks >= sm_count || (T > 32 && T < 64); }
 
-// One token's product in a pass goes to k_gemv_ring where a row's 16-byte pieces fit a block's registers: four (bf16) or eight (float32) a lane. Longer rows, and products of rows that
-// are no multiple of 16 bytes, go where they go by themselves: lin_route's lines are those of cold products, whose first bytes nobody has asked for.
-bool ring_takes(int K) { return K <= 8192; }
-// Two to four tokens are as many layers of its grid, a token's blocks each (k_gemv's warps read every token's x again for each row). All of them read the weights at once, so that two
-// tokens of a large matrix, 16384 x 2048 and more, stay with k_gemv: a pass of two of Matulorn (width 2048, bf16, four layers) 399 us behind k_gemv, 376 with every product here, 332 with
-// the line between 34 and 65 MB; Bozisun 497, 490 and 450; float32 at width 1024 300 and 250. Three and four tokens 479 and 555 us behind k_gemv, 408 and 462 here (Bozisun 556, 659; 541, 650).
-bool ring_takes_tokens(int dtype, int T, int N, int K) { return T > 2 || (size_t) N * K * (dtype == STACK_F32 ? 4 : 2) < (size_t) 48 << 20; }
 template <typename WT, int TEAM, int CH>
 void launch_ring_as(const Lane & lane, const LinArgs & a, int batch, int sm_count) {
     constexpr int RS = gr_rows(CH) * (GR_THREADS / 32 / TEAM);
@@ -1514,21 +1503,11 @@ void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X
     const auto al16 = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
     a.vec = K % vecw == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % vecw == 0 && al16(X) && al16(W);
     if (launches) (*launches)++;
-    const LinRoute route = lin_route(dtype, T, N, K, batch, a.vec != 0, a.glu != 0, a.seg != nullptr, us && us->err, (size_t) xbatch * T * K, us && us->xb ? us->elems : 0, us && us->part ? us->part_floats : 0, us ? us->sm_count : 148);
-    if (a.vec && lane.cold && ring_takes(K) && (T == 1 || (T <= GEMV_MAX_T && batch == 1 && !a.seg && !a.w_index && !a.x_scale && ring_takes_tokens(dtype, T, N, K)))) {
+    const LinRoute route = lin_route(dtype, T, N, K, batch, a.vec != 0, a.glu != 0, a.seg != nullptr, a.w_index || a.x_scale, us && us->err, (size_t) xbatch * T * K, us && us->xb ? us->elems : 0,
+                                     us && us->part ? us->part_floats : 0, us ? us->sm_count : 148);
+    if (route == LIN_RING) {
         if (T > 1) { a.sX = ldx; a.sW = 0; a.sY = ldy; a.T = 1; }
         launch_ring(lane, a, dtype, T > 1 ? T : batch, us ? us->sm_count : 148);
-    }
-    else if (route == LIN_ROWS_X) {
-        const int ch = gx_chunks(K / vecw);
-        const dim3 grid((unsigned) ((N + GX_ROWS - 1) / GX_ROWS), 1, (unsigned) batch);
-        const auto go = [&](auto wt) {
-            using WT = decltype(wt);
-            if (ch == 1) pdl(lane, grid, GX_WARPS * 32, 0, k_gemv_x<WT, 1>, a);
-            else if (ch == 2) pdl(lane, grid, GX_WARPS * 32, 0, k_gemv_x<WT, 2>, a);
-            else pdl(lane, grid, GX_WARPS * 32, 0, k_gemv_x<WT, 4>, a);
-        };
-        if (dtype == STACK_F32) go(0.f); else go(__nv_bfloat16());
     } else if (route == LIN_ROWS_LONG) {
         if (dtype == STACK_F32) pdl(lane, (unsigned) N, 256, 0, k_gemv<float, 1, 8>, a); else pdl(lane, (unsigned) N, 256, 0, k_gemv<__nv_bfloat16, 1, 8>, a);
     } else if (route == LIN_ROWS) {
@@ -1539,32 +1518,23 @@ void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X
             const dim3 grid((unsigned) ((N + 7) / 8), 1, (unsigned) batch);
             if (dtype == STACK_F32) pdl(lane, grid, 256, 0, k_gemv<float, 1>, a); else pdl(lane, grid, 256, 0, k_gemv<__nv_bfloat16, 1>, a);
         }
-    } else if (route == LIN_UMMA) {
+    } else if (route == LIN_UMMA || route == LIN_PAIR) {
         // tensor memory path: activations to bfloat16 once, then tcgen05.mma over TMA-fed stages (a.vec: rows and batch strides are multiples of 16 bytes)
-        static size_t have[64] = {0};
-        raise_smem(k_gemm_bf16_umma, UM_SMEM, have);
         const __nv_bfloat16 * x16 = opt && opt->x16 ? opt->x16 : us->xb;
-        if (x16 == us->xb && !(opt && opt->x16)) pdl(lane, dim3((unsigned) std::min<long long>(((long long) T * (K / 8) + 255) / 256, 2048), (unsigned) xbatch), 256, 0, k_to_bf16, X, ldx, T, K, sX, us->xb, (long long) T * K);
-        if ((batch == 1 || a.seg) && pair_takes(N, a.seg ? batch : 0)) {
+        if (!(opt && opt->x16))
+            pdl(lane, dim3((unsigned) std::min<long long>(((long long) T * (K / 8) + 255) / 256, 2048), (unsigned) xbatch), 256, 0, k_to_bf16, X, ldx, T, K, sX, us->xb, (long long) T * K);
+        if (launches) (*launches)++;
+        if (route == LIN_PAIR) {
             const PairPlan p = pair_plan(T, N, K, a.seg ? batch : 0, !a.glu && !a.seg && us->part && split_k_enabled(), us->sm_count, us->part_floats);
             const CUtensorMap mx = map_bf16(x16, K, T, 1, K, (long long) T * K, a.seg ? 32 : p.n / 2), mw = map_bf16(W, K, N, batch, K, sW, 128);
-            const int row_tiles = (N + PG_ROWS - 1) / PG_ROWS, work = a.seg ? row_tiles * batch * ((T + 255) / 256) : row_tiles * ((T + p.acc * p.n - 1) / (p.acc * p.n)) * p.parts;
-            launch_pair(lane, mx, mw, a, p, work, us->sm_count, us->err, us->part);
+            launch_pair(lane, mx, mw, a, p, pair_work(p, T, N, batch), us->sm_count, us->err, us->part);
             if (p.parts > 1) { split_sum(lane, us->part, p.parts, T, N, bias, Y, ldy); if (launches) (*launches)++; }
-            if (launches) (*launches)++;
-            return;
+        } else {
+            static size_t have[64] = {0};
+            raise_smem(k_gemm_bf16_umma, UM_SMEM, have);
+            const CUtensorMap mx = map_bf16(x16, K, T, xbatch, K, (long long) T * K, UM_BM), mw = map_bf16(W, K, N, batch, K, sW, UM_BN);
+            pdl(lane, dim3((unsigned) ((N + UM_BN - 1) / UM_BN), (unsigned) ((T + UM_BM - 1) / UM_BM), (unsigned) batch), 256, UM_SMEM, k_gemm_bf16_umma, mx, mw, a, us->err);
         }
-        const dim3 grid((unsigned) ((N + UM_BN - 1) / UM_BN), (unsigned) ((T + UM_BM - 1) / UM_BM), (unsigned) batch);
-        const CUtensorMap mx = map_bf16(x16, K, T, xbatch, K, (long long) T * K, UM_BM), mw = map_bf16(W, K, N, batch, K, sW, UM_BN);
-        const int tiles = (int) (grid.x * grid.y), nk = (K + UM_BK - 1) / UM_BK;
-        const int ksplit = batch == 1 && !a.glu && !a.seg && us->part && split_k_enabled() ? std::min(us->sm_count / tiles, nk / 4) : 1;
-        if (ksplit > 1) {
-            pdl(lane, dim3(grid.x, grid.y, (unsigned) ksplit), 256, UM_SMEM, k_gemm_bf16_umma, mx, mw, a, us->err, ksplit, us->part);
-            split_sum(lane, us->part, ksplit, T, N, bias, Y, ldy);
-            if (launches) (*launches)++;
-        }
-        else pdl(lane, grid, 256, UM_SMEM, k_gemm_bf16_umma, mx, mw, a, us->err, 1, nullptr);
-        if (launches) (*launches)++;
     } else if (route == LIN_F32_PARTS) {
         const int parts = f32_k_parts(T, N, K, us->sm_count);
         launch_f32_umma(lane, a, us->err, 1, parts, us->part);
@@ -1597,8 +1567,8 @@ void linear(StackCtx * c, const float * X, int ldx, const DMat & W, float * Y, i
 
 // whether a bfloat16 model's product of this pass goes to pairs of SMs (n_seg > 0: rows sorted by that many experts)
 bool pairs(const StackCtx * c, int T, const DMat & W, int n_seg = 0) {
-    return c->m->dtype == STACK_BF16 && W.K % 8 == 0 && pair_takes(W.N, n_seg) &&
-           lin_route(STACK_BF16, T, W.N, W.K, std::max(1, n_seg), true, false, n_seg > 0, true, (size_t) T * W.K, c->xb_elems, c->xpart_floats, c->sm_count) == LIN_UMMA;
+    return c->m->dtype == STACK_BF16 && W.K % 8 == 0 &&
+           lin_route(STACK_BF16, T, W.N, W.K, std::max(1, n_seg), true, false, n_seg > 0, false, true, (size_t) T * W.K, c->xb_elems, c->xpart_floats, c->sm_count) == LIN_PAIR;
 }
 // a feed-forward of gated units: F [T][ff] holds them, or u16 their rounded values where both products take those
 void gated_ff(StackCtx * c, const float * X, const DMat & gateup, float * F, const DMat & down, float * Y, int T, float limit, const LinOpt * opt = nullptr, int n_seg = 0) {
@@ -3048,12 +3018,13 @@ int32_t stack_argmax(StackCtx * c) {
 }
 
 int stack_product_kernel(int dtype, int T, int N, int K, bool glu, int sm_count) {
-    return lin_route(dtype, T, N, K, 1, K % (dtype == STACK_F32 ? 4 : 8) == 0, glu, false, true, 0, 0, SIZE_MAX, sm_count);
+    const LinRoute route = lin_route(dtype, T, N, K, 1, K % (dtype == STACK_F32 ? 4 : 8) == 0, glu, false, false, true, 0, 0, SIZE_MAX, sm_count);
+    return route == LIN_PAIR ? LIN_UMMA : route;
 }
 
 void stack_product_plan(int dtype, int T, int N, int K, int batch, bool seg, bool glu, int sm_count, int32_t out[2]) {
     const bool vec = K % (dtype == STACK_F32 ? 4 : 8) == 0;
-    const LinRoute route = lin_route(dtype, T, N, K, batch, vec, glu, seg, true, 0, 0, SIZE_MAX, sm_count);
+    const LinRoute route = lin_route(dtype, T, N, K, batch, vec, glu, seg, false, true, 0, 0, SIZE_MAX, sm_count);
     out[0] = route;
     out[1] = route == LIN_SIMT && simt_whole(seg, T, (N + 63) / 64 * ((T + 63) / 64) * batch, sm_count) ? 1 : 0;
 }
@@ -3082,10 +3053,11 @@ float stack_time_linear(int device, int dtype, int T, int N, int K, int reps) {
         us.elems = (size_t) T * K;
         SCU(cudaMalloc(&us.xb, us.elems * 2)); us.part_floats = umma_part_floats(us.sm_count); SCU(cudaMalloc(&us.part, us.part_floats * 4)); SCU(cudaMalloc(&us.err, 4)); SCU(cudaMemset(us.err, 0, 4));
         SCU(cudaStreamCreate(&st)); SCU(cudaEventCreate(&e0)); SCU(cudaEventCreate(&e1));
-        for (int i = 0; i < 3; i++) linear_on(Lane{st}, dtype, nullptr, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
+        bool cold = true;                // one behind the other, as a pass's kernels run
+        for (int i = 0; i < 3; i++) linear_on(Lane{st, &cold}, dtype, nullptr, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
         SCU(cudaStreamSynchronize(st));
         SCU(cudaEventRecord(e0, st));
-        for (int i = 0; i < reps; i++) linear_on(Lane{st}, dtype, nullptr, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
+        for (int i = 0; i < reps; i++) linear_on(Lane{st, &cold}, dtype, nullptr, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
         SCU(cudaEventRecord(e1, st));
         SCU(cudaStreamSynchronize(st));
         cudaEventElapsedTime(&ms, e0, e1);
@@ -3132,9 +3104,7 @@ void products(int device, int dtype, int T, int N, int K, int batch, const int32
             o.seg = dseg;
         }
         if (rounded) {
-            const bool vec = K % 8 == 0;
-            if (!glu || dtype != STACK_BF16 || !(batch == 1 || seg) || !pair_takes(N, seg ? batch : 0) ||
-                lin_route(dtype, T, N, K, batch, vec, true, seg != nullptr, true, nx, us.elems, us.part_floats, us.sm_count) != LIN_UMMA) throw std::runtime_error("this product does not hand rounded units on");
+            if (!glu || dtype != STACK_BF16 || lin_route(dtype, T, N, K, batch, K % 8 == 0, true, seg != nullptr, false, true, nx, us.elems, us.part_floats, us.sm_count) != LIN_PAIR) throw std::runtime_error("this product does not hand rounded units on");
             o.y16 = reinterpret_cast<__nv_bfloat16 *>(Y);
         }
         bool cold = true;

@@ -343,96 +343,11 @@ __global__ void __launch_bounds__(256) k_gemv(const LinArgs a) {
     }
 }
 
-// one token against long rows: a block = GX_ROWS rows, its 8 warps cut K among them, and a lane keeps its entries of x in registers for all rows.
-// k_gemv reads 32 bytes of x for every 16 bytes of a row, which makes the first-level cache its bound and leaves 2 KB of a row in flight per warp; here
-// nothing but weights is read in the loop, up to eight rows at a time. A warp's eight sums are folded by halving (9 shuffles), the
-// warps' parts added in order. CH: 16-byte chunks of a row per lane, K <= 8 x 32 x VEC x CH. bf16, cold rows: 16000 x 2048 20.6 us with
-// k_gemv, 16.4 here; 16384 x 2048 with the gated unit 18.4 and 16.5; 2048 x 8192 16.6 and 14.8. Where it does not pay: gx_pays.
-constexpr int GX_ROWS = 8, GX_WARPS = 8;
-template <typename WT, int CH>
-__global__ void __launch_bounds__(GX_WARPS * 32) k_gemv_x(const LinArgs a) {
-    pdl_enter();
-    constexpr int VEC = 16 / (int) sizeof(WT), RB = CH >= 4 ? 2 : CH == 2 ? 4 : 8;      // rows whose loads are in flight together
-    __shared__ float sums[GX_WARPS][GX_ROWS];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n0 = blockIdx.x * GX_ROWS;
-    const int wi = a.w_index ? a.w_index[blockIdx.z] : (int) blockIdx.z;
-    if (a.n_w > 0 && wi >= a.n_w) return;
-    const WT * w = reinterpret_cast<const WT *>(a.W) + (size_t) wi * a.sW + (size_t) n0 * a.K;
-    const float * x = a.X + (size_t) (blockIdx.z / a.x_share) * a.sX;
-    const int rows = min(GX_ROWS, a.N - n0);
-    float xv[CH][VEC];
-    bool on[CH];
-#pragma unroll
-    for (int c = 0; c < CH; c++) {
-        const int k = ((c * GX_WARPS + warp) * 32 + lane) * VEC;
-        on[c] = k < a.K;
-#pragma unroll
-        for (int i = 0; i < VEC; i += 4) {
-            const float4 f = on[c] ? *reinterpret_cast<const float4 *>(x + k + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-            xv[c][i] = f.x; xv[c][i + 1] = f.y; xv[c][i + 2] = f.z; xv[c][i + 3] = f.w;
-        }
-    }
-    float acc[GX_ROWS];
-#pragma unroll
-    for (int r0 = 0; r0 < GX_ROWS; r0 += RB) {
-        uint4 raw[RB][CH];
-#pragma unroll
-        for (int r = 0; r < RB; r++) {
-#pragma unroll
-            for (int c = 0; c < CH; c++)
-                raw[r][c] = (on[c] && r0 + r < rows) ? *reinterpret_cast<const uint4 *>(w + (size_t) (r0 + r) * a.K + ((c * GX_WARPS + warp) * 32 + lane) * VEC) : make_uint4(0u, 0u, 0u, 0u);
-        }
-#pragma unroll
-        for (int r = 0; r < RB; r++) {
-            float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-            for (int c = 0; c < CH; c++) {
-                const uint32_t uu[4] = { raw[r][c].x, raw[r][c].y, raw[r][c].z, raw[r][c].w };
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    if constexpr (sizeof(WT) == 2) {
-                        s0 = fmaf(__uint_as_float(uu[i] << 16), xv[c][2 * i], s0);
-                        s1 = fmaf(__uint_as_float(uu[i] & 0xffff0000u), xv[c][2 * i + 1], s1);
-                    } else if (i & 1) s1 = fmaf(__uint_as_float(uu[i]), xv[c][i], s1);
-                    else s0 = fmaf(__uint_as_float(uu[i]), xv[c][i], s0);
-                }
-            }
-            acc[r0 + r] = s0 + s1;
-        }
-    }
-    // fold eight sums over 32 lanes: each step sends half of the values to the other half of the lanes; lane 4 r (of eight groups) ends with row r
-#pragma unroll
-    for (int half = 4, off = 16; half >= 1; half >>= 1, off >>= 1) {
-        const bool up = lane & off;
-#pragma unroll
-        for (int i = 0; i < half; i++) {
-            const float keep = up ? acc[half + i] : acc[i], send = up ? acc[i] : acc[half + i];
-            acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-        }
-    }
-    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
-    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-    if ((lane & 3) == 0) sums[warp][lane >> 2] = acc[0];
-    __syncthreads();
-    if (threadIdx.x < GX_ROWS) {
-        const int r = threadIdx.x, n = n0 + r;
-        float v = 0.f;
-#pragma unroll
-        for (int i = 0; i < GX_WARPS; i++) v += sums[i][r];
-        if (n < a.N) v = v * (a.x_scale ? a.x_scale[blockIdx.z] : 1.0f) + (a.bias ? a.bias[n] : 0.f);
-        float * y = a.Y + (size_t) blockIdx.z * a.sY;
-        if (a.glu) {
-            const float up = __shfl_down_sync(0xffu, v, 1);
-            if (!(r & 1) && n + 1 < a.N) y[n >> 1] = gated_unit(a, v, up);
-        } else if (n < a.N) y[n] = v;
-    }
-}
-
-// one token's product inside a pass: a block has `rpb` consecutive rows, which its threads copy through a ring in shared memory (each its own 16-byte pieces: nobody else reads
-// them, so that no barrier stands between a copy and its use), and x in registers. The first GR_STAGES - 1 stages, up to 80 KB a block and 12 MB on the whole GPU, are asked for
+// one token's product: a block has `rpb` consecutive rows, which its threads copy through a ring in shared memory (each its own 16-byte pieces: nobody else reads
+// them, so that no barrier stands between a copy and its use), and x in registers. All stages of the ring but one (gr_stages), up to 80 KB a block and 12 MB on the whole GPU, are asked for
 // before pdl_wait(): memory is busy while the kernels in front of this one normalise, rotate or drain, and what a layer's smaller products need is there when x is.
 // One block per SM with everything in flight: a gated unit of 16384 x 2048 in bf16 takes 12.4 us of a token's time and the 2048 x 8192 behind it 6.6 (5.5 and 5.1 TB/s, the second's
-// first 12 MB read under the first), where k_gemv_x started cold took 16.5 and 14.8; 2048 x 2048 2.5 us and not 7.3. A token of Matulorn (width 2048, four layers) 340 us before, 226 now.
+// first 12 MB read under the first), where a kernel with x in registers that started cold took 16.5 and 14.8; 2048 x 2048 2.5 us and not 7.3. A token of Matulorn (width 2048, four layers) 340 us before, 226 now.
 // TEAM warps cut a row's K among them (8 / TEAM rows at a time), CH: 16-byte pieces of a row per lane, K <= TEAM x 32 x VEC x CH.
 constexpr int GR_THREADS = 256, GR_PIECES = 24;                // pieces of a thread's in the ring
 __host__ __device__ constexpr int gr_rows(int ch) { return ch >= 4 ? 1 : 4 / ch; }                       // a team's rows per stage
@@ -837,8 +752,7 @@ __global__ void __launch_bounds__(256) k_gemm_bf16_mma(const LinArgs a) {
 //   epilogue   warp w owns TMEM lanes 32 (w & 3) .. + 31 (= tokens) and column half w >> 2: tcgen05.ld, bias / gated unit, stores
 // What bounds it: a tile moves 48 KB of L2 per 4.2 MFLOP. With 12 cp.async per thread and stage and a block-wide barrier per stage the copies were the
 // bound; 512 x 16384 x 2048 with the rounding of X: 144 us then (239 TFLOP/s), 54 us now (639), 4096 x 14336: 260 and 95 us.
-// Products with too few output tiles to fill the SMs are cut along K (ksplit > 1: blockIdx.z is the part): every part leaves its sums
-// in part [ksplit][T][N] and k_split_sum adds them in order, with the bias.
+// Left to it: the heads of a batch, and rows sorted by more experts than k_gemm_bf16_pair notes.
 // Every wait on an mbarrier is bounded: on a timeout the CTA raises *err, skips what is left and still frees its tensor memory.
 // vec: rows and bases allow 16-byte loads (then K is a multiple of 8: LinArgs::vec of a bf16 product): eight entries a thread, over all rows of a batch entry at once.
 // 512 x 2048 5.6 us with an entry a thread, 4.0 now; 512 x 8192 13.6 and 6.2.
@@ -895,7 +809,7 @@ __device__ __forceinline__ void tc_wait(uint32_t bar, uint32_t parity, bool & de
 }
 
 // maps: X as bf16 [xbatch][T][K] (box 64 x 128), W [batch][N][K] (box 64 x 256)
-__global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const LinArgs a, int * err, int ksplit = 1, float * part = nullptr) {
+__global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const LinArgs a, int * err) {
     pdl_enter();
     extern __shared__ uint8_t um_raw[];
     __shared__ __align__(8) uint64_t full[UM_STAGES], empty[UM_STAGES], done;
@@ -906,7 +820,7 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
     const int m0 = blockIdx.y * UM_BM, n0 = blockIdx.x * UM_BN;
     const int r0 = a.seg ? a.seg[blockIdx.z] : 0, T = a.seg ? a.seg[blockIdx.z + 1] - r0 : a.T;
     if (m0 >= T) return;                      // the whole block, before anything is allocated
-    const int bz = ksplit > 1 ? 0 : blockIdx.z;
+    const int bz = blockIdx.z;
     volatile int * failed = &failed_s;
     if (tid == 0) {
         failed_s = 0;
@@ -926,8 +840,7 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_s;
-    const int nk_all = (a.K + UM_BK - 1) / UM_BK, kbeg = ksplit > 1 ? (int) ((long long) nk_all * blockIdx.z / ksplit) : 0;
-    const int nk = (ksplit > 1 ? (int) ((long long) nk_all * (blockIdx.z + 1) / ksplit) : nk_all) - kbeg;       // at least one: ksplit <= nk_all
+    const int nk = (a.K + UM_BK - 1) / UM_BK;
     if (warp == 0) {
         const int zx = a.seg ? 0 : bz;
         bool dead = false;
@@ -937,8 +850,8 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
             if (elect_one() && !dead) {
                 const uint32_t sa = smem0 + (uint32_t) slot * UM_STAGE_BYTES, bar = smem_addr(&full[slot]);
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"((uint32_t) UM_STAGE_BYTES) : "memory");
-                tma_load_3d(sa, &map_x, (kbeg + kt) * UM_BK, r0 + m0, zx, bar);
-                tma_load_3d(sa + UM_A_BYTES, &map_w, (kbeg + kt) * UM_BK, n0, bz, bar);
+                tma_load_3d(sa, &map_x, kt * UM_BK, r0 + m0, zx, bar);
+                tma_load_3d(sa + UM_A_BYTES, &map_w, kt * UM_BK, n0, bz, bar);
             }
             __syncwarp();
             if (++slot == UM_STAGES) { slot = 0; turn++; }
@@ -978,9 +891,9 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
     if (ok) {
         const int m = m0 + 32 * (warp & 3) + lane, cbase = (warp >> 2) * (UM_BN / 2);
         const uint32_t taddr = tmem + ((uint32_t) (32 * (warp & 3)) << 16) + (uint32_t) cbase;
-        const int ldy = ksplit > 1 ? a.N : a.ldy;
-        const float * bias = ksplit > 1 ? nullptr : a.bias;
-        float * Y = (ksplit > 1 ? part + (size_t) blockIdx.z * T * a.N : a.seg ? a.Y + (size_t) r0 * ldy : a.Y + (size_t) blockIdx.z * a.sY) + (size_t) m * ldy;
+        const int ldy = a.ldy;
+        const float * bias = a.bias;
+        float * Y = (a.seg ? a.Y + (size_t) r0 * ldy : a.Y + (size_t) bz * a.sY) + (size_t) m * ldy;
 #pragma unroll 1
         for (int c = 0; c < UM_BN / 2; c += 16) {
             uint32_t r[16];
@@ -1023,7 +936,7 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
     }
 }
 
-// Y[t][n] = bias[n] + the parts' sums, in order. NV entries a thread (four where N, ldy and the bases allow 16-byte accesses: 4 x 512 x 2048 7.9 -> 5.6 us)
+// products with too few tiles to fill the SMs are cut along K, and every part leaves its sums in part [ksplit][T][N]: Y[t][n] = bias[n] + the parts' sums, in order. NV entries a thread (four where N, ldy and the bases allow 16-byte accesses: 4 x 512 x 2048 7.9 -> 5.6 us)
 template <int NV>
 __global__ void __launch_bounds__(256) k_split_sum(const float * part, int ksplit, int T, int N, const float * __restrict__ bias, float * Y, int ldy) {
     pdl_enter();

@@ -120,26 +120,25 @@ int64_t b200_get_tap(b200_ctx * c, const char * name, int layer, float * out, in
 /* µs-resolution counters (the reference's are ms-truncated at the bridge: cpp/bridge.cpp:650-655) */
 void b200_timings(b200_ctx * c, double * t_prompt_us, int64_t * n_prompt, double * t_gen_us, int64_t * n_gen);
 void b200_reset_timings(b200_ctx * c);
-/* mean ms of one [T x K] . [N x K]^T product through the layer-stack family's own kernels (dtype 0 bfloat16, 1 float32;
- * T <= 4 takes the decode mat-vec, larger T the prompt kernels), CUDA events around `reps` launches over distinct weights;
- * negative on error. bench.py's per-kernel roofline of the family. */
+/* mean ms of one [T x K] . [N x K]^T product through the layer-stack family's own kernels (dtype 0 bfloat16, 1 float32; b200_stack_product_kernel names the one that runs), CUDA events
+ * around `reps` products over distinct weights, each let in beside the end of the one before as in a model's pass; negative on error. bench.py's per-kernel roofline of the family. */
 float b200_stack_time_linear(int device, int dtype, int T, int N, int K, int reps);
-/* the kernel such a product takes by itself (in a model's pass one token's products go to the ring kernel, b200_stack_linear_in_pass; glu: gate and up rows interleaved): 0 a warp per row, 1 a block per row, 2 a block per eight rows with x in
- * registers, 3 tcgen05 (bfloat16), 4 tcgen05 (float32) in K parts, 5 mma.sync, 6 tiles on the fp32 pipe, 7 tcgen05 (float32) whole, -1 bad arguments (host arithmetic, tests) */
+/* the kernel such a product takes (glu: gate and up rows interleaved): 0 a warp per row, 1 a block per row, 2 the ring kernel of one to four tokens, 3 tcgen05
+ * (bfloat16), 4 tcgen05 (float32) in K parts, 5 mma.sync, 6 tiles on the fp32 pipe, 7 tcgen05 (float32) whole, -1 bad arguments (host arithmetic, tests) */
 int b200_stack_product_kernel(int dtype, int T, int N, int K, int glu, int sm_count);
 /* operator-level parity entry of the same products: y[T][N] = x[T][K] . w[N][K]^T (+ bias[N]); glu != 0: the rows of w are
  * interleaved (gate_i, up_i) and y is [T][N / 2], the clamped gated unit g sigmoid(1.702 g) (u + 1) with g = min(gate, limit),
- * u = clamp(up, +-limit). Host pointers; w is rounded to bfloat16 when dtype = 0. The shape picks the kernel as in serving:
- * T <= 4 the mat-vec, else (bfloat16) tcgen05.mma with TMEM accumulators for T >= 64, N >= 128, K >= 64, K % 8 == 0, mma.sync
- * for other 16-byte-aligned shapes, the CUDA-core product for float32 and odd shapes. */
+ * u = clamp(up, +-limit). Host pointers; w is rounded to bfloat16 when dtype = 0. The shape picks the kernel as in serving
+ * (b200_stack_product_kernel): up to four tokens the ring kernel, else tcgen05 where the portion is long or the matrix large enough, mma.sync for other bfloat16 rows of whole 16
+ * bytes, and tiles on the fp32 pipe. */
 int b200_stack_linear(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y);
-/* the same product as a model's pass launches it: one token's takes the kernel that asks for its rows ahead of the kernel in front of it, here the same product once more */
+/* the same product as a model's pass launches it, let in beside the end of the kernel in front of it: here the same product once more */
 int b200_stack_linear_in_pass(int device, int dtype, int T, int N, int K, const float * x, const float * w, const float * bias, int glu, float limit, float * y);
 /* a batch of products as a layer's heads run them, x[batch][T][K] on w[batch][N][K] -> y[batch][T][N], or as its experts do (seg: batch + 1 first rows, from 0): rows seg[z] to
  * seg[z + 1] - 1 of x[T][K] on matrix z -> y[T][N]. glu: 1 clamped sigmoid units, 2 GELU units (y has N / 2 columns); rounded: the units as bfloat16, as the kernel on pairs of
  * SMs hands them to the product behind it (an error where it does not take the product). Entries that no kernel stores are NaN */
 int b200_stack_products(int device, int dtype, int T, int N, int K, int batch, const int32_t * seg, const float * x, const float * w, int glu, float limit, int rounded, float * y);
-/* how a model's pass runs a product of a batch, or (seg != 0) of rows sorted by `batch` matrices: out[0] the kernel as b200_stack_product_kernel names them, out[1] 1 where it
+/* how a model's pass runs a product of a batch, or (seg != 0) of rows sorted by `batch` matrices: out[0] the kernel as b200_stack_product_kernel names them, with 8 for tcgen05 (bfloat16) on pairs of SMs, out[1] 1 where it
  * starts on empty SMs instead of beside the end of the kernel in front (host arithmetic, tests) */
 int b200_stack_product_plan(int dtype, int T, int N, int K, int batch, int seg, int glu, int sm_count, int32_t * out);
 /* launch shape of a latent-attention layer over a pass of T tokens (the decode kernels: T < 8): out = tokens per block, heads per block, key slices, score-row

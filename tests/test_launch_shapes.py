@@ -149,18 +149,18 @@ BF16, F32 = 0, 1
 
 @pytest.mark.parametrize("dtype,T,N,K,glu,want", [
     (BF16, 1, 16000, 2048, 0, 2), (BF16, 1, 2048, 8192, 0, 2), (BF16, 1, 16384, 2048, 1, 2), (F32, 1, 4096, 1024, 0, 2), (F32, 1, 16000, 4096, 1, 2),
-    (BF16, 1, 2048, 1536, 0, 2), (BF16, 1, 2048, 1536, 1, 0), (BF16, 1, 2048, 3072, 1, 2), (BF16, 1, 2048, 3072, 0, 0),      # three quarters of a block's lanes
-    (BF16, 1, 5120, 4096, 1, 2), (BF16, 1, 8192, 4096, 1, 0), (BF16, 1, 10240, 4096, 1, 2), (F32, 1, 8192, 4096, 1, 0),     # a gated unit's waves
-    (BF16, 1, 2048, 1024, 0, 0), (BF16, 1, 8192, 3072, 1, 0), (F32, 1, 2048, 3072, 0, 0),          # lanes without entries: 1.2 times as long
-    (BF16, 1, 16000, 16384, 0, 0), (F32, 1, 16000, 8192, 0, 0),                  # eight chunks a lane: 1.4 and 1.2 times
-    (BF16, 1, 512, 2048, 0, 1), (BF16, 4, 16000, 2048, 0, 0), (BF16, 1, 2048, 2044, 0, 0),
+    (BF16, 1, 1, 8, 0, 2), (BF16, 1, 2048, 1536, 1, 2), (BF16, 1, 8192, 4096, 1, 2), (BF16, 1, 512, 2048, 0, 2), (F32, 1, 16000, 8192, 0, 2),      # any number of rows
+    (BF16, 1, 16000, 8200, 0, 0), (BF16, 1, 16000, 16384, 0, 0), (F32, 1, 16000, 8196, 0, 0), (BF16, 1, 2048, 2044, 0, 0), (F32, 1, 2048, 2046, 0, 0),      # rows beyond a block's registers, and of odd bytes
+    (BF16, 1, 512, 16384, 0, 1), (BF16, 1, 513, 16384, 0, 0), (BF16, 1, 512, 16384, 1, 0), (BF16, 1, 512, 1020, 0, 0), (BF16, 1, 512, 1028, 0, 1),      # few of those that are long
+    (BF16, 3, 16000, 2048, 0, 2), (BF16, 4, 16000, 2048, 0, 2), (BF16, 2, 12287, 2048, 0, 2), (BF16, 2, 12288, 2048, 0, 0), (F32, 2, 12287, 1024, 0, 2), (F32, 2, 12288, 1024, 0, 0),      # 48 MB
+    (BF16, 5, 16000, 2044, 0, 6), (F32, 4, 16000, 8196, 0, 0),
     (F32, 300, 1024, 4096, 0, 4), (F32, 600, 1024, 512, 0, 4), (F32, 64, 4096, 2048, 0, 4),
     (F32, 64, 512, 512, 0, 4), (F32, 64, 512, 496, 0, 7), (F32, 64, 9472, 1024, 0, 4), (F32, 64, 9600, 1024, 0, 7), (F32, 64, 16000, 2048, 0, 7), (F32, 600, 4096, 4096, 0, 7),      # two blocks' worth of k, two SMs a tile
     (F32, 64, 512, 256, 0, 7), (F32, 300, 1024, 4096, 1, 7), (F32, 64, 64, 128, 0, 7), (F32, 64, 64, 124, 0, 6), (F32, 127, 512, 64, 0, 6), (F32, 128, 128, 64, 0, 7), (F32, 128, 127, 64, 0, 6), (F32, 64, 64, 4096, 0, 7), (F32, 64, 128, 4096, 0, 4),
     (F32, 63, 512, 512, 0, 6), (F32, 64, 63, 512, 0, 6), (F32, 64, 512, 60, 0, 6), (F32, 64, 512, 510, 0, 6),
     (BF16, 64, 128, 64, 0, 3), (BF16, 63, 128, 64, 0, 5), (BF16, 64, 128, 60, 0, 6)])
 def test_stack_product_kernel(dtype, T, N, K, glu, want):
-    """which kernel a layer stack's product takes: 0 a warp per row, 1 a block per row, 2 a block per eight rows with x in registers, 3 tcgen05 (bfloat16), 4 and 7
+    """which kernel a layer stack's product takes: 0 a warp per row, 1 a block per row, 2 the ring kernel, 3 tcgen05 (bfloat16), 4 and 7
     tcgen05 (float32) in K parts and whole, 5 mma.sync, 6 tiles on the fp32 pipe; the sizes on both sides of each line are among those measured"""
     assert _lib.lib().b200_stack_product_kernel(dtype, T, N, K, glu, 148) == want
 
@@ -180,9 +180,9 @@ def test_large_grids_of_fp32_tiles_start_on_empty_sms(dtype, T, N, K, batch, seg
 
 
 @pytest.mark.parametrize("T,N,K,batch,seg,want", [
-    (5, 256, 192, 1, 0, 3), (5, 256, 184, 1, 0, 5), (5, 255, 192, 1, 0, 5), (63, 256, 192, 1, 0, 3), (63, 4096, 64, 1, 0, 5), (63, 254, 4096, 1, 0, 5), (5, 256, 196, 1, 0, 6),
-    (5, 256, 192, 4, 1, 3), (63, 256, 192, 512, 1, 3), (63, 256, 192, 513, 1, 5), (63, 256, 192, 4, 0, 5),                       # experts, more of them than a block notes, heads
-    (64, 256, 64, 1, 0, 3), (64, 128, 64, 1, 0, 3), (64, 127, 64, 1, 0, 5), (64, 128, 64, 513, 1, 3), (64, 128, 64, 4, 0, 3), (64, 128, 56, 1, 0, 5)])
+    (5, 256, 192, 1, 0, 8), (5, 256, 184, 1, 0, 5), (5, 255, 192, 1, 0, 5), (63, 256, 192, 1, 0, 8), (63, 4096, 64, 1, 0, 5), (63, 254, 4096, 1, 0, 5), (5, 256, 196, 1, 0, 6),
+    (5, 256, 192, 4, 1, 8), (63, 256, 192, 512, 1, 8), (63, 256, 192, 513, 1, 5), (63, 256, 192, 4, 0, 5),                       # experts, more of them than a block notes, heads
+    (64, 256, 64, 1, 0, 8), (64, 128, 64, 1, 0, 8), (64, 127, 64, 1, 0, 5), (64, 128, 64, 513, 1, 3), (64, 128, 64, 4, 0, 3), (64, 128, 56, 1, 0, 5)])
 def test_bfloat16_products_of_portions(T, N, K, batch, seg, want):
-    """few tokens go to the tensor memory from 256 rows and three slices of k on, 64 and more from 128 rows and one slice"""
+    """8 pairs of SMs, 3 a block per tile, 5 mma.sync: few tokens go to the tensor memory from 256 rows and three slices of k on, 64 and more from 128 rows and one slice"""
     assert product_plan(BF16, T, N, K, batch, seg)[0] == want
