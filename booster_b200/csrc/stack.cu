@@ -300,7 +300,8 @@ struct StackCtx {
 namespace {
 
 // where a pass's launches go. cold: the next one waits for all before it as a whole (it may have to wait for another stream as well); nullptr: every one does (a product by itself)
-struct Lane { cudaStream_t st = nullptr; bool * cold = nullptr; };
+// count: launches so far
+struct Lane { cudaStream_t st = nullptr; bool * cold = nullptr; int64_t * count = nullptr; };
 // a launch that may become resident while the kernel before it runs (stack_kernels.cuh: pdl_wait)
 template <typename... P, typename... A>
 void pdl(const Lane & l, dim3 grid, dim3 block, size_t smem, void (*kern)(P...), A... args) {
@@ -312,9 +313,11 @@ void pdl(const Lane & l, dim3 grid, dim3 block, size_t smem, void (*kern)(P...),
     cfg.attrs = at; cfg.numAttrs = l.cold && !*l.cold ? 1 : 0;
     if (l.cold) *l.cold = false;
     SCU(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+    if (l.count) ++*l.count;
 }
+Lane lane_of(StackCtx * c) { return Lane{c->st, &c->cold, &c->launches}; }
 template <typename... P, typename... A>
-void pdl(StackCtx * c, dim3 grid, dim3 block, size_t smem, void (*kern)(P...), A... args) { pdl(Lane{c->st, &c->cold}, grid, block, smem, kern, args...); }
+void pdl(StackCtx * c, dim3 grid, dim3 block, size_t smem, void (*kern)(P...), A... args) { pdl(lane_of(c), grid, block, smem, kern, args...); }
 
 // in front of a walk over a portion's tokens: its few blocks are chains of instructions, and let in while the kernel before still fills most SMs they crowd on the first that are
 // free (512 tokens of the delta rule, 128 blocks: 128 us one to an SM, 340 so). They wait for that kernel to end; a token's step is too short for that.
@@ -1492,7 +1495,7 @@ struct LinOpt {
     const __nv_bfloat16 * x16 = nullptr;    // tcgen05 (bfloat16): X rounded, rows K apart, if it is there already
     __nv_bfloat16 * y16 = nullptr;          // gated units of such a product on pairs of SMs (pairs()): rounded, here, instead of Y
 };
-void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X, int ldx, const void * W, const float * bias, float * Y, int ldy,
+void linear_on(const Lane & lane, int dtype, const float * X, int ldx, const void * W, const float * bias, float * Y, int ldy,
                int T, int N, int K, int batch = 1, long long sX = 0, long long sW = 0, long long sY = 0, bool glu = false, float glu_limit = 0.f,
                const UmmaScratch * us = nullptr, const LinOpt * opt = nullptr) {
     if (T <= 0 || N <= 0) return;
@@ -1502,7 +1505,6 @@ void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X
     const int vecw = dtype == STACK_F32 ? 4 : 8;
     const auto al16 = [](const void * p) { return ((uintptr_t) p & 15) == 0; };
     a.vec = K % vecw == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % vecw == 0 && al16(X) && al16(W);
-    if (launches) (*launches)++;
     const LinRoute route = lin_route(dtype, T, N, K, batch, a.vec != 0, a.glu != 0, a.seg != nullptr, a.w_index || a.x_scale, us && us->err, (size_t) xbatch * T * K, us && us->xb ? us->elems : 0,
                                      us && us->part ? us->part_floats : 0, us ? us->sm_count : 148);
     if (route == LIN_RING) {
@@ -1523,12 +1525,11 @@ void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X
         const __nv_bfloat16 * x16 = opt && opt->x16 ? opt->x16 : us->xb;
         if (!(opt && opt->x16))
             pdl(lane, dim3((unsigned) std::min<long long>(((long long) T * (K / 8) + 255) / 256, 2048), (unsigned) xbatch), 256, 0, k_to_bf16, X, ldx, T, K, sX, us->xb, (long long) T * K);
-        if (launches) (*launches)++;
         if (route == LIN_PAIR) {
             const PairPlan p = pair_plan(T, N, K, a.seg ? batch : 0, !a.glu && !a.seg && us->part && split_k_enabled(), us->sm_count, us->part_floats);
             const CUtensorMap mx = map_bf16(x16, K, T, 1, K, (long long) T * K, a.seg ? 32 : p.n / 2), mw = map_bf16(W, K, N, batch, K, sW, 128);
             launch_pair(lane, mx, mw, a, p, pair_work(p, T, N, batch), us->sm_count, us->err, us->part);
-            if (p.parts > 1) { split_sum(lane, us->part, p.parts, T, N, bias, Y, ldy); if (launches) (*launches)++; }
+            if (p.parts > 1) split_sum(lane, us->part, p.parts, T, N, bias, Y, ldy);
         } else {
             static size_t have[64] = {0};
             raise_smem(k_gemm_bf16_umma, UM_SMEM, have);
@@ -1539,7 +1540,6 @@ void linear_on(const Lane & lane, int dtype, int64_t * launches, const float * X
         const int parts = f32_k_parts(T, N, K, us->sm_count);
         launch_f32_umma(lane, a, us->err, 1, parts, us->part);
         split_sum(lane, us->part, parts, T, N, bias, Y, ldy);
-        if (launches) (*launches)++;
     } else if (route == LIN_F32_UMMA) {
         launch_f32_umma(lane, a, us->err, batch);
     } else if (route == LIN_MMA) {
@@ -1562,7 +1562,7 @@ void linear(StackCtx * c, const float * X, int ldx, const DMat & W, float * Y, i
         rounded.x16 = c->h16;
         opt = &rounded;
     }
-    linear_on(Lane{c->st, &c->cold}, c->m->dtype, &c->launches, X, ldx, W.w, W.bias, Y, ldy, T, W.N, W.K, batch, sX, (long long) W.N * W.K, sY, glu, glu_limit, &us, opt);
+    linear_on(lane_of(c), c->m->dtype, X, ldx, W.w, W.bias, Y, ldy, T, W.N, W.K, batch, sX, (long long) W.N * W.K, sY, glu, glu_limit, &us, opt);
 }
 
 // whether a bfloat16 model's product of this pass goes to pairs of SMs (n_seg > 0: rows sorted by that many experts)
@@ -1586,13 +1586,11 @@ void gated_ff(StackCtx * c, const float * X, const DMat & gateup, float * F, con
 void post_norm_add(StackCtx * c, const float * w_post, const float * w_next, int T) {
     const StackModel & m = *c->m;
     pdl(c, T, std::min(256, 32 * m.groups), 0, k_post_norm_add, c->Y, w_post, c->X, w_next, c->Hn, m.E, m.groups, m.eps, c->h16_on ? c->h16 : nullptr);
-    c->launches++;
 }
 
 void norm(StackCtx * c, const float * X, int ldx, const int32_t * rows, const float * w, int n, int groups, float * Y, int ldy, int T, bool accumulate) {
     const int threads = std::min(256, 32 * groups);
     pdl(c, T, threads, 0, k_group_norm, X, ldx, rows, w, n, groups, c->m->eps, Y, ldy, accumulate ? 1 : 0);
-    c->launches++;
     SCU(cudaGetLastError());
 }
 
@@ -1610,7 +1608,6 @@ void mixer_mingru(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     spread(c, T);
     if (T > 8) pdl(c, (L.width + 31) / 32, MG_WARPS * 32, 0, k_mingru_tiles, c->P, T, L.width, c->rec + R.off_rec, c->A);
     else pdl(c, (L.width + 127) / 128, 128, 0, k_mingru_scan, c->P, T, L.width, c->rec + R.off_rec, c->A);
-    c->launches++;
     linear(c, c->A, L.width, L.o, c->out, c->m->E, T);
 }
 
@@ -1667,11 +1664,10 @@ void gemm_f32(StackCtx * c, const float * X, int ldx, long long sX, const float 
     LinArgs a{X, W, nullptr, Y, M, N, K, ldx, ldy, sX, sW, sY, 0, 0, 0.f, 0.f, w_kn, ldw, nz2, sX2, sW2, sY2};
     a.vec = K % 4 == 0 && ldx % 4 == 0 && sX % 4 == 0 && sW % 4 == 0 && sX2 % 4 == 0 && sW2 % 4 == 0 && ldw % 4 == 0 && al16(X) && al16(W);
     a.accum = accum; a.see_rows = see.rows; a.see_pos = see.pos; a.see_step = see.step; a.rows_all = rows_all;
-    if (f32_umma_takes(a.vec != 0, M, N, K)) launch_f32_umma(Lane{c->st, &c->cold}, a, c->d_err, batch * nz2);
+    if (f32_umma_takes(a.vec != 0, M, N, K)) launch_f32_umma(lane_of(c), a, c->d_err, batch * nz2);
     else if (a.vec && M >= SG_BM && N >= SG_BN && simt_big_enabled())       // operands that fill 128 x 128 tiles
         pdl(c, dim3((unsigned) ((N + SG_BN - 1) / SG_BN), (unsigned) ((M + SG_BM - 1) / SG_BM), (unsigned) (batch * nz2)), 256, 0, k_gemm_simt_big, a);
     else pdl(c, dim3((unsigned) ((N + 63) / 64), (unsigned) ((M + 63) / 64), (unsigned) (batch * nz2)), 256, 0, k_gemm_simt<float>, a);
-    c->launches++;
 }
 constexpr int ATT_TQ = 16;                 // tokens per tile of the prompt attention
 constexpr size_t ATT_SCORE_BYTES = (size_t) 256 << 20;
@@ -1680,7 +1676,7 @@ constexpr size_t ATT_SCORE_BYTES = (size_t) 256 << 20;
 void latent_values_out(StackCtx * c, const LayerSpec & L, int T, int ldp, int gate_off) {
     const int H = L.H, V = L.V, rank = L.rank;
     linear(c, c->OL, H * rank, L.uv, c->A, H * V, T, H, rank, V);
-    if (L.head_gate) { pdl(c, dim3((unsigned) T, T <= 16 ? (unsigned) ((H * V + 255) / 256) : 1u), 256, 0, k_head_gate, c->A, c->P + gate_off, ldp, H, V, L.gate_rows == H ? 0 : 1); c->launches++; }
+    if (L.head_gate) { pdl(c, dim3((unsigned) T, T <= 16 ? (unsigned) ((H * V + 255) / 256) : 1u), 256, 0, k_head_gate, c->A, c->P + gate_off, ldp, H, V, L.gate_rows == H ? 0 : 1); }
     linear(c, c->A, H * V, L.o, c->out, c->m->E, T);
 }
 
@@ -1720,9 +1716,7 @@ void mixer_latent(StackCtx * c, const LayerSpec & L, const RunSpec & Rn, int T) 
             gemm_f32(c, c->QK + (size_t) g0 * M * W, W, (long long) M * W, keys, 0, 0, sK, c->att_scores, nk, (long long) M * nk, M, nk, W, ng, 1, 0, 0, 0, 0, See(), rows);
             pdl(c, (rows + 7) / 8, 256, 0, k_latent_softmax_rows, c->att_scores, rows, H, TQ, nk, L.window, span, L.sink, &c->d_step->st, L.scale, g0);
             gemm_f32(c, c->att_scores, nk, (long long) M * nk, keys, 1, W, sK, c->OL + (size_t) g0 * M * rank, rank, (long long) M * rank, M, rank, nk, ng, 1, 0, 0, 0, 0, See(), rows);
-            c->launches++;
         }
-        c->launches++;
         latent_values_out(c, L, T, ldp, gate_off);
         return;
     }
@@ -1733,8 +1727,7 @@ void mixer_latent(StackCtx * c, const LayerSpec & L, const RunSpec & Rn, int T) 
     else if (W % 4 == 0 && ap.TQ * ap.HQ <= 4) pdl(c, grid, 256, ap.smem, k_latent_attn_staged<true, 4>, aa);
     else if (W % 4 == 0) pdl(c, grid, 256, ap.smem, k_latent_attn_staged<true, LAT_NQ_MAX>, aa);
     else pdl(c, grid, 256, ap.smem, k_latent_attn_staged<false, LAT_NQ_MAX>, aa);
-    if (ap.nsplit > 1) { pdl(c, dim3((unsigned) T, (unsigned) H, (unsigned) ((rank + 63) / 64)), 256, 0, k_latent_combine, aa); c->launches++; }
-    c->launches += 2;
+    if (ap.nsplit > 1) { pdl(c, dim3((unsigned) T, (unsigned) H, (unsigned) ((rank + 63) / 64)), 256, 0, k_latent_combine, aa); }
     latent_values_out(c, L, T, ldp, gate_off);
 }
 
@@ -1743,8 +1736,7 @@ void causal_conv(StackCtx * c, ConvArgs a, int batch = 1) {
     a.fuse_hist = a.T == 1 ? 1 : 0;
     if (a.T > 1 && a.taps <= CONV_TAPS) pdl(c, dim3((unsigned) ((a.C + 127) / 128), (unsigned) ((a.T + CONV_TT - 1) / CONV_TT), (unsigned) batch), 128, 0, k_causal_conv_rows, a);
     else pdl(c, dim3((unsigned) ((a.C + 127) / 128), (unsigned) a.T, (unsigned) batch), 128, 0, k_causal_conv, a);
-    c->launches++;
-    if (a.taps > 1 && !a.fuse_hist) { pdl(c, dim3((unsigned) ((a.C + 127) / 128), 1, (unsigned) batch), 128, 0, k_causal_conv_hist, a); c->launches++; }
+    if (a.taps > 1 && !a.fuse_hist) { pdl(c, dim3((unsigned) ((a.C + 127) / 128), 1, (unsigned) batch), 128, 0, k_causal_conv_hist, a); }
 }
 
 void mixer_delta(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
@@ -1758,7 +1750,6 @@ void mixer_delta(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     else if (D <= 128) launch_delta_scan<128>(c, L, T, C, S);
     else launch_delta_scan<256>(c, L, T, C, S);
     pdl(c, dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, k_delta_out, c->O, c->P, ldp, C + 2 * H, H, V, L.dnorm, 0, 0, c->m->eps, c->A);
-    c->launches += 3;
     linear(c, c->A, H * V, L.o, c->out, E, T);
 }
 
@@ -1787,7 +1778,6 @@ void mixer_gdelta(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     else if (D <= 128) launch_gdelta_scan<128>(c, L, T, ldp, S);
     else launch_gdelta_scan<256>(c, L, T, ldp, S);
     pdl(c, dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, k_delta_out, c->O, c->P, ldp, 2 * HD + HV, H, V, L.dnorm, V, 1, c->m->eps, c->A);
-    c->launches += 3;
     linear(c, c->A, HV, L.o, c->out, E, T);
 }
 
@@ -1826,10 +1816,8 @@ void mixer_diffattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T)
             pdl(c, (rows + 7) / 8, 256, 0, k_diff_softmax_rows, c->att_scores, ng * M, G, Rh, TQ, nk, L.window, span, &c->d_step->st, L.scale, L.lambda, g0, T);
             gemm_f32(c, c->att_scores, nk, (long long) M * nk, keys + (size_t) G * 2 * D, 1, row, sK, c->OL + (size_t) g0 * M * V, V, (long long) M * V, M, V, nk, ng,
                      G, 2 * grp, V, (long long) Tpad * Rh * V);
-            c->launches++;
         }
         pdl(c, dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, k_diff_norm_out, c->OL, Tpad, H, G, V, c->m->eps, 1.0f - L.diff, c->A);
-        c->launches += 2;
         linear(c, c->A, H * V, L.o, c->out, E, T);
         return;
     }
@@ -1845,7 +1833,6 @@ void mixer_diffattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T)
     else if (V <= 64) pdl(c, grid, 256, smem, k_diff_attn<2>, a);
     else if (V <= 128) pdl(c, grid, 256, smem, k_diff_attn<4>, a);
     else pdl(c, grid, 256, smem, k_diff_attn<8>, a);
-    c->launches++;
     linear(c, c->A, H * V, L.o, c->out, E, T);
 }
 
@@ -1864,7 +1851,6 @@ void launch_outer_walk(StackCtx * c, const OuterScan & s) {
     while (ncols > 16 && s.H * ((cols + ncols - 1) / ncols) < c->sm_count) ncols = (ncols / 2 + 7) / 8 * 8;
     spread(c, s.T);
     pdl(c, dim3((unsigned) s.H, (unsigned) ((cols + ncols - 1) / ncols)), GD_RG * ncols, 0, k_outer_scan<DMAX>, s);
-    c->launches++;
 }
 template <int NC>
 void launch_outer_chunks(StackCtx * c, const OuterScan & s) {
@@ -1876,7 +1862,6 @@ void launch_outer_chunks(StackCtx * c, const OuterScan & s) {
     pdl(c, grid, 256, 0, k_outer_chunk_kv<NC>, s, vec, c->scan_sb, c->scan_ac);
     pdl(c, dim3((unsigned) s.H, (unsigned) ((n + 255) / 256)), 256, 0, k_outer_chunk_state, n, s.head_stride, nch, c->scan_ac, s.S, c->scan_sb);
     pdl(c, grid, 128, outer_chunk_smem(s.D, NC), k_outer_chunk_out<NC>, s, vec, c->scan_sb);
-    c->launches += 3;
 }
 // the outer-product recurrence over a portion: long ones chunk by chunk, short ones token by token
 void outer_scan(StackCtx * c, const OuterScan & s) {
@@ -1896,7 +1881,6 @@ void launch_outer_token(StackCtx * c, const OuterToken & t) {
     else if (t.D <= 64) pdl(c, t.H, threads, sm, k_outer_token<64, KIND>, t);
     else if (t.D <= 128) pdl(c, t.H, threads, sm, k_outer_token<128, KIND>, t);
     else pdl(c, t.H, threads, sm, k_outer_token<256, KIND>, t);
-    c->launches++;
 }
 
 // retention: P[t] = [ q | k | v | gate ] -> rotation, key scale -> recurrence -> per-head unit norm, silu gate -> output product
@@ -1920,7 +1904,6 @@ void mixer_retention(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T
     s.T = T; s.H = H; s.share = 1; s.D = D; s.V = V; s.kind = SCAN_CONST; s.decay = L.decay; s.S = S; s.head_stride = (long long) L.head_stride; s.O = c->O;
     outer_scan(c, s);
     pdl(c, dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, k_delta_out, c->O, c->P, ldp, 2 * HD + HV, H, V, nullptr, 0, 0, c->m->eps, c->A);
-    c->launches += 2;
     linear(c, c->A, HV, L.o, c->out, E, T);
 }
 
@@ -1947,7 +1930,6 @@ void mixer_mlstm(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     s.norm = 1; s.O = c->O; s.den = c->den;
     outer_scan(c, s);
     pdl(c, dim3((unsigned) T, (unsigned) ((H + 3) / 4)), 128, 0, k_mlstm_out, c->O, c->den, c->BG, ldg, q_scale, c->P, ldp, 2 * HD + HV, H, V, L.dnorm, c->m->eps, c->A);
-    c->launches += 2;
     linear(c, c->A, HV, L.o, c->out, E, T);
 }
 
@@ -1964,13 +1946,11 @@ void mixer_ssd(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     if (T == 1) { s.kind = SCAN_STEP; s.ab = c->P + inner + C; s.ld_ab = ldp; s.dt_bias = L.dt_bias; s.A_log = L.A_log; }
     else {
         pdl(c, T, H >= 128 ? 128 : 32, 0, k_step_table, c->P + inner + C, ldp, L.dt_bias, L.A_log, H, c->BG, 2 * H);
-        c->launches++;
         s.kind = SCAN_TABLE; s.ab = c->BG; s.ld_ab = 2 * H;
     }
     outer_scan(c, s);
     const int n = inner / L.norm_parts, nt = T > 16 ? 256 : std::min(1024, std::max(128, (n + 63) / 64 * 32));
     pdl(c, dim3((unsigned) T, (unsigned) L.norm_parts), nt, 0, k_gated_part_norm, c->O, c->CV, C, L.skip, c->P, ldp, inner, V, L.norm_parts, L.dnorm, c->m->eps, c->A);
-    c->launches++;
     linear(c, c->A, inner, L.o, c->out, E, T);
 }
 
@@ -1982,12 +1962,10 @@ void launch_selective(StackCtx * c, const LayerSpec & L, const SelScan & s) {
         const unsigned rest = (unsigned) ((s.T + s.seg - 1) / s.seg - 1);
         pdl(c, dim3((unsigned) nblk, rest), 256, 0, k_selective_scan<LANES, NS, SEL_FIRST>, s);
         pdl(c, dim3((unsigned) nblk, rest), 256, 0, k_selective_scan<LANES, NS, SEL_REST>, s);
-        c->launches++;
     }
     else if (s.T > 1) pdl(c, nblk, 256, 0, k_selective_scan<LANES, NS, SEL_WHOLE>, s);
     else if (c->m->dtype == STACK_F32) pdl(c, nblk, 256, (size_t) L.dt_rank * 4, k_selective_token<float, LANES, NS>, s, (const float *) L.wdt.w, L.wdt.bias, L.dt_rank);
     else pdl(c, nblk, 256, (size_t) L.dt_rank * 4, k_selective_token<__nv_bfloat16, LANES, NS>, s, (const __nv_bfloat16 *) L.wdt.w, L.wdt.bias, L.dt_rank);
-    c->launches++;
 }
 // selective scan: P[t] = [ x | z ] -> convolution of x -> [ step latent | B | C ] from it -> step sizes -> scan with skip and gate -> output product
 void mixer_selscan(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
@@ -2016,7 +1994,6 @@ void mixer_sigattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) 
     float * cache = c->caches[(size_t) R.cache_index];
     linear(c, c->in, E, L.proj, c->P, L.proj.N, T);
     pdl(c, T, 256, 0, k_sigattn_prep, c->P, L.proj.N, H, G, D, V, L.qw, L.kw, c->m->eps, L.t_coef, L.t_every, &c->d_step->st, c->CV, cache);
-    c->launches++;
     if (T >= 8) {
         // prompt portion: float32 products over tiles of ATT_TQ tokens, one batch entry per (tile, key/value head)
         const int TQ = ATT_TQ, Rh = H / G, M = TQ * Rh, ntile = (T + TQ - 1) / TQ, Tpad = ntile * TQ;
@@ -2034,10 +2011,8 @@ void mixer_sigattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) 
             pdl(c, (rows + 7) / 8, 256, 0, k_sig_weight_rows, c->att_scores, ng * M, G, Rh, TQ, nk, &c->d_step->st, L.scale, L.slope, L.pb, g0, T);
             gemm_f32(c, c->att_scores, nk, (long long) M * nk, cache + (size_t) G * D, 1, row, 0, c->OL + (size_t) g0 * M * V, V, (long long) M * V, M, V, nk, ng,
                      G, grp, V, (long long) Tpad * Rh * V);
-            c->launches++;
         }
         pdl(c, T, 256, 0, k_group_o_layout, c->OL, Tpad, H, G, V, c->A, nullptr, 0, 0);
-        c->launches += 2;
         linear(c, c->A, H * V, L.o, c->out, E, T);
         return;
     }
@@ -2053,7 +2028,6 @@ void mixer_sigattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) 
     else if (VPL == 2) pdl(c, grid, 256, smem, k_sig_attn<2>, a);
     else if (VPL == 4) pdl(c, grid, 256, smem, k_sig_attn<4>, a);
     else pdl(c, grid, 256, smem, k_sig_attn<8>, a);
-    c->launches++;
     linear(c, c->A, H * V, L.o, c->out, E, T);
 }
 
@@ -2089,8 +2063,7 @@ void mixer_gqattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     const GqaPrepArgs pa{c->P, ldp, H, G, D, V, L.qw, L.kw, c->m->eps, RopeArgs{L.rope_freq, L.rope_dims, L.rope_mag, L.rope_adjacent ? 1 : 0}, st, c->CV, cache, row,
                          c->VF, L.vmode, L.vlambda, L.unit_qk ? 1 : 0};
     pdl(c, dim3((unsigned) T, T <= 16 ? (unsigned) ((H + G + 7) / 8) : 1u), 256, 0, k_gqa_prep, pa);      // few tokens: a token's heads over several blocks
-    c->launches++;
-    if (L.pool > 0) { pdl(c, dim3((unsigned) (T / L.pool + 1), (unsigned) ((row + 127) / 128)), 128, 0, k_pool_rows, cache, row, pool, L.pool, st); c->launches++; }
+    if (L.pool > 0) { pdl(c, dim3((unsigned) (T / L.pool + 1), (unsigned) ((row + 127) / 128)), 128, 0, k_pool_rows, cache, row, pool, L.pool, st); }
     const float * gate = L.head_gate ? c->P + nq + row : nullptr;
     const int gate_per_entry = L.head_gate && L.gate_rows == H * V && V > 1 ? 1 : 0;
     const GqaMask mask{L.mask_kind, L.window, L.pool};
@@ -2126,10 +2099,8 @@ void mixer_gqattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
                      G, grp, V, (long long) Tpad * Rh * V, 0, masked ? See() : See{Rh, pos0 + g0 * TQ, TQ});
             if (npc) gemm_f32(c, c->att_scores, ld, (long long) M * ld, pool + (size_t) G * D, 1, row, 0, c->OL + (size_t) g0 * M * V, V, (long long) M * V, M, V, npc, ng,
                               G, grp, V, (long long) Tpad * Rh * V, 1);
-            c->launches++;
         }
         pdl(c, T, 256, 0, k_group_o_layout, c->OL, Tpad, H, G, V, c->A, gate, ldp, gate_per_entry);      // the gates ride on the regrouping
-        c->launches += 2;
         linear(c, c->A, H * V, L.o, c->out, E, T);
         return;
     }
@@ -2145,7 +2116,6 @@ void mixer_gqattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
         else if (RT == 2) { if (wide) pdl(c, grid, 256, smem, k_gqa_attn_group<2, 2>, a); else pdl(c, grid, 256, smem, k_gqa_attn_group<2, 1>, a); }
         else if (RT == 4) { if (wide) pdl(c, grid, 256, smem, k_gqa_attn_group<4, 2>, a); else pdl(c, grid, 256, smem, k_gqa_attn_group<4, 1>, a); }
         else pdl(c, grid, 256, smem, k_gqa_attn_group<8, 1>, a);
-        c->launches++;
         // (this kernel has two blocks for every SM: the few blocks of a float32 product behind it would crowd on the first SMs that it leaves. Bozisun at width 1024, seven tokens at
         // position 2000: 4.79 ms so and 4.36 whole)
         if (T > GEMV_MAX_T && c->m->dtype == STACK_F32) c->cold = true;
@@ -2164,7 +2134,6 @@ void mixer_gqattn(StackCtx * c, const LayerSpec & L, const RunSpec & R, int T) {
     else if (VPL == 2) pdl(c, grid, 256, smem, k_gqa_attn<2>, a);
     else if (VPL == 4) pdl(c, grid, 256, smem, k_gqa_attn<4>, a);
     else pdl(c, grid, 256, smem, k_gqa_attn<8>, a);
-    c->launches++;
     linear(c, c->A, H * V, L.o, c->out, E, T);
 }
 
@@ -2213,7 +2182,6 @@ void enqueue_layers_sequential(StackCtx * c, int T) {
     const float * w0 = m.layers[(size_t) m.runs[0].layer].norm1;
     if (m.dtype == STACK_F32) pdl(c, T, nthreads, 0, k_embed_rows<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, c->X, w0, m.groups, m.eps, c->Hn, c->h16_on ? c->h16 : nullptr);
     else pdl(c, T, nthreads, 0, k_embed_rows<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, c->X, w0, m.groups, m.eps, c->Hn, c->h16_on ? c->h16 : nullptr);
-    c->launches++;
     c->in = c->Hn; c->out = c->Y;
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
         const RunSpec & R = m.runs[ri];
@@ -2239,7 +2207,6 @@ void enqueue_layers_parallel(StackCtx * c, int T) {
     const bool looped = m.loop_step != nullptr;
     if (m.dtype == STACK_F32) pdl(c, T, 128, 0, k_embed_plain<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, c->X, looped ? c->XC + E : nullptr, 2 * E, 1.0f);
     else pdl(c, T, 128, 0, k_embed_plain<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, c->X, looped ? c->XC + E : nullptr, 2 * E, 1.0f);
-    c->launches++;
     const float * ya = nullptr, * yb = nullptr;        // outputs of the layer before, not yet added to X
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
         const RunSpec & R = m.runs[ri];
@@ -2248,7 +2215,6 @@ void enqueue_layers_parallel(StackCtx * c, int T) {
         if (R.pass >= 0) {
             // x <- W_in [x; x0] + step[pass]: the finished x goes to the left half of XC (x0 is in the right half since the embedding)
             pdl(c, T, 256, 0, k_add_norm2, c->X, ya, yb, c->XC, 2 * E, nullptr, nullptr, nullptr, nullptr, E, m.eps);
-            c->launches++;
             ya = yb = nullptr;
             DMat w = m.loop_in;
             w.bias = m.loop_step + (size_t) R.pass * E;
@@ -2259,11 +2225,9 @@ void enqueue_layers_parallel(StackCtx * c, int T) {
         float * hist = c->rec + R.off_rec + (L.n_rec - (size_t) nsub * std::max(ct - 1, 0) * E);
         if (T == 1 && ct > 0) {                        // one token: sum, both norms, both input convolutions and their history in one launch
             pdl(c, CANON1_CTAS, 256, 0, k_add_norm2_canon1, c->X, ya, yb, L.norm1, L.has_mlp ? L.norm2 : nullptr, L.canon, hist, c->U, (long long) plane, E, ct, m.eps);
-            c->launches++;
             u1 = c->U; u2 = c->U + plane;
         } else {
             pdl(c, T, 256, 0, k_add_norm2, c->X, ya, yb, nullptr, 0, L.norm1, L.has_mlp ? L.norm2 : nullptr, H1, H2, E, m.eps);
-            c->launches++;
         }
         if (ct > 0 && T > 1) {
             causal_conv(c, ConvArgs{c->Hn, E, (long long) plane, L.canon, (long long) E * ct, hist, (long long) (ct - 1) * E, c->U, E, (long long) plane,
@@ -2276,13 +2240,11 @@ void enqueue_layers_parallel(StackCtx * c, int T) {
         if (L.has_mlp) {
             linear(c, u2, E, L.gateup, c->A, L.ff, T);
             pdl(c, T, 256, 0, k_polynorm, c->A, L.ff, L.act, m.eps);
-            c->launches++;
             linear(c, c->A, L.ff, L.down, c->Y2, E, T);
             yb = c->Y2;
         }
         if (c->taps || ri + 1 == m.runs.size()) {      // the residual stream itself is wanted now
             pdl(c, T, 256, 0, k_add_norm2, c->X, ya, yb, nullptr, 0, nullptr, nullptr, nullptr, nullptr, E, m.eps);
-            c->launches++;
             ya = yb = nullptr;
             if (c->taps) tap_layer(c, ri, T);
         }
@@ -2297,7 +2259,6 @@ void mixture_ff(StackCtx * c, const LayerSpec & L, const float * h, int T, const
     const int E = c->m->E, top = L.top, ff = L.e_ff, slots = T * top, n = L.n_exp + L.n_ident;
     const RouteArgs ra{h, E, E, L.router, L.w_sg, n, top, L.n_groups, L.keep_groups, L.r_scale, c->r_sel, c->r_wt, c->r_sg, c->r_z, c->r_counter, L.route_fn, T <= 16 ? 8 : 1, L.corr, L.norm_w ? 1 : 0, L.r_bias};
     pdl(c, dim3((unsigned) T, (unsigned) ((n + (L.w_sg ? 1 : 0) + 8 / ra.wpr - 1) / (8 / ra.wpr))), 256, (size_t) (2 * n + L.n_groups) * 4, k_moe_route, ra);
-    c->launches++;
     LinOpt o;
     o.glu_kind = L.act_kind; o.alpha = L.act_alpha; o.shift = L.act_shift;
     if (T <= GEMV_MAX_T) {
@@ -2319,7 +2280,6 @@ void mixture_ff(StackCtx * c, const LayerSpec & L, const float * h, int T, const
         if (L.scale_input) pdl(c, slots, 128, 0, k_spread_rows, h, E, c->r_slot, c->r_wt, top, E, c->Xp);
         else if (c->h16_on && h == c->Hn && E % 8 == 0 && pairs(c, slots, L.e_gateup, L.n_exp)) { pdl(c, slots, 128, 0, k_gather_rows16, c->h16, c->r_src, E, c->xb); o.x16 = c->xb; }
         else pdl(c, slots, 128, 0, k_gather_rows, h, E, c->r_src, E, c->Xp);
-        c->launches += 2;
         o.seg = c->r_seg;
         gated_ff(c, c->Xp, L.e_gateup, c->Ap, L.e_down, c->Yk, slots, L.e_limit, &o, L.n_exp);      // rows of identity outputs sort behind the last matrix
         *slot_of = c->r_slot;
@@ -2344,7 +2304,6 @@ void enqueue_layers_prenorm(StackCtx * c, int T) {
         const DytW ne{m.embed_w, m.embed_b, m.embed_alpha}, n1{L0.norm1, L0.n1_b, L0.n1_alpha};
         if (m.dtype == STACK_F32) pdl(c, T, 256, 0, k_embed_dyt<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, ne, n1, c->X, m.depth_avg ? c->keep : nullptr, c->Hn);
         else pdl(c, T, 256, 0, k_embed_dyt<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, ne, n1, c->X, m.depth_avg ? c->keep : nullptr, c->Hn);
-        c->launches++;
     }
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
         const RunSpec & R = m.runs[ri];
@@ -2361,7 +2320,6 @@ void enqueue_layers_prenorm(StackCtx * c, int T) {
         };
         if (L.has_mlp) { j.nw = L.norm2; j.nb = L.n2_b; j.alpha = L.n2_alpha; j.Hn = c->Hn; } else layer_end(j);
         pdl(c, jgrid, 256, 0, k_join, j);
-        c->launches++;
         if (L.has_mlp) {
             JoinArgs f{};
             f.X = c->X; f.E = E; f.eps = m.eps;
@@ -2370,7 +2328,6 @@ void enqueue_layers_prenorm(StackCtx * c, int T) {
             if (L.ff > 0) { f.Ysh = c->Y; f.sg = c->r_sg; }
             layer_end(f);
             pdl(c, jgrid, 256, 0, k_join, f);
-            c->launches++;
         }
         if (c->taps) tap_layer(c, ri, T);
     }
@@ -2388,7 +2345,6 @@ void enqueue_layers_hyper(StackCtx * c, int T) {
         const LayerSpec & L0 = m.layers[(size_t) m.runs[0].layer];
         if (m.dtype == STACK_F32) pdl(c, T, hc_threads(T, E), 0, k_hc_embed<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, S, c->XS, plane, L0.hc[0], L0.g1, m.eps, c->Hn);
         else pdl(c, T, hc_threads(T, E), 0, k_hc_embed<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, S, c->XS, plane, L0.hc[0], L0.g1, m.eps, c->Hn);
-        c->launches++;
     }
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
         const RunSpec & R = m.runs[ri];
@@ -2404,7 +2360,6 @@ void enqueue_layers_hyper(StackCtx * c, int T) {
             if (last_sub && c->taps) j.Xsum = c->X;
             if (E % 4 == 0) pdl(c, T, hc_threads(T, E, 4, 512), 0, k_hc_join<4>, j);      // every buffer of a context is 16-byte aligned and its rows are E floats apart
             else pdl(c, T, hc_threads(T, E), 0, k_hc_join<1>, j);
-            c->launches++;
         };
         c->in = c->Hn; c->out = c->Y;
         run_mixer(c, L, R, T);
@@ -2430,7 +2385,6 @@ void enqueue_layers_postnorm(StackCtx * c, int T) {
     const int E = m.E;
     if (m.dtype == STACK_F32) pdl(c, T, hc_threads(T, E), 0, k_embed_plain<float>, (const float *) m.embed, c->d_step->tokens, E, m.vocab, c->X, nullptr, 0, m.embed_scale);
     else pdl(c, T, hc_threads(T, E), 0, k_embed_plain<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, c->d_step->tokens, E, m.vocab, c->X, nullptr, 0, m.embed_scale);
-    c->launches++;
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
         const RunSpec & R = m.runs[ri];
         const LayerSpec & L = m.layers[(size_t) R.layer];
@@ -2440,7 +2394,6 @@ void enqueue_layers_postnorm(StackCtx * c, int T) {
             if (end && last) { j.fw = m.final_norm; j.Hn = c->Hn; }
             if (E % 4 == 0) pdl(c, T, hc_threads(T, E, 4), 0, k_post_join<4>, j);      // every buffer of a context is 16-byte aligned and its rows are E floats apart
             else pdl(c, T, hc_threads(T, E), 0, k_post_join<1>, j);
-            c->launches++;
         };
         c->in = c->X; c->out = c->Y;
         run_mixer(c, L, R, T);
@@ -2503,12 +2456,10 @@ void layer_end(StackCtx * c, const LayerSpec & L, SumArgs a, const float * nw, i
         if (m.dtype == STACK_F32) { if (E % 4 == 0) go(k_side_in<float>, k_side_out<float, 4>); else go(k_side_in<float>, k_side_out<float, 1>); }
         else if (E % 4 == 0) go(k_side_in<__nv_bfloat16>, k_side_out<__nv_bfloat16, 4>);
         else go(k_side_in<__nv_bfloat16>, k_side_out<__nv_bfloat16, 1>);
-        c->launches += 2;
         return;
     }
     if (E % 4 == 0) pdl(c, T, nt, 0, k_sum_join<4>, a);      // every buffer of a context is 16-byte aligned and its rows are E floats apart
     else pdl(c, T, hc_threads(T, E), 0, k_sum_join<1>, a);
-    c->launches++;
     if (dim <= 0) return;
     linear(c, c->X, E, L.side_gate, c->SZ, dim, T);
     const dim3 zgrid((unsigned) T, (unsigned) ((dim + 127) / 128));
@@ -2519,7 +2470,6 @@ void layer_end(StackCtx * c, const LayerSpec & L, SumArgs a, const float * nw, i
     j.X = c->X; j.E = E; j.eps = m.eps; j.mult = 1.f; j.w = L.side_norm; j.scratch = c->Hn; j.Ya = c->Y; j.fw = nw; j.Hn = c->Hn; j.H16 = c->h16_on ? c->h16 : nullptr;
     if (E % 4 == 0) pdl(c, T, nt, 0, k_post_join<4>, j);
     else pdl(c, T, hc_threads(T, E), 0, k_post_join<1>, j);
-    c->launches += 2;
 }
 
 // blocks whose two sub-layers read one normed input: h = norm1(x), x += mixer(h) + ff(h), then the token's own input. The norm of the
@@ -2532,7 +2482,6 @@ void enqueue_layers_shared(StackCtx * c, int T) {
     const PairTable pt{m.pair_table, (unsigned long long) m.pair_mul_prev, (unsigned long long) m.pair_mul_cur, (unsigned long long) m.pair_buckets};
     if (m.dtype == STACK_F32) pdl(c, T, nt, 0, k_embed_pair<float>, (const float *) m.embed, pt, &c->d_step->st, c->d_step->tokens, E, m.vocab, w0, m.eps, c->X, c->Hn, c->h16_on ? c->h16 : nullptr);
     else pdl(c, T, nt, 0, k_embed_pair<__nv_bfloat16>, (const __nv_bfloat16 *) m.embed, pt, &c->d_step->st, c->d_step->tokens, E, m.vocab, w0, m.eps, c->X, c->Hn, c->h16_on ? c->h16 : nullptr);
-    c->launches++;
     for (size_t ri = 0; ri < m.runs.size(); ri++) {
         const RunSpec & R = m.runs[ri];
         const LayerSpec & L = m.layers[(size_t) R.layer];
@@ -2582,16 +2531,15 @@ void enqueue_head(StackCtx * c, int n_rows, int64_t row_off, bool one_token = fa
     c->h16_on = false;      // (what the head reads is no pass's row by row)
     if (normed) {
         // the last join left the normed residual (the sum of the streams) in Hn for every row of the pass: the wanted rows are gathered for the head
-        if (!one_token) { pdl(c, n_rows, 128, 0, k_gather_rows, c->Hn, m.E, c->d_step->rows, m.E, c->Y); c->launches++; hn = c->Y; }
+        if (!one_token) { pdl(c, n_rows, 128, 0, k_gather_rows, c->Hn, m.E, c->d_step->rows, m.E, c->Y); hn = c->Y; }
     }
     else if (one_token && m.block == BLOCK_SEQUENTIAL) {}      // the last layer left it in Hn
-    else if (m.dyt) { pdl(c, n_rows, 256, 0, k_dyt_rows, c->X, m.E, one_token ? nullptr : c->d_step->rows, DytW{m.final_norm, m.final_b, m.final_alpha}, m.E, c->Hn, m.E); c->launches++; }
+    else if (m.dyt) { pdl(c, n_rows, 256, 0, k_dyt_rows, c->X, m.E, one_token ? nullptr : c->d_step->rows, DytW{m.final_norm, m.final_b, m.final_alpha}, m.E, c->Hn, m.E); }
     else norm(c, c->X, m.E, one_token ? nullptr : c->d_step->rows, m.final_norm, m.E, m.groups, c->Hn, m.E, n_rows, false);
     linear(c, hn, m.E, m.head, c->d_logits + row_off * m.vocab, m.vocab, n_rows);
     if (m.softcap > 0.f) {
         const size_t n = (size_t) n_rows * m.vocab;
         pdl(c, (unsigned) ((n + 255) / 256), 256, 0, k_softcap, c->d_logits + row_off * m.vocab, n, m.softcap);
-        c->launches++;
     }
 }
 
@@ -2962,7 +2910,6 @@ void stack_generate_greedy(StackCtx * c, int32_t first_token, int pos0, int n_st
         enqueue_head(c, 1, 0, true);
         c->token_step = false;
         pdl(c, 1, 1024, 0, k_argmax_advance, c->d_logits, m.vocab, &c->d_step->st, c->d_step->tokens, c->d_out_tokens, c->d_counter);
-        c->launches++;
     };
     if (!c->g_greedy) {
         const int64_t before = c->launches;
@@ -3011,7 +2958,6 @@ int32_t stack_argmax(StackCtx * c) {
     if (c->d_last_row < 0) throw std::runtime_error("no logits yet: the last step asked for none");
     SCU(cudaSetDevice(c->m->device));
     pdl(c, 1, 1024, 0, k_argmax_row, c->d_logits + (size_t) c->d_last_row * c->m->vocab, c->m->vocab, c->d_arg);
-    c->launches++;
     SCU(cudaMemcpyAsync(c->h_arg, c->d_arg, 4, cudaMemcpyDeviceToHost, c->st));
     SCU(cudaStreamSynchronize(c->st));
     return *c->h_arg;
@@ -3022,11 +2968,16 @@ int stack_product_kernel(int dtype, int T, int N, int K, bool glu, int sm_count)
     return route == LIN_PAIR ? LIN_UMMA : route;
 }
 
-void stack_product_plan(int dtype, int T, int N, int K, int batch, bool seg, bool glu, int sm_count, int32_t out[2]) {
+void stack_product_plan(int dtype, int T, int N, int K, int batch, bool seg, bool glu, int sm_count, int32_t out[8]) {
     const bool vec = K % (dtype == STACK_F32 ? 4 : 8) == 0;
     const LinRoute route = lin_route(dtype, T, N, K, batch, vec, glu, seg, false, true, 0, 0, SIZE_MAX, sm_count);
+    std::fill(out, out + 8, 0);
     out[0] = route;
     out[1] = route == LIN_SIMT && simt_whole(seg, T, (N + 63) / 64 * ((T + 63) / 64) * batch, sm_count) ? 1 : 0;
+    if (route != LIN_PAIR) return;
+    const PairPlan p = pair_plan(T, N, K, seg ? batch : 0, !glu && !seg, sm_count, umma_part_floats(sm_count));
+    const int32_t v[6] = { p.acc, p.n, p.parts, p.stages, p.sets, pair_work(p, T, N, batch) };
+    std::copy(v, v + 6, out + 2);
 }
 
 void stack_latent_plan(int heads, int rank, int rot, int window, int n_ctx, int T, int sm_count, int32_t out[6]) {
@@ -3054,10 +3005,10 @@ float stack_time_linear(int device, int dtype, int T, int N, int K, int reps) {
         SCU(cudaMalloc(&us.xb, us.elems * 2)); us.part_floats = umma_part_floats(us.sm_count); SCU(cudaMalloc(&us.part, us.part_floats * 4)); SCU(cudaMalloc(&us.err, 4)); SCU(cudaMemset(us.err, 0, 4));
         SCU(cudaStreamCreate(&st)); SCU(cudaEventCreate(&e0)); SCU(cudaEventCreate(&e1));
         bool cold = true;                // one behind the other, as a pass's kernels run
-        for (int i = 0; i < 3; i++) linear_on(Lane{st, &cold}, dtype, nullptr, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
+        for (int i = 0; i < 3; i++) linear_on(Lane{st, &cold}, dtype, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
         SCU(cudaStreamSynchronize(st));
         SCU(cudaEventRecord(e0, st));
-        for (int i = 0; i < reps; i++) linear_on(Lane{st, &cold}, dtype, nullptr, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
+        for (int i = 0; i < reps; i++) linear_on(Lane{st, &cold}, dtype, X, K, (char *) W + wbytes * (size_t) (i % copies), nullptr, Y, N, T, N, K, 1, 0, 0, 0, false, 0.f, &us);
         SCU(cudaEventRecord(e1, st));
         SCU(cudaStreamSynchronize(st));
         cudaEventElapsedTime(&ms, e0, e1);
@@ -3109,7 +3060,7 @@ void products(int device, int dtype, int T, int N, int K, int batch, const int32
         }
         bool cold = true;
         for (int i = 0; i < (in_pass ? 2 : 1); i++)
-            linear_on(Lane{nullptr, in_pass ? &cold : nullptr}, dtype, nullptr, X, K, d.w, d.bias, Y, ny, T, N, K, batch, seg ? 0 : (long long) T * K, (long long) N * K, (long long) T * ny, glu != 0, limit, &us, &o);
+            linear_on(Lane{nullptr, in_pass ? &cold : nullptr}, dtype, X, K, d.w, d.bias, Y, ny, T, N, K, batch, seg ? 0 : (long long) T * K, (long long) N * K, (long long) T * ny, glu != 0, limit, &us, &o);
         SCU(cudaDeviceSynchronize());
         if (rounded) {
             std::vector<uint16_t> h(n_out);

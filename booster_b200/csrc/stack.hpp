@@ -62,8 +62,8 @@ void    stack_linear(int device, int dtype, int T, int N, int K, const float * x
 // a batch of such products, x[batch][T][K] on w[batch][N][K], or (seg: batch + 1 first rows) the rows of one x[T][K] sorted by matrix; glu: 1 clamped sigmoid units, 2 GELU units; rounded:
 // bfloat16 units as the pair kernel hands them to the product behind (an error where it does not take the product)
 void    stack_products(int device, int dtype, int T, int N, int K, int batch, const int32_t * seg, const float * x, const float * w, int glu, float limit, bool rounded, float * y);
-// how a pass runs a product (host arithmetic, tests): the kernel, and whether it starts on empty SMs
-void    stack_product_plan(int dtype, int T, int N, int K, int batch, bool seg, bool glu, int sm_count, int32_t out[2]);
+// how a pass runs a product (host arithmetic, tests): the kernel, whether it starts on empty SMs, and on pairs of SMs the plan's accumulators, their columns, K parts, stages, sets, pieces of work
+void    stack_product_plan(int dtype, int T, int N, int K, int batch, bool seg, bool glu, int sm_count, int32_t out[8]);
 // launch shape of a latent layer's attention over a pass of T tokens: tokens and heads per block, key slices, score-row stride, shared memory, whether keys are staged (host arithmetic, tests)
 void    stack_latent_plan(int heads, int rank, int rot, int window, int n_ctx, int T, int sm_count, int32_t out[6]);
 

@@ -138,8 +138,9 @@ int b200_stack_linear_in_pass(int device, int dtype, int T, int N, int K, const 
  * seg[z + 1] - 1 of x[T][K] on matrix z -> y[T][N]. glu: 1 clamped sigmoid units, 2 GELU units (y has N / 2 columns); rounded: the units as bfloat16, as the kernel on pairs of
  * SMs hands them to the product behind it (an error where it does not take the product). Entries that no kernel stores are NaN */
 int b200_stack_products(int device, int dtype, int T, int N, int K, int batch, const int32_t * seg, const float * x, const float * w, int glu, float limit, int rounded, float * y);
-/* how a model's pass runs a product of a batch, or (seg != 0) of rows sorted by `batch` matrices: out[0] the kernel as b200_stack_product_kernel names them, with 8 for tcgen05 (bfloat16) on pairs of SMs, out[1] 1 where it
- * starts on empty SMs instead of beside the end of the kernel in front (host arithmetic, tests) */
+/* how a model's pass runs a product of a batch, or (seg != 0) of rows sorted by `batch` matrices (host arithmetic, tests). out[8]: the kernel as b200_stack_product_kernel names them,
+ * with 8 for tcgen05 (bfloat16) on pairs of SMs; 1 where it starts on empty SMs instead of beside the end of the kernel in front; for pairs also accumulators side by side,
+ * columns of each, K parts (each product of several is followed by a launch that adds them), ring stages, sets of accumulators, pieces of work at most */
 int b200_stack_product_plan(int dtype, int T, int N, int K, int batch, int seg, int glu, int sm_count, int32_t * out);
 /* launch shape of a latent-attention layer over a pass of T tokens (the decode kernels: T < 8): out = tokens per block, heads per block, key slices, score-row
  * stride, bytes of shared memory, 1 where a block's keys are staged in it (host arithmetic, tests) */

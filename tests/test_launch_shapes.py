@@ -166,7 +166,7 @@ def test_stack_product_kernel(dtype, T, N, K, glu, want):
 
 
 def product_plan(dtype, T, N, K, batch=1, seg=0, glu=0, sm_count=148):
-    out = (C.c_int32 * 2)()
+    out = (C.c_int32 * 8)()
     assert _lib.lib().b200_stack_product_plan(dtype, T, N, K, batch, seg, glu, sm_count, out) == 0
     return tuple(out)
 
@@ -176,7 +176,7 @@ def product_plan(dtype, T, N, K, batch=1, seg=0, glu=0, sm_count=148):
     (F32, 7, 4736, 1024, 1, 0, 0, 1), (F32, 7, 4672, 1024, 1, 0, 0, 0), (F32, 7, 64, 1024, 74, 0, 0, 1), (F32, 7, 64, 1024, 73, 0, 0, 0), (BF16, 7, 8192, 1020, 1, 0, 1, 1),      # 74 tiles of 64 rows
     (F32, 32, 1024, 1024, 1, 0, 0, 0), (F32, 33, 1024, 1024, 1, 0, 0, 1), (F32, 63, 1024, 1024, 1, 0, 0, 1), (F32, 64, 63, 1024, 1, 0, 0, 0)])
 def test_large_grids_of_fp32_tiles_start_on_empty_sms(dtype, T, N, K, batch, seg, glu, want):
-    assert product_plan(dtype, T, N, K, batch, seg, glu) == (6, want)
+    assert product_plan(dtype, T, N, K, batch, seg, glu)[:2] == (6, want)
 
 
 @pytest.mark.parametrize("T,N,K,batch,seg,want", [

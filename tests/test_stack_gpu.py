@@ -555,6 +555,20 @@ def run_products(x, w, seg=None, glu=0, limit=0.0, rounded=False):
     return y
 
 
+def test_launches_are_counted_as_they_are_made(tmp_path):
+    """a portion of one minGRU layer whose norm leaves rounded rows: embedding, input product (nothing to round) and gates, rounding, output product, end of the layer, last norm, head;
+    and a K-part sum where the plan has one"""
+    p = Pair(tmp_path, config([mingru(width=512)], width=256, groups=4, vocab=160), dtype="bfloat16")
+    def parts(N, K):
+        out = (C.c_int32 * 8)()
+        assert _lib.lib().b200_stack_product_plan(0, 64, N, K, 1, 0, 0, 148, out) == 0 and out[0] == 8
+        return 1 + (out[4] > 1)
+    before = p.ctx.kernel_launches()
+    p.ctx.decode_rows(p.tokens(64), 0, [63])
+    assert p.ctx.kernel_launches() - before == 1 + parts(1536, 256) + 1 + 1 + parts(256, 512) + 1 + 1 + 1
+    p.close()
+
+
 def sorted_rows(counts):
     return np.concatenate([[0], np.cumsum(counts)])
 
