@@ -281,7 +281,7 @@ struct StackCtx {
     int * da_counter = nullptr;           // per (token, head): slices done
     int sm_count = 148;
     __nv_bfloat16 * xb = nullptr;         // activations of a prompt pass rounded to bfloat16 (operand of the tcgen05 product)
-    __nv_bfloat16 * u16 = nullptr;        // gated units of a prompt pass as their product left them, rounded (as many entries as xb)
+    __nv_bfloat16 * u16 = nullptr;        // gated units of a prompt pass as their product left them, rounded
     __nv_bfloat16 * h16 = nullptr;        // Hn rounded, where this pass's norms leave it so ...
     bool h16_on = false;                  // ... and whether they do
     size_t xb_elems = 0;
@@ -2703,9 +2703,12 @@ StackCtx * stack_ctx_new(StackModel * m, int n_ctx) {
             c->xb_elems = std::max(cap * (size_t) std::max({ 2 * m->E, m->maxA, m->maxOL, m->maxP, m->max_dense, m->side_dim }), moe_rows * (size_t) std::max(m->E, m->max_eff));
             c->xb_elems = (c->xb_elems + 63) / 64 * 64;
             const bool norms = m->block == BLOCK_SHARED || m->block == BLOCK_SEQUENTIAL;
-            SCU(cudaMalloc(&c->xb, (2 * c->xb_elems + (norms ? cap * m->E : 0)) * 2));      // one allocation: a context is made per sequence
+            size_t units = moe_rows * (size_t) m->max_eff;             // gated_ff: the experts', and the dense feed-forwards of the blocks that use it
+            if (norms) for (const LayerSpec & L : m->layers) if (L.has_mlp) units = std::max(units, cap * (size_t) L.ff);
+            units = (units + 63) / 64 * 64;
+            SCU(cudaMalloc(&c->xb, (c->xb_elems + units + (norms ? cap * m->E : 0)) * 2));      // one allocation: a context is made per sequence
             c->u16 = c->xb + c->xb_elems;
-            if (norms) c->h16 = c->u16 + c->xb_elems;
+            if (norms) c->h16 = c->u16 + units;
             c->xpart_floats = umma_part_floats(c->sm_count);
         } else c->xpart_floats = f32_part_floats(*m, c->cap, c->sm_count);
         if (c->xpart_floats) SCU(cudaMalloc(&c->xpart, c->xpart_floats * 4));

@@ -398,3 +398,18 @@ def test_bad_models_fail_loudly(tmp_path):
     c4 = copy.deepcopy(cfg); c4["layers"][1]["mixer"]["kv_heads"] = 3
     with pytest.raises(_lib.B200Error, match="multiple of kv_heads"):
         engine.Model(do.write_model(str(tmp_path / "heads"), c4, w))
+
+
+def test_bfloat16_contexts_hold_no_room_for_units_they_never_make(tmp_path):
+    """this design's feed-forwards have no gated units: a context of one with 8192 entries has its float32 buffers (two), its rounded rows (one) and the K parts, and no rounded units
+    (8 MB)"""
+    torch = pytest.importorskip("torch")
+    p = Pair(tmp_path, config([gdelta(mlp=ff(8192))], width=64), dtype="bfloat16")
+    torch.cuda.init()
+    free = torch.cuda.mem_get_info()[0]
+    more = [engine.Context(p.model, 512) for _ in range(8)]
+    used = (free - torch.cuda.mem_get_info()[0]) / 8
+    assert used < 512 * 8192 * (4 + 4 + 2) + 148 * 128 * 256 * 4 + (8 << 20), used      # (the rest: 4 MB)
+    for c in more:
+        c.close()
+    p.close()
