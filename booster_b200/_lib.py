@@ -24,7 +24,7 @@ B200_SYMBOLS = ["b200_last_error", "b200_device_count", "b200_version", "b200_mo
                 "b200_comm_init", "b200_p2p_handle", "b200_p2p_connect", "b200_p2p_disable", "b200_pipeline_generate_greedy", "b200_pipeline_decode", "b200_stage_forward", "b200_stage_batch_usable", "b200_stage_forward_batch",
                 "b200_stage_logits", "b200_stage_argmax", "b200_stage_logits_view", "b200_decode_view", "b200_stage_sync", "b200_stage_raise", "b200_kv_write", "b200_kv_read", "b200_kv_seq_rm", "b200_kv_seq_add", "b200_kv_seq_div", "b200_op_quantize_q8_K", "b200_op_quantize_q8_0",
                 "b200_op_dequantize_row", "b200_op_mul_mat_vec", "b200_op_mul_mat", "b200_op_rms_norm", "b200_op_rope",
-                "b200_op_attention", "b200_set_attention_route", "b200_tokenizer_load", "b200_tokenizer_free", "b200_tokenizer_n_vocab", "b200_tokenize",
+                "b200_op_attention", "b200_op_attention_one_launch", "b200_op_attention_cluster", "b200_set_attention_route", "b200_tokenizer_load", "b200_tokenizer_free", "b200_tokenizer_n_vocab", "b200_tokenize",
                 "b200_token_to_piece", "b200_token_is_eog", "b200_token_nl", "b200_cpt_class", "b200_op_launch_shape", "b200_op_lanes_shape", "b200_op_score_tokens", "b200_op_prompt_kernel",
                 "b200_sampler_new", "b200_sampler_set_standard", "b200_sampler_free", "b200_sampler_reset", "b200_sampler_sample"]
 
@@ -130,6 +130,8 @@ def lib() -> C.CDLL:
     sig("b200_op_mul_mat", C.c_int, [C.c_int, vp, C.c_int64, C.c_int64, f32p, C.c_int64, f32p])
     sig("b200_op_rms_norm", C.c_int, [f32p, f32p, C.c_int64, C.c_float, f32p])
     sig("b200_op_rope", C.c_int, [f32p, C.c_int, C.c_int, C.c_int, C.c_float, C.c_float, f32p])
+    sig("b200_op_attention_one_launch", C.c_int, [C.c_int] * 5)
+    sig("b200_op_attention_cluster", C.c_int, [C.c_int] * 3)
     sig("b200_op_attention", C.c_int, [f32p, C.POINTER(C.c_uint16), C.POINTER(C.c_uint16), C.c_int, C.c_int, C.c_int,
                                        C.c_int, C.c_float, C.c_int, f32p])
     sig("b200_set_attention_route", None, [C.c_int])

@@ -6,7 +6,7 @@
 // (token, pos) live in device memory (DecodeState) so the graph never needs re-instantiation.
 //
 //   per layer:  qkv    (k_matvec_kq, k_matvec_q80) [RMSNorm(attn_norm)+Q8_K quant] -> wq|wk|wv -> RoPE -> q (f32), K/V (f16 cache)
-//               k_attn_cluster     short contexts of 4 and 8 heads per key head: all of a layer's attention, a cluster per KV head; else
+//               k_attn_cluster     contexts made for up to 1024 (4 heads per key head, Q8_0) or 1536 (8 heads) positions: all of a layer's attention, a cluster per KV head; else
 //               k_attn_scores      raw K.q scores of the f16 cache (GQA group per CTA, 64 positions each)
 //               k_attn_softmax_pv  soft-max of the score rows + P.V -> kqv_merged_cont
 //               wo              [quant] -> wo -> + residual                          (ffn_inp)
@@ -950,73 +950,97 @@ static bool attn_2k_enabled() {
     return v == 1 && g_attn_route != 1;
 }
 
-// one launch (k_attn_cluster): a cluster of CL blocks per KV head, all clusters on the GPU at once. False where the context's scores and weights leave no room for a ring, or the
-// clusters do not fit beside one another
+// one launch (k_attn_cluster): a cluster of CL blocks per KV head, all clusters on the GPU at once. No stages where the context's scores and weights leave no room for a ring, or the
+// clusters do not fit beside one another. What fits is asked once per device and KB of shared memory: the answer is the same whichever contexts came before
+struct AttnClusterPlan { int cl = 0, stages = 0; size_t smem = 0; };
 template <int GQA, int CL>
-static bool launch_attention_cluster_as(b200_ctx * c, const AttnArgs & a_in, int n_ctx_pad) {
+static AttnClusterPlan attn_cluster_plan_as(int device, int n_head_kv, int n_ctx_pad) {
     const int n16 = n_ctx_pad / 16, need = (ac_own(n16, CL) + AC_ROWS - 1) / AC_ROWS + (n16 * (16 / CL) + AC_ROWS - 1) / AC_ROWS + 1;
     const size_t beside = ac_beside(GQA, CL, n16);
     int stages = 0;
     for (int s : AC_STAGES) if ((size_t) s * AC_STAGE + beside <= AC_SMEM) { stages = s; if (s >= need) break; }
-    if (stages < std::min(need, 4)) return false;
-    const size_t smem = (size_t) stages * AC_STAGE + beside;
+    if (stages < std::min(need, 4)) return {};
+    const size_t kb = ((size_t) stages * AC_STAGE + beside + 1023) / 1024;      // AC_SMEM is a number of KB
     auto kern = k_attn_cluster<GQA, CL>;
+    static bool raised[64] = {false};
+    static int clusters[64][AC_SMEM / 1024 + 1] = {{0}};       // at once, and one more (0: not asked yet)
+    const int dv = device & 63;
+    std::lock_guard<std::mutex> attr_lock(g_attr_mu);
+    if (!raised[dv]) {
+        if (CL > 8) CU(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) AC_SMEM));
+        raised[dv] = true;
+    }
+    int & n = clusters[dv][kb];
+    if (n == 0) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(CL, 1); cfg.blockDim = dim3(AC_THREADS); cfg.dynamicSmemBytes = kb * 1024;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        n++;
+    }
+    return n - 1 < n_head_kv ? AttnClusterPlan{} : AttnClusterPlan{CL, stages, kb * 1024};
+}
+// Where the one launch is the faster one, by the size of the context and not by the position in it: a context keeps one route from its first token to its last. Behind Q8_0's qkv, and with
+// eight heads per key head, whose K-quant qkv fills the SMs as well, no block of k_attn_scores finds room before qkv
+// ends, and a second launch is 2.5 us a layer; blocks of a long context have more to do than half of the SMs do in that time. Tokens of one launch in parts of two launches' (B200; three file
+// types, at the end and at an eighth of contexts of 256 to 2048): eight heads per key head 0.93 to 1.01 up to 1536, 1.02 at 2048; four behind Q8_0 0.96 to 0.98 up to 1024, 1.00 at 1536;
+// four behind K-quants 0.99 to 1.00 up to 512 and 1.02 from 768 on; one and two heads 0.94 to 1.10. Where qkv leaves SMs to k_attn_scores two launches are as fast or faster: four heads per
+// key head on 1, 2, 4 and 6 key heads (24, 48, 96 and 144 units of qkv's rows) behind Q8_0 1.00 to 1.02, 1.00 to 1.02, 0.99 to 1.02 and 0.96 to 1.00; eight on 1, 2 and 4 (40, 80 and 160)
+// 0.99 to 1.01, 0.93 to 1.00 and 0.92 to 0.98. qkv_units: units of 32 rows, a block each while there are SMs.
+static bool attn_cluster_pays(int gqa, int n_ctx_pad, int qkv_units, bool q8_0, int sm_count) {
+    if (gqa == 8) return n_ctx_pad <= 1536 && qkv_units >= sm_count / 2;
+    return gqa == 4 && n_ctx_pad <= 1024 && q8_0 && qkv_units >= sm_count * 3 / 4;
+}
+extern "C" int b200_op_attention_one_launch(int gqa, int n_ctx, int qkv_units, int q8_0, int sm_count) { return attn_cluster_pays(gqa, n_ctx, qkv_units, q8_0 != 0, sm_count) ? 1 : 0; }
+// the plan that a context's attention takes on its device; cl 0: two launches or three
+template <int GQA>
+static AttnClusterPlan attn_cluster_plan(const b200_ctx * c, int n_head_kv, int n_ctx_pad) {
+    if constexpr (GQA >= 4) {
+        if (g_attn_route == 2 || !attn_2k_enabled()) return {};
+        if (g_attn_route != 3) {
+            if (!c->m || c->m->layers.empty()) return {};
+            const auto & qkv = c->m->layers[0].qkv;
+            if (!attn_cluster_pays(GQA, n_ctx_pad, qkv.n_units, qkv.seg[0].type == T_Q8_0, c->sm_count)) return {};
+        }
+        AttnClusterPlan p;
+        if (n_head_kv * 16 <= c->sm_count) p = attn_cluster_plan_as<GQA, 16>(c->device, n_head_kv, n_ctx_pad);
+        if (!p.cl && n_head_kv * 8 <= c->sm_count) p = attn_cluster_plan_as<GQA, 8>(c->device, n_head_kv, n_ctx_pad);
+        return p;
+    }
+    return {};
+}
+template <int GQA, int CL>
+static void launch_attention_cluster_as(b200_ctx * c, AttnArgs a, int n_ctx_pad, const AttnClusterPlan & p) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(CL, (unsigned) a_in.n_head_kv); cfg.blockDim = dim3(AC_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = c->st;
+    cfg.gridDim = dim3(CL, (unsigned) a.n_head_kv); cfg.blockDim = dim3(AC_THREADS); cfg.dynamicSmemBytes = p.smem; cfg.stream = c->st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
-    static size_t attr[64] = {0};
-    static int clusters[64] = {0};                             // at once, with the shared memory in attr
-    const int dv = c->device & 63;
-    {
-        std::lock_guard<std::mutex> attr_lock(g_attr_mu);
-        if (smem > attr[dv]) {
-            if (CL > 8) CU(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-            attr[dv] = smem;
-            if (cudaOccupancyMaxActiveClusters(&clusters[dv], kern, &cfg) != cudaSuccess) { cudaGetLastError(); clusters[dv] = 0; }
-        }
-        if (clusters[dv] < a_in.n_head_kv) return false;
-    }
-    AttnArgs a = a_in;
+    cfg.attrs = at; cfg.numAttrs = pdl_enabled() ? 2 : 1;
     g_kind = KIND_ATTN; ProfScope ps(c);
     a.trace = trace_slot(c, CL * a.n_head_kv);
-    if (pdl_enabled()) cfg.numAttrs = 2;
-    CU(cudaLaunchKernelEx(&cfg, kern, a, n16, stages));
+    CU(cudaLaunchKernelEx(&cfg, k_attn_cluster<GQA, CL>, a, n_ctx_pad / 16, p.stages));
     c->launches += 1;
-    return true;
-}
-// Where the one launch is the faster one. Behind Q8_0's qkv, and with eight heads per key head, whose K-quant qkv fills the SMs as well, no block of k_attn_scores finds room before qkv
-// ends, and a second launch is 2.5 us a layer; blocks of a long context have more to do than half of the SMs do in that time. Tokens of one launch in parts of two launches' (B200; three file
-// types, at the end and at an eighth of contexts of 256 to 2048): eight heads per key head 0.93 to 1.01 up to 1536, 1.02 at 2048; four behind Q8_0 0.96 to 0.98 up to 1024, 1.00 at 1536;
-// four behind K-quants 0.99 to 1.00 up to 512 and 1.02 from 768 on; one and two heads 0.94 to 1.10. Where qkv leaves SMs to k_attn_scores two launches are as fast or faster: four heads per
-// key head on 1, 2, 4 and 6 key heads (24, 48, 96 and 144 units of qkv's rows) behind Q8_0 1.00 to 1.02, 1.00 to 1.02, 0.99 to 1.02 and 0.96 to 1.00; eight on 1, 2 and 4 (40, 80 and 160)
-// 0.99 to 1.01, 0.93 to 1.00 and 0.92 to 0.98.
-static bool attn_cluster_pays(const b200_ctx * c, int gqa, int n_ctx_pad) {
-    if (g_attn_route == 3) return true;
-    if (!c->m || c->m->layers.empty()) return false;
-    const auto & qkv = c->m->layers[0].qkv;                    // units of 32 rows, a block each while there are SMs
-    if (gqa == 8) return n_ctx_pad <= 1536 && qkv.n_units >= c->sm_count / 2;
-    return gqa == 4 && n_ctx_pad <= 1024 && qkv.seg[0].type == T_Q8_0 && qkv.n_units >= c->sm_count * 3 / 4;
 }
 template <int GQA>
 static bool launch_attention_cluster(b200_ctx * c, const AttnArgs & a, int n_ctx_pad) {
+    const AttnClusterPlan p = attn_cluster_plan<GQA>(c, a.n_head_kv, n_ctx_pad);
     if constexpr (GQA >= 4) {
-        if (g_attn_route == 2 || !attn_cluster_pays(c, GQA, n_ctx_pad)) return false;
-        const int heads = a.n_head_kv, sms = c->sm_count;
-        if (heads * 16 <= sms && launch_attention_cluster_as<GQA, 16>(c, a, n_ctx_pad)) return true;
-        return heads * 8 <= sms && launch_attention_cluster_as<GQA, 8>(c, a, n_ctx_pad);
+        if (p.cl == 16) launch_attention_cluster_as<GQA, 16>(c, a, n_ctx_pad, p);
+        else if (p.cl == 8) launch_attention_cluster_as<GQA, 8>(c, a, n_ctx_pad, p);
     }
-    return false;
+    return p.cl != 0;
 }
 
 template <int GQA>
 static void launch_attention_t(b200_ctx * c, const AttnArgs & a_in, int n_ctx_pad) {
-    if (attn_2k_enabled() && launch_attention_cluster<GQA>(c, a_in, n_ctx_pad)) return;
+    if (launch_attention_cluster<GQA>(c, a_in, n_ctx_pad)) return;
     if (attn_2k_enabled() && launch_attention_2k<GQA>(c, a_in, n_ctx_pad)) return;
     // long-context route (the GQA score rows do not fit one CTA's shared memory): scores, softmax, chunked P.V
     AttnArgs a = a_in;
@@ -3032,6 +3056,17 @@ extern "C" int b200_op_rope(float * x, int n_heads, int head_dim, int pos, float
     } catch (const std::exception & e) { return set_err(e.what()); }
 }
 
+extern "C" int b200_op_attention_cluster(int n_head, int n_head_kv, int n_ctx) {
+    try {
+        require_gpu();
+        if (n_ctx <= 0 || n_head <= 0 || n_head_kv <= 0 || n_head % n_head_kv) throw std::runtime_error("bad arguments");
+        b200_ctx tmp;
+        CU(cudaGetDevice(&tmp.device));
+        CU(cudaDeviceGetAttribute(&tmp.sm_count, cudaDevAttrMultiProcessorCount, tmp.device));
+        const int n_pad = (n_ctx + 31) / 32 * 32;
+        return n_head / n_head_kv == 4 ? attn_cluster_plan<4>(&tmp, n_head_kv, n_pad).cl : n_head / n_head_kv == 8 ? attn_cluster_plan<8>(&tmp, n_head_kv, n_pad).cl : 0;
+    } catch (const std::exception & e) { set_err(e.what()); return -1; }
+}
 extern "C" int b200_op_attention(const float * q, const uint16_t * k_cache, const uint16_t * v_cache, int n_kv,
                                  int n_head, int n_head_kv, int head_dim, float scale, int round_q, float * out) {
     try {

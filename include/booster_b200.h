@@ -328,6 +328,11 @@ int b200_op_rope(float * x, int n_heads, int head_dim, int pos, float freq_base,
  * round_q = 0: batch-1 arithmetic (tinyBLAS F16xF32); 1: batch>1 (q rounded to f16, ggml_vec_dot_f16). */
 int b200_op_attention(const float * q, const uint16_t * k_cache, const uint16_t * v_cache, int n_kv,
                       int n_head, int n_head_kv, int head_dim, float scale, int round_q, float * out);
+/* whether a decode step's attention takes one launch a layer (a cluster of blocks per key head) instead of two: `gqa` heads per key head, a context allocated with n_ctx positions, qkv of
+ * qkv_units x 32 rows in Q8_0 or not (host arithmetic, tests) */
+int b200_op_attention_one_launch(int gqa, int n_ctx, int qkv_units, int q8_0, int sm_count);
+/* blocks of the cluster that b200_op_attention launches per key head under the present route over n_ctx positions, 0 where it takes two or three launches, -1 on error */
+int b200_op_attention_cluster(int n_head, int n_head_kv, int n_ctx);
 /* which kernels run the attention: 0 = automatic (scores + fused softmax/P.V when the GQA score rows of the context fit
  * one CTA's shared memory, else the three-launch long-context route), 1 = always the long-context route. Process-wide;
  * exists so that tests cover both routes at every size. */

@@ -186,3 +186,41 @@ def test_large_grids_of_fp32_tiles_start_on_empty_sms(dtype, T, N, K, batch, seg
 def test_bfloat16_products_of_portions(T, N, K, batch, seg, want):
     """8 pairs of SMs, 3 a block per tile, 5 mma.sync: few tokens go to the tensor memory from 256 rows and three slices of k on, 64 and more from 128 rows and one slice"""
     assert product_plan(BF16, T, N, K, batch, seg)[0] == want
+
+
+@pytest.mark.parametrize("sm_count", [2, 20, 132, 148])
+@pytest.mark.parametrize("seg", [0, 1, 8, 512])
+def test_every_plan_of_a_pair_is_one_the_kernel_takes(seg, sm_count):
+    """what k_gemm_bf16_pair assumes, over portions of 5 to 40000 tokens: accumulators that fit tensor memory and cover the tokens, a ring of two stages and more, K parts with a slice each whose
+    sums fit their room, and at least one piece of work"""
+    for T in (5, 31, 32, 33, 63, 64, 65, 96, 255, 256, 257, 300, 511, 512, 513, 700, 1024, 2048, 5000, 32768, 40000):
+        for N in (128, 254, 256, 258, 512, 2048, 16384, 32000):
+            for K in (64, 72, 192, 520, 2048, 8192, 16384):
+                for glu in (0, 1):
+                    route, _, acc, n, parts, stages, sets, work = product_plan(BF16, T, N, K, max(seg, 1), 1 if seg else 0, glu, sm_count)
+                    if route != 8:
+                        assert T < 64 and (N < 256 or K < 192)
+                        continue
+                    assert acc in (1, 2) and n % 32 == 0 and 32 <= n <= 256 and sets in (1, 2) and sets * acc * n <= 512
+                    stage = (128 + acc * n // 2) * 64 * 2
+                    assert 2 <= stages <= 8 and stages * stage <= 200 * 1024 and (stages == 8 or (stages + 1) * stage > 200 * 1024)
+                    assert 1 <= parts <= max(1, (K + 63) // 64 // 2) and (parts == 1 or not (glu or seg)) and (parts == 1 or parts * T * N <= sm_count * 128 * 256)
+                    rows = (N + 255) // 256
+                    assert work == (rows * seg * ((T + 255) // 256) if seg else rows * -(-T // (acc * n)) * parts)
+
+
+@pytest.mark.parametrize("T,N,K,glu,want", [
+    (512, 16384, 2048, 1, (2, 256, 1, 4, 1, 64)), (512, 2048, 8192, 0, (1, 256, 4, 6, 2, 64)), (512, 2048, 2048, 0, (1, 64, 1, 8, 2, 64)),
+    (16, 2048, 8192, 0, (1, 32, 8, 8, 2, 64)), (64, 16384, 2048, 1, (1, 64, 1, 8, 2, 64))])
+def test_plans_of_pairs(T, N, K, glu, want):
+    """the measured shapes: accumulators, columns of each, K parts, stages, sets, pieces of work"""
+    assert product_plan(BF16, T, N, K, 1, 0, glu)[2:] == want
+
+
+@pytest.mark.parametrize("gqa,n_ctx,units,q8_0,want", [
+    (8, 1536, 320, 0, 1), (8, 1537, 320, 0, 0), (8, 512, 74, 1, 1), (8, 512, 73, 1, 0),                                           # 64 heads on 8; half of the SMs
+    (4, 1024, 192, 1, 1), (4, 1025, 192, 1, 0), (4, 512, 192, 0, 0), (4, 512, 111, 1, 1), (4, 512, 110, 1, 0),                     # 32 heads on 8 in Q8_0; three quarters
+    (2, 256, 400, 1, 0), (1, 256, 400, 1, 0)])
+def test_one_launch_attention(gqa, n_ctx, units, q8_0, want):
+    """whether a token's attention takes one launch a layer; the context's allocated size decides, wherever the token is in it"""
+    assert _lib.lib().b200_op_attention_one_launch(gqa, n_ctx, units, q8_0, 148) == want

@@ -133,6 +133,26 @@ def test_attention_routes_bit_exact(cfg, round_q, route):
         engine.set_attention_route(0)
 
 
+@pytest.mark.parametrize("cfg,want", [((4, 1, 17), {16}), ((8, 1, 33), {16}), ((16, 4, 2050), {16}), ((32, 8, 130), {8, 16}), ((32, 8, 333), {8, 16}), ((64, 8, 1029), {8, 16}),
+                                      ((64, 16, 700), {0, 8}), ((8, 1, 9000), {0}), ((8, 2, 20011), {0}), ((64, 32, 100), {0}), ((2, 2, 100), {0})])
+def test_the_one_launch_attention_runs_where_it_is_asked_for(cfg, want):
+    """blocks of a cluster: as many as fit beside one another (eight clusters of 16 do not on every GPU, nor sixteen of 8), whatever was asked for before; 0 where the routes test
+    compares two launches with themselves"""
+    ask = _lib.lib().b200_op_attention_cluster
+    try:
+        engine.set_attention_route(3)
+        first = ask(*cfg)
+        assert first in want
+        for n_kv in (8000, 32, 4200, 1536):
+            ask(cfg[0], cfg[1], n_kv)
+        assert ask(*cfg) == first
+        for route in (2, 1, 0):                               # (0: products by themselves stand behind no qkv)
+            engine.set_attention_route(route)
+            assert ask(*cfg) == 0
+    finally:
+        engine.set_attention_route(0)
+
+
 @pytest.mark.parametrize("cfg", [(2, 2, 50176), (2, 2, 12000), (4, 2, 25088), (8, 2, 12544), (8, 1, 6272), (8, 2, 7200), (2, 2, 14208), (2, 2, 11360), (2, 2, 11361)])
 def test_attention_where_v_goes_round_its_slots(cfg):
     """soft-max . V of one token: the longest context of each number of heads per key head (slots of 96 to 352 positions), and V that just fits its four slots and just does not"""
