@@ -23,8 +23,11 @@ namespace stk {
 
 // Programmatic dependent launch: a pass's kernels are launched so that one may become resident while the one before it still runs. pdl_launch_dependents() lets the next
 // kernel's blocks in as soon as there is room, pdl_wait() returns when the kernel before has completed and its writes are visible. Every kernel here waits before it reads
-// anything another kernel writes and before it writes anything: what may come first are its own set-up and reads of weights. A kernel that waits for its predecessor thereby
-// waits for all before it, since that one has waited too: no path through a kernel leaves out the wait. Without the launch attribute both are no-ops.
+// anything that another kernel of its pass writes, and before it writes anything. A kernel that waits for its predecessor thereby waits for all before it, since that one has waited
+// too: no path through a kernel leaves out the wait. Without the launch attribute both are no-ops.
+// Ahead of the wait stand set-up, weights, and what was written before the pass's first launch: the step's header (StepState, tokens), cached rows of positions below pos0
+// (k_latent_attn_staged, k_gqa_attn_group) and the recurrent state that only the kernel itself moves on (k_delta_scan). That holds because the first launch of every pass is whole:
+// enqueue_layers sets StackCtx::cold, and the copies of a header and other streams stand in front of such a launch. Whoever lets a pass's first launch overlap breaks these four.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The next kernel is let in behind the wait and not in front of it: earlier, several kernels queue up on the SMs one behind the other, and a large one finds some SMs with room for

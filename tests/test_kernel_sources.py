@@ -81,3 +81,30 @@ def test_stack_kernels_wait_for_the_kernel_before_them(name):
         bad += [f"{kernel}: {m}" for m in re.findall(r"\*\s*__restrict__\s*(\w+)", signature) if m not in weights]
         bad += [f"{kernel}: __ldg of {m}" for m in re.findall(r"__ldg\((.*)", b) if "(w + i)" not in m]
     assert not bad, bad
+
+
+# pointers that a kernel of a pass names ahead of its (last) wait. Weights: read. "st" and "tokens": the step's header, written before the pass's first launch, which is launched
+# whole; so are cached rows below pos0 ("cache" of the two attention kernels) and the state of the delta rule ("S"). The others give addresses, or are used behind a wait further up
+# (k_post_norm_add's `waited`, k_gemv_ring's indexed batch, k_gemm_bf16_pair's segments), or are another thing of that name (a tile's part).
+EARLY = {
+    "k_post_norm_add": {"w_post", "w_next", "Y", "X", "Hn", "H16"}, "k_gemv_ring": {"W", "w_index"}, "k_latent_prep": {"cnorm", "st", "P", "cache"}, "k_latent_attn_staged": {"st", "cache"},
+    "k_causal_conv_rows": {"w", "bias"}, "k_delta_gates": {"CV"}, "k_delta_scan": {"S"}, "k_gqa_prep": {"st", "P", "cache"}, "k_gqa_attn_group": {"st", "cache", "pool"},
+    "k_moe_route": {"Wr", "w_sg", "Hn", "z"}, "k_side_in": {"tokens", "table", "Wg"}, "k_side_out": {"Wp"}, "k_gemm_bf16_pair": {"seg", "part"},
+}
+
+
+def test_what_stack_kernels_name_ahead_of_their_wait():
+    """EARLY, kernel by kernel: a pointer that joins the names ahead of a wait is looked at before it joins this table"""
+    known = {"X", "W", "Y", "Yb", "bias", "seg", "w_index", "x_scale", "QK", "cache", "sink", "st", "OL", "part", "ml", "P", "A", "hist", "w", "Q", "Vv", "S", "O", "ab", "den", "Wg", "Wp", "pool", "r1", "r2",
+             "Wr", "w_sg", "Hn", "z", "Ya", "Yb", "Yk", "wt", "slot_of", "nw", "H16", "keep", "coef", "XS", "counter", "table", "proj", "gate", "norm", "sel", "sg", "fw", "scratch"}
+    found = {}
+    for path in sorted(CSRC.glob("stack_kernels*.cuh")):
+        for body in re.split(r"__global__", "\n".join(_code(path)))[1:]:
+            kernel, start = re.search(r"\b(k_\w+)\s*\(", body).group(1), body.index("{")
+            ends = re.search(r"\n}\n", body).end()
+            early = body[start:max(m.start() for m in re.finditer(r"pdl_(enter|wait)\(\)", body[:ends]))]
+            names = {p for p in re.findall(r"\*\s*(?:__restrict__\s*)?(\w+)\s*[,)=]", body[:start]) if re.search(rf"\b{p}\b", early)}
+            names |= {f for f in re.findall(r"\b[as]\.(\w+)", early) if f in known}
+            if names:
+                found[kernel] = names
+    assert found == EARLY, {k: (found.get(k), EARLY.get(k)) for k in set(found) | set(EARLY) if found.get(k) != EARLY.get(k)}

@@ -573,6 +573,38 @@ def sorted_rows(counts):
     return np.concatenate([[0], np.cumsum(counts)])
 
 
+@pytest.mark.parametrize("counts,N,K", [
+    ([0, 300, 7, 0, 33, 0], 512, 128), ([1, 2, 600], 258, 264), ([257, 0, 0, 256], 130, 64), ([3, 1, 1], 300, 200), ([2] * 511 + [40], 256, 192),      # pairs of SMs: 512 experts at most
+    ([1] * 100 + [0] * 400 + [3] * 13, 128, 64), ([0] * 512 + [300], 136, 72),                                                                      # more: a block per tile
+    ([4, 0, 9], 140, 192), ([30, 1, 0, 25], 600, 72)], ids=lambda v: f"{len(v)}x{max(v)}" if isinstance(v, list) else str(v))      # mma.sync
+def test_rows_sorted_by_expert(counts, N, K):
+    """every row on its own expert's matrix: experts without rows beside full ones, several tiles of tokens to an expert, rows of no expert left alone. Bound:
+    test_bfloat16_products_on_pairs_of_sms"""
+    rng = np.random.default_rng(sum(counts) + N + K)
+    T, extra = sum(counts), 3
+    x = rng.standard_normal((T + extra, K)).astype(np.float32)
+    w = so.round_bf16((rng.standard_normal((len(counts), N, K)) / np.sqrt(K)).astype(np.float32))
+    seg = sorted_rows(counts)
+    y = run_products(x, w, seg)
+    assert np.isnan(y[T:]).all()
+    xe = so.round_bf16(x).astype(np.float64)
+    for z in range(len(counts)):
+        rows = slice(seg[z], seg[z + 1])
+        off = 2 * (K + 8) * 2.0 ** -24 * (np.abs(xe[rows]) @ np.abs(w[z].astype(np.float64)).T)
+        assert (np.abs(y[rows] - xe[rows] @ w[z].astype(np.float64).T) <= off).all(), z
+
+
+@pytest.mark.parametrize("batch,T,N,K", [(3, 64, 128, 64), (2, 129, 257, 328), (5, 70, 1030, 72), (4, 300, 140, 1032), (1, 64, 127, 64), (3, 33, 300, 200)])
+def test_products_of_heads(batch, T, N, K):
+    """k_gemm_bf16_umma, and mma.sync for few tokens: tiles that end inside T, N and K, more slices than stages. Bound: test_bfloat16_products_on_pairs_of_sms"""
+    rng = np.random.default_rng(batch + T + N + K)
+    x = rng.standard_normal((batch, T, K)).astype(np.float32)
+    w = so.round_bf16((rng.standard_normal((batch, N, K)) / np.sqrt(K)).astype(np.float32))
+    xe, we = so.round_bf16(x).astype(np.float64), w.astype(np.float64).transpose(0, 2, 1)
+    off = 2 * (K + 8) * 2.0 ** -24 * (np.abs(xe) @ np.abs(we))
+    assert (np.abs(run_products(x, w) - xe @ we) <= off).all()
+
+
 @pytest.mark.parametrize("counts,N,K,glu,limit", [
     ([5], 256, 192, 1, 7.0), ([300], 514, 136, 1, np.inf), ([600], 1030, 520, 1, 3.0), ([70], 300, 2048, 2, 0.0),              # one matrix: few columns, one accumulator and two
     ([0, 300, 7, 0, 33, 0], 512, 128, 1, np.inf), ([1, 2, 600], 258, 264, 1, 7.0), ([40, 0, 20], 320, 208, 2, 0.0)], ids=str)      # experts: empty ones, a second tile of tokens
