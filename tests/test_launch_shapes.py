@@ -180,11 +180,11 @@ def test_large_grids_of_fp32_tiles_start_on_empty_sms(dtype, T, N, K, batch, seg
 
 
 @pytest.mark.parametrize("T,N,K,batch,seg,want", [
-    (5, 256, 192, 1, 0, 8), (5, 256, 184, 1, 0, 5), (5, 255, 192, 1, 0, 5), (63, 256, 192, 1, 0, 8), (63, 4096, 64, 1, 0, 5), (63, 254, 4096, 1, 0, 5), (5, 256, 196, 1, 0, 6),
+    (5, 256, 64, 1, 0, 8), (5, 256, 56, 1, 0, 5), (5, 255, 64, 1, 0, 5), (63, 256, 64, 1, 0, 8), (63, 4096, 64, 1, 0, 8), (63, 254, 4096, 1, 0, 5), (5, 256, 196, 1, 0, 6),
     (5, 256, 192, 4, 1, 8), (63, 256, 192, 512, 1, 8), (63, 256, 192, 513, 1, 5), (63, 256, 192, 4, 0, 5),                       # experts, more of them than a block notes, heads
     (64, 256, 64, 1, 0, 8), (64, 128, 64, 1, 0, 8), (64, 127, 64, 1, 0, 5), (64, 128, 64, 513, 1, 3), (64, 128, 64, 4, 0, 3), (64, 128, 56, 1, 0, 5)])
 def test_bfloat16_products_of_portions(T, N, K, batch, seg, want):
-    """8 pairs of SMs, 3 a block per tile, 5 mma.sync: few tokens go to the tensor memory from 256 rows and three slices of k on, 64 and more from 128 rows and one slice"""
+    """8 pairs of SMs, 3 a block per tile, 5 mma.sync: few tokens go to the tensor memory from 256 rows on, 64 and more from 128"""
     assert product_plan(BF16, T, N, K, batch, seg)[0] == want
 
 
@@ -199,7 +199,7 @@ def test_every_plan_of_a_pair_is_one_the_kernel_takes(seg, sm_count):
                 for glu in (0, 1):
                     route, _, acc, n, parts, stages, sets, work = product_plan(BF16, T, N, K, max(seg, 1), 1 if seg else 0, glu, sm_count)
                     if route != 8:
-                        assert T < 64 and (N < 256 or K < 192)
+                        assert T < 64 and N < 256
                         continue
                     assert acc in (1, 2) and n % 32 == 0 and 32 <= n <= 256 and sets in (1, 2) and sets * acc * n <= 512
                     stage = (128 + acc * n // 2) * 64 * 2
