@@ -411,7 +411,7 @@ def bench_stack(args):
                            "decode_hbm_frac": m.weight_bytes * n_gen / (np.median(dec) / 1e3) / (hbm * 1e9),
                            "kernel_launches": int(L.b200_kernel_launches(c.h))}
         c.close(); m.close()
-        # the family's products alone: decode mat-vec (T = 1) and prompt product (T = 512) of the gate|up and down shapes
+        # the family's products alone, one behind the other as a pass runs them: decode mat-vec (T = 1) and prompt product (T = 512) of the gate|up and down shapes
         E, ff = sz["width"], sz["ff"]
         kern = {}
         for label, (N, K) in {"gate_up": (2 * ff, E), "down": (E, ff)}.items():

@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(1024) k_moe_sort(const int32_t * sel, int n_sl
     extern __shared__ int ssm[];
     __shared__ int wsum[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // (a word more every 32: neighbouring parts of 32 slots, the threads of a warp, would all be in one bank. 2048 slots 22 us so, 6 now)
+    // (a word more every 32: neighbouring parts of 32 slots, the threads of a warp, would all be in one bank. 2048 slots 22 us of a pass so, 9 now)
     int * cnt = ssm + (in_smem ? n_slots + n_slots / 32 : 0);
     if (in_smem) for (int i = tid; i < n_slots; i += 1024) ssm[i + i / 32] = sel[i];
     const auto es = [&](int i) { return in_smem ? ssm[i + i / 32] : sel[i]; };
@@ -611,14 +611,14 @@ __global__ void __launch_bounds__(1024) k_moe_sort(const int32_t * sel, int n_sl
         for (int i = s0; i < s1; i++) if (es(i) == e) { slot_of[i] = r; src_row[r] = i / top; r++; }
     }
 }
-// Y[r] = X[src_row[r]]
-// rows of 16-bit entries: E a multiple of 8, 16-byte aligned
+// Y[r] = X[src_row[r]], rows of 16-bit entries: E a multiple of 8, 16-byte aligned
 __global__ void k_gather_rows16(const __nv_bfloat16 * X, const int32_t * src_row, int E, __nv_bfloat16 * Y) {
     pdl_enter();
     const uint4 * x = reinterpret_cast<const uint4 *>(X + (size_t) src_row[blockIdx.x] * E);
     uint4 * y = reinterpret_cast<uint4 *>(Y + (size_t) blockIdx.x * E);
     for (int i = threadIdx.x; i < E / 8; i += blockDim.x) y[i] = x[i];
 }
+// Y[r] = X[src_row[r]]
 __global__ void k_gather_rows(const float * X, int ldx, const int32_t * src_row, int E, float * Y) {
     pdl_enter();
     const int r = blockIdx.x;
