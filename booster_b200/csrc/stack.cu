@@ -1397,7 +1397,7 @@ enum LinRoute { LIN_ROWS = 0, LIN_ROWS_LONG = 1, LIN_RING = 2, LIN_UMMA = 3, LIN
 LinRoute lin_route(int dtype, int T, int N, int K, int batch, bool vec, bool glu, bool seg, bool indexed, bool scratch, size_t x_elems, size_t xb_elems, size_t part_floats, int sm_count) {
     if (vec && ring_takes(K) && (T == 1 || (T <= GEMV_MAX_T && batch == 1 && !seg && !indexed && ring_takes_tokens(dtype, T, N, K)))) return LIN_RING;
     if (T <= GEMV_MAX_T) return !glu && batch == 1 && N <= GEMV_FEW_ROWS && K >= 1024 ? LIN_ROWS_LONG : LIN_ROWS;      // few, long rows: a block each
-    // 5 to 63 tokens: a pair's columns are as few, from half of its rows on. Inside a pass, with the rounding launch in front, 256 to 4096 rows of 5 to 63 tokens take 0.72 to 0.89 of mma.sync's
+    // 5 to 63 tokens: a pair's columns are as few, and its 256 rows are taken whole. Inside a pass, with the rounding launch in front, 256 to 4096 rows of 5 to 63 tokens take 0.72 to 0.89 of mma.sync's
     // time at k = 64 (5.7 to 6.9 us against 6.7 to 8.9), 0.63 to 0.79 at 128, 0.60 to 0.76 at 160. (Started cold, by themselves, 9.3 us against 8.3 at k = 64 and the same from 128 on.)
     const bool few = N >= PG_ROWS && (batch == 1 || seg) && pair_takes(N, seg ? batch : 0);
     if (dtype == STACK_BF16 && vec && umma_enabled() && K >= 64 && x_elems <= xb_elems && ((T >= 64 && N >= 128) || few)) return (batch == 1 || seg) && pair_takes(N, seg ? batch : 0) ? LIN_PAIR : LIN_UMMA;
