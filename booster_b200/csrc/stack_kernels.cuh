@@ -889,7 +889,7 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
         if (dead) { *failed = 1; atomicExch(err, 1); for (int i = 0; i < 1000; i++) __nanosleep(1000); }      // MMAs under way end before tensor memory is given back
         __syncwarp();
     }
-    const bool ok = mbar_wait_limited(smem_addr(&done), 0u, failed, err) && !*failed;
+    const bool ok = __all_sync(0xffffffffu, mbar_wait_limited(smem_addr(&done), 0u, failed, err) && !*failed);      // for a whole warp: it loads its accumulators together
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok) {
         const int m = m0 + 32 * (warp & 3) + lane, cbase = (warp >> 2) * (UM_BN / 2);
@@ -901,6 +901,7 @@ __global__ void __launch_bounds__(256, 1) k_gemm_bf16_umma(const __grid_constant
         for (int c = 0; c < UM_BN / 2; c += 16) {
             uint32_t r[16];
             float v[16];
+            __syncwarp();
 #pragma unroll
             for (int j = 0; j < 16; j += 4)
                 asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[j]), "=r"(r[j + 1]), "=r"(r[j + 2]), "=r"(r[j + 3]) : "r"(taddr + (uint32_t) (c + j)) : "memory");

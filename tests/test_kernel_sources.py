@@ -66,6 +66,20 @@ def test_accumulators_are_read_behind_the_wait_for_them(name):
 
 
 @pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("stack_kernels*.cuh")))
+def test_a_warp_loads_accumulators_whole(name):
+    """tcgen05.ld is an instruction of the whole warp. A bounded wait may run out for some of its lanes and not for others: what decides by it whether accumulators are loaded is the same for
+    all lanes, and a loop that lanes leave early in (continue) meets before the next load"""
+    text = "\n".join(_code(CSRC / name))
+    bad = [m.group(0) for m in re.finditer(r"const bool \w+ = [^;]*mbar_wait_limited\([^;]*;", text) if "__all_sync(" not in m.group(0)]
+    for m in re.finditer(r"continue;", text):
+        head = text.rfind("#pragma unroll 1", 0, m.start())
+        loop = text[head:m.start()]
+        if head >= 0 and "tcgen05.ld" in loop and "__syncwarp();" not in loop[:loop.index("tcgen05.ld")]:
+            bad.append(text[:m.start()].count("\n") + 1)
+    assert not bad, bad
+
+
+@pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("stack_kernels*.cuh")))
 def test_stack_kernels_wait_for_the_kernel_before_them(name):
     """a pass's kernels become resident while the one before still runs: each waits before it reads what another wrote, and reads that coherently (no __ldg, no read-only pointer of
     what a pass computes: the compiler may take such a load for one of a constant and move it ahead of the wait)"""
